@@ -157,6 +157,16 @@ int spion_block_attn_backward(spion_ctx* ctx, const float* Q, const float* K, co
                               float* dQ, float* dK, float* dV,
                               const int* offsets, const int* columns, const int* sum_mat, int nnz);
 
+/* The same two calls with every operand in [BH, L, d] (no transposed copies of K and V) and, in the backward, the forward's
+ * output O: with it the fused kernels need one pass over a block row instead of two (O may be NULL).  dP_scratch is used by the
+ * per-stage kernels only: NULL when spion_block_attn_needs_scratch(ctx) is 0. */
+int spion_block_attn_forward_rm(spion_ctx* ctx, const float* Q, const float* K, const float* V, const float* keypad,
+                                float* attn, float* out, const int* offsets, const int* columns, const int* sum_mat, int nnz);
+int spion_block_attn_backward_rm(spion_ctx* ctx, const float* Q, const float* K, const float* V, const float* P,
+                                 const float* O, const float* dO, float* dP_scratch, float* dS_scratch, float* dQ, float* dK,
+                                 float* dV, const int* offsets, const int* columns, const int* sum_mat, int nnz);
+int spion_block_attn_needs_scratch(const spion_ctx* ctx);
+
 /* No counterpart in the reference.  stable != 0: the caller promises that the (offsets, columns,
  * sum_mat) arrays it passes to the two calls above stay allocated and unchanged for as long as it
  * passes them (a cache per mask, as spion_b200/attention_blockcuda.py keeps).  The block structure is
@@ -182,6 +192,18 @@ int spion_dense_attn_forward(spion_ctx* ctx, const float* Qt, const float* K, co
 int spion_dense_attn_backward(spion_ctx* ctx, const float* Qt, const float* Kt, const float* V,
                               const float* attn, const float* dOt, float* s1, float* s2, float* s3,
                               float* dQt, float* dKt, float* dVt);
+
+/* The same two calls with every operand and output in [BH, L, d]; attn keeps its transposed storage.  s1, s3: scratch of
+ * spion_dense_attn_scratch_floats(ctx) floats each (NULL when that is 0); O: the forward's output (may be NULL). */
+int spion_dense_attn_forward_rm(spion_ctx* ctx, const float* Q, const float* K, const float* V, const float* keypad,
+                                float* attn, float* out);
+int spion_dense_attn_backward_rm(spion_ctx* ctx, const float* Q, const float* K, const float* V, const float* attn,
+                                 const float* O, const float* dO, float* s1, float* s3, float* dQ, float* dK, float* dV);
+long long spion_dense_attn_scratch_floats(const spion_ctx* ctx);
+
+/* Key-padding mask [batch, L] of 1 (token) / 0 (padding) -> penalty 1e6 (1 - mask) per (b,h) matrix, [batch * heads, L]
+ * (models/attention_blockcuda_mask.py:42-43). */
+int spion_expand_keypad(const float* mask, int batch, int heads, int L, float* pen, void* cuda_stream);
 
 /* Head/batch mean of the dense attention tensor (models/model_transformer.py:137):
  * A[i,j] = mean_h mean_b P[b,h,i,j].  `attn` is [B*H, L, L]; transposed != 0 means it is
@@ -361,6 +383,38 @@ int spion_embedding_forward(const long long* ids, const float* tok, const float*
                             int V, int N, void* cuda_stream);
 int spion_embedding_backward(const long long* ids, const void* g, int g_is_bf16, long long T, int V, int N,
                              float* dW, float* workspace, void* cuda_stream);
+
+/* ------------------------------------------------------------------------------------------
+ * Linear layers around the attention call (torch.nn.Linear in the reference: models/attention.py:55-57,102) on the tensor
+ * cores, reading and writing token matrices in the form their neighbours use.
+ *   spion_tokens: `count` (1 .. 3) equally wide matrices of T tokens x cols features side by side, fp32 or bf16, 32-byte
+ *   aligned; heads == 0: row-major [T, cols]; heads > 0: split into heads, [T / seq_len, heads, seq_len, head_dim].
+ *   W[i]: nw (1 .. 3) fp32 matrices [out_features / nw, in_features] stacked along their rows; bias[i] likewise (bias may be NULL).
+ *   fp32 == 0: operands rounded to bf16, fp32 accumulation.  fp32 != 0: all matrices fp32; every product keeps the
+ *   accuracy of fp32 arithmetic (operands split into three bf16 parts).
+ * Feature counts are multiples of 32; spion_linear_supported tells whether a shape is served. */
+typedef struct spion_tokens {
+  void* ptr[3];
+  int count, cols, is_bf16;
+  int heads, head_dim, seq_len;
+} spion_tokens;
+int spion_linear_supported(int in_features, int out_features, int fp32);
+/* Y = X W^T + bias.  gelu_out (may be NULL; Y bf16, row-major): receives gelu(Y) as bf16 [T, out_features]. */
+int spion_linear_forward(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
+                         const spion_tokens* Y, void* gelu_out, long long T, int in_features, int out_features,
+                         void* cuda_stream);
+/* dX = dY W, times gelu'(gelu_in) element by element when gelu_in (bf16 [T, in_features]) is not NULL (dX bf16 then).
+ * dX fp32: one fp32 sum over all stacked layers.  dX bf16 and nw == 3: the sum of the three layers' gradients, each rounded to
+ * bf16 and added in bf16 from the last to the first, which is what separate layers give (out_features / 3 a multiple of 64). */
+int spion_linear_backward_input(const spion_tokens* dY, const float* const* W, int nw, int fp32, const void* gelu_in,
+                                const spion_tokens* dX, long long T, int in_features, int out_features, void* cuda_stream);
+/* dW [out_features, in_features] = dY^T X and db [out_features] = column sums of dY, fp32, fixed summation order.
+ * workspace: spion_linear_workspace_floats(...) floats, 16-byte aligned. */
+long long spion_linear_workspace_floats(long long T, int in_features, int out_features, int fp32);
+int spion_linear_backward_weight(const spion_tokens* dY, const spion_tokens* X, int fp32, float* dW, float* db,
+                                 float* workspace, long long T, int in_features, int out_features, void* cuda_stream);
+/* SPION_ERR_TIMEOUT when a bounded wait of these kernels has given up since the last reset (synchronises the device). */
+int spion_linear_status(int reset);
 
 #ifdef __cplusplus
 }

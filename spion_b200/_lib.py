@@ -20,6 +20,14 @@ KIND_DENSE, KIND_DENSE_KPM, KIND_BLOCK, KIND_BLOCK_KPM = 0, 1, 2, 3
 ENGINE_AUTO, ENGINE_SIMT, ENGINE_TCGEN05, ENGINE_SIMT_STAGED = 0, 1, 2, 3
 STAGE_COUNT = 15
 
+
+
+class Tokens(ctypes.Structure):
+    """spion_tokens: up to three equally wide token matrices side by side (see include/spion_b200.h)."""
+    _fields_ = [("ptr", c_void_p * 3), ("count", c_int), ("cols", c_int), ("is_bf16", c_int),
+                ("heads", c_int), ("head_dim", c_int), ("seq_len", c_int)]
+
+
 # name -> (restype, argtypes); every symbol include/spion_b200.h declares
 SIGNATURES = {
     "spion_status_string": (ctypes.c_char_p, [c_int]),
@@ -58,6 +66,13 @@ SIGNATURES = {
     "spion_block_attn_backward": (c_int, [c_void_p] * 14 + [c_int]),
     "spion_dense_attn_forward": (c_int, [c_void_p] * 7),
     "spion_dense_attn_backward": (c_int, [c_void_p] * 12),
+    "spion_block_attn_forward_rm": (c_int, [c_void_p] * 10 + [c_int]),
+    "spion_block_attn_backward_rm": (c_int, [c_void_p] * 15 + [c_int]),
+    "spion_block_attn_needs_scratch": (c_int, [c_void_p]),
+    "spion_dense_attn_forward_rm": (c_int, [c_void_p] * 7),
+    "spion_dense_attn_backward_rm": (c_int, [c_void_p] * 12),
+    "spion_dense_attn_scratch_floats": (c_longlong, [c_void_p]),
+    "spion_expand_keypad": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
     "spion_mean_attention_map": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "spion_mean_map_tiles": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "spion_discover_pattern": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_double] + [c_void_p] * 13),
@@ -73,6 +88,12 @@ SIGNATURES = {
     "spion_mean_map_recompute": (c_int, [c_void_p] * 6),
     "spion_softmax_forward_ex": (c_int, [c_void_p] * 4),
     "spion_softmax_backward_ex": (c_int, [c_void_p] * 4),
+    "spion_linear_supported": (c_int, [c_int] * 3),
+    "spion_linear_forward": (c_int, [c_void_p] * 3 + [c_int] * 2 + [c_void_p] * 2 + [c_longlong, c_int, c_int, c_void_p]),
+    "spion_linear_backward_input": (c_int, [c_void_p] * 2 + [c_int] * 2 + [c_void_p] * 2 + [c_longlong, c_int, c_int, c_void_p]),
+    "spion_linear_workspace_floats": (c_longlong, [c_longlong] + [c_int] * 3),
+    "spion_linear_backward_weight": (c_int, [c_void_p] * 2 + [c_int] + [c_void_p] * 3 + [c_longlong, c_int, c_int, c_void_p]),
+    "spion_linear_status": (c_int, [c_int]),
     "spion_static_scratch_capacity": (ctypes.c_size_t, []),
     "spion_attn_forward_static": (c_int, [c_void_p] * 9 + [c_int] * 6 + [c_void_p]),
 }

@@ -20,13 +20,15 @@ from ctypes import c_int
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, _ops
+from .layernorm import BiasGradLinear
 
 # tasks whose inputs carry padding and therefore use the key-padding variants (models/attention.py:11)
 mask_task = ['lra-listops', 'lra-text', 'lra-news', 'lra-yelp', 'lra-text1', 'lra-news1', 'lra-yelp1',
              'lra-text2', 'lra-news2', 'lra-yelp2', 'lra-retrieval']
 
 _P = ctypes.c_void_p
+_PLAIN_LINEAR = (nn.Linear, BiasGradLinear)
 
 
 def _load_shim(name, n_init, n_fwd, n_bwd, trailing_int):
@@ -58,9 +60,7 @@ class Attention(nn.Module):
 
         # same parameters and forward arithmetic as nn.Linear (models/attention.py:55-57); on the native path the
         # bias gradient of the backward is summed by the library's column-sum kernel
-        Linear = nn.Linear
-        if config.get("native") and config.get("fused_bias_grad", True):
-            from .layernorm import BiasGradLinear as Linear
+        Linear = BiasGradLinear if config.get("native") and config.get("fused_bias_grad", True) else nn.Linear
         self.W_q = Linear(self.dim, self.num_head * self.head_dim)
         self.W_k = Linear(self.dim, self.num_head * self.head_dim)
         self.W_v = Linear(self.dim, self.num_head * self.head_dim)
@@ -80,10 +80,56 @@ class Attention(nn.Module):
             if not attn_handle:
                 raise _lib.SpionError("init() of the dense attention library returned NULL")
             self.attn = Dense(config, attn_cpp, attn_handle)
+            self._dense_type = Dense
+            self._dense_ctx = _ops.make_context(attn_handle, _ops.DROPIN_DENSE, config["batch_size"], self.num_head, self.seq_len,
+                                                self.head_dim, torch.cuda.current_device(), False, self.with_keypad)
 
         self.ff = Linear(self.num_head * self.head_dim, self.dim)
 
+    def _linears_are_plain(self) -> bool:
+        """The projections are what __init__ made: no replaced module, no hook that a one-node layer would pass over."""
+        for m in (self.W_q, self.W_k, self.W_v, self.ff):
+            if type(m) not in _PLAIN_LINEAR or m.bias is None or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks \
+                    or m._backward_pre_hooks:
+                return False
+        return True
+
+    def _one_node(self, X, mask, mat):
+        """The whole layer as one autograd node on the library's kernels: projections, attention and output projection back to
+        back in the layouts the next kernel reads.  None when something about the call is not served (the stages then run
+        one by one): a width that is not a multiple of 32, another autocast dtype, replaced or hooked projections."""
+        if torch.is_autocast_enabled():
+            if not self.native or self.native_dtype != torch.bfloat16 or torch.get_autocast_dtype("cuda") != torch.bfloat16:
+                return None
+            fp32 = False
+        else:
+            if self.native and self.native_dtype != torch.float32:
+                return None
+            fp32 = True
+        if not self._linears_are_plain():
+            return None
+        block = None
+        if self.native:
+            block = self.attn.block if mat is None else self.block_attn
+            block.use_mask(mat)
+            ctx = block._ctx
+        elif mat is None:
+            return None          # in the dense phase the key bias has no effect: its gradient is the rounding noise of the stages
+        else:
+            ctx = self.block_attn.context(mat)
+        W = [m.weight for m in (self.W_q, self.W_k, self.W_v, self.ff)]
+        b = [m.bias for m in (self.W_q, self.W_k, self.W_v, self.ff)]
+        if not _ops.ops.layer_supported(ctx, X, W, b, fp32):
+            return None
+        out, P, lse, pen, q, k, heads = _ops.ops.attention_layer(ctx, X, mask if self.with_keypad else None, W, b, fp32)
+        if block is not None:
+            return block.result(out, P, lse, pen, q, k, heads)
+        return out, (0 if self.with_keypad else P)
+
     def forward(self, X, mask, mat=None):
+        layer = self._one_node(X, mask, mat)
+        if layer is not None:
+            return layer
         Q = self.split_heads(self.W_q(X))
         K = self.split_heads(self.W_k(X))
         V = self.split_heads(self.W_v(X))
@@ -91,6 +137,9 @@ class Attention(nn.Module):
             if mat is None and self.native:
                 attn_out, attn = self.attn(Q, K, V, mask.float())
                 attn_out = attn_out.to(X.dtype)
+            elif mat is None and type(self.attn) is self._dense_type:
+                attn_out, P = _ops.ops.attention(self._dense_ctx, Q.float(), K.float(), V.float(), mask if self.with_keypad else None)[:2]
+                attn = P.permute(0, 1, 3, 2)
             elif mat is None:
                 attn_out, attn = self.attn(Q.float(), K.float(), V.float(), mask.float())
             elif self.native:

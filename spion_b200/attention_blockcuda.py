@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, _ops
 from ._lib import SpionError, lib, ptr
 from .pattern import pattern_from_mask
 
@@ -31,15 +31,18 @@ class _CsrCache:
         self.block_size = block_size
         self.key = None
         self.ref = None
+        self.version = -1
         self.value = None
         self.on_new = on_new          # called whenever new arrays replace the cached ones
 
     def get(self, mat: torch.Tensor):
+        if mat is self.ref and mat._version == self.version:
+            return self.value
         key = (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device))
         if key != self.key:
             pat = pattern_from_mask(mat, self.block_size)
             sum_mat, offsets, columns, nnz = pat.element_csr(1)
-            self.key, self.ref, self.value = key, mat, (sum_mat, offsets, columns, nnz)
+            self.key, self.ref, self.version, self.value = key, mat, mat._version, (sum_mat, offsets, columns, nnz)
             if self.on_new is not None:
                 self.on_new()
         return self.value
@@ -109,6 +112,19 @@ def make_block_function(config, attn_cpp, attn_handle, with_keypad: bool):
                   ptr(d_p), ptr(d_s), ptr(dq), ptr(dk), ptr(dv), ptr(offsets), ptr(columns), ptr(sum_mat), nnz)
             return dq, dk, dv, None, None
 
+    # the same context for a caller that goes through the native host path (attention.Attention): the element CSR follows the mask
+    ctx = _ops.make_context(handle.value, _ops.DROPIN_SPARSE, batch_size, num_heads, seq_len, emb_dim, torch.cuda.current_device(),
+                            False, with_keypad)
+    held = [None]
+
+    def context(mat):
+        value = cache.get(mat)
+        if value is not held[0]:
+            ctx.sum_mat, ctx.offsets, ctx.columns, ctx.nnz = value
+            held[0] = value
+        return ctx
+
+    BlockAttnFunction.context = staticmethod(context)
     return BlockAttnFunction
 
 
@@ -116,6 +132,9 @@ class CUDABlockAttention(nn.Module):
     def __init__(self, config, attn_cpp, attn_handle):
         super().__init__()
         self.attn_func = make_block_function(config, attn_cpp, attn_handle, with_keypad=False)
+
+    def context(self, mat):
+        return self.attn_func.context(mat)
 
     def forward(self, query, key, value, mask, mat):
         return self.attn_func.apply(query, key, value, mask, mat)

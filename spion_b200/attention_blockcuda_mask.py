@@ -16,6 +16,9 @@ class CUDABlockMaskAttention(nn.Module):
         super().__init__()
         self.attn_func = make_block_function(config, attn_cpp, attn_handle, with_keypad=True)
 
+    def context(self, mat):
+        return self.attn_func.context(mat)
+
     def forward(self, query, key, value, mask, mat):
         out, _ = self.attn_func.apply(query, key, value, mask, mat)
         return out, 0

@@ -6,6 +6,7 @@ Outputs (git-ignored, but shipped with the working tree):
     spion_b200/lib/libspion_b200.so        all kernels + the C ABI of include/spion_b200.h
     spion_b200/lib/{attn,attn_mask,block_attn,block_attn_mask}.so
                                            shims with the reference's own symbol names
+    spion_b200/lib/_torch_ops.so           autograd nodes of the Python modules (csrc/torch_ops.cpp)
 """
 from __future__ import annotations
 
@@ -65,7 +66,30 @@ def build_all(force: bool = False, verbose: bool = False) -> str:
         if force or _newer([shim_src, main] + headers, out):
             _run(["g++", "-O2", "-fPIC", "-shared", f"-DSPION_SHIM_KIND={kind}", shim_src, "-o", out,
                   "-L" + LIB, "-lspion_b200", "-Wl,-rpath,$ORIGIN"])
+    build_torch_ops(main, force)
     return main
+
+
+def build_torch_ops(main, force: bool = False) -> str:
+    """The modules' host path: a CPython extension over the C ABI, compiled against the installed torch."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    src = os.path.join(CSRC, "torch_ops.cpp")
+    out = os.path.join(LIB, "_torch_ops.so")
+    header = os.path.join(os.path.dirname(HERE), "include", "spion_b200.h")
+    if not force and not _newer([src, header, main], out):
+        return out
+    inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
+    tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    obj = os.path.join(OBJ, "torch_ops.o")
+    if force or _newer([src, header], obj):
+        _run(["g++", "-O2", "-std=c++17", "-fPIC", "-w", "-DTORCH_EXTENSION_NAME=_torch_ops", "-DTORCH_API_INCLUDE_EXTENSION_H",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + ["-I" + i for i in inc] + ["-c", src, "-o", obj])
+    _run(["g++", "-shared", obj, "-o", out, "-L" + LIB, "-lspion_b200", "-L" + tlib, "-ltorch_python", "-ltorch", "-ltorch_cpu",
+          "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"])
+    return out
 
 
 if __name__ == "__main__":

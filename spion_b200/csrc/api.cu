@@ -265,10 +265,11 @@ static int legacy_structure(spion_ctx* c, const int* offsets, const int* columns
   return SPION_OK;
 }
 
-extern "C" int spion_block_attn_forward(spion_ctx* c, const float* Q, const float* Kt, const float* V,
-                                        const float* keypad, float* attn, float* out, const int* offsets,
-                                        const int* columns, const int* sum_mat, int nnz) {
-  if (!c || !Q || !Kt || !V || !attn || !out || !offsets || !columns || !sum_mat) return SPION_ERR_ARG;
+// The K operand of the forward and the V operand of the backward come transposed from the reference's Python, row-major from
+// callers of the _rm forms.
+static int block_forward(spion_ctx* c, const float* Q, const float* K, OperandLayout lk, const float* V, const float* keypad,
+                         float* attn, float* out, const int* offsets, const int* columns, const int* sum_mat, int nnz) {
+  if (!c || !Q || !K || !V || !attn || !out || !offsets || !columns || !sum_mat) return SPION_ERR_ARG;
   if (is_dense(c) || c->dtype != SPION_F32) return SPION_ERR_STATE;
   if (is_kpm(c) && !keypad) return SPION_ERR_ARG;
   DeviceGuard guard(c->device);
@@ -276,16 +277,16 @@ extern "C" int spion_block_attn_forward(spion_ctx* c, const float* Q, const floa
   if (rc) return rc;
   const Pattern p = ctx_pattern(c);
   const ValueLayout vl{VAL_ELEMCSR, c->L, (long long)nnz};
-  const OperandLayout rm = row_major_operand(c->L, c->d), tr = transposed_operand(c->L, c->d);
+  const OperandLayout rm = row_major_operand(c->L, c->d);
   // floor of the running maximum: -100 (models/block_attn.cu:48) or 0 (models/block_attn_mask.cu:105)
   if (use_simt_fused(c, VAL_ELEMCSR)) {
-    rc = simt_fused_forward(Q, rm, Kt, tr, V, rm, is_kpm(c) ? keypad : nullptr, is_kpm(c) ? 0.0f : -100.0f, attn, vl, out,
+    rc = simt_fused_forward(Q, rm, K, lk, V, rm, is_kpm(c) ? keypad : nullptr, is_kpm(c) ? 0.0f : -100.0f, attn, vl, out,
                             rm, p, c->BH, c->L, c->d, c->scale, c->stream);
     if (!rc) prof_mark(c, SPION_STAGE_FUSED_FWD);
     c->launches += 1;
     return rc;
   }
-  rc = simt_sddmm(SPION_F32, SPION_F32, Q, rm, Kt, tr, attn, vl, p, c->nnzb, c->BH, c->d, c->stream);
+  rc = simt_sddmm(SPION_F32, SPION_F32, Q, rm, K, lk, attn, vl, p, c->nnzb, c->BH, c->d, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SDDMM_S);
   if (rc) return rc;
   rc = softmax_fwd_rows(SPION_F32, attn, vl, attn, vl, p, c->BH, c->L, c->scale, is_kpm(c) ? keypad : nullptr,
@@ -298,12 +299,10 @@ extern "C" int spion_block_attn_forward(spion_ctx* c, const float* Q, const floa
   return rc;
 }
 
-extern "C" int spion_block_attn_backward(spion_ctx* c, const float* Q, const float* K, const float* Vt, const float* P,
-                                         const float* dO, float* dP_scratch, float* dS_scratch, float* dQ, float* dK,
-                                         float* dV, const int* offsets, const int* columns, const int* sum_mat,
-                                         int nnz) {
-  if (!c || !Q || !K || !Vt || !P || !dO || !dP_scratch || !dS_scratch || !dQ || !dK || !dV || !offsets || !columns ||
-      !sum_mat)
+static int block_backward(spion_ctx* c, const float* Q, const float* K, const float* V, OperandLayout lv, const float* P,
+                          const float* O, const float* dO, float* dP_scratch, float* dS_scratch, float* dQ, float* dK,
+                          float* dV, const int* offsets, const int* columns, const int* sum_mat, int nnz) {
+  if (!c || !Q || !K || !V || !P || !dO || !dS_scratch || !dQ || !dK || !dV || !offsets || !columns || !sum_mat)
     return SPION_ERR_ARG;
   if (is_dense(c) || c->dtype != SPION_F32) return SPION_ERR_STATE;
   DeviceGuard guard(c->device);
@@ -311,13 +310,14 @@ extern "C" int spion_block_attn_backward(spion_ctx* c, const float* Q, const flo
   if (rc) return rc;
   const Pattern p = ctx_pattern(c);
   const ValueLayout vl{VAL_ELEMCSR, c->L, (long long)nnz};
-  const OperandLayout rm = row_major_operand(c->L, c->d), tr = transposed_operand(c->L, c->d);
+  const OperandLayout rm = row_major_operand(c->L, c->d);
   if (use_simt_fused(c, VAL_ELEMCSR)) {
     c->launches += 2;
-    return simt_fused_backward(Q, rm, K, rm, Vt, tr, P, vl, nullptr, rm, dO, rm, dS_scratch, vl, dQ, rm, dK, rm, dV, rm, p, c->BH, c->d,
+    return simt_fused_backward(Q, rm, K, rm, V, lv, P, vl, O, rm, dO, rm, dS_scratch, vl, dQ, rm, dK, rm, dV, rm, p, c->BH, c->d,
                                c->scale, c->stream, c);
   }
-  rc = simt_sddmm(SPION_F32, SPION_F32, dO, rm, Vt, tr, dP_scratch, vl, p, c->nnzb, c->BH, c->d, c->stream);
+  if (!dP_scratch) return SPION_ERR_ARG;
+  rc = simt_sddmm(SPION_F32, SPION_F32, dO, rm, V, lv, dP_scratch, vl, p, c->nnzb, c->BH, c->d, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SDDMM_DP);
   if (rc) return rc;
   rc = softmax_bwd_rows(SPION_F32, dP_scratch, vl, P, vl, dS_scratch, vl, p, c->BH, c->L, c->scale, c->stream);
@@ -335,57 +335,138 @@ extern "C" int spion_block_attn_backward(spion_ctx* c, const float* Q, const flo
   return rc;
 }
 
+extern "C" int spion_block_attn_forward(spion_ctx* c, const float* Q, const float* Kt, const float* V,
+                                        const float* keypad, float* attn, float* out, const int* offsets,
+                                        const int* columns, const int* sum_mat, int nnz) {
+  if (!c) return SPION_ERR_ARG;
+  return block_forward(c, Q, Kt, transposed_operand(c->L, c->d), V, keypad, attn, out, offsets, columns, sum_mat, nnz);
+}
+
+extern "C" int spion_block_attn_forward_rm(spion_ctx* c, const float* Q, const float* K, const float* V, const float* keypad,
+                                           float* attn, float* out, const int* offsets, const int* columns,
+                                           const int* sum_mat, int nnz) {
+  if (!c) return SPION_ERR_ARG;
+  return block_forward(c, Q, K, row_major_operand(c->L, c->d), V, keypad, attn, out, offsets, columns, sum_mat, nnz);
+}
+
+extern "C" int spion_block_attn_backward(spion_ctx* c, const float* Q, const float* K, const float* Vt, const float* P,
+                                         const float* dO, float* dP_scratch, float* dS_scratch, float* dQ, float* dK,
+                                         float* dV, const int* offsets, const int* columns, const int* sum_mat,
+                                         int nnz) {
+  if (!c || !dP_scratch) return SPION_ERR_ARG;
+  return block_backward(c, Q, K, Vt, transposed_operand(c->L, c->d), P, nullptr, dO, dP_scratch, dS_scratch, dQ, dK, dV, offsets,
+                        columns, sum_mat, nnz);
+}
+
+extern "C" int spion_block_attn_backward_rm(spion_ctx* c, const float* Q, const float* K, const float* V, const float* P,
+                                            const float* O, const float* dO, float* dP_scratch, float* dS_scratch, float* dQ,
+                                            float* dK, float* dV, const int* offsets, const int* columns, const int* sum_mat,
+                                            int nnz) {
+  if (!c) return SPION_ERR_ARG;
+  return block_backward(c, Q, K, V, row_major_operand(c->L, c->d), P, O, dO, dP_scratch, dS_scratch, dQ, dK, dV, offsets, columns,
+                        sum_mat, nnz);
+}
+
+extern "C" int spion_block_attn_needs_scratch(const spion_ctx* c) {
+  return (c && !is_dense(c) && !use_simt_fused(c, VAL_ELEMCSR)) ? 1 : 0;
+}
+
 // ============================================================ reference-layout dense
-extern "C" int spion_dense_attn_forward(spion_ctx* c, const float* Qt, const float* K, const float* Vt,
-                                        const float* keypad, float* attn, float* out) {
-  if (!c || !Qt || !K || !Vt || !attn || !out) return SPION_ERR_ARG;
+static int dense_forward(spion_ctx* c, const float* Q, const float* K, const float* V, const float* keypad, float* attn,
+                         float* out, OperandLayout lo) {
+  if (!c || !Q || !K || !V || !attn || !out) return SPION_ERR_ARG;
   if (!is_dense(c) || c->dtype != SPION_F32) return SPION_ERR_STATE;
   if (is_kpm(c) && !keypad) return SPION_ERR_ARG;
   DeviceGuard guard(c->device);
   const Pattern p = ctx_pattern(c);
   const ValueLayout vl{VAL_DENSE_T, c->L, (long long)c->L * c->L};
-  const OperandLayout rm = row_major_operand(c->L, c->d), tr = transposed_operand(c->L, c->d);
+  const OperandLayout rm = row_major_operand(c->L, c->d);
   prof_mark(c, -1);
-  int rc = simt_sddmm(SPION_F32, SPION_F32, Qt, tr, K, rm, attn, vl, p, c->nnzb, c->BH, c->d, c->stream);
+  int rc = simt_sddmm(SPION_F32, SPION_F32, Q, lo, K, rm, attn, vl, p, c->nnzb, c->BH, c->d, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SDDMM_S);
   if (rc) return rc;
   // running-maximum floor -10 (models/attn.cu:21); key padding as models/attn_mask.cu:20
   rc = softmax_fwd_dense_t(attn, c->BH, c->L, c->scale, is_kpm(c) ? keypad : nullptr, -10.0f, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SOFTMAX_FWD);
   if (rc) return rc;
-  rc = simt_spmm(SPION_F32, SPION_F32, false, attn, vl, Vt, tr, out, tr, p, c->BH, c->d, c->stream);
+  rc = simt_spmm(SPION_F32, SPION_F32, false, attn, vl, V, lo, out, lo, p, c->BH, c->d, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SPMM_O);
   c->launches += 3;
   return rc;
+}
+
+static int dense_backward(spion_ctx* c, const float* Q, const float* K, const float* V, const float* attn, const float* dO,
+                          float* s1, float* s3, float* dQ, float* dK, float* dV, OperandLayout lo) {
+  if (!c || !Q || !K || !V || !attn || !dO || !s1 || !s3 || !dQ || !dK || !dV) return SPION_ERR_ARG;
+  if (!is_dense(c) || c->dtype != SPION_F32) return SPION_ERR_STATE;
+  DeviceGuard guard(c->device);
+  const Pattern p = ctx_pattern(c);
+  const ValueLayout vl{VAL_DENSE_T, c->L, (long long)c->L * c->L};
+  const OperandLayout rm = row_major_operand(c->L, c->d);
+  prof_mark(c, -1);
+  int rc = simt_sddmm(SPION_F32, SPION_F32, dO, lo, V, rm, s1, vl, p, c->nnzb, c->BH, c->d, c->stream);
+  if (!rc) prof_mark(c, SPION_STAGE_SDDMM_DP);
+  if (rc) return rc;
+  rc = softmax_bwd_dense_t(s1, attn, s3, c->BH, c->L, c->scale, c->stream);
+  if (!rc) prof_mark(c, SPION_STAGE_SOFTMAX_BWD);
+  if (rc) return rc;
+  rc = simt_spmm(SPION_F32, SPION_F32, false, s3, vl, K, lo, dQ, lo, p, c->BH, c->d, c->stream);
+  if (!rc) prof_mark(c, SPION_STAGE_SPMM_DQ);
+  if (rc) return rc;
+  rc = simt_spmm(SPION_F32, SPION_F32, true, s3, vl, Q, lo, dK, lo, p, c->BH, c->d, c->stream);
+  if (!rc) prof_mark(c, SPION_STAGE_SPMM_DK);
+  if (rc) return rc;
+  rc = simt_spmm(SPION_F32, SPION_F32, true, attn, vl, dO, lo, dV, lo, p, c->BH, c->d, c->stream);
+  if (!rc) prof_mark(c, SPION_STAGE_SPMM_DV);
+  c->launches += 5;
+  return rc;
+}
+
+// The reference hands over Q, V, dO and takes the outputs as [BH, d, L] (K and, in the backward, V row-major; K transposed).
+extern "C" int spion_dense_attn_forward(spion_ctx* c, const float* Qt, const float* K, const float* Vt,
+                                        const float* keypad, float* attn, float* out) {
+  if (!c) return SPION_ERR_ARG;
+  return dense_forward(c, Qt, K, Vt, keypad, attn, out, transposed_operand(c->L, c->d));
 }
 
 extern "C" int spion_dense_attn_backward(spion_ctx* c, const float* Qt, const float* Kt, const float* V,
                                          const float* attn, const float* dOt, float* s1, float* s2, float* s3,
                                          float* dQt, float* dKt, float* dVt) {
   (void)s2;
-  if (!c || !Qt || !Kt || !V || !attn || !dOt || !s1 || !s3 || !dQt || !dKt || !dVt) return SPION_ERR_ARG;
-  if (!is_dense(c) || c->dtype != SPION_F32) return SPION_ERR_STATE;
-  DeviceGuard guard(c->device);
-  const Pattern p = ctx_pattern(c);
-  const ValueLayout vl{VAL_DENSE_T, c->L, (long long)c->L * c->L};
-  const OperandLayout rm = row_major_operand(c->L, c->d), tr = transposed_operand(c->L, c->d);
-  prof_mark(c, -1);
-  int rc = simt_sddmm(SPION_F32, SPION_F32, dOt, tr, V, rm, s1, vl, p, c->nnzb, c->BH, c->d, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SDDMM_DP);
-  if (rc) return rc;
-  rc = softmax_bwd_dense_t(s1, attn, s3, c->BH, c->L, c->scale, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SOFTMAX_BWD);
-  if (rc) return rc;
-  rc = simt_spmm(SPION_F32, SPION_F32, false, s3, vl, Kt, tr, dQt, tr, p, c->BH, c->d, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SPMM_DQ);
-  if (rc) return rc;
-  rc = simt_spmm(SPION_F32, SPION_F32, true, s3, vl, Qt, tr, dKt, tr, p, c->BH, c->d, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SPMM_DK);
-  if (rc) return rc;
-  rc = simt_spmm(SPION_F32, SPION_F32, true, attn, vl, dOt, tr, dVt, tr, p, c->BH, c->d, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SPMM_DV);
-  c->launches += 5;
-  return rc;
+  if (!c) return SPION_ERR_ARG;
+  return dense_backward(c, Qt, Kt, V, attn, dOt, s1, s3, dQt, dKt, dVt, transposed_operand(c->L, c->d));
+}
+
+extern "C" int spion_dense_attn_forward_rm(spion_ctx* c, const float* Q, const float* K, const float* V, const float* keypad,
+                                           float* attn, float* out) {
+  if (!c) return SPION_ERR_ARG;
+  return dense_forward(c, Q, K, V, keypad, attn, out, row_major_operand(c->L, c->d));
+}
+
+extern "C" int spion_dense_attn_backward_rm(spion_ctx* c, const float* Q, const float* K, const float* V, const float* attn,
+                                            const float* O, const float* dO, float* s1, float* s3, float* dQ, float* dK,
+                                            float* dV) {
+  (void)O;
+  if (!c) return SPION_ERR_ARG;
+  return dense_backward(c, Q, K, V, attn, dO, s1, s3, dQ, dK, dV, row_major_operand(c->L, c->d));
+}
+
+extern "C" long long spion_dense_attn_scratch_floats(const spion_ctx* c) { return c ? (long long)c->BH * c->L * c->L : 0; }
+
+__global__ void k_expand_keypad(const float* __restrict__ mask, int heads, int L, long long n, float* __restrict__ pen) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const long long bh = i / L;
+    pen[i] = 1e6f * (1.0f - mask[(bh / heads) * L + (i - bh * L)]);
+  }
+}
+
+extern "C" int spion_expand_keypad(const float* mask, int batch, int heads, int L, float* pen, void* cuda_stream) {
+  if (!mask || !pen || batch < 1 || heads < 1 || L < 1) return SPION_ERR_ARG;
+  const long long n = (long long)batch * heads * L;
+  const long long blocks = (n + 255) / 256;
+  k_expand_keypad<<<(unsigned)(blocks < 1184 ? blocks : 1184), 256, 0, (cudaStream_t)cuda_stream>>>(mask, heads, L, n, pen);
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
 }
 
 // ============================================================ native (block-tile) API

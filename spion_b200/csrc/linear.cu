@@ -1,0 +1,980 @@
+// The narrow linear layers around the attention call (torch.nn.Linear in the reference: models/attention.py:55-57,102 and the
+// feed-forward block of models/model_transformer.py) as two tensor-core kernels:
+//
+//   k_lin_gemm    Y[T, N] = A[T, K] B + bias     A: tokens x features; B = W^T (forward) or W (gradient of the input)
+//   k_lin_wgrad   dW[N, K] = dY^T X, db = column sums of dY, partial sums per CTA, then k_lin_reduce
+//
+// With K, N of 32 .. a few hundred and T of 10^3 .. 10^6 tokens the work is bound by the passes over the token matrices, so
+// the kernels read every token matrix once, in the form its producer left it (fp32 or bf16, row-major or split into heads,
+// up to three matrices side by side), convert on the way into shared memory, add the bias and write the form the consumer
+// reads: no casts, no head-split copies, no concatenation, no separate bias or bias-gradient pass.
+//
+// Precision.  bf16 mode: operands rounded to bf16, fp32 accumulation (what mixed precision asks for).  fp32 mode: every fp32
+// operand is split into three bf16 parts (8 + 8 + 8 significant bits: the split is exact) and the six partial products of
+// weight 2^0, 2^-8 and 2^-16 are accumulated in fp32; the dropped ones are below 2^-25 of the product, i.e. below the rounding
+// of an fp32 multiplication.  In the weight gradient, where a sum runs over thousands of tokens, the leading products go to
+// two accumulators in turn and the small ones to a third, and the partial sums of the CTAs are added in fp32, which keeps
+// the chains short.
+#include <type_traits>
+
+#include "common.cuh"
+#include "tc_ptx.cuh"
+#include "tc_tiles.cuh"
+
+using namespace tc;
+
+namespace {
+
+__device__ int g_lin_status;              // set by a bounded wait that gave up
+
+// Tokens x features, up to three equally wide matrices side by side, row-major or split into heads [T / L, heads, L, d].
+// Row-major is the same with one head of width `per` and one sequence of all tokens.
+struct TokMat {
+  void* p[3];
+  int per, d, dsh, L;       // features per matrix; head width, its log2 (31: one head); tokens per sequence
+  long long hstride, bstride;
+};
+// Row and column parts of an element's offset are kept apart: rows advance by a constant step, columns hardly change, so the
+// loops below compute no division.
+struct RowIt {
+  int b, l;                 // sequence, position
+  __device__ __forceinline__ void init(const TokMat& m, int t) { b = t / m.L; l = t - b * m.L; }
+  __device__ __forceinline__ long long off(const TokMat& m) const { return (long long)b * m.bstride + (long long)l * m.d; }
+  __device__ __forceinline__ void add(const TokMat& m, int db, int dl) {      // step = db sequences + dl positions, dl < L
+    b += db; l += dl;
+    if (l >= m.L) { l -= m.L; ++b; }
+  }
+};
+template <typename E> __device__ __forceinline__ E* tok_col(const TokMat& m, int c) {       // column c of the stack, token 0
+  const int i = (c >= m.per) + (c >= 2 * m.per);
+  c -= i * m.per;
+  const int h = c >> m.dsh;
+  return reinterpret_cast<E*>(i == 0 ? m.p[0] : (i == 1 ? m.p[1] : m.p[2])) + (h * m.hstride + (c - h * m.d));
+}
+
+__device__ __forceinline__ void ld_v8(const void* p, uint32_t (&r)[8]) {     // 32 bytes, 32-byte aligned
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "l"(p));
+}
+// ... or zeros.  One predicated load: with a branch around it the compiler joins the two values through register copies, which
+// wait for the load where it is issued instead of where it is used.
+__device__ __forceinline__ void ld_v8_if(bool in, const void* p, uint32_t (&r)[8]) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %9, 0;\n\t"
+      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+      "mov.b32 %4, 0;\n\tmov.b32 %5, 0;\n\tmov.b32 %6, 0;\n\tmov.b32 %7, 0;\n\t"
+      "@q ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7])
+      : "l"(p), "r"((int)in));
+}
+__device__ __forceinline__ void st_v8(void* p, const uint32_t (&r)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+               "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void st_shared16(uint32_t a, const uint32_t (&w)[4]) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+
+// bf16 operands need no conversion: sixteen bytes straight into their place in shared memory (zeros when !in), asynchronously
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Eight features of one token in registers: 8 fp32 words, or 4 words of bf16 pairs.
+template <bool BF16> struct Raw { uint32_t w[BF16 ? 4 : 8]; };
+// ... into the shared-memory images: SPLIT == 1 one bf16 image, SPLIT == 3 three (leading, middle, last 8 bits), `part` bytes apart
+template <int SPLIT, bool BF16> __device__ __forceinline__ void raw_store(const Raw<BF16>& r, uint32_t addr, uint32_t part) {
+  if constexpr (BF16) {
+    st_shared16(addr, r.w);
+  } else {
+    uint32_t w[4];
+    float f[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r.w[i]);
+#pragma unroll
+    for (int s = 0; s < SPLIT; ++s) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        w[i] = pack_bf16(f[2 * i], f[2 * i + 1]);
+        if (s + 1 < SPLIT) { f[2 * i] -= bf16_lo(w[i]); f[2 * i + 1] -= bf16_hi(w[i]); }
+      }
+      st_shared16(addr + s * part, w);
+    }
+  }
+}
+
+// the partial products of the split operands, smallest first: (part of A, part of B)
+template <int SPLIT> struct Prod { static constexpr int N = 1; __device__ static int a(int) { return 0; } __device__ static int b(int) { return 0; } };
+template <> struct Prod<3> {
+  static constexpr int N = 6;
+  __device__ static constexpr int a(int i) { return i == 0 ? 0 : i == 1 ? 1 : i == 2 ? 2 : i == 3 ? 0 : i == 4 ? 1 : 0; }
+  __device__ static constexpr int b(int i) { return i == 0 ? 2 : i == 1 ? 1 : i == 2 ? 0 : i == 3 ? 1 : i == 4 ? 0 : 0; }
+};
+
+__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+  if (!ok && (threadIdx.x & 31) == 0) atomicOr(&g_lin_status, ERR_MMA_WAIT);
+  return ok;
+}
+
+// ------------------------------------------------------------------------------------------------ GEMM over tokens
+enum { EPI_NONE = 0, EPI_GELU = 1, EPI_DGELU = 2 };
+
+struct GemmArgs {
+  TokMat A, Y;
+  const float* W[3];        // stacked along their rows, each [wper, wld]
+  const float* bias[3];     // [wper] each, or null (forward only)
+  int wper, wld;
+  int T, K, N;              // tokens, contraction length of this launch, output features
+  int k0;                   // first contraction index of this launch
+  int accum;                // add to Y (fp32) instead of overwriting it: a contraction split over several launches
+  int nc, nstages;          // output features per CTA (blockIdx.y), stages of the A ring
+  int nacc;                 // accumulators per tile (fp32 mode): the leading products rotate over nacc - 1 of them by chunk
+  int parts;                // bf16 gradient of three stacked layers: chunks per layer (0: one accumulator for the whole contraction)
+  const __nv_bfloat16* h;   // EPI_DGELU: pre-activation [T, N]
+  __nv_bfloat16* g;         // EPI_GELU: activation [T, N] (Y receives the pre-activation)
+};
+
+constexpr int LG_LOADERS = 8;
+constexpr int LG_DEPTH = 4;                              // bf16 operands: stages whose copies are in flight
+constexpr int LG_THREADS = 32 * (LG_LOADERS + 1 + 8);
+constexpr uint32_t CHUNK = 128 * 128;                    // [128 tokens x 64 features] bf16
+
+// Gauss error linear unit, exact form (torch.nn.GELU's default)
+__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
+__device__ __forceinline__ float dgelu(float x) {
+  return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
+}
+
+// One persistent CTA per SM over tiles of 128 tokens: warps 0-7 bring 64-feature chunks of A through registers (a chunk of
+// loads in flight while the previous one is converted) into a ring of shared-memory stages, warp 8 issues the MMAs
+// (M = 128, two accumulator buffers in tensor memory), warps 9-16 write finished tiles.  W sits in shared memory for the
+// whole run.  Bound by the HBM passes over A and Y.
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
+__global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constant__ GemmArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t sbase = smem_u32(smem_raw);
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
+  const int nchunks = (a.K + 63) >> 6;
+  const int n0 = blockIdx.y * a.nc;
+  const int nc = min(a.nc, a.N - n0);
+  const int G = (a.nc + 63) >> 6;
+  // bytes of one part of B: [nc rows x 64] per chunk (K-major), or G tiles [64 x 64] per chunk (contraction rows)
+  const uint32_t bchunk = TRANSB ? (uint32_t)G * 8192u : (uint32_t)a.nc * 128u;
+  const uint32_t bpart = ((uint32_t)nchunks * bchunk + 1023u) & ~1023u;
+  const uint32_t sA = sbase + SPLIT * bpart;
+  const uint32_t sBias = sA + a.nstages * SPLIT * CHUNK;
+  const uint32_t bars = sBias + 1024u;
+  const uint32_t full = bars, empty = bars + 64, acc_full = bars + 128, acc_empty = bars + 144, slot = bars + 160;
+  uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
+  float* bias_ptr = reinterpret_cast<float*>(smem_raw + (sBias - sbase));
+
+  const int ntiles = (a.T + 127) >> 7;
+  const int G_x = (int)gridDim.x;
+
+  if (warp == LG_LOADERS) {
+    if (lane == 0) {
+      for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, LG_LOADERS); mbar_init(empty + 8 * i, 1); }
+      for (int i = 0; i < 2; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 8); }
+      fence_barrier_init();
+    }
+    __syncwarp();
+    tmem_alloc(slot, 512u);
+    tmem_relinquish();
+  }
+  // first chunk of the first tile is requested before the weights are converted
+  constexpr int R = 4;
+  const int lrow = tid >> 3, lc8 = tid & 7;
+  using AE = typename std::conditional<A_BF16, __nv_bfloat16, float>::type;
+  auto a_col = [&](int ch) -> const AE* {                // this thread's eight features of chunk ch, null past the end
+    const int c = ch * 64 + lc8 * 8;
+    return c < a.K ? tok_col<const AE>(a.A, c + a.k0) : nullptr;
+  };
+  RowIt row[R];                                          // rows of the tile whose loads are issued next
+  const int step = G_x * 128, step_b = step / a.A.L, step_l = step - step_b * a.A.L;
+  if (warp < LG_LOADERS) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) row[i].init(a.A, min(a.T - 1, (int)blockIdx.x * 128 + lrow + 32 * i));
+  }
+  auto load_row = [&](const AE* col, int tile, int i) {
+    Raw<false> r;
+    ld_v8_if(col && tile * 128 + lrow + 32 * i < a.T, col + row[i].off(a.A), r.w);
+    return r;
+  };
+  Raw<false> cur[R];
+  if (!A_BF16 && warp < LG_LOADERS) {
+    const AE* col = a_col(0);
+#pragma unroll
+    for (int i = 0; i < R; ++i) cur[i] = load_row(col, blockIdx.x, i);
+  }
+
+  {                                                      // weights -> shared memory
+    const int per_row = TRANSB ? nc >> 3 : a.K >> 3;
+    const int rows = TRANSB ? a.K : nc;
+    for (int idx = tid; idx < rows * per_row; idx += LG_THREADS) {
+      const int r = idx / per_row, c8 = idx - r * per_row;
+      const int gr = TRANSB ? a.k0 + r : n0 + r;         // row of the stacked W
+      const int m = gr / a.wper;
+      const float* src = (m == 0 ? a.W[0] : m == 1 ? a.W[1] : a.W[2]) + (size_t)(gr - m * a.wper) * a.wld + (TRANSB ? n0 : a.k0) + c8 * 8;
+      Raw<false> v;
+      const uint4 x = *reinterpret_cast<const uint4*>(src), y = *reinterpret_cast<const uint4*>(src + 4);
+      v.w[0] = x.x; v.w[1] = x.y; v.w[2] = x.z; v.w[3] = x.w; v.w[4] = y.x; v.w[5] = y.y; v.w[6] = y.z; v.w[7] = y.w;
+      const uint32_t dst = TRANSB ? ((uint32_t)((r >> 6) * G + (c8 >> 3)) * 8192u + (r & 63) * 128)
+                                  : ((uint32_t)(c8 >> 3) * bchunk + r * 128);
+      raw_store<SPLIT, false>(v, sbase + dst + (((c8 & 7) ^ (r & 7)) << 4), bpart);
+    }
+    for (int n = tid; n < nc; n += LG_THREADS) {
+      float b = 0.f;
+      if (a.bias[0]) {
+        const int m = (n0 + n) / a.wper;
+        b = (m == 0 ? a.bias[0] : m == 1 ? a.bias[1] : a.bias[2])[n0 + n - m * a.wper];
+        if (SPLIT == 1) b = __bfloat162float(__float2bfloat16_rn(b));
+      }
+      bias_ptr[n] = b;
+    }
+    fence_proxy_async();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *slot_ptr;
+
+  if (warp < LG_LOADERS) {
+    // ------------------------------------------------------------------ loaders
+    int n = 0;
+    bool ok = true;
+    int tile = blockIdx.x, ch = 0;
+    if constexpr (A_BF16) {
+      // LG_DEPTH chunks of copies in flight per thread; a chunk is handed over when the thread's own copies have landed
+      auto hand_over = [&](int m) {
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + 8 * (m % a.nstages));
+      };
+      while (ok && tile < ntiles) {
+        const int st = n % a.nstages, use = n / a.nstages;
+        if (use > 0) ok = warp_wait(empty + 8 * st, (uint32_t)(use - 1) & 1u);
+        if (!ok) break;
+        const uint32_t dst = sA + st * CHUNK;
+        const AE* col = a_col(ch);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const int r = lrow + 32 * i;
+          const bool in = col && tile * 128 + r < a.T;
+          cp_async16(dst + r * 128 + ((lc8 ^ (r & 7)) << 4), in ? col + row[i].off(a.A) : reinterpret_cast<const AE*>(a.A.p[0]), in);
+        }
+        cp_async_commit();
+        if (n >= LG_DEPTH) { cp_async_wait<LG_DEPTH>(); hand_over(n - LG_DEPTH); }
+        ++n;
+        if (++ch == nchunks) {
+          ch = 0; tile += G_x;
+#pragma unroll
+          for (int i = 0; i < R; ++i) row[i].add(a.A, step_b, step_l);
+        }
+      }
+      cp_async_wait<0>();
+      if (ok)
+        for (int m = max(0, n - LG_DEPTH); m < n; ++m) hand_over(m);
+    } else
+    while (ok && tile < ntiles) {
+      int tile_n = tile, ch_n = ch + 1;
+      if (ch_n == nchunks) {
+        ch_n = 0; tile_n += G_x;
+#pragma unroll
+        for (int i = 0; i < R; ++i) row[i].add(a.A, step_b, step_l);
+      }
+      const AE* col = a_col(ch_n);
+      const int st = n % a.nstages, use = n / a.nstages;
+      if (use > 0) ok = warp_wait(empty + 8 * st, (uint32_t)(use - 1) & 1u);
+      if (!ok) break;
+      const uint32_t dst = sA + st * SPLIT * CHUNK;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {                      // registers freed by a store take the next chunk's load
+        const int r = lrow + 32 * i;
+        raw_store<SPLIT, false>(cur[i], dst + r * 128 + ((lc8 ^ (r & 7)) << 4), CHUNK);
+        cur[i] = load_row(col, tile_n, i);
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + 8 * st);
+      ++n;
+      tile = tile_n; ch = ch_n;
+    }
+  } else if (warp == LG_LOADERS) {
+    // ------------------------------------------------------------------ MMA issue
+    int n = 0, j = 0;
+    bool ok = true;
+    // every operand descriptor is an add on one of these two
+    const uint64_t DA = make_smem_desc(sA, 16, 1024, LAYOUT_SW128);
+    const uint64_t DB = TRANSB ? make_smem_desc(sbase, 8192, 1024, LAYOUT_SW128) : make_smem_desc(sbase, 16, 1024, LAYOUT_SW128);
+    const uint32_t idesc = make_idesc_bf16(128, nc, 0, 0);
+    for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++j) {
+      const int buf = j & 1;
+      if (j >= 2) ok = warp_wait(acc_empty + 8 * buf, (uint32_t)(j / 2 - 1) & 1u);
+      for (int ch = 0; ok && ch < nchunks; ++ch, ++n) {
+        const int st = n % a.nstages;
+        ok = warp_wait(full + 8 * st, (uint32_t)(n / a.nstages) & 1u);
+        if (!ok) break;
+        if (elect_one()) {
+          tc_fence_after();
+          const int nk = min(4, (a.K - 64 * ch) >> 4);
+          const uint64_t da = desc_advance(DA, (uint32_t)st * SPLIT * CHUNK), db = desc_advance(DB, (uint32_t)ch * bchunk);
+          // fp32 mode: a sum in tensor memory is truncated at every step, so the small products have an accumulator of
+          // their own and the leading ones one per chunk as far as they go (nacc == 1: one chunk, everything in one)
+          const uint32_t d0 = tmem + buf * 256;
+          const bool spread = SPLIT == 3 && a.nacc > 1;
+          const int part = SPLIT == 1 && a.parts ? ch / a.parts : 0, ch_in = SPLIT == 1 && a.parts ? ch - part * a.parts : ch;
+          const uint32_t dl = part ? d0 + part * 64u : spread ? d0 + (uint32_t)(1 + ch % (a.nacc - 1)) * (256u / a.nacc) : d0;
+          const uint32_t acc_s = ch > 0, acc_l = spread ? (ch >= a.nacc - 1) : (ch_in > 0 || SPLIT == 3);
+          const int groups = TRANSB ? (nc + 63) >> 6 : 1;
+          for (int g = 0; g < groups; ++g) {
+            const uint32_t id = TRANSB ? (64 * g + 64 <= nc ? make_idesc_bf16(128, 64, 0, 1) : make_idesc_bf16(128, 32, 0, 1)) : idesc;
+#pragma unroll
+            for (int pr = 0; pr < Prod<SPLIT>::N; ++pr) {
+              const bool lead = pr + 1 == Prod<SPLIT>::N;
+              const uint64_t pa = desc_advance(da, Prod<SPLIT>::a(pr) * CHUNK);
+              const uint64_t pb = desc_advance(db, Prod<SPLIT>::b(pr) * bpart + (TRANSB ? g * 8192u : 0u));
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)
+                if (kk < nk)
+                  mma_bf16((lead ? dl : d0) + (TRANSB ? g * 64u : 0u), desc_advance(pa, kk * 32), desc_advance(pb, TRANSB ? kk * 2048 : kk * 32),
+                           id, kk > 0 ? 1u : (lead ? acc_l : (pr > 0 ? 1u : acc_s)));
+            }
+          }
+          mma_commit(empty + 8 * st);
+          if (ch + 1 == nchunks) mma_commit(acc_full + 8 * buf);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ output rows
+    const int q = warp & 3, half = (warp - LG_LOADERS - 1) >> 2;
+    const int ngroups = nc >> 5;
+    int j = 0;
+    RowIt orow;
+    const int ostep = G_x * 128, ostep_b = ostep / a.Y.L, ostep_l = ostep - ostep_b * a.Y.L;
+    orow.init(a.Y, min(a.T - 1, (int)blockIdx.x * 128 + q * 32 + lane));
+    for (int tile = blockIdx.x; tile < ntiles; tile += G_x, ++j, orow.add(a.Y, ostep_b, ostep_l)) {
+      const int buf = j & 1;
+      if (!warp_wait(acc_full + 8 * buf, (uint32_t)(j >> 1) & 1u)) break;
+      tc_fence_after();
+      const int t = tile * 128 + q * 32 + lane;
+      const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16) + buf * 256;
+      for (int g = half; g < ngroups; g += 2) {
+        uint32_t v[32];
+        __syncwarp();
+        tmem_ld32(tl + g * 32, v);
+        tmem_ld_wait();
+        if (SPLIT == 3) {
+          for (int x = 1; x < a.nacc && x <= nchunks; ++x) {
+            uint32_t u[32];
+            tmem_ld32(tl + x * (256 / a.nacc) + g * 32, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(u[i]));
+          }
+        }
+        if (SPLIT == 1 && TRANSB && a.parts) {
+          // what three separate layers would hand to their common input: each gradient rounded to bf16, added in bf16 from the
+          // last layer to the first
+          uint32_t u[32], w[32];
+          tmem_ld32(tl + 64 + g * 32, u);
+          tmem_ld32(tl + 128 + g * 32, w);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            v[i] = __float_as_uint(round_bf16(round_bf16(__uint_as_float(w[i])) + round_bf16(__uint_as_float(u[i]))) +
+                                   round_bf16(__uint_as_float(v[i])));
+        }
+        if (g + 2 >= ngroups) {                          // this warp has read its columns of the tile
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty + 8 * buf);
+        }
+        if (t >= a.T) continue;
+        const float4* bp = reinterpret_cast<const float4*>(bias_ptr + g * 32);
+        float f[32];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 b = bp[i];
+          f[4 * i] = __uint_as_float(v[4 * i]) + b.x; f[4 * i + 1] = __uint_as_float(v[4 * i + 1]) + b.y;
+          f[4 * i + 2] = __uint_as_float(v[4 * i + 2]) + b.z; f[4 * i + 3] = __uint_as_float(v[4 * i + 3]) + b.w;
+        }
+        const int c = n0 + g * 32;
+        if (EPI == EPI_DGELU) {
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            uint32_t hw[8];
+            ld_v8(a.h + (size_t)t * a.N + c + 16 * x, hw);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { f[16 * x + 2 * i] = round_bf16(f[16 * x + 2 * i]) * dgelu(bf16_lo(hw[i])); f[16 * x + 2 * i + 1] = round_bf16(f[16 * x + 2 * i + 1]) * dgelu(bf16_hi(hw[i])); }
+          }
+        }
+        if (Y_BF16) {
+          __nv_bfloat16* dst = tok_col<__nv_bfloat16>(a.Y, c) + orow.off(a.Y);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = pack_bf16(f[16 * x + 2 * i], f[16 * x + 2 * i + 1]);
+            st_v8(dst + 16 * x, w);
+            if (EPI == EPI_GELU) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) w[i] = pack_bf16(gelu(bf16_lo(w[i])), gelu(bf16_hi(w[i])));
+              st_v8(a.g + (size_t)t * a.N + c + 16 * x, w);
+            }
+          }
+        } else {
+          float* dst = tok_col<float>(a.Y, c) + orow.off(a.Y);
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = __float_as_uint(f[8 * x + i]);
+            if (a.accum) {
+              uint32_t o[8];
+              ld_v8(dst + 8 * x, o);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) + __uint_as_float(o[i]));
+            }
+            st_v8(dst + 8 * x, w);
+          }
+        }
+      }
+      if (half >= ngroups) {                             // nc == 32: the second half of the warps only hands the buffer back
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty + 8 * buf);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == LG_LOADERS) tmem_dealloc(tmem, 512u);
+}
+
+// ------------------------------------------------------------------------------------------------ weight gradient
+struct WgradArgs {
+  TokMat dY, X;
+  int T, N, K;
+  int nc, kc, nstages;      // features of dY / X per CTA (blockIdx.y, blockIdx.z); nc + kc <= 256, multiples of 64 except at the end
+  float* part;              // [gridDim.x][N * K + N]
+};
+
+constexpr int WG_THREADS = 32 * (LG_LOADERS + 1);
+constexpr uint32_t WCHUNK = 64 * 128;                    // [64 tokens x 64 features] bf16
+
+// One CTA per SM and slice of the tokens.  dW^T accumulates in tensor memory over all tokens of the CTA: the chunks of X are one
+// MN-major A operand (M = 64 or 128), those of dY one MN-major B operand (N up to 192), so nothing is transposed.  The bias gradient is summed from the registers the loaders hold.
+template <int SPLIT, bool DY_BF16, bool X_BF16>
+__global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_constant__ WgradArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t sbase = smem_u32(smem_raw);
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
+  const int n0 = blockIdx.y * a.nc, k0 = blockIdx.z * a.kc;
+  const int nlen = min(a.nc, a.N - n0), klen = min(a.kc, a.K - k0);
+  const int nch = (nlen + 63) >> 6, kch = (klen + 63) >> 6, cpt = nch + kch;    // chunks per tile of 64 tokens
+  const uint32_t stage = (uint32_t)cpt * SPLIT * WCHUNK;
+  const uint32_t bars = sbase + a.nstages * ((a.nc + 63) / 64 + (a.kc + 63) / 64) * SPLIT * WCHUNK;
+  const uint32_t full = bars, empty = bars + 64, acc_done = bars + 128, slot = bars + 136, sdb = bars + 256;
+  uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
+  float* sdb_ptr = reinterpret_cast<float*>(smem_raw + (sdb - sbase));        // [8 warps][256]
+  const int ntiles = (a.T + 63) >> 6;
+  const int G_x = (int)gridDim.x;
+
+  if (warp == LG_LOADERS) {
+    if (lane == 0) {
+      for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, LG_LOADERS); mbar_init(empty + 8 * i, 1); }
+      mbar_init(acc_done, 1);
+      fence_barrier_init();
+    }
+    __syncwarp();
+    tmem_alloc(slot, 512u);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *slot_ptr;
+
+  if (warp < LG_LOADERS) {
+    const int lrow = tid >> 3, lc8 = tid & 7;
+    // chunk i of a tile: features i of dY for i < nch, then those of X.  fp32 chunks pass through registers (a tile ahead),
+    // bf16 ones are copied straight into their stage (AHEAD tiles ahead).
+    Raw<false> cur[4][2];
+    constexpr int AHEAD = (DY_BF16 || X_BF16) ? 2 : 0;
+    float db[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) db[i][e] = 0.f;
+    using DE = typename std::conditional<DY_BF16, __nv_bfloat16, float>::type;
+    using XE = typename std::conditional<X_BF16, __nv_bfloat16, float>::type;
+    const DE* dcol[4];                                     // this thread's eight features of every chunk, null past the end
+    const XE* xcol[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int cd = n0 + i * 64 + lc8 * 8, cx = k0 + (i - nch) * 64 + lc8 * 8;
+      dcol[i] = i < nch && cd < n0 + nlen ? tok_col<const DE>(a.dY, cd) : nullptr;
+      xcol[i] = i >= nch && i < cpt && cx < k0 + klen ? tok_col<const XE>(a.X, cx) : nullptr;
+    }
+    const int step = G_x * 64;
+    const int dstep_b = step / a.dY.L, dstep_l = step - dstep_b * a.dY.L, xstep_b = step / a.X.L, xstep_l = step - xstep_b * a.X.L;
+    RowIt drow[2], xrow[2];                                // rows of the tile whose loads are issued next
+    auto row_init = [&](int t0) {
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        drow[x].init(a.dY, min(a.T - 1, t0 + lrow + 32 * x));
+        xrow[x].init(a.X, min(a.T - 1, t0 + lrow + 32 * x));
+      }
+    };
+    // fp32 chunks of the tile the row iterators stand at -> registers
+    auto load_row = [&](int tile, int i, int x) {
+      const bool isd = !DY_BF16 && (X_BF16 || i < nch);
+      const void* p = isd ? (const void*)(dcol[i] + drow[x].off(a.dY)) : (const void*)(xcol[i] + xrow[x].off(a.X));
+      const bool in = (isd ? dcol[i] != nullptr : xcol[i] != nullptr) && tile * 64 + lrow + 32 * x < a.T;
+      ld_v8_if(in, p, cur[i][x].w);
+    };
+    // bf16 chunks of the current tile -> shared memory
+    auto copy_row = [&](int tile, int i, int x, uint32_t dst) {
+      const bool tin = tile * 64 + lrow + 32 * x < a.T;
+      if (i < nch) {
+        const bool in = tin && dcol[i];
+        cp_async16(dst, in ? dcol[i] + drow[x].off(a.dY) : reinterpret_cast<const DE*>(a.dY.p[0]), in);
+      } else {
+        const bool in = tin && xcol[i];
+        cp_async16(dst, in ? xcol[i] + xrow[x].off(a.X) : reinterpret_cast<const XE*>(a.X.p[0]), in);
+      }
+    };
+    auto place = [&](int st, int i, int x) -> uint32_t {
+      const int r = lrow + 32 * x;
+      return sbase + st * stage + i * SPLIT * WCHUNK + r * 128 + ((lc8 ^ (r & 7)) << 4);
+    };
+    bool ok = true;
+    int n = 0;
+    // this thread's share of tile m is complete: column sums of its bf16 dY pieces, then the hand-over
+    auto hand_over = [&](int m) {
+      const int st = m % a.nstages;
+      if (DY_BF16) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (i < nch) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              uint32_t w[4];
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(place(st, i, x)) : "memory");
+#pragma unroll
+              for (int e = 0; e < 4; ++e) { db[i][2 * e] += bf16_lo(w[e]); db[i][2 * e + 1] += bf16_hi(w[e]); }
+            }
+          }
+        }
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + 8 * st);
+    };
+    row_init((int)blockIdx.x * 64);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) load_row(blockIdx.x, i, x);
+    for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++n) {
+      const int st = n % a.nstages, use = n / a.nstages;
+      if (use > 0) ok = warp_wait(empty + 8 * st, (uint32_t)(use - 1) & 1u);
+      if (!ok) break;
+      if (DY_BF16 || X_BF16) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            if (i < cpt && (i < nch ? DY_BF16 : X_BF16)) copy_row(tile, i, x, place(st, i, x));
+      }
+#pragma unroll
+      for (int x = 0; x < 2; ++x) { drow[x].add(a.dY, dstep_b, dstep_l); xrow[x].add(a.X, xstep_b, xstep_l); }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i < cpt && !(i < nch ? DY_BF16 : X_BF16)) {
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            raw_store<SPLIT, false>(cur[i][x], place(st, i, x), WCHUNK);
+            if (i < nch) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) db[i][e] += __uint_as_float(cur[i][x].w[e]);
+            }
+            load_row(tile + G_x, i, x);
+          }
+        }
+      }
+      if (AHEAD > 0) {
+        cp_async_commit();
+        if (n >= AHEAD) { cp_async_wait<AHEAD>(); hand_over(n - AHEAD); }
+      } else {
+        hand_over(n);
+      }
+    }
+    if (AHEAD > 0) {
+      cp_async_wait<0>();
+      if (ok)
+        for (int m = max(0, n - AHEAD); m < n; ++m) hand_over(m);
+    }
+    // column sums of dY: lanes with the same lc8 of a warp, then the eight warps in order
+    if (blockIdx.z == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i < nch) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            float s = db[i][e];
+            s += __shfl_xor_sync(0xffffffffu, s, 8);
+            s += __shfl_xor_sync(0xffffffffu, s, 16);
+            if (lane < 8) sdb_ptr[warp * 256 + i * 64 + lane * 8 + e] = s;
+          }
+        }
+      }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");        // the eight loader warps
+    float* part = a.part + (size_t)blockIdx.x * ((size_t)a.N * a.K + a.N);
+    if (blockIdx.z == 0 && tid < nlen) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < LG_LOADERS; ++w) s += sdb_ptr[w * 256 + tid];
+      part[(size_t)a.N * a.K + n0 + tid] = s;
+    }
+    if (ok) ok = warp_wait(acc_done, 0u);
+    if (ok) {
+      tc_fence_after();
+      const int q = warp & 3, half = warp >> 2;
+      const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16);
+      const bool two = ((ntiles - (int)blockIdx.x + G_x - 1) / G_x) > 1;       // both leading accumulators were used
+      const int m = kch == 1 ? q * 16 + (lane & 15) : q * 32 + lane;           // feature of X
+      const bool min_ = (kch == 2 || lane < 16) && m < klen;
+      for (int g = half; g < (nlen >> 5); g += 2) {
+        uint32_t v[32], u[32];
+        __syncwarp();
+        tmem_ld32(tl + g * 32, v);
+        tmem_ld_wait();
+        if (SPLIT == 3) {
+          if (kch == 1) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) u[e] = __shfl_xor_sync(0xffffffffu, v[e], 16);
+          } else {
+            tmem_ld32(tl + 128 + g * 32, u);
+            tmem_ld_wait();
+          }
+          if (two) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e]));
+          }
+          tmem_ld32(tl + 256 + g * 32, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e]));
+        }
+        if (min_) {
+          float* dst = part + (size_t)(n0 + g * 32) * a.K + k0 + m;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) dst[(size_t)e * a.K] = __uint_as_float(v[e]);
+        }
+      }
+    }
+  } else {
+    bool ok = true;
+    int n = 0;
+    // D[features of X, features of dY]: both operands MN-major, chunks of 64 features SPLIT * WCHUNK apart
+    const uint32_t idesc = make_idesc_bf16(kch == 1 ? 64 : 128, nlen, 1, 1);
+    const uint64_t D0 = make_smem_desc(sbase, SPLIT * WCHUNK, 1024, LAYOUT_SW128);
+    for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++n) {
+      const int st = n % a.nstages;
+      ok = warp_wait(full + 8 * st, (uint32_t)(n / a.nstages) & 1u);
+      if (!ok) break;
+      if (elect_one()) {
+        tc_fence_after();
+        const uint64_t dd = desc_advance(D0, st * stage), dx = desc_advance(dd, (uint32_t)nch * SPLIT * WCHUNK);
+        const uint32_t lead_set = tmem + (SPLIT == 3 ? (uint32_t)(n & 1) * (kch == 1 ? 16u << 16 : 128u) : 0u), small_set = tmem + 256;
+        const uint32_t acc_l = SPLIT == 3 ? n > 1 : n > 0, acc_s = n > 0;
+#pragma unroll
+        for (int pr = 0; pr < Prod<SPLIT>::N; ++pr) {
+          const bool lead = pr + 1 == Prod<SPLIT>::N;
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_bf16(lead ? lead_set : small_set, desc_advance(dx, Prod<SPLIT>::b(pr) * WCHUNK + kk * 2048),
+                     desc_advance(dd, Prod<SPLIT>::a(pr) * WCHUNK + kk * 2048), idesc, kk > 0 ? 1u : (lead ? acc_l : (pr > 0 ? 1u : acc_s)));
+        }
+        mma_commit(empty + 8 * st);
+        if (tile + G_x >= ntiles) mma_commit(acc_done);
+      }
+      __syncwarp();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == LG_LOADERS) tmem_dealloc(tmem, 512u);
+}
+
+// out[i] = sum over the CTAs' partial results, in a fixed order: 32 groups of four values x 8 slices of the CTAs per block
+__global__ void __launch_bounds__(256) k_lin_reduce(const float* __restrict__ part, int nparts, long long n, long long nw,
+                                                    float* __restrict__ dW, float* __restrict__ db) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long i = ((long long)blockIdx.x * 32 + lane) * 4;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < n) {
+    const int per = (nparts + 7) / 8, b0 = w * per, b1 = min(nparts, b0 + per);
+#pragma unroll 10
+    for (int b = b0; b < b1; ++b) {
+      const float4 v = *reinterpret_cast<const float4*>(part + (size_t)b * n + i);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+  }
+  __shared__ float4 sm[8][32];
+  sm[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && i < n) {
+    for (int x = 1; x < 8; ++x) { s.x += sm[x][lane].x; s.y += sm[x][lane].y; s.z += sm[x][lane].z; s.w += sm[x][lane].w; }
+    float* dst = i < nw ? dW + i : db + (i - nw);         // both lengths are multiples of four
+    *reinterpret_cast<float4*>(dst) = s;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ host
+constexpr size_t SMEM_MAX = 227 * 1024 - 1024;
+
+int sm_count() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev < 64 && cached[dev]) return cached[dev];
+  int n = 0;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (dev < 64) cached[dev] = n;
+  return n;
+}
+
+TokMat to_mat(const spion_tokens* t) {
+  TokMat m;
+  for (int i = 0; i < 3; ++i) m.p[i] = t->ptr[i];
+  m.per = t->cols;
+  if (t->heads > 0) {
+    m.d = t->head_dim; m.L = t->seq_len;
+    m.dsh = 0;
+    while ((1 << m.dsh) < m.d) ++m.dsh;
+    m.hstride = (long long)m.L * m.d; m.bstride = m.hstride * t->heads;
+  } else {
+    m.d = t->cols; m.L = 0x7fffffff; m.dsh = 31; m.hstride = 0; m.bstride = 0;
+  }
+  return m;
+}
+bool mat_ok(const spion_tokens* t) {
+  if (!t || t->count < 1 || t->count > 3 || t->cols < 32 || t->cols % 32) return false;
+  if (t->heads > 0 && (t->head_dim < 32 || (t->head_dim & (t->head_dim - 1)) || t->heads * t->head_dim != t->cols || t->seq_len < 1))
+    return false;
+  for (int i = 0; i < t->count; ++i)
+    if (!t->ptr[i] || ((uintptr_t)t->ptr[i] & 31)) return false;
+  return true;
+}
+
+// columns per CTA, accumulators and ring stages of the GEMM; false when the weights do not fit
+bool plan_gemm(int split, bool trans, int K, int N, int* nc, int* nacc, int* stages, size_t* smem, int widest = 256) {
+  const int least = split == 1 ? LG_DEPTH + 1 : 2;           // bf16 operands keep LG_DEPTH chunks in flight
+  const int nchunks = (K + 63) / 64;
+  const int most = split == 3 && nchunks > 1 ? 64 : widest;     // several accumulators of 64 columns keep the fp32 chains short
+  for (int parts = 1; parts <= 64; ++parts) {
+    int c = ((N + parts - 1) / parts + 31) / 32 * 32;
+    if (parts > 1 && trans) c = (c + 63) / 64 * 64;
+    if (c > most) continue;
+    const size_t bchunk = trans ? (size_t)((c + 63) / 64) * 8192 : (size_t)c * 128;
+    const size_t b = split * ((nchunks * bchunk + 1023) / 1024 * 1024);
+    for (int st = split == 1 ? 8 : 4; st >= least; --st) {
+      const size_t total = b + (size_t)st * split * CHUNK + 1024 + 256;
+      if (total <= SMEM_MAX) { *nc = c; *nacc = split == 3 && nchunks > 1 ? 4 : 1; *stages = st; *smem = total; return true; }
+    }
+    if (c <= 64) break;
+  }
+  return false;
+}
+
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
+int launch_gemm(const GemmArgs& a, size_t smem, cudaStream_t st) {
+  static bool set[64] = {false};
+  int dev = 0;
+  SPION_CUDA_TRY(cudaGetDevice(&dev));
+  auto k = k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>;
+  if (dev >= 64 || !set[dev]) {
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    if (dev < 64) set[dev] = true;
+  }
+  const int ny = (a.N + a.nc - 1) / a.nc;
+  const int sms = sm_count(), tiles = (a.T + 127) / 128;
+  if (sms < 1) return SPION_ERR_CUDA;
+  int gx = sms / ny > 0 ? sms / ny : 1;
+  if (gx > tiles) gx = tiles;
+  k<<<dim3(gx, ny), LG_THREADS, smem, st>>>(a);
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}
+
+template <int SPLIT, bool DY_BF16, bool X_BF16>
+int launch_wgrad(const WgradArgs& a, int gx, size_t smem, cudaStream_t st) {
+  static bool set[64] = {false};
+  int dev = 0;
+  SPION_CUDA_TRY(cudaGetDevice(&dev));
+  auto k = k_lin_wgrad<SPLIT, DY_BF16, X_BF16>;
+  if (dev >= 64 || !set[dev]) {
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    if (dev < 64) set[dev] = true;
+  }
+  k<<<dim3(gx, (a.N + a.nc - 1) / a.nc, (a.K + a.kc - 1) / a.kc), WG_THREADS, smem, st>>>(a);
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}
+
+// chunking of the weight gradient: at most four 64-wide chunks of dY and X per CTA, and what tensor memory holds
+bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, size_t* smem) {
+  const int kw = K <= 64 ? 64 : 128;
+  int nw = (N + 63) / 64 * 64;
+  if (nw + kw > 256) nw = 256 - kw;
+  const int cpt = (nw + kw) / 64;
+  const size_t stage = (size_t)cpt * split * WCHUNK;
+  for (int st = split == 1 ? 6 : 4; st >= (split == 1 ? 3 : 2); --st) {     // bf16 operands: two stages of copies in flight
+    const size_t total = st * stage + 256 + 8 * 256 * 4;
+    if (total <= SMEM_MAX) { *nc = nw; *kc = kw; *stages = st; *smem = total; return true; }
+  }
+  return false;
+}
+
+int wgrad_grid(long long T, int N, int K, int split) {
+  int nc, kc, st;
+  size_t smem;
+  if (!plan_wgrad(split, N, K, &nc, &kc, &st, &smem)) return 0;
+  const int per = ((N + nc - 1) / nc) * ((K + kc - 1) / kc);
+  const long long tiles = (T + 63) / 64;
+  int gx = sm_count() / per;
+  if (gx < 1) gx = 1;
+  return (int)(gx < tiles ? gx : tiles);
+}
+
+}  // namespace
+
+// longest contraction (a multiple of 64) of one launch of the input-gradient GEMM
+static int max_contraction(int split, int N) {
+  int nc, nacc, st;
+  size_t smem;
+  int k = 1024;
+  while (k > 64 && !plan_gemm(split, true, k, N, &nc, &nacc, &st, &smem)) k -= 64;
+  return k;
+}
+
+extern "C" int spion_linear_supported(int in_features, int out_features, int fp32) {
+  int nc, kc, nacc, st;
+  size_t smem;
+  const int sp = fp32 ? 3 : 1;
+  if (in_features < 32 || out_features < 32 || in_features % 32 || out_features % 32) return 0;
+  if (in_features > 1024 || out_features > 1024) return 0;
+  return plan_gemm(sp, false, in_features, out_features, &nc, &nacc, &st, &smem) &&
+         plan_gemm(sp, true, fp32 ? 64 : out_features, in_features, &nc, &nacc, &st, &smem) &&
+         plan_wgrad(sp, out_features, in_features, &nc, &kc, &st, &smem);
+}
+
+extern "C" int spion_linear_status(int reset) {
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_lin_status, sizeof(int)) != cudaSuccess) return SPION_ERR_CUDA;
+  if (reset && v) { const int z = 0; if (cudaMemcpyToSymbol(g_lin_status, &z, sizeof(int)) != cudaSuccess) return SPION_ERR_CUDA; }
+  return v == 0 ? SPION_OK : SPION_ERR_TIMEOUT;
+}
+
+extern "C" int spion_linear_forward(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
+                                    const spion_tokens* Y, void* gelu_out, long long T, int in_features, int out_features,
+                                    void* cuda_stream) {
+  if (!mat_ok(X) || !mat_ok(Y) || !W || nw < 1 || nw > 3 || T < 1 || T > 0x7fffffffLL - 256) return SPION_ERR_ARG;
+  if (X->cols * X->count != in_features || Y->cols * Y->count != out_features || out_features % nw) return SPION_ERR_ARG;
+  if (fp32 && (X->is_bf16 || Y->is_bf16 || gelu_out)) return SPION_ERR_UNSUPPORTED;
+  if (gelu_out && (!Y->is_bf16 || ((uintptr_t)gelu_out & 31))) return SPION_ERR_UNSUPPORTED;
+  GemmArgs a;
+  a.A = to_mat(X); a.Y = to_mat(Y);
+  a.wper = out_features / nw; a.wld = in_features;
+  for (int i = 0; i < 3; ++i) { a.W[i] = i < nw ? W[i] : nullptr; a.bias[i] = (bias && i < nw) ? bias[i] : nullptr; }
+  for (int i = 0; i < nw; ++i) if (!a.W[i] || ((uintptr_t)a.W[i] & 15)) return SPION_ERR_ARG;
+  a.T = (int)T; a.K = in_features; a.N = out_features;
+  a.h = nullptr; a.g = (__nv_bfloat16*)gelu_out;
+  size_t smem;
+  a.k0 = 0; a.accum = 0; a.parts = 0;
+  if (!plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)cuda_stream;
+  if (fp32) return launch_gemm<3, false, false, EPI_NONE, false>(a, smem, st);
+  if (gelu_out)
+    return X->is_bf16 ? launch_gemm<1, true, false, EPI_GELU, true>(a, smem, st) : launch_gemm<1, false, false, EPI_GELU, true>(a, smem, st);
+  if (Y->is_bf16)
+    return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, true>(a, smem, st) : launch_gemm<1, false, false, EPI_NONE, true>(a, smem, st);
+  return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, false>(a, smem, st) : launch_gemm<1, false, false, EPI_NONE, false>(a, smem, st);
+}
+
+extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* const* W, int nw, int fp32, const void* gelu_in,
+                                           const spion_tokens* dX, long long T, int in_features, int out_features,
+                                           void* cuda_stream) {
+  if (!mat_ok(dY) || !mat_ok(dX) || !W || nw < 1 || nw > 3 || T < 1 || T > 0x7fffffffLL - 256) return SPION_ERR_ARG;
+  if (dX->cols * dX->count != in_features || dY->cols * dY->count != out_features || out_features % nw) return SPION_ERR_ARG;
+  if (fp32 && (dX->is_bf16 || dY->is_bf16 || gelu_in)) return SPION_ERR_UNSUPPORTED;
+  if (gelu_in && (!dX->is_bf16 || ((uintptr_t)gelu_in & 31))) return SPION_ERR_UNSUPPORTED;
+  GemmArgs a;
+  a.A = to_mat(dY); a.Y = to_mat(dX);
+  a.wper = out_features / nw; a.wld = in_features;
+  for (int i = 0; i < 3; ++i) { a.W[i] = i < nw ? W[i] : nullptr; a.bias[i] = nullptr; }
+  for (int i = 0; i < nw; ++i) if (!a.W[i] || ((uintptr_t)a.W[i] & 15)) return SPION_ERR_ARG;
+  a.T = (int)T; a.K = out_features; a.N = in_features;
+  a.h = (const __nv_bfloat16*)gelu_in; a.g = nullptr;
+  size_t smem;
+  a.k0 = 0; a.accum = 0;
+  a.parts = !fp32 && dX->is_bf16 && nw == 3 ? a.wper / 64 : 0;
+  if (a.parts && a.wper % 64) return SPION_ERR_UNSUPPORTED;
+  cudaStream_t st = (cudaStream_t)cuda_stream;
+  if (fp32) {                                            // the split weights of a long contraction fill shared memory: several launches
+    const int total = a.K, step = max_contraction(3, a.N);
+    for (a.k0 = 0; a.k0 < total; a.k0 += step) {
+      a.K = total - a.k0 < step ? total - a.k0 : step;
+      a.accum = a.k0 > 0;
+      if (!plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
+      const int rc = launch_gemm<3, false, true, EPI_NONE, false>(a, smem, st);
+      if (rc) return rc;
+    }
+    return SPION_OK;
+  }
+  if (!plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256)) return SPION_ERR_UNSUPPORTED;
+  if (gelu_in)
+    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_DGELU, true>(a, smem, st) : launch_gemm<1, false, true, EPI_DGELU, true>(a, smem, st);
+  if (dX->is_bf16)
+    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, true>(a, smem, st) : launch_gemm<1, false, true, EPI_NONE, true>(a, smem, st);
+  return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, false>(a, smem, st) : launch_gemm<1, false, true, EPI_NONE, false>(a, smem, st);
+}
+
+extern "C" long long spion_linear_workspace_floats(long long T, int in_features, int out_features, int fp32) {
+  return (long long)wgrad_grid(T, out_features, in_features, fp32 ? 3 : 1) * ((long long)in_features * out_features + out_features);
+}
+
+extern "C" int spion_linear_backward_weight(const spion_tokens* dY, const spion_tokens* X, int fp32, float* dW, float* db,
+                                            float* workspace, long long T, int in_features, int out_features, void* cuda_stream) {
+  if (!mat_ok(dY) || !mat_ok(X) || !dW || !db || !workspace || T < 1 || T > 0x7fffffffLL - 256) return SPION_ERR_ARG;
+  if (((uintptr_t)dW | (uintptr_t)db | (uintptr_t)workspace) & 15) return SPION_ERR_ARG;
+  if (X->cols * X->count != in_features || dY->cols * dY->count != out_features) return SPION_ERR_ARG;
+  if (fp32 && (X->is_bf16 || dY->is_bf16)) return SPION_ERR_UNSUPPORTED;
+  WgradArgs a;
+  a.dY = to_mat(dY); a.X = to_mat(X);
+  a.T = (int)T; a.N = out_features; a.K = in_features; a.part = workspace;
+  size_t smem;
+  if (!plan_wgrad(fp32 ? 3 : 1, a.N, a.K, &a.nc, &a.kc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
+  const int gx = wgrad_grid(T, a.N, a.K, fp32 ? 3 : 1);
+  if (gx < 1) return SPION_ERR_CUDA;
+  cudaStream_t st = (cudaStream_t)cuda_stream;
+  int rc;
+  if (fp32) rc = launch_wgrad<3, false, false>(a, gx, smem, st);
+  else if (dY->is_bf16) rc = X->is_bf16 ? launch_wgrad<1, true, true>(a, gx, smem, st) : launch_wgrad<1, true, false>(a, gx, smem, st);
+  else rc = X->is_bf16 ? launch_wgrad<1, false, true>(a, gx, smem, st) : launch_wgrad<1, false, false>(a, gx, smem, st);
+  if (rc) return rc;
+  const long long nw = (long long)a.N * a.K, n = nw + a.N;
+  k_lin_reduce<<<(unsigned)((n / 4 + 31) / 32), 256, 0, st>>>(workspace, gx, n, nw, dW, db);
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}

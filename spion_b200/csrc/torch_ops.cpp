@@ -1,0 +1,609 @@
+// Host path of the Python modules in native code: the autograd nodes around the C ABI (include/spion_b200.h).
+//
+// A call through torch.autograd.Function costs 30 - 60 us of interpreter time in each direction, and an attention layer is six of
+// them (projections, attention, output projection) plus casts, copies and reductions: 1.1 ms per forward + backward of a layer
+// whose kernels take 50 us.  Here a layer is one node: projections, attention and output projection call the library
+// back to back, in the layouts the next kernel reads, and the backward does the same.
+//
+// Only orchestration lives here; every kernel is behind the C ABI.
+#include <torch/extension.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <memory>
+#include <vector>
+
+#include "../../include/spion_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+using c10::optional;
+
+struct Failure : std::runtime_error { using std::runtime_error::runtime_error; };
+
+void check(int rc, const char* what) {
+  if (rc != 0) throw Failure(std::string(what) + " failed: " + spion_status_string(rc) + " (" + std::to_string(rc) + ")");
+}
+
+void* stream_of(const Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+void* p(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+const float* pf(const Tensor& t) { return t.defined() ? (const float*)t.data_ptr() : nullptr; }
+
+// ------------------------------------------------------------------------------------------------ token matrices
+spion_tokens tok(const std::vector<Tensor>& ts, int cols) {
+  spion_tokens t = {};
+  t.count = (int)ts.size();
+  for (int i = 0; i < t.count; ++i) t.ptr[i] = ts[i].data_ptr();
+  t.cols = cols;
+  t.is_bf16 = ts[0].scalar_type() == at::kBFloat16;
+  return t;
+}
+spion_tokens tok_heads(const std::vector<Tensor>& ts, int H, int d, int L) {
+  spion_tokens t = tok(ts, H * d);
+  t.heads = H; t.head_dim = d; t.seq_len = L;
+  return t;
+}
+bool aligned32(const Tensor& t) { return ((uintptr_t)t.data_ptr() & 31) == 0; }
+
+struct Weights {                        // up to three stacked linear layers
+  std::vector<Tensor> W, b;
+  int n() const { return (int)W.size(); }
+  int in() const { return (int)W[0].size(1); }
+  int out() const { return (int)(W[0].size(0) * W.size()); }
+};
+
+void linear_forward(const spion_tokens& X, const Weights& w, bool fp32, const spion_tokens& Y, void* gelu_out, int64_t T, void* st) {
+  const float *W[3], *b[3];
+  for (int i = 0; i < w.n(); ++i) { W[i] = pf(w.W[i]); b[i] = pf(w.b[i]); }
+  check(spion_linear_forward(&X, W, b, w.n(), fp32, &Y, gelu_out, T, w.in(), w.out(), st), "spion_linear_forward");
+}
+void linear_backward_input(const spion_tokens& dY, const Weights& w, bool fp32, const void* gelu_in, const spion_tokens& dX, int64_t T, void* st) {
+  const float* W[3];
+  for (int i = 0; i < w.n(); ++i) W[i] = pf(w.W[i]);
+  check(spion_linear_backward_input(&dY, W, w.n(), fp32, gelu_in, &dX, T, w.in(), w.out(), st), "spion_linear_backward_input");
+}
+// Weight and bias gradients of the stacked layers from dY (one [T, per] matrix per layer, or their head-split form) and X.
+// fp32 tokens: the library's kernel, views of one buffer.  bf16 tokens (a layer inside a mixed-precision encoder): the
+// framework's bf16 products and the column-sum kernel, so that a training step repeats bit for bit what separate layers give.
+void linear_backward_weight(const std::vector<Tensor>& dY, const spion_tokens& tY, const Tensor& X, const spion_tokens& tX, const Weights& w,
+                            bool fp32, int64_t T, void* st, std::vector<Tensor>& dW, std::vector<Tensor>& db) {
+  const int64_t in = w.in(), out = w.out(), per = out / w.n();
+  const auto opt = w.W[0].options();
+  if (tX.is_bf16 && tY.heads == 0 && tX.heads == 0) {
+    Tensor x2 = X.view({T, in});
+    for (int i = 0; i < w.n(); ++i) {
+      Tensor dy2 = dY[i].view({T, per});
+      dW.push_back(at::mm(dy2.t(), x2).to(at::kFloat));
+      if (per == 64 || per == 128 || per == 256 || per == 512) {
+        Tensor g = at::empty({per}, opt), ws = at::empty({(int64_t)spion_layernorm_workspace_floats((int)per)}, opt);
+        check(spion_column_sums(dy2.data_ptr(), 1, (float*)g.data_ptr(), (float*)ws.data_ptr(), T, (int)per, st), "spion_column_sums");
+        db.push_back(g);
+      } else {
+        db.push_back(dy2.sum(0).to(at::kFloat));
+      }
+    }
+    return;
+  }
+  Tensor g = at::empty({out * in + out}, opt);
+  Tensor ws = at::empty({(int64_t)spion_linear_workspace_floats(T, (int)in, (int)out, fp32)}, opt);
+  float* gp = (float*)g.data_ptr();
+  check(spion_linear_backward_weight(&tY, &tX, fp32, gp, gp + out * in, (float*)ws.data_ptr(), T, (int)in, (int)out, st),
+        "spion_linear_backward_weight");
+  for (int i = 0; i < w.n(); ++i) {
+    dW.push_back(g.narrow(0, i * per * in, per * in).view({per, in}));
+    db.push_back(g.narrow(0, out * in + i * per, per));
+  }
+}
+
+bool weights_ok(const std::vector<Tensor>& W, const std::vector<Tensor>& b, const Tensor& like, bool fp32) {
+  const int64_t in = W[0].size(1), out = W[0].size(0);
+  for (size_t i = 0; i < W.size(); ++i) {
+    if (W[i].scalar_type() != at::kFloat || !W[i].is_contiguous() || W[i].device() != like.device() || !aligned32(W[i])) return false;
+    if (!b[i].defined() || b[i].scalar_type() != at::kFloat || !b[i].is_contiguous() || b[i].device() != like.device()) return false;
+    if (W[i].size(0) != out || W[i].size(1) != in) return false;
+  }
+  return spion_linear_supported((int)in, (int)(out * W.size()), fp32) != 0;
+}
+
+// ------------------------------------------------------------------------------------------------ attention context
+enum Mode { NATIVE = 0, DROPIN_SPARSE = 1, DROPIN_DENSE = 2 };
+
+// What the Python modules keep per attention context: the C ABI's handle and the sizes it was created with.
+struct Context {
+  int64_t handle = 0;
+  int mode = NATIVE;
+  int64_t B = 0, H = 0, L = 0, d = 0;
+  int device = 0;
+  bool bf16 = false, keypad = false, fused = false, recompute = false, return_probs = true, needs_scratch = false;
+  bool owned = false;                   // destroys the handle
+  int64_t nnz = 0;                      // selected elements per (b,h) matrix
+  Tensor sum_mat, offsets, columns;     // element CSR of the drop-in layout
+  spion_ctx* ctx() const { return reinterpret_cast<spion_ctx*>(handle); }
+  at::ScalarType type() const { return bf16 ? at::kBFloat16 : at::kFloat; }
+  void close() { if (owned && handle) { spion_destroy(ctx()); } handle = 0; }
+  ~Context() { close(); }
+};
+using ContextPtr = std::shared_ptr<Context>;
+
+std::string shape_str(const Tensor& t) {
+  std::string s = "(";
+  for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
+  return s + ")";
+}
+void check_operand(const Context& c, const Tensor& t, const char* name) {
+  if (t.dim() != 4 || t.size(0) != c.B || t.size(1) != c.H || t.size(2) != c.L || t.size(3) != c.d)
+    throw Failure(std::string(name) + " has shape " + shape_str(t) + ", this module was built for (" + std::to_string(c.B) + ", " +
+                  std::to_string(c.H) + ", " + std::to_string(c.L) + ", " + std::to_string(c.d) +
+                  ") (batch_size, num_head, max_seq_len, head_dim of its config)");
+  if (!t.is_cuda() || t.device().index() != c.device)
+    throw Failure(std::string(name) + " is on " + t.device().str() + ", the module's context is on cuda:" + std::to_string(c.device));
+}
+
+// key-padding mask [B, L] of 1 / 0 -> penalty per (b,h) matrix [BH, L]
+Tensor penalty(const Context& c, const Tensor& mask, const Tensor& like, void* st) {
+  if (!mask.defined() || mask.dim() != 2 || mask.size(0) != c.B || mask.size(1) != c.L)
+    throw Failure("key-padding mask must have shape (" + std::to_string(c.B) + ", " + std::to_string(c.L) + ")");
+  Tensor m = mask.to(like.device(), at::kFloat).contiguous();
+  Tensor pen = at::empty({c.B, c.H, c.L}, like.options().dtype(at::kFloat));
+  check(spion_expand_keypad(pf(m), (int)c.B, (int)c.H, (int)c.L, (float*)pen.data_ptr(), st), "spion_expand_keypad");
+  return pen;
+}
+
+// One forward call: operands in, results out (everything the backward needs).
+struct Attn {
+  Tensor q, k, v, pen, O, lse, P;
+  int heads = 0;                        // 0: operands [B, H, L, d] contiguous; H: views of [B, L, H, d]
+};
+
+Tensor empty_operand(const Context& c, int heads, const Tensor& like) {
+  const auto opt = like.options().dtype(c.type());
+  if (heads) return at::empty({c.B, c.L, c.H, c.d}, opt).transpose(1, 2);
+  return at::empty({c.B, c.H, c.L, c.d}, opt);
+}
+// 0: contiguous [B, H, L, d]; H: the head-split view of a contiguous [B, L, H, d] tensor; -1: neither
+int operand_form(const Context& c, const Tensor& t) {
+  if (t.is_contiguous()) return 0;
+  if (t.stride(0) == c.L * c.H * c.d && t.stride(1) == c.d && t.stride(2) == c.H * c.d && t.stride(3) == 1) return (int)c.H;
+  return -1;
+}
+
+void attn_forward(const Context& c, Attn& a, void* st) {
+  spion_ctx* x = c.ctx();
+  const auto f32 = a.q.options().dtype(at::kFloat);
+  check(spion_set_stream(x, st), "spion_set_stream");
+  if (c.mode == DROPIN_SPARSE) {
+    a.O = empty_operand(c, 0, a.q);
+    a.P = at::empty({c.B * c.H * c.nnz}, f32);
+    check(spion_block_attn_forward_rm(x, pf(a.q), pf(a.k), pf(a.v), pf(a.pen), (float*)a.P.data_ptr(), (float*)a.O.data_ptr(),
+                                      (const int*)c.offsets.data_ptr(), (const int*)c.columns.data_ptr(),
+                                      (const int*)c.sum_mat.data_ptr(), (int)c.nnz), "spion_block_attn_forward_rm");
+    return;
+  }
+  if (c.mode == DROPIN_DENSE) {
+    a.O = empty_operand(c, 0, a.q);
+    a.P = at::empty({c.B, c.H, c.L, c.L}, f32);
+    check(spion_dense_attn_forward_rm(x, pf(a.q), pf(a.k), pf(a.v), pf(a.pen), (float*)a.P.data_ptr(), (float*)a.O.data_ptr()),
+          "spion_dense_attn_forward_rm");
+    return;
+  }
+  check(spion_set_head_layout(x, a.heads), "spion_set_head_layout");
+  a.O = empty_operand(c, a.heads, a.q);
+  if (c.fused) {
+    a.lse = at::empty({c.B * c.H * c.L}, f32);
+    // the probabilities are stored only for callers that want them back; the backward rebuilds its tiles
+    if (c.return_probs || !c.recompute) a.P = at::empty({c.B * c.H * c.nnz}, a.q.options());
+    check(spion_attn_forward_fused(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.O), (float*)a.lse.data_ptr(), p(a.P)),
+          "spion_attn_forward_fused");
+  } else {
+    a.P = at::empty({c.B * c.H * c.nnz}, a.q.options());
+    Tensor scratch;
+    if (c.needs_scratch) scratch = at::empty({c.B * c.H * c.nnz}, f32);
+    check(spion_attn_forward_ex(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.P), p(a.O), (float*)p(scratch)), "spion_attn_forward_ex");
+  }
+}
+
+void attn_backward(const Context& c, const Attn& a, const Tensor& dO, Tensor& dq, Tensor& dk, Tensor& dv, void* st) {
+  spion_ctx* x = c.ctx();
+  const auto f32 = a.q.options().dtype(at::kFloat);
+  dq = empty_operand(c, a.heads, a.q); dk = empty_operand(c, a.heads, a.q); dv = empty_operand(c, a.heads, a.q);
+  check(spion_set_stream(x, st), "spion_set_stream");
+  if (c.mode == DROPIN_SPARSE) {
+    Tensor dS = at::empty({c.B * c.H * c.nnz}, f32);
+    Tensor dP;
+    if (spion_block_attn_needs_scratch(x)) dP = at::empty({c.B * c.H * c.nnz}, f32);
+    check(spion_block_attn_backward_rm(x, pf(a.q), pf(a.k), pf(a.v), pf(a.P), pf(a.O), pf(dO), (float*)p(dP), (float*)dS.data_ptr(),
+                                       (float*)dq.data_ptr(), (float*)dk.data_ptr(), (float*)dv.data_ptr(),
+                                       (const int*)c.offsets.data_ptr(), (const int*)c.columns.data_ptr(),
+                                       (const int*)c.sum_mat.data_ptr(), (int)c.nnz), "spion_block_attn_backward_rm");
+    return;
+  }
+  if (c.mode == DROPIN_DENSE) {
+    const long long n = spion_dense_attn_scratch_floats(x);
+    Tensor s1, s3;
+    if (n > 0) { s1 = at::empty({n}, f32); s3 = at::empty({n}, f32); }
+    check(spion_dense_attn_backward_rm(x, pf(a.q), pf(a.k), pf(a.v), pf(a.P), pf(a.O), pf(dO), (float*)p(s1), (float*)p(s3),
+                                       (float*)dq.data_ptr(), (float*)dk.data_ptr(), (float*)dv.data_ptr()),
+          "spion_dense_attn_backward_rm");
+    return;
+  }
+  check(spion_set_head_layout(x, a.heads), "spion_set_head_layout");
+  if (c.fused && !a.P.defined()) {
+    check(spion_attn_backward_fused(x, p(a.q), p(a.k), p(a.v), p(a.O), p(dO), pf(a.lse), pf(a.pen), p(dq), p(dk), p(dv)),
+          "spion_attn_backward_fused");
+    return;
+  }
+  Tensor dS = at::empty({c.B * c.H * c.nnz}, a.q.options()), scratch;
+  if (!c.fused && c.needs_scratch) scratch = at::empty({c.B * c.H * c.nnz}, f32);
+  check(spion_attn_backward_ex(x, p(a.q), p(a.k), p(a.v), p(a.P), p(a.O), p(dO), p(dS), (float*)p(scratch), nullptr, p(dq), p(dk), p(dv)),
+        "spion_attn_backward_ex");
+}
+
+// ------------------------------------------------------------------------------------------------ autograd nodes
+SavedVariable save(const Tensor& t) { return SavedVariable(t, false); }
+
+struct AttnNode : public Node {
+  ContextPtr c;
+  Attn a;                                // q, k, v hold what the kernels read (copies where a cast or a packing was needed)
+  SavedVariable sq, sk, sv;              // the inputs themselves, where the kernels read them in place
+  bool iq = false, ik = false, iv = false;
+  at::ScalarType tq, tk, tv;
+  bool released = false;
+  std::string name() const override { return "BlockSparseAttentionBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    sq.reset_data(); sk.reset_data(); sv.reset_data();
+    a = Attn();
+    released = true;
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    TORCH_CHECK(!released, "Trying to backward through the graph a second time (the saved tensors have been freed)");
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    c10::cuda::CUDAGuard guard(c->device);
+    Attn s = a;
+    if (iq) s.q = sq.unpack();
+    if (ik) s.k = sk.unpack();
+    if (iv) s.v = sv.unpack();
+    Tensor go = grads[0].to(c->type());
+    if (s.heads && operand_form(*c, go) != s.heads) go = go.transpose(1, 2).contiguous().transpose(1, 2);
+    else if (!s.heads) go = go.contiguous();
+    Tensor dq, dk, dv;
+    attn_backward(*c, s, go, dq, dk, dv, stream_of(go));
+    out[0] = dq.to(tq); out[1] = dk.to(tk); out[2] = dv.to(tv);
+    return out;
+  }
+};
+
+// attention(q, k, v) -> out, probs (undefined when none were stored), lse, pen, q used, k used, heads
+py::tuple attention(const ContextPtr& c, const Tensor& query, const Tensor& key, const Tensor& value, const optional<Tensor>& mask) {
+  check_operand(*c, query, "query");
+  check_operand(*c, key, "key");
+  check_operand(*c, value, "value");
+  c10::cuda::CUDAGuard guard(c->device);
+  void* st = stream_of(query);
+  const bool need = at::GradMode::is_enabled() && (query.requires_grad() || key.requires_grad() || value.requires_grad());
+  Attn a;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    if (c->keypad) a.pen = penalty(*c, mask.has_value() ? *mask : Tensor(), query, st);
+    a.q = query.detach().to(c->type()); a.k = key.detach().to(c->type()); a.v = value.detach().to(c->type());
+    // head-split views of [B, L, H*d] projections are read where they lie; anything else is packed
+    if (c->fused && operand_form(*c, a.q) == c->H && operand_form(*c, a.k) == c->H && operand_form(*c, a.v) == c->H) a.heads = (int)c->H;
+    if (!a.heads) { a.q = a.q.contiguous(); a.k = a.k.contiguous(); a.v = a.v.contiguous(); }
+    attn_forward(*c, a, st);
+  }
+  Tensor out = a.O;
+  if (need) {
+    auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(query, key, value));
+    node->c = c;
+    node->a = a;
+    if (c->fused && c->recompute) node->a.P = Tensor();
+    node->tq = query.scalar_type(); node->tk = key.scalar_type(); node->tv = value.scalar_type();
+    node->iq = a.q.is_same(query) || a.q.data_ptr() == query.data_ptr();
+    node->ik = a.k.data_ptr() == key.data_ptr();
+    node->iv = a.v.data_ptr() == value.data_ptr();
+    if (node->iq) { node->sq = save(query); node->a.q = Tensor(); }
+    if (node->ik) { node->sk = save(key); node->a.k = Tensor(); }
+    if (node->iv) { node->sv = save(value); node->a.v = Tensor(); }
+    if (node->iq) node->a.q = Tensor();
+    out = a.O.detach();
+    node->a.O = a.O;
+    torch::autograd::set_history(out, node);
+  }
+  return py::make_tuple(out, a.P.defined() ? py::cast(a.P) : py::none(), a.lse.defined() ? py::cast(a.lse) : py::none(),
+                        a.pen.defined() ? py::cast(a.pen) : py::none(), a.q, a.k, a.heads);
+}
+
+// A whole multi-head attention layer: x [B, L, dim] -> projections -> attention -> output projection [B, L, dim_out].
+struct LayerNode : public Node {
+  ContextPtr c;
+  bool fp32 = false;
+  Attn a;
+  SavedVariable x, w[4];                 // Wq, Wk, Wv, Wf
+  at::ScalarType out_type;
+  bool released = false;
+  std::string name() const override { return "SparseAttentionLayerBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    x.reset_data();
+    for (auto& s : w) s.reset_data();
+    a = Attn();
+    released = true;
+  }
+  // inputs: x, Wq, bq, Wk, bk, Wv, bv, Wf, bf
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    TORCH_CHECK(!released, "Trying to backward through the graph a second time (the saved tensors have been freed)");
+    variable_list out(9);
+    if (!grads[0].defined()) return out;
+    c10::cuda::CUDAGuard guard(c->device);
+    const int H = (int)c->H, d = (int)c->d, L = (int)c->L;
+    const int64_t T = c->B * c->L;
+    Tensor X = x.unpack();
+    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    const int dim = (int)X.size(2);
+    Weights qkv, ff;
+    for (int i = 0; i < 3; ++i) qkv.W.push_back(w[i].unpack());
+    ff.W.push_back(w[3].unpack());
+    Tensor go = grads[0].to(out_type).contiguous();
+    if (!aligned32(go)) go = go.clone();
+    void* st = stream_of(go);
+    auto form = [&](const std::vector<Tensor>& ts) { return a.heads ? tok(ts, H * d) : tok_heads(ts, H, d, L); };
+    auto rows = [&](const Tensor& t) { return a.heads ? t.transpose(1, 2).view({T, H * d}) : t; };
+    const spion_tokens tgo = tok({go}, (int)ff.W[0].size(0));
+    const spion_tokens tO = form({a.O});
+    std::vector<Tensor> dW, db;
+    if (task_should_compute_output(7) || task_should_compute_output(8)) {
+      linear_backward_weight({go}, tgo, rows(a.O), tO, ff, fp32, T, st, dW, db);
+      out[7] = dW[0]; out[8] = db[0];
+    }
+    Tensor dO = empty_operand(*c, a.heads, a.q);
+    linear_backward_input(tgo, ff, fp32, nullptr, form({dO}), T, st);
+    Tensor dq, dk, dv;
+    attn_backward(*c, a, dO, dq, dk, dv, st);
+    const spion_tokens tg = form({dq, dk, dv});
+    bool any = false;
+    for (int i = 1; i < 7; ++i) any = any || task_should_compute_output(i);
+    if (any) {
+      dW.clear(); db.clear();
+      linear_backward_weight({rows(dq), rows(dk), rows(dv)}, tg, X, tok({X}, dim), qkv, fp32, T, st, dW, db);
+      for (int i = 0; i < 3; ++i) { out[1 + 2 * i] = dW[i]; out[2 + 2 * i] = db[i]; }
+    }
+    if (task_should_compute_output(0)) {
+      Tensor dX = at::empty(X.sizes(), X.options());
+      linear_backward_input(tg, qkv, fp32, nullptr, tok({dX}, dim), T, st);
+      out[0] = dX;
+    }
+    return out;
+  }
+};
+
+// Can the layer run as one node?  fp32: everything in fp32; else bf16 operands (mixed precision).
+bool layer_supported(const ContextPtr& c, const Tensor& x, const std::vector<Tensor>& W, const std::vector<Tensor>& b, bool fp32) {
+  if (c->bf16 == fp32) return false;
+  if (!x.is_cuda() || x.device().index() != c->device || x.dim() != 3 || x.size(0) != c->B || x.size(1) != c->L) return false;
+  if (x.scalar_type() != at::kFloat && (fp32 || x.scalar_type() != at::kBFloat16)) return false;
+  if ((c->d & (c->d - 1)) || c->d < 32 || x.size(2) != W[0].size(1) || W[3].size(1) != c->H * c->d || W[0].size(0) != c->H * c->d) return false;
+  if (x.scalar_type() == at::kBFloat16 && (W[0].size(0) % 64 || !c->fused)) return false;      // see spion_linear_backward_input
+  return weights_ok({W[0], W[1], W[2]}, {b[0], b[1], b[2]}, x, fp32) && weights_ok({W[3]}, {b[3]}, x, fp32);
+}
+
+// -> out, P (or None), lse, pen, q, k, heads
+py::tuple attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tensor>& mask, const std::vector<Tensor>& W,
+                          const std::vector<Tensor>& b, bool fp32) {
+  c10::cuda::CUDAGuard guard(c->device);
+  void* st = stream_of(x);
+  const int H = (int)c->H, d = (int)c->d, L = (int)c->L;
+  const int64_t T = c->B * c->L;
+  bool need = x.requires_grad();
+  for (int i = 0; i < 4; ++i) need = need || W[i].requires_grad() || b[i].requires_grad();
+  need = need && at::GradMode::is_enabled();
+  Attn a;
+  Tensor out;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    Tensor X = x.detach();
+    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    const auto opt = X.options().dtype(c->type());
+    if (c->keypad) a.pen = penalty(*c, mask.has_value() ? *mask : Tensor(), X, st);
+    // bf16 tokens: operands stay [B, L, H, d], whose rows the weight gradients' matrix products read
+    a.heads = X.scalar_type() == at::kBFloat16 && c->fused ? H : 0;
+    auto form = [&](const std::vector<Tensor>& ts) { return a.heads ? tok(ts, H * d) : tok_heads(ts, H, d, L); };
+    const Tensor like = at::empty({0}, opt);
+    a.q = empty_operand(*c, a.heads, like); a.k = empty_operand(*c, a.heads, like); a.v = empty_operand(*c, a.heads, like);
+    Weights qkv{{W[0].detach(), W[1].detach(), W[2].detach()}, {b[0].detach(), b[1].detach(), b[2].detach()}};
+    Weights ff{{W[3].detach()}, {b[3].detach()}};
+    linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st);
+    attn_forward(*c, a, st);
+    out = at::empty({c->B, c->L, ff.out()}, opt);
+    linear_forward(form({a.O}), ff, fp32, tok({out}, ff.out()), nullptr, T, st);
+  }
+  if (need) {
+    auto node = std::shared_ptr<LayerNode>(new LayerNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, W[0], b[0], W[1], b[1], W[2], b[2], W[3], b[3]));
+    node->c = c; node->fp32 = fp32; node->a = a; node->out_type = out.scalar_type();
+    if (c->mode == NATIVE && c->fused && c->recompute) node->a.P = Tensor();
+    node->x = save(x);
+    for (int i = 0; i < 4; ++i) node->w[i] = save(W[i]);
+    torch::autograd::set_history(out, node);
+  }
+  return py::make_tuple(out, a.P.defined() ? py::cast(a.P) : py::none(), a.lse.defined() ? py::cast(a.lse) : py::none(),
+                        a.pen.defined() ? py::cast(a.pen) : py::none(), a.q, a.k, a.heads);
+}
+
+// ------------------------------------------------------------------------------------------------ linear layers on their own
+struct LinearNode : public Node {
+  bool fp32 = false;
+  SavedVariable x, w;
+  at::ScalarType out_type;
+  std::string name() const override { return "TokenLinearBackward"; }
+  void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); x.reset_data(); w.reset_data(); }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    Tensor X = x.unpack();
+    Weights l; l.W.push_back(w.unpack());
+    c10::cuda::CUDAGuard guard(X.device());
+    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    Tensor go = grads[0].to(out_type).contiguous();
+    if (!aligned32(go)) go = go.clone();
+    void* st = stream_of(X);
+    const int64_t T = X.numel() / l.in();
+    const spion_tokens tg = tok({go}, l.out());
+    if (task_should_compute_output(1) || task_should_compute_output(2)) {
+      std::vector<Tensor> dW, db;
+      linear_backward_weight({go}, tg, X, tok({X}, l.in()), l, fp32, T, st, dW, db);
+      out[1] = dW[0]; out[2] = db[0];
+    }
+    if (task_should_compute_output(0)) {
+      out[0] = at::empty(X.sizes(), X.options());
+      linear_backward_input(tg, l, fp32, nullptr, tok({out[0]}, l.in()), T, st);
+    }
+    return out;
+  }
+};
+
+bool linear_supported(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
+  if (!x.is_cuda() || x.numel() == 0 || x.dim() < 2 || x.size(-1) != W.size(1)) return false;
+  if (x.scalar_type() != at::kFloat && (fp32 || x.scalar_type() != at::kBFloat16)) return false;
+  return x.numel() / W.size(1) < 0x7fffff00LL && weights_ok({W}, {b}, x, fp32);
+}
+
+Tensor linear(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    Tensor X = x.detach();
+    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    Weights l{{W.detach()}, {b.detach()}};
+    auto sizes = x.sizes().vec();
+    sizes.back() = l.out();
+    out = at::empty(sizes, X.options().dtype(fp32 ? at::kFloat : at::kBFloat16));
+    linear_forward(tok({X}, l.in()), l, fp32, tok({out}, l.out()), nullptr, X.numel() / l.in(), stream_of(X));
+  }
+  if (at::GradMode::is_enabled() && (x.requires_grad() || W.requires_grad() || b.requires_grad())) {
+    auto node = std::shared_ptr<LinearNode>(new LinearNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, W, b));
+    node->fp32 = fp32; node->x = save(x); node->w = save(W); node->out_type = out.scalar_type();
+    torch::autograd::set_history(out, node);
+  }
+  return out;
+}
+
+// Feed-forward block Linear -> GELU -> Linear under mixed precision, the activation inside the first product's kernel.
+struct MlpNode : public Node {
+  SavedVariable x, w1, w2;
+  Tensor h, g;                           // pre-activation and activation, bf16
+  bool released = false;
+  std::string name() const override { return "FeedForwardBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    x.reset_data(); w1.reset_data(); w2.reset_data();
+    h = Tensor(); g = Tensor();
+    released = true;
+  }
+  // inputs: x, W1, b1, W2, b2
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    TORCH_CHECK(!released, "Trying to backward through the graph a second time (the saved tensors have been freed)");
+    variable_list out(5);
+    if (!grads[0].defined()) return out;
+    Tensor X = x.unpack();
+    c10::cuda::CUDAGuard guard(X.device());
+    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    Weights l1, l2;
+    l1.W.push_back(w1.unpack()); l2.W.push_back(w2.unpack());
+    Tensor go = grads[0].to(at::kBFloat16).contiguous();
+    if (!aligned32(go)) go = go.clone();
+    void* st = stream_of(X);
+    const int64_t T = X.numel() / l1.in();
+    std::vector<Tensor> dW, db;
+    const spion_tokens tg = tok({go}, l2.out());
+    linear_backward_weight({go}, tg, g, tok({g}, l2.in()), l2, false, T, st, dW, db);
+    Tensor dh = at::empty(h.sizes(), h.options());
+    linear_backward_input(tg, l2, false, p(h), tok({dh}, l2.in()), T, st);
+    const spion_tokens th = tok({dh}, l1.out());
+    linear_backward_weight({dh}, th, X, tok({X}, l1.in()), l1, false, T, st, dW, db);
+    if (task_should_compute_output(0)) {
+      out[0] = at::empty(X.sizes(), X.options());
+      linear_backward_input(th, l1, false, nullptr, tok({out[0]}, l1.in()), T, st);
+    }
+    out[1] = dW[1]; out[2] = db[1]; out[3] = dW[0]; out[4] = db[0];
+    return out;
+  }
+};
+
+Tensor mlp(const Tensor& x, const Tensor& W1, const Tensor& b1, const Tensor& W2, const Tensor& b2) {
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out, h, g;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    Tensor X = x.detach();
+    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    Weights l1{{W1.detach()}, {b1.detach()}}, l2{{W2.detach()}, {b2.detach()}};
+    const int64_t T = X.numel() / l1.in();
+    const auto opt = X.options().dtype(at::kBFloat16);
+    h = at::empty({T, l1.out()}, opt);
+    g = at::empty({T, l1.out()}, opt);
+    void* st = stream_of(X);
+    linear_forward(tok({X}, l1.in()), l1, false, tok({h}, l1.out()), g.data_ptr(), T, st);
+    auto sizes = x.sizes().vec();
+    sizes.back() = l2.out();
+    out = at::empty(sizes, opt);
+    linear_forward(tok({g}, l2.in()), l2, false, tok({out}, l2.out()), nullptr, T, st);
+  }
+  if (at::GradMode::is_enabled() &&
+      (x.requires_grad() || W1.requires_grad() || b1.requires_grad() || W2.requires_grad() || b2.requires_grad())) {
+    auto node = std::shared_ptr<MlpNode>(new MlpNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, W1, b1, W2, b2));
+    node->x = save(x); node->w1 = save(W1); node->w2 = save(W2);
+    node->h = h; node->g = g;
+    torch::autograd::set_history(out, node);
+  }
+  return out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  static py::object error = py::module_::import("spion_b200._lib").attr("SpionError");
+  py::register_local_exception_translator([](std::exception_ptr e) {
+    try {
+      if (e) std::rethrow_exception(e);
+    } catch (const Failure& f) {
+      PyErr_SetString(error.ptr(), f.what());
+    }
+  });
+  py::class_<Context, ContextPtr>(m, "Context")
+      .def(py::init<>())
+      .def("close", &Context::close)
+      .def_readwrite("handle", &Context::handle)
+      .def_readwrite("mode", &Context::mode)
+      .def_readwrite("B", &Context::B).def_readwrite("H", &Context::H).def_readwrite("L", &Context::L).def_readwrite("d", &Context::d)
+      .def_readwrite("device", &Context::device)
+      .def_readwrite("bf16", &Context::bf16).def_readwrite("keypad", &Context::keypad).def_readwrite("fused", &Context::fused)
+      .def_readwrite("recompute", &Context::recompute).def_readwrite("return_probs", &Context::return_probs)
+      .def_readwrite("needs_scratch", &Context::needs_scratch).def_readwrite("owned", &Context::owned)
+      .def_readwrite("nnz", &Context::nnz)
+      .def_readwrite("sum_mat", &Context::sum_mat).def_readwrite("offsets", &Context::offsets).def_readwrite("columns", &Context::columns);
+  m.def("attention", &attention);
+  m.def("layer_supported", &layer_supported);
+  m.def("attention_layer", &attention_layer);
+  m.def("linear_supported", &linear_supported);
+  m.def("linear", &linear);
+  m.def("mlp", &mlp);
+}

@@ -82,6 +82,7 @@ class TransformerLayer(nn.Module):
         Linear = nn.Linear
         if config.get("native") and config.get("fused_bias_grad", True):
             from .layernorm import BiasGradLinear as Linear
+        self.fuse_mlp = Linear is not nn.Linear
         self.mlpblock = nn.Sequential(Linear(dim, hid), nn.GELU(), nn.Dropout(p), Linear(hid, dim), nn.Dropout(p))
 
     def forward(self, X, mask, mat=None):
@@ -89,13 +90,24 @@ class TransformerLayer(nn.Module):
         X = self.dropout1(out) + X
         return self.mlpblock(self.norm2(X)) + X, attn
 
+    def feed_forward(self, n2):
+        """The feed-forward block; under mixed precision and without active dropout its two products run with the activation
+        between them inside the kernels."""
+        lin1, drop, lin2 = self.mlpblock[0], self.mlpblock[2], self.mlpblock[3]
+        if self.fuse_mlp and torch.is_autocast_enabled() and torch.get_autocast_dtype("cuda") == torch.bfloat16 \
+                and (not self.training or drop.p == 0):
+            from ._ops import ops
+            if ops.linear_supported(n2, lin1.weight, lin1.bias, False) and lin2.in_features % 32 == 0 and lin2.out_features % 32 == 0:
+                return ops.mlp(n2, lin1.weight, lin1.bias, lin2.weight, lin2.bias)
+        return self.mlpblock(n2)
+
     def forward_add_norm(self, X, Xn, mask, mat, next_norm):
         """The same layer with each residual addition done inside the normalisation that follows it
         (FusedLayerNorm.add_norm): ``Xn`` is ``self.norm1(X)``, already formed by the previous stage; returns the
         layer's output together with ``next_norm`` of it (the next layer's norm1, or the encoder's final norm)."""
         out, attn = self.mha(Xn, mask, mat)
         X, n2 = self.norm2.add_norm(X, self.dropout1(out))
-        X, nn_ = next_norm.add_norm(X, self.mlpblock(n2))
+        X, nn_ = next_norm.add_norm(X, self.feed_forward(n2))
         return X, nn_, attn
 
 

@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from . import _lib
+from . import _lib, _ops
 from ._lib import check, lib, ptr
 
 SUPPORTED_WIDTHS = (64, 128, 256, 512)
@@ -197,12 +197,17 @@ class _LinearFn(torch.autograd.Function):
 
 
 class BiasGradLinear(nn.Linear):
-    """``nn.Linear`` (same parameters, same forward arithmetic) whose backward sums the bias gradient with the
-    library's column-sum kernel when the output width is one it serves."""
+    """``nn.Linear`` (same parameters, same arithmetic) on the library's linear-layer kernels: conversion of the operands, bias and
+    bias gradient happen inside them.  Widths they do not serve (not a multiple of 32) go through the framework's GEMMs, with
+    the bias gradient summed by the library's column-sum kernel."""
 
     def forward(self, x):
         if self.bias is None or not x.is_cuda:
             return super().forward(x)
+        amp = torch.is_autocast_enabled()
+        if not amp or torch.get_autocast_dtype("cuda") == torch.bfloat16:
+            if _ops.ops.linear_supported(x, self.weight, self.bias, not amp):
+                return _ops.ops.linear(x, self.weight, self.bias, not amp)
         return _LinearFn.apply(x, self.weight, self.bias)
 
 

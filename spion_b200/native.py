@@ -19,7 +19,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, _ops
 from ._lib import check, lib, ptr
 
 _DTYPES = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16}
@@ -52,12 +52,16 @@ class BlockSparseAttention(nn.Module):
         if not h:
             raise _lib.SpionError("spion_create failed (unsupported shape, or no CUDA device)")
         self.handle = _lib.c_void_p(h)
+        # what the native host path knows of this module; it owns the handle (a backward can outlive the module)
+        self._ctx = _ops.make_context(h, _ops.NATIVE, self.B, self.H, self.L, self.d, self.device.index or 0,
+                                      dtype == torch.bfloat16, keypad)
+        self._ctx.owned = True
         check(lib.spion_set_engine(self.handle, engine), "spion_set_engine")
         self.engine = engine
         # 32-wide masks, bf16, head_dim 64, calls without stored probabilities: kernels on the mask's own blocks
         # ("own"), on 64-wide super-blocks ("super"), or chosen per mask by how full the gathered operands are
         check(lib.spion_set_block32_path(self.handle, {"auto": 0, "own": 1, "super": 2}[block32]), "spion_set_block32_path")
-        self.needs_scratch = bool(lib.spion_needs_scratch(self.handle))
+        self._ctx.needs_scratch = self.needs_scratch = bool(lib.spion_needs_scratch(self.handle))
         # fused kernels (S, P, dP, dS stay on chip) where the tensor-core engine covers the shape
         can_fuse = bool(lib.spion_supports_fused(self.handle))
         if fused and not can_fuse:
@@ -77,13 +81,32 @@ class BlockSparseAttention(nn.Module):
         self.nnzb = -1
         self._mask_key = None
         self._mask_ref = None
-        self._fn = _make_function(self)
+        self._mask_version = -1
 
-    def __del__(self):
-        h = getattr(self, "handle", None)
-        if h:
-            lib.spion_destroy(h)
-            self.handle = None
+    # settings the native host path reads: kept in its context
+    @property
+    def fused(self):
+        return self._ctx.fused
+
+    @fused.setter
+    def fused(self, v):
+        self._ctx.fused = bool(v)
+
+    @property
+    def recompute(self):
+        return self._ctx.recompute
+
+    @recompute.setter
+    def recompute(self, v):
+        self._ctx.recompute = bool(v)
+
+    @property
+    def return_probs(self):
+        return self._ctx.return_probs
+
+    @return_probs.setter
+    def return_probs(self, v):
+        self._ctx.return_probs = bool(v)
 
     # ------------------------------------------------------------------ pattern
     def set_mask(self, mat: torch.Tensor) -> int:
@@ -101,7 +124,8 @@ class BlockSparseAttention(nn.Module):
         # The key names the tensor by address and version; the tensor itself is kept alive so that the
         # address cannot be handed to another mask while the key is in use.
         self._mask_key = (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device))
-        self._mask_ref = mat
+        self._mask_ref, self._mask_version = mat, mat._version
+        self._ctx.nnz = self.nnz
         return self.nnzb
 
     @property
@@ -150,19 +174,13 @@ class BlockSparseAttention(nn.Module):
         return torch.cat(out, dim=1)
 
     # ------------------------------------------------------------------ call
-    def _check_operands(self, query, key, value, mask):
-        """The kernels take sizes from the context, not from the tensors: refuse anything else loudly
-        (a short last batch would otherwise read and write past the buffers)."""
-        want = (self.B, self.H, self.L, self.d)
-        for name, t in (("query", query), ("key", key), ("value", value)):
-            if tuple(t.shape) != want:
-                raise _lib.SpionError(f"{name} has shape {tuple(t.shape)}, this module was built for {want} "
-                                      "(batch_size, num_head, max_seq_len, head_dim of its config)")
-            if t.device != self.device:
-                raise _lib.SpionError(f"{name} is on {t.device}, the module's context is on {self.device}")
-        if self.keypad:
-            if mask is None or tuple(mask.shape) != (self.B, self.L):
-                raise _lib.SpionError(f"key-padding mask must have shape {(self.B, self.L)}")
+    def use_mask(self, mat) -> None:
+        """Make ``mat`` the current mask unless it already is (None: keep the current one)."""
+        if mat is not None and not (mat is self._mask_ref and mat._version == self._mask_version):
+            if (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device)) != self._mask_key:
+                self.set_mask(mat)
+        if self.nnzb < 0:
+            raise _lib.SpionError("no block mask set (call set_mask or pass mat)")
 
     def operand_form(self, t) -> int:
         """0: contiguous [B, H, L, d]; H: the head-split view of a contiguous [B, L, H, d] tensor; -1: neither."""
@@ -178,19 +196,19 @@ class BlockSparseAttention(nn.Module):
             return torch.empty(self.B, self.L, self.H, self.d, dtype=self.dtype, device=device).transpose(1, 2)
         return torch.empty(self.B, self.H, self.L, self.d, dtype=self.dtype, device=device)
 
-    def forward(self, query, key, value, mask=None, mat=None):
-        if mat is not None and (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device)) != self._mask_key:
-            self.set_mask(mat)
-        if self.nnzb < 0:
-            raise _lib.SpionError("no block mask set (call set_mask or pass mat)")
-        self._check_operands(query, key, value, mask)
-        pen = None
-        if self.keypad:
-            pen = (1e6 * (1 - mask.to(torch.float32)))[:, None, :].expand(self.B, self.H, self.L).contiguous()
-        out, P = self._fn.apply(query, key, value, pen)
+    def result(self, out, probs, lse, pen, q, k, heads):
+        """What a forward returns beside its output: the tiles, or a handle from which they can be rebuilt."""
+        if lse is not None:
+            self.last = ProbsHandle(q, k, lse, pen, heads)
         if not self.return_probs:
             return out, self.last
-        return out, P
+        return out, probs
+
+    def forward(self, query, key, value, mask=None, mat=None):
+        # The kernels take sizes from the context, not from the tensors: the call refuses any other shape, device or key-padding
+        # mask with a SpionError (a short last batch would otherwise read and write past the buffers).
+        self.use_mask(mat)
+        return self.result(*_ops.ops.attention(self._ctx, query, key, value, mask if self.keypad else None))
 
 
 class DenseViaBlocks(nn.Module):
@@ -211,98 +229,3 @@ class DenseViaBlocks(nn.Module):
 
     def mean_attention_map(self, P_tiles):
         return self.block.mean_attention_map(P_tiles)
-
-
-def _make_function(mod: BlockSparseAttention):
-    class FusedBlockAttnFunction(torch.autograd.Function):
-        @staticmethod
-        def forward(ctx, query, key, value, pen):
-            q, k, v = query.to(mod.dtype), key.to(mod.dtype), value.to(mod.dtype)
-            # head-split views of [B, L, H*d] projections are read where they lie; anything else is packed
-            heads = mod.H if all(mod.operand_form(t) == mod.H for t in (q, k, v)) else 0
-            if not heads:
-                q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-            dev = q.device
-            O = mod.empty_operand(heads, dev)
-            lse = torch.empty(mod.BH * mod.L, dtype=torch.float32, device=dev)
-            # the probabilities are stored only for callers that want them back; the backward rebuilds its tiles
-            want_p = mod.return_probs or not mod.recompute
-            P = torch.empty(mod.BH * mod.nnz, dtype=mod.dtype, device=dev) if want_p else None
-            check(lib.spion_set_stream(mod.handle, _lib.current_stream_ptr()))
-            check(lib.spion_set_head_layout(mod.handle, heads), "spion_set_head_layout")
-            check(lib.spion_attn_forward_fused(mod.handle, ptr(q), ptr(k), ptr(v), ptr(pen), ptr(O), ptr(lse), ptr(P)),
-                  "spion_attn_forward_fused")
-            ctx.save_for_backward(q, k, v, O, lse)
-            ctx.pen = pen
-            ctx.heads = heads
-            ctx.P = None if mod.recompute else P
-            mod.last = ProbsHandle(q.detach(), k.detach(), lse, pen, heads)
-            if P is None:
-                P = torch.empty(0, dtype=mod.dtype, device=dev)
-            ctx.mark_non_differentiable(P)
-            # without this the engine hands the backward a zero-filled gradient of the size of the probabilities
-            ctx.set_materialize_grads(False)
-            return O, P
-
-        @staticmethod
-        def backward(ctx, grad_output, grad_p):
-            q, k, v, O, lse = ctx.saved_tensors
-            dev = q.device
-            heads = ctx.heads
-            go = grad_output.to(mod.dtype)
-            if heads and mod.operand_form(go) != heads:
-                go = go.transpose(1, 2).contiguous().transpose(1, 2)
-            elif not heads:
-                go = go.contiguous()
-            dq, dk, dv = (mod.empty_operand(heads, dev) for _ in range(3))
-            check(lib.spion_set_stream(mod.handle, _lib.current_stream_ptr()))
-            check(lib.spion_set_head_layout(mod.handle, heads), "spion_set_head_layout")
-            if ctx.P is None:
-                check(lib.spion_attn_backward_fused(mod.handle, ptr(q), ptr(k), ptr(v), ptr(O), ptr(go), ptr(lse),
-                                                    ptr(ctx.pen), ptr(dq), ptr(dk), ptr(dv)), "spion_attn_backward_fused")
-            else:
-                dS = torch.empty(mod.BH * mod.nnz, dtype=mod.dtype, device=dev)
-                check(lib.spion_attn_backward_ex(mod.handle, ptr(q), ptr(k), ptr(v), ptr(ctx.P), ptr(O), ptr(go), ptr(dS),
-                                                 None, None, ptr(dq), ptr(dk), ptr(dv)), "spion_attn_backward_ex")
-            return dq, dk, dv, None
-
-    if mod.fused:
-        return FusedBlockAttnFunction
-
-    class NativeBlockAttnFunction(torch.autograd.Function):
-        @staticmethod
-        def forward(ctx, query, key, value, pen):
-            q = query.to(mod.dtype).contiguous()
-            k = key.to(mod.dtype).contiguous()
-            v = value.to(mod.dtype).contiguous()
-            dev = q.device
-            n = mod.BH * mod.nnz
-            P = torch.empty(n, dtype=mod.dtype, device=dev)
-            O = torch.empty_like(q)
-            scratch = torch.empty(n, dtype=torch.float32, device=dev) if mod.needs_scratch else None
-            check(lib.spion_set_stream(mod.handle, _lib.current_stream_ptr()))
-            check(lib.spion_set_head_layout(mod.handle, 0), "spion_set_head_layout")
-            check(lib.spion_attn_forward_ex(mod.handle, ptr(q), ptr(k), ptr(v), ptr(pen), ptr(P), ptr(O), ptr(scratch)),
-                  "spion_attn_forward_ex")
-            ctx.save_for_backward(q, k, v, P, O)
-            ctx.mark_non_differentiable(P)
-            # without this the engine hands the backward a zero-filled gradient of the size of the probabilities
-            ctx.set_materialize_grads(False)
-            return O, P
-
-        @staticmethod
-        def backward(ctx, grad_output, grad_p):
-            q, k, v, P, O = ctx.saved_tensors
-            dev = q.device
-            go = grad_output.to(mod.dtype).contiguous()
-            n = mod.BH * mod.nnz
-            dS = torch.empty(n, dtype=mod.dtype, device=dev)
-            scratch = torch.empty(n, dtype=torch.float32, device=dev) if mod.needs_scratch else None
-            dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
-            check(lib.spion_set_stream(mod.handle, _lib.current_stream_ptr()))
-            check(lib.spion_attn_backward_ex(mod.handle, ptr(q), ptr(k), ptr(v), ptr(P), ptr(O), ptr(go), ptr(dS),
-                                             ptr(scratch), None, ptr(dq), ptr(dk), ptr(dv)),
-                  "spion_attn_backward_ex")
-            return dq, dk, dv, None
-
-    return NativeBlockAttnFunction

@@ -1,0 +1,122 @@
+"""GPU tests of the linear-layer kernels (csrc/linear.cu) and of the one-node attention layer, against fp64 products."""
+import ctypes
+
+import pytest
+import torch
+
+from spion_b200 import _lib
+from spion_b200._lib import Tokens, check, lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _tokens(ts, heads=0, d=0, L=0):
+    t = Tokens()
+    t.count, t.is_bf16, t.heads, t.head_dim, t.seq_len = len(ts), int(ts[0].dtype == torch.bfloat16), heads, d, L
+    for i, x in enumerate(ts):
+        t.ptr[i] = x.data_ptr()
+    t.cols = heads * d if heads else ts[0].shape[-1]
+    return t
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+# tokens per sequence around the 64 / 128-token tiles; widths with a partial 64-feature chunk (32, 96), one and three stacked
+# matrices, contractions of several chunks and (fp32, 384) one that takes several launches
+@pytest.mark.parametrize("B,L,H,d,K,nw", [(1, 1, 1, 32, 32, 1), (1, 129, 2, 32, 64, 3), (3, 63, 3, 32, 96, 3), (2, 191, 4, 32, 128, 3),
+                                          (1, 20000, 2, 32, 64, 1), (2, 100, 3, 64, 192, 1), (1, 300, 4, 64, 256, 3)])
+@pytest.mark.parametrize("mode", ["bf16", "bf16_x", "fp32"])
+@pytest.mark.parametrize("split", [False, True])
+def test_linear_kernels(B, L, H, d, K, nw, mode, split):
+    fp32 = int(mode == "fp32")
+    N1, T = H * d, B * L
+    N = nw * N1
+    if not lib.spion_linear_supported(K, N, fp32) or (mode == "bf16_x" and nw == 3 and N1 % 64):
+        pytest.skip("width not served")
+    g = torch.Generator(device="cuda").manual_seed(T + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    P = ctypes.c_void_p
+    st = P(torch.cuda.current_stream().cuda_stream)
+    yt = torch.float32 if fp32 else torch.bfloat16
+    X = rnd(T, K).to(torch.bfloat16 if mode == "bf16_x" else torch.float32)
+    Ws, bs = [rnd(N1, K) for _ in range(nw)], [rnd(N1) for _ in range(nw)]
+    ptrs = lambda ts: (P * 3)(*([t.data_ptr() for t in ts] + [None] * (3 - len(ts))))
+    shape, lay = ((B, H, L, d), (H, d, L)) if split else ((T, N1), (0, 0, 0))
+    cat = lambda ts: torch.cat([(t.permute(0, 2, 1, 3).reshape(T, N1) if split else t) for t in ts], 1).double()
+    Ys = [torch.full(shape, 7.0, dtype=yt, device="cuda") for _ in range(nw)]
+    dYs = [rnd(*shape).to(yt) for _ in range(nw)]
+    dX = torch.full((T, K), 7.0, dtype=X.dtype, device="cuda")
+    dW, db = torch.full((N, K), 7.0, device="cuda"), torch.full((N,), 7.0, device="cuda")
+    ws = torch.empty(lib.spion_linear_workspace_floats(T, K, N, fp32), device="cuda")
+    tx, ty, td, tdx = _tokens([X]), _tokens(Ys, *lay), _tokens(dYs, *lay), _tokens([dX])
+    ref = ctypes.byref
+    check(lib.spion_linear_forward(ref(tx), ptrs(Ws), ptrs(bs), nw, fp32, ref(ty), None, T, K, N, st))
+    check(lib.spion_linear_backward_input(ref(td), ptrs(Ws), nw, fp32, None, ref(tdx), T, K, N, st))
+    check(lib.spion_linear_backward_weight(ref(td), ref(tx), fp32, P(dW.data_ptr()), P(db.data_ptr()), P(ws.data_ptr()), T, K, N, st))
+    torch.cuda.synchronize()
+    assert lib.spion_linear_status(1) == 0
+    W, b, dY = torch.cat(Ws).double(), torch.cat(bs).double(), cat(dYs)
+    # bf16: operands and result carry a relative error of 2^-9 each (uniformly distributed rounding: 2^-9 / sqrt(3) rms per
+    # factor).  fp32: rounding of the result plus the fp32 additions of the contraction, a few 2^-24.
+    tol = 5e-7 if fp32 else 5e-3
+    assert _rel(cat(Ys), X.double() @ W.t() + b) < tol
+    assert _rel(dX, dY @ W) < tol
+    assert _rel(dW, dY.t() @ X.double()) < (2e-6 if fp32 else tol)
+    assert _rel(db, dY.sum(0)) < 2e-6
+
+
+@pytest.mark.parametrize("native,dtype,bs,L,dense", [(True, "bf16", 64, 192, False), (True, "bf16", 64, 128, True),
+                                                     (True, "fp32", 32, 160, False), (False, "fp32", 32, 96, False)])
+def test_attention_layer_in_one_node_equals_its_stages(native, dtype, bs, L, dense):
+    """The same layer with a forward hook on one projection runs stage by stage: same results, same gradients."""
+    from contextlib import nullcontext
+
+    from spion_b200.attention import Attention
+    B, H, d = 3, 2, 32
+    cfg = {"head_dim": d, "num_head": H, "max_seq_len": L, "batch_size": B, "block_size": bs, "transformer_dim": H * d,
+           "task": "lra-text", "native": native, "dtype": dtype}
+    torch.manual_seed(1)
+    layer = Attention(cfg).cuda()
+    mat = None
+    if not dense:
+        layer.reconstruct_for_blocksparse(cfg)
+        mat = (torch.rand(L // bs, L // bs, device="cuda") < 0.5).float()
+        mat.fill_diagonal_(1)
+    x = torch.randn(B, L, H * d, device="cuda", requires_grad=True)
+    mask = torch.ones(B, L, device="cuda")
+    mask[1, L // 2:] = 0
+    amp = torch.autocast("cuda", dtype=torch.bfloat16) if dtype == "bf16" else nullcontext()
+    outs = []
+    for hooked in (False, True):                              # (the drop-in dense phase always runs stage by stage)
+        h = layer.W_k.register_forward_hook(lambda m, i, o: None) if hooked else None
+        with amp:
+            out, _ = layer(x, mask, mat)
+        g = torch.autograd.grad(out, [x] + list(layer.parameters()), torch.ones_like(out))
+        outs.append([out, *g])
+        if h:
+            h.remove()
+    # bf16: the stages round dX of each projection to bf16 and add; the node adds first (two roundings of 2^-9 apart)
+    tol = 2e-2 if dtype == "bf16" else 1e-5
+    for a, b in zip(*outs):
+        assert a.shape == b.shape and a.dtype == b.dtype
+        err = float((a.double() - b.double()).norm())
+        assert err <= tol * float(b.double().norm()) + 1e-6, (err, float(b.double().norm()))
+
+
+def test_feed_forward_block():
+    """Linear -> GELU -> Linear with the activation inside the kernels, against the framework's operators in bf16."""
+    from spion_b200._ops import ops
+    torch.manual_seed(0)
+    l1, l2 = torch.nn.Linear(64, 128).cuda(), torch.nn.Linear(128, 64).cuda()
+    x = torch.randn(2, 77, 64, device="cuda").bfloat16().requires_grad_(True)
+    go = torch.randn(2, 77, 64, device="cuda").bfloat16()
+    ps = [x, l1.weight, l1.bias, l2.weight, l2.bias]
+    y = ops.mlp(x, l1.weight, l1.bias, l2.weight, l2.bias)
+    got = [y, *torch.autograd.grad(y, ps, go)]
+    pd = [t.detach().double().requires_grad_(True) for t in ps]
+    yd = torch.nn.functional.linear(torch.nn.functional.gelu(torch.nn.functional.linear(pd[0], pd[1], pd[2])), pd[3], pd[4])
+    want = [yd, *torch.autograd.grad(yd, pd, go.double())]
+    for a, b in zip(got, want):
+        assert _rel(a.detach(), b.detach()) < 1.5e-2          # a chain of up to four roundings to bf16
