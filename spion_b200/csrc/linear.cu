@@ -115,11 +115,7 @@ template <> struct Prod<3> {
 
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
-  const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
-  if (!ok && (threadIdx.x & 31) == 0) atomicOr(&g_lin_status, ERR_MMA_WAIT);
-  return ok;
-}
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) { return tc::warp_wait(bar, parity, &g_lin_status, ERR_MMA_WAIT); }
 
 // ------------------------------------------------------------------------------------------------ GEMM over tokens
 enum { EPI_NONE = 0, EPI_GELU = 1, EPI_DGELU = 2 };

@@ -211,7 +211,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
   const uint32_t bars = smem_u32(s_bars);
   auto bar = [&](int which, int i) -> uint32_t { return bars + (which + i) * 8; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int total = nlines * BH;
   const float sc2 = scale * LOG2E;
 
@@ -289,7 +289,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
     }
   } else if (warp == 5) {
     // =================================================================== first products (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_1 = make_idesc_bf16(128, B32, 0, 0);      // [128 x 64] . [32 x 64]^T
       Cursor<MODE> cm;
       cm.init(recs, total, BH);
@@ -328,7 +328,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
     __syncwarp();                     // the idle lanes wait here for the issuing lane: the CTA barrier below is warp-aligned
   } else if (warp == 6) {
     // =================================================================== second products (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_2 = make_idesc_bf16(64, B32, 1, 1);       // [128 x 64]^T . [128 x 32]
       Cursor<MODE> co;
       co.init(recs, total, BH);

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_bwd_row(const __grid_constan
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - raw));
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, q = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, q = warp_uniform(tid >> 5), lane = tid & 31;
   const int hf = lane >> 4;
   const int row = q * 16 + (lane & 15);
   const int total = nrows * BH;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_bwd_row(const __grid_constan
   const uint32_t t_lane = tmem + ((uint32_t)(q * 32) << 16);
   constexpr uint32_t IDESC_P = make_idesc_bf16(64, 64, 0, 0);
   constexpr uint32_t IDESC_Q = make_idesc_bf16(64, D, 0, 1);
-  // parities run on across units.  pv, pk: one bit per half, thread 0 only; pp (one bit per half), ps, po: every thread
+  // parities run on across units.  pv, pk: one bit per half, warp 0 only; pp (one bit per half), ps, po: every thread
   uint32_t pv = 0, pk = 0, pp = 0, ps = 0, po = 0;
   bool ok = true;
 
@@ -147,21 +147,26 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_bwd_row(const __grid_constan
     const bool single = R.single();
     const OpPos pos = op_pos(bh, L, heads, D);
 
-    // tid 0: dP MMAs of chunk ch (its dO / V tiles were requested earlier), pair p of the chunk in columns col0 + 64 p
+    // warp 0: dP MMAs of chunk ch (its dO / V tiles were requested earlier), pair p of the chunk in columns col0 + 64 p
     auto issue_dp = [&](int ch, uint32_t col0) -> bool {
       const int CH = single ? NCH : 2;
       const int t0 = ch * CH, nt = min(CH, nblk - t0);
       const int hb = single ? 0 : (ch & 1), b0 = 2 * hb;
-      if (!mbar_wait(bar_v + 8 * hb, (pv >> hb) & 1)) { report(status, ERR_LOAD_WAIT); return false; }
+      if (!warp_wait(bar_v + 8 * hb, (pv >> hb) & 1, status, ERR_LOAD_WAIT)) return false;
       pv ^= 1u << hb;
-      tc_fence_after();
-      for (int t = 0; t < nt; ++t) {
-        const uint32_t d_addr = tmem + ((uint32_t)((t & 1) * 16) << 16) + col0 + (uint32_t)(t >> 1) * 64u;
+      if (elect_one()) {
+        tc_fence_after();
+        const uint64_t da = T::kmajor(sA, 0);
+        uint64_t db = T::kmajor(sB + b0 * T::BYTES, 0);
+        for (int t = 0; t < nt; ++t, db = desc_advance(db, T::BYTES)) {
+          const uint32_t d_addr = tmem + ((uint32_t)((t & 1) * 16) << 16) + col0 + (uint32_t)(t >> 1) * 64u;
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          mma_bf16(d_addr, T::kmajor(sA, kk), T::kmajor(sB + (b0 + t) * T::BYTES, kk), IDESC_P, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk)
+            mma_bf16(d_addr, desc_advance(da, kk * T::K_STEP), desc_advance(db, kk * T::K_STEP), IDESC_P, kk > 0);
+        }
+        mma_commit(bar_s);
       }
-      mma_commit(bar_s);
+      __syncwarp();
       return true;
     };
     // warp 0, all lanes: the dP MMAs have consumed the V tiles of this chunk: bring K into the same buffers
@@ -201,27 +206,34 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_bwd_row(const __grid_constan
         }
       }
     };
-    // tid 0: store the dS tiles of a chunk and issue dQ += dS K (every tile into the one accumulator at lane offset 0)
-    auto issue_dq = [&](int hb, int t0, int nt, bool first_chunk) -> bool {
+    // warp 0: store the dS tiles of a chunk and issue dQ += dS K (every tile into the one accumulator at lane offset 0)
+    auto issue_dq = [&](int hb, int t0, int nt, bool first_chunk, bool last) -> bool {
       const int b0 = 2 * hb;
-      for (int t = 0; t < nt; ++t)
-        tma_store_2d(&tmdS, sP + (b0 + t) * VT_BYTES, 0, (int)(((size_t)bh * nnzb + rp + t0 + t) * BS));
-      bulk_commit();
-      if (!mbar_wait(bar_k + 8 * hb, (pk >> hb) & 1)) { report(status, ERR_LOAD_WAIT); return false; }
-      pk ^= 1u << hb;
-      tc_fence_after();
-      for (int t = 0; t < nt; ++t) {
-        const uint32_t first = (first_chunk && t == 0) ? 0u : 1u;
-#pragma unroll
-        for (int kk = 0; kk < BS / 16; ++kk)
-          mma_bf16(tmem, ValTile::kmajor(sP + (b0 + t) * VT_BYTES, kk), T::mnmajor(sB + (b0 + t) * T::BYTES, kk), IDESC_Q,
-                   (kk > 0) ? 1u : first);
+      if (lane == 0) {
+        for (int t = 0; t < nt; ++t)
+          tma_store_2d(&tmdS, sP + (b0 + t) * VT_BYTES, 0, (int)(((size_t)bh * nnzb + rp + t0 + t) * BS));
+        bulk_commit();
       }
+      __syncwarp();
+      if (!warp_wait(bar_k + 8 * hb, (pk >> hb) & 1, status, ERR_LOAD_WAIT)) return false;
+      pk ^= 1u << hb;
+      if (elect_one()) {
+        tc_fence_after();
+        uint64_t da = ValTile::kmajor(sP + b0 * VT_BYTES, 0), db = T::mnmajor(sB + b0 * T::BYTES, 0);
+        for (int t = 0; t < nt; ++t, da = desc_advance(da, VT_BYTES), db = desc_advance(db, T::BYTES)) {
+          const uint32_t first = (first_chunk && t == 0) ? 0u : 1u;
+#pragma unroll
+          for (int kk = 0; kk < BS / 16; ++kk)
+            mma_bf16(tmem, desc_advance(da, kk * ValTile::K_STEP), desc_advance(db, kk * T::MN_STEP), IDESC_Q, (kk > 0) ? 1u : first);
+        }
+        if (last) mma_commit(bar_o);
+      }
+      __syncwarp();
       return true;
     };
 
     if (nblk > 0) {
-      if (tid == 0) issue_dp(0, single ? 0u : 64u);
+      if (q == 0) issue_dp(0, single ? 0u : 64u);
       // delta_i = sum_n dO_in O_in: the two owners of a row take one half of the head dimension each
       float delta;
       {
@@ -261,10 +273,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_bwd_row(const __grid_constan
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
-        if (tid == 0 && issue_dq(hb, t0, nt, c == 0)) {
-          if (c + 1 < n) issue_dp(c + 1, 64u);
-          else mma_commit(bar_o);
-        }
+        if (q == 0 && issue_dq(hb, t0, nt, c == 0, c + 1 == n) && c + 1 < n) issue_dp(c + 1, 64u);
       }
       if (ok) {
         if (!__syncthreads_and(mbar_wait(bar_o, po))) { if (tid == 0) report(status, ERR_MMA2_WAIT); ok = false; }
@@ -350,7 +359,7 @@ __global__ void __launch_bounds__(COL_THREADS) k_bwd_col(const __grid_constant__
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - raw));
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int total = nb * BH, G = (int)gridDim.x;
   constexpr uint32_t TMEM_COLS = 128u;                              // two buffers of 64 columns
 
@@ -371,6 +380,7 @@ __global__ void __launch_bounds__(COL_THREADS) k_bwd_col(const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = *slot_ptr;
   constexpr uint32_t IDESC = make_idesc_bf16(64, D, 1, 1);
+  const uint64_t VMN = ValTile::mnmajor(sbase, 0), OMN = T::mnmajor(sbase, 0);
 
   // unit u -> (bh, block column); columns of one (b,h) matrix together, the longest first
   auto unit_line = [&](int uu, int& bh, int& line, int& beg, int& end) {
@@ -434,17 +444,17 @@ __global__ void __launch_bounds__(COL_THREADS) k_bwd_col(const __grid_constant__
         if (!ok) break;
         const int st = nuse % NST;
         if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * st, (uint32_t)(nuse / NST) & 1u))) { ok = false; break; }
-        if (lane == 0) {
+        if (elect_one()) {
           tc_fence_after();
-          const uint32_t sa = sbase + st * STAGE_BYTES;
           const uint32_t first = i == 0 ? 0u : 1u;
+          const uint64_t da = desc_advance(VMN, st * STAGE_BYTES), db = desc_advance(OMN, st * STAGE_BYTES + VT_BYTES);
 #pragma unroll
           for (int kk = 0; kk < BS / 16; ++kk)                       // dK += dS^T Q  (lanes 0-15 of every quadrant)
-            mma_bf16(acc, ValTile::mnmajor(sa, kk), T::mnmajor(sa + VT_BYTES, kk), IDESC, (kk > 0) ? 1u : first);
+            mma_bf16(acc, desc_advance(da, kk * ValTile::MN_STEP), desc_advance(db, kk * T::MN_STEP), IDESC, (kk > 0) ? 1u : first);
 #pragma unroll
           for (int kk = 0; kk < BS / 16; ++kk)                       // dV += P^T dO  (lanes 16-31)
-            mma_bf16(acc + (16u << 16), ValTile::mnmajor(sa + VT_BYTES + T::BYTES, kk),
-                     T::mnmajor(sa + 2 * VT_BYTES + T::BYTES, kk), IDESC, (kk > 0) ? 1u : first);
+            mma_bf16(acc + (16u << 16), desc_advance(da, VT_BYTES + T::BYTES + kk * ValTile::MN_STEP),
+                     desc_advance(db, VT_BYTES + T::BYTES + kk * T::MN_STEP), IDESC, (kk > 0) ? 1u : first);
           mma_commit(bar_empty + 8 * st);
           if (i + 1 == n) mma_commit(bar_done + 8 * buf);
         }

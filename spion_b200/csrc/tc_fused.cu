@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - raw));
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const bool ctl = warp == 4;                                  // control warp: no arithmetic, no TMEM reads
   const int q = warp & 3;                                      // TMEM quadrant of a math warp
   const int hf = lane >> 4;                                    // 0: even tiles, 1: odd tiles
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
   constexpr uint32_t IDESC_O = make_idesc_bf16(64, D, 0, 1);
   const float sc2 = scale * LOG2E;
   // Barrier parities run on across the units of this CTA.  pk / pv: one bit per half of the buffers
-  // (only thread 0 waits on the load barriers); ps / po: bar_s / bar_o (every thread waits on each phase).
+  // (only the control warp waits on the load barriers); ps / po: bar_s / bar_o (every thread waits on each phase).
   uint32_t pk = 0, pv = 0, ps = 0, po = 0;
   bool ok = true;
 
@@ -217,14 +217,15 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       }
     };
 
-    // control lane: wait for the K tiles of job g (already requested) and issue the S MMAs of its chunk into
+    // control warp: wait for the K tiles of job g (already requested) and issue the S MMAs of its chunk into
     // accumulator columns col(t); the commit arrives on bar
     auto issue_s = [&](int g, uint32_t pair_stride, uint32_t col0, uint32_t bar) -> bool {
       const int ch = (single || g < nchunks) ? g : g - nchunks;
       const int t0 = ch * CH, nt = min(CH, nblk - t0);
       const int hb = single ? 0 : (g & 1), b0 = 2 * hb;
-      if (!mbar_wait(hb ? bar_k1 : bar_k0, (pk >> hb) & 1)) { report(status, ERR_LOAD_WAIT); return false; }
+      if (!warp_wait(hb ? bar_k1 : bar_k0, (pk >> hb) & 1, status, ERR_LOAD_WAIT)) return false;
       pk ^= 1u << hb;
+      if (elect_one()) {
       tc_fence_after();
       const uint64_t dq0 = T::kmajor(sQ, 0);
       uint64_t dk0 = T::kmajor(sK + b0 * T::BYTES, 0);
@@ -235,6 +236,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
           mma_bf16(d_addr, desc_advance(dq0, kk * T::K_STEP), desc_advance(dk0, kk * T::K_STEP), IDESC_S, kk > 0);
       }
       mma_commit(bar);
+      }
+      __syncwarp();
       return true;
     };
 
@@ -345,12 +348,13 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       }
     };
 
-    // control lane: O += P V for the tiles of one chunk (after its V tiles have arrived), then the P tile stores.
+    // control warp: O += P V for the tiles of one chunk (after its V tiles have arrived), then the P tile stores.
     // Every tile of the row accumulates into the one [64 x D] accumulator at lane offset 0.
-    auto issue_pv = [&](int hb, int t0, int nt, bool first_chunk) -> bool {
+    auto issue_pv = [&](int hb, int t0, int nt, bool first_chunk, bool last) -> bool {
       const int b0 = 2 * hb;
-      if (!mbar_wait(hb ? bar_v1 : bar_v0, (pv >> hb) & 1)) { report(status, ERR_LOAD_WAIT); return false; }
+      if (!warp_wait(hb ? bar_v1 : bar_v0, (pv >> hb) & 1, status, ERR_LOAD_WAIT)) return false;
       pv ^= 1u << hb;
+      if (elect_one()) {
       tc_fence_after();
       uint64_t dp0 = ValTile::kmajor(sP + b0 * VT_BYTES, 0), dv0 = T::mnmajor(sV + b0 * T::BYTES, 0);
       for (int t = 0; t < nt; ++t, dp0 = desc_advance(dp0, VT_BYTES), dv0 = desc_advance(dv0, T::BYTES)) {
@@ -360,7 +364,10 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
           mma_bf16(tmem + o_col, desc_advance(dp0, kk * ValTile::K_STEP), desc_advance(dv0, kk * T::MN_STEP), IDESC_O,
                    (kk > 0) ? 1u : first);
       }
-      if (STORE_P) {                                                // these tiles are final: store them now
+      if (last) mma_commit(bar_o);
+      }
+      __syncwarp();
+      if (STORE_P && lane == 0) {                                   // these tiles are final: store them now
         for (int t = 0; t < nt; ++t)
           tma_store_2d(&tmP, sP + (b0 + t) * VT_BYTES, 0, (int)(((size_t)bh * nnzb + rp + t0 + t) * BS));
         bulk_commit();
@@ -381,7 +388,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
 
     if (single && nblk > 0) {
       // ---------------------------------------------------------------- rows of at most 4 blocks
-      if (ctl && lane == 0) issue_s(0, 64u, 0u, bar_s);
+      if (ctl) issue_s(0, 64u, 0u, bar_s);
       if (!__syncthreads_and(mbar_wait(bar_s, ps))) { if (tid == 0) report(status, ERR_MMA_WAIT); ok = false; }
       ps ^= 1u;
       tc_fence_after();
@@ -444,7 +451,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
         tc_fence_before();
         __syncthreads();
         SPION_STAMP(ord, 4);
-        if (ctl && lane == 0 && issue_pv(0, 0, nblk, true)) mma_commit(bar_o);
+        if (ctl) issue_pv(0, 0, nblk, true, true);
         if (!__syncthreads_and(mbar_wait(bar_o, po))) { if (tid == 0) report(status, ERR_MMA2_WAIT); ok = false; }
         po ^= 1u;
         tc_fence_after();
@@ -454,10 +461,10 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       // Pass A (statistics): the pair of chunk c sits in columns 64 (c & 1); the MMAs of chunk c+1 are
       // issued before the arithmetic on chunk c.  bar_s serves the even chunks, bar_o the odd ones.
       const int n = nchunks;
-      if (ctl && lane == 0) issue_s(0, 0u, 0u, bar_s);
+      if (ctl) issue_s(0, 0u, 0u, bar_s);
       for (int c = 0; c < n && ok; ++c) {
         const int b = c & 1;
-        if (ctl && lane == 0 && c + 1 < n) issue_s(c + 1, 0u, (uint32_t)(b ^ 1) * 64u, b ? bar_s : bar_o);
+        if (ctl && c + 1 < n) issue_s(c + 1, 0u, (uint32_t)(b ^ 1) * 64u, b ? bar_s : bar_o);
         if (!__syncthreads_and(mbar_wait(b ? bar_o : bar_s, b ? po : ps))) {
           if (tid == 0) report(status, ERR_MMA_WAIT);
           ok = false;
@@ -474,7 +481,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       // Pass B: S of a chunk in columns [64,128), O accumulates in [0,64).  The tensor pipe completes in
       // issue order: once S(c+1) has arrived, O += P V of chunk c is complete too, and its half of the
       // buffers is requested again.
-      if (ok && ctl && lane == 0) issue_s(n, 0u, 64u, bar_s);
+      if (ok && ctl) issue_s(n, 0u, 64u, bar_s);
       for (int c = 0; c < n && ok; ++c) {
         const int g = n + c, hb = g & 1, t0 = 2 * c, nt = min(2, nblk - t0);
         if (!__syncthreads_and(mbar_wait(bar_s, ps))) { if (tid == 0) report(status, ERR_MMA_WAIT); ok = false; break; }
@@ -489,10 +496,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
-        if (ctl && lane == 0 && issue_pv(hb, t0, nt, c == 0)) {
-          if (c + 1 < n) issue_s(g + 1, 0u, 64u, bar_s);
-          else mma_commit(bar_o);
-        }
+        if (ctl && issue_pv(hb, t0, nt, c == 0, c + 1 == n) && c + 1 < n) issue_s(g + 1, 0u, 64u, bar_s);
       }
       if (ok) {
         if (!__syncthreads_and(mbar_wait(bar_o, po))) { if (tid == 0) report(status, ERR_MMA2_WAIT); ok = false; }

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
   volatile int* abort_ptr = reinterpret_cast<volatile int*>(smem_raw + (abort_w - sbase));
   auto sP = [&](int s, int t) -> uint32_t { return D == 64 ? sK + (s * NCH + t) * T::BYTES : sPsep + t * VT_BYTES; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const bool ctl = warp == 4;
   const int q = warp & 3;
   const int hf = lane >> 4;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
       }
       if (!wait_all(bar_qk + 8 * s, (ph_qk >> s) & 1, ERR_LOAD_WAIT)) return false;
       ph_qk ^= 1u << s;
-      if (lane == 0) {
+      if (elect_one()) {
         tc_fence_after();
         const uint64_t dq0 = T::kmajor(sQ + s * T::BYTES, 0);
         uint64_t dk0 = T::kmajor(sK + s * NCH * T::BYTES, 0);
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
       ph_p ^= 1u << s;
       if (!wait_all(bar_v, ph_v & 1, ERR_LOAD_WAIT)) return false;
       ph_v ^= 1u;
-      if (lane == 0) {
+      if (elect_one()) {
         tc_fence_after();
         uint64_t dp0 = ValTile::kmajor(sP(s, 0), 0), dv0 = T::mnmajor(sV, 0);
         for (int t = 0; t < R.nblk; ++t, dp0 = desc_advance(dp0, VT_BYTES), dv0 = desc_advance(dv0, T::BYTES)) {

@@ -16,7 +16,7 @@
 // The kernels are persistent (grid = CTAs the device holds at once, units taken with stride grid) and
 // use 8 math warps: warps w and w + 4 share TMEM quadrant w & 3 and split the 64 columns of a tile in
 // two halves, which the backward allows without any exchange (lse and delta are per-row inputs).
-// Thread 0 issues the TMA loads' MMAs; every wait on an mbarrier is bounded.
+// Warp 0 issues the TMA loads and the MMAs; every wait on an mbarrier is bounded.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(RC_THREADS, 2) k_bwd_row_rc(const __grid_const
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - raw));
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int q = warp & 3, g = warp >> 2;                       // TMEM quadrant, column half of the tiles
   const int hf = lane >> 4;                                    // 0: even tiles of a pair, 1: odd tiles
   const int row = q * 16 + (lane & 15);
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(RC_THREADS, 2) k_bwd_row_rc(const __grid_const
   constexpr uint32_t IDESC_S = make_idesc_bf16(64, 64, 0, 0);
   constexpr uint32_t IDESC_Q = make_idesc_bf16(64, D, 0, 1);
   const float sc2 = scale * LOG2E;
-  uint32_t pqk = 0, pov = 0, ps = 0, po = 0;                    // pqk / pov: one bit per half, thread 0 only
+  uint32_t pqk = 0, pov = 0, ps = 0, po = 0;                    // pqk / pov: one bit per half, warp 0 only
   bool ok = true;
 
   for (; u < total && ok; u += gridDim.x) {
@@ -192,47 +192,51 @@ __global__ void __launch_bounds__(RC_THREADS, 2) k_bwd_row_rc(const __grid_const
     // 32-wide masks: bit (2*(row/32) + col/32) of submask[block] tells whether that quarter is selected
     auto quarter_ok = [&](int blk) -> bool { return !SUB || ((submask[blk] >> ((q >> 1) * 2 + g)) & 1); };
 
-    // tid 0: S and dP MMAs of chunk ch; pair p of the chunk goes to columns colS + 64 p and colP + 64 p
+    // warp 0: S and dP MMAs of chunk ch; pair p of the chunk goes to columns colS + 64 p and colP + 64 p
     auto issue_sdp = [&](int ch, uint32_t colS, uint32_t colP) -> bool {
       const int CH = single ? NCH : 2;
       const int t0 = ch * CH, nt = min(CH, nblk - t0);
       const int hb = single ? 0 : (ch & 1), b0 = 2 * hb;
-      if (!mbar_wait(bar_qk + 8 * hb, (pqk >> hb) & 1)) { report(status, ERR_LOAD_WAIT); return false; }
+      auto products = [&](uint32_t sa, uint32_t sb, uint32_t col) {
+        const uint64_t da = T::kmajor(sa, 0);
+        uint64_t db = T::kmajor(sb + b0 * T::BYTES, 0);
+        for (int t = 0; t < nt; ++t, db = desc_advance(db, T::BYTES)) {
+          const uint32_t d_addr = tmem + ((uint32_t)((t & 1) * 16) << 16) + col + (uint32_t)(t >> 1) * 64u;
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            mma_bf16(d_addr, desc_advance(da, kk * T::K_STEP), desc_advance(db, kk * T::K_STEP), IDESC_S, kk > 0);
+        }
+      };
+      if (!warp_wait(bar_qk + 8 * hb, (pqk >> hb) & 1, status, ERR_LOAD_WAIT)) return false;
       pqk ^= 1u << hb;
-      tc_fence_after();
-      for (int t = 0; t < nt; ++t) {
-        const uint32_t d_addr = tmem + ((uint32_t)((t & 1) * 16) << 16) + colS + (uint32_t)(t >> 1) * 64u;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          mma_bf16(d_addr, T::kmajor(sQ, kk), T::kmajor(sK + (b0 + t) * T::BYTES, kk), IDESC_S, kk > 0);
-      }
-      if (!mbar_wait(bar_ov + 8 * hb, (pov >> hb) & 1)) { report(status, ERR_LOAD_WAIT); return false; }
+      if (elect_one()) { tc_fence_after(); products(sQ, sK, colS); }
+      __syncwarp();
+      if (!warp_wait(bar_ov + 8 * hb, (pov >> hb) & 1, status, ERR_LOAD_WAIT)) return false;
       pov ^= 1u << hb;
-      tc_fence_after();
-      for (int t = 0; t < nt; ++t) {
-        const uint32_t d_addr = tmem + ((uint32_t)((t & 1) * 16) << 16) + colP + (uint32_t)(t >> 1) * 64u;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-          mma_bf16(d_addr, T::kmajor(sdO, kk), T::kmajor(sV + (b0 + t) * T::BYTES, kk), IDESC_S, kk > 0);
-      }
-      mma_commit(bar_s);
+      if (elect_one()) { tc_fence_after(); products(sdO, sV, colP); mma_commit(bar_s); }
+      __syncwarp();
       return true;
     };
-    // tid 0: dQ += dS K for the tiles of a chunk (every tile into the one accumulator at lane offset 0)
-    auto issue_dq = [&](int hb, int nt, bool first_chunk) {
+    // warp 0: dQ += dS K for the tiles of a chunk (every tile into the one accumulator at lane offset 0)
+    auto issue_dq = [&](int hb, int nt, bool first_chunk, bool last) {
       const int b0 = 2 * hb;
-      for (int t = 0; t < nt; ++t) {
-        const uint32_t first = (first_chunk && t == 0) ? 0u : 1u;
+      if (elect_one()) {
+        tc_fence_after();
+        uint64_t da = ValTile::kmajor(sDS + b0 * VT_BYTES, 0), db = T::mnmajor(sK + b0 * T::BYTES, 0);
+        for (int t = 0; t < nt; ++t, da = desc_advance(da, VT_BYTES), db = desc_advance(db, T::BYTES)) {
+          const uint32_t first = (first_chunk && t == 0) ? 0u : 1u;
 #pragma unroll
-        for (int kk = 0; kk < BS / 16; ++kk)
-          mma_bf16(tmem, ValTile::kmajor(sDS + (b0 + t) * VT_BYTES, kk), T::mnmajor(sK + (b0 + t) * T::BYTES, kk), IDESC_Q,
-                   (kk > 0) ? 1u : first);
+          for (int kk = 0; kk < BS / 16; ++kk)
+            mma_bf16(tmem, desc_advance(da, kk * ValTile::K_STEP), desc_advance(db, kk * T::MN_STEP), IDESC_Q, (kk > 0) ? 1u : first);
+        }
+        if (last) mma_commit(bar_o);
       }
+      __syncwarp();
     };
 
     float delta = 0.f;
     if (nblk > 0) {
-      if (tid == 0) issue_sdp(0, single ? 0u : 64u, 128u);
+      if (warp == 0) issue_sdp(0, single ? 0u : 64u, 128u);
       // delta_i = sum_n dO_in O_in: the two owners of a row take one half of the head dimension each
       {
         const size_t off = (size_t)(pos.row0 + r * BS + row) * pos.ld + pos.x0 + hf * (D / 2);
@@ -277,11 +281,9 @@ __global__ void __launch_bounds__(RC_THREADS, 2) k_bwd_row_rc(const __grid_const
         fence_proxy_async();
         tc_fence_before();
         __syncthreads();
-        if (tid == 0) {
-          tc_fence_after();
-          issue_dq(hb, nt, c == 0);
+        if (warp == 0) {
+          issue_dq(hb, nt, c == 0, c + 1 == n);
           if (c + 1 < n) issue_sdp(c + 1, 64u, 128u);
-          else mma_commit(bar_o);
         }
       }
       if (ok) {
@@ -366,7 +368,7 @@ __global__ void __launch_bounds__(128) k_mean_map_rc(const __grid_constant__ CUt
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - raw));
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, q = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, q = warp_uniform(tid >> 5), lane = tid & 31;
   const int hf = lane >> 4, row = q * 16 + (lane & 15);
   const int blk = blockIdx.x;
   const int r = blk_row[blk], c = col_idx[blk];
@@ -413,20 +415,23 @@ __global__ void __launch_bounds__(128) k_mean_map_rc(const __grid_constant__ CUt
   const float sc2 = scale * LOG2E;
   bool ok = true;
 
-  // tid 0: S tiles of pair `it` into columns 64 (it & 1)
+  // warp 0: S tiles of pair `it` into columns 64 (it & 1)
   auto issue_s = [&](int it) -> bool {
     const int st = it & 1;
     const int cnt = min(2, BH - 2 * it);
-    if (!mbar_wait(bar_full + 8 * st, (uint32_t)(it >> 1) & 1u)) { report(status, ERR_LOAD_WAIT); return false; }
-    tc_fence_after();
-    const uint32_t base = sbase + st * 4 * T::BYTES;
-    for (int hb = 0; hb < cnt; ++hb) {
+    if (!warp_wait(bar_full + 8 * st, (uint32_t)(it >> 1) & 1u, status, ERR_LOAD_WAIT)) return false;
+    if (elect_one()) {
+      tc_fence_after();
+      const uint64_t base = T::kmajor(sbase + st * 4 * T::BYTES, 0);
+      for (int hb = 0; hb < cnt; ++hb) {
 #pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk)
-        mma_bf16(tmem + ((uint32_t)(hb * 16) << 16) + (uint32_t)st * 64u, T::kmajor(base + hb * T::BYTES, kk),
-                 T::kmajor(base + (2 + hb) * T::BYTES, kk), IDESC_S, kk > 0);
+        for (int kk = 0; kk < D / 16; ++kk)
+          mma_bf16(tmem + ((uint32_t)(hb * 16) << 16) + (uint32_t)st * 64u, desc_advance(base, hb * T::BYTES + kk * T::K_STEP),
+                   desc_advance(base, (2 + hb) * T::BYTES + kk * T::K_STEP), IDESC_S, kk > 0);
+      }
+      mma_commit(bar_s + 8 * st);
     }
-    mma_commit(bar_s + 8 * st);
+    __syncwarp();
     return true;
   };
 
@@ -436,10 +441,10 @@ __global__ void __launch_bounds__(128) k_mean_map_rc(const __grid_constant__ CUt
   const bool live0 = !SUB || ((submask[blk] >> ((q >> 1) * 2 + 0)) & 1);
   const bool live1 = !SUB || ((submask[blk] >> ((q >> 1) * 2 + 1)) & 1);
 
-  if (tid == 0) issue_s(0);
+  if (q == 0) issue_s(0);
   for (int it = 0; it < npair && ok; ++it) {
     const int st = it & 1;
-    if (tid == 0 && it + 1 < npair) issue_s(it + 1);
+    if (q == 0 && it + 1 < npair) issue_s(it + 1);
     if (!__syncthreads_and(mbar_wait(bar_s + 8 * st, (uint32_t)(it >> 1) & 1u))) {
       if (tid == 0) report(status, ERR_MMA_WAIT);
       ok = false;

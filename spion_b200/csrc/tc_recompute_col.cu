@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(CS_THREADS, 1) k_bwd_col_stream(const __grid_c
   auto sP = [&](int set, int e) { return sPD + set * C::PD_SET + (2 * e) * VT_BYTES; };
   auto sDS = [&](int set, int e) { return sPD + set * C::PD_SET + (2 * e + 1) * VT_BYTES; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int G = (int)gridDim.x;
   const int total = nb * BH;
   const int n_my = total > (int)blockIdx.x ? (total - (int)blockIdx.x + G - 1) / G : 0;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(CS_THREADS, 1) k_bwd_col_stream(const __grid_c
         if (par) ++kv_waits1; else ++kv_waits0;
       }
       if (!wait_all(pfull + 8 * ps, (uint32_t)(j / NP) & 1u, ERR_LOAD_WAIT)) return false;
-      if (lane == 0) {
+      if (elect_one()) {
         tc_fence_after();
         // every operand descriptor is one add on a descriptor of the buffer base (built once, outside the loop)
         const uint64_t dq0 = desc_advance(KM_BASE, ps * C::SLOT), do0 = desc_advance(dq0, 2 * T::BYTES);
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(CS_THREADS, 1) k_bwd_col_stream(const __grid_c
       }
       if (!wait_all(p_ready + 8 * set, (uint32_t)(j >> 1) & 1u, ERR_MMA_WAIT)) return false;
       SPION_STAMP_T(320, j, 5);
-      if (lane == 0) {
+      if (elect_one()) {
         tc_fence_after();
         const int cnt = c.cnt();
         const uint32_t acc = tmem + ACC + (uint32_t)par * 64u;

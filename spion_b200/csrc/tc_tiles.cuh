@@ -15,6 +15,13 @@ enum : int { ERR_LOAD_WAIT = 1, ERR_MMA_WAIT = 2, ERR_MMA2_WAIT = 4 };
 
 __device__ __forceinline__ void report(int* status, int code) { atomicOr(status, code); }
 
+// whole warp: bounded wait, reported once
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* status, int code) {
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+  if (!ok && (threadIdx.x & 31) == 0) report(status, code);
+  return ok;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
