@@ -78,7 +78,8 @@ __device__ __forceinline__ void store_row_swizzled(uint32_t tile, int i, const u
 // memory tiles the second product reads): rows of one chunk are rescaled in place once the
 // denominator is known; longer rows accumulate the denominator on line in pass A instead.
 // heads: 0 = operands [BH, L, D]; H = operands [B, L, H, D] (see op_pos).
-template <int D, bool STORE_P, bool SUB>
+// KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of every loop).
+template <int D, bool STORE_P, bool SUB, bool KP>
 __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_constant__ CUtensorMap tmQ,
                                                               const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV,
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
     const int CH = R.chunk();
     const int nchunks = R.nchunks();
     const int njobs = R.njobs();
-    const float* kp = keypad ? keypad + (size_t)bh * L : nullptr;
+    const float* kp = KP ? keypad + (size_t)bh * L : nullptr;
     const OpPos pos = op_pos(bh, L, heads, D);
 
     // All buffers of this unit are free (its last MMA has retired): ask for the next unit's first tiles.
@@ -254,13 +255,14 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
           const int t = 2 * p + hf;
           const bool mine = t < nt;
           const int c = mine ? col_of(t0 + t) : 0;
+          const float* kpc = KP && any_padded(kp + c * BS) ? kp + c * BS : nullptr;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             uint32_t v[32];
             tmem_ld32(t_lane + colbase + p * 64 + half * 32, v);
             tmem_ld_wait();
             if (mine && quarter_ok(rp + t0 + t, half)) {
-              if (!kp) {                                            // the scale is positive: compare raw scores
+              if (!kpc) {                                            // the scale is positive: compare raw scores
                 float ma = mraw, mb = -INFINITY, mc = -INFINITY, md = -INFINITY;   // four chains instead of one
 #pragma unroll
                 for (int j = 0; j < 32; j += 8) {
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
               } else {
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
-                  m2 = fmaxf(m2, fmaf(__uint_as_float(v[j]), sc2, -kp[c * BS + half * 32 + j] * LOG2E));
+                  m2 = fmaxf(m2, fmaf(__uint_as_float(v[j]), sc2, -kpc[half * 32 + j] * LOG2E));
               }
             }
           }
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
           const int t = 2 * p + hf;
           const bool mine = t < nt;
           const int c = mine ? col_of(t0 + t) : 0;
+          const float* kpc = KP && any_padded(kp + c * BS) ? kp + c * BS : nullptr;
           uint32_t v0[32], v1[32];
           tmem_ld32(t_lane + colbase + p * 64, v0);
           tmem_ld32(t_lane + colbase + p * 64 + 32, v1);
@@ -293,7 +296,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
               float x0 = __uint_as_float(v0[j]) * sc2, x1 = __uint_as_float(v1[j]) * sc2;
-              if (kp) { x0 -= kp[c * BS + j] * LOG2E; x1 -= kp[c * BS + 32 + j] * LOG2E; }
+              if (kpc) { x0 -= kpc[j] * LOG2E; x1 -= kpc[32 + j] * LOG2E; }
               if (!ok0) x0 = -INFINITY;
               if (!ok1) x1 = -INFINITY;
               v0[j] = __float_as_uint(x0); v1[j] = __float_as_uint(x1);
@@ -320,6 +323,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
         const int t = 2 * p + hf;
         const bool mine = t < nt;
         const int c = mine ? col_of(t0 + t) : 0;
+        const float* kpc = KP && any_padded(kp + c * BS) ? kp + c * BS : nullptr;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t v[32], w[16];
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
               float h0 = m2, h1 = m2;
-              if (kp) { h0 = fmaf(kp[c * BS + half * 32 + j], LOG2E, m2); h1 = fmaf(kp[c * BS + half * 32 + j + 1], LOG2E, m2); }
+              if (kpc) { h0 = fmaf(kpc[half * 32 + j], LOG2E, m2); h1 = fmaf(kpc[half * 32 + j + 1], LOG2E, m2); }
               const float e0 = ex2(fmaf(__uint_as_float(v[j]), sc2, -h0)), e1 = ex2(fmaf(__uint_as_float(v[j + 1]), sc2, -h1));
               if ((j & 6) == 0) la += e0 + e1;
               else if ((j & 6) == 2) lb += e0 + e1;
@@ -408,6 +412,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
             const int t = 2 * p + hf;
             const bool mine = t < nblk;
             const int c = mine ? col_of(t) : 0;
+            const float* kpc = KP && any_padded(kp + c * BS) ? kp + c * BS : nullptr;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
               uint32_t v[32];
@@ -417,7 +422,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) {
                   float h0 = m2, h1 = m2;
-                  if (kp) { h0 = fmaf(kp[c * BS + half * 32 + j], LOG2E, m2); h1 = fmaf(kp[c * BS + half * 32 + j + 1], LOG2E, m2); }
+                  if (kpc) { h0 = fmaf(kpc[half * 32 + j], LOG2E, m2); h1 = fmaf(kpc[half * 32 + j + 1], LOG2E, m2); }
                   const float e0 = ex2(fmaf(__uint_as_float(v[j]), sc2, -h0)), e1 = ex2(fmaf(__uint_as_float(v[j + 1]), sc2, -h1));
                   l_part += e0 + e1;
                   wp[p][half * 16 + (j >> 1)] = pack_bf16(e0, e1);
@@ -575,14 +580,18 @@ template <int D>
 static int fwd_attrs(TcState* s, int device) {
   const int bytes = (int)fwd_smem_bytes<D>();
   int occ = 1 << 30, n = 0, rc;
-#define SPION_FWD_ATTR(SP, SB)                                                                                      \
-  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_fused<D, SP, SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
-  if ((rc = resident_ctas(k_fwd_fused<D, SP, SB>, device, FWD_THREADS, (size_t)bytes, 128, &n))) return rc;         \
+#define SPION_FWD_ATTR(SP, SB, KP)                                                                                      \
+  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_fused<D, SP, SB, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
+  if ((rc = resident_ctas(k_fwd_fused<D, SP, SB, KP>, device, FWD_THREADS, (size_t)bytes, 128, &n))) return rc;         \
   occ = n < occ ? n : occ;
-  SPION_FWD_ATTR(false, false)
-  SPION_FWD_ATTR(true, false)
-  SPION_FWD_ATTR(false, true)
-  SPION_FWD_ATTR(true, true)
+  SPION_FWD_ATTR(false, false, false)
+  SPION_FWD_ATTR(false, false, true)
+  SPION_FWD_ATTR(true, false, false)
+  SPION_FWD_ATTR(true, false, true)
+  SPION_FWD_ATTR(false, true, false)
+  SPION_FWD_ATTR(false, true, true)
+  SPION_FWD_ATTR(true, true, false)
+  SPION_FWD_ATTR(true, true, true)
 #undef SPION_FWD_ATTR
   s->fwd_ctas = occ;
   return SPION_OK;
@@ -612,12 +621,14 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
   const float floor_v = keypad ? 0.0f : -100.0f;
   if (total > 0) {
     const int grid = (int)(total < (long long)s->sms * s->fwd_ctas ? total : (long long)s->sms * s->fwd_ctas);
-#define SPION_FWD_LAUNCH(SP, SB)                                                                                  \
-  k_fwd_fused<D, SP, SB><<<grid, FWD_THREADS, fwd_smem_bytes<D>(), c->stream>>>(                                   \
+#define SPION_FWD_LAUNCH(SP, SB, KP)                                                                                  \
+  k_fwd_fused<D, SP, SB, KP><<<grid, FWD_THREADS, fwd_smem_bytes<D>(), c->stream>>>(                                   \
       mq, mk, mv, mp, (__nv_bfloat16*)O, lse, keypad, vw.row_info, vw.col_idx, vw.submask, c->L, vw.nnzb, c->BH,   \
       rows_here, c->heads, c->scale, floor_v, c->status_dev)
-    if (P64) { if (vw.submask) SPION_FWD_LAUNCH(true, true); else SPION_FWD_LAUNCH(true, false); }
-    else { if (vw.submask) SPION_FWD_LAUNCH(false, true); else SPION_FWD_LAUNCH(false, false); }
+#define SPION_FWD_PICK(SP, SB) do { if (keypad) SPION_FWD_LAUNCH(SP, SB, true); else SPION_FWD_LAUNCH(SP, SB, false); } while (0)
+    if (P64) { if (vw.submask) SPION_FWD_PICK(true, true); else SPION_FWD_PICK(true, false); }
+    else { if (vw.submask) SPION_FWD_PICK(false, true); else SPION_FWD_PICK(false, false); }
+#undef SPION_FWD_PICK
 #undef SPION_FWD_LAUNCH
     SPION_LAUNCH_CHECK();
     c->launches += 1;

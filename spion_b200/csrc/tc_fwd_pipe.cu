@@ -53,7 +53,8 @@ __device__ __forceinline__ void store_half_row(uint32_t tile, int i, int g, cons
   }
 }
 
-template <int D, bool STORE_P, bool SUB>
+// KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of every loop).
+template <int D, bool STORE_P, bool SUB, bool KP>
 __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_constant__ CUtensorMap tmQ,
                                                               const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV,
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
       const int s = i & 1;
       const int rp = R.rp, nblk = R.nblk;
       const uint32_t t_set = t_lane + (uint32_t)s * 128u;
-      const float* kp = keypad ? keypad + (size_t)bh * L : nullptr;
+      const float* kp = KP ? keypad + (size_t)bh * L : nullptr;
       const OpPos pos = op_pos(bh, L, heads, D);
       const int rh2 = (q >> 1) * 2;
       auto quarter_ok = [&](int blk, int half) -> bool { return !SUB || ((submask[blk] >> (rh2 + half)) & 1); };
@@ -321,13 +322,14 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
           const int t = 2 * p + hf;
           const bool mine = t < nblk;
           const int c = mine ? R.col(t, col_idx) : 0;
+          const float* kpc = KP && any_padded(kp + c * BS) ? kp + c * BS : nullptr;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             uint32_t v[32];
             tmem_ld32(t_set + p * 64 + half * 32, v);
             tmem_ld_wait();
             if (mine && quarter_ok(rp + t, half)) {
-              if (!kp) {                                          // the scale is positive: compare raw scores
+              if (!kpc) {                                          // the scale is positive: compare raw scores
                 float ma = mraw, mb = -INFINITY, mc = -INFINITY, md = -INFINITY;
 #pragma unroll
                 for (int j = 0; j < 32; j += 8) {
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
               } else {
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
-                  m2 = fmaxf(m2, fmaf(__uint_as_float(v[j]), sc2, -kp[c * BS + half * 32 + j] * LOG2E));
+                  m2 = fmaxf(m2, fmaf(__uint_as_float(v[j]), sc2, -kpc[half * 32 + j] * LOG2E));
               }
             }
           }
@@ -362,6 +364,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
           const int t = 2 * p + hf;
           const bool mine = t < nblk;
           const int c = mine ? R.col(t, col_idx) : 0;
+          const float* kpc = KP && any_padded(kp + c * BS) ? kp + c * BS : nullptr;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             uint32_t v[32];
@@ -372,7 +375,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
 #pragma unroll
               for (int j = 0; j < 32; j += 2) {
                 float h0 = m2, h1 = m2;
-                if (kp) { h0 = fmaf(kp[c * BS + half * 32 + j], LOG2E, m2); h1 = fmaf(kp[c * BS + half * 32 + j + 1], LOG2E, m2); }
+                if (kpc) { h0 = fmaf(kpc[half * 32 + j], LOG2E, m2); h1 = fmaf(kpc[half * 32 + j + 1], LOG2E, m2); }
                 const float e0 = ex2(fmaf(__uint_as_float(v[j]), sc2, -h0)), e1 = ex2(fmaf(__uint_as_float(v[j + 1]), sc2, -h1));
                 if (j & 2) lb += e0 + e1; else la += e0 + e1;
                 wp[p][half * 16 + (j >> 1)] = pack_bf16(e0, e1);
@@ -450,14 +453,18 @@ template <int D>
 static int pipe_attrs(TcState* s, int device) {
   const int bytes = (int)pipe_smem_bytes<D>();
   int occ = 1 << 30, n = 0, rc;
-#define SPION_PIPE_ATTR(SP, SB)                                                                                    \
-  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_pipe<D, SP, SB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
-  if ((rc = resident_ctas(k_fwd_pipe<D, SP, SB>, device, PIPE_THREADS, (size_t)bytes, 256, &n))) return rc;        \
+#define SPION_PIPE_ATTR(SP, SB, KP)                                                                                    \
+  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_pipe<D, SP, SB, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
+  if ((rc = resident_ctas(k_fwd_pipe<D, SP, SB, KP>, device, PIPE_THREADS, (size_t)bytes, 256, &n))) return rc;        \
   occ = n < occ ? n : occ;
-  SPION_PIPE_ATTR(false, false)
-  SPION_PIPE_ATTR(true, false)
-  SPION_PIPE_ATTR(false, true)
-  SPION_PIPE_ATTR(true, true)
+  SPION_PIPE_ATTR(false, false, false)
+  SPION_PIPE_ATTR(false, false, true)
+  SPION_PIPE_ATTR(true, false, false)
+  SPION_PIPE_ATTR(true, false, true)
+  SPION_PIPE_ATTR(false, true, false)
+  SPION_PIPE_ATTR(false, true, true)
+  SPION_PIPE_ATTR(true, true, false)
+  SPION_PIPE_ATTR(true, true, true)
 #undef SPION_PIPE_ATTR
   s->pipe_ctas = occ;
   return SPION_OK;
@@ -474,12 +481,14 @@ static int pipe_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CU
   const long long cap = (long long)s->sms * s->pipe_ctas;
   const int grid = (int)(total < cap ? total : cap);
   const float floor_v = keypad ? 0.0f : -100.0f;
-#define SPION_PIPE_LAUNCH(SP, SB)                                                                                    \
-  k_fwd_pipe<D, SP, SB><<<grid, PIPE_THREADS, pipe_smem_bytes<D>(), c->stream>>>(                                     \
+#define SPION_PIPE_LAUNCH(SP, SB, KP)                                                                                    \
+  k_fwd_pipe<D, SP, SB, KP><<<grid, PIPE_THREADS, pipe_smem_bytes<D>(), c->stream>>>(                                     \
       mq, mk, mv, mp, (__nv_bfloat16*)O, lse, keypad, vw.row_info, vw.col_idx, vw.submask, c->L, vw.nnzb, c->BH, rank0, \
       vw.nb, c->heads, c->scale, floor_v, c->status_dev)
-  if (store_p) { if (vw.submask) SPION_PIPE_LAUNCH(true, true); else SPION_PIPE_LAUNCH(true, false); }
-  else { if (vw.submask) SPION_PIPE_LAUNCH(false, true); else SPION_PIPE_LAUNCH(false, false); }
+#define SPION_PIPE_PICK(SP, SB) do { if (keypad) SPION_PIPE_LAUNCH(SP, SB, true); else SPION_PIPE_LAUNCH(SP, SB, false); } while (0)
+  if (store_p) { if (vw.submask) SPION_PIPE_PICK(true, true); else SPION_PIPE_PICK(true, false); }
+  else { if (vw.submask) SPION_PIPE_PICK(false, true); else SPION_PIPE_PICK(false, false); }
+#undef SPION_PIPE_PICK
 #undef SPION_PIPE_LAUNCH
   SPION_LAUNCH_CHECK();
   c->launches += 1;

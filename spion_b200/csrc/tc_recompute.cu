@@ -455,7 +455,8 @@ __global__ void __launch_bounds__(128) k_mean_map_rc(const __grid_constant__ CUt
     const int bh = 2 * it + hf;
     const bool mine = bh < BH;
     const float lse = mine ? lse_in[(size_t)bh * L + r * BS + row] : 0.f;
-    const float* kp = (keypad && mine) ? keypad + (size_t)bh * L + c * BS : nullptr;
+    const float* kp = keypad ? keypad + (size_t)(mine ? bh : 0) * L + c * BS : nullptr;
+    if (kp && !any_padded(kp)) kp = nullptr;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       uint32_t v[32];
