@@ -611,6 +611,11 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
     return rc;
   if (P64) { if ((rc = make_map(s, &mp, P64, vrows, BS, BS, BS))) return rc; } else mp = mq;
   prof_mark(c, -1);
+  if (!P64 && s->n_long > 0) {
+    if ((rc = stream_forward(c, s, mq, mk, mv, keypad, O, lse))) return rc;
+    prof_mark(c, SPION_STAGE_FUSED_FWD);
+    return SPION_OK;
+  }
   // Masks whose rows all have at most four blocks run on the pipelined kernel for short rows
   // (tc_fwd_pipe.cu: about 1.7x less time per row, two CTAs per SM).  As soon as some rows are longer,
   // everything goes through this file's kernel: a second launch for a handful of long rows costs more

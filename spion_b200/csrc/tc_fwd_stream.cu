@@ -1,0 +1,441 @@
+// Forward of the block-sparse attention as a streaming pipeline (sm_100a, bf16, 64 x 64 blocks, no stored P): O and one fp32
+// log-sum-exp per row (models/block_attn.cu:453-487 fused; softmax semantics as in tc_fused.cu).
+//
+// One persistent CTA per SM with four groups.  A group has one service warp (TMA loads, MMA issue) and four arithmetic warps (one per
+// tensor-memory quadrant) and walks block rows of its own, two blocks ("a pair") at a time:
+//     S = Q K_e^T   (M = 64, the second block at lane offset 16: query rows along the lanes, a row owned by lanes l and l + 16)
+//     P = exp2(S scale log2e - m), unnormalised, bf16 into shared memory (over the K tiles when they are as large)
+//     O += P V_e    (M = 64, tensor memory, lane offset 16 x parity of the row)
+// S of pair j + 1 is computed while pair j is in the arithmetic (its 64 values per lane are in registers), and the rows of a
+// finished unit are written after the first pair of the next one.  Nothing is exchanged between the groups: they only fill each
+// other's waits.
+//
+// One pass over a row: m is the maximum of its first pair and is only moved (O and the running sum rescaled) when a later
+// score exceeds it by more than 2^8, so that almost no row is ever rescaled; the result is divided by the sum against the true
+// maximum at the end.  P <= 2^8 loses nothing in bf16 or in the fp32 sums.
+//
+// What bounds it: the exponentials, 8192 per pair at 16 per cycle and SM = 512 cycles, and 16 MMAs of 33 cycles at head_dim 64.
+// Measured (forward alone, this kernel against one unit per CTA and two passes over a row, tc_fused.cu):  see fwd_launch there.
+//
+// Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
+#include "tc_stream.cuh"
+
+using namespace tc;
+
+namespace {
+
+constexpr int NG = 4;                                             // groups
+constexpr int FS_THREADS = 32 * (4 + 4 * NG);
+constexpr float MOVE = 8.0f;                                      // log2 units by which a score may exceed m
+
+template <int D> struct Fs {
+  using T = OpTile<D>;
+  static constexpr bool ALIAS = D == 64;                          // P tiles over the K tiles
+  static constexpr uint32_t PB = 2 * VT_BYTES;                    // P tiles of a pair (ALIAS: K tiles first), two buffers
+  static constexpr uint32_t O_Q = 0, O_P = T::BYTES, O_V = O_P + 2 * PB, O_K = O_V + 2 * T::BYTES;
+  static constexpr uint32_t GROUP = O_K + (ALIAS ? 0 : 2 * T::BYTES);
+  static constexpr uint32_t O_BAR = NG * GROUP;
+  static constexpr uint32_t GBAR = 112;                           // barriers of a group
+  static constexpr size_t SMEM = O_BAR + NG * GBAR + 16 + NG * 32;
+  static constexpr uint32_t COLS = 64 + D;                        // tensor-memory columns of a group: S, O
+};
+
+__device__ __forceinline__ void tmem_ld8(uint32_t a, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t a, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+struct FsArgs {
+  __nv_bfloat16* O;
+  float* lse;
+  const float* keypad;
+  const int4 *rec, *pair;                                         // block rows and their pairs (k_line_recs)
+  const uint8_t* submask;
+  int L, BH, nb, heads, by_rank;
+  float scale, floor_v;
+  int* status;
+};
+
+template <int D, bool KP, bool SUB>
+__global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                                                              const __grid_constant__ CUtensorMap tmV, const __grid_constant__ FsArgs a) {
+  using C = Fs<D>;
+  using T = OpTile<D>;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t sbase = smem_u32(smem_raw);                      // must be 1024-aligned (checked below)
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
+  const int grp = warp < 4 ? warp : (warp - 4) >> 2;
+  const uint32_t gb = sbase + grp * C::GROUP, bars = sbase + C::O_BAR + grp * C::GBAR;
+  // q_full, k_full[2], v_full: tiles landed; s_ready: S of a pair complete; s_free: read out (4 warps); p_ready[2]: P tiles written (4
+  // warps); pv_done[2]: O += P V of a pair complete, with every MMA issued before it; pi_full[2]: flags of a pair written
+  const uint32_t q_full = bars, k_full = bars + 8, v_full = bars + 24, s_ready = bars + 32, s_free = bars + 40, p_ready = bars + 48,
+                 pv_done = bars + 64, pi_full = bars + 80;
+  const uint32_t slot = sbase + C::O_BAR + NG * C::GBAR, abort_w = slot + 4;
+  uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
+  volatile int* abort_ptr = reinterpret_cast<volatile int*>(smem_raw + (abort_w - sbase));
+  int* info = reinterpret_cast<int*>(smem_raw + (slot - sbase) + 16 + grp * 32);        // [2][4]: flags, block columns of the pair
+
+  if (warp == 0 && lane == 0) {
+    int ab = *reinterpret_cast<volatile int*>(a.status);
+    if ((sbase & 1023u) != 0u) { report(a.status, ERR_LOAD_WAIT); ab = 1; }
+    *abort_ptr = ab;
+    for (int g = 0; g < NG; ++g) {
+      const uint32_t b = sbase + C::O_BAR + g * C::GBAR;
+      for (int x = 0; x < 5; ++x) mbar_init(b + 8 * x, 1);        // q_full, k_full[2], v_full, s_ready
+      for (int x = 5; x < 8; ++x) mbar_init(b + 8 * x, 4);        // s_free, p_ready[2]
+      for (int x = 8; x < 12; ++x) mbar_init(b + 8 * x, 1);       // pv_done[2], pi_full[2]
+    }
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (*abort_ptr != 0) return;
+  if (warp == 0) {
+    tmem_alloc(slot, 512u);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *slot_ptr, tS = tmem + grp * C::COLS, tO = tS + 64u;
+  auto wait_all = [&](uint32_t bar, uint32_t parity, int code) -> bool { return warp_wait(bar, parity & 1u, a.status, code); };
+  const UnitMap um{a.nb, a.BH, a.by_rank};
+  // group g of CTA b walks units b + g G, + NG G, ...
+  const int first = (int)blockIdx.x + grp * (int)gridDim.x, step = NG * (int)gridDim.x, total = a.nb * a.BH;
+
+  if (warp < 4) {
+    // ================================================================== service warp of a group
+    constexpr uint32_t IDESC_S = make_idesc_bf16(64, 64, 0, 0), IDESC_O = make_idesc_bf16(64, D, 0, 1);
+    const uint64_t dQ = T::kmajor(gb + C::O_Q, 0);
+    Walk c, ld;                                                   // MMAs; loads (a pair ahead)
+    c.init(um, a.rec, first, step, total);
+    c.skip();
+    ld = c;
+    int4 pr = ld.valid() ? a.pair[ld.cur.y] : make_int4(0, -1, 0, 0);      // record of the pair whose K tiles are loaded next
+    int4 prv = pr;                                                // ... whose V tiles are loaded next
+    bool pad_l = false;
+    uint8_t sub_l = 0xff;
+    auto flags_load = [&](const Walk& w, const int4& p) {         // requested with the pair's K tiles, used a pair later
+      const int e = lane >> 4, o = e ? p.y : p.x;
+      if (KP) pad_l = o >= 0 && pad4(a.keypad + (size_t)w.bh * a.L + o * BS);
+      if (SUB) sub_l = o >= 0 ? a.submask[e ? p.w : p.z] : (uint8_t)0;
+    };
+    auto load_k = [&](int j) {                                    // K tiles of the pair at `ld` (pair j), Q with the first of a unit
+      const uint32_t bar = k_full + 8 * (C::ALIAS ? (j & 1) : 0), dst = gb + (C::ALIAS ? C::O_P + (j & 1) * C::PB : C::O_K);
+      const int cnt = ld.cnt();
+      const OpPos pos = op_pos(ld.bh, a.L, a.heads, D);
+      if (lane == 0) {
+        mbar_expect_tx(bar, cnt * T::BYTES);
+        if (ld.k == 0) mbar_expect_tx(q_full, T::BYTES);
+      }
+      __syncwarp();
+      if (lane < cnt) tma_load_2d(dst + lane * T::BYTES, &tmK, bar, pos.x0, pos.row0 + (lane ? pr.y : pr.x) * BS);
+      if (lane == 4 && ld.k == 0) tma_load_2d(gb + C::O_Q, &tmQ, q_full, pos.x0, pos.row0 + ld.cur.x * BS);
+    };
+    auto load_v = [&](const Walk& w) {
+      const int cnt = w.cnt();
+      const OpPos pos = op_pos(w.bh, a.L, a.heads, D);
+      if (lane == 0) mbar_expect_tx(v_full, cnt * T::BYTES);
+      __syncwarp();
+      if (lane < cnt) tma_load_2d(gb + C::O_V + lane * T::BYTES, &tmV, v_full, pos.x0, pos.row0 + (lane ? prv.y : prv.x) * BS);
+    };
+    bool ok = true;
+    int units = 0;                                                // units begun
+    if (c.valid()) {
+      flags_load(ld, pr);
+      load_k(0);
+      prv = pr;
+      load_v(ld);
+      ld.next();
+      if (ld.valid()) pr = a.pair[ld.cur.y + ld.k];
+    }
+    int p_cnt = 0, p_par = 0;                                     // the pair before c
+    bool p_first = false;
+    for (int j = 0; ok; ++j) {
+      const bool have = c.valid();
+      if (have) {
+        if (KP || SUB) {                                          // flags of pair j: its buffer was read before P of pair j - 2 was written
+          const uint32_t any = KP ? __ballot_sync(0xffffffffu, pad_l) : 0u;
+          const int s1 = SUB ? __shfl_sync(0xffffffffu, (int)sub_l, 16) : 0xff;
+          if (lane == 0) {
+            int* x = info + 4 * (j & 1);
+            x[0] = ((any & 0xffffu) ? 1 : 0) | ((any >> 16) ? 2 : 0) | ((SUB ? (int)sub_l : 0xff) << 8) | (s1 << 16);
+            x[1] = prv.x; x[2] = prv.y;
+            mbar_arrive(pi_full + 8 * (j & 1));
+          }
+          __syncwarp();
+        }
+        // S of pair j
+        const int kb = C::ALIAS ? (j & 1) : 0, ku = C::ALIAS ? (j >> 1) : j;
+        if (c.k == 0) { if (!wait_all(q_full, (uint32_t)units, ERR_LOAD_WAIT)) { ok = false; break; } ++units; }
+        if (!wait_all(k_full + 8 * kb, (uint32_t)ku, ERR_LOAD_WAIT)) { ok = false; break; }
+        if (j >= 1 && !wait_all(s_free, (uint32_t)(j - 1), ERR_MMA_WAIT)) { ok = false; break; }
+        const bool two = warp_uniform(c.cnt() == 2);
+        if (elect_one()) {
+          tc_fence_after();
+          const uint64_t dK = T::kmajor(gb + (C::ALIAS ? C::O_P + kb * C::PB : C::O_K), 0);
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk) mma_bf16(tS, desc_advance(dQ, kk * T::K_STEP), desc_advance(dK, kk * T::K_STEP), IDESC_S, kk > 0);
+          if (two) {
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk)
+              mma_bf16(tS + (16u << 16), desc_advance(dQ, kk * T::K_STEP), desc_advance(dK, T::BYTES + kk * T::K_STEP), IDESC_S, kk > 0);
+          }
+          mma_commit(s_ready);
+        }
+        __syncwarp();
+      }
+      if (j >= 1) {                                               // O += P V of pair j - 1
+        const int jp = j - 1;
+        if (!wait_all(p_ready + 8 * (jp & 1), (uint32_t)(jp >> 1), ERR_MMA_WAIT)) { ok = false; break; }
+        if (!wait_all(v_full, (uint32_t)jp, ERR_LOAD_WAIT)) { ok = false; break; }
+        const bool two = warp_uniform(p_cnt == 2), fresh = warp_uniform((int)p_first) != 0;
+        if (elect_one()) {
+          tc_fence_after();
+          const uint32_t acc = tO + ((uint32_t)(p_par * 16) << 16);
+          const uint64_t dP = ValTile::kmajor(gb + C::O_P + (jp & 1) * C::PB, 0), dV = T::mnmajor(gb + C::O_V, 0);
+#pragma unroll
+          for (int kk = 0; kk < BS / 16; ++kk)
+            mma_bf16(acc, desc_advance(dP, kk * ValTile::K_STEP), desc_advance(dV, kk * T::MN_STEP), IDESC_O, (kk > 0 || !fresh) ? 1u : 0u);
+          if (two) {
+#pragma unroll
+            for (int kk = 0; kk < BS / 16; ++kk)
+              mma_bf16(acc, desc_advance(dP, VT_BYTES + kk * ValTile::K_STEP), desc_advance(dV, T::BYTES + kk * T::MN_STEP), IDESC_O, 1u);
+          }
+          mma_commit(pv_done + 8 * (jp & 1));
+        }
+        __syncwarp();
+      }
+      if (!have) break;
+      // Loads.  O += P V of pair j - 1 complete implies S of pair j (issued before it): K (its own buffer, or the P buffer of
+      // pair j - 1), Q and V are free.
+      if (j >= 1) {
+        if (!wait_all(pv_done + 8 * ((j - 1) & 1), (uint32_t)((j - 1) >> 1), ERR_MMA2_WAIT)) { ok = false; break; }
+        load_v(c);                                                // V of pair j (pair 0's was requested above)
+      } else if (!wait_all(s_ready, 0u, ERR_MMA_WAIT)) { ok = false; break; }
+      if (ld.valid()) {
+        flags_load(ld, pr);
+        load_k(j + 1);
+        prv = pr;
+        ld.next();
+        if (ld.valid()) pr = a.pair[ld.cur.y + ld.k];
+      }
+      p_cnt = c.cnt(); p_par = c.i & 1; p_first = c.k == 0;
+      c.next();
+    }
+  } else {
+    // ================================================================== arithmetic warps of a group
+    const int q = warp & 3, hf = lane >> 4, row = q * 16 + (lane & 15);
+    const uint32_t lS = tS + ((uint32_t)(q * 32) << 16), lO = tO + ((uint32_t)(q * 32) << 16);
+    const float sc2 = a.scale * LOG2E, floor2 = a.floor_v * LOG2E;
+    bool ok = true;
+    // the finished unit whose rows are still in tensor memory
+    bool pend = false;
+    int pend_par = 0, pend_j = 0;
+    float pend_inv = 0.f;
+    __nv_bfloat16* pend_dst = nullptr;
+    auto write_rows = [&](__nv_bfloat16* dst, bool have, float inv, bool mine) {
+#pragma unroll
+      for (int h = 0; h < D / 32; ++h) {
+        uint32_t v[32];
+        if (have) {
+          tmem_ld32(lO + h * 32, v);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int x = 0; x < 32; ++x) v[x] = 0u;
+        }
+        if (mine) {
+#pragma unroll
+          for (int x = 0; x < 32; x += 8)
+            *reinterpret_cast<uint4*>(dst + h * 32 + x) = make_uint4(pack_bf16(__uint_as_float(v[x]) * inv, __uint_as_float(v[x + 1]) * inv),
+                                                                     pack_bf16(__uint_as_float(v[x + 2]) * inv, __uint_as_float(v[x + 3]) * inv),
+                                                                     pack_bf16(__uint_as_float(v[x + 4]) * inv, __uint_as_float(v[x + 5]) * inv),
+                                                                     pack_bf16(__uint_as_float(v[x + 6]) * inv, __uint_as_float(v[x + 7]) * inv));
+        }
+      }
+    };
+    auto flush = [&]() -> bool {
+      if (!wait_all(pv_done + 8 * (pend_j & 1), (uint32_t)(pend_j >> 1), ERR_MMA2_WAIT)) return false;
+      tc_fence_after();
+      write_rows(pend_dst, true, pend_inv, hf == pend_par);
+      tc_fence_before();
+      pend = false;
+      return true;
+    };
+    Walk u;
+    u.init(um, a.rec, first, step, total);
+    int j = 0;
+    for (; u.valid() && ok; u.shift()) {
+      const int n = u.cur.w, par = u.i & 1;
+      const OpPos pos = op_pos(u.bh, a.L, a.heads, D);
+      __nv_bfloat16* dst = a.O + (size_t)(pos.row0 + u.cur.x * BS + row) * pos.ld + pos.x0;
+      float* lse = a.lse + (size_t)u.bh * a.L + u.cur.x * BS + row;
+      if (n == 0) {                                               // a row without blocks: every key counts as score 0
+        const float m0 = fmaxf(floor2, -INFINITY);
+        if (hf == 0) *lse = m0 + log2f((float)a.L * exp2f(-m0));
+        write_rows(dst, false, 0.f, hf == 0);
+        continue;
+      }
+      const float* kpu = KP ? a.keypad + (size_t)u.bh * a.L : nullptr;
+      float m = floor2, mx = floor2, l = 0.f;                     // reference exponent, true maximum, sum
+      int n_sel = 0;
+      const int np = u.pairs();
+      for (int k = 0; k < np && ok; ++k, ++j) {
+        const bool mine = 2 * k + hf < n;
+        const float* kp = nullptr;
+        bool live0 = mine, live1 = mine;
+        if (KP || SUB) {
+          if (!wait_all(pi_full + 8 * (j & 1), (uint32_t)(j >> 1), ERR_MMA_WAIT)) { ok = false; break; }
+          const int* x = info + 4 * (j & 1);
+          const int f = x[0];
+          // blocks without padded keys (most of them) take no penalty
+          if (KP && ((f >> hf) & 1)) kp = kpu + x[1 + hf] * BS;
+          if (SUB) {
+            const int bits = (f >> (8 + 8 * hf + (q >> 1) * 2)) & 3;
+            live0 = mine && (bits & 1);
+            live1 = mine && (bits & 2);
+            n_sel += mine ? 32 * __popc(bits) : 0;
+          }
+        }
+        if (!SUB) n_sel += mine ? BS : 0;
+        if (!wait_all(s_ready, (uint32_t)j, ERR_MMA_WAIT)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t v0[32], v1[32];
+        tmem_ld32(lS, v0);
+        tmem_ld32(lS + 32u, v1);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_free);
+        float cm = -INFINITY;
+        if (!kp) {                                                // the scale is positive: compare raw scores
+          float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+#pragma unroll
+          for (int x = 0; x < 32; x += 2) {
+            m0 = fmaxf(m0, __uint_as_float(v0[x]));
+            m1 = fmaxf(m1, __uint_as_float(v0[x + 1]));
+            m2 = fmaxf(m2, __uint_as_float(v1[x]));
+            m3 = fmaxf(m3, __uint_as_float(v1[x + 1]));
+          }
+          if (live0) cm = fmaxf(m0, m1) * sc2;
+          if (live1) cm = fmaxf(cm, fmaxf(m2, m3) * sc2);
+        } else {
+#pragma unroll
+          for (int x = 0; x < 32; ++x) {
+            if (live0) cm = fmaxf(cm, fmaf(__uint_as_float(v0[x]), sc2, -kp[x] * LOG2E));
+            if (live1) cm = fmaxf(cm, fmaf(__uint_as_float(v1[x]), sc2, -kp[32 + x] * LOG2E));
+          }
+        }
+        cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 16));     // both owners of a row agree
+        mx = fmaxf(mx, cm);
+        if (k == 0) {
+          m = mx;
+        } else if (__any_sync(0xffffffffu, mx > m + MOVE)) {      // rare: move the reference, rescale what has been summed
+          const float m_new = mx > m + MOVE ? mx : m, f = exp2f(m - m_new);
+          l *= f;
+          m = m_new;
+          if (!wait_all(pv_done + 8 * ((j - 1) & 1), (uint32_t)((j - 1) >> 1), ERR_MMA2_WAIT)) { ok = false; break; }
+          tc_fence_after();
+#pragma unroll 1
+          for (int h = 0; h < D; h += 8) {
+            uint32_t o[8];
+            tmem_ld8(lO + h, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int x = 0; x < 8; ++x) o[x] = __float_as_uint(__uint_as_float(o[x]) * f);
+            tmem_st8(lO + h, o);
+          }
+          tmem_st_wait();
+        }
+        // the P tiles of pair j - 2 have been consumed
+        if (j >= 2 && !wait_all(pv_done + 8 * (j & 1), (uint32_t)(j >> 1) - 1u, ERR_MMA2_WAIT)) { ok = false; break; }
+        const uint32_t tile = gb + C::O_P + (j & 1) * C::PB + hf * VT_BYTES + row * 128;
+        float la = 0.f, lb = 0.f;
+        auto half_row = [&](const uint32_t (&v)[32], int g, bool live) {
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) {                        // eight columns: one 16-byte piece of the tile row
+            uint32_t w[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              const int c = cc * 8 + 2 * x;
+              float h0 = m, h1 = m;
+              if (KP && kp) { h0 = fmaf(kp[g * 32 + c], LOG2E, m); h1 = fmaf(kp[g * 32 + c + 1], LOG2E, m); }
+              const float e0 = ex2_approx(fmaf(__uint_as_float(v[c]), sc2, -h0)), e1 = ex2_approx(fmaf(__uint_as_float(v[c + 1]), sc2, -h1));
+              if (!SUB || live) { la += e0; lb += e1; }
+              w[x] = !SUB || live ? pack_bf16(e0, e1) : 0u;
+            }
+            st_shared_v4(tile + (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4), w);
+          }
+        };
+        if (mine) {
+          half_row(v0, 0, live0);
+          half_row(v1, 1, live1);
+          l += la + lb;
+        }
+        fence_proxy_async();                                      // P rows -> visible to the MMA
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_ready + 8 * (j & 1));
+        if (pend) ok = flush();                                   // the previous unit: its last product has long been issued
+      }
+      if (!ok) break;
+      n_sel += __shfl_xor_sync(0xffffffffu, n_sel, 16);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+      const float f = exp2f(m - mx), z = l * f + (float)(a.L - n_sel) * exp2f(-mx);
+      if (hf == 0) *lse = mx + log2f(z);
+      pend = true; pend_par = par; pend_j = j - 1; pend_inv = f / z; pend_dst = dst;
+    }
+    if (ok && pend) flush();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512u);
+}
+
+}  // namespace
+
+namespace tc {
+
+template <int D, bool KP, bool SUB>
+static int fs_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FsArgs& a) {
+  using C = Fs<D>;
+  static_assert(C::SMEM <= 227 * 1024 && NG * C::COLS <= 512, "shared or tensor memory");
+  auto k = k_fwd_stream<D, KP, SUB>;
+  static bool set[64] = {false};
+  if (c->device >= 64 || !set[c->device]) {
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+    if (c->device < 64) set[c->device] = true;
+  }
+  const long long total = (long long)c->BH * a.nb;
+  const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
+  k<<<grid, FS_THREADS, C::SMEM, c->stream>>>(mq, mk, mv, a);
+  SPION_LAUNCH_CHECK();
+  c->launches += 1;
+  return SPION_OK;
+}
+
+template <int D>
+static int fs_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad,
+                      void* O, float* lse) {
+  const TcView vw = tc_view(c, s);
+  FsArgs a;
+  a.O = (__nv_bfloat16*)O; a.lse = lse; a.keypad = keypad;
+  a.rec = s->line_rec + SPION_MAX_NB; a.pair = s->line_pair + s->line_pair_cap;
+  a.submask = vw.submask;
+  a.L = c->L; a.BH = c->BH; a.nb = vw.nb; a.heads = c->heads; a.by_rank = order_by_rank(c);
+  a.scale = c->scale; a.floor_v = keypad ? 0.0f : -100.0f; a.status = c->status_dev;
+  if (keypad) return vw.submask ? fs_launch<D, true, true>(c, s, mq, mk, mv, a) : fs_launch<D, true, false>(c, s, mq, mk, mv, a);
+  return vw.submask ? fs_launch<D, false, true>(c, s, mq, mk, mv, a) : fs_launch<D, false, false>(c, s, mq, mk, mv, a);
+}
+
+int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
+                   float* lse) {
+  return c->d == 64 ? fs_forward<64>(c, s, mq, mk, mv, keypad, O, lse) : fs_forward<32>(c, s, mq, mk, mv, keypad, O, lse);
+}
+
+}  // namespace tc

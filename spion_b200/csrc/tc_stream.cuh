@@ -1,0 +1,69 @@
+// What the streaming kernels (tc_fwd_stream.cu, tc_bwd_stream.cu) share: the order in which a CTA walks its lines (block rows or
+// block columns) and the pairs of entries of a line.
+#pragma once
+#include "tc_tiles.cuh"
+
+namespace tc {
+
+// Unit ordinal -> (b,h) matrix and rank of its line.  by_rank: the longest lines of all matrices first (even shares of long and
+// short lines); else matrix by matrix, so that tiles shared by the lines of a matrix stay in L2, the lines rotated from matrix to
+// matrix so that no CTA meets the long ones every time.
+struct UnitMap {
+  int nb, BH, by_rank;
+  __device__ __forceinline__ void at(int u, int& bh, int& rank) const {
+    if (by_rank) { rank = u / BH; bh = u - rank * BH; }
+    else { bh = u / nb; rank = u - bh * nb + bh % nb; if (rank >= nb) rank -= nb; }
+  }
+};
+// The streamed matrices of all (b,h) pairs stay in L2 (126 MB) whatever the order of the lines; beyond that the order has to keep the
+// lines of one matrix together.
+inline int order_by_rank(const spion_ctx* c) { return (size_t)2 * c->BH * c->L * c->d * 2 <= (size_t)80 << 20; }
+
+// A walk over units first, first + step, ... < total: unit ordinal i, pair k of its line.  The record of the next unit is requested a
+// unit early.  rec[rank] = {line, first pair, pairs, entries}.
+struct Walk {
+  UnitMap um;
+  const int4* rec;
+  int first, step, n_my;                              // units of this walk
+  int i, k, bh, bh_n;
+  int4 cur, nxt;
+  __device__ __forceinline__ int4 record(int x, int& b) const {
+    if (x >= n_my) { b = 0; return make_int4(0, 0, 0, 0); }
+    int rank;
+    um.at(first + x * step, b, rank);
+    return rec[rank];
+  }
+  __device__ __forceinline__ void init(const UnitMap& m, const int4* r, int f, int s, int total) {
+    um = m; rec = r; first = f; step = s;
+    n_my = total > f ? (total - f + s - 1) / s : 0;
+    i = 0; k = 0;
+    cur = record(0, bh);
+    nxt = record(1, bh_n);
+  }
+  __device__ __forceinline__ bool valid() const { return i < n_my; }
+  __device__ __forceinline__ int pairs() const { return cur.z; }
+  __device__ __forceinline__ int cnt() const { return min(2, cur.w - 2 * k); }          // entries of pair k
+  __device__ __forceinline__ bool last() const { return k + 1 == cur.z; }
+  __device__ __forceinline__ void shift() { ++i; k = 0; cur = nxt; bh = bh_n; nxt = record(i + 1, bh_n); }
+  __device__ __forceinline__ void skip() { while (i < n_my && cur.w == 0) shift(); }      // lines without entries
+  __device__ __forceinline__ void next() { if (++k >= cur.z) { shift(); skip(); } }
+};
+
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t (&w)[4]) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+
+// Padded keys in a block (the penalties of its 64 keys)?  Half a warp, four keys per lane; the result is this lane's own four.
+__device__ __forceinline__ bool pad4(const float* kp) {
+  bool v = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v |= kp[(threadIdx.x & 15) + 16 * i] != 0.f;
+  return v;
+}
+
+}  // namespace tc

@@ -149,17 +149,16 @@ struct TcState {
   EncodeTiledFn encode = nullptr;
   int sms = 0;                  // multiprocessors of the context's device
   int fwd_ctas = 0, row_ctas = 0, col_ctas = 0;   // resident CTAs per SM of the persistent kernels
-  int rc_row_ctas = 0;                            // ... of the recompute row kernel (the column kernel: one per SM)
   int pipe_ctas = 0;                              // ... of the pipelined forward for short rows
   int n_long = 0;               // block rows with more than ROW_NCH blocks: the first n_long records of row_info
   int* n_long_dev = nullptr;
   float* delta_ws = nullptr;    // [BH*L] delta_i = sum_n dO_in O_in, written by the row kernel, read by the column kernel
   float* lse_ws = nullptr;      // [BH*L] log-sum-exp workspace for the calls that do not expose it
   int* col_order = nullptr;     // block columns from the longest to the shortest
-  // the same columns as records for the streaming column kernel: one load per column / per pair of entries
-  int4* col_rec = nullptr;      // [nb] in col_order: {block column, first pair, pairs, entries}
-  int4* col_pair = nullptr;     // [sum of pairs] {block row of entry 0, of entry 1 (-1: none), CSR block id 0, 1}
-  size_t col_pair_cap = 0;
+  // lines as records for the streaming kernels: block columns, then block rows from SPION_MAX_NB on
+  int4* line_rec = nullptr;     // {line, first pair, pairs, entries}, the longest lines first
+  int4* line_pair = nullptr;    // {other line of entry 0, of entry 1 (-1: none), CSR block ids}; the rows' pairs from line_pair_cap on
+  size_t line_pair_cap = 0;
   int4* row_info = nullptr;     // per block row: {row_ptr, blocks, col0 | col1 << 16, col2 | col3 << 16}: one load instead of two dependent ones
   // 32-wide masks run on 64-wide super-blocks: derived structure + which 32x32 quarters are selected
   bool super = false;
@@ -243,17 +242,18 @@ inline int make_operand_map(const spion_ctx* c, TcState* s, CUtensorMap* m, cons
   return make_map(s, m, base, (uint64_t)(c->BH / c->heads) * c->L, (uint32_t)(c->heads * D), (uint32_t)D, BS);
 }
 
-// tc_recompute_col.cu: streaming column kernel of the recompute backward (reads the context's delta array)
-int col_stream_set_attrs(int d);
-int col_stream_backward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                        const CUtensorMap& mdo, const float* lse, const float* keypad, void* dK, void* dV);
-
-// tc_recompute.cu
-int recompute_set_attrs(TcState* s, int d, int device);
+// tc_bwd_stream.cu
+int stream_prepare(spion_ctx* c, TcState* s);              // pattern set: line and pair records of the streaming kernels
 int recompute_backward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const void* O,
                        const void* dO, const float* lse, const float* keypad, void* dQ, void* dK, void* dV);
+// tc_recompute.cu
+int mean_map_set_attrs(int d);
 int recompute_mean_map(spion_ctx* c, TcState* s, const void* Q, const void* K, const float* lse, const float* keypad,
                        float* A);
+
+// tc_fwd_stream.cu: forward without stored probabilities
+int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
+                   float* lse);
 
 // tc_fwd_pipe.cu: forward of the records [rank0, nb) of row_info (rows of at most ROW_NCH blocks)
 int pipe_set_attrs(TcState* s, int d, int device);
