@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
     const int row = SIDE == COL ? (q & 1) * 32 + lane : q * 16 + (lane & 15);
     const int orow = q * 16 + (lane & 15);                            // output row (64-row accumulators)
     const uint32_t t_lane = tmem + ((uint32_t)(q * 32) << 16);
-    const float sc2 = a.scale * LOG2E;
+    const float sc2 = a.scale * LOG2E, inv_scale = 1.0f / a.scale;
     bool ok = true;
     bool pend = false;                                                // a finished unit whose rows this group has to write
     int pend_par = 0, pend_phase = 0;
@@ -449,35 +449,28 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         tmem_ld32(ts + 64u, gv);
         tmem_ld_wait();
         if (mine) {
+          if (kp) take_penalty(sv, kp, inv_scale);
           const uint32_t tds = sbase + C::O_PD + grp * C::PD + es * VT_BYTES + row * 128, tp = tds + 2 * VT_BYTES;
-          auto piece = [&](int cc, const float (&o)[8]) {             // eight columns: one 16-byte piece of each tile
+          const uint64_t sc22 = pack2(sc2, sc2), scale2 = pack2(a.scale, a.scale), nds2 = pack2(nds, nds), nh2 = pack2(-h, -h);
+          auto piece = [&](int cc) {             // eight columns: one 16-byte piece of each tile
             uint32_t wp[4], wd[4];
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
               const int e = cc * 8 + 2 * x;
-              const float p0 = ex2_approx(fmaf(__uint_as_float(sv[e]), sc2, o[2 * x])), p1 = ex2_approx(fmaf(__uint_as_float(sv[e + 1]), sc2, o[2 * x + 1]));
+              float p0, p1, d0, d1;
+              unpack2(fma2(pack2(sv[e], sv[e + 1]), sc22, nh2), p0, p1);
+              p0 = ex2_approx(p0); p1 = ex2_approx(p1);
               wp[x] = pack_bf16(p0, p1);
-              wd[x] = pack_bf16(p0 * fmaf(__uint_as_float(gv[e]), a.scale, nds), p1 * fmaf(__uint_as_float(gv[e + 1]), a.scale, nds));
+              unpack2(mul2(pack2(p0, p1), fma2(pack2(gv[e], gv[e + 1]), scale2, nds2)), d0, d1);
+              wd[x] = pack_bf16(d0, d1);
               if (SUB && !live) { wp[x] = 0u; wd[x] = 0u; }
             }
             const uint32_t off = (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4);
             st_shared_v4(tds + off, wd);
             if (SIDE == COL) st_shared_v4(tp + off, wp);
           };
-          if (!kp) {
-            const float nh = -h;
-            const float o[8] = {nh, nh, nh, nh, nh, nh, nh, nh};
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) piece(cc, o);
-          } else {
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-              float o[8];
-#pragma unroll
-              for (int x = 0; x < 8; ++x) o[x] = -fmaf(kp[cc * 8 + x], LOG2E, h);
-              piece(cc, o);
-            }
-          }
+          for (int cc = 0; cc < 4; ++cc) piece(cc);
         }
         tc_fence_before();
         fence_proxy_async();                                          // tiles -> visible to the MMAs

@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
     // ================================================================== arithmetic warps of a group
     const int q = warp & 3, hf = lane >> 4, row = q * 16 + (lane & 15);
     const uint32_t lS = tS + ((uint32_t)(q * 32) << 16), lO = tO + ((uint32_t)(q * 32) << 16);
-    const float sc2 = a.scale * LOG2E, floor2 = a.floor_v * LOG2E;
+    const float sc2 = a.scale * LOG2E, floor2 = a.floor_v * LOG2E, inv_scale = 1.0f / a.scale;
     bool ok = true;
     // the finished unit whose rows are still in tensor memory
     bool pend = false;
@@ -312,24 +312,22 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_free);
+        if (KP && kp) {
+          take_penalty(v0, kp, inv_scale);
+          take_penalty(v1, kp + 32, inv_scale);
+        }
         float cm = -INFINITY;
-        if (!kp) {                                                // the scale is positive: compare raw scores
+        {                                                         // the scale is positive: compare raw scores
           float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) {
-            m0 = fmaxf(m0, __uint_as_float(v0[x]));
-            m1 = fmaxf(m1, __uint_as_float(v0[x + 1]));
-            m2 = fmaxf(m2, __uint_as_float(v1[x]));
-            m3 = fmaxf(m3, __uint_as_float(v1[x + 1]));
+          for (int x = 0; x < 32; x += 4) {
+            m0 = max3(m0, __uint_as_float(v0[x]), __uint_as_float(v0[x + 1]));
+            m1 = max3(m1, __uint_as_float(v0[x + 2]), __uint_as_float(v0[x + 3]));
+            m2 = max3(m2, __uint_as_float(v1[x]), __uint_as_float(v1[x + 1]));
+            m3 = max3(m3, __uint_as_float(v1[x + 2]), __uint_as_float(v1[x + 3]));
           }
           if (live0) cm = fmaxf(m0, m1) * sc2;
           if (live1) cm = fmaxf(cm, fmaxf(m2, m3) * sc2);
-        } else {
-#pragma unroll
-          for (int x = 0; x < 32; ++x) {
-            if (live0) cm = fmaxf(cm, fmaf(__uint_as_float(v0[x]), sc2, -kp[x] * LOG2E));
-            if (live1) cm = fmaxf(cm, fmaf(__uint_as_float(v1[x]), sc2, -kp[32 + x] * LOG2E));
-          }
         }
         cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 16));     // both owners of a row agree
         mx = fmaxf(mx, cm);
@@ -355,7 +353,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         // the P tiles of pair j - 2 have been consumed
         if (j >= 2 && !wait_all(pv_done + 8 * (j & 1), (uint32_t)(j >> 1) - 1u, ERR_MMA2_WAIT)) { ok = false; break; }
         const uint32_t tile = gb + C::O_P + (j & 1) * C::PB + hf * VT_BYTES + row * 128;
-        float la = 0.f, lb = 0.f;
+        uint64_t l2 = 0ull;
+        const uint64_t sc22 = pack2(sc2, sc2), nm2 = pack2(-m, -m);
         auto half_row = [&](const uint32_t (&v)[32], int g, bool live) {
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) {                        // eight columns: one 16-byte piece of the tile row
@@ -363,10 +362,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
               const int c = cc * 8 + 2 * x;
-              float h0 = m, h1 = m;
-              if (KP && kp) { h0 = fmaf(kp[g * 32 + c], LOG2E, m); h1 = fmaf(kp[g * 32 + c + 1], LOG2E, m); }
-              const float e0 = ex2_approx(fmaf(__uint_as_float(v[c]), sc2, -h0)), e1 = ex2_approx(fmaf(__uint_as_float(v[c + 1]), sc2, -h1));
-              if (!SUB || live) { la += e0; lb += e1; }
+              float e0, e1;
+              unpack2(fma2(pack2(v[c], v[c + 1]), sc22, nm2), e0, e1);
+              e0 = ex2_approx(e0); e1 = ex2_approx(e1);
+              if (!SUB || live) l2 = add2(l2, pack2(e0, e1));
               w[x] = !SUB || live ? pack_bf16(e0, e1) : 0u;
             }
             st_shared_v4(tile + (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4), w);
@@ -375,6 +374,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         if (mine) {
           half_row(v0, 0, live0);
           half_row(v1, 1, live1);
+          float la, lb;
+          unpack2(l2, la, lb);
           l += la + lb;
         }
         fence_proxy_async();                                      // P rows -> visible to the MMA

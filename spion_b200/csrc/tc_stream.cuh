@@ -54,8 +54,43 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Two fp32 values per instruction, each rounded as fmaf / + would; three-way maximum.
+__device__ __forceinline__ uint64_t pack2(uint32_t a, uint32_t b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) { return pack2(__float_as_uint(a), __float_as_uint(b)); }
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t (&w)[4]) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+
+// Raw scores of 32 keys with their penalties: (s - pad / scale) scale = s scale - pad.  Done in place, in the few blocks that have
+// padded keys, so that the arithmetic behind it has one form only (two forms cost 20 % of the forward in registers).
+__device__ __forceinline__ void take_penalty(uint32_t (&s)[32], const float* kp, float inv_scale) {
+#pragma unroll
+  for (int x = 0; x < 32; ++x) s[x] = __float_as_uint(fmaf(kp[x], -inv_scale, __uint_as_float(s[x])));
 }
 
 // Padded keys in a block (the penalties of its 64 keys)?  Half a warp, four keys per lane; the result is this lane's own four.
