@@ -174,7 +174,8 @@ int operand_form(const Context& c, const Tensor& t) {
   return -1;
 }
 
-void attn_forward(const Context& c, Attn& a, void* st) {
+// need: a backward may follow
+void attn_forward(const Context& c, Attn& a, bool need, void* st) {
   spion_ctx* x = c.ctx();
   const auto f32 = a.q.options().dtype(at::kFloat);
   check(spion_set_stream(x, st), "spion_set_stream");
@@ -197,8 +198,8 @@ void attn_forward(const Context& c, Attn& a, void* st) {
   a.O = empty_operand(c, a.heads, a.q);
   if (c.fused) {
     a.lse = at::empty({c.B * c.H * c.L}, f32);
-    // the probabilities are stored only for callers that want them back; the backward rebuilds its tiles
-    if (c.return_probs || !c.recompute) a.P = at::empty({c.B * c.H * c.nnz}, a.q.options());
+    // the probabilities are stored only for callers that want them back and for a backward that reads them
+    if (c.return_probs || (need && !c.recompute)) a.P = at::empty({c.B * c.H * c.nnz}, a.q.options());
     check(spion_attn_forward_fused(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.O), (float*)a.lse.data_ptr(), p(a.P)),
           "spion_attn_forward_fused");
   } else {
@@ -298,7 +299,7 @@ py::tuple attention(const ContextPtr& c, const Tensor& query, const Tensor& key,
     // head-split views of [B, L, H*d] projections are read where they lie; anything else is packed
     if (c->fused && operand_form(*c, a.q) == c->H && operand_form(*c, a.k) == c->H && operand_form(*c, a.v) == c->H) a.heads = (int)c->H;
     if (!a.heads) { a.q = a.q.contiguous(); a.k = a.k.contiguous(); a.v = a.v.contiguous(); }
-    attn_forward(*c, a, st);
+    attn_forward(*c, a, need, st);
   }
   Tensor out = a.O;
   if (need) {
@@ -424,7 +425,7 @@ py::tuple attention_layer(const ContextPtr& c, const Tensor& x, const optional<T
     Weights qkv{{W[0].detach(), W[1].detach(), W[2].detach()}, {b[0].detach(), b[1].detach(), b[2].detach()}};
     Weights ff{{W[3].detach()}, {b[3].detach()}};
     linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st);
-    attn_forward(*c, a, st);
+    attn_forward(*c, a, need, st);
     out = at::empty({c->B, c->L, ff.out()}, opt);
     linear_forward(form({a.O}), ff, fp32, tok({out}, ff.out()), nullptr, T, st);
   }

@@ -72,9 +72,7 @@ class BlockSparseAttention(nn.Module):
         self.return_probs = bool(return_probs) or not self.fused
         # recompute=True (fused kernels): the backward rebuilds P and dS on chip from the log-sum-exp and nothing
         # of size nnz exists in memory; False: the forward stores P, the backward reads it and writes dS
-        # (spion_attn_backward_ex).  None: chosen per mask in set_mask -- recompute for 32-wide blocks (no tile
-        # conversion passes: measured 6 - 25 % faster) and for the full mask of the warm-up phase (equal speed,
-        # 2 * BH * L^2 elements less memory); stored tiles for sparse 64-wide masks (measured 10 - 15 % faster).
+        # (spion_attn_backward_ex).  None: chosen per mask in set_mask.
         self._recompute_arg = recompute
         self.recompute = self.fused and (recompute is None or bool(recompute))
         self.last = None
@@ -117,8 +115,7 @@ class BlockSparseAttention(nn.Module):
         check(lib.spion_set_pattern(self.handle, ptr(m8)), "spion_set_pattern")
         self.nnzb = int(lib.spion_pattern_nnzb(self.handle))
         if self.fused and self._recompute_arg is None:
-            nb = self.L // self.bs
-            self.recompute = self.bs == 32 or self.nnzb == nb * nb
+            self.recompute = self._recompute_pays()
         from .pattern import pattern_from_mask
         self._pattern = pattern_from_mask(m8, self.bs)          # block CSR for the helpers above
         # The key names the tensor by address and version; the tensor itself is kept alive so that the
@@ -127,6 +124,24 @@ class BlockSparseAttention(nn.Module):
         self._mask_ref, self._mask_version = mat, mat._version
         self._ctx.nnz = self.nnz
         return self.nnzb
+
+    def _recompute_pays(self) -> bool:
+        """Which backward serves the current mask (forward + backward, 64 matrices unless stated, one B200):
+
+        * 32-wide blocks and the full mask: rebuilt tiles (no conversion passes; 2 * BH * L^2 elements less memory);
+        * a caller that wants P back: stored tiles, the forward writes them anyway (L = 4096, 5 %: 227 us; rebuilt 242);
+        * rows of three blocks or more: rebuilt (L = 4096, 5 %: 217 us, stored 227; 30 %: 607, 906; L = 16384, 5 %: 1650, 2610);
+          shorter rows: stored (L = 1024, two blocks per row: 66 us, rebuilt 69);
+        * head_dim 32 with fewer than 2^15 selected blocks in all matrices: stored.  The rebuilt tiles are 20 % faster there too
+          (32 matrices, L = 4096, 10 %: 152 against 196 us), but P is normalised before and not after it is rounded to bf16: a
+          training step of the encoder classifier repeats bit for bit only on the path it has always had.  At 256 matrices
+          (1013 against 1413 us) the layer, not the step around it, is what counts."""
+        nb = self.L // self.bs
+        if self.bs == 32 or self.nnzb == nb * nb:
+            return True
+        if self.return_probs or self.nnzb < 3 * nb:
+            return False
+        return self.d == 64 or self.BH * self.nnzb >= 1 << 15
 
     @property
     def nnz(self) -> int:
