@@ -348,12 +348,15 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         }
 #pragma unroll
         for (int x = 0; x < UN; ++x) {
-          float t = bf16_lo(u[x].x) * bf16_lo(v[x].x) + bf16_hi(u[x].x) * bf16_hi(v[x].x) + bf16_lo(u[x].y) * bf16_lo(v[x].y) +
-                    bf16_hi(u[x].y) * bf16_hi(v[x].y) + bf16_lo(u[x].z) * bf16_lo(v[x].z) + bf16_hi(u[x].z) * bf16_hi(v[x].z) +
-                    bf16_lo(u[x].w) * bf16_lo(v[x].w) + bf16_hi(u[x].w) * bf16_hi(v[x].w);
+          const float t = bf16_lo(u[x].x) * bf16_lo(v[x].x) + bf16_hi(u[x].x) * bf16_hi(v[x].x) + bf16_lo(u[x].y) * bf16_lo(v[x].y) +
+                          bf16_hi(u[x].y) * bf16_hi(v[x].y) + bf16_lo(u[x].z) * bf16_lo(v[x].z) + bf16_hi(u[x].z) * bf16_hi(v[x].z) +
+                          bf16_lo(u[x].w) * bf16_lo(v[x].w) + bf16_hi(u[x].w) * bf16_hi(v[x].w);
+          // half of the head dimension in order, then the two halves: as the row kernel of the stored path adds them
+          float half = __shfl_sync(0xffffffffu, t, lane & ~(LPR / 2 - 1));
 #pragma unroll
-          for (int o = 1; o < LPR; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-          if (lane % LPR == 0 && i0 + x < c.n_my && r0 < BS) a.delta_out[ri[x]] = t;
+          for (int y = 1; y < LPR / 2; ++y) half += __shfl_sync(0xffffffffu, t, (lane & ~(LPR / 2 - 1)) + y);
+          const float d = half + __shfl_xor_sync(0xffffffffu, half, LPR / 2);
+          if (lane % LPR == 0 && i0 + x < c.n_my && r0 < BS) a.delta_out[ri[x]] = d;
         }
       }
       __threadfence_block();
@@ -512,10 +515,10 @@ __global__ void k_line_recs(const int32_t* __restrict__ ptr, const int32_t* __re
     for (int x = 0; x < nb; ++x) { s_first[x] = acc; acc += (s_n[s_order[x]] + 1) >> 1; }
   }
   __syncthreads();
-  for (int x = threadIdx.x; x < nb; x += blockDim.x) {
+  for (int x = threadIdx.x >> 5; x < nb; x += blockDim.x >> 5) {
     const int c = s_order[x], beg = ptr[c], n = s_n[c], np = (n + 1) >> 1;
-    rec[x] = make_int4(c, s_first[x], np, n);
-    for (int k = 0; k < np; ++k) {
+    if ((threadIdx.x & 31) == 0) rec[x] = make_int4(c, s_first[x], np, n);
+    for (int k = threadIdx.x & 31; k < np; k += 32) {
       const int e0 = beg + 2 * k;
       const bool two = 2 * k + 1 < n;
       pair[s_first[x] + k] = make_int4(idx[e0], two ? idx[e0 + 1] : -1, pos ? pos[e0] : e0, two ? (pos ? pos[e0 + 1] : e0 + 1) : 0);

@@ -25,6 +25,8 @@
 // status word, frees its TMEM and returns.
 #include <cuda.h>
 
+#include <mutex>
+
 #include "common.cuh"
 #include "tc_tiles.cuh"
 
@@ -746,6 +748,32 @@ bool tc_engine_supports(const spion_ctx* c) {
          (unsigned long long)c->BH * c->L < 0x7fffffffULL;
 }
 
+// Shared-memory opt-ins and resident CTAs of all kernels, once per device and head dimension of the process (about 60 attribute
+// calls, a millisecond: every layer of a model has a context of its own).
+static int kernel_attrs(spion_ctx* c, TcState* s) {
+  struct Known { bool have = false; int fwd, row, col, pipe, b32[3]; };
+  static std::mutex mutex;
+  static Known known[64][2][2];                                    // device, head dimension, 32-wide blocks
+  const bool b32 = b32_applies(c);
+  std::lock_guard<std::mutex> lock(mutex);
+  Known fresh, *k = c->device < 64 ? &known[c->device][c->d == 64][b32] : &fresh;
+  if (!k->have) {
+    int rc = (c->d == 64) ? set_attrs<64>(s, c->device) : set_attrs<32>(s, c->device);
+    if (!rc) rc = fused_set_attrs(s, c->d, c->device);
+    if (!rc) rc = mean_map_set_attrs(c->d);
+    if (!rc) rc = pipe_set_attrs(s, c->d, c->device);
+    if (!rc && b32) rc = b32_set_attrs(s, c->device);
+    if (rc) return rc;
+    k->fwd = s->fwd_ctas; k->row = s->row_ctas; k->col = s->col_ctas; k->pipe = s->pipe_ctas;
+    for (int i = 0; i < 3; ++i) k->b32[i] = s->b32_ctas[i];
+    k->have = true;
+  }
+  s->fwd_ctas = k->fwd; s->row_ctas = k->row; s->col_ctas = k->col; s->pipe_ctas = k->pipe;
+  for (int i = 0; i < 3; ++i) s->b32_ctas[i] = k->b32[i];
+  s->b32 = b32;
+  return SPION_OK;
+}
+
 int tc_engine_prepare(spion_ctx* c) {
   TcState* s = (TcState*)c->tc;
   if (!s) {
@@ -763,11 +791,7 @@ int tc_engine_prepare(spion_ctx* c) {
       delete s;
       return SPION_ERR_CUDA;
     }
-    int rc = (c->d == 64) ? set_attrs<64>(s, c->device) : set_attrs<32>(s, c->device);
-    if (!rc) rc = fused_set_attrs(s, c->d, c->device);
-    if (!rc) rc = mean_map_set_attrs(c->d);
-    if (!rc) rc = pipe_set_attrs(s, c->d, c->device);
-    if (!rc && b32_applies(c)) { rc = b32_set_attrs(s, c->device); s->b32 = rc == SPION_OK; }
+    int rc = kernel_attrs(c, s);
     if (!rc && cudaMalloc(&s->delta_ws, (size_t)c->BH * c->L * sizeof(float)) != cudaSuccess) rc = SPION_ERR_ALLOC;
     if (!rc && cudaMalloc(&s->lse_ws, (size_t)c->BH * c->L * sizeof(float)) != cudaSuccess) rc = SPION_ERR_ALLOC;
     if (rc) { delete s; return rc; }

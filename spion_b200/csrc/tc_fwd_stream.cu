@@ -61,7 +61,10 @@ struct FsArgs {
   int* status;
 };
 
-template <int D, bool KP, bool SUB>
+// EXACT: two passes over a row, the maximum first, and the sums in the order of tc_fused.cu: O and lse bit for bit as that kernel
+// gives them.  For the full mask, where some results are sums that cancel to nothing but rounding (the gradient of the key
+// projection's bias is zero in dense attention), so that every other order of the additions gives other numbers.
+template <int D, bool KP, bool SUB, bool EXACT>
 __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ FsArgs a) {
   using C = Fs<D>;
@@ -117,6 +120,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
     ld = c;
     int4 pr = ld.valid() ? a.pair[ld.cur.y] : make_int4(0, -1, 0, 0);      // record of the pair whose K tiles are loaded next
     int4 prv = pr;                                                // ... whose V tiles are loaded next
+    bool c_val = !EXACT, ld_val = !EXACT, p_val = false;          // pair of the value pass: c, ld, the pair before c
     bool pad_l = false;
     uint8_t sub_l = 0xff;
     auto flags_load = [&](const Walk& w, const int4& p) {         // requested with the pair's K tiles, used a pair later
@@ -128,13 +132,14 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       const uint32_t bar = k_full + 8 * (C::ALIAS ? (j & 1) : 0), dst = gb + (C::ALIAS ? C::O_P + (j & 1) * C::PB : C::O_K);
       const int cnt = ld.cnt();
       const OpPos pos = op_pos(ld.bh, a.L, a.heads, D);
+      const bool with_q = ld.k == 0 && (!EXACT || !ld_val);
       if (lane == 0) {
         mbar_expect_tx(bar, cnt * T::BYTES);
-        if (ld.k == 0) mbar_expect_tx(q_full, T::BYTES);
+        if (with_q) mbar_expect_tx(q_full, T::BYTES);
       }
       __syncwarp();
       if (lane < cnt) tma_load_2d(dst + lane * T::BYTES, &tmK, bar, pos.x0, pos.row0 + (lane ? pr.y : pr.x) * BS);
-      if (lane == 4 && ld.k == 0) tma_load_2d(gb + C::O_Q, &tmQ, q_full, pos.x0, pos.row0 + ld.cur.x * BS);
+      if (lane == 4 && with_q) tma_load_2d(gb + C::O_Q, &tmQ, q_full, pos.x0, pos.row0 + ld.cur.x * BS);
     };
     auto load_v = [&](const Walk& w) {
       const int cnt = w.cnt();
@@ -143,14 +148,21 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       __syncwarp();
       if (lane < cnt) tma_load_2d(gb + C::O_V + lane * T::BYTES, &tmV, v_full, pos.x0, pos.row0 + (lane ? prv.y : prv.x) * BS);
     };
+    // EXACT: the pairs of a unit come twice, for the maximum and for the values
+    auto step_on = [&](Walk& w, bool& values) {
+      if (EXACT && w.last() && !values) { values = true; w.k = 0; return; }
+      const bool end = w.last();
+      w.next();
+      if (EXACT && end) values = false;
+    };
     bool ok = true;
-    int units = 0;                                                // units begun
+    int units = 0, jv = 0;                                        // units begun; value pairs before pair j
     if (c.valid()) {
       flags_load(ld, pr);
       load_k(0);
       prv = pr;
-      load_v(ld);
-      ld.next();
+      if (ld_val) load_v(ld);
+      step_on(ld, ld_val);
       if (ld.valid()) pr = a.pair[ld.cur.y + ld.k];
     }
     int p_cnt = 0, p_par = 0;                                     // the pair before c
@@ -171,7 +183,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         }
         // S of pair j
         const int kb = C::ALIAS ? (j & 1) : 0, ku = C::ALIAS ? (j >> 1) : j;
-        if (c.k == 0) { if (!wait_all(q_full, (uint32_t)units, ERR_LOAD_WAIT)) { ok = false; break; } ++units; }
+        if (c.k == 0 && (!EXACT || !c_val)) { if (!wait_all(q_full, (uint32_t)units, ERR_LOAD_WAIT)) { ok = false; break; } ++units; }
         if (!wait_all(k_full + 8 * kb, (uint32_t)ku, ERR_LOAD_WAIT)) { ok = false; break; }
         if (j >= 1 && !wait_all(s_free, (uint32_t)(j - 1), ERR_MMA_WAIT)) { ok = false; break; }
         const bool two = warp_uniform(c.cnt() == 2);
@@ -192,12 +204,14 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       if (j >= 1) {                                               // O += P V of pair j - 1
         const int jp = j - 1;
         if (!wait_all(p_ready + 8 * (jp & 1), (uint32_t)(jp >> 1), ERR_MMA_WAIT)) { ok = false; break; }
-        if (!wait_all(v_full, (uint32_t)jp, ERR_LOAD_WAIT)) { ok = false; break; }
-        const bool two = warp_uniform(p_cnt == 2), fresh = warp_uniform((int)p_first) != 0;
+        if (p_val) { if (!wait_all(v_full, (uint32_t)jv, ERR_LOAD_WAIT)) { ok = false; break; } ++jv; }
+        const bool two = warp_uniform(p_cnt == 2), fresh = warp_uniform((int)p_first) != 0, value_pair = warp_uniform((int)p_val) != 0;
         if (elect_one()) {
           tc_fence_after();
           const uint32_t acc = tO + ((uint32_t)(p_par * 16) << 16);
           const uint64_t dP = ValTile::kmajor(gb + C::O_P + (jp & 1) * C::PB, 0), dV = T::mnmajor(gb + C::O_V, 0);
+          if (EXACT && !value_pair) {                             // nothing to multiply: the commit alone says that S has been read
+          } else {
 #pragma unroll
           for (int kk = 0; kk < BS / 16; ++kk)
             mma_bf16(acc, desc_advance(dP, kk * ValTile::K_STEP), desc_advance(dV, kk * T::MN_STEP), IDESC_O, (kk > 0 || !fresh) ? 1u : 0u);
@@ -205,6 +219,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
 #pragma unroll
             for (int kk = 0; kk < BS / 16; ++kk)
               mma_bf16(acc, desc_advance(dP, VT_BYTES + kk * ValTile::K_STEP), desc_advance(dV, T::BYTES + kk * T::MN_STEP), IDESC_O, 1u);
+          }
           }
           mma_commit(pv_done + 8 * (jp & 1));
         }
@@ -215,17 +230,17 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       // pair j - 1), Q and V are free.
       if (j >= 1) {
         if (!wait_all(pv_done + 8 * ((j - 1) & 1), (uint32_t)((j - 1) >> 1), ERR_MMA2_WAIT)) { ok = false; break; }
-        load_v(c);                                                // V of pair j (pair 0's was requested above)
+        if (c_val) load_v(c);                                     // V of pair j (pair 0's was requested above)
       } else if (!wait_all(s_ready, 0u, ERR_MMA_WAIT)) { ok = false; break; }
       if (ld.valid()) {
         flags_load(ld, pr);
         load_k(j + 1);
         prv = pr;
-        ld.next();
+        step_on(ld, ld_val);
         if (ld.valid()) pr = a.pair[ld.cur.y + ld.k];
       }
-      p_cnt = c.cnt(); p_par = c.i & 1; p_first = c.k == 0;
-      c.next();
+      p_cnt = c.cnt(); p_par = c.i & 1; p_first = c.k == 0; p_val = c_val;
+      step_on(c, c_val);
     }
   } else {
     // ================================================================== arithmetic warps of a group
@@ -285,7 +300,9 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       float m = floor2, mx = floor2, l = 0.f;                     // reference exponent, true maximum, sum
       int n_sel = 0;
       const int np = u.pairs();
-      for (int k = 0; k < np && ok; ++k, ++j) {
+      for (int kx = EXACT ? -np : 0; kx < np && ok; ++kx, ++j) {
+        const bool values = !EXACT || kx >= 0;
+        const int k = values ? kx : kx + np;
         const bool mine = 2 * k + hf < n;
         const float* kp = nullptr;
         bool live0 = mine, live1 = mine;
@@ -299,10 +316,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
             const int bits = (f >> (8 + 8 * hf + (q >> 1) * 2)) & 3;
             live0 = mine && (bits & 1);
             live1 = mine && (bits & 2);
-            n_sel += mine ? 32 * __popc(bits) : 0;
+            n_sel += mine && values ? 32 * __popc(bits) : 0;
           }
         }
-        if (!SUB) n_sel += mine ? BS : 0;
+        if (!SUB && values) n_sel += mine ? BS : 0;
         if (!wait_all(s_ready, (uint32_t)j, ERR_MMA_WAIT)) { ok = false; break; }
         tc_fence_after();
         uint32_t v0[32], v1[32];
@@ -317,7 +334,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
           take_penalty(v1, kp + 32, inv_scale);
         }
         float cm = -INFINITY;
-        {                                                         // the scale is positive: compare raw scores
+        if (!EXACT || !values) {                                                         // the scale is positive: compare raw scores
           float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
           for (int x = 0; x < 32; x += 4) {
@@ -331,7 +348,9 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         }
         cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 16));     // both owners of a row agree
         mx = fmaxf(mx, cm);
-        if (k == 0) {
+        if (EXACT) {
+          m = mx;
+        } else if (k == 0) {
           m = mx;
         } else if (__any_sync(0xffffffffu, mx > m + MOVE)) {      // rare: move the reference, rescale what has been summed
           const float m_new = mx > m + MOVE ? mx : m, f = exp2f(m - m_new);
@@ -356,6 +375,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         uint64_t l2 = 0ull;
         const uint64_t sc22 = pack2(sc2, sc2), nm2 = pack2(-m, -m);
         auto half_row = [&](const uint32_t (&v)[32], int g, bool live) {
+          float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) {                        // eight columns: one 16-byte piece of the tile row
             uint32_t w[4];
@@ -365,18 +385,25 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
               float e0, e1;
               unpack2(fma2(pack2(v[c], v[c + 1]), sc22, nm2), e0, e1);
               e0 = ex2_approx(e0); e1 = ex2_approx(e1);
-              if (!SUB || live) l2 = add2(l2, pack2(e0, e1));
+              if (EXACT) {
+                if (!SUB || live) l4[x] += e0 + e1;
+              } else if (!SUB || live) {
+                l2 = add2(l2, pack2(e0, e1));
+              }
               w[x] = !SUB || live ? pack_bf16(e0, e1) : 0u;
             }
             st_shared_v4(tile + (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4), w);
           }
+          if (EXACT && (!SUB || live)) l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
         };
-        if (mine) {
+        if (mine && values) {
           half_row(v0, 0, live0);
           half_row(v1, 1, live1);
-          float la, lb;
-          unpack2(l2, la, lb);
-          l += la + lb;
+          if (!EXACT) {
+            float la, lb;
+            unpack2(l2, la, lb);
+            l += la + lb;
+          }
         }
         fence_proxy_async();                                      // P rows -> visible to the MMA
         tc_fence_before();
@@ -387,7 +414,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       if (!ok) break;
       n_sel += __shfl_xor_sync(0xffffffffu, n_sel, 16);
       l += __shfl_xor_sync(0xffffffffu, l, 16);
-      const float f = exp2f(m - mx), z = l * f + (float)(a.L - n_sel) * exp2f(-mx);
+      const float f = EXACT ? 1.0f : exp2f(m - mx), z = l * f + (float)(a.L - n_sel) * exp2f(-mx);
       if (hf == 0) *lse = mx + log2f(z);
       pend = true; pend_par = par; pend_j = j - 1; pend_inv = f / z; pend_dst = dst;
     }
@@ -402,11 +429,11 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
 
 namespace tc {
 
-template <int D, bool KP, bool SUB>
+template <int D, bool KP, bool SUB, bool EXACT>
 static int fs_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FsArgs& a) {
   using C = Fs<D>;
   static_assert(C::SMEM <= 227 * 1024 && NG * C::COLS <= 512, "shared or tensor memory");
-  auto k = k_fwd_stream<D, KP, SUB>;
+  auto k = k_fwd_stream<D, KP, SUB, EXACT>;
   static bool set[64] = {false};
   if (c->device >= 64 || !set[c->device]) {
     SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
@@ -430,8 +457,10 @@ static int fs_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUt
   a.submask = vw.submask;
   a.L = c->L; a.BH = c->BH; a.nb = vw.nb; a.heads = c->heads; a.by_rank = order_by_rank(c);
   a.scale = c->scale; a.floor_v = keypad ? 0.0f : -100.0f; a.status = c->status_dev;
-  if (keypad) return vw.submask ? fs_launch<D, true, true>(c, s, mq, mk, mv, a) : fs_launch<D, true, false>(c, s, mq, mk, mv, a);
-  return vw.submask ? fs_launch<D, false, true>(c, s, mq, mk, mv, a) : fs_launch<D, false, false>(c, s, mq, mk, mv, a);
+  if (c->nnzb == c->nb * c->nb)                                   // the full mask has no unselected quarters
+    return keypad ? fs_launch<D, true, false, true>(c, s, mq, mk, mv, a) : fs_launch<D, false, false, true>(c, s, mq, mk, mv, a);
+  if (keypad) return vw.submask ? fs_launch<D, true, true, false>(c, s, mq, mk, mv, a) : fs_launch<D, true, false, false>(c, s, mq, mk, mv, a);
+  return vw.submask ? fs_launch<D, false, true, false>(c, s, mq, mk, mv, a) : fs_launch<D, false, false, false>(c, s, mq, mk, mv, a);
 }
 
 int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
