@@ -237,6 +237,15 @@ int spion_discover_pattern(const float* A, int L, int block_size, int conv_kind,
                            int32_t* col_ptr, int32_t* row_idx, int32_t* csc_pos,
                            int32_t* work, int32_t* host_nnzb, void* cuda_stream);
 
+/* The same for the `layers` (1 .. 16) maps of a model in one go: host_A is a host array of device pointers; the arrays of layer l
+ * lie l * nb * nb (row_ptr, col_ptr: l * (nb + 1); thresh, nnzb, host_nnzb: l) entries behind those of layer 0.  mats (may be NULL):
+ * `copies` copies of the [layers, nb, nb] masks as 0/1 floats (the stacked list of main_conv_ff.py:298-299). */
+int spion_discover_patterns(const float* const* host_A, int layers, int L, int block_size, int conv_kind, int F, int select,
+                            double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,
+                            int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
+                            int32_t* row_idx, int32_t* csc_pos, int32_t* work, float* mats, int copies,
+                            int32_t* host_nnzb, void* cuda_stream);
+
 /* Block CSR + CSC of a given 0/1 mask (e.g. one loaded from the reference's pickle,
  * main_inference.py:164-166).  Same outputs as above. */
 int spion_build_structure(const uint8_t* mat, int nb, int32_t* nnzb,

@@ -8,6 +8,7 @@
 // Integer outputs are bit-exact against oracle/pattern.py because the float stages use the
 // same fixed order of fp64 additions (documented at each loop) and the same fused lerp.
 #include "common.cuh"
+#include "structure.cuh"
 
 namespace {
 
@@ -66,85 +67,106 @@ __global__ void __launch_bounds__(256) conv_pool_kernel(const float* __restrict_
 // ((d_k + d_k+1) + d_k+2) + ... in ascending order -- eight independent fp64 chains.  Runs start at
 // i0 = 0, 8, .., j0 = -7 .. BS - 1 (outputs left of the block are skipped).  The pooled rows are padded by one
 // double so that the row sums (one thread per row) do not collide in shared memory.
+// Persistent CTAs, three per SM, over the cells of all maps of the call: while two warps form the row sums of a cell (64 dependent
+// additions), the tile of the next one arrives by cp.async; the total of the row sums is one lane's work beside the next cell's
+// sums.  Tile rows are 16-byte pieces (A 16-byte aligned; a piece is inside or outside the map as a whole), 96 floats from column
+// j - 16 on; taps left or right of a row read its neighbours' values, but only for the skipped outputs.
+// Bound by the fp64 additions of the filter (31 per output, ordered): 62.8 us per L = 4096 map, 63.9 with one CTA per cell.  What
+// the loop over maps saves is a launch and a wave's tail per layer.
+struct MapList { const float* A[16]; };
 template <int BS, int F>
-__global__ void __launch_bounds__(256) conv_pool_diag_kernel(const float* __restrict__ A, int L, float* __restrict__ pooled) {
-  constexpr int H = F / 2, T = BS + 2 * H, RUN = 8, CS = BS + 1;
+__global__ void __launch_bounds__(256, 3) conv_pool_diag_kernel(const __grid_constant__ MapList maps, int layers, int L, float* __restrict__ pooled) {
+  constexpr int H = F / 2, T = BS + 2 * H, RUN = 8, CS = BS + 1, TP = BS + 32, SLACK = 8;
+  static_assert(H <= 16, "halo");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* tile = reinterpret_cast<float*>(smem_raw);
-  double* cval = reinterpret_cast<double*>(smem_raw + (((size_t)T * T * sizeof(float) + 15) & ~(size_t)15));
+  float* tile = reinterpret_cast<float*>(smem_raw) + SLACK;
+  double* cval = reinterpret_cast<double*>(smem_raw + (size_t)(T * TP + 2 * SLACK) * sizeof(float));
   double* rsum = cval + (size_t)BS * CS;
-  const int bi = blockIdx.y, bj = blockIdx.x, nb = gridDim.x;
-  const int i0g = bi * BS - H, j0g = bj * BS - H;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // all of a thread's loads are issued before the first store (the tile is read with the latency of one load,
-  // not of one load per row)
-  constexpr int NR = (T + 7) / 8, NCOL = (T + 31) / 32;
-  float v[NR][NCOL];
-#pragma unroll
-  for (int a = 0; a < NR; ++a) {
-    const int ti = warp + 8 * a, gi = i0g + ti;
-#pragma unroll
-    for (int b = 0; b < NCOL; ++b) {
-      const int tj = lane + 32 * b, gj = j0g + tj;
-      v[a][b] = (ti < T && tj < T && gi >= 0 && gi < L && gj >= 0 && gj < L) ? A[(size_t)gi * L + gj] : 0.0f;
+  const int nb = L / BS, per = nb * nb;
+  const int total = layers * per, G = (int)gridDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int RUNS = (BS / RUN) * (BS + RUN - 1), CHUNKS = (RUNS + 31) / 32;
+  auto load = [&](int cell) {
+    const int m = cell / per, rest = cell - m * per;
+    const float* A = maps.A[m];
+    const int i0g = (rest / nb) * BS - H, j0g = (rest % nb) * BS - 16;
+    constexpr int PIECES = TP / 4;
+    for (int e = tid; e < T * PIECES; e += 256) {
+      const int ti = e / PIECES, p4 = e - ti * PIECES;
+      const int gi = i0g + ti, gj = j0g + 4 * p4;
+      const bool in = gi >= 0 && gi < L && gj >= 0 && gj < L;
+      const float* src = A + (in ? (size_t)gi * L + gj : 0);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(tile + ti * TP + 4 * p4)),
+                   "l"(src), "r"(in ? 16u : 0u) : "memory");
     }
-  }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (tid < 2 * SLACK) { if (tid < SLACK) tile[-1 - tid] = 0.0f; else tile[T * TP + tid - SLACK] = 0.0f; }
+  load(blockIdx.x);
+  int before = -1;                                     // cell whose total is still to be formed
+  for (int cell = blockIdx.x; cell < total; cell += G) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // p = sum_ii r[ii] (ii ascending): pool_fixed_order
+    auto finish = [&]() {
+      double p = 0.0;
+#pragma unroll 16
+      for (int ii = 0; ii < BS; ++ii) p = p + rsum[ii];
+      pooled[before] = (float)(p / (double)(BS * BS));
+    };
+    if (before >= 0 && tid == 224) finish();
+    __syncwarp();
+    // the warp of the total takes the fewest runs: its chain is as long as two of them
+    for (int q = warp == 7 ? CHUNKS - 1 : warp; q < CHUNKS; q += 7) {
+      if (warp != 7 && q == CHUNKS - 1) break;
+      const int r = q * 32 + lane;
+      if (r >= RUNS) break;
+      const int i0 = (r / (BS + RUN - 1)) * RUN, j0 = r % (BS + RUN - 1) - (RUN - 1);
+      const float* d0 = tile + i0 * TP + j0 + (16 - H);
+      double c[RUN];
 #pragma unroll
-  for (int a = 0; a < NR; ++a) {
-    const int ti = warp + 8 * a;
+      for (int k = 0; k < RUN; ++k) c[k] = 0.0;
+      // c[k] = sum_{t = 0 .. F-1} d[k + t], t ascending (oracle: conv_fixed_order)
 #pragma unroll
-    for (int b = 0; b < NCOL; ++b) {
-      const int tj = lane + 32 * b;
-      if (ti < T && tj < T) tile[ti * T + tj] = v[a][b];
+      for (int m = 0; m < F + RUN - 1; ++m) {
+        const double d = (double)d0[m * (TP + 1)];
+#pragma unroll
+        for (int k = 0; k < RUN; ++k)
+          if (m >= k && m < k + F) c[k] = c[k] + d;
+      }
+#pragma unroll
+      for (int k = 0; k < RUN; ++k) {
+        const int j = j0 + k;
+        if (j >= 0 && j < BS) cval[(i0 + k) * CS + j] = c[k];
+      }
     }
-  }
-  __syncthreads();
-  constexpr int RUNS = (BS / RUN) * (BS + RUN - 1);
-  for (int r = threadIdx.x; r < RUNS; r += blockDim.x) {
-    const int i0 = (r / (BS + RUN - 1)) * RUN, j0 = r % (BS + RUN - 1) - (RUN - 1);
-    float d[F + RUN - 1];
-#pragma unroll
-    for (int m = 0; m < F + RUN - 1; ++m)          // taps left or right of the tile belong to skipped outputs only
-      d[m] = (j0 + m >= 0 && j0 + m < T) ? tile[(i0 + m) * T + (j0 + m)] : 0.0f;
-    double c[RUN];
-#pragma unroll
-    for (int k = 0; k < RUN; ++k) c[k] = 0.0;
-    // c[k] = sum_{t = 0 .. F-1} d[k + t], t ascending (oracle: conv_fixed_order); the eight chains interleave
-#pragma unroll
-    for (int t = 0; t < F; ++t) {
-#pragma unroll
-      for (int k = 0; k < RUN; ++k) c[k] = c[k] + (double)d[k + t];
+    __syncthreads();
+    if (cell + G < total) load(cell + G);
+    if (tid < BS) {                                    // r[i] = sum_jj c[i, jj]  (jj ascending)
+      double rr = 0.0;
+#pragma unroll 16
+      for (int jj = 0; jj < BS; ++jj) rr = rr + cval[tid * CS + jj];
+      rsum[tid] = rr;
     }
-#pragma unroll
-    for (int k = 0; k < RUN; ++k) {
-      const int j = j0 + k;
-      if (j >= 0 && j < BS) cval[(i0 + k) * CS + j] = c[k];
+    before = cell;
+    if (cell + G >= total) {
+      __syncthreads();
+      if (tid == 224) finish();
     }
-  }
-  __syncthreads();
-  // r[i] = sum_jj c[i, jj]  (jj ascending), then p = sum_ii r[ii] (ii ascending): pool_fixed_order
-  for (int i = threadIdx.x; i < BS; i += blockDim.x) {
-    double rr = 0.0;
-#pragma unroll 8
-    for (int jj = 0; jj < BS; ++jj) rr = rr + cval[i * CS + jj];
-    rsum[i] = rr;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double p = 0.0;
-#pragma unroll 8
-    for (int ii = 0; ii < BS; ++ii) p = p + rsum[ii];
-    pooled[(size_t)bi * nb + bj] = (float)(p / (double)(BS * BS));
   }
 }
 
 template <int BS, int F>
-int launch_conv_pool_diag(const float* A, int L, int nb, float* pooled, cudaStream_t st) {
+int launch_conv_pool_diag(const MapList& maps, int layers, int L, int nb, float* pooled, cudaStream_t st) {
   constexpr int T = BS + F - 1;
-  const size_t smem = (((size_t)T * T * sizeof(float) + 15) & ~(size_t)15) + ((size_t)BS * (BS + 1) + BS) * sizeof(double);
+  const size_t smem = (size_t)(T * (BS + 32) + 16) * sizeof(float) + ((size_t)BS * (BS + 1) + BS) * sizeof(double);
+  int dev = 0, sms = 0;
+  SPION_CUDA_TRY(cudaGetDevice(&dev));
+  SPION_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (smem > 48 * 1024)
     SPION_CUDA_TRY(cudaFuncSetAttribute(conv_pool_diag_kernel<BS, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  conv_pool_diag_kernel<BS, F><<<dim3(nb, nb), 256, smem, st>>>(A, L, pooled);
+  const long long cells = (long long)layers * nb * nb, cap = 3LL * sms;        // three CTAs per SM (70 KB each)
+  conv_pool_diag_kernel<BS, F><<<(int)(cells < cap ? cells : cap), 256, smem, st>>>(maps, layers, L, pooled);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
@@ -159,26 +181,43 @@ __device__ __forceinline__ float key_to_float(uint32_t k) {
   return __uint_as_float(u);
 }
 
-// k-th smallest (0-based) of vals[0..n) by 4 passes of 8-bit radix select.  All threads call it.
-__device__ float select_kth(const float* __restrict__ vals, int n, int k, int* hist, int* s_sel) {
+// k-th smallest (0-based) of vals[0..n) by 4 passes of 8-bit radix select.  All threads call it.  The values of a map share their
+// leading bytes, so a warp whose digits are all equal counts them in one go (one thread scanning it and 4096 colliding
+// atomics per pass were most of the 36 us of this kernel at nb = 64).
+__device__ float select_kth(const float* vals, int n, int k, int* hist, int* s_sel) {
   uint32_t prefix = 0, mask = 0;
+  const int lane = threadIdx.x & 31;
   for (int pass = 3; pass >= 0; --pass) {
     const int shift = pass * 8;
     for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const uint32_t key = order_key(vals[i]);
-      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1);
+    for (int i0 = 0; i0 < n; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      const uint32_t key = i < n ? order_key(vals[i]) : 0u;
+      const bool in = i < n && (key & mask) == prefix;
+      const int digit = in ? (int)((key >> shift) & 255u) : 256;
+      int all;
+      __match_all_sync(0xffffffffu, digit, &all);
+      if (all) { if (in && lane == 0) atomicAdd(&hist[digit], 32); }
+      else if (in) atomicAdd(&hist[digit], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = 0, digit = 255, kk = k;
-      for (int b = 0; b < 256; ++b) {
-        if (kk < acc + hist[b]) { digit = b; kk -= acc; break; }
-        acc += hist[b];
+    if (threadIdx.x < 32) {                            // eight bins per lane
+      int sum = 0;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) sum += hist[lane * 8 + x];
+      int upto = sum;                                  // inclusive scan
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += y;
       }
-      s_sel[0] = digit;
-      s_sel[1] = kk;
+      if (k >= upto - sum && k < upto) {
+        int kk = k - (upto - sum), x = 0;
+        while (kk >= hist[lane * 8 + x]) { kk -= hist[lane * 8 + x]; ++x; }
+        s_sel[0] = lane * 8 + x;
+        s_sel[1] = kk;
+      }
     }
     __syncthreads();
     prefix |= (uint32_t)s_sel[0] << shift;
@@ -192,10 +231,29 @@ __device__ float select_kth(const float* __restrict__ vals, int n, int k, int* h
 // ---------------------------------------------------------------- selection (one CTA)
 // select == PATHS: thresh = torch.quantile(pooled, q) (linear), then 2*nb greedy walkers.
 // select == TOPK : the kcount largest cells (ties: lower flat index first).
-__global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ pooled, int nb, int select, float q,
-                                                      int kcount, uint8_t* __restrict__ mat,
-                                                      float* __restrict__ thresh_out) {
+// One CTA per map; its block structure follows in the same kernel: a chain of latencies, 23 us for two 64 x 64 maps, against 36 us
+// of selection and 13 us of structure for each of them with one launch per map and step.  copies: how many times the 0/1 float mask is written, `mats_step`
+// floats apart (the driver's stacked list, main_conv_ff.py:298-299).
+constexpr int SELECT_SMEM_CELLS = 128 * 128;           // maps up to this size are kept in shared memory
+struct SelectOut {
+  uint8_t* mat;
+  float *thresh, *mats;
+  int32_t *nnzb, *row_ptr, *col_idx, *blk_row, *col_ptr, *row_idx, *csc_pos, *work;
+  int copies;
+  long long mats_step;
+};
+__global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ pooled_all, int nb, int select, float q,
+                                                      int kcount, const __grid_constant__ SelectOut out) {
+  extern __shared__ float s_val[];
   __shared__ int hist[256];
+  const size_t cells = (size_t)nb * nb;
+  uint8_t* __restrict__ mat = out.mat + blockIdx.x * cells;
+  float* thresh_out = out.thresh ? out.thresh + blockIdx.x : nullptr;
+  const float* pooled = pooled_all + blockIdx.x * cells;
+  if (cells <= SELECT_SMEM_CELLS) {
+    for (int i = threadIdx.x; i < (int)cells; i += blockDim.x) s_val[i] = pooled[i];
+    pooled = s_val;
+  }
   __shared__ int s_sel[2];
   __shared__ float s_thresh;
   __shared__ int s_warp[32];
@@ -212,7 +270,28 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
     const int hi_i = (int)ceilf(rank);
     const float w = __fsub_rn(rank, fl);
     const float lo = select_kth(pooled, n, lo_i, hist, s_sel);
-    const float hi = (hi_i == lo_i) ? lo : select_kth(pooled, n, hi_i, hist, s_sel);
+    // the next order statistic: lo again if it occurs often enough, else the smallest value above it
+    float hi = lo;
+    if (hi_i != lo_i) {
+      const uint32_t klo = order_key(lo);
+      int le = 0;
+      uint32_t above = 0xffffffffu;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t key = order_key(pooled[i]);
+        if (key <= klo) ++le; else above = min(above, key);
+      }
+      le = __reduce_add_sync(0xffffffffu, le);
+      above = __reduce_min_sync(0xffffffffu, above);
+      if (threadIdx.x == 0) { hist[0] = 0; hist[1] = -1; }
+      __syncthreads();
+      if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&hist[0], le);
+        atomicMin(reinterpret_cast<unsigned int*>(&hist[1]), above);
+      }
+      __syncthreads();
+      if (hist[0] <= hi_i) hi = key_to_float((uint32_t)hist[1]);
+      __syncthreads();
+    }
     if (threadIdx.x == 0) {
       const float d = __fsub_rn(hi, lo);
       float t;
@@ -223,21 +302,36 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
     }
     __syncthreads();
     const float thresh = s_thresh;
-    // walkers: seeds (0,k) then (k,0); main_conv_ff.py:271-274.  Order-free: marks are idempotent.
+    // walkers: seeds (0,k) then (k,0); main_conv_ff.py:271-274.  Order-free: marks are idempotent.  Stops on the zero guard row /
+    // column (:37).  step(): where a walker goes from (x, y), and whether the cell it reaches is marked.
+    auto step = [&](int x, int y) -> int {
+      const float D = (x + 1 < nb) ? pooled[(size_t)(x + 1) * nb + y] : 0.0f;
+      const float R = (y + 1 < nb) ? pooled[(size_t)x * nb + y + 1] : 0.0f;
+      const float G = (x + 1 < nb && y + 1 < nb) ? pooled[(size_t)(x + 1) * nb + y + 1] : 0.0f;
+      int to;
+      float v;
+      if (D > R) {
+        if (D > G) { to = 1; v = D; } else { to = 3; v = G; }
+      } else {
+        if (R > G) { to = 2; v = R; } else { to = 3; v = G; }
+      }
+      return to | (v > thresh && v > 0.0f ? 4 : 0);
+    };
+    // small maps: all steps first, in parallel, so that a walker's chain is one byte per cell
+    const bool table = cells <= SELECT_SMEM_CELLS;
+    uint8_t* s_step = reinterpret_cast<uint8_t*>(s_val + (table ? cells : 0));
+    if (table) {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) s_step[i] = (uint8_t)step(i / nb, i % nb);
+      __syncthreads();
+    }
     for (int s = threadIdx.x; s < 2 * nb; s += blockDim.x) {
       int x = (s < nb) ? 0 : s - nb;
       int y = (s < nb) ? s : 0;
-      while (x < nb && y < nb) {                       // stops on the zero guard row / column (:37)
-        const float D = (x + 1 < nb) ? pooled[(size_t)(x + 1) * nb + y] : 0.0f;
-        const float R = (y + 1 < nb) ? pooled[(size_t)x * nb + y + 1] : 0.0f;
-        const float G = (x + 1 < nb && y + 1 < nb) ? pooled[(size_t)(x + 1) * nb + y + 1] : 0.0f;
-        float v;
-        if (D > R) {
-          if (D > G) { x += 1; v = D; } else { x += 1; y += 1; v = G; }
-        } else {
-          if (R > G) { y += 1; v = R; } else { x += 1; y += 1; v = G; }
-        }
-        if (v > thresh && v > 0.0f && x < nb && y < nb) mat[(size_t)x * nb + y] = 1;
+      while (x < nb && y < nb) {
+        const int t = table ? s_step[x * nb + y] : step(x, y);
+        x += t & 1;
+        y += (t >> 1) & 1;
+        if ((t & 4) && x < nb && y < nb) mat[(size_t)x * nb + y] = 1;
       }
     }
   } else {
@@ -281,6 +375,14 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nb; i += blockDim.x) mat[(size_t)i * nb + i] = 1;   // main_conv_ff.py:277-278
+  __syncthreads();
+  for (int c = 0; c < out.copies; ++c) {
+    float* m = out.mats + c * out.mats_step + blockIdx.x * cells;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) m[i] = (float)mat[i];
+  }
+  build_structure(mat, nb, out.nnzb + blockIdx.x, out.row_ptr + (size_t)blockIdx.x * (nb + 1), out.col_idx + blockIdx.x * cells,
+                  out.blk_row + blockIdx.x * cells, out.col_ptr + (size_t)blockIdx.x * (nb + 1), out.row_idx + blockIdx.x * cells,
+                  out.csc_pos + blockIdx.x * cells, out.work + blockIdx.x * cells);
 }
 
 // ---------------------------------------------------------------- mean over (b,h) of the dense map
@@ -385,12 +487,15 @@ extern "C" int spion_mean_map_tiles(const void* P, int dtype, const int32_t* blk
   return SPION_OK;
 }
 
-extern "C" int spion_discover_pattern(const float* A, int L, int block_size, int conv_kind, int F, int select,
-                                      double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,
-                                      int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
-                                      int32_t* row_idx, int32_t* csc_pos, int32_t* work, int32_t* host_nnzb,
-                                      void* cuda_stream) {
-  if (!A || !mat || !pooled || !nnzb || !row_ptr || !col_idx || !blk_row || !col_ptr || !row_idx || !csc_pos || !work)
+extern "C" int spion_discover_patterns(const float* const* host_A, int layers, int L, int block_size, int conv_kind, int F, int select,
+                                       double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,
+                                       int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
+                                       int32_t* row_idx, int32_t* csc_pos, int32_t* work, float* mats, int copies,
+                                       int32_t* host_nnzb, void* cuda_stream) {
+  if (!host_A || layers < 1 || layers > 16 || copies < 0 || (copies > 0 && !mats)) return SPION_ERR_ARG;
+  MapList maps = {};
+  for (int i = 0; i < layers; ++i) { maps.A[i] = host_A[i]; if (!host_A[i]) return SPION_ERR_ARG; }
+  if (!mat || !pooled || !nnzb || !row_ptr || !col_idx || !blk_row || !col_ptr || !row_idx || !csc_pos || !work)
     return SPION_ERR_ARG;
   if (L < 1 || block_size < 1 || L % block_size != 0) return SPION_ERR_SHAPE;
   const int bs = block_size, nb = L / bs;
@@ -400,32 +505,47 @@ extern "C" int spion_discover_pattern(const float* A, int L, int block_size, int
   if (select != SPION_SELECT_PATHS && select != SPION_SELECT_TOPK) return SPION_ERR_ARG;
   if (select == SPION_SELECT_PATHS && !(param >= 0.0 && param <= 1.0)) return SPION_ERR_ARG;
   cudaStream_t st = (cudaStream_t)cuda_stream;
+  const size_t cells = (size_t)nb * nb;
 
   const int T = bs + F - 1;
   size_t smem = (((size_t)T * T * sizeof(float) + 15) & ~(size_t)15) + ((size_t)bs * bs + bs) * sizeof(double);
   // The opt-in above 48 KB belongs to the current device only (a process may drive several), and the
   // call is cheap: make it on every launch that needs it instead of remembering one process-wide size.
-  if (conv_kind == SPION_CONV_DIAG && F == 31 && (bs == 64 || bs == 32)) {      // the reference's filter: the faster kernel
-    int rc = bs == 64 ? launch_conv_pool_diag<64, 31>(A, L, nb, pooled, st) : launch_conv_pool_diag<32, 31>(A, L, nb, pooled, st);
+  bool aligned = true;
+  for (int i = 0; i < layers; ++i) aligned = aligned && ((uintptr_t)host_A[i] & 15u) == 0;
+  if (conv_kind == SPION_CONV_DIAG && F == 31 && (bs == 64 || bs == 32) && aligned) {      // the reference's filter: the faster kernel
+    int rc = bs == 64 ? launch_conv_pool_diag<64, 31>(maps, layers, L, nb, pooled, st) : launch_conv_pool_diag<32, 31>(maps, layers, L, nb, pooled, st);
     if (rc) return rc;
   } else {
     if (smem > 48 * 1024)
       SPION_CUDA_TRY(cudaFuncSetAttribute(conv_pool_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    conv_pool_kernel<<<dim3(nb, nb), 256, smem, st>>>(A, L, bs, conv_kind, F, pooled);
-    SPION_LAUNCH_CHECK();
+    for (int i = 0; i < layers; ++i) {
+      conv_pool_kernel<<<dim3(nb, nb), 256, smem, st>>>(host_A[i], L, bs, conv_kind, F, pooled + i * cells);
+      SPION_LAUNCH_CHECK();
+    }
   }
 
   int kcount = 0;
   if (select == SPION_SELECT_TOPK) kcount = (int)((double)(nb * nb) * param - (double)nb);   // main_conv.py:247
-  select_kernel<<<1, 1024, 0, st>>>(pooled, nb, select, (float)param, kcount, mat, thresh);
+  const size_t dyn = cells <= SELECT_SMEM_CELLS ? cells * (sizeof(float) + 1) : 0;
+  SPION_CUDA_TRY(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SELECT_SMEM_CELLS * ((int)sizeof(float) + 1)));
+  const SelectOut out{mat, thresh, mats, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, copies, (long long)(layers * cells)};
+  select_kernel<<<layers, 1024, dyn, st>>>(pooled, nb, select, (float)param, kcount, out);
   SPION_LAUNCH_CHECK();
-  int rc = spion_launch_build_structure(mat, nb, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, st);
-  if (rc) return rc;
   if (host_nnzb) {
-    SPION_CUDA_TRY(cudaMemcpyAsync(host_nnzb, nnzb, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    SPION_CUDA_TRY(cudaMemcpyAsync(host_nnzb, nnzb, layers * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     SPION_CUDA_TRY(cudaStreamSynchronize(st));
   }
   return SPION_OK;
+}
+
+extern "C" int spion_discover_pattern(const float* A, int L, int block_size, int conv_kind, int F, int select,
+                                      double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,
+                                      int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
+                                      int32_t* row_idx, int32_t* csc_pos, int32_t* work, int32_t* host_nnzb,
+                                      void* cuda_stream) {
+  return spion_discover_patterns(&A, 1, L, block_size, conv_kind, F, select, param, mat, pooled, thresh, nnzb, row_ptr, col_idx, blk_row,
+                                 col_ptr, row_idx, csc_pos, work, nullptr, 0, host_nnzb, cuda_stream);
 }
 
 extern "C" int spion_mean_attention_map(const float* attn, int batch, int heads, int L, int transposed, float* A,

@@ -4,69 +4,14 @@
 // models/attention_blockcuda.py:31-43 (sum / repeat / cumsum / Upsample / nonzero /
 // repeat(BH)), which the reference re-runs on every forward call of every layer.
 #include "common.cuh"
+#include "structure.cuh"
 
 namespace {
 
-// One CTA.  mat [nb*nb] uint8 -> CSR (row_ptr, col_idx, blk_row), CSC (col_ptr, row_idx,
-// csc_pos) and the block count.  work [nb*nb] receives the CSR block id of every set cell.
 __global__ void __launch_bounds__(1024) build_structure_kernel(
-    const uint8_t* __restrict__ mat, int nb, int32_t* __restrict__ nnzb, int32_t* __restrict__ row_ptr,
-    int32_t* __restrict__ col_idx, int32_t* __restrict__ blk_row, int32_t* __restrict__ col_ptr,
-    int32_t* __restrict__ row_idx, int32_t* __restrict__ csc_pos, int32_t* __restrict__ work) {
-  __shared__ int s_cnt[SPION_MAX_NB + 1];
-  __shared__ int s_ptr[SPION_MAX_NB + 1];
-  const int tid = threadIdx.x;
-  // ---- rows
-  for (int r = tid; r < nb; r += blockDim.x) {
-    int n = 0;
-    for (int c = 0; c < nb; ++c) n += mat[(size_t)r * nb + c] != 0;
-    s_cnt[r] = n;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int acc = 0;
-    for (int r = 0; r < nb; ++r) { s_ptr[r] = acc; acc += s_cnt[r]; }
-    s_ptr[nb] = acc;
-    *nnzb = acc;
-  }
-  __syncthreads();
-  for (int r = tid; r <= nb; r += blockDim.x) row_ptr[r] = s_ptr[r];
-  for (int r = tid; r < nb; r += blockDim.x) {
-    int pos = s_ptr[r];
-    for (int c = 0; c < nb; ++c) {
-      if (mat[(size_t)r * nb + c]) {
-        col_idx[pos] = c;
-        blk_row[pos] = r;
-        work[(size_t)r * nb + c] = pos;
-        ++pos;
-      }
-    }
-  }
-  __syncthreads();
-  // ---- columns
-  for (int c = tid; c < nb; c += blockDim.x) {
-    int n = 0;
-    for (int r = 0; r < nb; ++r) n += mat[(size_t)r * nb + c] != 0;
-    s_cnt[c] = n;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int acc = 0;
-    for (int c = 0; c < nb; ++c) { s_ptr[c] = acc; acc += s_cnt[c]; }
-    s_ptr[nb] = acc;
-  }
-  __syncthreads();
-  for (int c = tid; c <= nb; c += blockDim.x) col_ptr[c] = s_ptr[c];
-  for (int c = tid; c < nb; c += blockDim.x) {
-    int pos = s_ptr[c];
-    for (int r = 0; r < nb; ++r) {
-      if (mat[(size_t)r * nb + c]) {
-        row_idx[pos] = r;
-        csc_pos[pos] = work[(size_t)r * nb + c];
-        ++pos;
-      }
-    }
-  }
+    const uint8_t* mat, int nb, int32_t* nnzb, int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr, int32_t* row_idx,
+    int32_t* csc_pos, int32_t* work) {
+  build_structure(mat, nb, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work);
 }
 
 // Recover the block mask from the reference's element-level CSR (one CTA per block row).

@@ -68,29 +68,65 @@ def discover_pattern(A: torch.Tensor, block_size: int, threshold: float, conv: s
 
     ``A`` is the [L, L] fp32 mean attention map on the GPU.
     """
-    if not A.is_cuda:
-        raise ValueError("discover_pattern needs the attention map on the GPU (there is no CPU path)")
-    A = A.detach().to(torch.float32).contiguous()
-    L = A.shape[0]
-    if A.dim() != 2 or A.shape[1] != L or L % block_size != 0:
-        raise ValueError("A must be [L, L] with L a multiple of block_size")
-    nb = L // block_size
-    s = _alloc_structure(nb, A.device)
-    pooled = torch.empty(nb, nb, dtype=torch.float32, device=A.device)
-    thresh = torch.zeros(1, dtype=torch.float32, device=A.device)
-    host_n = _lib.ctypes.c_int32(0)
-    with torch.cuda.device(A.device):
-        check(lib.spion_discover_pattern(
-            ptr(A), L, block_size, CONV_KINDS[conv], F,
-            _lib.SELECT_PATHS if select == "paths" else _lib.SELECT_TOPK, float(threshold),
-            ptr(s["mat"]), ptr(pooled), ptr(thresh), ptr(s["nnzb_dev"]),
-            ptr(s["row_ptr"]), ptr(s["col_idx"]), ptr(s["blk_row"]),
-            ptr(s["col_ptr"]), ptr(s["row_idx"]), ptr(s["csc_pos"]), ptr(s["work"]),
-            _lib.ctypes.cast(_lib.ctypes.byref(host_n), _lib.c_void_p), _lib.current_stream_ptr()),
-            "spion_discover_pattern")
-    n = int(host_n.value)
-    return BlockPattern(block_size, nb, n, s["mat"], pooled, thresh, s["row_ptr"], s["col_idx"][:n], s["blk_row"][:n],
-                        s["col_ptr"], s["row_idx"][:n], s["csc_pos"][:n])
+    return _discover([A], block_size, threshold, conv, F, select, 0)[0][0]
+
+
+_MAPS_PER_CALL = 16
+
+
+def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select: str, copies: int):
+    """Patterns of several equally large maps (one call of the library per 16: every stage runs over all of them, one host
+    synchronisation) and ``copies`` stacked copies of their masks as [copies, maps, nb, nb] floats (None for 0)."""
+    for A in maps:
+        if not A.is_cuda:
+            raise ValueError("discover_pattern needs the attention map on the GPU (there is no CPU path)")
+    maps = [A.detach().to(torch.float32).contiguous() for A in maps]
+    L = maps[0].shape[0]
+    for A in maps:
+        if A.dim() != 2 or tuple(A.shape) != (L, L) or L % block_size != 0:
+            raise ValueError("A must be [L, L] with L a multiple of block_size")
+    n, nb, dev = len(maps), L // block_size, maps[0].device
+    cells = nb * nb
+    # one allocation per element type for all layers
+    mat = torch.empty(n, nb, nb, dtype=torch.uint8, device=dev)
+    flt = torch.empty(n * cells + n + copies * n * cells, dtype=torch.float32, device=dev)
+    ints = torch.empty(n * (5 * cells + 2 * (nb + 1) + 1), dtype=torch.int32, device=dev)
+    pf, pi, pm = flt.data_ptr(), ints.data_ptr(), mat.data_ptr()
+    int_at, off = {}, 0
+    for name, size in (("col_idx", cells), ("blk_row", cells), ("row_idx", cells), ("csc_pos", cells), ("work", cells),
+                       ("row_ptr", nb + 1), ("col_ptr", nb + 1), ("nnzb", 1)):
+        int_at[name] = (off, size)
+        off += n * size
+    copies_at = n * cells + n
+    with torch.cuda.device(dev):
+        stream = _lib.current_stream_ptr()
+        for l0 in range(0, n, _MAPS_PER_CALL):
+            m = min(_MAPS_PER_CALL, n - l0)
+            ptrs = (_lib.c_void_p * m)(*[A.data_ptr() for A in maps[l0:l0 + m]])
+            at = {k: pi + 4 * (o + l0 * size) for k, (o, size) in int_at.items()}
+            # the copies of the masks are written in one go when a single call covers the model
+            direct = copies if n <= _MAPS_PER_CALL else 0
+            check(lib.spion_discover_patterns(
+                ptrs, m, L, block_size, CONV_KINDS[conv], F,
+                _lib.SELECT_PATHS if select == "paths" else _lib.SELECT_TOPK, float(threshold),
+                pm + l0 * cells, pf + 4 * l0 * cells, pf + 4 * (n * cells + l0), at["nnzb"], at["row_ptr"], at["col_idx"], at["blk_row"],
+                at["col_ptr"], at["row_idx"], at["csc_pos"], at["work"], pf + 4 * copies_at if direct else None, direct,
+                None, stream), "spion_discover_patterns")
+        # views that do not depend on the block counts are made while the kernels run; reading the counts waits for them
+        mats = flt[copies_at:].view(copies, n, nb, nb) if copies else None
+        if copies and n > _MAPS_PER_CALL:
+            mats.copy_(mat[None])
+        pooled = flt[:n * cells].view(n, nb, nb).unbind(0)
+        thresh = flt[n * cells:copies_at].split(1)
+        row_ptr, col_ptr = (ints[int_at[k][0]:int_at[k][0] + n * (nb + 1)].split(nb + 1) for k in ("row_ptr", "col_ptr"))
+        mat_l = mat.unbind(0)
+        o = int_at["nnzb"][0]
+        counts = ints[o:o + n].tolist()
+    out = []
+    for l, k in enumerate(counts):
+        col_idx, blk_row, row_idx, csc_pos = (ints.narrow(0, int_at[x][0] + l * cells, k) for x in ("col_idx", "blk_row", "row_idx", "csc_pos"))
+        out.append(BlockPattern(block_size, nb, k, mat_l[l], pooled[l], thresh[l], row_ptr[l], col_idx, blk_row, col_ptr[l], row_idx, csc_pos))
+    return out, mats
 
 
 def pattern_from_mask(mat: torch.Tensor, block_size: int) -> BlockPattern:
@@ -150,9 +186,8 @@ def discover_layers(attn_lst, model_config, conv: str = "diag", F: int = 31, sel
     bs = model_config["block_size"]
     L = model_config["max_seq_len"]
     key = model_config["threshold"] if select == "paths" else model_config["density"]
-    patterns = [discover_pattern(a[:L], bs, key, conv, F, select) for a in attn_lst]
-    mats = torch.stack([p.float_mat() for p in patterns], 0)
-    return torch.stack([mats, mats, mats, mats], 0), patterns
+    patterns, mats = _discover([a[:L] for a in attn_lst], bs, key, conv, F, select, 4)
+    return mats, patterns
 
 
 def save_mask_pickle(mat_lst: torch.Tensor, path: str) -> None:
