@@ -15,45 +15,69 @@
 // reads them back, writes the probabilities over them and feeds the second product.  The backward
 // row kernel does the same with dP in the dS tiles.
 //
-// Thread layout: a bs x bs tile is computed by (bs/4)^2 threads with 4x4 micro-tiles (rows
-// contiguous, columns interleaved by bs/4 so that shared-memory reads of the second operand are
-// conflict-free); a CTA of 256 threads therefore works on 256/(bs/4)^2 consecutive (b,h) matrices of
-// the same block row: they share the mask, so the CTA runs in lock step.
+// Bound by the FMA pipes: scalar multiply-adds reach 47 TFLOP/s on this chip (register ports) and packed pairs 61, so the loops use
+// pairs.  With 4 x 4 micro-tiles every 64 multiply-adds took eight 16-byte reads of shared memory; now a bs x bs tile is
+// computed by bs^2/32 threads (one warp at bs 32, four at 64) with 8 x 4 micro-tiles, 12 to 16 reads per 128.  The threads of
+// one (b,h) matrix run on their own: a warp needs no CTA barrier, four warps a named one.  Tiles are unpadded, the 16-byte
+// pieces of row i exchanged by i / 4 (mod 8): a thread owns contiguous rows and four contiguous columns, so value tiles
+// move in 16-byte pieces, and the reads take no bank twice.
+// 512 matrices, L = 1024, d 32, 154 blocks of 32 (10.3 GFLOP a kernel, 170 us at the rate of packed pairs), before and now:
+// forward 474 -> 358 us (it also writes the values twice and reads them once), rows 441 -> 310, columns 320 -> 270.
+// 15 matrices, L = 3008, d 64, blocks of 64 at 8 % and one full column: columns 314 -> 158 (see SPLIT at that kernel).
 //
 // Layouts: operands through (row, column) strides, value tiles through tile_address(); only
 // layouts whose tile rows are contiguous (element CSR, block tiles) are accepted.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace {
 
-template <int BS, int D>
+// R: rows of a tile per thread, 8, or 4 for calls that do not fill the chip (FEW_WARPS below)
+template <int BS, int D, int R>
 struct Cfg {
   static constexpr int TX = BS / 4;            // threads along a tile row
-  static constexpr int NT = TX * TX;           // threads per (b,h) problem
-  static constexpr int G = 256 / NT;           // problems per CTA
+  static constexpr int NT = BS * BS / (4 * R); // threads per (b,h) problem
+  static constexpr int CTA = NT > 128 ? NT : 128;
+  static constexpr int G = CTA / NT;           // problems per CTA
   static constexpr int TN = D / TX;            // output columns per thread in the bs x d products
-  static constexpr int SA = D + 4;             // shared-memory row stride of a [bs x d] operand tile
-  static constexpr int SP = BS + 4;            // ... of a [bs x bs] value tile
+  static constexpr int TILE = BS * D;          // floats of an operand tile
+  static constexpr int VALS = BS * BS;         // ... of a value tile
+  static constexpr int RESIDENT = R == 4 || (BS == 32 && D == 64) ? 2 : 3;   // CTAs per SM that the tiles leave room for (five at 64, 32: registers)
+  static constexpr int RESIDENT2 = R == 4 || (BS == 32 && D == 64) ? 2 : 4;  // ... of the two-pass kernels
   static_assert(TN == 2 || TN == 4 || TN == 8, "unsupported shape");
 };
 
+// float offset of 16-byte piece `piece` of row `row` in a tile of COLS columns
+template <int COLS>
+__device__ __forceinline__ int at(int row, int piece) { return row * COLS + ((piece ^ ((row >> 2) & 7)) << 2); }
+
+// the threads of problem g
+template <int NT>
+__device__ __forceinline__ void group_sync(int g) {
+  if (NT == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(NT) : "memory");
+}
+
 // column of the thread's y-th output in a bs x d product: groups of 4 (or 2) contiguous columns
-template <int BS, int D>
+template <int BS, int D, int R>
 __device__ __forceinline__ int out_col(int tx, int y) {
-  using C = Cfg<BS, D>;
+  using C = Cfg<BS, D, R>;
   if (C::TN == 2) return tx * 2 + y;
   return (y >> 2) * (C::TX * 4) + tx * 4 + (y & 3);
 }
 
-template <int TN>
-__device__ __forceinline__ void load_vec(const float* row, int tx, int TX, float (&b)[TN]) {
-  if (TN == 2) {
-    const float2 v = *reinterpret_cast<const float2*>(row + tx * 2);
+// the thread's columns of row `row` of a [bs x d] tile
+template <int BS, int D, int R>
+__device__ __forceinline__ void load_vec(const float* tile, int row, int tx, float (&b)[Cfg<BS, D, R>::TN]) {
+  using C = Cfg<BS, D, R>;
+  if constexpr (C::TN == 2) {
+    const float2 v = *reinterpret_cast<const float2*>(tile + at<D>(row, tx >> 1) + (tx & 1) * 2);
     b[0] = v.x; b[1] = v.y;
   } else {
 #pragma unroll
-    for (int g4 = 0; g4 < TN / 4; ++g4) {
-      const float4 v = *reinterpret_cast<const float4*>(row + g4 * TX * 4 + tx * 4);
+    for (int g4 = 0; g4 < C::TN / 4; ++g4) {
+      const float4 v = *reinterpret_cast<const float4*>(tile + at<D>(row, g4 * C::TX + tx));
       b[4 * g4] = v.x; b[4 * g4 + 1] = v.y; b[4 * g4 + 2] = v.z; b[4 * g4 + 3] = v.w;
     }
   }
@@ -70,95 +94,173 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Start the asynchronous copy of a [ROWS x COLS] tile (element (i, n) at src + i*s_row + n*s_col) into
-// shared memory, row-major with the given stride, by the NT threads of one problem.  The caller
+// A [L x d] operand of one (b,h) matrix, or a value tile: element (i, n) at base + i*s_row + n*s_col.
+struct Operand {
+  const float* base;
+  long long s_row, s_col;
+  bool pieces;                                       // rows in 16-byte pieces
+  __device__ __forceinline__ Operand(const float* p, const OperandLayout& l, int bh)
+      : base(p + (long long)bh * l.bh_stride), s_row(l.sl), s_col(l.sd) {
+    pieces = s_col == 1 && (s_row & 3) == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
+  }
+  __device__ __forceinline__ Operand(const float* p, int stride)
+      : base(p), s_row(stride), s_col(1), pieces((reinterpret_cast<uintptr_t>(p) & 15) == 0) {}
+};
+
+// Start the asynchronous copy of rows row0 .. row0 + ROWS - 1 into
+// shared memory by the NT threads of one problem.  The caller
 // commits the group, waits for it and synchronises before the tile is read.
 template <int ROWS, int COLS, int NT>
-__device__ __forceinline__ void load_tile(float* dst, int stride, const float* __restrict__ src, long long s_row,
-                                          long long s_col, int t) {
-  if (s_col == 1 && (s_row & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+__device__ __forceinline__ void load_tile(float* dst, const Operand& o, int row0, int t) {
+  const float* src = o.base + row0 * o.s_row;
+  if (o.pieces) {
+    constexpr int STEP = NT / (COLS / 4);            // rows per round
+    const int row = t / (COLS / 4), c4 = t % (COLS / 4);
+    src += row * o.s_row + c4 * 4;
+    const long long step = STEP * o.s_row;
 #pragma unroll
-    for (int idx = t; idx < ROWS * COLS / 4; idx += NT) {
-      const int row = idx / (COLS / 4), c4 = idx % (COLS / 4);
-      cp_async16(dst + row * stride + c4 * 4, src + (long long)row * s_row + c4 * 4);
+    for (int i = 0; i < ROWS / STEP; ++i) {
+      cp_async16(dst + at<COLS>(row + i * STEP, c4), src);
+      src += step;
     }
-  } else if (s_col == 1) {
+  } else if (o.s_col == 1) {
     for (int idx = t; idx < ROWS * COLS; idx += NT) {
       const int row = idx / COLS, col = idx % COLS;
-      cp_async4(dst + row * stride + col, src + (long long)row * s_row + col);
+      cp_async4(dst + at<COLS>(row, col >> 2) + (col & 3), src + row * o.s_row + col);
     }
   } else {
+#pragma unroll 4
     for (int idx = t; idx < ROWS * COLS; idx += NT) {
       const int row = idx % ROWS, col = idx / ROWS;
-      cp_async4(dst + row * stride + col, src + (long long)row * s_row + (long long)col * s_col);
+      cp_async4(dst + at<COLS>(row, col >> 2) + (col & 3), src + row * o.s_row + col * o.s_col);
     }
   }
 }
 
-// acc[x][y] += sum_n A[ty*4+x][n] * B[tx + y*TX][n]   (both tiles [bs x d] in shared memory)
+// The value tiles of one block row: element (i, j) of its k-th tile at base + k * step + i * si + j.
+struct RowTiles {
+  long long base;
+  int si, step;
+  template <int BS>
+  static __device__ __forceinline__ RowTiles of(const ValueLayout& vl, int rp, int nblk) {
+    const long long base = (long long)rp * BS * BS;
+    return vl.mode == VAL_ELEMCSR ? RowTiles{base, nblk * BS, BS} : RowTiles{base, BS, BS * BS};
+  }
+};
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+constexpr float LOG2_E = 1.4426950408889634f;
+
+// Four consecutive values of a value tile (tile rows are contiguous; `vec`: 16-byte aligned).
+__device__ __forceinline__ float4 load_vals(const float* p, bool vec) {
+  return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ void store_vals(float* p, float4 v, bool vec) {
+  if (vec) *reinterpret_cast<float4*>(p) = v;
+  else p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
+}
+__device__ __forceinline__ bool vec_ok(const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Packed pairs of fp32: one instruction, two multiply-adds per lane.  The FMA pipe is no faster for it, but the loops below were
+// limited by issue slots (two multiply-adds in three instructions).
+using pair_t = unsigned long long;
+__device__ __forceinline__ pair_t pack2(float x, float y) {
+  pair_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(pair_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(pair_t& acc, pair_t a, pair_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+struct Quad { pair_t lo, hi; };
+__device__ __forceinline__ Quad load_quad(const float* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return Quad{v.x, v.y};
+}
+
+// out[x][y] = sum_n A[row0+x][n] * B[tx*4+y][n], x = 0..3   (both tiles [bs x d] in shared memory; row0 a multiple of four; even and
+// odd n in one sum each).  A thread's eight rows are taken in two halves: the registers of all sixty-four sums would cost
+// a resident CTA.
 template <int BS, int D>
-__device__ __forceinline__ void tile_abt(const float* As, const float* Bs, int ty, int tx, float (&acc)[4][4]) {
-  using C = Cfg<BS, D>;
+__device__ __forceinline__ void tile_abt(const float* As, const float* Bs, int row0, int tx, float (&out)[4][4]) {
+  pair_t acc[4][4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
 #pragma unroll 2
-  for (int n = 0; n < D; n += 4) {
-    float4 a[4], b[4];
+  for (int n = 0; n < D / 4; ++n) {
+    Quad a[4], b[4];
 #pragma unroll
-    for (int x = 0; x < 4; ++x) a[x] = *reinterpret_cast<const float4*>(As + (ty * 4 + x) * C::SA + n);
+    for (int y = 0; y < 4; ++y) b[y] = load_quad(Bs + at<D>(tx * 4, n) + y * D);
 #pragma unroll
-    for (int y = 0; y < 4; ++y) b[y] = *reinterpret_cast<const float4*>(Bs + (tx + y * C::TX) * C::SA + n);
+    for (int x = 0; x < 4; ++x) a[x] = load_quad(As + at<D>(row0, n) + x * D);
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        acc[x][y] = fmaf(a[x].x, b[y].x, acc[x][y]);
-        acc[x][y] = fmaf(a[x].y, b[y].y, acc[x][y]);
-        acc[x][y] = fmaf(a[x].z, b[y].z, acc[x][y]);
-        acc[x][y] = fmaf(a[x].w, b[y].w, acc[x][y]);
-      }
+      for (int y = 0; y < 4; ++y) fma2(acc[x][y], a[x].lo, b[y].lo);
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int y = 0; y < 4; ++y) fma2(acc[x][y], a[x].hi, b[y].hi);
   }
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      const float2 v = unpack2(acc[x][y]);
+      out[x][y] = v.x + v.y;
+    }
 }
 
-// acc[x][y] += sum_j Vt[ty*4+x][j] * B[j][out_col(y)]   (Vt: [bs x bs] value tile, B: [bs x d])
-template <int BS, int D>
-__device__ __forceinline__ void tile_ab(const float* Vt, const float* Bs, int ty, int tx,
-                                        float (&acc)[4][Cfg<BS, D>::TN]) {
-  using C = Cfg<BS, D>;
-#pragma unroll 2
-  for (int j = 0; j < BS; j += 4) {
-    float a[4][4];
+// The thread's R x TN sums of a bs x d product, rows in pairs: v[x][y] = (row ty*R + 2 x, row ty*R + 2 x + 1), column out_col(y).
+template <int BS, int D, int R>
+struct Sums {
+  pair_t v[R / 2][Cfg<BS, D, R>::TN];
+  __device__ __forceinline__ Sums() {
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const float4 v = *reinterpret_cast<const float4*>(Vt + (ty * 4 + x) * C::SP + j);
-      a[x][0] = v.x; a[x][1] = v.y; a[x][2] = v.z; a[x][3] = v.w;
-    }
+    for (int x = 0; x < R / 2; ++x)
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      float b[C::TN];
-      load_vec<C::TN>(Bs + (j + jj) * C::SA, tx, C::TX, b);
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < C::TN; ++y) acc[x][y] = fmaf(a[x][jj], b[y], acc[x][y]);
-    }
+      for (int y = 0; y < Cfg<BS, D, R>::TN; ++y) v[x][y] = 0ull;
   }
-}
+};
 
-// acc[x][y] += sum_i Vt[i][ty*4+x] * B[i][out_col(y)]   (transposed use of the value tile)
-template <int BS, int D>
-__device__ __forceinline__ void tile_atb(const float* Vt, const float* Bs, int ty, int tx,
-                                         float (&acc)[4][Cfg<BS, D>::TN]) {
-  using C = Cfg<BS, D>;
+// acc += sum_i Vt[i][rows] * B[i][columns]   (Vt: [bs x bs] value tile, transposed use; B: [bs x d])
+template <int BS, int D, int R>
+__device__ __forceinline__ void tile_atb(const float* Vt, const float* Bs, int ty, int tx, Sums<BS, D, R>& acc) {
+  using C = Cfg<BS, D, R>;
 #pragma unroll 4
   for (int i = 0; i < BS; ++i) {
-    const float4 v = *reinterpret_cast<const float4*>(Vt + i * C::SP + ty * 4);
-    const float a[4] = {v.x, v.y, v.z, v.w};
+    pair_t a[R / 2];
+#pragma unroll
+    for (int x = 0; x < R / 4; ++x) {
+      const Quad v = load_quad(Vt + at<BS>(i, R / 4 * ty + x));
+      a[2 * x] = v.lo;
+      a[2 * x + 1] = v.hi;
+    }
     float b[C::TN];
-    load_vec<C::TN>(Bs + i * C::SA, tx, C::TX, b);
+    load_vec<BS, D, R>(Bs, i, tx, b);
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int y = 0; y < C::TN; ++y) {
+      const pair_t bb = pack2(b[y], b[y]);
 #pragma unroll
-      for (int y = 0; y < C::TN; ++y) acc[x][y] = fmaf(a[x], b[y], acc[x][y]);
+      for (int x = 0; x < R / 2; ++x) fma2(acc.v[x][y], a[x], bb);
+    }
   }
+}
+
+// Four rows of the thread's values of a tile into shared memory, transposed (16-byte piece `piece` of each row there), so that tile_atb multiplies with the tile itself.
+template <int BS>
+__device__ __forceinline__ void put_transposed(float* Vt, int piece, int tx, const float (&v)[4][4]) {
+#pragma unroll
+  for (int y = 0; y < 4; ++y)
+    *reinterpret_cast<float4*>(Vt + at<BS>(tx * 4 + y, piece)) = make_float4(v[0][y], v[1][y], v[2][y], v[3][y]);
 }
 
 template <int TX>
@@ -174,280 +276,274 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 
-// store the thread's 4 x TN outputs of a bs x d product
-template <int BS, int D>
+// store the thread's R x TN outputs of a bs x d product
+template <int BS, int D, int R>
 __device__ __forceinline__ void store_out(float* __restrict__ out, OperandLayout lo, int row0, int ty, int tx,
-                                          const float (&acc)[4][Cfg<BS, D>::TN]) {
-  using C = Cfg<BS, D>;
+                                          const Sums<BS, D, R>& sums) {
+  using C = Cfg<BS, D, R>;
+  float acc[R][C::TN];
 #pragma unroll
-  for (int x = 0; x < 4; ++x) {
-    float* o = out + (long long)(row0 + ty * 4 + x) * lo.sl;
-    if (lo.sd == 1 && C::TN >= 4 && (lo.sl & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+  for (int x = 0; x < R / 2; ++x)
+#pragma unroll
+    for (int y = 0; y < C::TN; ++y) {
+      const float2 v = unpack2(sums.v[x][y]);
+      acc[2 * x][y] = v.x;
+      acc[2 * x + 1][y] = v.y;
+    }
+  const bool vec = lo.sd == 1 && (lo.sl & 3) == 0 && vec_ok(out);
+#pragma unroll
+  for (int x = 0; x < R; ++x) {
+    float* o = out + (long long)(row0 + ty * R + x) * lo.sl;
+    if (C::TN >= 4 && vec) {
 #pragma unroll
       for (int g4 = 0; g4 < C::TN / 4; ++g4)
-        *reinterpret_cast<float4*>(o + out_col<BS, D>(tx, 4 * g4)) =
+        *reinterpret_cast<float4*>(o + out_col<BS, D, R>(tx, 4 * g4)) =
             make_float4(acc[x][4 * g4], acc[x][4 * g4 + 1], acc[x][4 * g4 + 2], acc[x][4 * g4 + 3]);
     } else {
 #pragma unroll
-      for (int y = 0; y < C::TN; ++y) o[(long long)out_col<BS, D>(tx, y) * lo.sd] = acc[x][y];
+      for (int y = 0; y < C::TN; ++y) o[(long long)out_col<BS, D, R>(tx, y) * lo.sd] = acc[x][y];
     }
   }
 }
 
+// Shared memory of the two-pass kernels: the row's own operand (pass 1) and the value tile (pass 2) take turns.
+template <int BS, int D, int R> constexpr int ONE = Cfg<BS, D, R>::TILE > Cfg<BS, D, R>::VALS ? Cfg<BS, D, R>::TILE : Cfg<BS, D, R>::VALS;
+template <int BS, int D, int R> __host__ __device__ constexpr int two_pass_floats() { return ONE<BS, D, R> + 2 * Cfg<BS, D, R>::TILE; }
+
 // ------------------------------------------------------------------------------ forward
 //   v = S*scale - keypad[col];  m = max(floor, max v);  Z = sum exp(v-m) + (L-n_i) exp(-m);  P = exp(v-m)/Z
 // The K (pass 1) and V (pass 2) tiles are double-buffered: the copy of tile k+1 is in flight while
-// tile k is used.
-template <int BS, int D>
-__global__ void __launch_bounds__(256, 3) fused_fwd_kernel(const float* __restrict__ Q, OperandLayout lq,
+// tile k is used.  Every thread keeps the maximum and the sum of its own columns of a row; the threads of a row join them
+// once, after the last tile.
+template <int BS, int D, int R>
+__global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) fused_fwd_kernel(const float* __restrict__ Q, OperandLayout lq,
                                                            const float* __restrict__ K, OperandLayout lk,
                                                            const float* __restrict__ V, OperandLayout lv,
                                                            const float* __restrict__ keypad, float floor_v, float* P,
                                                            ValueLayout vl, float* __restrict__ O, OperandLayout lo,
                                                            Pattern p, int BH, int L, float scale) {
-  using C = Cfg<BS, D>;
-  constexpr int TILE = BS * C::SA;
+  using C = Cfg<BS, D, R>;
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int r = blockIdx.x;
-  const int bh_raw = blockIdx.y * C::G + g;
-  const bool active = bh_raw < BH;
-  const int bh = active ? bh_raw : BH - 1;                       // idle problems shadow the last one, store nothing
-  float* Qs = smem + g * (3 * TILE + BS * C::SP);
-  float* Bs = Qs + TILE;                                        // two buffers: K tiles, then V tiles
-  float* Ps = Qs + 3 * TILE;
+  const int r = blockIdx.x, bh = blockIdx.y * C::G + g;
+  if (bh >= BH) return;
+  float* Qs = smem + g * two_pass_floats<BS, D, R>();
+  float* Bs = Qs + ONE<BS, D, R>;                                // two buffers: K tiles, then V tiles
+  float* Ps = Qs;                                               // pass 2
 
   const int rp = p.row_ptr[r], nblk = p.row_ptr[r + 1] - rp;
   const int* cols = p.col_idx + rp;
-  const float* Qb = Q + (long long)bh * lq.bh_stride + (long long)r * BS * lq.sl;
-  const float* Kb = K + (long long)bh * lk.bh_stride;
-  const float* Vb = V + (long long)bh * lv.bh_stride;
+  const Operand Kb(K, lk, bh), Vb(V, lv, bh);
   float* Pb = P + (long long)bh * vl.bh_stride;
-  const float* kp = keypad ? keypad + (long long)bh * L : nullptr;
+  const float* kp = keypad ? keypad + (long long)bh * L + tx * 4 : nullptr;
+  const bool vec = vec_ok(Pb);
+  const RowTiles rt = RowTiles::of<BS>(vl, rp, nblk);
+  float* mine = Pb + rt.base + ty * R * rt.si + tx * 4;         // the thread's values of the row's first tile
+  const float scale2 = scale * LOG2_E;                          // scores in base-2 units
 
   int c_cur = nblk > 0 ? cols[0] : 0, c_nxt = nblk > 1 ? cols[1] : 0;
-  load_tile<BS, D, C::NT>(Qs, C::SA, Qb, lq.sl, lq.sd, t);
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, C::SA, Kb + (long long)c_cur * BS * lk.sl, lk.sl, lk.sd, t);
+  load_tile<BS, D, C::NT>(Qs, Operand(Q, lq, bh), r * BS, t);
+  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Kb, c_cur * BS, t);
   cp_async_commit();
 
   // ---- pass 1: scores into the P tiles, running maximum and denominator per row
-  float m[4], l[4];
+  float m[R], l[R];
 #pragma unroll
-  for (int x = 0; x < 4; ++x) { m[x] = floor_v; l[x] = 0.f; }
+  for (int x = 0; x < R; ++x) { m[x] = floor_v * LOG2_E; l[x] = 0.f; }
   for (int k = 0; k < nblk; ++k) {
     const int c = c_cur;
     if (k + 1 < nblk)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * TILE, C::SA, Kb + (long long)c_nxt * BS * lk.sl, lk.sl, lk.sd, t);
+      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
-    cp_async_wait<1>();
-    __syncthreads();                                             // tile k (and Q) have landed
-    float acc[4][4];
+    float pad[4] = {0.f, 0.f, 0.f, 0.f};
+    if (kp) {
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) acc[x][y] = 0.f;
-    tile_abt<BS, D>(Qs, Bs + (k & 1) * TILE, ty, tx, acc);
-    long long base, si, sj;
-    tile_address(vl, p, r, c, rp + k, base, si, sj);
-    float* tile = Pb + base;
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      float mx = -INFINITY;
-#pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const int j = tx + y * C::TX;
-        float v = acc[x][y] * scale;
-        if (kp) v -= kp[c * BS + j];
-        acc[x][y] = v;
-        mx = fmaxf(mx, v);
-        if (active) tile[(long long)(ty * 4 + x) * si + j] = v;
-      }
-      mx = group_max<C::TX>(mx);
-      const float m_new = fmaxf(m[x], mx);
-      float s = 0.f;
-#pragma unroll
-      for (int y = 0; y < 4; ++y) s += __expf(acc[x][y] - m_new);
-      s = group_sum<C::TX>(s);
-      l[x] = l[x] * __expf(m[x] - m_new) + s;
-      m[x] = m_new;
+      for (int y = 0; y < 4; ++y) pad[y] = kp[c * BS + y] * LOG2_E;
     }
-    __syncthreads();                                             // buffer k&1 may be refilled
-  }
-  float inv[4];
+    cp_async_wait<1>();
+    group_sync<C::NT>(g);                                        // tile k (and Q) have landed
+    float* tile = mine + (long long)k * rt.step;
 #pragma unroll
-  for (int x = 0; x < 4; ++x) {
-    const float z = l[x] + (float)(L - nblk * BS) * __expf(-m[x]);
+    for (int half = 0; half < R / 4; ++half) {
+      float acc[4][4];
+      tile_abt<BS, D>(Qs, Bs + (k & 1) * C::TILE, ty * R + half * 4, tx, acc);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        float &mx = m[half * 4 + x], &lx = l[half * 4 + x];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) acc[x][y] = fmaf(acc[x][y], scale2, -pad[y]);
+        store_vals(tile + (half * 4 + x) * rt.si, make_float4(acc[x][0], acc[x][1], acc[x][2], acc[x][3]), vec);
+        const float m_new = fmaxf(mx, fmaxf(fmaxf(acc[x][0], acc[x][1]), fmaxf(acc[x][2], acc[x][3])));
+        const float s = (ex2(acc[x][0] - m_new) + ex2(acc[x][1] - m_new)) + (ex2(acc[x][2] - m_new) + ex2(acc[x][3] - m_new));
+        lx = fmaf(lx, ex2(mx - m_new), s);
+        mx = m_new;
+      }
+    }
+    group_sync<C::NT>(g);                                        // buffer k&1 may be refilled
+  }
+  c_cur = nblk > 0 ? cols[0] : 0;
+  c_nxt = nblk > 1 ? cols[1] : 0;
+  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Vb, c_cur * BS, t);
+  cp_async_commit();
+  float inv[R];
+#pragma unroll
+  for (int x = 0; x < R; ++x) {
+    const float row_m = group_max<C::TX>(m[x]);
+    const float z = group_sum<C::TX>(l[x] * ex2(m[x] - row_m)) + (float)(L - nblk * BS) * ex2(-row_m);
+    m[x] = row_m;
     inv[x] = 1.0f / z;
   }
 
   // ---- pass 2: probabilities over the scores, O = P V
-  float o[4][C::TN];
+  Sums<BS, D, R> o;
+  float4 sc[R];                                                  // scores of the tile about to be used
+  auto fetch_scores = [&](int k) {
+    const float* tile = mine + (long long)k * rt.step;
 #pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < C::TN; ++y) o[x][y] = 0.f;
-  c_cur = nblk > 0 ? cols[0] : 0;
-  c_nxt = nblk > 1 ? cols[1] : 0;
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, C::SA, Vb + (long long)c_cur * BS * lv.sl, lv.sl, lv.sd, t);
-  cp_async_commit();
-  float sc[4][4];                                                // scores of the tile about to be used
-  auto fetch_scores = [&](int k, int c) {
-    long long base, si, sj;
-    tile_address(vl, p, r, c, rp + k, base, si, sj);
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) sc[x][y] = Pb[base + (long long)(ty * 4 + x) * si + tx + y * C::TX];
+    for (int x = 0; x < R; ++x) sc[x] = load_vals(tile + x * rt.si, vec);
   };
-  if (nblk > 0) fetch_scores(0, c_cur);
+  if (nblk > 0) fetch_scores(0);
   for (int k = 0; k < nblk; ++k) {
-    const int c = c_cur;
     if (k + 1 < nblk)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * TILE, C::SA, Vb + (long long)c_nxt * BS * lv.sl, lv.sl, lv.sd, t);
+      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
     cp_async_commit();
-    long long base, si, sj;
-    tile_address(vl, p, r, c, rp + k, base, si, sj);
-    float* tile = Pb + base;
+    float* tile = mine + (long long)k * rt.step;
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int half = 0; half < R / 4; ++half) {
+      float pr[4][4];
 #pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const int j = tx + y * C::TX;
-        const float pv = (inv[x] == 0.f) ? 0.f : __expf(sc[x][y] - m[x]) * inv[x];
-        if (active) tile[(long long)(ty * 4 + x) * si + j] = pv;
-        Ps[(ty * 4 + x) * C::SP + j] = pv;
+      for (int x = 0; x < 4; ++x) {
+        const int i = half * 4 + x;
+        const float v[4] = {sc[i].x, sc[i].y, sc[i].z, sc[i].w};
+#pragma unroll
+        for (int y = 0; y < 4; ++y) pr[x][y] = inv[i] == 0.f ? 0.f : ex2(v[y] - m[i]) * inv[i];
+        store_vals(tile + i * rt.si, make_float4(pr[x][0], pr[x][1], pr[x][2], pr[x][3]), vec);
       }
-    if (k + 1 < nblk) fetch_scores(k + 1, c_nxt);                // in flight during the product below
+      put_transposed<BS>(Ps, R / 4 * ty + half, tx, pr);
+    }
+    if (k + 1 < nblk) fetch_scores(k + 1);                       // in flight during the product below
     c_cur = c_nxt;
     c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
     cp_async_wait<1>();
-    __syncthreads();                                             // V tile k has landed, Ps is complete
-    tile_ab<BS, D>(Ps, Bs + (k & 1) * TILE, ty, tx, o);
-    __syncthreads();                                             // Ps and buffer k&1 may be overwritten
+    group_sync<C::NT>(g);                                        // V tile k has landed, Ps is complete
+    tile_atb<BS, D, R>(Ps, Bs + (k & 1) * C::TILE, ty, tx, o);
+    group_sync<C::NT>(g);                                        // Ps and buffer k&1 may be overwritten
   }
   cp_async_wait<0>();
-  if (active) store_out<BS, D>(O + (long long)bh * lo.bh_stride, lo, r * BS, ty, tx, o);
+  store_out<BS, D, R>(O + (long long)bh * lo.bh_stride, lo, r * BS, ty, tx, o);
 }
 
 // ------------------------------------------------------------------------------ backward, row side
 //   t = dP.P ; s = rowsum(t) ; dS = (t - P s) scale ; dQ = dS K     (models/block_attn.cu:90-130, :498-516)
-template <int BS, int D>
-__global__ void __launch_bounds__(256, 3) fused_bwd_row_kernel(const float* __restrict__ dO, OperandLayout ldo,
+template <int BS, int D, int R>
+__global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) fused_bwd_row_kernel(const float* __restrict__ dO, OperandLayout ldo,
                                                                const float* __restrict__ V, OperandLayout lv,
                                                                const float* __restrict__ K, OperandLayout lk,
                                                                const float* __restrict__ P, ValueLayout vp, float* dS,
                                                                ValueLayout vds, float* __restrict__ dQ,
                                                                OperandLayout ldq, Pattern p, int BH, float scale) {
-  using C = Cfg<BS, D>;
-  constexpr int TILE = BS * C::SA;
+  using C = Cfg<BS, D, R>;
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int r = blockIdx.x;
-  const int bh_raw = blockIdx.y * C::G + g;
-  const bool active = bh_raw < BH;
-  const int bh = active ? bh_raw : BH - 1;
-  float* As = smem + g * (3 * TILE + BS * C::SP);               // dO tile
-  float* Bs = As + TILE;                                        // two buffers: V tiles, then K tiles
-  float* Ss = As + 3 * TILE;                                    // dS tile
+  const int r = blockIdx.x, bh = blockIdx.y * C::G + g;
+  if (bh >= BH) return;
+  float* As = smem + g * two_pass_floats<BS, D, R>();              // dO tile
+  float* Bs = As + ONE<BS, D, R>;                                // two buffers: V tiles, then K tiles
+  float* Ss = As;                                               // dS tile, pass 2
 
   const int rp = p.row_ptr[r], nblk = p.row_ptr[r + 1] - rp;
   const int* cols = p.col_idx + rp;
-  const float* Vb = V + (long long)bh * lv.bh_stride;
-  const float* Kb = K + (long long)bh * lk.bh_stride;
-  const float* Pb = P + (long long)bh * vp.bh_stride;
-  float* dSb = dS + (long long)bh * vds.bh_stride;
+  const Operand Vb(V, lv, bh), Kb(K, lk, bh);
+  const RowTiles rp_t = RowTiles::of<BS>(vp, rp, nblk), rs_t = RowTiles::of<BS>(vds, rp, nblk);
+  const float* Pb = P + (long long)bh * vp.bh_stride + rp_t.base + ty * R * rp_t.si + tx * 4;   // the thread's values of the first tile
+  float* dSb = dS + (long long)bh * vds.bh_stride + rs_t.base + ty * R * rs_t.si + tx * 4;
+  const bool vec_p = vec_ok(Pb), vec_s = vec_ok(dSb);
 
   int c_cur = nblk > 0 ? cols[0] : 0, c_nxt = nblk > 1 ? cols[1] : 0;
-  load_tile<BS, D, C::NT>(As, C::SA, dO + (long long)bh * ldo.bh_stride + (long long)r * BS * ldo.sl, ldo.sl, ldo.sd, t);
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, C::SA, Vb + (long long)c_cur * BS * lv.sl, lv.sl, lv.sd, t);
+  load_tile<BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
+  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Vb, c_cur * BS, t);
   cp_async_commit();
 
   // ---- pass 1: dP into the dS tiles, row sums of dP.P
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  float s[R];
+#pragma unroll
+  for (int x = 0; x < R; ++x) s[x] = 0.f;
   for (int k = 0; k < nblk; ++k) {
-    const int c = c_cur;
     if (k + 1 < nblk)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * TILE, C::SA, Vb + (long long)c_nxt * BS * lv.sl, lv.sl, lv.sd, t);
+      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
-    long long b1, s1, t1, b2, s2, t2;
-    tile_address(vp, p, r, c, rp + k, b1, s1, t1);
-    tile_address(vds, p, r, c, rp + k, b2, s2, t2);
-    float pv[4][4];                                              // requested before the wait: both latencies overlap
+    float4 pv[R];                                                // requested before the wait: both latencies overlap
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) pv[x][y] = Pb[b1 + (long long)(ty * 4 + x) * s1 + tx + y * C::TX];
+    for (int x = 0; x < R; ++x) pv[x] = load_vals(Pb + (long long)k * rp_t.step + x * rp_t.si, vec_p);
     cp_async_wait<1>();
-    __syncthreads();
-    float acc[4][4];
+    group_sync<C::NT>(g);
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int half = 0; half < R / 4; ++half) {
+      float acc[4][4];
+      tile_abt<BS, D>(As, Bs + (k & 1) * C::TILE, ty * R + half * 4, tx, acc);
 #pragma unroll
-      for (int y = 0; y < 4; ++y) acc[x][y] = 0.f;
-    tile_abt<BS, D>(As, Bs + (k & 1) * TILE, ty, tx, acc);
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        s[x] = fmaf(acc[x][y], pv[x][y], s[x]);
-        if (active) dSb[b2 + (long long)(ty * 4 + x) * s2 + tx + y * C::TX] = acc[x][y];
+      for (int x = 0; x < 4; ++x) {
+        const int i = half * 4 + x;
+        s[i] = fmaf(acc[x][0], pv[i].x, s[i]);
+        s[i] = fmaf(acc[x][1], pv[i].y, s[i]);
+        s[i] = fmaf(acc[x][2], pv[i].z, s[i]);
+        s[i] = fmaf(acc[x][3], pv[i].w, s[i]);
+        store_vals(dSb + (long long)k * rs_t.step + i * rs_t.si, make_float4(acc[x][0], acc[x][1], acc[x][2], acc[x][3]), vec_s);
       }
-    __syncthreads();
+    }
+    group_sync<C::NT>(g);
   }
 #pragma unroll
-  for (int x = 0; x < 4; ++x) s[x] = group_sum<C::TX>(s[x]);
+  for (int x = 0; x < R; ++x) s[x] = group_sum<C::TX>(s[x]);
 
   // ---- pass 2: dS over dP, dQ = dS K
-  float o[4][C::TN];
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < C::TN; ++y) o[x][y] = 0.f;
+  Sums<BS, D, R> o;
   c_cur = nblk > 0 ? cols[0] : 0;
   c_nxt = nblk > 1 ? cols[1] : 0;
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, C::SA, Kb + (long long)c_cur * BS * lk.sl, lk.sl, lk.sd, t);
+  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Kb, c_cur * BS, t);
   cp_async_commit();
   for (int k = 0; k < nblk; ++k) {
-    const int c = c_cur;
     if (k + 1 < nblk)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * TILE, C::SA, Kb + (long long)c_nxt * BS * lk.sl, lk.sl, lk.sd, t);
+      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
-    long long b1, s1, t1, b2, s2, t2;
-    tile_address(vp, p, r, c, rp + k, b1, s1, t1);
-    tile_address(vds, p, r, c, rp + k, b2, s2, t2);
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int half = 0; half < R / 4; ++half) {
+      float ds[4][4];
 #pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const int j = tx + y * C::TX;
-        float* e = dSb + b2 + (long long)(ty * 4 + x) * s2 + j;
-        const float pv = Pb[b1 + (long long)(ty * 4 + x) * s1 + j];
-        const float ds = (*e * pv - pv * s[x]) * scale;
-        if (active) *e = ds;
-        Ss[(ty * 4 + x) * C::SP + j] = ds;
+      for (int x = 0; x < 4; ++x) {
+        const int i = half * 4 + x;
+        float* e = dSb + (long long)k * rs_t.step + i * rs_t.si;
+        const float4 dp = load_vals(e, vec_s), pv = load_vals(Pb + (long long)k * rp_t.step + i * rp_t.si, vec_p);
+        ds[x][0] = (dp.x * pv.x - pv.x * s[i]) * scale;
+        ds[x][1] = (dp.y * pv.y - pv.y * s[i]) * scale;
+        ds[x][2] = (dp.z * pv.z - pv.z * s[i]) * scale;
+        ds[x][3] = (dp.w * pv.w - pv.w * s[i]) * scale;
+        store_vals(e, make_float4(ds[x][0], ds[x][1], ds[x][2], ds[x][3]), vec_s);
       }
+      put_transposed<BS>(Ss, R / 4 * ty + half, tx, ds);
+    }
     cp_async_wait<1>();
-    __syncthreads();
-    tile_ab<BS, D>(Ss, Bs + (k & 1) * TILE, ty, tx, o);
-    __syncthreads();
+    group_sync<C::NT>(g);
+    tile_atb<BS, D, R>(Ss, Bs + (k & 1) * C::TILE, ty, tx, o);
+    group_sync<C::NT>(g);
   }
   cp_async_wait<0>();
-  if (active) store_out<BS, D>(dQ + (long long)bh * ldq.bh_stride, ldq, r * BS, ty, tx, o);
+  store_out<BS, D, R>(dQ + (long long)bh * ldq.bh_stride, ldq, r * BS, ty, tx, o);
 }
 
 // Row backward when O is at hand: rowsum(dP.P) = rowsum(dO.O) (delta), so dS of a tile needs nothing
 // from the other tiles of its row and one pass suffices.  Two stages per block, V tile (for dP) and
 // K tile (for dQ); the copy of one is in flight while the other is used.
-template <int BS, int D>
-__global__ void __launch_bounds__(256, 3) fused_bwd_row_delta_kernel(const float* __restrict__ dO, OperandLayout ldo,
+template <int BS, int D, int R>
+__global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) fused_bwd_row_delta_kernel(const float* __restrict__ dO, OperandLayout ldo,
                                                                      const float* __restrict__ O, OperandLayout lo,
                                                                      const float* __restrict__ V, OperandLayout lv,
                                                                      const float* __restrict__ K, OperandLayout lk,
@@ -455,145 +551,147 @@ __global__ void __launch_bounds__(256, 3) fused_bwd_row_delta_kernel(const float
                                                                      float* __restrict__ dS, ValueLayout vds,
                                                                      float* __restrict__ dQ, OperandLayout ldq,
                                                                      Pattern p, int BH, float scale) {
-  using C = Cfg<BS, D>;
-  constexpr int TILE = BS * C::SA;
+  using C = Cfg<BS, D, R>;
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int r = blockIdx.x;
-  const int bh_raw = blockIdx.y * C::G + g;
-  const bool active = bh_raw < BH;
-  const int bh = active ? bh_raw : BH - 1;
-  float* As = smem + g * (3 * TILE + BS * C::SP);               // dO tile
-  float* Vs = As + TILE;
-  float* Ks = As + 2 * TILE;
-  float* Ss = As + 3 * TILE;                                    // dS tile
+  const int r = blockIdx.x, bh = blockIdx.y * C::G + g;
+  if (bh >= BH) return;
+  float* As = smem + g * (3 * C::TILE + C::VALS);               // dO tile
+  float* Vs = As + C::TILE;
+  float* Ks = As + 2 * C::TILE;
+  float* Ss = As + 3 * C::TILE;                                 // dS tile
 
   const int rp = p.row_ptr[r], nblk = p.row_ptr[r + 1] - rp;
   const int* cols = p.col_idx + rp;
-  const float* Vb = V + (long long)bh * lv.bh_stride;
-  const float* Kb = K + (long long)bh * lk.bh_stride;
-  const float* Pb = P + (long long)bh * vp.bh_stride;
-  float* dSb = dS + (long long)bh * vds.bh_stride;
+  const Operand Vb(V, lv, bh), Kb(K, lk, bh);
+  const RowTiles rp_t = RowTiles::of<BS>(vp, rp, nblk), rs_t = RowTiles::of<BS>(vds, rp, nblk);
+  const float* Pb = P + (long long)bh * vp.bh_stride + rp_t.base + ty * R * rp_t.si + tx * 4;   // the thread's values of the first tile
+  float* dSb = dS + (long long)bh * vds.bh_stride + rs_t.base + ty * R * rs_t.si + tx * 4;
+  const bool vec_p = vec_ok(Pb), vec_s = vec_ok(dSb);
 
   int c_cur = nblk > 0 ? cols[0] : 0, c_nxt = nblk > 1 ? cols[1] : 0;
-  load_tile<BS, D, C::NT>(As, C::SA, dO + (long long)bh * ldo.bh_stride + (long long)r * BS * ldo.sl, ldo.sl, ldo.sd, t);
-  if (nblk > 0) load_tile<BS, D, C::NT>(Vs, C::SA, Vb + (long long)c_cur * BS * lv.sl, lv.sl, lv.sd, t);
+  load_tile<BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
+  if (nblk > 0) load_tile<BS, D, C::NT>(Vs, Vb, c_cur * BS, t);
   cp_async_commit();
-  if (nblk > 0) load_tile<BS, D, C::NT>(Ks, C::SA, Kb + (long long)c_cur * BS * lk.sl, lk.sl, lk.sd, t);
+  if (nblk > 0) load_tile<BS, D, C::NT>(Ks, Kb, c_cur * BS, t);
   cp_async_commit();
 
-  float delta[4] = {0.f, 0.f, 0.f, 0.f};
-  float o[4][C::TN];
+  float delta[R];
 #pragma unroll
-  for (int x = 0; x < 4; ++x)
+  for (int x = 0; x < R; ++x) delta[x] = 0.f;
+  Sums<BS, D, R> o;
+  float4 pv[R];                                                  // the tile's probabilities, requested one tile ahead
+  auto fetch_p = [&](int k) {
 #pragma unroll
-    for (int y = 0; y < C::TN; ++y) o[x][y] = 0.f;
+    for (int x = 0; x < R; ++x) pv[x] = load_vals(Pb + (long long)k * rp_t.step + x * rp_t.si, vec_p);
+  };
+  if (nblk > 0) fetch_p(0);
 
   for (int k = 0; k < nblk; ++k) {
-    const int c = c_cur;
-    long long b1, s1, t1, b2, s2, t2;
-    tile_address(vp, p, r, c, rp + k, b1, s1, t1);
-    tile_address(vds, p, r, c, rp + k, b2, s2, t2);
-    float pv[4][4];                                              // requested before the wait: the latencies overlap
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) pv[x][y] = Pb[b1 + (long long)(ty * 4 + x) * s1 + tx + y * C::TX];
     cp_async_wait<1>();
-    __syncthreads();                                             // V tile k (and dO) have landed
+    group_sync<C::NT>(g);                                        // V tile k (and dO) have landed
     if (k == 0) {
-      const float* Ob = O + (long long)bh * lo.bh_stride + (long long)(r * BS + ty * 4) * lo.sl;
+      const float* Ob = O + (long long)bh * lo.bh_stride + (long long)(r * BS + ty * R) * lo.sl;
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        float a = 0.f;
+      for (int x = 0; x < R; ++x) {
+        float a = 0.f, d[C::TN];
+        load_vec<BS, D, R>(As, ty * R + x, tx, d);
 #pragma unroll
-        for (int y = 0; y < C::TN; ++y) {
-          const int n = out_col<BS, D>(tx, y);
-          a = fmaf(As[(ty * 4 + x) * C::SA + n], Ob[(long long)x * lo.sl + (long long)n * lo.sd], a);
-        }
+        for (int y = 0; y < C::TN; ++y) a = fmaf(d[y], Ob[(long long)x * lo.sl + (long long)out_col<BS, D, R>(tx, y) * lo.sd], a);
         delta[x] = group_sum<C::TX>(a);
       }
     }
-    float acc[4][4];
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
+    for (int half = 0; half < R / 4; ++half) {
+      float acc[4][4];
+      tile_abt<BS, D>(As, Vs, ty * R + half * 4, tx, acc);
 #pragma unroll
-      for (int y = 0; y < 4; ++y) acc[x][y] = 0.f;
-    tile_abt<BS, D>(As, Vs, ty, tx, acc);
+      for (int x = 0; x < 4; ++x) {
+        const int i = half * 4 + x;
+        const float pr[4] = {pv[i].x, pv[i].y, pv[i].z, pv[i].w};
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const int j = tx + y * C::TX;
-        const float ds = pv[x][y] * (acc[x][y] - delta[x]) * scale;
-        if (active) dSb[b2 + (long long)(ty * 4 + x) * s2 + j] = ds;
-        Ss[(ty * 4 + x) * C::SP + j] = ds;
+        for (int y = 0; y < 4; ++y) acc[x][y] = pr[y] * (acc[x][y] - delta[i]) * scale;
+        store_vals(dSb + (long long)k * rs_t.step + i * rs_t.si, make_float4(acc[x][0], acc[x][1], acc[x][2], acc[x][3]), vec_s);
       }
-    __syncthreads();                                             // Ss complete, V buffer free
-    if (k + 1 < nblk) load_tile<BS, D, C::NT>(Vs, C::SA, Vb + (long long)c_nxt * BS * lv.sl, lv.sl, lv.sd, t);
+      put_transposed<BS>(Ss, R / 4 * ty + half, tx, acc);
+    }
+    group_sync<C::NT>(g);                                        // Ss complete, V buffer free
+    if (k + 1 < nblk) {
+      load_tile<BS, D, C::NT>(Vs, Vb, c_nxt * BS, t);
+      fetch_p(k + 1);
+    }
     cp_async_commit();
     cp_async_wait<1>();
-    __syncthreads();                                             // K tile k has landed
-    tile_ab<BS, D>(Ss, Ks, ty, tx, o);
-    __syncthreads();                                             // Ss and the K buffer are free
-    if (k + 1 < nblk) load_tile<BS, D, C::NT>(Ks, C::SA, Kb + (long long)c_nxt * BS * lk.sl, lk.sl, lk.sd, t);
+    group_sync<C::NT>(g);                                        // K tile k has landed
+    tile_atb<BS, D, R>(Ss, Ks, ty, tx, o);
+    group_sync<C::NT>(g);                                        // Ss and the K buffer are free
+    if (k + 1 < nblk) load_tile<BS, D, C::NT>(Ks, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
   }
   cp_async_wait<0>();
-  if (active) store_out<BS, D>(dQ + (long long)bh * ldq.bh_stride, ldq, r * BS, ty, tx, o);
+  store_out<BS, D, R>(dQ + (long long)bh * ldq.bh_stride, ldq, r * BS, ty, tx, o);
 }
 
 // ------------------------------------------------------------------------------ backward, column side
 //   dK[c] = sum_r dS(r,c)^T Q[r],  dV[c] = sum_r P(r,c)^T dO[r]     (models/block_attn.cu:526-536)
 // Two stages per entry of the column: (dS, Q) for dK and (P, dO) for dV; the copy of one stage is in
 // flight while the other is used.
-template <int BS, int D>
-__global__ void __launch_bounds__(256, 3) fused_bwd_col_kernel(const float* __restrict__ dS, ValueLayout vds,
+// SPLIT: a cluster of SPLIT_WAYS CTAs per column.  Discovered masks have columns that every row selects; one CTA would walk
+// such a column long after the others are done.  The CTAs of the cluster take a share of its entries each and the
+// first adds the others' sums, in their order, through distributed shared memory.  Columns below SPLIT_MIN entries
+// are left to the first CTA; the others end at once.  Eight CTAs per column were slower than four (16 matrices, L = 1024, blocks
+// of 32 at 15 %: 57 against 24 us, 41 without a split).
+constexpr int SPLIT_WAYS = 4, SPLIT_MIN = 3;
+template <int BS, int D, int R, bool SPLIT>
+__global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) fused_bwd_col_kernel(const float* __restrict__ dS, ValueLayout vds,
                                                                const float* __restrict__ P, ValueLayout vp,
                                                                const float* __restrict__ Q, OperandLayout lq,
                                                                const float* __restrict__ dO, OperandLayout ldo,
                                                                float* __restrict__ dK, OperandLayout ldk,
                                                                float* __restrict__ dV, OperandLayout ldv, Pattern p,
                                                                int BH) {
-  using C = Cfg<BS, D>;
+  using C = Cfg<BS, D, R>;
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int c = blockIdx.x;
+  const int c = SPLIT ? blockIdx.x / SPLIT_WAYS : blockIdx.x, part = SPLIT ? blockIdx.x % SPLIT_WAYS : 0;
   const int bh_raw = blockIdx.y * C::G + g;
   const bool active = bh_raw < BH;
-  const int bh = active ? bh_raw : BH - 1;
-  float* dSs = smem + g * (2 * BS * C::SA + 2 * BS * C::SP);
-  float* Qs = dSs + BS * C::SP;
-  float* Ps = Qs + BS * C::SA;
-  float* Os = Ps + BS * C::SP;
+  if (!SPLIT && !active) return;
+  const int bh = active ? bh_raw : BH - 1;                      // SPLIT: the cluster barriers take every thread
+  int e0 = p.col_ptr[c], e1 = p.col_ptr[c + 1];
+  const bool shared = SPLIT && e1 - e0 >= SPLIT_MIN;
+  if (SPLIT && !shared && (part > 0 || !active)) return;
+  if (shared) {
+    const int first = e0, n = e1 - e0;
+    e0 = first + n * part / SPLIT_WAYS;
+    e1 = active ? first + n * (part + 1) / SPLIT_WAYS : e0;
+  }
+  float* dSs = smem + g * (2 * C::TILE + 2 * C::VALS);
+  float* Qs = dSs + C::VALS;
+  float* Ps = Qs + C::TILE;
+  float* Os = Ps + C::VALS;
 
   const float* dSb = dS + (long long)bh * vds.bh_stride;
   const float* Pb = P + (long long)bh * vp.bh_stride;
-  const float* Qb = Q + (long long)bh * lq.bh_stride;
-  const float* dOb = dO + (long long)bh * ldo.bh_stride;
+  const Operand Qb(Q, lq, bh), dOb(dO, ldo, bh);
 
-  float ak[4][C::TN], av[4][C::TN];
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < C::TN; ++y) { ak[x][y] = 0.f; av[x][y] = 0.f; }
+  Sums<BS, D, R> ak, av;
 
-  const int e0 = p.col_ptr[c], e1 = p.col_ptr[c + 1];
   auto fetch_k = [&](int r, int blk) {                          // stage A: dS tile and Q rows of entry (r, blk)
     long long b1, s1, t1;
     tile_address(vds, p, r, c, blk, b1, s1, t1);
-    load_tile<BS, BS, C::NT>(dSs, C::SP, dSb + b1, s1, t1, t);
-    load_tile<BS, D, C::NT>(Qs, C::SA, Qb + (long long)r * BS * lq.sl, lq.sl, lq.sd, t);
+    load_tile<BS, BS, C::NT>(dSs, Operand(dSb + b1, (int)s1), 0, t);
+    load_tile<BS, D, C::NT>(Qs, Qb, r * BS, t);
   };
   auto fetch_v = [&](int r, int blk) {                          // stage B: P tile and dO rows
     long long b2, s2, t2;
     tile_address(vp, p, r, c, blk, b2, s2, t2);
-    load_tile<BS, BS, C::NT>(Ps, C::SP, Pb + b2, s2, t2, t);
-    load_tile<BS, D, C::NT>(Os, C::SA, dOb + (long long)r * BS * ldo.sl, ldo.sl, ldo.sd, t);
+    load_tile<BS, BS, C::NT>(Ps, Operand(Pb + b2, (int)s2), 0, t);
+    load_tile<BS, D, C::NT>(Os, dOb, r * BS, t);
   };
   int r_cur = e0 < e1 ? p.row_idx[e0] : 0, b_cur = e0 < e1 ? p.csc_pos[e0] : 0;
   if (e0 < e1) fetch_k(r_cur, b_cur);
@@ -603,73 +701,121 @@ __global__ void __launch_bounds__(256, 3) fused_bwd_col_kernel(const float* __re
     fetch_v(r_cur, b_cur);                                       // stage B was released at the end of the last iteration
     cp_async_commit();
     cp_async_wait<1>();
-    __syncthreads();                                             // stage A has landed
-    tile_atb<BS, D>(dSs, Qs, ty, tx, ak);
-    __syncthreads();                                             // stage A may be refilled
+    group_sync<C::NT>(g);                                        // stage A has landed
+    tile_atb<BS, D, R>(dSs, Qs, ty, tx, ak);
+    group_sync<C::NT>(g);                                        // stage A may be refilled
     if (e + 1 < e1) fetch_k(r_nxt, b_nxt);
     cp_async_commit();
     cp_async_wait<1>();
-    __syncthreads();                                             // stage B has landed
-    tile_atb<BS, D>(Ps, Os, ty, tx, av);
-    __syncthreads();
+    group_sync<C::NT>(g);                                        // stage B has landed
+    tile_atb<BS, D, R>(Ps, Os, ty, tx, av);
+    group_sync<C::NT>(g);
     r_cur = r_nxt;
     b_cur = b_nxt;
   }
   cp_async_wait<0>();
-  if (active) {
-    store_out<BS, D>(dK + (long long)bh * ldk.bh_stride, ldk, c * BS, ty, tx, ak);
-    store_out<BS, D>(dV + (long long)bh * ldv.bh_stride, ldv, c * BS, ty, tx, av);
+  if (shared) {                                                  // the same for all CTAs of the cluster
+    auto cluster = cooperative_groups::this_cluster();
+    group_sync<C::NT>(g);                                        // the tiles are read: their place takes the sums
+    pair_t* mine = reinterpret_cast<pair_t*>(dSs) + t;           // pair i of thread t at i * NT + t
+    if (part > 0) {
+#pragma unroll
+      for (int x = 0; x < R / 2; ++x)
+#pragma unroll
+        for (int y = 0; y < C::TN; ++y) {
+          mine[(x * C::TN + y) * C::NT] = ak.v[x][y];
+          mine[(R / 2 * C::TN + x * C::TN + y) * C::NT] = av.v[x][y];
+        }
+    }
+    cluster.sync();
+    if (part == 0) {
+      auto add = [](pair_t& sum, pair_t v) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum) : "l"(v)); };
+      for (int q = 1; q < SPLIT_WAYS; ++q) {
+        const pair_t* theirs = cluster.map_shared_rank(mine, q);
+#pragma unroll
+        for (int x = 0; x < R / 2; ++x)
+#pragma unroll
+          for (int y = 0; y < C::TN; ++y) {
+            add(ak.v[x][y], theirs[(x * C::TN + y) * C::NT]);
+            add(av.v[x][y], theirs[(R / 2 * C::TN + x * C::TN + y) * C::NT]);
+          }
+      }
+    }
+    cluster.sync();                                              // nobody leaves while its sums are read
+    if (part > 0 || !active) return;
   }
+  store_out<BS, D, R>(dK + (long long)bh * ldk.bh_stride, ldk, c * BS, ty, tx, ak);
+  store_out<BS, D, R>(dV + (long long)bh * ldv.bh_stride, ldv, c * BS, ty, tx, av);
 }
 
-template <int BS, int D> constexpr size_t smem_row() { return sizeof(float) * Cfg<BS, D>::G * (3 * BS * Cfg<BS, D>::SA + BS * Cfg<BS, D>::SP); }
-template <int BS, int D> constexpr size_t smem_col() { return sizeof(float) * Cfg<BS, D>::G * (2 * BS * Cfg<BS, D>::SA + 2 * BS * Cfg<BS, D>::SP); }
+template <int BS, int D, int R> constexpr size_t smem_two_pass() { return sizeof(float) * Cfg<BS, D, R>::G * two_pass_floats<BS, D, R>(); }
+template <int BS, int D, int R> constexpr size_t smem_row() { return sizeof(float) * Cfg<BS, D, R>::G * (3 * Cfg<BS, D, R>::TILE + Cfg<BS, D, R>::VALS); }
+template <int BS, int D, int R> constexpr size_t smem_col() { return sizeof(float) * Cfg<BS, D, R>::G * (2 * Cfg<BS, D, R>::TILE + 2 * Cfg<BS, D, R>::VALS); }
 
-template <int BS, int D>
+constexpr int SPLIT_WAVES = 4;
+
+template <int BS, int D, int R>
 int set_attrs() {
   static bool done[64] = {};
   int dev = 0;
   SPION_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 64 && done[dev]) return SPION_OK;
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_fwd_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D>()));
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D>()));
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_delta_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D>()));
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_fwd_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_delta_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D, R>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
   if (dev < 64) done[dev] = true;
   return SPION_OK;
 }
 
-template <int BS, int D>
+template <int BS, int D, int R>
 int fwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V, OperandLayout lv,
                const float* keypad, float floor_v, float* P, ValueLayout vl, float* O, OperandLayout lo, Pattern p,
                int BH, int L, float scale, cudaStream_t st) {
-  int rc = set_attrs<BS, D>();
+  int rc = set_attrs<BS, D, R>();
   if (rc) return rc;
-  const dim3 grid(p.nb, (BH + Cfg<BS, D>::G - 1) / Cfg<BS, D>::G);
-  fused_fwd_kernel<BS, D><<<grid, 256, smem_row<BS, D>(), st>>>(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH,
+  const dim3 grid(p.nb, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
+  fused_fwd_kernel<BS, D, R><<<grid, Cfg<BS, D, R>::CTA, smem_two_pass<BS, D, R>(), st>>>(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH,
                                                                L, scale);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
 
-template <int BS, int D>
+template <int BS, int D, int R>
 int bwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V, OperandLayout lv,
                const float* P, ValueLayout vp, const float* O, OperandLayout lo, const float* dO, OperandLayout ldo,
                float* dS, ValueLayout vds, float* dQ, OperandLayout ldq, float* dK, OperandLayout ldk, float* dV,
                OperandLayout ldv, Pattern p, int BH, float scale, cudaStream_t st, spion_ctx* prof) {
-  int rc = set_attrs<BS, D>();
+  int rc = set_attrs<BS, D, R>();
   if (rc) return rc;
-  const dim3 grid(p.nb, (BH + Cfg<BS, D>::G - 1) / Cfg<BS, D>::G);
+  const dim3 grid(p.nb, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
   if (O)
-    fused_bwd_row_delta_kernel<BS, D><<<grid, 256, smem_row<BS, D>(), st>>>(dO, ldo, O, lo, V, lv, K, lk, P, vp, dS, vds,
+    fused_bwd_row_delta_kernel<BS, D, R><<<grid, Cfg<BS, D, R>::CTA, smem_row<BS, D, R>(), st>>>(dO, ldo, O, lo, V, lv, K, lk, P, vp, dS, vds,
                                                                            dQ, ldq, p, BH, scale);
   else
-    fused_bwd_row_kernel<BS, D><<<grid, 256, smem_row<BS, D>(), st>>>(dO, ldo, V, lv, K, lk, P, vp, dS, vds, dQ, ldq, p,
+    fused_bwd_row_kernel<BS, D, R><<<grid, Cfg<BS, D, R>::CTA, smem_two_pass<BS, D, R>(), st>>>(dO, ldo, V, lv, K, lk, P, vp, dS, vds, dQ, ldq, p,
                                                                      BH, scale);
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_BWD_ROW);
-  fused_bwd_col_kernel<BS, D><<<grid, 256, smem_col<BS, D>(), st>>>(dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p,
-                                                                   BH);
+  // Many (b,h) matrices even out columns of different lengths by themselves; below SPLIT_WAVES waves of CTAs the longest
+  // column would decide, and there is room for the CTAs that a split column takes.
+  if ((long long)grid.x * grid.y < SPLIT_WAVES * 148LL * Cfg<BS, D, R>::RESIDENT) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid.x * SPLIT_WAYS, grid.y);
+    cfg.blockDim = dim3(Cfg<BS, D, R>::CTA);
+    cfg.dynamicSmemBytes = smem_col<BS, D, R>();
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = SPLIT_WAYS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    SPION_CUDA_TRY(cudaLaunchKernelEx(&cfg, fused_bwd_col_kernel<BS, D, R, true>, (const float*)dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH));
+  } else {
+    fused_bwd_col_kernel<BS, D, R, false><<<grid, Cfg<BS, D, R>::CTA, smem_col<BS, D, R>(), st>>>(dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH);
+  }
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_SPMM_DKDV);
   return SPION_OK;
@@ -682,12 +828,17 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
          (value_mode == VAL_ELEMCSR || value_mode == VAL_BLOCKTILE);
 }
 
+// With eight rows per thread a block row is one warp (block 32) or four (64).  Up to two warps per scheduler (148 SMs x 4) each of
+// them is a chain of latencies, and half the rows per thread shorten it (16 matrices, L = 1024, d 32, blocks of 32 at 15 %:
+// forward 31 -> 22 us, rows 22 -> 20); above, the larger micro-tile is worth more.
+constexpr long long FEW_WARPS = 148 * 4 * 2;
 #define SPION_FUSED_DISPATCH(FN, ...)                                   \
   do {                                                                  \
-    if (p.bs == 32 && d == 32) return FN<32, 32>(__VA_ARGS__);          \
-    if (p.bs == 32 && d == 64) return FN<32, 64>(__VA_ARGS__);          \
-    if (p.bs == 64 && d == 32) return FN<64, 32>(__VA_ARGS__);          \
-    if (p.bs == 64 && d == 64) return FN<64, 64>(__VA_ARGS__);          \
+    const bool few = (long long)p.nb * BH * p.bs * p.bs / 1024 <= FEW_WARPS; \
+    if (p.bs == 32 && d == 32) return few ? FN<32, 32, 4>(__VA_ARGS__) : FN<32, 32, 8>(__VA_ARGS__); \
+    if (p.bs == 32 && d == 64) return few ? FN<32, 64, 4>(__VA_ARGS__) : FN<32, 64, 8>(__VA_ARGS__); \
+    if (p.bs == 64 && d == 32) return few ? FN<64, 32, 4>(__VA_ARGS__) : FN<64, 32, 8>(__VA_ARGS__); \
+    if (p.bs == 64 && d == 64) return few ? FN<64, 64, 4>(__VA_ARGS__) : FN<64, 64, 8>(__VA_ARGS__); \
     return SPION_ERR_UNSUPPORTED;                                       \
   } while (0)
 
