@@ -6,7 +6,50 @@
 //   backward  dP = dO V^T on the mask -> dS = softmax'(dP, P) -> dQ = dS K ; dK = dS^T Q ; dV = P^T dO
 #include <new>
 
+#include <mutex>
+
 #include "common.cuh"
+
+namespace {
+struct DevicePool { cudaMemPool_t pool; cudaStream_t stream; };
+// the pool of the current device, made on first use; nullptr if that failed
+DevicePool* device_pool() {
+  static std::mutex lock;
+  static DevicePool* pools[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> hold(lock);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    DevicePool d{};
+    uint64_t keep = 64ull << 20;
+    if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) return nullptr;
+    if (cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaMemPoolDestroy(d.pool);
+      return nullptr;
+    }
+    pools[dev] = new DevicePool(d);
+  }
+  return pools[dev];
+}
+}  // namespace
+
+int device_alloc(void** p, size_t bytes) {
+  *p = nullptr;
+  DevicePool* d = device_pool();
+  if (!d || cudaMallocFromPoolAsync(p, bytes, d->pool, d->stream) != cudaSuccess) return SPION_ERR_ALLOC;
+  return cudaStreamSynchronize(d->stream) == cudaSuccess ? SPION_OK : SPION_ERR_ALLOC;   // usable on every stream from here on
+}
+
+void device_free(void* p) {
+  if (!p) return;
+  cudaDeviceSynchronize();
+  if (DevicePool* d = device_pool()) cudaFreeAsync(p, d->stream);
+}
 
 namespace {
 
@@ -24,7 +67,7 @@ struct DeviceGuard {
 };
 
 template <typename T>
-bool dev_alloc(T** p, size_t n) { return cudaMalloc((void**)p, n * sizeof(T)) == cudaSuccess; }
+bool dev_alloc(T** p, size_t n) { return device_alloc((void**)p, n * sizeof(T)) == SPION_OK; }
 
 int rebuild_structure(spion_ctx* c) {
   c->launches += 1;
@@ -103,8 +146,8 @@ extern "C" void spion_destroy(spion_ctx* c) {
   DeviceGuard guard(c->device);
   tc_engine_release(c);
   for (int i = 0; i < SPION_PROF_MAX_MARKS; ++i) if (c->prof_ev[i]) cudaEventDestroy(c->prof_ev[i]);
-  cudaFree(c->mat); cudaFree(c->row_ptr); cudaFree(c->col_idx); cudaFree(c->blk_row); cudaFree(c->col_ptr);
-  cudaFree(c->row_idx); cudaFree(c->csc_pos); cudaFree(c->work); cudaFree(c->nnzb_dev); cudaFree(c->status_dev);
+  device_free(c->mat); device_free(c->row_ptr); device_free(c->col_idx); device_free(c->blk_row); device_free(c->col_ptr);
+  device_free(c->row_idx); device_free(c->csc_pos); device_free(c->work); device_free(c->nnzb_dev); device_free(c->status_dev);
   delete c;
 }
 

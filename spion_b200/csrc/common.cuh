@@ -121,6 +121,11 @@ static inline Pattern ctx_pattern(const spion_ctx* c) {
     }                                                                                 \
   } while (0)
 
+// Device memory of the contexts, from one pool per device that keeps up to 64 MB of what was given back: mapping and unmapping two
+// or three megabytes took 2 to 4 ms of every context's life.  Freeing waits for the device, as cudaFree does.  Any thread.
+int device_alloc(void** p, size_t bytes);
+void device_free(void* p);
+
 // ------------------------------------------------------------------ element conversions
 __device__ __forceinline__ float to_f32(float x) { return x; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 x) { return __bfloat162float(x); }

@@ -718,9 +718,9 @@ int b32_set_attrs(TcState* s, int device) {
 // band) the unused rows and the per-unit overhead cost more than the quarters the super-blocks waste
 // (measured on the L x density grid of the kernel sweep: the paths break even at 2.8 - 3.0 blocks per job).
 int b32_prepare(spion_ctx* c, TcState* s) {
-  if (!s->b32_row_rec && cudaMalloc(&s->b32_row_rec, (size_t)SPION_MAX_NB * sizeof(int4)) != cudaSuccess) return SPION_ERR_ALLOC;
-  if (!s->b32_col_rec && cudaMalloc(&s->b32_col_rec, (size_t)SPION_MAX_NB * sizeof(int4)) != cudaSuccess) return SPION_ERR_ALLOC;
-  if (!s->b32_jobs_dev && cudaMalloc(&s->b32_jobs_dev, sizeof(int)) != cudaSuccess) return SPION_ERR_ALLOC;
+  if (!s->b32_row_rec && device_alloc((void**)&s->b32_row_rec, (size_t)SPION_MAX_NB * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
+  if (!s->b32_col_rec && device_alloc((void**)&s->b32_col_rec, (size_t)SPION_MAX_NB * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
+  if (!s->b32_jobs_dev && device_alloc((void**)&s->b32_jobs_dev, sizeof(int)) != SPION_OK) return SPION_ERR_ALLOC;
   k_b32_recs<<<1, 512, 0, c->stream>>>(c->row_ptr, c->col_idx, c->nb, s->b32_row_rec, s->b32_jobs_dev);
   SPION_LAUNCH_CHECK();
   k_b32_recs<<<1, 512, 0, c->stream>>>(c->col_ptr, c->row_idx, c->nb, s->b32_col_rec, nullptr);
@@ -735,9 +735,9 @@ int b32_prepare(spion_ctx* c, TcState* s) {
 }
 
 void b32_release(TcState* s) {
-  cudaFree(s->b32_row_rec);
-  cudaFree(s->b32_col_rec);
-  cudaFree(s->b32_jobs_dev);
+  device_free(s->b32_row_rec);
+  device_free(s->b32_col_rec);
+  device_free(s->b32_jobs_dev);
   s->b32_row_rec = s->b32_col_rec = nullptr;
   s->b32_jobs_dev = nullptr;
 }

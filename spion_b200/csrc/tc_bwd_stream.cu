@@ -551,12 +551,12 @@ static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUte
 
 int stream_prepare(spion_ctx* c, TcState* s) {
   const TcView vw = tc_view(c, s);
-  if (!s->line_rec && cudaMalloc(&s->line_rec, 2 * (size_t)SPION_MAX_NB * sizeof(int4)) != cudaSuccess) return SPION_ERR_ALLOC;
+  if (!s->line_rec && device_alloc((void**)&s->line_rec, 2 * (size_t)SPION_MAX_NB * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
   if ((size_t)vw.nnzb > s->line_pair_cap) {                         // at most one pair per entry, columns and rows
-    cudaFree(s->line_pair);
+    device_free(s->line_pair);
     s->line_pair = nullptr;
     s->line_pair_cap = 0;
-    if (cudaMalloc(&s->line_pair, 2 * (size_t)vw.nnzb * sizeof(int4)) != cudaSuccess) return SPION_ERR_ALLOC;
+    if (device_alloc((void**)&s->line_pair, 2 * (size_t)vw.nnzb * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
     s->line_pair_cap = (size_t)vw.nnzb;
   }
   k_line_recs<<<1, 512, 0, c->stream>>>(vw.col_ptr, vw.row_idx, vw.csc_pos, vw.nb, s->line_rec, s->line_pair);

@@ -683,9 +683,9 @@ int run_backward(spion_ctx* c, TcState* s, const void* Q, const void* K, const v
 }
 
 void free_super(TcState* s) {
-  cudaFree(s->mat64); cudaFree(s->submask); cudaFree(s->row_ptr64); cudaFree(s->col_idx64); cudaFree(s->blk_row64);
-  cudaFree(s->col_ptr64); cudaFree(s->row_idx64); cudaFree(s->csc_pos64); cudaFree(s->work64); cudaFree(s->nnzb64_dev);
-  cudaFree(s->p64_ws); cudaFree(s->ds64_ws);
+  device_free(s->mat64); device_free(s->submask); device_free(s->row_ptr64); device_free(s->col_idx64); device_free(s->blk_row64);
+  device_free(s->col_ptr64); device_free(s->row_idx64); device_free(s->csc_pos64); device_free(s->work64); device_free(s->nnzb64_dev);
+  device_free(s->p64_ws); device_free(s->ds64_ws);
   s->mat64 = s->submask = nullptr;
   s->row_ptr64 = s->col_idx64 = s->blk_row64 = s->col_ptr64 = s->row_idx64 = s->csc_pos64 = s->work64 = s->nnzb64_dev = nullptr;
   s->p64_ws = s->ds64_ws = nullptr;
@@ -696,10 +696,10 @@ void free_super(TcState* s) {
 int ensure_super_ws(spion_ctx* c, TcState* s) {
   const size_t need = (size_t)c->BH * s->nnzb64 * 4096;
   if (need <= s->ws_elems) return SPION_OK;
-  cudaFree(s->p64_ws); cudaFree(s->ds64_ws);
+  device_free(s->p64_ws); device_free(s->ds64_ws);
   s->p64_ws = s->ds64_ws = nullptr;
   s->ws_elems = 0;
-  if (cudaMalloc(&s->p64_ws, need * 2) != cudaSuccess || cudaMalloc(&s->ds64_ws, need * 2) != cudaSuccess)
+  if (device_alloc((void**)&s->p64_ws, need * 2) != SPION_OK || device_alloc((void**)&s->ds64_ws, need * 2) != SPION_OK)
     return SPION_ERR_ALLOC;
   s->ws_elems = need;
   return SPION_OK;
@@ -710,11 +710,11 @@ int build_super(spion_ctx* c, TcState* s) {
   const int nb64 = c->nb / 2;
   const size_t cap = (size_t)nb64 * nb64;
   if (!s->mat64) {
-    bool ok = cudaMalloc(&s->mat64, cap) == cudaSuccess && cudaMalloc(&s->submask, cap) == cudaSuccess &&
-              cudaMalloc(&s->row_ptr64, (nb64 + 1) * 4) == cudaSuccess && cudaMalloc(&s->col_idx64, cap * 4) == cudaSuccess &&
-              cudaMalloc(&s->blk_row64, cap * 4) == cudaSuccess && cudaMalloc(&s->col_ptr64, (nb64 + 1) * 4) == cudaSuccess &&
-              cudaMalloc(&s->row_idx64, cap * 4) == cudaSuccess && cudaMalloc(&s->csc_pos64, cap * 4) == cudaSuccess &&
-              cudaMalloc(&s->work64, cap * 4) == cudaSuccess && cudaMalloc(&s->nnzb64_dev, 4) == cudaSuccess;
+    bool ok = device_alloc((void**)&s->mat64, cap) == SPION_OK && device_alloc((void**)&s->submask, cap) == SPION_OK &&
+              device_alloc((void**)&s->row_ptr64, (nb64 + 1) * 4) == SPION_OK && device_alloc((void**)&s->col_idx64, cap * 4) == SPION_OK &&
+              device_alloc((void**)&s->blk_row64, cap * 4) == SPION_OK && device_alloc((void**)&s->col_ptr64, (nb64 + 1) * 4) == SPION_OK &&
+              device_alloc((void**)&s->row_idx64, cap * 4) == SPION_OK && device_alloc((void**)&s->csc_pos64, cap * 4) == SPION_OK &&
+              device_alloc((void**)&s->work64, cap * 4) == SPION_OK && device_alloc((void**)&s->nnzb64_dev, 4) == SPION_OK;
     if (!ok) return SPION_ERR_ALLOC;
   }
   s->nb64 = nb64;
@@ -792,8 +792,8 @@ int tc_engine_prepare(spion_ctx* c) {
       return SPION_ERR_CUDA;
     }
     int rc = kernel_attrs(c, s);
-    if (!rc && cudaMalloc(&s->delta_ws, (size_t)c->BH * c->L * sizeof(float)) != cudaSuccess) rc = SPION_ERR_ALLOC;
-    if (!rc && cudaMalloc(&s->lse_ws, (size_t)c->BH * c->L * sizeof(float)) != cudaSuccess) rc = SPION_ERR_ALLOC;
+    if (!rc && device_alloc((void**)&s->delta_ws, (size_t)c->BH * c->L * sizeof(float)) != SPION_OK) rc = SPION_ERR_ALLOC;
+    if (!rc && device_alloc((void**)&s->lse_ws, (size_t)c->BH * c->L * sizeof(float)) != SPION_OK) rc = SPION_ERR_ALLOC;
     if (rc) { delete s; return rc; }
     s->super = c->bs == 32;
     c->tc = s;
@@ -805,13 +805,13 @@ int tc_engine_prepare(spion_ctx* c) {
   const TcView vw = tc_view(c, s);
   // value-tile rows are 32-bit TMA coordinates: (bh * nnzb + block) * 64 must stay below 2^31
   if ((unsigned long long)c->BH * (unsigned long long)vw.nnzb * BS >= 0x7fffffffULL) return SPION_ERR_SHAPE;
-  if (!s->row_info && cudaMalloc(&s->row_info, (size_t)SPION_MAX_NB * sizeof(int4)) != cudaSuccess) return SPION_ERR_ALLOC;
-  if (!s->n_long_dev && cudaMalloc(&s->n_long_dev, sizeof(int)) != cudaSuccess) return SPION_ERR_ALLOC;
+  if (!s->row_info && device_alloc((void**)&s->row_info, (size_t)SPION_MAX_NB * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
+  if (!s->n_long_dev && device_alloc((void**)&s->n_long_dev, sizeof(int)) != SPION_OK) return SPION_ERR_ALLOC;
   k_row_info<<<1, 512, 0, c->stream>>>(vw.row_ptr, vw.col_idx, vw.nb, s->row_info, s->n_long_dev);
   SPION_LAUNCH_CHECK();
   SPION_CUDA_TRY(cudaMemcpyAsync(&s->n_long, s->n_long_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   SPION_CUDA_TRY(cudaStreamSynchronize(c->stream));                // set_pattern time: once per mask
-  if (!s->col_order && cudaMalloc(&s->col_order, (size_t)SPION_MAX_NB * sizeof(int)) != cudaSuccess) return SPION_ERR_ALLOC;
+  if (!s->col_order && device_alloc((void**)&s->col_order, (size_t)SPION_MAX_NB * sizeof(int)) != SPION_OK) return SPION_ERR_ALLOC;
   k_line_order<<<1, 512, 0, c->stream>>>(vw.col_ptr, vw.nb, s->col_order);
   SPION_LAUNCH_CHECK();
   if ((rc = stream_prepare(c, s))) return rc;
@@ -824,13 +824,13 @@ void tc_engine_release(spion_ctx* c) {
   TcState* s = (TcState*)c->tc;
   free_super(s);
   b32_release(s);
-  cudaFree(s->lse_ws);
-  cudaFree(s->delta_ws);
-  cudaFree(s->n_long_dev);
-  cudaFree(s->row_info);
-  cudaFree(s->col_order);
-  cudaFree(s->line_rec);
-  cudaFree(s->line_pair);
+  device_free(s->lse_ws);
+  device_free(s->delta_ws);
+  device_free(s->n_long_dev);
+  device_free(s->row_info);
+  device_free(s->col_order);
+  device_free(s->line_rec);
+  device_free(s->line_pair);
   delete s;
   c->tc = nullptr;
 }
