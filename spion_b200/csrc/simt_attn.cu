@@ -589,6 +589,278 @@ __global__ void __launch_bounds__(DENSE_WARPS * 32) softmax_bwd_dense_t_kernel(c
   }
 }
 
+// The same with the slab on chip: sixteen columns per CTA, their values in shared memory (backward: P there, dP in registers), so
+// that they are read once instead of three times (twice) and all loads of a CTA are in flight together; two or three
+// CTAs per SM overlap one's loads with another's arithmetic.  Slices, expressions and order of additions are those above.
+// 16 matrices, L = 1024 (64 MB each way): SOFTMAX_FIGURES.
+constexpr int SLAB = 16;
+__host__ __device__ inline int slab_per(int L) { return (L + DENSE_WARPS - 1) / DENSE_WARPS; }
+__host__ __device__ inline int slab_slice(int L) { return slab_per(L) * SLAB + SLAB; }   // floats; the pad keeps a warp's two slices on different banks
+__device__ __forceinline__ void load_slab(float* slab, const float* src, int L) {        // src: row 0 of the CTA's columns
+  const int per = slab_per(L);
+  for (int e = threadIdx.x; e < L * (SLAB / 4); e += DENSE_WARPS * SLAB) {
+    const int j = e / (SLAB / 4), c4 = e % (SLAB / 4), w = j / per;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slab + w * slab_slice(L) + (j - w * per) * SLAB + c4 * 4)),
+                 "l"(src + (long long)j * L + c4 * 4) : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(DENSE_WARPS * SLAB) softmax_fwd_dense_t_slab(float* __restrict__ S, int L, float scale,
+                                                                               const float* __restrict__ keypad, float floor_v) {
+  extern __shared__ __align__(16) float s_slab[];
+  __shared__ float s_red[DENSE_WARPS][SLAB];
+  const int col = threadIdx.x % SLAB, w = threadIdx.x / SLAB;
+  const int per = slab_per(L), j0 = w * per, n = max(0, min(L, j0 + per) - j0);
+  float* Sb = S + (long long)blockIdx.y * L * L + blockIdx.x * SLAB;
+  const float* kp = keypad ? keypad + (long long)blockIdx.y * L + j0 : nullptr;
+  const float* x = s_slab + w * slab_slice(L) + col;
+  load_slab(s_slab, Sb, L);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  Sb += (long long)j0 * L + col;
+  float m = floor_v;
+#pragma unroll 8
+  for (int u = 0; u < n; ++u) {
+    float v = x[u * SLAB] * scale;
+    if (kp) v -= kp[u];
+    m = fmaxf(m, v);
+  }
+  s_red[w][col] = m;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < DENSE_WARPS; ++k) m = fmaxf(m, s_red[k][col]);
+  __syncthreads();
+  float sum = 0.f;
+#pragma unroll 8
+  for (int u = 0; u < n; ++u) {
+    float v = x[u * SLAB] * scale;
+    if (kp) v -= kp[u];
+    sum += expf(v - m);
+  }
+  s_red[w][col] = sum;
+  __syncthreads();
+  sum = 0.f;
+#pragma unroll
+  for (int k = 0; k < DENSE_WARPS; ++k) sum += s_red[k][col];       // slices added in slice order
+  const float inv = 1.0f / sum;
+#pragma unroll 8
+  for (int u = 0; u < n; ++u) {
+    float v = x[u * SLAB] * scale;
+    if (kp) v -= kp[u];
+    Sb[(long long)u * L] = expf(v - m) * inv;
+  }
+}
+
+template <int PER>
+__global__ void __launch_bounds__(DENSE_WARPS * SLAB) softmax_bwd_dense_t_slab(const float* __restrict__ dP, const float* __restrict__ P,
+                                                                               float* __restrict__ dS, int L, float scale) {
+  extern __shared__ __align__(16) float s_slab[];
+  __shared__ float s_red[DENSE_WARPS][SLAB];
+  const int col = threadIdx.x % SLAB, w = threadIdx.x / SLAB;
+  const int per = slab_per(L), j0 = w * per, n = max(0, min(L, j0 + per) - j0);
+  const long long base = (long long)blockIdx.y * L * L + blockIdx.x * SLAB, o = base + (long long)j0 * L + col;
+  const float* p = s_slab + w * slab_slice(L) + col;
+  load_slab(s_slab, P + base, L);
+  float x[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u)
+    if (u < n) x[u] = dP[o + (long long)u * L];
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float s = 0.f;
+#pragma unroll
+  for (int u = 0; u < PER; ++u)
+    if (u < n) s += x[u] * p[u * SLAB];
+  s_red[w][col] = s;
+  __syncthreads();
+  s = 0.f;
+#pragma unroll
+  for (int k = 0; k < DENSE_WARPS; ++k) s += s_red[k][col];
+#pragma unroll
+  for (int u = 0; u < PER; ++u)
+    if (u < n) {
+      const float pv = p[u * SLAB];
+      dS[o + (long long)u * L] = (x[u] * pv - pv * s) * scale;
+    }
+}
+
+// ------------------------------------------------------------------------------ full masks, fp32, S^T-stored values
+// The reference-layout dense path: every value tile is selected, value(i, j) at j*L + i.  The block kernels above spend a scalar
+// shared-memory read on every other multiply-add and hold one tile in flight; these keep the order of additions of
+// every output (n, or k, ascending into one fp32 sum), so the results are the same bit for bit, with packed pairs of
+// multiply-adds, 16-byte reads and cp.async.  16 matrices, L = 1024, d 32: SDDMM_FIGURES.
+__device__ __forceinline__ uint32_t dense_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void dense_cp16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dense_smem(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void dense_cp4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dense_smem(dst)), "l"(src) : "memory");
+}
+using pair_t = unsigned long long;
+__device__ __forceinline__ pair_t twice(float x) {
+  pair_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void fma2(pair_t& acc, pair_t a, pair_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ float4 as_float4(pair_t lo, pair_t hi) {
+  float4 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(lo));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.z), "=f"(v.w) : "l"(hi));
+  return v;
+}
+
+// S^T[j][i] = sum_n A[i][n] B[j][n]: a 64 x 64 tile by 64 threads, rows j = ty + 8 y, columns i = 4 tx .. and 32 + 4 tx ..
+constexpr int DT = 64;
+__global__ void __launch_bounds__(64) sddmm_dense_kernel(const float* __restrict__ A, OperandLayout la, const float* __restrict__ B,
+                                                         OperandLayout lb, float* __restrict__ vals, int L, int d) {
+  __shared__ __align__(16) float As[KC][DT];           // [n][i], pieces of four i exchanged by n / 4: written along n, read along i
+  __shared__ __align__(16) float Bs[DT][KC + 4];       // [j][n]
+  const int t = threadIdx.x, ty = t >> 3, tx = t & 7;
+  const int i0 = blockIdx.x * DT, j0 = blockIdx.y * DT, bh = blockIdx.z;
+  const float* Ab = A + (long long)bh * la.bh_stride + (long long)i0 * la.sl;
+  const float* Bb = B + (long long)bh * lb.bh_stride + (long long)j0 * lb.sl;
+  pair_t acc[8][4];
+#pragma unroll
+  for (int y = 0; y < 8; ++y)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) acc[y][x] = 0ull;
+  for (int n0 = 0; n0 < d; n0 += KC) {
+    if (la.sl == 1 && (la.sd & 3) == 0 && (reinterpret_cast<uintptr_t>(Ab) & 15) == 0) {
+#pragma unroll
+      for (int e = t; e < KC * DT / 4; e += 64) dense_cp16(&As[e >> 4][((e & 15) ^ (e >> 6)) * 4], Ab + (long long)(n0 + (e >> 4)) * la.sd + (e & 15) * 4);
+    } else if (la.sd == 1 && (la.sl & 3) == 0 && (reinterpret_cast<uintptr_t>(Ab) & 15) == 0) {
+#pragma unroll
+      for (int e = t; e < KC * DT / 4; e += 64) {
+        const int i = e >> 3, n4 = e & 7;
+        const float4 v = *reinterpret_cast<const float4*>(Ab + (long long)i * la.sl + n0 + 4 * n4);
+        float* to = &As[4 * n4][i ^ (4 * n4)];
+        to[0] = v.x, to[DT] = v.y, to[2 * DT] = v.z, to[3 * DT] = v.w;
+      }
+    } else {
+      for (int n = 0; n < KC; ++n) As[n][t ^ (n & ~3)] = Ab[(long long)t * la.sl + (long long)(n0 + n) * la.sd];
+    }
+    if (lb.sd == 1 && (lb.sl & 3) == 0 && (reinterpret_cast<uintptr_t>(Bb) & 15) == 0) {
+#pragma unroll
+      for (int e = t; e < DT * KC / 4; e += 64) dense_cp16(&Bs[e >> 3][(e & 7) * 4], Bb + (long long)(e >> 3) * lb.sl + n0 + (e & 7) * 4);
+    } else {
+      for (int e = t; e < DT * KC; e += 64) dense_cp4(&Bs[e & 63][e >> 6], Bb + (long long)(e & 63) * lb.sl + (long long)(n0 + (e >> 6)) * lb.sd);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll 2
+    for (int n = 0; n < KC; n += 4) {
+      float b[8][4];
+#pragma unroll
+      for (int y = 0; y < 8; ++y) {
+        const float4 v = *reinterpret_cast<const float4*>(&Bs[ty + 8 * y][n]);
+        b[y][0] = v.x, b[y][1] = v.y, b[y][2] = v.z, b[y][3] = v.w;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(&As[n + k][(4 * tx) ^ n]), hi = *reinterpret_cast<const ulonglong2*>(&As[n + k][32 + ((4 * tx) ^ n)]);
+#pragma unroll
+        for (int y = 0; y < 8; ++y) {
+          const pair_t bb = twice(b[y][k]);
+          fma2(acc[y][0], lo.x, bb), fma2(acc[y][1], lo.y, bb), fma2(acc[y][2], hi.x, bb), fma2(acc[y][3], hi.y, bb);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  float* out = vals + (long long)bh * L * L + (long long)j0 * L + i0 + 4 * tx;
+#pragma unroll
+  for (int y = 0; y < 8; ++y) {
+    float* row = out + (long long)(ty + 8 * y) * L;
+    *reinterpret_cast<float4*>(row) = as_float4(acc[y][0], acc[y][1]);
+    *reinterpret_cast<float4*>(row + 32) = as_float4(acc[y][2], acc[y][3]);
+  }
+}
+
+// TRANS == false: out[i] = sum_j value(i, j) Bop[j];  true: out[j] = sum_i value(i, j) Bop[i].  64 rows x 32 columns by 64 threads
+// (4 x 8 each), the sum over L in steps of 32 through three stages.  The sum of an output stays one chain, so the rows
+// cannot be split further: 64 threads a tile put 256 tiles of a small call on every scheduler.
+constexpr int DK = 32, DSTAGES = 3;
+template <bool TRANS>
+__global__ void __launch_bounds__(64) spmm_dense_kernel(const float* __restrict__ vals, const float* __restrict__ Bop, OperandLayout lb,
+                                                        float* __restrict__ out, OperandLayout lo, int L) {
+  constexpr int VR = TRANS ? DT : DK, VC = TRANS ? DK : DT, VP = TRANS ? DK + 4 : DT;   // value tile as in memory: rows j, columns i
+  __shared__ __align__(16) float Vs[DSTAGES][VR][VP];
+  __shared__ __align__(16) float Bs[DSTAGES][DK][DK + 4];                               // [k][n]
+  const int t = threadIdx.x, ty = t >> 2, tx = t & 3;
+  const int r0 = blockIdx.x * DT, bh = blockIdx.y, n0 = blockIdx.z * 32;
+  const float* vb = vals + (long long)bh * L * L + (TRANS ? (long long)r0 * L : (long long)r0);
+  const float* Bb = Bop + (long long)bh * lb.bh_stride + (long long)n0 * lb.sd;
+  const bool rows = lb.sd == 1 && (lb.sl & 3) == 0 && (reinterpret_cast<uintptr_t>(Bb) & 15) == 0;
+  auto load = [&](int c) {
+    const int st = c % DSTAGES, k0 = c * DK;
+    const float* v = vb + (TRANS ? (long long)k0 : (long long)k0 * L);
+#pragma unroll
+    for (int e = t; e < VR * VC / 4; e += 64) dense_cp16(&Vs[st][e / (VC / 4)][e % (VC / 4) * 4], v + (long long)(e / (VC / 4)) * L + e % (VC / 4) * 4);
+    if (rows) {
+#pragma unroll
+      for (int e = t; e < DK * 32 / 4; e += 64) dense_cp16(&Bs[st][e >> 3][(e & 7) * 4], Bb + (long long)(k0 + (e >> 3)) * lb.sl + (e & 7) * 4);
+    } else {
+#pragma unroll 4
+      for (int e = t; e < DK * 32; e += 64) dense_cp4(&Bs[st][e & 31][e >> 5], Bb + (long long)(k0 + (e & 31)) * lb.sl + (long long)(e >> 5) * lb.sd);
+    }
+  };
+  pair_t acc[4][4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
+  const int chunks = L / DK;
+  for (int c = 0; c < DSTAGES - 1; ++c) {
+    if (c < chunks) load(c);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(DSTAGES - 2) : "memory");
+    __syncthreads();                                   // chunk c has landed; the stage of chunk c - 1 is free
+    if (c + DSTAGES - 1 < chunks) load(c + DSTAGES - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int st = c % DSTAGES;
+#pragma unroll 2
+    for (int k = 0; k < DK; k += 4) {
+      float a[4][4];                                   // [k][row]
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 v = TRANS ? *reinterpret_cast<const float4*>(&Vs[st][ty + 16 * u][k]) : *reinterpret_cast<const float4*>(&Vs[st][k + u][4 * ty]);
+        if (TRANS) a[0][u] = v.x, a[1][u] = v.y, a[2][u] = v.z, a[3][u] = v.w;
+        else a[u][0] = v.x, a[u][1] = v.y, a[u][2] = v.z, a[u][3] = v.w;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const ulonglong2 lo2 = *reinterpret_cast<const ulonglong2*>(&Bs[st][k + u][4 * tx]), hi2 = *reinterpret_cast<const ulonglong2*>(&Bs[st][k + u][16 + 4 * tx]);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const pair_t aa = twice(a[u][x]);
+          fma2(acc[x][0], aa, lo2.x), fma2(acc[x][1], aa, lo2.y), fma2(acc[x][2], aa, hi2.x), fma2(acc[x][3], aa, hi2.y);
+        }
+      }
+    }
+  }
+  float* ob = out + (long long)bh * lo.bh_stride;
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const int row = r0 + (TRANS ? ty + 16 * x : 4 * ty + x);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float4 v = as_float4(acc[x][2 * h], acc[x][2 * h + 1]);
+      float* o = ob + (long long)row * lo.sl + (long long)(n0 + 16 * h + 4 * tx) * lo.sd;
+      if (lo.sd == 1 && (reinterpret_cast<uintptr_t>(o) & 15) == 0) *reinterpret_cast<float4*>(o) = v;
+      else o[0] = v.x, o[lo.sd] = v.y, o[2 * lo.sd] = v.z, o[3 * lo.sd] = v.w;
+    }
+  }
+}
+
+// Only the dense context stores values this way, and its mask is always full; blocks of 64 stand for L being a multiple of 64.
+bool full_dense(const ValueLayout& vl, const Pattern& p, const void* vals) {
+  return vl.mode == VAL_DENSE_T && p.bs == DT && (reinterpret_cast<uintptr_t>(vals) & 15) == 0;
+}
+
 }  // namespace
 
 // ================================================================================ launchers
@@ -610,6 +882,11 @@ int simt_sddmm(int dtype_in, int dtype_val, const void* A, OperandLayout la, con
                ValueLayout vl, Pattern p, int nnzb, int BH, int d, cudaStream_t st) {
   if (d % KC != 0 || BH > 65535) return SPION_ERR_UNSUPPORTED;
   if (nnzb == 0) return SPION_OK;
+  if (dtype_in == SPION_F32 && dtype_val == SPION_F32 && full_dense(vl, p, vals)) {
+    sddmm_dense_kernel<<<dim3(p.nb, p.nb, BH), 64, 0, st>>>((const float*)A, la, (const float*)B, lb, (float*)vals, vl.L, d);
+    SPION_LAUNCH_CHECK();
+    return SPION_OK;
+  }
   if (dtype_in == SPION_F32 && dtype_val == SPION_F32)
     return sddmm_dispatch<float, float>(A, la, B, lb, vals, vl, p, nnzb, BH, d, st);
   if (dtype_in == SPION_BF16 && dtype_val == SPION_F32)
@@ -634,6 +911,13 @@ static int spmm_dispatch(bool trans, const void* vals, ValueLayout vl, const voi
 int simt_spmm(int dtype_val, int dtype_op, bool trans, const void* vals, ValueLayout vl, const void* Bop,
               OperandLayout lb, void* out, OperandLayout lo, Pattern p, int BH, int d, cudaStream_t st) {
   if (d % 32 != 0 || BH > 65535) return SPION_ERR_UNSUPPORTED;
+  if (dtype_val == SPION_F32 && dtype_op == SPION_F32 && full_dense(vl, p, vals)) {
+    const dim3 grid(p.nb, BH, d / 32);
+    if (trans) spmm_dense_kernel<true><<<grid, 64, 0, st>>>((const float*)vals, (const float*)Bop, lb, (float*)out, lo, vl.L);
+    else spmm_dense_kernel<false><<<grid, 64, 0, st>>>((const float*)vals, (const float*)Bop, lb, (float*)out, lo, vl.L);
+    SPION_LAUNCH_CHECK();
+    return SPION_OK;
+  }
   if (dtype_val == SPION_F32 && dtype_op == SPION_F32)
     return spmm_dispatch<float, float>(trans, vals, vl, Bop, lb, out, lo, p, BH, d, st);
   if (dtype_val == SPION_BF16 && dtype_op == SPION_BF16)
@@ -712,16 +996,34 @@ int softmax_bwd_rows(int dtype_p, const float* dP, ValueLayout vdp, const void* 
   return SPION_OK;
 }
 
+constexpr int SLAB_SMEM = 112 * 1024;
 int softmax_fwd_dense_t(float* S, int BH, int L, float scale, const float* keypad, float floor_v, cudaStream_t st) {
   if (BH > 65535) return SPION_ERR_UNSUPPORTED;
-  softmax_fwd_dense_t_kernel<<<dim3((L + 31) / 32, BH), DENSE_WARPS * 32, 0, st>>>(S, L, scale, keypad, floor_v);
+  // the slab kernel while at least two CTAs of it fit an SM
+  const int smem = DENSE_WARPS * slab_slice(L) * (int)sizeof(float);
+  if (L % SLAB == 0 && ((uintptr_t)S & 15) == 0 && smem <= SLAB_SMEM) {
+    SPION_CUDA_TRY(cudaFuncSetAttribute(softmax_fwd_dense_t_slab, cudaFuncAttributeMaxDynamicSharedMemorySize, SLAB_SMEM));
+    softmax_fwd_dense_t_slab<<<dim3(L / SLAB, BH), DENSE_WARPS * SLAB, smem, st>>>(S, L, scale, keypad, floor_v);
+  } else {
+    softmax_fwd_dense_t_kernel<<<dim3((L + 31) / 32, BH), DENSE_WARPS * 32, 0, st>>>(S, L, scale, keypad, floor_v);
+  }
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
 
 int softmax_bwd_dense_t(const float* dP, const float* P, float* dS, int BH, int L, float scale, cudaStream_t st) {
   if (BH > 65535) return SPION_ERR_UNSUPPORTED;
-  softmax_bwd_dense_t_kernel<<<dim3((L + 31) / 32, BH), DENSE_WARPS * 32, 0, st>>>(dP, P, dS, L, scale);
+  // the slab kernel while a slice of dP fits a thread's registers
+  const int smem = DENSE_WARPS * slab_slice(L) * (int)sizeof(float), per = slab_per(L);
+  auto slab = [&](auto kernel) -> int {
+    SPION_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SLAB_SMEM));
+    kernel<<<dim3(L / SLAB, BH), DENSE_WARPS * SLAB, smem, st>>>(dP, P, dS, L, scale);
+    return SPION_OK;
+  };
+  int rc = SPION_OK;
+  if (L % SLAB == 0 && ((uintptr_t)P & 15) == 0 && per <= 128) rc = per <= 64 ? slab(softmax_bwd_dense_t_slab<64>) : slab(softmax_bwd_dense_t_slab<128>);
+  else softmax_bwd_dense_t_kernel<<<dim3((L + 31) / 32, BH), DENSE_WARPS * 32, 0, st>>>(dP, P, dS, L, scale);
+  if (rc) return rc;
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
