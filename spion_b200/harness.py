@@ -206,9 +206,8 @@ class Trainer:
         self.allreduce_events = None     # set to a list to collect (start, end) CUDA events around the gradient all-reduce
 
     def step(self, ids, label, is_attn=False):
-        self.bucket.zero()
         loss, maps = self.model(ids, label, self.mat_lst, is_attn)
-        loss.backward()
+        self.bucket.backward(loss)
         if self.allreduce_events is not None:
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
@@ -217,7 +216,7 @@ class Trainer:
             self.allreduce_events.append((e0, e1))
         else:
             self.bucket.allreduce_mean()
-        torch.nn.utils.clip_grad_value_(self.model.parameters(), 1.0)   # main_conv_ff.py:186
+        self.bucket.flat.clamp_(-1.0, 1.0)                              # clip_grad_value_ (main_conv_ff.py:186), all gradients at once
         self.opt.step()
         self._refresh_shadows()
         return loss.detach(), maps
@@ -257,13 +256,12 @@ class Trainer:
         # other threads of the process (the collective library's watchdog) may query events while this thread
         # captures: only this thread's calls belong to the capture
         with torch.cuda.graph(self._graph, capture_error_mode="thread_local"):
-            self.bucket.zero()
             loss, _ = self.model(self._g_ids, self._g_lab, self.mat_lst, False)
-            loss.backward()
+            self.bucket.backward(loss)
             self._g_loss = loss.detach()
         self._graph_opt = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self._graph_opt, capture_error_mode="thread_local"):
-            torch.nn.utils.clip_grad_value_(self.model.parameters(), 1.0)
+            self.bucket.flat.clamp_(-1.0, 1.0)
             self.opt.step()
             self._refresh_shadows()
         return self._graph
