@@ -192,7 +192,7 @@ class Trainer:
         torch.manual_seed(seed)                      # identical initial weights on every rank
         self.model = Classifier(config).to(self.device)
         self.bucket = dp.FlatGradBucket(self.model.parameters())
-        self.opt = torch.optim.AdamW(self.model.parameters(), lr=lr, weight_decay=0.0, capturable=True, fused=True)
+        self.opt = torch.optim.AdamW(self.bucket.pieces(), lr=lr, weight_decay=0.0, capturable=True, fused=True)
         self.mat_lst = None
         self.patterns = None
         self._graph = None
