@@ -377,6 +377,10 @@ int spion_add_layernorm_backward(const float* x, const void* dy, int dy_is_bf16,
  * fixed-order reduction.  workspace: spion_layernorm_workspace_floats(N) floats. */
 int spion_column_sums(const void* dy, int dy_is_bf16, float* out, float* workspace, long long M, int N,
                       void* cuda_stream);
+/* The same for count <= 4 matrices (dys: host array of device pointers) in the same two launches: out [count, N],
+ * workspace count times as large. */
+int spion_column_sums_many(const void* const* dys, int count, int dy_is_bf16, float* out, float* workspace, long long M, int N,
+                           void* cuda_stream);
 
 /* Weight gradient of a token embedding with a small table (torch.nn.Embedding(vocab_size, embedding_dim) in the
  * reference's encoder, models/model_transformer.py; vocab_size 256 - 512 in its tasks):

@@ -212,8 +212,11 @@ __global__ void __launch_bounds__(LN_WARPS * 32) colsum_kernel(const void* __res
 }
 
 // out[c] = sum over the partial rows of an [rows, N] matrix, fixed order (see ln_bwd_reduce_kernel)
+// (blockIdx.y: one of several matrices, partial rows and results one after another)
 __global__ void __launch_bounds__(1024) colsum_reduce_kernel(const float* __restrict__ partial, int rows, int N,
                                                               float* __restrict__ out) {
+  partial += (size_t)blockIdx.y * rows * N;
+  out += (size_t)blockIdx.y * N;
   __shared__ float s_p[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -309,10 +312,14 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_bwd4_kernel(const float* __r
 }
 
 // Column sums with 16-byte loads: a row of N values takes LPR = N * sizeof(T) / 16 lanes (8 or 16 for N = 64, 16 or 32
-// for N = 128), a warp reads 32 / LPR rows per step, four steps in flight.
+// for N = 128), a warp reads 32 / LPR rows per step, four steps in flight.  blockIdx.y: one of several matrices of one size (the
+// query, key and value layers' bias gradients in two launches instead of six of 3 us).
+struct ColumnSumList { const void* p[4]; };
 template <int N, typename T>
-__global__ void __launch_bounds__(LN_WARPS * 32) colsum4_kernel(const T* __restrict__ dy, float* __restrict__ partial,
+__global__ void __launch_bounds__(LN_WARPS * 32) colsum4_kernel(const __grid_constant__ ColumnSumList list, float* __restrict__ partial,
                                                                 long long M) {
+  const T* __restrict__ dy = static_cast<const T*>(list.p[blockIdx.y]);
+  partial += (size_t)blockIdx.y * gridDim.x * N;
   constexpr int PER = 16 / (int)sizeof(T), LPR = N / PER, RPW = 32 / LPR;
   __shared__ float s_b[LN_WARPS * RPW][N];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane % LPR, sub = lane / LPR;
@@ -474,37 +481,51 @@ extern "C" int spion_add_layernorm_backward(const float* x, const void* dy, int 
                      N, (cudaStream_t)cuda_stream);
 }
 
-// Sum of the rows of an [M, N] matrix (fp32 or bf16), N in {64, 128, 256, 512}: out[N] fp32.  The bias gradient of a
-// linear layer.  workspace: spion_layernorm_workspace_floats(N) floats.  Fixed summation order.
-extern "C" int spion_column_sums(const void* dy, int dy_is_bf16, float* out, float* workspace, long long M, int N,
-                                 void* cuda_stream) {
+// Sums of the rows of `count` [M, N] matrices (fp32 or bf16), N in {64, 128, 256, 512}: out [count, N] fp32.  The bias gradients of
+// linear layers.  workspace: count * spion_layernorm_workspace_floats(N) floats.  Fixed summation order.
+extern "C" int spion_column_sums_many(const void* const* dys, int count, int dy_is_bf16, float* out, float* workspace, long long M, int N,
+                                      void* cuda_stream) {
   cudaStream_t stream = (cudaStream_t)cuda_stream;
-  if (!dy || !out || !workspace || M < 1) return SPION_ERR_ARG;
+  if (!dys || count < 1 || count > 4 || !out || !workspace || M < 1) return SPION_ERR_ARG;
   const int grid = ln_grid(M);
   if (grid < 1) return SPION_ERR_CUDA;
-  if ((N == 64 || N == 128) && ((uintptr_t)dy & 15) == 0) {
-    if (N == 64 && dy_is_bf16) colsum4_kernel<64, __nv_bfloat16><<<grid, LN_WARPS * 32, 0, stream>>>((const __nv_bfloat16*)dy, workspace, M);
-    else if (N == 64) colsum4_kernel<64, float><<<grid, LN_WARPS * 32, 0, stream>>>((const float*)dy, workspace, M);
-    else if (dy_is_bf16) colsum4_kernel<128, __nv_bfloat16><<<grid, LN_WARPS * 32, 0, stream>>>((const __nv_bfloat16*)dy, workspace, M);
-    else colsum4_kernel<128, float><<<grid, LN_WARPS * 32, 0, stream>>>((const float*)dy, workspace, M);
+  ColumnSumList list = {};
+  bool aligned = true;
+  for (int i = 0; i < count; ++i) {
+    if (!dys[i]) return SPION_ERR_ARG;
+    list.p[i] = dys[i];
+    aligned = aligned && ((uintptr_t)dys[i] & 15) == 0;
+  }
+  if ((N == 64 || N == 128) && aligned) {
+    const dim3 g(grid, count);
+    if (N == 64 && dy_is_bf16) colsum4_kernel<64, __nv_bfloat16><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
+    else if (N == 64) colsum4_kernel<64, float><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
+    else if (dy_is_bf16) colsum4_kernel<128, __nv_bfloat16><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
+    else colsum4_kernel<128, float><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
     SPION_LAUNCH_CHECK();
-    colsum_reduce_kernel<<<N / 32, 1024, 0, stream>>>(workspace, grid, N, out);
+    colsum_reduce_kernel<<<dim3(N / 32, count), 1024, 0, stream>>>(workspace, grid, N, out);
     SPION_LAUNCH_CHECK();
     return SPION_OK;
   }
-#define SPION_COLSUM(K)                                                                                   \
-  if (dy_is_bf16) colsum_kernel<K, true><<<grid, LN_WARPS * 32, 0, stream>>>(dy, workspace, M);            \
-  else colsum_kernel<K, false><<<grid, LN_WARPS * 32, 0, stream>>>(dy, workspace, M);
-  switch (N) {
-    case 64: SPION_COLSUM(1) break;
-    case 128: SPION_COLSUM(2) break;
-    case 256: SPION_COLSUM(4) break;
-    case 512: SPION_COLSUM(8) break;
-    default: return SPION_ERR_SHAPE;
+#define SPION_COLSUM(K)                                                                                                        \
+  if (dy_is_bf16) colsum_kernel<K, true><<<grid, LN_WARPS * 32, 0, stream>>>(dys[i], workspace + (size_t)i * grid * N, M);     \
+  else colsum_kernel<K, false><<<grid, LN_WARPS * 32, 0, stream>>>(dys[i], workspace + (size_t)i * grid * N, M);
+  for (int i = 0; i < count; ++i) {
+    switch (N) {
+      case 64: SPION_COLSUM(1) break;
+      case 128: SPION_COLSUM(2) break;
+      case 256: SPION_COLSUM(4) break;
+      case 512: SPION_COLSUM(8) break;
+      default: return SPION_ERR_SHAPE;
+    }
+    SPION_LAUNCH_CHECK();
   }
 #undef SPION_COLSUM
-  SPION_LAUNCH_CHECK();
-  colsum_reduce_kernel<<<N / 32, 1024, 0, stream>>>(workspace, grid, N, out);
+  colsum_reduce_kernel<<<dim3(N / 32, count), 1024, 0, stream>>>(workspace, grid, N, out);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
+}
+
+extern "C" int spion_column_sums(const void* dy, int dy_is_bf16, float* out, float* workspace, long long M, int N, void* cuda_stream) {
+  return spion_column_sums_many(&dy, 1, dy_is_bf16, out, workspace, M, N, cuda_stream);
 }

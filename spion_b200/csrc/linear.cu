@@ -208,6 +208,30 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     for (int i = 0; i < R; ++i) cur[i] = load_row(col, blockIdx.x, i);
   }
 
+  // bf16: the first LG_DEPTH chunks are on their way before the weights are converted (their stages are free)
+  int ld_n = 0, ld_tile = blockIdx.x, ld_ch = 0;
+  auto copy_chunk = [&]() {
+    const uint32_t dst = sA + (ld_n % a.nstages) * CHUNK;
+    const AE* col = a_col(ld_ch);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = lrow + 32 * i;
+      const bool in = col && ld_tile * 128 + r < a.T;
+      cp_async16(dst + r * 128 + ((lc8 ^ (r & 7)) << 4), in ? col + row[i].off(a.A) : reinterpret_cast<const AE*>(a.A.p[0]), in);
+    }
+    cp_async_commit();
+    ++ld_n;
+    if (++ld_ch == nchunks) {
+      ld_ch = 0; ld_tile += G_x;
+#pragma unroll
+      for (int i = 0; i < R; ++i) row[i].add(a.A, step_b, step_l);
+    }
+  };
+  if constexpr (A_BF16) {
+    if (warp < LG_LOADERS)
+      while (ld_n < LG_DEPTH && ld_tile < ntiles) copy_chunk();
+  }
+
   {                                                      // weights -> shared memory
     const int per_row = TRANSB ? nc >> 3 : a.K >> 3;
     const int rows = TRANSB ? a.K : nc;
@@ -251,30 +275,17 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive(full + 8 * (m % a.nstages));
       };
-      while (ok && tile < ntiles) {
-        const int st = n % a.nstages, use = n / a.nstages;
+      while (ld_tile < ntiles) {
+        const int st = ld_n % a.nstages, use = ld_n / a.nstages;
         if (use > 0) ok = warp_wait(empty + 8 * st, (uint32_t)(use - 1) & 1u);
         if (!ok) break;
-        const uint32_t dst = sA + st * CHUNK;
-        const AE* col = a_col(ch);
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-          const int r = lrow + 32 * i;
-          const bool in = col && tile * 128 + r < a.T;
-          cp_async16(dst + r * 128 + ((lc8 ^ (r & 7)) << 4), in ? col + row[i].off(a.A) : reinterpret_cast<const AE*>(a.A.p[0]), in);
-        }
-        cp_async_commit();
-        if (n >= LG_DEPTH) { cp_async_wait<LG_DEPTH>(); hand_over(n - LG_DEPTH); }
-        ++n;
-        if (++ch == nchunks) {
-          ch = 0; tile += G_x;
-#pragma unroll
-          for (int i = 0; i < R; ++i) row[i].add(a.A, step_b, step_l);
-        }
+        copy_chunk();
+        cp_async_wait<LG_DEPTH>();
+        hand_over(ld_n - 1 - LG_DEPTH);
       }
       cp_async_wait<0>();
       if (ok)
-        for (int m = max(0, n - LG_DEPTH); m < n; ++m) hand_over(m);
+        for (int m = max(0, ld_n - LG_DEPTH); m < ld_n; ++m) hand_over(m);
     } else
     while (ok && tile < ntiles) {
       int tile_n = tile, ch_n = ch + 1;

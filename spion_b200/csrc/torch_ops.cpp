@@ -78,16 +78,24 @@ void linear_backward_weight(const std::vector<Tensor>& dY, const spion_tokens& t
   const auto opt = w.W[0].options();
   if (tX.is_bf16 && tY.heads == 0 && tX.heads == 0) {
     Tensor x2 = X.view({T, in});
-    for (int i = 0; i < w.n(); ++i) {
-      Tensor dy2 = dY[i].view({T, per});
-      dW.push_back(at::mm(dy2.t(), x2).to(at::kFloat));
-      if (per == 64 || per == 128 || per == 256 || per == 512) {
-        Tensor g = at::empty({per}, opt), ws = at::empty({(int64_t)spion_layernorm_workspace_floats((int)per)}, opt);
-        check(spion_column_sums(dy2.data_ptr(), 1, (float*)g.data_ptr(), (float*)ws.data_ptr(), T, (int)per, st), "spion_column_sums");
-        db.push_back(g);
-      } else {
-        db.push_back(dy2.sum(0).to(at::kFloat));
-      }
+    const int n = w.n();
+    Tensor prod = at::empty({out, in}, x2.options());        // the products side by side: one conversion for all of them
+    std::vector<const void*> dys;
+    for (int i = 0; i < n; ++i) {
+      Tensor dy2 = dY[i].view({T, per}), part = prod.narrow(0, i * per, per);
+      at::mm_out(part, dy2.t(), x2);
+      dys.push_back(dy2.data_ptr());
+    }
+    Tensor g32 = prod.to(at::kFloat), sums;
+    const bool kernel = per == 64 || per == 128 || per == 256 || per == 512;
+    if (kernel) {
+      sums = at::empty({out}, opt);
+      Tensor ws = at::empty({(int64_t)n * spion_layernorm_workspace_floats((int)per)}, opt);
+      check(spion_column_sums_many(dys.data(), n, 1, (float*)sums.data_ptr(), (float*)ws.data_ptr(), T, (int)per, st), "spion_column_sums_many");
+    }
+    for (int i = 0; i < n; ++i) {
+      dW.push_back(g32.narrow(0, i * per, per));
+      db.push_back(kernel ? sums.narrow(0, i * per, per) : dY[i].view({T, per}).sum(0).to(at::kFloat));
     }
     return;
   }
