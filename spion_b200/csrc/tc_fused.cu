@@ -1,9 +1,9 @@
 // Fused block-sparse attention forward (sm_100a, bf16, 64x64 blocks): S and the sparse row softmax
-// stay on chip; Q, K, V are read once per use, O and one fp32 log-sum-exp per row are written
-// (the P tiles only when the caller asks for them, e.g. for the backward pass).
+// stay on chip; Q, K, V are read once per use, O, one fp32 log-sum-exp per row and the P tiles are
+// written.  Calls without P run on tc_fwd_stream.cu, masks of short rows on tc_fwd_pipe.cu (fwd_launch).
 //
 //   k_fwd_fused   per block row:   S = Q K^T (tcgen05, TMEM) -> row softmax (fp32, registers)
-//                                  -> P (bf16, swizzled shared memory) -> O = P V (tcgen05)
+//                                  -> P (bf16, swizzled shared memory, stored) -> O = P V (tcgen05)
 //                 replaces the three forward stages of models/block_attn.cu:453-487.
 //
 // Softmax semantics are the reference's (models/block_attn.cu:48-87): every non-selected key of a
@@ -72,14 +72,13 @@ __device__ __forceinline__ void store_row_swizzled(uint32_t tile, int i, const u
 // A row of the block is owned by two threads of one warp (lane l: even tiles, lane l+16: odd tiles), so
 // the row statistics need only one warp shuffle.  Rows with at most 4 blocks are done in one chunk (S in
 // all 128 columns, O then overwrites the first 64); longer rows stream chunks of 2 tiles through columns
-// [64,128) in two passes (row maximum, then exp / P / O).  P is kept unnormalised (exp2(x - m) <= 1) and
-// the output row is divided by the denominator at the end.
-// STORE_P: also write the normalised probabilities as [64 x 64] bf16 tiles (TMA store from the shared
-// memory tiles the second product reads): rows of one chunk are rescaled in place once the
-// denominator is known; longer rows accumulate the denominator on line in pass A instead.
+// [64,128) in two passes (row maximum and denominator, then exp / P / O).
+// The normalised probabilities are written as [64 x 64] bf16 tiles (TMA store from the shared memory tiles the second
+// product reads): rows of one chunk are rescaled in place once the denominator is known; longer rows accumulate it on
+// line in pass A.
 // heads: 0 = operands [BH, L, D]; H = operands [B, L, H, D] (see op_pos).
 // KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of every loop).
-template <int D, bool STORE_P, bool SUB, bool KP>
+template <int D, bool SUB, bool KP>
 __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_constant__ CUtensorMap tmQ,
                                                               const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV,
@@ -209,10 +208,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
     // All buffers of this unit are free (its last MMA has retired): ask for the next unit's first tiles.
     auto prefetch_next = [&]() {
       if (ctl && has_next) {
-        if (STORE_P) {                                           // the tile stores must have read their tiles
-          if (lane == 0) bulk_wait_read_all();
-          __syncwarp();
-        }
+        if (lane == 0) bulk_wait_read_all();                     // the tile stores must have read their tiles
+        __syncwarp();
         if (Rn.njobs() > 0) issue_job(Rn, bhn, 0);
         if (Rn.njobs() > 1) issue_job(Rn, bhn, 1);
       }
@@ -245,7 +242,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
     float m2 = floor_v * LOG2E;
     float mraw = -INFINITY;
     float l_part = 0.f;
-    const bool online = STORE_P && !single;                        // denominator needed before P is written
+    const bool online = !single;                                   // denominator needed before P is written
 
     // Row statistics of one chunk whose pair p sits in columns colbase + 64 p: the maximum, and for
     // `online` also the running sum of exponentials.
@@ -316,8 +313,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       }
     };
 
-    // Exponentials of one chunk against the fixed m2 (the row maximum, or the log-sum-exp when the
-    // denominator is already known), packed to bf16 and stored as the K-major P tiles b0 + t.
+    // Probabilities of one chunk (m2 is the row's log-sum-exp by now), packed to bf16 and stored as the K-major P tiles b0 + t.
     auto prob_math = [&](uint32_t colbase, int b0, int t0, int nt, int npairs) {
       for (int p = 0; p < npairs; ++p) {
         const int t = 2 * p + hf;
@@ -330,19 +326,13 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
           tmem_ld32(t_lane + colbase + p * 64 + half * 32, v);
           tmem_ld_wait();
           if (mine && quarter_ok(rp + t0 + t, half)) {
-            float la = 0.f, lb = 0.f, lc = 0.f, ld = 0.f;               // four independent running sums
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
               float h0 = m2, h1 = m2;
               if (kpc) { h0 = fmaf(kpc[half * 32 + j], LOG2E, m2); h1 = fmaf(kpc[half * 32 + j + 1], LOG2E, m2); }
               const float e0 = ex2(fmaf(__uint_as_float(v[j]), sc2, -h0)), e1 = ex2(fmaf(__uint_as_float(v[j + 1]), sc2, -h1));
-              if ((j & 6) == 0) la += e0 + e1;
-              else if ((j & 6) == 2) lb += e0 + e1;
-              else if ((j & 6) == 4) lc += e0 + e1;
-              else ld += e0 + e1;
               w[j >> 1] = pack_bf16(e0, e1);
             }
-            l_part += (la + lb) + (lc + ld);
           } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) w[j] = 0u;
@@ -371,7 +361,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       if (last) mma_commit(bar_o);
       }
       __syncwarp();
-      if (STORE_P && lane == 0) {                                   // these tiles are final: store them now
+      if (lane == 0) {                                              // these tiles are final: store them now
         for (int t = 0; t < nt; ++t)
           tma_store_2d(&tmP, sP + (b0 + t) * VT_BYTES, 0, (int)(((size_t)bh * nnzb + rp + t0 + t) * BS));
         bulk_commit();
@@ -386,7 +376,6 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
         const float l = l_part + __shfl_xor_sync(0xffffffffu, l_part, 16) + (float)(L - n_sel) * exp2f(-m2);
         lse_fixed = m2 + log2f(l);
         m2 = lse_fixed;                                             // pass B then produces normalised P directly
-        l_part = 0.f;
       }
     };
 
@@ -403,8 +392,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
           finish_stats();
         }
         SPION_STAMP(ord, 2);
-        if (ctl) {
-        } else if (STORE_P) {
+        if (!ctl) {
           // keep both tiles' exponentials packed in registers, normalise once the denominator is known
           uint32_t wp[2][32];
 #pragma unroll
@@ -448,8 +436,6 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
               store_row_swizzled(sP + t * VT_BYTES, row, wp[p]);
             }
           }
-        } else {
-          prob_math(0u, 0, 0, nblk, 2);
         }
         SPION_STAMP(ord, 3);
         fence_proxy_async();                                        // P rows -> visible to the MMA proxy
@@ -493,7 +479,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
         ps ^= 1u;
         tc_fence_after();
         if (c > 0 && ctl && g + 1 < njobs) {                        // chunk c-1 is finished: its half takes job g+1
-          if (STORE_P && lane == 0) bulk_wait_read_all();           // once the tile stores have read it
+          if (lane == 0) bulk_wait_read_all();                      // once the tile stores have read it
           __syncwarp();
           issue_job(R, bh, g + 1);
         }
@@ -516,14 +502,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
     SPION_STAMP(ord, 6);
     // ------------------------------------------------------------------ output rows of this unit
     if (ok && !ctl) {
-      float inv = 1.0f, lse2 = lse_fixed;
-      if (!STORE_P) {
-        const float l = l_part + __shfl_xor_sync(0xffffffffu, l_part, 16) + (float)(L - n_sel) * exp2f(-m2);
-        inv = 1.0f / l;
-        lse2 = m2 + log2f(l);
-      } else if (nblk == 0) {
-        lse2 = m2 + log2f((float)L * exp2f(-m2));
-      }
+      const float lse2 = nblk == 0 ? m2 + log2f((float)L * exp2f(-m2)) : lse_fixed;
       if (hf == 0) lse_out[(size_t)bh * L + r * BS + row] = lse2;
       // the accumulator rows sit in lanes 0-15 of every quadrant: those lanes write the whole row
       __nv_bfloat16* dst = O + (size_t)(pos.row0 + r * BS + row) * pos.ld + pos.x0;
@@ -541,10 +520,10 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
             uint4 pk4;
-            pk4.x = pack_bf16(__uint_as_float(v[j]) * inv, __uint_as_float(v[j + 1]) * inv);
-            pk4.y = pack_bf16(__uint_as_float(v[j + 2]) * inv, __uint_as_float(v[j + 3]) * inv);
-            pk4.z = pack_bf16(__uint_as_float(v[j + 4]) * inv, __uint_as_float(v[j + 5]) * inv);
-            pk4.w = pack_bf16(__uint_as_float(v[j + 6]) * inv, __uint_as_float(v[j + 7]) * inv);
+            pk4.x = pack_bf16(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+            pk4.y = pack_bf16(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+            pk4.z = pack_bf16(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5]));
+            pk4.w = pack_bf16(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7]));
             *reinterpret_cast<uint4*>(dst + h * 32 + j) = pk4;
           }
         }
@@ -564,7 +543,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
     R = Rn;
     bh = bhn;
   }
-  if (STORE_P && ctl && lane == 0) bulk_wait_read_all();          // shared memory must outlive the tile stores
+  if (ctl && lane == 0) bulk_wait_read_all();                     // shared memory must outlive the tile stores
   tc_fence_before();
   __syncthreads();
   if (ctl) tmem_dealloc(tmem, ncols);
@@ -580,18 +559,14 @@ template <int D>
 static int fwd_attrs(TcState* s, int device) {
   const int bytes = (int)fwd_smem_bytes<D>();
   int occ = 1 << 30, n = 0, rc;
-#define SPION_FWD_ATTR(SP, SB, KP)                                                                                      \
-  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_fused<D, SP, SB, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
-  if ((rc = resident_ctas(k_fwd_fused<D, SP, SB, KP>, device, FWD_THREADS, (size_t)bytes, 128, &n))) return rc;         \
+#define SPION_FWD_ATTR(SB, KP)                                                                                       \
+  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_fused<D, SB, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));  \
+  if ((rc = resident_ctas(k_fwd_fused<D, SB, KP>, device, FWD_THREADS, (size_t)bytes, 128, &n))) return rc;          \
   occ = n < occ ? n : occ;
-  SPION_FWD_ATTR(false, false, false)
-  SPION_FWD_ATTR(false, false, true)
-  SPION_FWD_ATTR(true, false, false)
-  SPION_FWD_ATTR(true, false, true)
-  SPION_FWD_ATTR(false, true, false)
-  SPION_FWD_ATTR(false, true, true)
-  SPION_FWD_ATTR(true, true, false)
-  SPION_FWD_ATTR(true, true, true)
+  SPION_FWD_ATTR(false, false)
+  SPION_FWD_ATTR(false, true)
+  SPION_FWD_ATTR(true, false)
+  SPION_FWD_ATTR(true, true)
 #undef SPION_FWD_ATTR
   s->fwd_ctas = occ;
   return SPION_OK;
@@ -611,34 +586,29 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
     return rc;
   if (P64) { if ((rc = make_map(s, &mp, P64, vrows, BS, BS, BS))) return rc; } else mp = mq;
   prof_mark(c, -1);
-  if (!P64 && s->n_long > 0) {
-    if ((rc = stream_forward(c, s, mq, mk, mv, keypad, O, lse))) return rc;
-    prof_mark(c, SPION_STAGE_FUSED_FWD);
-    return SPION_OK;
-  }
   // Masks whose rows all have at most four blocks run on the pipelined kernel for short rows
   // (tc_fwd_pipe.cu: about 1.7x less time per row, two CTAs per SM).  As soon as some rows are longer,
-  // everything goes through this file's kernel: a second launch for a handful of long rows costs more
-  // than the pipelining gains (measured at 5 % density, L = 4096: 79 us split against 70 us in one launch).
-  const bool all_short = s->n_long == 0;
-  const int rows_here = all_short ? 0 : vw.nb;
-  const long long total = (long long)c->BH * rows_here;
-  const float floor_v = keypad ? 0.0f : -100.0f;
-  if (total > 0) {
-    const int grid = (int)(total < (long long)s->sms * s->fwd_ctas ? total : (long long)s->sms * s->fwd_ctas);
-#define SPION_FWD_LAUNCH(SP, SB, KP)                                                                                  \
-  k_fwd_fused<D, SP, SB, KP><<<grid, FWD_THREADS, fwd_smem_bytes<D>(), c->stream>>>(                                   \
-      mq, mk, mv, mp, (__nv_bfloat16*)O, lse, keypad, vw.row_info, vw.col_idx, vw.submask, c->L, vw.nnzb, c->BH,   \
-      rows_here, c->heads, c->scale, floor_v, c->status_dev)
-#define SPION_FWD_PICK(SP, SB) do { if (keypad) SPION_FWD_LAUNCH(SP, SB, true); else SPION_FWD_LAUNCH(SP, SB, false); } while (0)
-    if (P64) { if (vw.submask) SPION_FWD_PICK(true, true); else SPION_FWD_PICK(true, false); }
-    else { if (vw.submask) SPION_FWD_PICK(false, true); else SPION_FWD_PICK(false, false); }
-#undef SPION_FWD_PICK
-#undef SPION_FWD_LAUNCH
+  // everything goes through one kernel: a second launch for a handful of long rows costs more
+  // than the pipelining gains (measured at 5 % density, L = 4096: 79 us split against 70 us in one launch).  Without P that is the
+  // streaming kernel (tc_fwd_stream.cu), with P this file's, whose probabilities are rounded after the normalisation.
+  if (s->n_long == 0) {
+    if ((rc = pipe_forward(c, s, mq, mk, mv, mp, P64 != nullptr, keypad, O, lse, 0))) return rc;
+  } else if (!P64) {
+    if ((rc = stream_forward(c, s, mq, mk, mv, keypad, O, lse))) return rc;
+  } else {
+    const long long total = (long long)c->BH * vw.nb, cap = (long long)s->sms * s->fwd_ctas;
+    const float floor_v = keypad ? 0.0f : -100.0f;
+    const int grid = (int)(total < cap ? total : cap);
+    auto launch = [&](auto k) {
+      k<<<grid, FWD_THREADS, fwd_smem_bytes<D>(), c->stream>>>(mq, mk, mv, mp, (__nv_bfloat16*)O, lse, keypad, vw.row_info, vw.col_idx,
+                                                              vw.submask, c->L, vw.nnzb, c->BH, vw.nb, c->heads, c->scale, floor_v,
+                                                              c->status_dev);
+    };
+    if (vw.submask) { if (keypad) launch(k_fwd_fused<D, true, true>); else launch(k_fwd_fused<D, true, false>); }
+    else { if (keypad) launch(k_fwd_fused<D, false, true>); else launch(k_fwd_fused<D, false, false>); }
     SPION_LAUNCH_CHECK();
     c->launches += 1;
   }
-  if (all_short && (rc = pipe_forward(c, s, mq, mk, mv, mp, P64 != nullptr, keypad, O, lse, 0))) return rc;
   prof_mark(c, SPION_STAGE_FUSED_FWD);
   return SPION_OK;
 }

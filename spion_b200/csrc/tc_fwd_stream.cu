@@ -15,7 +15,8 @@
 // maximum at the end.  P <= 2^8 loses nothing in bf16 or in the fp32 sums.
 //
 // What bounds it: the exponentials, 8192 per pair at 16 per cycle and SM = 512 cycles, and 16 MMAs of 33 cycles at head_dim 64.
-// Measured (forward alone, this kernel against one unit per CTA and two passes over a row, tc_fused.cu):  see fwd_launch there.
+// Measured, forward alone, before (one unit per CTA, two passes over a row) and now: 64 matrices, L = 4096, d 64, 5 % 62 -> 44 us,
+// 30 % 314 -> 151; L = 16384, 5 % 847 -> 385; 256 matrices, L = 4096, d 32, 10 %, padded keys 585 -> 229.
 //
 // Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
 #include "tc_stream.cuh"
@@ -61,7 +62,7 @@ struct FsArgs {
   int* status;
 };
 
-// EXACT: two passes over a row, the maximum first, and the sums in the order of tc_fused.cu: O and lse bit for bit as that kernel
+// EXACT: two passes over a row, the maximum first, and the sums in a fixed order (four chains a half tile): O and lse bit for bit as a two-pass kernel
 // gives them.  For the full mask, where some results are sums that cancel to nothing but rounding (the gradient of the key
 // projection's bias is zero in dense attention), so that every other order of the additions gives other numbers.
 template <int D, bool KP, bool SUB, bool EXACT>

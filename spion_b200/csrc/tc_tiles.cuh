@@ -70,7 +70,7 @@ struct ValTile {
 
 // Padded keys in the blocks of a warp whose half-warps work on one 64-key block each (kp: the penalties of this half-warp's block).
 // Padding is a tail of the sequence, so most blocks have none and take the path without 64 penalty loads per row: the forward of
-// 128 x 2 matrices, L = 4096, d = 32, 10 % goes from 556 to 420 us (O only) with half of the keys of a sequence padded at most.
+// 128 x 2 matrices, L = 4096, d = 32, 10 % went from 556 to 485 us (O only) with half of the keys of a sequence padded at most.
 __device__ __forceinline__ bool any_padded(const float* kp) {
   bool v = false;
 #pragma unroll
