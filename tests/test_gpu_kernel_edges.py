@@ -1,0 +1,134 @@
+"""The attention and discovery kernels at the sizes where their loops and dispatch rules end: lines of every length, empty lines,
+full masks, one more and one fewer than what fills the chip, several maps per call."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import attention as oatt
+from oracle import csr as ocsr
+from oracle import pattern as opat
+from spion_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+# fp32: the reference's parity bound, max-abs
+FP32_TOL = 1e-4
+# bf16: P, dS and the results are rounded to 2^-9 each, and an output is a sum of products of two of them: at most 3 * 2^-9 = 6e-3
+# of the sum of magnitudes, which exceeds the largest output by a factor of about three in these inputs
+BF16_REL = 2e-2
+
+
+def cfg(B, H, L, d, bs):
+    return {"head_dim": d, "num_head": H, "max_seq_len": L, "batch_size": B, "block_size": bs, "transformer_dim": H * d, "task": "t"}
+
+
+def far(a, b, relative):
+    a, b = a.detach().float().cpu(), b.detach().float().cpu()
+    return float((a - b).abs().max() / (b.abs().max().clamp_min(1e-30) if relative else 1.0))
+
+
+def lines_of_every_length(nb, zero=True):
+    """Row r has r + 1 blocks, column c nb - c; with `zero` one row and one column without any."""
+    mat = np.tril(np.ones((nb, nb), dtype=np.uint8))
+    if zero:
+        mat[nb // 2, :] = 0
+        mat[:, nb // 3] = 0
+    return mat
+
+
+def run(mod, Q, K, V, dO, mat, kp):
+    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+    out, _ = mod(q, k, v, None if kp is None else kp.cuda(), torch.as_tensor(mat).cuda())
+    out.backward(dO.cuda())
+    mod.check_device_status()
+    return out, q.grad, k.grad, v.grad
+
+
+def compare(got, Q, K, V, dO, mat, bs, kp, tol, relative):
+    O, _, gQ, gK, gV = oatt.sparse_attention(Q.float(), K.float(), V.float(), mat, bs, kp, dO.float())
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), got, (O, gQ, gK, gV)):
+        assert far(a, b, relative) <= tol, f"{name}: {far(a, b, relative):.3e}"
+
+
+@pytest.mark.parametrize("d,bs", [(64, 64), (32, 64), (32, 32)])
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("case", ["lines", "full", "growing"])
+def test_streaming_forward_and_backward(d, bs, padded, case):
+    """No stored P: rows and columns of 1 to 11 blocks, none at all, an odd last pair; the full mask; scores that outgrow the
+    maximum a row started with.  bs 32: the super-block form, with quarters of a block switched off."""
+    from spion_b200.native import BlockSparseAttention
+    B, H, nb = 2, 3, 11 if bs == 64 else 22
+    L = nb * bs
+    Q, K, V, dO = (t.to(torch.bfloat16) for t in synthetic.qkv(3 + d, B, H, L, d))
+    if case == "growing":
+        K = (K.float() * torch.linspace(0.5, 12.0, L)[:, None]).to(torch.bfloat16)
+    mat = np.ones((nb, nb), np.uint8) if case == "full" else lines_of_every_length(nb, case == "lines")
+    kp = synthetic.key_padding(5, B, L) if padded else None
+    mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.bfloat16, keypad=padded, recompute=True, return_probs=False)
+    got = run(mod, Q, K, V, dO, mat, kp)
+    compare(got, Q, K, V, dO, mat, bs, kp, BF16_REL, True)
+    with torch.no_grad():                                    # and without a backward
+        out, _ = mod(Q.cuda(), K.cuda(), V.cuda(), None if kp is None else kp.cuda(), torch.as_tensor(mat).cuda())
+    assert torch.equal(out, got[0].detach())
+
+
+# (bs, d, B, H, blocks per side): few threads' worth of work (four rows per thread), more (eight; columns split over clusters), many
+# (eight; one CTA per column group); groups of four matrices with one, two and three left over
+@pytest.mark.parametrize("bs,d,B,H,nb", [(32, 32, 1, 1, 1), (32, 64, 1, 3, 7), (64, 32, 1, 1, 2), (64, 64, 2, 1, 9),
+                                         (32, 32, 50, 3, 8), (32, 64, 42, 5, 7), (64, 32, 40, 1, 8), (64, 64, 7, 5, 9),
+                                         (32, 32, 301, 3, 8), (64, 64, 119, 3, 5)])
+def test_fp32_fused_kernels(bs, d, B, H, nb):
+    from spion_b200.native import BlockSparseAttention
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(17 + nb, B, H, L, d)
+    mat = lines_of_every_length(nb, nb > 4)
+    kp = synthetic.key_padding(9, B, L) if nb % 2 else None
+    mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.float32, keypad=kp is not None)
+    compare(run(mod, Q, K, V, dO, mat, kp), Q, K, V, dO, mat, bs, kp, FP32_TOL, False)
+
+
+@pytest.mark.parametrize("L,d", [(64, 64), (192, 32), (512, 32), (576, 32), (1024, 64), (1088, 32), (1856, 32)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_dense_fp32_kernels(L, d, padded):
+    """One tile, ragged softmax slices, the longest slice in registers (64 and 128 values) and one more, a slab too long for shared
+    memory."""
+    from spion_b200.attention import Attention
+    from spion_b200.attention_cuda import CUDAAttention
+    from spion_b200.attention_cuda_mask import CUDAMaskAttention
+    B, H = 1, 2
+    Q, K, V, dO = synthetic.qkv(31 + L, B, H, L, d)
+    kp = synthetic.key_padding(2, B, L) if padded else torch.ones(B, L)
+    cpp = Attention._cuda_mask_compile_module() if padded else Attention._cuda_compile_module()
+    handle = cpp.init(d, L, B * H)
+    mod = (CUDAMaskAttention if padded else CUDAAttention)(cfg(B, H, L, d, 32), cpp, handle)
+    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+    out, attn = mod(q, k, v, kp.cuda())
+    out.backward(dO.cuda())
+    O, P, gQ, gK, gV = oatt.dense_attention(Q, K, V, kp if padded else None, dO)
+    assert far(attn, P, False) <= 1e-6
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), (out, q.grad, k.grad, v.grad), (O, gQ, gK, gV)):
+        assert far(a, b, False) <= FP32_TOL, f"{name}: {far(a, b, False):.3e}"
+    cpp.destroy(handle)
+
+
+@pytest.mark.parametrize("layers,L,bs,misaligned", [(1, 64, 64, False), (3, 160, 32, False), (2, 320, 64, True), (17, 128, 32, False)])
+def test_discovery_of_several_layers(layers, L, bs, misaligned):
+    """One cell, ragged map counts, maps that do not start on 16 bytes, more maps than one call takes: bit for bit the oracle."""
+    from spion_b200 import pattern
+    maps = [synthetic.structured_map(40 + i, L) for i in range(layers)]
+    gpu = []
+    for A in maps:
+        room = torch.empty(L * L + 1, device="cuda")
+        part = room[1:] if misaligned else room[:-1]
+        gpu.append(part.view(L, L).copy_(A))
+    mats, patterns = pattern.discover_layers(gpu, {"block_size": bs, "max_seq_len": L, "threshold": 0.8})
+    assert mats.shape == (4, layers, L // bs, L // bs)
+    for i, A in enumerate(maps):
+        want, thresh, pooled = opat.discover_block_mask(A.numpy(), bs, 0.8, 31, 0, float_path="fixed")
+        p = patterns[i]
+        assert np.array_equal(p.pooled.cpu().numpy(), pooled) and float(p.thresh) == float(thresh)
+        assert np.array_equal(p.mat.cpu().numpy(), want)
+        assert all(np.array_equal(mats[r, i].cpu().numpy(), want.astype(np.float32)) for r in range(4))
+        rp, ci, br = ocsr.block_csr(want)
+        cp, ri, pos = ocsr.block_csc(want)
+        for got, ref in ((p.row_ptr, rp), (p.col_idx, ci), (p.blk_row, br), (p.col_ptr, cp), (p.row_idx, ri), (p.csc_pos, pos)):
+            assert np.array_equal(got.cpu().numpy(), ref)
