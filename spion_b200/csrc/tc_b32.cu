@@ -9,7 +9,8 @@
 //               S^T[128 keys x 32 q] = K_g Q_r^T           (K_g: four selected key blocks, K-major A, M = 128)
 //               row statistics across the keys, P^T = exp2(.) as bf16 rows of 32 queries
 //               O^T[64 d x 32 q]   += V_g^T P^T            (V_g as MN-major A, P^T as MN-major B)
-//               two passes over the row's blocks (maximum, then exponentials); replaces
+//               two passes over the row's blocks (maximum, then exponentials), S kept in tensor memory between them for rows of
+//               up to twelve blocks; replaces
 //               models/block_attn.cu:453-487 for 32-wide masks
 //   k_b32<ROW>  unit = block row r:   S^T, dP^T = V_g dO_r^T  ->  dS^T  ->  dQ^T += K_g^T dS^T;  writes delta
 //   k_b32<COL>  unit = block column c (32 keys): four selected query blocks gathered,
@@ -58,9 +59,13 @@ template <int MODE> struct Cfg {
   static constexpr uint32_t OFF_G1 = D0 * GB, OFF_V = OFF_G1 + D1 * GB, OFF_U = OFF_V + 2 * NVAL * VB;
   static constexpr uint32_t TILES = OFF_U + UBUF * NUNIT * TB;
   static constexpr uint32_t SMEM = 1024 + TILES;       // + alignment slack
-  static constexpr uint32_t TMEM_COLS = FWD ? 128 : 256;
-  // tensor-memory columns: S (two stages), dP (two stages), accumulators
-  static constexpr uint32_t S_COL = 0, DP_COL = 64, ACC_COL = FWD ? 64 : 128;
+  static constexpr uint32_t TMEM_COLS = 256;
+  // S slots in tensor memory.  The forward keeps the S tiles of a unit of at most KEEP jobs from its first pass to its second (which
+  // then needs no S product and no K_g), with as many slots for the unit after it: at 5 % of 128 x 128 blocks nearly all units
+  // (64 matrices: 128 -> 124 us with the later output rows).
+  static constexpr int SL = FWD ? 6 : 2, KEEP = FWD ? 3 : 0;
+  // tensor-memory columns: S slots, dP (two stages), accumulators
+  static constexpr uint32_t S_COL = 0, DP_COL = 64, ACC_COL = FWD ? 32 * SL : 128;
 };
 
 __device__ __forceinline__ float ex2a(float x) {
@@ -108,6 +113,7 @@ template <int MODE> struct Cursor {
   const int4* rec;
   int total, BH, stride;
   int u, uc, jg, jb;           // unit index in the launch; units with work, jobs, jobs with second products seen so far
+  int js, us;                  // first products seen so far, and at the start of the unit
   int rp, n, line, bh;         // the unit: start in the index array, blocks, block row / column, (b,h) matrix
   int id01, id23;              // its first four block ids
   int nch, njobs, jl;
@@ -129,7 +135,7 @@ template <int MODE> struct Cursor {
   }
   __device__ void init(const int4* rec_, int total_, int BH_) {
     rec = rec_; total = total_; BH = BH_; stride = gridDim.x;
-    u = blockIdx.x; uc = 0; jg = 0; jb = 0; jl = 0;
+    u = blockIdx.x; uc = 0; jg = 0; jb = 0; jl = 0; js = 0; us = 0;
     valid = u < total;
     if (valid) set(rec[u / BH]);
     request_next();
@@ -145,6 +151,9 @@ template <int MODE> struct Cursor {
   __device__ int first_id(int t) const { return (((t & 2) ? id23 : id01) >> ((t & 1) * 16)) & 0xffff; }
   // the job at the cursor
   __device__ bool is_b() const { return !Cfg<MODE>::FWD || jl >= nch; }       // has second products
+  __device__ bool keep() const { return nch <= Cfg<MODE>::KEEP; }               // S stays from pass A to pass B
+  __device__ bool is_a() const { return !Cfg<MODE>::FWD || jl < nch || !keep(); }   // has a first product
+  __device__ bool last_a() const { return jl == (Cfg<MODE>::FWD && keep() ? nch : njobs) - 1; }
   __device__ int chunk() const { return (Cfg<MODE>::FWD && jl >= nch) ? jl - nch : jl; }
   __device__ int t0() const { return chunk() * GN; }
   __device__ int nt() const { return min(GN, n - t0()); }
@@ -153,28 +162,29 @@ template <int MODE> struct Cursor {
   // step to the next job (callers skip empty units themselves)
   __device__ void advance() {
     ++jg;
+    if (is_a()) ++js;
     if (is_b()) ++jb;
-    if (++jl == njobs) { ++uc; next_unit(); }
+    if (++jl == njobs) { ++uc; us = js; next_unit(); }
   }
 };
 
 // Barrier slots (8 bytes each) in shared memory.  A parity wait only tells two consecutive phases of a barrier
 // apart, so every waiter waits for every phase of the barriers it uses: the barriers of K_g / Q_g, S and dP
-// get one phase per job (index j), those of V_g / dO_g, the value buffers and the second products one phase
-// per job that has second products (index jb; in the backward kernels every job has them, jb = j).
+// get one phase per first product (index js; in the backward kernels every job has one, js = j), those of V_g / dO_g, the value
+// buffers and the second products one phase per job that has second products (index jb; in the backward kernels jb = j).
 enum : int {
   BAR_FULL0 = 0,    // [3] gathered operand 0 (+ the unit's small operands with the unit's first job) has landed
   BAR_FULL1 = 3,    // [2] gathered operand 1 has landed
   BAR_FREE0 = 5,    // [3] the products that read slot j % D0 of ring 0 have retired
   BAR_FREE1 = 8,    // [2] ... slot j & 1 of ring 1
-  BAR_SREADY = 10,  // [2] first products of the job retired: S (and dP) are in tensor memory
-  BAR_MDONE = 12,   // [2] the four math warps have read S / dP out of tensor memory
-  BAR_ODONE = 14,   // [2] second products of the job retired: its value buffers are free
-  BAR_OFULL = 16,   // [2] the unit's accumulator is complete
-  BAR_OFREE = 18,   // [2] ... and has been read out
-  BAR_UFREE = 20,   // [2] the first products of a unit no longer need its small operands
-  BAR_PREADY = 22,  // [2] the four math warps have written the value rows of a job with second products
-  BAR_COUNT = 24
+  BAR_SREADY = 10,  // [6] first products of the job retired: S (and dP) are in tensor memory
+  BAR_MDONE = 16,   // [6] the four math warps have read S / dP out of tensor memory
+  BAR_ODONE = 22,   // [2] second products of the job retired: its value buffers are free
+  BAR_OFULL = 24,   // [2] the unit's accumulator is complete
+  BAR_OFREE = 26,   // [2] ... and has been read out
+  BAR_UFREE = 28,   // [2] the first products of a unit no longer need its small operands
+  BAR_PREADY = 30,  // [2] the four math warps have written the value rows of a job with second products
+  BAR_COUNT = 32
 };
 
 template <int MODE>
@@ -200,7 +210,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
   __shared__ __align__(16) float s_red0[4][32];   // FWD: per-warp maxima; ROW: lse; COL: key padding (two units each)
   __shared__ __align__(16) float s_red1[4][32];   // FWD: per-warp sums;   ROW: -delta scale (two units)
   __shared__ __align__(16) float s_mw[4][32];     // FWD: the unit's maxima, one copy per math warp
-  __shared__ __align__(16) float s_inv[32];       // FWD: 1 / denominator
+  __shared__ __align__(16) float s_inv[2][32];    // FWD: 1 / denominator (two units)
 
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   auto sG0 = [&](int k) -> uint32_t { return sbase + k * GB; };
@@ -218,7 +228,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
   if (tid == 0) {
     s_abort = *reinterpret_cast<volatile int*>(status);
     for (int i = 0; i < BAR_COUNT; ++i) {
-      const bool by_math = (i >= BAR_MDONE && i < BAR_MDONE + 2) || (i >= BAR_OFREE && i < BAR_OFREE + 2) || i >= BAR_PREADY;
+      const bool by_math = (i >= BAR_MDONE && i < BAR_MDONE + 6) || (i >= BAR_OFREE && i < BAR_OFREE + 2) || i >= BAR_PREADY;
       mbar_init(bar(i, 0), by_math ? 4 : 1);
     }
     mbar_init(smem_u32(&s_math_bar), 4);
@@ -254,11 +264,11 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
     int pblk = 0;
     bool ok = true;
     while (ok && cl.valid) {
-      const int j = cl.jg, jb = cl.jb, s0 = j % C::D0, s1 = jb & 1;
+      const int j = cl.js, jb = cl.jb, s0 = j % C::D0, s1 = jb & 1;
       const int ub = C::UBUF == 2 ? (cl.uc & 1) : 0;
-      const bool two = !C::FWD || cl.is_b();                               // G1 as well
+      const bool one = cl.is_a(), two = !C::FWD || cl.is_b();              // G0, G1
       if (lane == 0) {
-        if (j >= C::D0) ok = wait1(bar(BAR_FREE0, s0), ((uint32_t)(j / C::D0) & 1u) ^ 1u, ERR_MMA2_WAIT | 0x10);
+        if (one && j >= C::D0) ok = wait1(bar(BAR_FREE0, s0), ((uint32_t)(j / C::D0) & 1u) ^ 1u, ERR_MMA2_WAIT | 0x10);
         if (ok && two && jb >= 2) ok = wait1(bar(BAR_FREE1, s1), ((uint32_t)(jb >> 1) & 1u) ^ 1u, ERR_MMA2_WAIT | 0x20);
         if (ok && cl.jl == 0 && cl.uc >= C::UBUF)          // the unit that used this set of small operands before
           ok = wait1(bar(BAR_UFREE, ub), (C::UBUF == 2 ? ((uint32_t)(cl.uc >> 1) & 1u) : ((uint32_t)cl.uc & 1u)) ^ 1u, ERR_MMA_WAIT | 0x40);
@@ -270,11 +280,11 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
       const OpPos pos = op_pos(cl.bh, L, heads, HD);
       const int blk = t0 == 0 ? cl.first_id(li & 3) : pblk;
       if (lane == 0) {
-        mbar_expect_tx(bar(BAR_FULL0, s0), (uint32_t)nt * TB + (cl.jl == 0 ? C::NUNIT * TB : 0u));
+        if (one) mbar_expect_tx(bar(BAR_FULL0, s0), (uint32_t)nt * TB + (cl.jl == 0 ? C::NUNIT * TB : 0u));
         if (two) mbar_expect_tx(bar(BAR_FULL1, s1), (uint32_t)nt * TB);
       }
       __syncwarp();
-      if (lane < nt) tma_load_2d(sG0(s0) + lane * TB, &tmG0, bar(BAR_FULL0, s0), pos.x0, pos.row0 + blk * B32);
+      if (one && lane < nt) tma_load_2d(sG0(s0) + lane * TB, &tmG0, bar(BAR_FULL0, s0), pos.x0, pos.row0 + blk * B32);
       if (two && lane >= 8 && lane < 8 + nt)
         tma_load_2d(sG1(s1) + (lane - 8) * TB, &tmG1, bar(BAR_FULL1, s1), pos.x0, pos.row0 + blk * B32);
       if (cl.jl == 0) {
@@ -296,13 +306,18 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
       while (cm.empty()) cm.next_unit();
       bool ok = true;
       while (ok && cm.valid) {
-        const int j = cm.jg, s0 = j % C::D0, s1 = cm.jb & 1, st = j & 1;      // backward kernels: jb = j
-        const uint32_t ph = (uint32_t)(j >> 1) & 1u;
+        if (!cm.is_a()) {
+          cm.advance();
+          while (cm.empty()) cm.next_unit();
+          continue;
+        }
+        const int j = cm.js, s0 = j % C::D0, s1 = cm.jb & 1, st = j % C::SL;  // backward kernels: jb = j
+        const uint32_t ph = (uint32_t)(j / C::SL) & 1u;
         const int ub = C::UBUF == 2 ? (cm.uc & 1) : 0;
         SPION_STAMP_T(160, j, 2);
         ok = wait1(bar(BAR_FULL0, s0), (uint32_t)(j / C::D0) & 1u, ERR_LOAD_WAIT | 0x100);
         if (ok && !C::FWD) ok = wait1(bar(BAR_FULL1, s1), ph, ERR_LOAD_WAIT | 0x200);
-        if (ok && j >= 2) ok = wait1(bar(BAR_MDONE, st), ph ^ 1u, ERR_MMA_WAIT | 0x400);      // S / dP columns read out
+        if (ok && j >= C::SL) ok = wait1(bar(BAR_MDONE, st), ph ^ 1u, ERR_MMA_WAIT | 0x400);      // S / dP columns read out
         if (!ok) break;
         SPION_STAMP_T(160, j, 3);
         tc_fence_after();
@@ -319,7 +334,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
         mma_commit(bar(BAR_SREADY, st));
         if (C::FWD) mma_commit(bar(BAR_FREE0, s0));                      // K_g is not read again
         if (C::ROW) mma_commit(bar(BAR_FREE1, s1));                      // V_g is not read again
-        if (cm.last()) mma_commit(bar(BAR_UFREE, ub));
+        if (cm.last_a()) mma_commit(bar(BAR_UFREE, ub));
         SPION_STAMP_T(160, j, 4);
         cm.advance();
         while (cm.empty()) cm.next_unit();
@@ -336,7 +351,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
       bool ok = true;
       while (ok && co.valid) {
         if (co.is_b()) {
-          const int j = co.jg, jb = co.jb, s0 = j % C::D0, s1 = jb & 1, ob = co.uc & 1;
+          const int j = co.js, jb = co.jb, s0 = j % C::D0, s1 = jb & 1, ob = co.uc & 1;
           const int st = s1;                                                  // value buffers of the job
           const uint32_t ph = (uint32_t)(jb >> 1) & 1u;
           SPION_STAMP_T(192, j, 5);
@@ -428,6 +443,41 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
     int pblk = 0;
     bool pre_job = false;
 
+    // The output rows of a unit (transposed accumulators) are written after the first pass (FWD) or the per-unit vectors (ROW, COL)
+    // of the next one: the wait for its last product is 0.2 - 0.7 us otherwise, of 4.6 us per unit (64 matrices, L = 4096, 5 %:
+    // ROW 116 -> 88 us; COL, whose two ring slots are the limit, 113 either way; inside the job loop it cost spills, COL 133).
+    bool pend = false;
+    size_t p_off = 0;
+    int p_ob = 0;
+    uint32_t p_full = 0;
+    const int out_ld = op_pos(0, L, heads, HD).ld;
+    auto flush = [&]() -> bool {
+      if (!pend) return true;
+      pend = false;
+      if (!mbar_wait(bar(BAR_OFULL, p_ob), p_full)) { report(status, ERR_MMA2_WAIT | 0x80000); return false; }
+      tc_fence_after();
+      uint32_t v[32];
+      tmem_ld32(t_lane + C::ACC_COL + (C::COL ? p_ob * 32 : 0), v);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(BAR_OFREE, p_ob));
+      // lanes 0-15 / 16-31 of every quadrant hold rows 16 warp + (lane & 15) of two accumulators:
+      // FWD / ROW: the units of even / odd ordinal; COL: dK^T / dV^T of this unit
+      const int jd = warp * 16 + (lane & 15);
+      if (C::COL) {
+        __nv_bfloat16* dst = (lane < 16 ? out0 : out1) + p_off + jd;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) dst[(size_t)i * out_ld] = __float2bfloat16(__uint_as_float(v[i]));
+      } else if ((lane >> 4) == p_ob) {
+        __nv_bfloat16* dst = out0 + p_off + jd;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          dst[(size_t)i * out_ld] = __float2bfloat16(__uint_as_float(v[i]) * (C::FWD ? s_inv[p_ob][i] : 1.0f));
+      }
+      return true;
+    };
+
     while (ok && c.valid) {
       const OpPos pos = op_pos(c.bh, L, heads, HD);
       const int line = c.line, bh = c.bh, n = c.n, rp = c.rp, nch = c.nch;
@@ -454,15 +504,17 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
 
       if (C::FWD) {
         // ------------------------------------------------ pass A: maxima per query, kept per lane (= per key slot)
+        const bool keep = c.keep();
+        const int us = c.us;
         float mx[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) mx[i] = -INFINITY;
         for (int jl = 0; jl < nch && ok; ++jl) {
-          const int st = c.jg & 1, t0 = jl * GN, nt = min(GN, n - t0);
+          const int st = c.js % C::SL, t0 = jl * GN, nt = min(GN, n - t0);
           float pad = 0.f;
           if (kp && warp < nt) pad = kp[(t0 == 0 ? c.first_id(warp) : idx[rp + t0 + warp]) * B32 + lane] * LOG2E;
           SPION_STAMP_T(0, c.jg, 8);
-          if (!mbar_wait(bar(BAR_SREADY, st), (uint32_t)(c.jg >> 1) & 1u)) { report(status, ERR_MMA_WAIT | 0x20000); ok = false; break; }
+          if (!mbar_wait(bar(BAR_SREADY, st), (uint32_t)(c.js / C::SL) & 1u)) { report(status, ERR_MMA_WAIT | 0x20000); ok = false; break; }
           SPION_STAMP_T(0, c.jg, 9);
           tc_fence_after();
           if (warp < nt) {
@@ -473,12 +525,13 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
             for (int i = 0; i < 32; ++i) mx[i] = fmaxf(mx[i], fmaf(__uint_as_float(v[i]), sc2, -pad));
           }
           SPION_STAMP_T(0, c.jg, 10);
-          job_done(st, -1);
+          if (!keep) job_done(st, -1);
           c.advance();
         }
         if (!ok) break;
         s_red0[warp][lane] = lanes_reduce32<true>(mx, lane);
         if (!math_sync()) { report(status, ERR_MMA_WAIT | 0x100000); ok = false; break; }
+        if (!flush()) { ok = false; break; }
         // every warp keeps its own copy of the 32 maxima (no second CTA-wide meeting)
         s_mw[warp][lane] = fmaxf(fmaxf(floor2, s_red0[0][lane]), fmaxf(fmaxf(s_red0[1][lane], s_red0[2][lane]), s_red0[3][lane]));
         __syncwarp();
@@ -487,11 +540,11 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
 #pragma unroll
         for (int i = 0; i < 32; ++i) z[i] = 0.f;
         for (int jl = 0; jl < nch && ok; ++jl) {
-          const int st = c.jg & 1, t0 = jl * GN, nt = min(GN, n - t0);
+          const int sj = keep ? us + jl : c.js, st = sj % C::SL, t0 = jl * GN, nt = min(GN, n - t0);
           float pad = 0.f;
           if (kp && warp < nt) pad = kp[(t0 == 0 ? c.first_id(warp) : idx[rp + t0 + warp]) * B32 + lane] * LOG2E;
           SPION_STAMP_T(0, c.jg, 8);
-          if (!mbar_wait(bar(BAR_SREADY, st), (uint32_t)(c.jg >> 1) & 1u)) { report(status, ERR_MMA_WAIT | 0x20000); ok = false; break; }
+          if (!keep && !mbar_wait(bar(BAR_SREADY, st), (uint32_t)(sj / C::SL) & 1u)) { report(status, ERR_MMA_WAIT | 0x20000); ok = false; break; }
           SPION_STAMP_T(0, c.jg, 9);
           tc_fence_after();
           const int sv = c.jb & 1;
@@ -521,10 +574,9 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
           const float m = s_mw[0][lane];
           const float l = (s_red1[0][lane] + s_red1[1][lane]) + (s_red1[2][lane] + s_red1[3][lane]) +
                           (float)(L - n * B32) * exp2f(-m);
-          s_inv[lane] = 1.0f / l;
+          s_inv[ob][lane] = 1.0f / l;                                   // read by flush(), after the next meeting
           fout[vec0 + lane] = m + log2f(l);
         }
-        if (!math_sync()) { report(status, ERR_MMA_WAIT | 0x100000); ok = false; break; }
       } else {
         // ------------------------------------------------ backward: per-unit vectors into shared memory
         if (C::ROW) {
@@ -551,6 +603,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
           if (tid < 32) s_red0[ub][tid] = kp ? kp[line * B32 + tid] * LOG2E : 0.f;     // penalty of the unit's 32 keys
         }
         if (!math_sync()) { report(status, ERR_MMA_WAIT | 0x100000); ok = false; break; }
+        if (!flush()) { ok = false; break; }                          // in the loop its registers would not fit
         for (int jl = 0; jl < nch && ok; ++jl) {
           const int st = c.jg & 1, t0 = jl * GN, nt = min(GN, n - t0);
           // ROW: this thread is a key of gathered block `warp` (its padding penalty); COL: a query row (its lse and
@@ -617,33 +670,14 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
         if (!ok) break;
       }
 
-      // ------------------------------------------------ output rows of the unit (transposed accumulators)
-      SPION_STAMP_T(0, c.jg - 1, 12);
-      if (!mbar_wait(bar(BAR_OFULL, ob), pfull)) { report(status, ERR_MMA2_WAIT | 0x80000); ok = false; break; }
-      SPION_STAMP_T(0, c.jg - 1, 13);
-      tc_fence_after();
-      {
-        uint32_t v[32];
-        tmem_ld32(t_lane + C::ACC_COL + (C::COL ? ob * 32 : 0), v);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(BAR_OFREE, ob));
-        // lanes 0-15 / 16-31 of every quadrant hold rows 16 warp + (lane & 15) of two accumulators:
-        // FWD / ROW: the units of even / odd ordinal; COL: dK^T / dV^T of this unit
-        const int jd = warp * 16 + (lane & 15);
-        if (C::COL) {
-          __nv_bfloat16* dst = (lane < 16 ? out0 : out1) + out_off + jd;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) dst[(size_t)i * pos.ld] = __float2bfloat16(__uint_as_float(v[i]));
-        } else if ((lane >> 4) == ob) {
-          __nv_bfloat16* dst = out0 + out_off + jd;
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            dst[(size_t)i * pos.ld] = __float2bfloat16(__uint_as_float(v[i]) * (C::FWD ? s_inv[i] : 1.0f));
-        }
-      }
-      SPION_STAMP_T(0, c.jg - 1, 14);
+      pend = true;
+      p_off = out_off;
+      p_ob = ob;
+      p_full = pfull;
+    }
+    if (ok) {
+      if (C::FWD && !math_sync()) report(status, ERR_MMA_WAIT | 0x100000);
+      else flush();
     }
   }
 
