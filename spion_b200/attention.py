@@ -109,12 +109,12 @@ class Attention(nn.Module):
         if not self._linears_are_plain():
             return None
         block = None
+        if mat is None and fp32:
+            return None          # in the dense phase the key bias has no effect: its gradient is the rounding noise of the stages
         if self.native:
             block = self.attn.block if mat is None else self.block_attn
             block.use_mask(mat)
             ctx = block._ctx
-        elif mat is None:
-            return None          # in the dense phase the key bias has no effect: its gradient is the rounding noise of the stages
         else:
             ctx = self.block_attn.context(mat)
         W = [m.weight for m in (self.W_q, self.W_k, self.W_v, self.ff)]
@@ -130,9 +130,15 @@ class Attention(nn.Module):
         layer = self._one_node(X, mask, mat)
         if layer is not None:
             return layer
-        Q = self.split_heads(self.W_q(X))
-        K = self.split_heads(self.W_k(X))
-        V = self.split_heads(self.W_v(X))
+        # native dense phase in fp32: the products whose rounding the key bias's gradient consists of stay the framework's
+        as_before = mat is None and self.native and not torch.is_autocast_enabled()
+
+        def linear(m, x):
+            return m(x, framework=True) if as_before and type(m) is BiasGradLinear else m(x)
+
+        Q = self.split_heads(linear(self.W_q, X))
+        K = self.split_heads(linear(self.W_k, X))
+        V = self.split_heads(linear(self.W_v, X))
         with torch.autocast(device_type="cuda", enabled=False):
             if mat is None and self.native:
                 attn_out, attn = self.attn(Q, K, V, mask.float())
@@ -148,7 +154,7 @@ class Attention(nn.Module):
             else:
                 attn_out, attn = self.block_attn(Q.float(), K.float(), V.float(), mask.float(), mat)
         attn_out = self.combine_heads(attn_out)
-        out = self.ff(attn_out)
+        out = linear(self.ff, attn_out)
         return out, attn
 
     def reconstruct_for_blocksparse(self, config):

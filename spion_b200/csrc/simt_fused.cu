@@ -842,10 +842,12 @@ constexpr long long FEW_WARPS = 148 * 4 * 2;
     return SPION_ERR_UNSUPPORTED;                                       \
   } while (0)
 
+// full: every block is selected (simt_full.cu)
 int simt_fused_forward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,
                        OperandLayout lv, const float* keypad, float floor_v, float* P, ValueLayout vl, float* O,
-                       OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st) {
+                       OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st, bool full) {
   if (!simt_fused_supports(p.bs, d, BH, vl.mode)) return SPION_ERR_UNSUPPORTED;
+  if (full) return simt_full_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
   SPION_FUSED_DISPATCH(fwd_launch, Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, scale, st);
 }
 
@@ -853,8 +855,10 @@ int simt_fused_backward(const float* Q, OperandLayout lq, const float* K, Operan
                         OperandLayout lv, const float* P, ValueLayout vp, const float* O, OperandLayout lo,
                         const float* dO, OperandLayout ldo, float* dS, ValueLayout vds, float* dQ, OperandLayout ldq,
                         float* dK, OperandLayout ldk, float* dV, OperandLayout ldv, Pattern p, int BH, int d,
-                        float scale, cudaStream_t st, spion_ctx* prof) {
+                        float scale, cudaStream_t st, spion_ctx* prof, bool full) {
   if (!simt_fused_supports(p.bs, d, BH, vp.mode) || vds.mode != vp.mode) return SPION_ERR_UNSUPPORTED;
+  if (full && O)
+    return simt_full_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof);
   SPION_FUSED_DISPATCH(bwd_launch, Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH,
                        scale, st, prof);
 }

@@ -199,13 +199,13 @@ class _LinearFn(torch.autograd.Function):
 class BiasGradLinear(nn.Linear):
     """``nn.Linear`` (same parameters, same arithmetic) on the library's linear-layer kernels: conversion of the operands, bias and
     bias gradient happen inside them.  Widths they do not serve (not a multiple of 32) go through the framework's GEMMs, with
-    the bias gradient summed by the library's column-sum kernel."""
+    the bias gradient summed by the library's column-sum kernel; so does every width with ``framework=True``."""
 
-    def forward(self, x):
+    def forward(self, x, framework: bool = False):
         if self.bias is None or not x.is_cuda:
             return super().forward(x)
         amp = torch.is_autocast_enabled()
-        if not amp or torch.get_autocast_dtype("cuda") == torch.bfloat16:
+        if not framework and (not amp or torch.get_autocast_dtype("cuda") == torch.bfloat16):
             if _ops.ops.linear_supported(x, self.weight, self.bias, not amp):
                 return _ops.ops.linear(x, self.weight, self.bias, not amp)
         return _LinearFn.apply(x, self.weight, self.bias)

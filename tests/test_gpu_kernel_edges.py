@@ -75,12 +75,13 @@ def test_streaming_forward_and_backward(d, bs, padded, case):
 # (eight; one CTA per column group); groups of four matrices with one, two and three left over
 @pytest.mark.parametrize("bs,d,B,H,nb", [(32, 32, 1, 1, 1), (32, 64, 1, 3, 7), (64, 32, 1, 1, 2), (64, 64, 2, 1, 9),
                                          (32, 32, 50, 3, 8), (32, 64, 42, 5, 7), (64, 32, 40, 1, 8), (64, 64, 7, 5, 9),
-                                         (32, 32, 301, 3, 8), (64, 64, 119, 3, 5)])
+                                         (32, 32, 301, 3, 8), (64, 64, 119, 3, 5),
+                                         (32, 64, 2, 1, 3), (64, 64, 1, 2, 3), (64, 32, 1, 1, 3)])   # nb 3: the full mask's kernels
 def test_fp32_fused_kernels(bs, d, B, H, nb):
     from spion_b200.native import BlockSparseAttention
     L = nb * bs
     Q, K, V, dO = synthetic.qkv(17 + nb, B, H, L, d)
-    mat = lines_of_every_length(nb, nb > 4)
+    mat = np.ones((3, 3), np.uint8) if nb == 3 else lines_of_every_length(nb, nb > 4)
     kp = synthetic.key_padding(9, B, L) if nb % 2 else None
     mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.float32, keypad=kp is not None)
     compare(run(mod, Q, K, V, dO, mat, kp), Q, K, V, dO, mat, bs, kp, FP32_TOL, False)
