@@ -5,7 +5,7 @@
 // tensor-memory quadrant) and walks block rows of its own, two blocks ("a pair") at a time:
 //     S = Q K_e^T   (M = 64, the second block at lane offset 16: query rows along the lanes, a row owned by lanes l and l + 16)
 //     P = exp2(S scale log2e - m), unnormalised, bf16 into shared memory (over the K tiles when they are as large)
-//     O += P V_e    (M = 64, tensor memory, lane offset 16 x parity of the row)
+//     O += P V_e    (M = 64, tensor memory, lane offset 16 x parity of the row among the rows with blocks)
 // S of pair j + 1 is computed while pair j is in the arithmetic (its 64 values per lane are in registers), and the rows of a
 // finished unit are written after the first pair of the next one.  Nothing is exchanged between the groups: they only fill each
 // other's waits.
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       if (EXACT && end) values = false;
     };
     bool ok = true;
-    int units = 0, jv = 0;                                        // units begun; value pairs before pair j
+    int units = 0, jv = 0;                                        // units with blocks begun; value pairs before pair j
     if (c.valid()) {
       flags_load(ld, pr);
       load_k(0);
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         step_on(ld, ld_val);
         if (ld.valid()) pr = a.pair[ld.cur.y + ld.k];
       }
-      p_cnt = c.cnt(); p_par = c.i & 1; p_first = c.k == 0; p_val = c_val;
+      p_cnt = c.cnt(); p_par = units & 1; p_first = c.k == 0; p_val = c_val;
       step_on(c, c_val);
     }
   } else {
@@ -286,8 +286,11 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
     Walk u;
     u.init(um, a.rec, first, step, total);
     int j = 0;
+    // Units with blocks begun.  Two of them in a row must not share their lanes: the rows of the first are read while the product of
+    // the second is issued.  Rows without blocks have no product and hand nothing over, so they do not count.
+    int units = 0;
     for (; u.valid() && ok; u.shift()) {
-      const int n = u.cur.w, par = u.i & 1;
+      const int n = u.cur.w;
       const OpPos pos = op_pos(u.bh, a.L, a.heads, D);
       __nv_bfloat16* dst = a.O + (size_t)(pos.row0 + u.cur.x * BS + row) * pos.ld + pos.x0;
       float* lse = a.lse + (size_t)u.bh * a.L + u.cur.x * BS + row;
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         write_rows(dst, false, 0.f, hf == 0);
         continue;
       }
+      const int par = ++units & 1;
       const float* kpu = KP ? a.keypad + (size_t)u.bh * a.L : nullptr;
       float m = floor2, mx = floor2, l = 0.f;                     // reference exponent, true maximum, sum
       int n_sel = 0;

@@ -133,3 +133,33 @@ def test_discovery_of_several_layers(layers, L, bs, misaligned):
         cp, ri, pos = ocsr.block_csc(want)
         for got, ref in ((p.row_ptr, rp), (p.col_idx, ci), (p.blk_row, br), (p.col_ptr, cp), (p.row_idx, ri), (p.csc_pos, pos)):
             assert np.array_equal(got.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("d,H", [(64, 2), (32, 4)])
+@pytest.mark.parametrize("full_mask", [False, True])
+def test_streaming_forward_with_rows_without_blocks_between_others(d, H, full_mask):
+    """More matrices than stay in L2, so that the rows are walked matrix by matrix: rows with blocks follow each other directly, after
+    one row without any, and after several.  Every output row against the masked softmax in fp32."""
+    from spion_b200.native import BlockSparseAttention
+    B, nb, bs = 84, 32, 64
+    L = nb * bs
+    assert 2 * B * H * L * d * 2 > 80 << 20
+    mat = np.ones((nb, nb), np.uint8)
+    if not full_mask:
+        rng = np.random.default_rng(d)
+        mat = np.zeros((nb, nb), np.uint8)
+        mat[5] = 1                                           # a long row: the mask is the streaming kernel's
+        for r in rng.permutation(nb)[:nb // 2]:
+            mat[r, rng.choice(nb, size=rng.integers(1, 5), replace=False)] = 1
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v = (torch.randn(B, H, L, d, generator=g, device="cuda").to(torch.bfloat16) for _ in range(3))
+    mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.bfloat16, return_probs=False)
+    with torch.no_grad():
+        out, _ = mod(q, k, v, None, torch.as_tensor(mat).cuda())
+    mod.check_device_status()
+    sel = torch.as_tensor(np.kron(mat, np.ones((bs, bs), np.uint8))).cuda().bool()
+    others = (~sel).sum(1, keepdim=True).float()
+    for b in range(B):
+        e = torch.exp(q[b].float() @ k[b].float().transpose(1, 2) / d ** 0.5) * sel
+        want = (e / (e.sum(-1, keepdim=True) + others)) @ v[b].float()
+        assert far(out[b], want, True) <= BF16_REL, (b, far(out[b], want, True))
