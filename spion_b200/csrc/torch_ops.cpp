@@ -168,6 +168,9 @@ Tensor penalty(const Context& c, const Tensor& mask, const Tensor& like, void* s
 struct Attn {
   Tensor q, k, v, pen, O, lse, P;
   int heads = 0;                        // 0: operands [B, H, L, d] contiguous; H: views of [B, L, H, d]
+  // drop-in sparse calls: the element CSR the forward ran on; the context moves on to another mask's with the next call
+  Tensor sum_mat, offsets, columns;
+  int64_t nnz = 0;
 };
 
 Tensor empty_operand(const Context& c, int heads, const Tensor& like) {
@@ -188,11 +191,12 @@ void attn_forward(const Context& c, Attn& a, bool need, void* st) {
   const auto f32 = a.q.options().dtype(at::kFloat);
   check(spion_set_stream(x, st), "spion_set_stream");
   if (c.mode == DROPIN_SPARSE) {
+    a.sum_mat = c.sum_mat; a.offsets = c.offsets; a.columns = c.columns; a.nnz = c.nnz;
     a.O = empty_operand(c, 0, a.q);
-    a.P = at::empty({c.B * c.H * c.nnz}, f32);
+    a.P = at::empty({c.B * c.H * a.nnz}, f32);
     check(spion_block_attn_forward_rm(x, pf(a.q), pf(a.k), pf(a.v), pf(a.pen), (float*)a.P.data_ptr(), (float*)a.O.data_ptr(),
-                                      (const int*)c.offsets.data_ptr(), (const int*)c.columns.data_ptr(),
-                                      (const int*)c.sum_mat.data_ptr(), (int)c.nnz), "spion_block_attn_forward_rm");
+                                      (const int*)a.offsets.data_ptr(), (const int*)a.columns.data_ptr(),
+                                      (const int*)a.sum_mat.data_ptr(), (int)a.nnz), "spion_block_attn_forward_rm");
     return;
   }
   if (c.mode == DROPIN_DENSE) {
@@ -224,13 +228,13 @@ void attn_backward(const Context& c, const Attn& a, const Tensor& dO, Tensor& dq
   dq = empty_operand(c, a.heads, a.q); dk = empty_operand(c, a.heads, a.q); dv = empty_operand(c, a.heads, a.q);
   check(spion_set_stream(x, st), "spion_set_stream");
   if (c.mode == DROPIN_SPARSE) {
-    Tensor dS = at::empty({c.B * c.H * c.nnz}, f32);
+    Tensor dS = at::empty({c.B * c.H * a.nnz}, f32);
     Tensor dP;
-    if (spion_block_attn_needs_scratch(x)) dP = at::empty({c.B * c.H * c.nnz}, f32);
+    if (spion_block_attn_needs_scratch(x)) dP = at::empty({c.B * c.H * a.nnz}, f32);
     check(spion_block_attn_backward_rm(x, pf(a.q), pf(a.k), pf(a.v), pf(a.P), pf(a.O), pf(dO), (float*)p(dP), (float*)dS.data_ptr(),
                                        (float*)dq.data_ptr(), (float*)dk.data_ptr(), (float*)dv.data_ptr(),
-                                       (const int*)c.offsets.data_ptr(), (const int*)c.columns.data_ptr(),
-                                       (const int*)c.sum_mat.data_ptr(), (int)c.nnz), "spion_block_attn_backward_rm");
+                                       (const int*)a.offsets.data_ptr(), (const int*)a.columns.data_ptr(),
+                                       (const int*)a.sum_mat.data_ptr(), (int)a.nnz), "spion_block_attn_backward_rm");
     return;
   }
   if (c.mode == DROPIN_DENSE) {

@@ -1,0 +1,75 @@
+"""What callers do with the modules between and around the kernels: several masks before a backward, changed outputs, hooks, transforms
+of the framework, copies of modules."""
+import contextlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+B, H, L, D, BS = 2, 2, 256, 32, 64
+KINDS = {"native bf16": (True, "bf16"), "native fp32": (True, "fp32"), "drop-in": (False, "fp32")}
+
+
+def config(native=True, dtype="fp32", task="lra-text", **more):
+    return dict({"head_dim": D, "num_head": H, "max_seq_len": L, "batch_size": B, "block_size": BS, "transformer_dim": H * D,
+                 "task": task, "native": native, "dtype": dtype}, **more)
+
+
+def make_layer(kind, dense=False, task="lra-text", seed=0):
+    from spion_b200.attention import Attention
+    native, dtype = KINDS[kind]
+    torch.manual_seed(seed)
+    cfg = config(native, dtype, task)
+    layer = Attention(cfg).cuda()
+    if not dense:
+        layer.reconstruct_for_blocksparse(cfg)
+    return layer
+
+
+def amp(kind):
+    return torch.autocast("cuda", dtype=torch.bfloat16) if KINDS[kind][1] == "bf16" else contextlib.nullcontext()
+
+
+def make_mask(seed, density=0.5):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    mat = (torch.rand(L // BS, L // BS, generator=g, device="cuda") < density).float()
+    mat.fill_diagonal_(1)
+    return mat
+
+
+def make_inputs(seed=1):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(B, L, H * D, generator=g, device="cuda", requires_grad=True)
+    keys = torch.ones(B, L, device="cuda")
+    keys[1, L // 2:] = 0
+    return x, keys
+
+
+def run_layer(layer, kind, x, keys, mat):
+    with amp(kind):
+        return layer(x, keys, mat)[0]
+
+
+def gradients(layer, out, x):
+    return torch.autograd.grad(out.float().square().sum(), [x] + list(layer.parameters()))
+
+
+def same(a, b):
+    assert len(a) == len(b)
+    for s, t in zip(a, b):
+        assert torch.equal(s, t), float((s - t).abs().max())
+
+
+def test_two_masks_before_the_backward_of_a_drop_in_layer():
+    """Every call's backward runs on the mask of its own forward, whatever the layer was called with since."""
+    kind, masks = "drop-in", (make_mask(1, 0.2), make_mask(2, 0.9))
+    x, keys = make_inputs()
+    want = []
+    for mat in masks:
+        layer = make_layer(kind)
+        want.append(gradients(layer, run_layer(layer, kind, x, keys, mat), x))
+    layer = make_layer(kind)
+    outs = [run_layer(layer, kind, x, keys, mat) for mat in masks]
+    for i in (0, 1):
+        same(gradients(layer, outs[i], x), want[i])
