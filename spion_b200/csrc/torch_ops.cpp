@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "../../include/spion_b200.h"
@@ -123,7 +124,9 @@ bool weights_ok(const std::vector<Tensor>& W, const std::vector<Tensor>& b, cons
 // ------------------------------------------------------------------------------------------------ attention context
 enum Mode { NATIVE = 0, DROPIN_SPARSE = 1, DROPIN_DENSE = 2 };
 
-// What the Python modules keep per attention context: the C ABI's handle and the sizes it was created with.
+// What the Python modules keep per attention context: the C ABI's handle and the sizes it was created with.  The handle has a
+// stream, a head layout and a mask of its own: `mutex` is held from setting them to the last launch that reads them, and never
+// waited for by a thread that holds the interpreter's lock (the holder may need that one).
 struct Context {
   int64_t handle = 0;
   int mode = NATIVE;
@@ -133,6 +136,9 @@ struct Context {
   bool owned = false;                   // destroys the handle
   int64_t nnz = 0;                      // selected elements per (b,h) matrix
   Tensor sum_mat, offsets, columns;     // element CSR of the drop-in layout
+  Tensor mask;                          // native: the block mask [nb, nb] the handle is set to; generation counts the masks
+  int64_t generation = 0;
+  std::mutex mutex;
   spion_ctx* ctx() const { return reinterpret_cast<spion_ctx*>(handle); }
   at::ScalarType type() const { return bf16 ? at::kBFloat16 : at::kFloat; }
   void close() { if (owned && handle) { spion_destroy(ctx()); } handle = 0; }
@@ -145,6 +151,21 @@ std::string shape_str(const Tensor& t) {
   for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
   return s + ")";
 }
+
+// native contexts: a new block mask (uint8 [nb, nb] on the context's device, owned by the caller's module and never changed)
+void set_pattern(const ContextPtr& c, const Tensor& mask, int64_t bs) {
+  py::gil_scoped_release nogil;
+  if (mask.numel() < (c->L / bs) * (c->L / bs))
+    throw Failure("block mask has shape " + shape_str(mask) + ", this module needs " + std::to_string(c->L / bs) + " blocks per side");
+  c10::cuda::CUDAGuard guard(c->device);
+  std::lock_guard<std::mutex> hold(c->mutex);
+  check(spion_set_stream(c->ctx(), (void*)c10::cuda::getCurrentCUDAStream(c->device).stream()), "spion_set_stream");
+  c->mask = mask;
+  ++c->generation;
+  check(spion_set_pattern(c->ctx(), (const uint8_t*)mask.data_ptr()), "spion_set_pattern");
+  c->nnz = (int64_t)spion_pattern_nnzb(c->ctx()) * bs * bs;
+}
+
 void check_operand(const Context& c, const Tensor& t, const char* name) {
   if (t.dim() != 4 || t.size(0) != c.B || t.size(1) != c.H || t.size(2) != c.L || t.size(3) != c.d)
     throw Failure(std::string(name) + " has shape " + shape_str(t) + ", this module was built for (" + std::to_string(c.B) + ", " +
@@ -168,9 +189,9 @@ Tensor penalty(const Context& c, const Tensor& mask, const Tensor& like, void* s
 struct Attn {
   Tensor q, k, v, pen, O, lse, P;
   int heads = 0;                        // 0: operands [B, H, L, d] contiguous; H: views of [B, L, H, d]
-  // drop-in sparse calls: the element CSR the forward ran on; the context moves on to another mask's with the next call
-  Tensor sum_mat, offsets, columns;
-  int64_t nnz = 0;
+  // the mask the forward ran on (drop-in: as element CSR); the context may move on to another before the backward
+  Tensor sum_mat, offsets, columns, mask;
+  int64_t nnz = 0, generation = 0;
 };
 
 Tensor empty_operand(const Context& c, int heads, const Tensor& like) {
@@ -186,12 +207,14 @@ int operand_form(const Context& c, const Tensor& t) {
 }
 
 // need: a backward may follow
-void attn_forward(const Context& c, Attn& a, bool need, void* st) {
+void attn_forward(Context& c, Attn& a, bool need, void* st) {
   spion_ctx* x = c.ctx();
   const auto f32 = a.q.options().dtype(at::kFloat);
+  std::lock_guard<std::mutex> hold(c.mutex);
+  a.nnz = c.nnz;
   check(spion_set_stream(x, st), "spion_set_stream");
   if (c.mode == DROPIN_SPARSE) {
-    a.sum_mat = c.sum_mat; a.offsets = c.offsets; a.columns = c.columns; a.nnz = c.nnz;
+    a.sum_mat = c.sum_mat; a.offsets = c.offsets; a.columns = c.columns;
     a.O = empty_operand(c, 0, a.q);
     a.P = at::empty({c.B * c.H * a.nnz}, f32);
     check(spion_block_attn_forward_rm(x, pf(a.q), pf(a.k), pf(a.v), pf(a.pen), (float*)a.P.data_ptr(), (float*)a.O.data_ptr(),
@@ -206,27 +229,49 @@ void attn_forward(const Context& c, Attn& a, bool need, void* st) {
           "spion_dense_attn_forward_rm");
     return;
   }
+  a.mask = c.mask; a.generation = c.generation;
   check(spion_set_head_layout(x, a.heads), "spion_set_head_layout");
   a.O = empty_operand(c, a.heads, a.q);
   if (c.fused) {
     a.lse = at::empty({c.B * c.H * c.L}, f32);
     // the probabilities are stored only for callers that want them back and for a backward that reads them
-    if (c.return_probs || (need && !c.recompute)) a.P = at::empty({c.B * c.H * c.nnz}, a.q.options());
+    if (c.return_probs || (need && !c.recompute)) a.P = at::empty({c.B * c.H * a.nnz}, a.q.options());
     check(spion_attn_forward_fused(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.O), (float*)a.lse.data_ptr(), p(a.P)),
           "spion_attn_forward_fused");
   } else {
-    a.P = at::empty({c.B * c.H * c.nnz}, a.q.options());
+    a.P = at::empty({c.B * c.H * a.nnz}, a.q.options());
     Tensor scratch;
-    if (c.needs_scratch) scratch = at::empty({c.B * c.H * c.nnz}, f32);
+    if (c.needs_scratch) scratch = at::empty({c.B * c.H * a.nnz}, f32);
     check(spion_attn_forward_ex(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.P), p(a.O), (float*)p(scratch)), "spion_attn_forward_ex");
   }
 }
 
-void attn_backward(const Context& c, const Attn& a, const Tensor& dO, Tensor& dq, Tensor& dk, Tensor& dv, void* st) {
+// Runs f with the handle set to the forward's mask.  A module that has been given another mask since takes it back afterwards; both
+// read the mask's size back, so such a backward cannot be captured.
+template <class F>
+void on_mask_of(const Context& c, const Attn& a, F f) {
+  if (c.mode != NATIVE || a.generation == c.generation) return f();
+  check(spion_set_pattern(c.ctx(), (const uint8_t*)a.mask.data_ptr()), "spion_set_pattern");
+  try {
+    f();
+  } catch (...) {
+    spion_set_pattern(c.ctx(), (const uint8_t*)c.mask.data_ptr());
+    throw;
+  }
+  check(spion_set_pattern(c.ctx(), (const uint8_t*)c.mask.data_ptr()), "spion_set_pattern");
+}
+
+void attn_backward_on(const Context& c, const Attn& a, const Tensor& dO, Tensor& dq, Tensor& dk, Tensor& dv);
+void attn_backward(Context& c, const Attn& a, const Tensor& dO, Tensor& dq, Tensor& dk, Tensor& dv, void* st) {
+  std::lock_guard<std::mutex> hold(c.mutex);
+  check(spion_set_stream(c.ctx(), st), "spion_set_stream");
+  on_mask_of(c, a, [&] { attn_backward_on(c, a, dO, dq, dk, dv); });
+}
+
+void attn_backward_on(const Context& c, const Attn& a, const Tensor& dO, Tensor& dq, Tensor& dk, Tensor& dv) {
   spion_ctx* x = c.ctx();
   const auto f32 = a.q.options().dtype(at::kFloat);
   dq = empty_operand(c, a.heads, a.q); dk = empty_operand(c, a.heads, a.q); dv = empty_operand(c, a.heads, a.q);
-  check(spion_set_stream(x, st), "spion_set_stream");
   if (c.mode == DROPIN_SPARSE) {
     Tensor dS = at::empty({c.B * c.H * a.nnz}, f32);
     Tensor dP;
@@ -252,8 +297,8 @@ void attn_backward(const Context& c, const Attn& a, const Tensor& dO, Tensor& dq
           "spion_attn_backward_fused");
     return;
   }
-  Tensor dS = at::empty({c.B * c.H * c.nnz}, a.q.options()), scratch;
-  if (!c.fused && c.needs_scratch) scratch = at::empty({c.B * c.H * c.nnz}, f32);
+  Tensor dS = at::empty({c.B * c.H * a.nnz}, a.q.options()), scratch;
+  if (!c.fused && c.needs_scratch) scratch = at::empty({c.B * c.H * a.nnz}, f32);
   check(spion_attn_backward_ex(x, p(a.q), p(a.k), p(a.v), p(a.P), p(a.O), p(dO), p(dS), (float*)p(scratch), nullptr, p(dq), p(dk), p(dv)),
         "spion_attn_backward_ex");
 }
@@ -295,8 +340,24 @@ struct AttnNode : public Node {
   }
 };
 
-// attention(q, k, v) -> out, probs (undefined when none were stored), lse, pen, q used, k used, heads
-py::tuple attention(const ContextPtr& c, const Tensor& query, const Tensor& key, const Tensor& value, const optional<Tensor>& mask) {
+struct Result {
+  Tensor out;
+  Attn a;
+};
+// out, probs (None when none were stored), lse, pen, q used, k used, heads; f runs without the interpreter's lock
+template <class F>
+py::tuple as_tuple(F f) {
+  Result r;
+  {
+    py::gil_scoped_release nogil;
+    r = f();
+  }
+  auto or_none = [](const Tensor& t) -> py::object { return t.defined() ? py::cast(t) : py::none(); };
+  return py::make_tuple(r.out, or_none(r.a.P), or_none(r.a.lse), or_none(r.a.pen), r.a.q, r.a.k, r.a.heads);
+}
+
+// attention(q, k, v)
+Result attention(const ContextPtr& c, const Tensor& query, const Tensor& key, const Tensor& value, const optional<Tensor>& mask) {
   check_operand(*c, query, "query");
   check_operand(*c, key, "key");
   check_operand(*c, value, "value");
@@ -332,8 +393,7 @@ py::tuple attention(const ContextPtr& c, const Tensor& query, const Tensor& key,
     node->a.O = a.O;
     torch::autograd::set_history(out, node);
   }
-  return py::make_tuple(out, a.P.defined() ? py::cast(a.P) : py::none(), a.lse.defined() ? py::cast(a.lse) : py::none(),
-                        a.pen.defined() ? py::cast(a.pen) : py::none(), a.q, a.k, a.heads);
+  return Result{out, a};
 }
 
 // A whole multi-head attention layer: x [B, L, dim] -> projections -> attention -> output projection [B, L, dim_out].
@@ -410,8 +470,7 @@ bool layer_supported(const ContextPtr& c, const Tensor& x, const std::vector<Ten
   return weights_ok({W[0], W[1], W[2]}, {b[0], b[1], b[2]}, x, fp32) && weights_ok({W[3]}, {b[3]}, x, fp32);
 }
 
-// -> out, P (or None), lse, pen, q, k, heads
-py::tuple attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tensor>& mask, const std::vector<Tensor>& W,
+Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tensor>& mask, const std::vector<Tensor>& W,
                           const std::vector<Tensor>& b, bool fp32) {
   c10::cuda::CUDAGuard guard(c->device);
   void* st = stream_of(x);
@@ -450,8 +509,7 @@ py::tuple attention_layer(const ContextPtr& c, const Tensor& x, const optional<T
     for (int i = 0; i < 4; ++i) node->w[i] = save(W[i]);
     torch::autograd::set_history(out, node);
   }
-  return py::make_tuple(out, a.P.defined() ? py::cast(a.P) : py::none(), a.lse.defined() ? py::cast(a.lse) : py::none(),
-                        a.pen.defined() ? py::cast(a.pen) : py::none(), a.q, a.k, a.heads);
+  return Result{out, a};
 }
 
 // ------------------------------------------------------------------------------------------------ linear layers on their own
@@ -604,6 +662,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<Context, ContextPtr>(m, "Context")
       .def(py::init<>())
       .def("close", &Context::close)
+      .def("set_pattern", &set_pattern)
       .def_readwrite("handle", &Context::handle)
       .def_readwrite("mode", &Context::mode)
       .def_readwrite("B", &Context::B).def_readwrite("H", &Context::H).def_readwrite("L", &Context::L).def_readwrite("d", &Context::d)
@@ -613,9 +672,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("needs_scratch", &Context::needs_scratch).def_readwrite("owned", &Context::owned)
       .def_readwrite("nnz", &Context::nnz)
       .def_readwrite("sum_mat", &Context::sum_mat).def_readwrite("offsets", &Context::offsets).def_readwrite("columns", &Context::columns);
-  m.def("attention", &attention);
+  m.def("attention", [](const ContextPtr& c, const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& mask) {
+    return as_tuple([&] { return attention(c, q, k, v, mask); });
+  });
   m.def("layer_supported", &layer_supported);
-  m.def("attention_layer", &attention_layer);
+  m.def("attention_layer", [](const ContextPtr& c, const Tensor& x, const optional<Tensor>& mask, const std::vector<Tensor>& W,
+                              const std::vector<Tensor>& b, bool fp32) {
+    return as_tuple([&] { return attention_layer(c, x, mask, W, b, fp32); });
+  });
   m.def("linear_supported", &linear_supported);
   m.def("linear", &linear);
   m.def("mlp", &mlp);

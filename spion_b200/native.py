@@ -111,8 +111,7 @@ class BlockSparseAttention(nn.Module):
         """Fix the layer's block mask ([nb, nb], non-zero = selected).  Called once per layer at the
         dense->sparse switch, where the reference calls reconstruct_for_blocksparse."""
         m8 = (mat != 0).to(torch.uint8).contiguous().to(self.device)
-        check(lib.spion_set_stream(self.handle, _lib.current_stream_ptr()))
-        check(lib.spion_set_pattern(self.handle, ptr(m8)), "spion_set_pattern")
+        self._ctx.set_pattern(m8, self.bs)
         self.nnzb = int(lib.spion_pattern_nnzb(self.handle))
         if self.fused and self._recompute_arg is None:
             self.recompute = self._recompute_pays()
@@ -122,7 +121,6 @@ class BlockSparseAttention(nn.Module):
         # address cannot be handed to another mask while the key is in use.
         self._mask_key = (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device))
         self._mask_ref, self._mask_version = mat, mat._version
-        self._ctx.nnz = self.nnz
         return self.nnzb
 
     def _recompute_pays(self) -> bool:

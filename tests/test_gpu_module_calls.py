@@ -73,3 +73,25 @@ def test_two_masks_before_the_backward_of_a_drop_in_layer():
     outs = [run_layer(layer, kind, x, keys, mat) for mat in masks]
     for i in (0, 1):
         same(gradients(layer, outs[i], x), want[i])
+
+
+@pytest.mark.parametrize("bs", [64, 32])
+@pytest.mark.parametrize("dtype,recompute", [(torch.bfloat16, True), (torch.bfloat16, False), (torch.float32, None)])
+def test_two_masks_before_the_backward_of_a_native_module(dtype, recompute, bs):
+    from spion_b200.native import BlockSparseAttention
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(B, H, L, D, generator=g, device="cuda").to(dtype).requires_grad_() for _ in range(3))
+    masks = [(torch.rand(L // bs, L // bs, generator=g, device="cuda") < p).float() + torch.eye(L // bs, device="cuda") for p in (0.2, 0.8)]
+
+    def module():
+        return BlockSparseAttention(dict(config(), block_size=bs), dtype=dtype, recompute=recompute)
+
+    def grads(out):
+        return torch.autograd.grad(out.float().square().sum(), (q, k, v))
+
+    want = [grads(module()(q, k, v, None, mat)[0]) for mat in masks]
+    mod = module()
+    outs = [mod(q, k, v, None, mat)[0] for mat in masks]
+    same(grads(outs[0]), want[0])
+    assert torch.equal(mod(q, k, v)[0], outs[1])                 # the module is on its last mask again
+    same(grads(outs[1]), want[1])
