@@ -306,18 +306,47 @@ void attn_backward_on(const Context& c, const Attn& a, const Tensor& dO, Tensor&
 // ------------------------------------------------------------------------------------------------ autograd nodes
 SavedVariable save(const Tensor& t) { return SavedVariable(t, false); }
 
+// What a backward reads of its forward, as saved variables: a tensor that a caller also holds (the output, the probabilities) is
+// checked for changes since, and hooks on saved tensors see all of them.
+struct SavedAttn {
+  SavedVariable q, k, v, pen, O, lse, P, sum_mat, offsets, columns;
+  Attn rest;
+  // q_in, k_in, v_in: the caller's tensors where the kernels read them in place, else what a holds
+  void save_all(const Attn& a, const Tensor& q_in, const Tensor& k_in, const Tensor& v_in) {
+    q = save(q_in); k = save(k_in); v = save(v_in);
+    pen = save(a.pen); O = save(a.O); lse = save(a.lse); P = save(a.P);
+    sum_mat = save(a.sum_mat); offsets = save(a.offsets); columns = save(a.columns);
+    rest.heads = a.heads; rest.mask = a.mask; rest.nnz = a.nnz; rest.generation = a.generation;
+  }
+  Attn unpack(const Context& c) const {
+    Attn a = rest;
+    // a hook may hand a tensor back in other strides
+    auto operand = [&](const SavedVariable& s) {
+      Tensor t = s.unpack();
+      if (!a.heads) return t.contiguous();
+      return operand_form(c, t) == a.heads ? t : t.transpose(1, 2).contiguous().transpose(1, 2);
+    };
+    auto values = [](const SavedVariable& s) { Tensor t = s.unpack(); return t.defined() ? t.contiguous() : t; };
+    a.q = operand(q); a.k = operand(k); a.v = operand(v); a.O = operand(O);
+    a.pen = values(pen); a.lse = values(lse); a.P = values(P);
+    a.sum_mat = values(sum_mat); a.offsets = values(offsets); a.columns = values(columns);
+    return a;
+  }
+  void reset() {
+    for (SavedVariable* s : {&q, &k, &v, &pen, &O, &lse, &P, &sum_mat, &offsets, &columns}) s->reset_data();
+    rest = Attn();
+  }
+};
+
 struct AttnNode : public Node {
   ContextPtr c;
-  Attn a;                                // q, k, v hold what the kernels read (copies where a cast or a packing was needed)
-  SavedVariable sq, sk, sv;              // the inputs themselves, where the kernels read them in place
-  bool iq = false, ik = false, iv = false;
+  SavedAttn saved;
   at::ScalarType tq, tk, tv;
   bool released = false;
   std::string name() const override { return "BlockSparseAttentionBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    sq.reset_data(); sk.reset_data(); sv.reset_data();
-    a = Attn();
+    saved.reset();
     released = true;
   }
   variable_list apply(variable_list&& grads) override {
@@ -326,10 +355,7 @@ struct AttnNode : public Node {
     variable_list out(3);
     if (!grads[0].defined()) return out;
     c10::cuda::CUDAGuard guard(c->device);
-    Attn s = a;
-    if (iq) s.q = sq.unpack();
-    if (ik) s.k = sk.unpack();
-    if (iv) s.v = sv.unpack();
+    const Attn s = saved.unpack(*c);
     Tensor go = grads[0].to(c->type());
     if (s.heads && operand_form(*c, go) != s.heads) go = go.transpose(1, 2).contiguous().transpose(1, 2);
     else if (!s.heads) go = go.contiguous();
@@ -379,18 +405,12 @@ Result attention(const ContextPtr& c, const Tensor& query, const Tensor& key, co
     auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(query, key, value));
     node->c = c;
-    node->a = a;
-    if (c->fused && c->recompute) node->a.P = Tensor();
     node->tq = query.scalar_type(); node->tk = key.scalar_type(); node->tv = value.scalar_type();
-    node->iq = a.q.is_same(query) || a.q.data_ptr() == query.data_ptr();
-    node->ik = a.k.data_ptr() == key.data_ptr();
-    node->iv = a.v.data_ptr() == value.data_ptr();
-    if (node->iq) { node->sq = save(query); node->a.q = Tensor(); }
-    if (node->ik) { node->sk = save(key); node->a.k = Tensor(); }
-    if (node->iv) { node->sv = save(value); node->a.v = Tensor(); }
-    if (node->iq) node->a.q = Tensor();
-    out = a.O.detach();
-    node->a.O = a.O;
+    Attn kept = a;
+    if (c->fused && c->recompute) kept.P = Tensor();
+    auto in_place = [](const Tensor& in, const Tensor& used) { return used.data_ptr() == in.data_ptr() ? in : used; };
+    node->saved.save_all(kept, in_place(query, a.q), in_place(key, a.k), in_place(value, a.v));
+    out = a.O.detach();                  // shares the version counter of what was saved
     torch::autograd::set_history(out, node);
   }
   return Result{out, a};
@@ -400,7 +420,7 @@ Result attention(const ContextPtr& c, const Tensor& query, const Tensor& key, co
 struct LayerNode : public Node {
   ContextPtr c;
   bool fp32 = false;
-  Attn a;
+  SavedAttn saved;
   SavedVariable x, w[4];                 // Wq, Wk, Wv, Wf
   at::ScalarType out_type;
   bool released = false;
@@ -409,7 +429,7 @@ struct LayerNode : public Node {
     std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data();
     for (auto& s : w) s.reset_data();
-    a = Attn();
+    saved.reset();
     released = true;
   }
   // inputs: x, Wq, bq, Wk, bk, Wv, bv, Wf, bf
@@ -421,6 +441,7 @@ struct LayerNode : public Node {
     c10::cuda::CUDAGuard guard(c->device);
     const int H = (int)c->H, d = (int)c->d, L = (int)c->L;
     const int64_t T = c->B * c->L;
+    const Attn a = saved.unpack(*c);
     Tensor X = x.unpack();
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
     const int dim = (int)X.size(2);
@@ -503,8 +524,10 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
   if (need) {
     auto node = std::shared_ptr<LayerNode>(new LayerNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x, W[0], b[0], W[1], b[1], W[2], b[2], W[3], b[3]));
-    node->c = c; node->fp32 = fp32; node->a = a; node->out_type = out.scalar_type();
-    if (c->mode == NATIVE && c->fused && c->recompute) node->a.P = Tensor();
+    node->c = c; node->fp32 = fp32; node->out_type = out.scalar_type();
+    Attn kept = a;
+    if (c->mode == NATIVE && c->fused && c->recompute) kept.P = Tensor();
+    node->saved.save_all(kept, a.q, a.k, a.v);
     node->x = save(x);
     for (int i = 0; i < 4; ++i) node->w[i] = save(W[i]);
     torch::autograd::set_history(out, node);
@@ -576,14 +599,12 @@ Tensor linear(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
 
 // Feed-forward block Linear -> GELU -> Linear under mixed precision, the activation inside the first product's kernel.
 struct MlpNode : public Node {
-  SavedVariable x, w1, w2;
-  Tensor h, g;                           // pre-activation and activation, bf16
+  SavedVariable x, w1, w2, h_s, g_s;     // h_s, g_s: pre-activation and activation, bf16
   bool released = false;
   std::string name() const override { return "FeedForwardBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    x.reset_data(); w1.reset_data(); w2.reset_data();
-    h = Tensor(); g = Tensor();
+    for (SavedVariable* s : {&x, &w1, &w2, &h_s, &g_s}) s->reset_data();
     released = true;
   }
   // inputs: x, W1, b1, W2, b2
@@ -595,6 +616,7 @@ struct MlpNode : public Node {
     Tensor X = x.unpack();
     c10::cuda::CUDAGuard guard(X.device());
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    const Tensor h = h_s.unpack().contiguous(), g = g_s.unpack().contiguous();
     Weights l1, l2;
     l1.W.push_back(w1.unpack()); l2.W.push_back(w2.unpack());
     Tensor go = grads[0].to(at::kBFloat16).contiguous();
@@ -642,7 +664,7 @@ Tensor mlp(const Tensor& x, const Tensor& W1, const Tensor& b1, const Tensor& W2
     auto node = std::shared_ptr<MlpNode>(new MlpNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x, W1, b1, W2, b2));
     node->x = save(x); node->w1 = save(W1); node->w2 = save(W2);
-    node->h = h; node->g = g;
+    node->h_s = save(h); node->g_s = save(g);
     torch::autograd::set_history(out, node);
   }
   return out;

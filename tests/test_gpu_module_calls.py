@@ -95,3 +95,49 @@ def test_two_masks_before_the_backward_of_a_native_module(dtype, recompute, bs):
     same(grads(outs[0]), want[0])
     assert torch.equal(mod(q, k, v)[0], outs[1])                 # the module is on its last mask again
     same(grads(outs[1]), want[1])
+
+
+@pytest.mark.parametrize("dtype,recompute", [(torch.bfloat16, True), (torch.bfloat16, False), (torch.float32, None)])
+@pytest.mark.parametrize("what", ["output", "probabilities"])
+def test_a_changed_output_is_noticed(dtype, recompute, what):
+    """The backward reads the output (and, where they are stored, the probabilities): a change in between is an error."""
+    from spion_b200.native import BlockSparseAttention
+    if what == "probabilities" and recompute:
+        pytest.skip("the rebuilt path does not read them")
+    q, k, v = (torch.randn(B, H, L, D, device="cuda").to(dtype).requires_grad_() for _ in range(3))
+    mod = BlockSparseAttention(config(), dtype=dtype, recompute=recompute)
+    out, probs = mod(q, k, v, None, make_mask(4))
+    total = out.float().sum()
+    if what == "output":
+        out.mul_(2.0)
+        total = out.float().sum()
+    else:
+        probs.mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        total.backward()
+
+
+def test_changed_probabilities_of_a_drop_in_layer_are_noticed():
+    layer, (x, keys) = make_layer("drop-in", task="lra-image"), make_inputs()
+    out, probs = layer(x, keys, make_mask(4))
+    probs.mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.sum().backward()
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_hooks_on_saved_tensors_see_all_of_them(kind):
+    """Saved tensors may be packed elsewhere, in other strides, and rebuilt: same gradients."""
+    from torch.utils.checkpoint import checkpoint
+    x, keys = make_inputs()
+    layer, mat = make_layer(kind), make_mask(5)
+    xb = x.detach().to(torch.bfloat16).requires_grad_() if KINDS[kind][1] == "bf16" else x
+    for inp in (x, xb):                                          # bf16 input: operands in the other layout
+        want = gradients(layer, run_layer(layer, kind, inp, keys, mat), inp)
+        sizes = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: (sizes.append(t.numel()), t.cpu().contiguous())[1], lambda t: t.cuda()):
+            out = run_layer(layer, kind, inp, keys, mat)
+        same(gradients(layer, out, inp), want)
+        assert sum(sizes) >= 5 * B * L * H * D                   # input, Q, K, V, O
+        again = checkpoint(lambda t: run_layer(layer, kind, t, keys, mat), inp, use_reentrant=False)
+        same(gradients(layer, again, inp), want)
