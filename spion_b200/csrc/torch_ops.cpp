@@ -10,6 +10,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/Exceptions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -31,6 +32,25 @@ struct Failure : std::runtime_error { using std::runtime_error::runtime_error; }
 
 void check(int rc, const char* what) {
   if (rc != 0) throw Failure(std::string(what) + " failed: " + spion_status_string(rc) + " (" + std::to_string(rc) + ")");
+}
+
+py::object& error_type() {
+  static py::object* type = new py::object(py::module_::import("spion_b200._lib").attr("SpionError"));      // never destroyed
+  return *type;
+}
+// A backward runs on a thread of the autograd engine, which turns C++ exceptions into RuntimeError: raise the library's own
+// error there, as the forward does through the module's exception translator.
+template <class F>
+variable_list as_backward(F f) {
+  try {
+    return f();
+  } catch (const Failure& e) {
+    py::gil_scoped_acquire gil;
+    PyErr_SetString(error_type().ptr(), e.what());
+    python_error raised;
+    raised.persist();
+    throw raised;
+  }
 }
 
 void* stream_of(const Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
@@ -350,6 +370,9 @@ struct AttnNode : public Node {
     released = true;
   }
   variable_list apply(variable_list&& grads) override {
+    return as_backward([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
     std::lock_guard<std::mutex> lock(mutex_);
     TORCH_CHECK(!released, "Trying to backward through the graph a second time (the saved tensors have been freed)");
     variable_list out(3);
@@ -434,6 +457,9 @@ struct LayerNode : public Node {
   }
   // inputs: x, Wq, bq, Wk, bk, Wv, bv, Wf, bf
   variable_list apply(variable_list&& grads) override {
+    return as_backward([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
     std::lock_guard<std::mutex> lock(mutex_);
     TORCH_CHECK(!released, "Trying to backward through the graph a second time (the saved tensors have been freed)");
     variable_list out(9);
@@ -543,6 +569,9 @@ struct LinearNode : public Node {
   std::string name() const override { return "TokenLinearBackward"; }
   void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); x.reset_data(); w.reset_data(); }
   variable_list apply(variable_list&& grads) override {
+    return as_backward([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list out(3);
     if (!grads[0].defined()) return out;
@@ -609,6 +638,9 @@ struct MlpNode : public Node {
   }
   // inputs: x, W1, b1, W2, b2
   variable_list apply(variable_list&& grads) override {
+    return as_backward([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
     std::lock_guard<std::mutex> lock(mutex_);
     TORCH_CHECK(!released, "Trying to backward through the graph a second time (the saved tensors have been freed)");
     variable_list out(5);
@@ -673,12 +705,12 @@ Tensor mlp(const Tensor& x, const Tensor& W1, const Tensor& b1, const Tensor& W2
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  static py::object error = py::module_::import("spion_b200._lib").attr("SpionError");
+  error_type();
   py::register_local_exception_translator([](std::exception_ptr e) {
     try {
       if (e) std::rethrow_exception(e);
     } catch (const Failure& f) {
-      PyErr_SetString(error.ptr(), f.what());
+      PyErr_SetString(error_type().ptr(), f.what());
     }
   });
   py::class_<Context, ContextPtr>(m, "Context")

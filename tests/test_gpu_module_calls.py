@@ -141,3 +141,19 @@ def test_hooks_on_saved_tensors_see_all_of_them(kind):
         assert sum(sizes) >= 5 * B * L * H * D                   # input, Q, K, V, O
         again = checkpoint(lambda t: run_layer(layer, kind, t, keys, mat), inp, use_reentrant=False)
         same(gradients(layer, again, inp), want)
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_a_failing_backward_raises_the_library_s_error(kind):
+    from spion_b200._lib import SpionError
+    x, keys = make_inputs()
+    layer, mat = make_layer(kind), make_mask(6)
+    out = run_layer(layer, kind, x, keys, mat)
+    block = layer.block_attn
+    ctx = block._ctx if KINDS[kind][0] else block.context(mat)
+    handle, ctx.handle = ctx.handle, 0                            # every call of the library refuses it
+    try:
+        with pytest.raises(SpionError, match="failed"):
+            out.sum().backward()
+    finally:
+        ctx.handle = handle
