@@ -143,11 +143,14 @@ class Attention(nn.Module):
             if mat is None and self.native:
                 attn_out, attn = self.attn(Q, K, V, mask.float())
                 attn_out = attn_out.to(X.dtype)
-            elif mat is None and type(self.attn) is self._dense_type:
-                attn_out, P = _ops.ops.attention(self._dense_ctx, Q.float(), K.float(), V.float(), mask if self.with_keypad else None)[:2]
-                attn = P.permute(0, 1, 3, 2)
             elif mat is None:
-                attn_out, attn = self.attn(Q.float(), K.float(), V.float(), mask.float())
+                call = None
+                if type(self.attn) is self._dense_type:
+                    call = _ops.ops.attention(self._dense_ctx, Q.float(), K.float(), V.float(), mask if self.with_keypad else None)
+                if call is not None:
+                    attn_out, attn = call[0], call[1].permute(0, 1, 3, 2)
+                else:
+                    attn_out, attn = self.attn(Q.float(), K.float(), V.float(), mask.float())
             elif self.native:
                 attn_out, attn = self.block_attn(Q, K, V, mask.float(), mat)
                 attn_out = attn_out.to(X.dtype)

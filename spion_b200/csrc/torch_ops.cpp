@@ -9,6 +9,8 @@
 #include <torch/extension.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/Exceptions.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -56,6 +58,22 @@ variable_list as_backward(F f) {
 void* stream_of(const Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 void* p(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 const float* pf(const Tensor& t) { return t.defined() ? (const float*)t.data_ptr() : nullptr; }
+
+// The nodes below work on memory: they form no forward-mode tangents, and tracers, dispatch modes and transforms would not see what
+// they do.  Calls under one of those take the way over torch operators and Python autograd functions, which they know.
+bool plain(const Tensor& t) {
+  static const c10::DispatchKeySet wrapped({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::FuncTorchGradWrapper,
+                                            c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::Functionalize, c10::DispatchKey::Negative,
+                                            c10::DispatchKey::ZeroTensor});
+  return !t.key_set().has_any(wrapped) && !t._fw_grad(0).defined();
+}
+bool plain(std::initializer_list<at::ArrayRef<Tensor>> lists) {
+  if (torch::jit::tracer::isTracing() || c10::impl::TorchDispatchModeTLS::any_modes_set()) return false;
+  for (const auto& ts : lists)
+    for (const Tensor& t : ts)
+      if (!plain(t)) return false;
+  return true;
+}
 
 // ------------------------------------------------------------------------------------------------ token matrices
 spion_tokens tok(const std::vector<Tensor>& ts, int cols) {
@@ -509,7 +527,7 @@ struct LayerNode : public Node {
 
 // Can the layer run as one node?  fp32: everything in fp32; else bf16 operands (mixed precision).
 bool layer_supported(const ContextPtr& c, const Tensor& x, const std::vector<Tensor>& W, const std::vector<Tensor>& b, bool fp32) {
-  if (c->bf16 == fp32) return false;
+  if (c->bf16 == fp32 || !plain({x, W, b})) return false;
   if (!x.is_cuda() || x.device().index() != c->device || x.dim() != 3 || x.size(0) != c->B || x.size(1) != c->L) return false;
   if (x.scalar_type() != at::kFloat && (fp32 || x.scalar_type() != at::kBFloat16)) return false;
   if ((c->d & (c->d - 1)) || c->d < 32 || x.size(2) != W[0].size(1) || W[3].size(1) != c->H * c->d || W[0].size(0) != c->H * c->d) return false;
@@ -598,7 +616,7 @@ struct LinearNode : public Node {
 };
 
 bool linear_supported(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
-  if (!x.is_cuda() || x.numel() == 0 || x.dim() < 2 || x.size(-1) != W.size(1)) return false;
+  if (!x.is_cuda() || !plain({x, W, b}) || x.numel() == 0 || x.dim() < 2 || x.size(-1) != W.size(1)) return false;
   if (x.scalar_type() != at::kFloat && (fp32 || x.scalar_type() != at::kBFloat16)) return false;
   return x.numel() / W.size(1) < 0x7fffff00LL && weights_ok({W}, {b}, x, fp32);
 }
@@ -726,9 +744,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("needs_scratch", &Context::needs_scratch).def_readwrite("owned", &Context::owned)
       .def_readwrite("nnz", &Context::nnz)
       .def_readwrite("sum_mat", &Context::sum_mat).def_readwrite("offsets", &Context::offsets).def_readwrite("columns", &Context::columns);
-  m.def("attention", [](const ContextPtr& c, const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& mask) {
+  // None, unless `inside` (an autograd function that stands for the call), where something wants to see the call (plain())
+  m.def("attention", [](const ContextPtr& c, const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& mask, bool inside) -> py::object {
+    if (!inside && !plain({q, k, v})) return py::none();
     return as_tuple([&] { return attention(c, q, k, v, mask); });
-  });
+  }, py::arg("context"), py::arg("query"), py::arg("key"), py::arg("value"), py::arg("mask"), py::arg("inside") = false);
   m.def("layer_supported", &layer_supported);
   m.def("attention_layer", [](const ContextPtr& c, const Tensor& x, const optional<Tensor>& mask, const std::vector<Tensor>& W,
                               const std::vector<Tensor>& b, bool fp32) {

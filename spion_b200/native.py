@@ -221,7 +221,7 @@ class BlockSparseAttention(nn.Module):
         # The kernels take sizes from the context, not from the tensors: the call refuses any other shape, device or key-padding
         # mask with a SpionError (a short last batch would otherwise read and write past the buffers).
         self.use_mask(mat)
-        return self.result(*_ops.ops.attention(self._ctx, query, key, value, mask if self.keypad else None))
+        return self.result(*_ops.attention(self._ctx, query, key, value, mask if self.keypad else None))
 
 
 class DenseViaBlocks(nn.Module):

@@ -157,3 +157,61 @@ def test_a_failing_backward_raises_the_library_s_error(kind):
             out.sum().backward()
     finally:
         ctx.handle = handle
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_transforms_of_the_framework(kind, dense):
+    """Tracing records the call; forward-mode tangents, which nothing here forms, are refused and not dropped."""
+    import torch.autograd.forward_ad as fw
+    x, keys = make_inputs()
+    layer, mat = make_layer(kind, dense), None if dense else make_mask(7)
+
+    class Call(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.layer = layer
+
+        def forward(self, t):
+            return run_layer(layer, kind, t, keys, mat)
+
+    call = Call()
+    with torch.no_grad():
+        traced = torch.jit.trace(call, (x,), check_trace=False)
+        other = torch.randn_like(x)
+        got, want = traced(other).float(), call(other).float()
+    # stage by stage instead of one node: other roundings of the same products
+    assert float((got - want).norm() / want.norm()) < (2e-2 if KINDS[kind][1] == "bf16" else 1e-5)
+    with fw.dual_level(), pytest.raises(NotImplementedError):
+        call(fw.make_dual(x.detach(), torch.ones_like(x)))
+    assert not torch.isnan(call(x)).any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_transforms_of_an_attention_call(dtype):
+    import torch.autograd.forward_ad as fw
+    from spion_b200.native import BlockSparseAttention
+    q, k, v = (torch.randn(B, H, L, D, device="cuda").to(dtype).requires_grad_() for _ in range(3))
+    mod = BlockSparseAttention(config(), dtype=dtype)
+    mod.set_mask(make_mask(8))
+    call = lambda *t: mod(*t)[0]
+    traced = torch.jit.trace(call, (q, k, v), check_trace=False)
+    other = torch.randn_like(q).requires_grad_()
+    got, want = (torch.autograd.grad(f(other, k, v).float().square().sum(), (other, k, v)) for f in (traced, call))
+    same(got, want)
+    with fw.dual_level(), pytest.raises(NotImplementedError):
+        call(fw.make_dual(q.detach(), torch.ones_like(q)), k, v)
+
+
+def test_transforms_of_a_linear_layer():
+    import torch.autograd.forward_ad as fw
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from spion_b200.layernorm import BiasGradLinear
+    lin, x, other = BiasGradLinear(64, 128).cuda(), torch.randn(50, 64, device="cuda"), torch.randn(50, 64, device="cuda")
+    want = lin(other)
+    for f in (torch.jit.trace(lin, (x,), check_trace=False), make_fx(lambda t: lin(t))(x)):
+        assert float((f(other) - want).norm() / want.norm()) < 1e-5
+    with fw.dual_level(), pytest.raises(NotImplementedError):
+        lin(fw.make_dual(x, torch.ones_like(x)))
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lin)(x[None].expand(3, -1, -1))
