@@ -16,6 +16,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -376,6 +377,11 @@ struct SavedAttn {
   }
 };
 
+// A backward that is itself recorded (create_graph) is formed by torch operators from tensors that are part of the graph, as far as
+// the forward was: linear layers are differentiated again, the attention's gradients are constants, as they have always been.
+bool recorded() { return at::GradMode::is_enabled(); }
+struct OutsideAutocast { c10::impl::ExcludeDispatchKeyGuard guard{c10::autocast_dispatch_keyset}; };
+
 struct AttnNode : public Node {
   ContextPtr c;
   SavedAttn saved;
@@ -457,12 +463,35 @@ Result attention(const ContextPtr& c, const Tensor& query, const Tensor& key, co
   return Result{out, a};
 }
 
+// The attention call of a forward that has been made, as a node over other (equal) operands
+Tensor as_node(const ContextPtr& c, const Attn& a, const Tensor& query, const Tensor& key, const Tensor& value) {
+  auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(query, key, value));
+  node->c = c;
+  node->tq = query.scalar_type(); node->tk = key.scalar_type(); node->tv = value.scalar_type();
+  node->saved.save_all(a, a.q, a.k, a.v);
+  Tensor out = a.O.detach();
+  torch::autograd::set_history(out, node);
+  return out;
+}
+// gradients of `out` with respect to the inputs that the node has to serve, themselves differentiable
+variable_list gradients_of(const Tensor& out, const Tensor& go, const variable_list& inputs, const std::function<bool(size_t)>& wanted) {
+  variable_list some, result(inputs.size());
+  std::vector<size_t> at;
+  for (size_t i = 0; i < inputs.size(); ++i)
+    if (wanted(i) && inputs[i].requires_grad()) { some.push_back(inputs[i]); at.push_back(i); }
+  if (some.empty()) return result;
+  const variable_list g = torch::autograd::grad({out}, some, {go}, true, true, true);
+  for (size_t i = 0; i < at.size(); ++i) result[at[i]] = g[i];
+  return result;
+}
+
 // A whole multi-head attention layer: x [B, L, dim] -> projections -> attention -> output projection [B, L, dim_out].
 struct LayerNode : public Node {
   ContextPtr c;
   bool fp32 = false;
   SavedAttn saved;
-  SavedVariable x, w[4];                 // Wq, Wk, Wv, Wf
+  SavedVariable x, w[4], b[4];           // Wq, Wk, Wv, Wf; the biases are read by a recorded backward only
   at::ScalarType out_type;
   bool released = false;
   std::string name() const override { return "SparseAttentionLayerBackward"; }
@@ -470,8 +499,24 @@ struct LayerNode : public Node {
     std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data();
     for (auto& s : w) s.reset_data();
+    for (auto& s : b) s.reset_data();
     saved.reset();
     released = true;
+  }
+  // stage by stage; the attention's own results are the saved ones
+  variable_list recorded_backward(const Tensor& grad) {
+    OutsideAutocast outside;
+    const auto type = fp32 ? at::kFloat : at::kBFloat16;
+    const Attn a = saved.unpack(*c);
+    const Tensor X = x.unpack();
+    variable_list in{X};
+    for (int i = 0; i < 4; ++i) { in.push_back(w[i].unpack()); in.push_back(b[i].unpack()); }
+    auto linear = [&](const Tensor& t, int i) { return at::linear(t, in[1 + 2 * i].to(type), in[2 + 2 * i].to(type)); };
+    const Tensor t = X.to(type);
+    auto heads = [&](int i) { return linear(t, i).reshape({c->B, c->L, c->H, c->d}).transpose(1, 2); };
+    const Tensor O = as_node(c, a, heads(0), heads(1), heads(2));
+    const Tensor out = linear(O.transpose(1, 2).reshape({c->B, c->L, c->H * c->d}).to(type), 3);
+    return gradients_of(out, grad.to(out_type), in, [&](size_t i) { return task_should_compute_output(i); });
   }
   // inputs: x, Wq, bq, Wk, bk, Wv, bv, Wf, bf
   variable_list apply(variable_list&& grads) override {
@@ -483,6 +528,7 @@ struct LayerNode : public Node {
     variable_list out(9);
     if (!grads[0].defined()) return out;
     c10::cuda::CUDAGuard guard(c->device);
+    if (recorded()) return recorded_backward(grads[0]);
     const int H = (int)c->H, d = (int)c->d, L = (int)c->L;
     const int64_t T = c->B * c->L;
     const Attn a = saved.unpack(*c);
@@ -573,7 +619,7 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
     if (c->mode == NATIVE && c->fused && c->recompute) kept.P = Tensor();
     node->saved.save_all(kept, a.q, a.k, a.v);
     node->x = save(x);
-    for (int i = 0; i < 4; ++i) node->w[i] = save(W[i]);
+    for (int i = 0; i < 4; ++i) { node->w[i] = save(W[i]); node->b[i] = save(b[i]); }
     torch::autograd::set_history(out, node);
   }
   return Result{out, a};
@@ -596,6 +642,14 @@ struct LinearNode : public Node {
     Tensor X = x.unpack();
     Weights l; l.W.push_back(w.unpack());
     c10::cuda::CUDAGuard guard(X.device());
+    if (recorded()) {
+      OutsideAutocast outside;
+      const Tensor go = grads[0].to(out_type).reshape({-1, l.out()}), x2 = X.to(out_type).reshape({-1, l.in()});
+      if (task_should_compute_output(0)) out[0] = go.matmul(l.W[0].to(out_type)).reshape(X.sizes()).to(X.scalar_type());
+      if (task_should_compute_output(1)) out[1] = go.t().matmul(x2).to(at::kFloat);
+      if (task_should_compute_output(2)) out[2] = go.sum(0).to(at::kFloat);
+      return out;
+    }
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
     Tensor go = grads[0].to(out_type).contiguous();
     if (!aligned32(go)) go = go.clone();
@@ -647,11 +701,12 @@ Tensor linear(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
 // Feed-forward block Linear -> GELU -> Linear under mixed precision, the activation inside the first product's kernel.
 struct MlpNode : public Node {
   SavedVariable x, w1, w2, h_s, g_s;     // h_s, g_s: pre-activation and activation, bf16
+  SavedVariable b1, b2;                  // read by a recorded backward only
   bool released = false;
   std::string name() const override { return "FeedForwardBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&x, &w1, &w2, &h_s, &g_s}) s->reset_data();
+    for (SavedVariable* s : {&x, &w1, &w2, &h_s, &g_s, &b1, &b2}) s->reset_data();
     released = true;
   }
   // inputs: x, W1, b1, W2, b2
@@ -665,6 +720,13 @@ struct MlpNode : public Node {
     if (!grads[0].defined()) return out;
     Tensor X = x.unpack();
     c10::cuda::CUDAGuard guard(X.device());
+    if (recorded()) {
+      OutsideAutocast outside;
+      const variable_list in{X, w1.unpack(), b1.unpack(), w2.unpack(), b2.unpack()};
+      auto half = [](const Tensor& t) { return t.to(at::kBFloat16); };
+      const Tensor y = at::linear(at::gelu(at::linear(half(X), half(in[1]), half(in[2]))), half(in[3]), half(in[4]));
+      return gradients_of(y, half(grads[0]), in, [&](size_t i) { return task_should_compute_output(i); });
+    }
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
     const Tensor h = h_s.unpack().contiguous(), g = g_s.unpack().contiguous();
     Weights l1, l2;
@@ -715,6 +777,7 @@ Tensor mlp(const Tensor& x, const Tensor& W1, const Tensor& b1, const Tensor& W2
     node->set_next_edges(torch::autograd::collect_next_edges(x, W1, b1, W2, b2));
     node->x = save(x); node->w1 = save(W1); node->w2 = save(W2);
     node->h_s = save(h); node->g_s = save(g);
+    node->b1 = save(b1); node->b2 = save(b2);
     torch::autograd::set_history(out, node);
   }
   return out;

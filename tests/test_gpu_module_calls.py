@@ -215,3 +215,54 @@ def test_transforms_of_a_linear_layer():
         lin(fw.make_dual(x, torch.ones_like(x)))
     with pytest.raises(RuntimeError):
         torch.func.vmap(lin)(x[None].expand(3, -1, -1))
+
+
+def second_order(layer, kind, x, keys, mat):
+    out = run_layer(layer, kind, x, keys, mat)
+    first = torch.autograd.grad(out.float().square().sum(), [x] + list(layer.parameters()), create_graph=True)
+    total = sum(g.float().square().sum() for g in first if g.requires_grad)
+    second = torch.autograd.grad(total, [x] + list(layer.parameters()), allow_unused=True) if torch.is_tensor(total) else ()
+    return first, second
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_a_recorded_backward_of_a_layer(kind):
+    """create_graph: the same first gradients, and the second ones that the stages one by one give."""
+    x, keys = make_inputs()
+    layer, mat = make_layer(kind), make_mask(9)
+    if KINDS[kind][1] == "bf16":
+        x = x.detach().to(torch.bfloat16).requires_grad_()
+    plain = gradients(layer, run_layer(layer, kind, x, keys, mat), x)
+    first, second = second_order(layer, kind, x, keys, mat)
+    hook = layer.W_k.register_forward_hook(lambda *_: None)       # stage by stage
+    want_first, want_second = second_order(layer, kind, x, keys, mat)
+    hook.remove()
+    tol = 3e-2 if KINDS[kind][1] == "bf16" else 1e-5              # bf16: a chain of roundings of 2^-9 in another order
+    close = lambda a, b: float((a.float() - b.float()).norm()) <= tol * float(b.float().norm()) + 1e-6
+    assert all(close(a.detach(), b) for a, b in zip(first, plain))
+    assert all(close(a.detach(), b.detach()) for a, b in zip(first, want_first))
+    assert [g is None for g in second] == [g is None for g in want_second]
+    assert all(close(a, b) for a, b in zip(second, want_second) if a is not None)
+
+
+def test_second_derivatives_of_linear_layers():
+    from spion_b200._ops import ops
+    from spion_b200.layernorm import BiasGradLinear
+    lin, l2 = BiasGradLinear(64, 128).cuda(), torch.nn.Linear(128, 64).cuda()
+    x = torch.randn(50, 64, device="cuda", requires_grad=True)
+
+    def penalty(f, x, params):
+        g = torch.autograd.grad(f(x).square().sum(), x, create_graph=True)[0]
+        return torch.autograd.grad(g.square().sum(), [x] + params)
+
+    got = penalty(lin, x, [lin.weight])
+    w, xd = lin.weight.detach().double().requires_grad_(), x.detach().double().requires_grad_()
+    want = penalty(lambda t: torch.nn.functional.linear(t, w, lin.bias.detach().double()), xd, [w])
+    assert all(float((a - b).norm() / b.norm()) < 1e-6 for a, b in zip(got, want))
+    # mixed precision: through the input
+    xb = x.detach().to(torch.bfloat16).requires_grad_()
+    ff = lambda t: ops.mlp(t, lin.weight, lin.bias, l2.weight, l2.bias)
+    got = penalty(ff, xb, [])
+    ref = lambda t: torch.nn.functional.linear(torch.nn.functional.gelu(torch.nn.functional.linear(t, w, lin.bias.double())), l2.weight.double(), l2.bias.double())
+    want = penalty(ref, xb.detach().double().requires_grad_(), [])
+    assert float((got[0].double() - want[0]).norm() / want[0].norm()) < 3e-2
