@@ -416,6 +416,12 @@ int spion_linear_supported(int in_features, int out_features, int fp32);
 int spion_linear_forward(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
                          const spion_tokens* Y, void* gelu_out, long long T, int in_features, int out_features,
                          void* cuda_stream);
+/* The same in bf16 mode, leaving what a backward needs beside it, since the caller may change X and W before that: x_copy [T,
+ * in_features] bf16, the tokens as the products used them (fp32 tokens only), w_copy [out_features, in_features] fp32, the stacked W.
+ * Either may be NULL; 16-byte aligned. */
+int spion_linear_forward_keep(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
+                              const spion_tokens* Y, void* gelu_out, void* x_copy, float* w_copy, long long T, int in_features,
+                              int out_features, void* cuda_stream);
 /* dX = dY W, times gelu'(gelu_in) element by element when gelu_in (bf16 [T, in_features]) is not NULL (dX bf16 then).
  * dX fp32: one fp32 sum over all stacked layers.  dX bf16 and nw == 3: the sum of the three layers' gradients, each rounded to
  * bf16 and added in bf16 from the last to the first, which is what separate layers give (out_features / 3 a multiple of 64). */

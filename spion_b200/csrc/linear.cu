@@ -133,6 +133,8 @@ struct GemmArgs {
   int parts;                // bf16 gradient of three stacked layers: chunks per layer (0: one accumulator for the whole contraction)
   const __nv_bfloat16* h;   // EPI_DGELU: pre-activation [T, N]
   __nv_bfloat16* g;         // EPI_GELU: activation [T, N] (Y receives the pre-activation)
+  __nv_bfloat16* x_copy;    // or null: A as the products use it, [T, K] (fp32 tokens in bf16 mode)
+  float* w_copy;            // or null: the stacked W
 };
 
 constexpr int LG_LOADERS = 8;
@@ -246,6 +248,11 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
       const uint32_t dst = TRANSB ? ((uint32_t)((r >> 6) * G + (c8 >> 3)) * 8192u + (r & 63) * 128)
                                   : ((uint32_t)(c8 >> 3) * bchunk + r * 128);
       raw_store<SPLIT, false>(v, sbase + dst + (((c8 & 7) ^ (r & 7)) << 4), bpart);
+      if (!TRANSB && SPLIT == 1 && a.w_copy && blockIdx.x == 0) {
+        float4* to = reinterpret_cast<float4*>(a.w_copy + (size_t)gr * a.wld + c8 * 8);
+        to[0] = *reinterpret_cast<const float4*>(&x);
+        to[1] = *reinterpret_cast<const float4*>(&y);
+      }
     }
     for (int n = tid; n < nc; n += LG_THREADS) {
       float b = 0.f;
@@ -303,6 +310,14 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
       for (int i = 0; i < R; ++i) {                      // registers freed by a store take the next chunk's load
         const int r = lrow + 32 * i;
         raw_store<SPLIT, false>(cur[i], dst + r * 128 + ((lc8 ^ (r & 7)) << 4), CHUNK);
+        if (!TRANSB && SPLIT == 1 && a.x_copy && blockIdx.y == 0 && tile * 128 + r < a.T && ch * 64 + lc8 * 8 < a.K) {
+          uint4 w;
+          w.x = pack_bf16(__uint_as_float(cur[i].w[0]), __uint_as_float(cur[i].w[1]));
+          w.y = pack_bf16(__uint_as_float(cur[i].w[2]), __uint_as_float(cur[i].w[3]));
+          w.z = pack_bf16(__uint_as_float(cur[i].w[4]), __uint_as_float(cur[i].w[5]));
+          w.w = pack_bf16(__uint_as_float(cur[i].w[6]), __uint_as_float(cur[i].w[7]));
+          *reinterpret_cast<uint4*>(a.x_copy + (size_t)(tile * 128 + r) * a.K + ch * 64 + lc8 * 8) = w;
+        }
         cur[i] = load_row(col, tile_n, i);
       }
       fence_proxy_async();
@@ -896,17 +911,25 @@ extern "C" int spion_linear_status(int reset) {
 extern "C" int spion_linear_forward(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
                                     const spion_tokens* Y, void* gelu_out, long long T, int in_features, int out_features,
                                     void* cuda_stream) {
+  return spion_linear_forward_keep(X, W, bias, nw, fp32, Y, gelu_out, nullptr, nullptr, T, in_features, out_features, cuda_stream);
+}
+
+extern "C" int spion_linear_forward_keep(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
+                                         const spion_tokens* Y, void* gelu_out, void* x_copy, float* w_copy, long long T,
+                                         int in_features, int out_features, void* cuda_stream) {
   if (!mat_ok(X) || !mat_ok(Y) || !W || nw < 1 || nw > 3 || T < 1 || T > 0x7fffffffLL - 256) return SPION_ERR_ARG;
   if (X->cols * X->count != in_features || Y->cols * Y->count != out_features || out_features % nw) return SPION_ERR_ARG;
   if (fp32 && (X->is_bf16 || Y->is_bf16 || gelu_out)) return SPION_ERR_UNSUPPORTED;
   if (gelu_out && (!Y->is_bf16 || ((uintptr_t)gelu_out & 31))) return SPION_ERR_UNSUPPORTED;
+  if ((fp32 && (x_copy || w_copy)) || (x_copy && X->is_bf16)) return SPION_ERR_UNSUPPORTED;
+  if (((uintptr_t)x_copy | (uintptr_t)w_copy) & 15) return SPION_ERR_ARG;
   GemmArgs a;
   a.A = to_mat(X); a.Y = to_mat(Y);
   a.wper = out_features / nw; a.wld = in_features;
   for (int i = 0; i < 3; ++i) { a.W[i] = i < nw ? W[i] : nullptr; a.bias[i] = (bias && i < nw) ? bias[i] : nullptr; }
   for (int i = 0; i < nw; ++i) if (!a.W[i] || ((uintptr_t)a.W[i] & 15)) return SPION_ERR_ARG;
   a.T = (int)T; a.K = in_features; a.N = out_features;
-  a.h = nullptr; a.g = (__nv_bfloat16*)gelu_out;
+  a.h = nullptr; a.g = (__nv_bfloat16*)gelu_out; a.x_copy = (__nv_bfloat16*)x_copy; a.w_copy = w_copy;
   size_t smem;
   a.k0 = 0; a.accum = 0; a.parts = 0;
   if (!plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
@@ -932,7 +955,7 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
   for (int i = 0; i < 3; ++i) { a.W[i] = i < nw ? W[i] : nullptr; a.bias[i] = nullptr; }
   for (int i = 0; i < nw; ++i) if (!a.W[i] || ((uintptr_t)a.W[i] & 15)) return SPION_ERR_ARG;
   a.T = (int)T; a.K = out_features; a.N = in_features;
-  a.h = (const __nv_bfloat16*)gelu_in; a.g = nullptr;
+  a.h = (const __nv_bfloat16*)gelu_in; a.g = nullptr; a.x_copy = nullptr; a.w_copy = nullptr;
   size_t smem;
   a.k0 = 0; a.accum = 0;
   a.parts = !fp32 && dX->is_bf16 && nw == 3 ? a.wper / 64 : 0;

@@ -16,7 +16,6 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
-#include <functional>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -99,10 +98,24 @@ struct Weights {                        // up to three stacked linear layers
   int out() const { return (int)(W[0].size(0) * W.size()); }
 };
 
-void linear_forward(const spion_tokens& X, const Weights& w, bool fp32, const spion_tokens& Y, void* gelu_out, int64_t T, void* st) {
+// What a mixed-precision backward reads in place of the input and the weights: as under the framework's own autocast, the caller may
+// change both in between.  The forward's kernels write the copies on the way.
+struct Kept {
+  Tensor x, w;
+  // x: the input (bf16 input is kept as it is); fp32 layers keep nothing
+  Kept() {}
+  Kept(bool need, bool fp32, const Tensor& X, const Weights& l) {
+    if (!need || fp32) return;
+    w = at::empty({l.out(), l.in()}, l.W[0].options());
+    if (X.scalar_type() == at::kFloat) x = at::empty(X.sizes(), X.options().dtype(at::kBFloat16));
+  }
+};
+void linear_forward(const spion_tokens& X, const Weights& w, bool fp32, const spion_tokens& Y, void* gelu_out, int64_t T, void* st,
+                    const Kept& kept = Kept()) {
   const float *W[3], *b[3];
   for (int i = 0; i < w.n(); ++i) { W[i] = pf(w.W[i]); b[i] = pf(w.b[i]); }
-  check(spion_linear_forward(&X, W, b, w.n(), fp32, &Y, gelu_out, T, w.in(), w.out(), st), "spion_linear_forward");
+  check(spion_linear_forward_keep(&X, W, b, w.n(), fp32, &Y, gelu_out, p(kept.x), (float*)p(kept.w), T, w.in(), w.out(), st),
+        "spion_linear_forward_keep");
 }
 void linear_backward_input(const spion_tokens& dY, const Weights& w, bool fp32, const void* gelu_in, const spion_tokens& dX, int64_t T, void* st) {
   const float* W[3];
@@ -110,13 +123,13 @@ void linear_backward_input(const spion_tokens& dY, const Weights& w, bool fp32, 
   check(spion_linear_backward_input(&dY, W, w.n(), fp32, gelu_in, &dX, T, w.in(), w.out(), st), "spion_linear_backward_input");
 }
 // Weight and bias gradients of the stacked layers from dY (one [T, per] matrix per layer, or their head-split form) and X.
-// fp32 tokens: the library's kernel, views of one buffer.  bf16 tokens (a layer inside a mixed-precision encoder): the
-// framework's bf16 products and the column-sum kernel, so that a training step repeats bit for bit what separate layers give.
+// fp32 tokens (or the copy kept of them): the library's kernel, views of one buffer.  bf16 tokens (a layer inside a mixed-precision
+// encoder): the framework's bf16 products and the column-sum kernel, so that a training step repeats bit for bit what separate layers give.
 void linear_backward_weight(const std::vector<Tensor>& dY, const spion_tokens& tY, const Tensor& X, const spion_tokens& tX, const Weights& w,
-                            bool fp32, int64_t T, void* st, std::vector<Tensor>& dW, std::vector<Tensor>& db) {
+                            bool fp32, int64_t T, void* st, std::vector<Tensor>& dW, std::vector<Tensor>& db, bool copied = false) {
   const int64_t in = w.in(), out = w.out(), per = out / w.n();
   const auto opt = w.W[0].options();
-  if (tX.is_bf16 && tY.heads == 0 && tX.heads == 0) {
+  if (tX.is_bf16 && !copied && tY.heads == 0 && tX.heads == 0) {
     Tensor x2 = X.view({T, in});
     const int n = w.n();
     Tensor prod = at::empty({out, in}, x2.options());        // the products side by side: one conversion for all of them
@@ -463,6 +476,49 @@ Result attention(const ContextPtr& c, const Tensor& query, const Tensor& key, co
   return Result{out, a};
 }
 
+struct LinearNode : public Node {
+  bool fp32 = false;
+  SavedVariable x, w;
+  at::ScalarType out_type, x_type;
+  std::string name() const override { return "TokenLinearBackward"; }
+  void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); x.reset_data(); w.reset_data(); }
+  variable_list apply(variable_list&& grads) override {
+    return as_backward([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    Tensor X = x.unpack();
+    Weights l; l.W.push_back(w.unpack());
+    c10::cuda::CUDAGuard guard(X.device());
+    if (recorded()) {
+      OutsideAutocast outside;
+      const Tensor go = grads[0].to(out_type).reshape({-1, l.out()}), x2 = X.to(out_type).reshape({-1, l.in()});
+      if (task_should_compute_output(0)) out[0] = go.matmul(l.W[0].to(out_type)).reshape(X.sizes()).to(x_type);
+      if (task_should_compute_output(1)) out[1] = go.t().matmul(x2).to(at::kFloat);
+      if (task_should_compute_output(2)) out[2] = go.sum(0).to(at::kFloat);
+      return out;
+    }
+    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
+    Tensor go = grads[0].to(out_type).contiguous();
+    if (!aligned32(go)) go = go.clone();
+    void* st = stream_of(X);
+    const int64_t T = X.numel() / l.in();
+    const spion_tokens tg = tok({go}, l.out());
+    if (task_should_compute_output(1) || task_should_compute_output(2)) {
+      std::vector<Tensor> dW, db;
+      linear_backward_weight({go}, tg, X, tok({X}, l.in()), l, fp32, T, st, dW, db, X.scalar_type() != x_type);
+      out[1] = dW[0]; out[2] = db[0];
+    }
+    if (task_should_compute_output(0)) {
+      out[0] = at::empty(X.sizes(), X.options().dtype(x_type));
+      linear_backward_input(tg, l, fp32, nullptr, tok({out[0]}, l.in()), T, st);
+    }
+    return out;
+  }
+};
+
 // The attention call of a forward that has been made, as a node over other (equal) operands
 Tensor as_node(const ContextPtr& c, const Attn& a, const Tensor& query, const Tensor& key, const Tensor& value) {
   auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
@@ -474,16 +530,14 @@ Tensor as_node(const ContextPtr& c, const Attn& a, const Tensor& query, const Te
   torch::autograd::set_history(out, node);
   return out;
 }
-// gradients of `out` with respect to the inputs that the node has to serve, themselves differentiable
-variable_list gradients_of(const Tensor& out, const Tensor& go, const variable_list& inputs, const std::function<bool(size_t)>& wanted) {
-  variable_list some, result(inputs.size());
-  std::vector<size_t> at;
-  for (size_t i = 0; i < inputs.size(); ++i)
-    if (wanted(i) && inputs[i].requires_grad()) { some.push_back(inputs[i]); at.push_back(i); }
-  if (some.empty()) return result;
-  const variable_list g = torch::autograd::grad({out}, some, {go}, true, true, true);
-  for (size_t i = 0; i < at.size(); ++i) result[at[i]] = g[i];
-  return result;
+// The same for a linear layer; its inputs are given by their edges, its operands by what was saved of them.
+Tensor as_linear_node(const Tensor& y, bool fp32, const Tensor& x, const Tensor& w, at::ScalarType x_type, torch::autograd::edge_list edges) {
+  auto node = std::shared_ptr<LinearNode>(new LinearNode(), torch::autograd::deleteNode);
+  node->set_next_edges(std::move(edges));
+  node->fp32 = fp32; node->x = save(x); node->w = save(w); node->out_type = y.scalar_type(); node->x_type = x_type;
+  Tensor out = y.detach();
+  torch::autograd::set_history(out, node);
+  return out;
 }
 
 // A whole multi-head attention layer: x [B, L, dim] -> projections -> attention -> output projection [B, L, dim_out].
@@ -491,32 +545,53 @@ struct LayerNode : public Node {
   ContextPtr c;
   bool fp32 = false;
   SavedAttn saved;
-  SavedVariable x, w[4], b[4];           // Wq, Wk, Wv, Wf; the biases are read by a recorded backward only
-  at::ScalarType out_type;
+  SavedVariable x, w[4];                 // Wq, Wk, Wv, Wf
+  at::ScalarType out_type, x_type;
   bool released = false;
   std::string name() const override { return "SparseAttentionLayerBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
     x.reset_data();
     for (auto& s : w) s.reset_data();
-    for (auto& s : b) s.reset_data();
     saved.reset();
     released = true;
   }
-  // stage by stage; the attention's own results are the saved ones
-  variable_list recorded_backward(const Tensor& grad) {
+  // stage by stage: the saved results of the stages become outputs of nodes of their own
+  variable_list recorded_backward(const Tensor& grad, void* st) {
     OutsideAutocast outside;
+    variable_list out(9);
     const auto type = fp32 ? at::kFloat : at::kBFloat16;
     const Attn a = saved.unpack(*c);
-    const Tensor X = x.unpack();
-    variable_list in{X};
-    for (int i = 0; i < 4; ++i) { in.push_back(w[i].unpack()); in.push_back(b[i].unpack()); }
-    auto linear = [&](const Tensor& t, int i) { return at::linear(t, in[1 + 2 * i].to(type), in[2 + 2 * i].to(type)); };
-    const Tensor t = X.to(type);
-    auto heads = [&](int i) { return linear(t, i).reshape({c->B, c->L, c->H, c->d}).transpose(1, 2); };
-    const Tensor O = as_node(c, a, heads(0), heads(1), heads(2));
-    const Tensor out = linear(O.transpose(1, 2).reshape({c->B, c->L, c->H * c->d}).to(type), 3);
-    return gradients_of(out, grad.to(out_type), in, [&](size_t i) { return task_should_compute_output(i); });
+    const Tensor X = x.unpack(), x2 = X.to(type).reshape({c->B * c->L, X.size(2)});
+    Tensor W[4];
+    for (int i = 0; i < 4; ++i) W[i] = w[i].unpack();
+    auto rows = [&](const Tensor& t) { return t.transpose(1, 2).reshape({c->B, c->L, c->H * c->d}); };
+    auto operand = [&](const Tensor& t, int i) {
+      const Tensor y = as_linear_node(rows(t), fp32, X, W[i], x_type, {next_edge(0), next_edge(1 + 2 * i), next_edge(2 + 2 * i)});
+      return y.view({c->B, c->L, c->H, c->d}).transpose(1, 2);
+    };
+    const Tensor O = rows(as_node(c, a, operand(a.q, 0), operand(a.k, 1), operand(a.v, 2))).to(type);
+    const Tensor go = grad.to(out_type).reshape({c->B * c->L, W[3].size(0)});
+    if (task_should_compute_output(7)) out[7] = go.t().matmul(O.reshape({c->B * c->L, -1})).to(at::kFloat);
+    if (task_should_compute_output(8)) out[8] = go.sum(0).to(at::kFloat);
+    Tensor dO = go.matmul(W[3].to(type)).view({c->B, c->L, c->H, c->d}).transpose(1, 2), g[3];
+    {
+      at::NoGradGuard constant;
+      dO = dO.to(c->type());
+      if (!a.heads) dO = dO.contiguous();
+      attn_backward(*c, a, dO, g[0], g[1], g[2], st);
+    }
+    for (int i = 0; i < 3; ++i) {
+      const Tensor gi = rows(g[i]).reshape({c->B * c->L, c->H * c->d}).to(type);
+      if (task_should_compute_output(1 + 2 * i)) out[1 + 2 * i] = gi.t().matmul(x2).to(at::kFloat);
+      if (task_should_compute_output(2 + 2 * i)) out[2 + 2 * i] = gi.sum(0).to(at::kFloat);
+      if (task_should_compute_output(0)) {
+        const Tensor dx = gi.matmul(W[i].to(type));
+        out[0] = out[0].defined() ? out[0] + dx : dx;
+      }
+    }
+    if (out[0].defined()) out[0] = out[0].view(X.sizes()).to(x_type);
+    return out;
   }
   // inputs: x, Wq, bq, Wk, bk, Wv, bv, Wf, bf
   variable_list apply(variable_list&& grads) override {
@@ -528,7 +603,7 @@ struct LayerNode : public Node {
     variable_list out(9);
     if (!grads[0].defined()) return out;
     c10::cuda::CUDAGuard guard(c->device);
-    if (recorded()) return recorded_backward(grads[0]);
+    if (recorded()) return recorded_backward(grads[0], stream_of(grads[0]));
     const int H = (int)c->H, d = (int)c->d, L = (int)c->L;
     const int64_t T = c->B * c->L;
     const Attn a = saved.unpack(*c);
@@ -559,11 +634,11 @@ struct LayerNode : public Node {
     for (int i = 1; i < 7; ++i) any = any || task_should_compute_output(i);
     if (any) {
       dW.clear(); db.clear();
-      linear_backward_weight({rows(dq), rows(dk), rows(dv)}, tg, X, tok({X}, dim), qkv, fp32, T, st, dW, db);
+      linear_backward_weight({rows(dq), rows(dk), rows(dv)}, tg, X, tok({X}, dim), qkv, fp32, T, st, dW, db, X.scalar_type() != x_type);
       for (int i = 0; i < 3; ++i) { out[1 + 2 * i] = dW[i]; out[2 + 2 * i] = db[i]; }
     }
     if (task_should_compute_output(0)) {
-      Tensor dX = at::empty(X.sizes(), X.options());
+      Tensor dX = at::empty(X.sizes(), X.options().dtype(x_type));
       linear_backward_input(tg, qkv, fp32, nullptr, tok({dX}, dim), T, st);
       out[0] = dX;
     }
@@ -592,6 +667,7 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
   need = need && at::GradMode::is_enabled();
   Attn a;
   Tensor out;
+  Kept kept_in, kept_out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
@@ -606,10 +682,12 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
     a.q = empty_operand(*c, a.heads, like); a.k = empty_operand(*c, a.heads, like); a.v = empty_operand(*c, a.heads, like);
     Weights qkv{{W[0].detach(), W[1].detach(), W[2].detach()}, {b[0].detach(), b[1].detach(), b[2].detach()}};
     Weights ff{{W[3].detach()}, {b[3].detach()}};
-    linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st);
+    kept_in = Kept(need, fp32, X, qkv);
+    linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st, kept_in);
     attn_forward(*c, a, need, st);
     out = at::empty({c->B, c->L, ff.out()}, opt);
-    linear_forward(form({a.O}), ff, fp32, tok({out}, ff.out()), nullptr, T, st);
+    kept_out = Kept(need, fp32, a.O, ff);
+    linear_forward(form({a.O}), ff, fp32, tok({out}, ff.out()), nullptr, T, st, kept_out);
   }
   if (need) {
     auto node = std::shared_ptr<LayerNode>(new LayerNode(), torch::autograd::deleteNode);
@@ -618,57 +696,16 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
     Attn kept = a;
     if (c->mode == NATIVE && c->fused && c->recompute) kept.P = Tensor();
     node->saved.save_all(kept, a.q, a.k, a.v);
-    node->x = save(x);
-    for (int i = 0; i < 4; ++i) { node->w[i] = save(W[i]); node->b[i] = save(b[i]); }
+    node->x_type = x.scalar_type();
+    node->x = save(kept_in.x.defined() ? kept_in.x : x);
+    const int64_t per = W[0].size(0);
+    for (int i = 0; i < 4; ++i) node->w[i] = save(!kept_in.w.defined() ? W[i] : i < 3 ? kept_in.w.narrow(0, i * per, per) : kept_out.w);
     torch::autograd::set_history(out, node);
   }
   return Result{out, a};
 }
 
 // ------------------------------------------------------------------------------------------------ linear layers on their own
-struct LinearNode : public Node {
-  bool fp32 = false;
-  SavedVariable x, w;
-  at::ScalarType out_type;
-  std::string name() const override { return "TokenLinearBackward"; }
-  void release_variables() override { std::lock_guard<std::mutex> lock(mutex_); x.reset_data(); w.reset_data(); }
-  variable_list apply(variable_list&& grads) override {
-    return as_backward([&] { return backward(grads); });
-  }
-  variable_list backward(const variable_list& grads) {
-    std::lock_guard<std::mutex> lock(mutex_);
-    variable_list out(3);
-    if (!grads[0].defined()) return out;
-    Tensor X = x.unpack();
-    Weights l; l.W.push_back(w.unpack());
-    c10::cuda::CUDAGuard guard(X.device());
-    if (recorded()) {
-      OutsideAutocast outside;
-      const Tensor go = grads[0].to(out_type).reshape({-1, l.out()}), x2 = X.to(out_type).reshape({-1, l.in()});
-      if (task_should_compute_output(0)) out[0] = go.matmul(l.W[0].to(out_type)).reshape(X.sizes()).to(X.scalar_type());
-      if (task_should_compute_output(1)) out[1] = go.t().matmul(x2).to(at::kFloat);
-      if (task_should_compute_output(2)) out[2] = go.sum(0).to(at::kFloat);
-      return out;
-    }
-    if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
-    Tensor go = grads[0].to(out_type).contiguous();
-    if (!aligned32(go)) go = go.clone();
-    void* st = stream_of(X);
-    const int64_t T = X.numel() / l.in();
-    const spion_tokens tg = tok({go}, l.out());
-    if (task_should_compute_output(1) || task_should_compute_output(2)) {
-      std::vector<Tensor> dW, db;
-      linear_backward_weight({go}, tg, X, tok({X}, l.in()), l, fp32, T, st, dW, db);
-      out[1] = dW[0]; out[2] = db[0];
-    }
-    if (task_should_compute_output(0)) {
-      out[0] = at::empty(X.sizes(), X.options());
-      linear_backward_input(tg, l, fp32, nullptr, tok({out[0]}, l.in()), T, st);
-    }
-    return out;
-  }
-};
-
 bool linear_supported(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
   if (!x.is_cuda() || !plain({x, W, b}) || x.numel() == 0 || x.dim() < 2 || x.size(-1) != W.size(1)) return false;
   if (x.scalar_type() != at::kFloat && (fp32 || x.scalar_type() != at::kBFloat16)) return false;
@@ -677,22 +714,27 @@ bool linear_supported(const Tensor& x, const Tensor& W, const Tensor& b, bool fp
 
 Tensor linear(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
   c10::cuda::CUDAGuard guard(x.device());
+  const bool need = at::GradMode::is_enabled() && (x.requires_grad() || W.requires_grad() || b.requires_grad());
   Tensor out;
+  Kept kept;
   {
     at::AutoDispatchBelowADInplaceOrView below;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     Tensor X = x.detach();
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
     Weights l{{W.detach()}, {b.detach()}};
+    kept = Kept(need, fp32, X, l);
     auto sizes = x.sizes().vec();
     sizes.back() = l.out();
     out = at::empty(sizes, X.options().dtype(fp32 ? at::kFloat : at::kBFloat16));
-    linear_forward(tok({X}, l.in()), l, fp32, tok({out}, l.out()), nullptr, X.numel() / l.in(), stream_of(X));
+    linear_forward(tok({X}, l.in()), l, fp32, tok({out}, l.out()), nullptr, X.numel() / l.in(), stream_of(X), kept);
   }
-  if (at::GradMode::is_enabled() && (x.requires_grad() || W.requires_grad() || b.requires_grad())) {
+  if (need) {
     auto node = std::shared_ptr<LinearNode>(new LinearNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x, W, b));
-    node->fp32 = fp32; node->x = save(x); node->w = save(W); node->out_type = out.scalar_type();
+    node->fp32 = fp32; node->out_type = out.scalar_type(); node->x_type = x.scalar_type();
+    node->x = save(kept.x.defined() ? kept.x : x);
+    node->w = save(kept.w.defined() ? kept.w : W);
     torch::autograd::set_history(out, node);
   }
   return out;
@@ -701,12 +743,12 @@ Tensor linear(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
 // Feed-forward block Linear -> GELU -> Linear under mixed precision, the activation inside the first product's kernel.
 struct MlpNode : public Node {
   SavedVariable x, w1, w2, h_s, g_s;     // h_s, g_s: pre-activation and activation, bf16
-  SavedVariable b1, b2;                  // read by a recorded backward only
+  at::ScalarType x_type;
   bool released = false;
   std::string name() const override { return "FeedForwardBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&x, &w1, &w2, &h_s, &g_s, &b1, &b2}) s->reset_data();
+    for (SavedVariable* s : {&x, &w1, &w2, &h_s, &g_s}) s->reset_data();
     released = true;
   }
   // inputs: x, W1, b1, W2, b2
@@ -722,10 +764,18 @@ struct MlpNode : public Node {
     c10::cuda::CUDAGuard guard(X.device());
     if (recorded()) {
       OutsideAutocast outside;
-      const variable_list in{X, w1.unpack(), b1.unpack(), w2.unpack(), b2.unpack()};
       auto half = [](const Tensor& t) { return t.to(at::kBFloat16); };
-      const Tensor y = at::linear(at::gelu(at::linear(half(X), half(in[1]), half(in[2]))), half(in[3]), half(in[4]));
-      return gradients_of(y, half(grads[0]), in, [&](size_t i) { return task_should_compute_output(i); });
+      const Tensor W1 = w1.unpack(), W2 = w2.unpack(), x2 = half(X).reshape({-1, W1.size(1)});
+      auto sizes = X.sizes().vec();
+      sizes.back() = W1.size(0);
+      const Tensor pre = as_linear_node(h_s.unpack().reshape(sizes), false, X, W1, x_type, {next_edge(0), next_edge(1), next_edge(2)}).reshape({-1, W1.size(0)});
+      const Tensor go = half(grads[0]).reshape({-1, W2.size(0)}), dh = at::gelu_backward(go.matmul(half(W2)), pre);
+      if (task_should_compute_output(0)) out[0] = dh.matmul(half(W1)).reshape(X.sizes()).to(x_type);
+      if (task_should_compute_output(1)) out[1] = dh.t().matmul(x2).to(at::kFloat);
+      if (task_should_compute_output(2)) out[2] = dh.sum(0).to(at::kFloat);
+      if (task_should_compute_output(3)) out[3] = go.t().matmul(at::gelu(pre)).to(at::kFloat);
+      if (task_should_compute_output(4)) out[4] = go.sum(0).to(at::kFloat);
+      return out;
     }
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
     const Tensor h = h_s.unpack().contiguous(), g = g_s.unpack().contiguous();
@@ -741,9 +791,9 @@ struct MlpNode : public Node {
     Tensor dh = at::empty(h.sizes(), h.options());
     linear_backward_input(tg, l2, false, p(h), tok({dh}, l2.in()), T, st);
     const spion_tokens th = tok({dh}, l1.out());
-    linear_backward_weight({dh}, th, X, tok({X}, l1.in()), l1, false, T, st, dW, db);
+    linear_backward_weight({dh}, th, X, tok({X}, l1.in()), l1, false, T, st, dW, db, X.scalar_type() != x_type);
     if (task_should_compute_output(0)) {
-      out[0] = at::empty(X.sizes(), X.options());
+      out[0] = at::empty(X.sizes(), X.options().dtype(x_type));
       linear_backward_input(th, l1, false, nullptr, tok({out[0]}, l1.in()), T, st);
     }
     out[1] = dW[1]; out[2] = db[1]; out[3] = dW[0]; out[4] = db[0];
@@ -753,7 +803,10 @@ struct MlpNode : public Node {
 
 Tensor mlp(const Tensor& x, const Tensor& W1, const Tensor& b1, const Tensor& W2, const Tensor& b2) {
   c10::cuda::CUDAGuard guard(x.device());
+  const bool need = at::GradMode::is_enabled() &&
+                    (x.requires_grad() || W1.requires_grad() || b1.requires_grad() || W2.requires_grad() || b2.requires_grad());
   Tensor out, h, g;
+  Kept kept1, kept2;
   {
     at::AutoDispatchBelowADInplaceOrView below;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
@@ -765,19 +818,19 @@ Tensor mlp(const Tensor& x, const Tensor& W1, const Tensor& b1, const Tensor& W2
     h = at::empty({T, l1.out()}, opt);
     g = at::empty({T, l1.out()}, opt);
     void* st = stream_of(X);
-    linear_forward(tok({X}, l1.in()), l1, false, tok({h}, l1.out()), g.data_ptr(), T, st);
+    kept1 = Kept(need, false, X, l1); kept2 = Kept(need, false, g, l2);
+    linear_forward(tok({X}, l1.in()), l1, false, tok({h}, l1.out()), g.data_ptr(), T, st, kept1);
     auto sizes = x.sizes().vec();
     sizes.back() = l2.out();
     out = at::empty(sizes, opt);
-    linear_forward(tok({g}, l2.in()), l2, false, tok({out}, l2.out()), nullptr, T, st);
+    linear_forward(tok({g}, l2.in()), l2, false, tok({out}, l2.out()), nullptr, T, st, kept2);
   }
-  if (at::GradMode::is_enabled() &&
-      (x.requires_grad() || W1.requires_grad() || b1.requires_grad() || W2.requires_grad() || b2.requires_grad())) {
+  if (need) {
     auto node = std::shared_ptr<MlpNode>(new MlpNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x, W1, b1, W2, b2));
-    node->x = save(x); node->w1 = save(W1); node->w2 = save(W2);
+    node->x_type = x.scalar_type();
+    node->x = save(kept1.x.defined() ? kept1.x : x); node->w1 = save(kept1.w); node->w2 = save(kept2.w);
     node->h_s = save(h); node->g_s = save(g);
-    node->b1 = save(b1); node->b2 = save(b2);
     torch::autograd::set_history(out, node);
   }
   return out;

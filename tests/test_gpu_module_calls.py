@@ -266,3 +266,42 @@ def test_second_derivatives_of_linear_layers():
     ref = lambda t: torch.nn.functional.linear(torch.nn.functional.gelu(torch.nn.functional.linear(t, w, lin.bias.double())), l2.weight.double(), l2.bias.double())
     want = penalty(ref, xb.detach().double().requires_grad_(), [])
     assert float((got[0].double() - want[0]).norm() / want[0].norm()) < 3e-2
+
+
+@pytest.mark.parametrize("what", ["input", "weights"])
+@pytest.mark.parametrize("call", ["layer", "linear", "feed-forward"])
+def test_mixed_precision_calls_keep_what_their_backward_reads(call, what):
+    """Under autocast the casts are copies: the fp32 input and the weights may change before the backward, as with torch.nn.Linear."""
+    from spion_b200._ops import ops
+    from spion_b200.layernorm import BiasGradLinear
+    x, keys = make_inputs()
+    if call == "layer":
+        mod, mat = make_layer("native bf16"), make_mask(10)
+        f = lambda t: mod(t, keys, mat)[0]
+    elif call == "linear":
+        mod = BiasGradLinear(H * D, 96).cuda()
+        f = mod
+    else:
+        mod = torch.nn.Sequential(BiasGradLinear(H * D, 160), BiasGradLinear(160, H * D)).cuda()
+        f = lambda t: ops.mlp(t, mod[0].weight, mod[0].bias, mod[1].weight, mod[1].bias)
+    params = list(mod.parameters())
+
+    def grads(change):
+        h = x * 1.0
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = f(h)
+        old = [p.detach().clone() for p in params]
+        if change:
+            with torch.no_grad():
+                if what == "input":
+                    h.mul_(3.0)
+                else:
+                    for p in params:
+                        p.mul_(3.0)
+        g = torch.autograd.grad(y.float().square().sum(), [x] + params)
+        with torch.no_grad():
+            for p, o in zip(params, old):
+                p.copy_(o)
+        return g
+
+    same(grads(True), grads(False))
