@@ -21,7 +21,12 @@ import torch
 import torch.nn as nn
 
 from . import _lib, _ops
+from .attention_blockcuda import CUDABlockAttention
+from .attention_blockcuda_mask import CUDABlockMaskAttention
+from .attention_cuda import CUDAAttention
+from .attention_cuda_mask import CUDAMaskAttention
 from .layernorm import BiasGradLinear
+from .native import BlockSparseAttention, DenseViaBlocks
 
 # tasks whose inputs carry padding and therefore use the key-padding variants (models/attention.py:11)
 mask_task = ['lra-listops', 'lra-text', 'lra-news', 'lra-yelp', 'lra-text1', 'lra-news1', 'lra-yelp1',
@@ -29,6 +34,18 @@ mask_task = ['lra-listops', 'lra-text', 'lra-news', 'lra-yelp', 'lra-text1', 'lr
 
 _P = ctypes.c_void_p
 _PLAIN_LINEAR = (nn.Linear, BiasGradLinear)
+_DROPIN_DENSE = (CUDAAttention, CUDAMaskAttention)
+_DROPIN_SPARSE = (CUDABlockAttention, CUDABlockMaskAttention)
+
+
+def untouched(m, types) -> bool:
+    """``m`` is of one of the types and a call that passes its forward over is no different: no hooks, no forward of its own."""
+    return type(m) in types and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                                     or "forward" in m.__dict__)
+
+
+def no_global_hooks() -> bool:
+    return not nn.modules.module._has_any_global_hook()
 
 
 def _load_shim(name, n_init, n_fwd, n_bwd, trailing_int):
@@ -66,33 +83,37 @@ class Attention(nn.Module):
         self.W_v = Linear(self.dim, self.num_head * self.head_dim)
 
         if not inference and self.native:
-            from .native import DenseViaBlocks
             self.attn = DenseViaBlocks(config, dtype=self.native_dtype, keypad=self.with_keypad)
         elif not inference:
             num_batches = config["num_head"] * config["batch_size"]
             if self.with_keypad:
                 attn_cpp = Attention._cuda_mask_compile_module()
-                from .attention_cuda_mask import CUDAMaskAttention as Dense
+                Dense = CUDAMaskAttention
             else:
                 attn_cpp = Attention._cuda_compile_module()
-                from .attention_cuda import CUDAAttention as Dense
+                Dense = CUDAAttention
             attn_handle = attn_cpp.init(config["head_dim"], config["max_seq_len"], num_batches)
             if not attn_handle:
                 raise _lib.SpionError("init() of the dense attention library returned NULL")
             self.attn = Dense(config, attn_cpp, attn_handle)
-            self._dense_type = Dense
             self._dense_ctx = _ops.make_context(attn_handle, _ops.DROPIN_DENSE, config["batch_size"], self.num_head, self.seq_len,
                                                 self.head_dim, torch.cuda.current_device(), False, self.with_keypad)
 
         self.ff = Linear(self.num_head * self.head_dim, self.dim)
 
-    def _linears_are_plain(self) -> bool:
-        """The projections are what __init__ made: no replaced module, no hook that a one-node layer would pass over."""
+    def _stages_are_untouched(self, mat) -> bool:
+        """The projections and the attention module are what was made here: nothing replaced, no hook that a one-node layer would
+        pass over."""
+        if not no_global_hooks():
+            return False
         for m in (self.W_q, self.W_k, self.W_v, self.ff):
-            if type(m) not in _PLAIN_LINEAR or m.bias is None or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks \
-                    or m._backward_pre_hooks:
+            if m.bias is None or not untouched(m, _PLAIN_LINEAR):
                 return False
-        return True
+        if not self.native:
+            return untouched(self.block_attn, _DROPIN_SPARSE)
+        if mat is None:
+            return untouched(self.attn, (DenseViaBlocks,)) and untouched(self.attn.block, (BlockSparseAttention,))
+        return untouched(self.block_attn, (BlockSparseAttention,))
 
     def _one_node(self, X, mask, mat):
         """The whole layer as one autograd node on the library's kernels: projections, attention and output projection back to
@@ -106,11 +127,11 @@ class Attention(nn.Module):
             if self.native and self.native_dtype != torch.float32:
                 return None
             fp32 = True
-        if not self._linears_are_plain():
-            return None
-        block = None
         if mat is None and fp32:
             return None          # in the dense phase the key bias has no effect: its gradient is the rounding noise of the stages
+        if not self._stages_are_untouched(mat):
+            return None
+        block = None
         if self.native:
             block = self.attn.block if mat is None else self.block_attn
             block.use_mask(mat)
@@ -145,7 +166,7 @@ class Attention(nn.Module):
                 attn_out = attn_out.to(X.dtype)
             elif mat is None:
                 call = None
-                if type(self.attn) is self._dense_type:
+                if untouched(self.attn, _DROPIN_DENSE) and no_global_hooks():
                     call = _ops.ops.attention(self._dense_ctx, Q.float(), K.float(), V.float(), mask if self.with_keypad else None)
                 if call is not None:
                     attn_out, attn = call[0], call[1].permute(0, 1, 3, 2)
@@ -164,7 +185,6 @@ class Attention(nn.Module):
         num_batches = int(config["num_head"] * config["batch_size"])
         model_dev = next(self.parameters()).device
         if self.native:
-            from .native import BlockSparseAttention
             # the layer above ignores the probabilities of the sparse phase (models/model_transformer.py:137 reads
             # them in the dense phase only): none are stored
             self.block_attn = BlockSparseAttention(config, dtype=self.native_dtype, keypad=self.with_keypad,
@@ -172,10 +192,10 @@ class Attention(nn.Module):
             return
         if self.with_keypad:
             block_attn_cpp = Attention._blockcuda_mask_compile_module()
-            from .attention_blockcuda_mask import CUDABlockMaskAttention as Sparse
+            Sparse = CUDABlockMaskAttention
         else:
             block_attn_cpp = Attention._blockcuda_compile_module()
-            from .attention_blockcuda import CUDABlockAttention as Sparse
+            Sparse = CUDABlockAttention
         with torch.cuda.device(model_dev):
             handle = block_attn_cpp.init(config["head_dim"], config["max_seq_len"], num_batches, config["block_size"])
         if not handle:

@@ -305,3 +305,36 @@ def test_mixed_precision_calls_keep_what_their_backward_reads(call, what):
         return g
 
     same(grads(True), grads(False))
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_hooks_and_replacements_of_the_attention_module(kind, dense):
+    """What is hooked into or put in the place of the attention module of a layer is called."""
+    x, keys = make_inputs()
+    layer, mat = make_layer(kind, dense), None if dense else make_mask(11)
+    want = run_layer(layer, kind, x, keys, mat)
+    name = "attn" if dense else "block_attn"
+    inner = getattr(layer, name)
+    calls = []
+    hook = inner.register_forward_hook(lambda *_: calls.append("hook"))
+    got = run_layer(layer, kind, x, keys, mat)
+    hook.remove()
+    assert calls == ["hook"]
+    tol = 2e-2 if KINDS[kind][1] == "bf16" else 1e-5              # stage by stage: other roundings of the same products
+    assert float((got.float() - want.float()).norm()) <= tol * float(want.float().norm())
+    everywhere = torch.nn.modules.module.register_module_forward_hook(lambda m, *_: calls.append(type(m).__name__))
+    run_layer(layer, kind, x, keys, mat)
+    everywhere.remove()
+    assert {type(layer).__name__, type(inner).__name__, type(layer.W_q).__name__} <= set(calls)
+
+    class Other(torch.nn.Module):
+        def forward(self, q, k, v, *rest):
+            calls.append("other")
+            return inner(q, k, v, *rest)
+
+    setattr(layer, name, Other())
+    run_layer(layer, kind, x, keys, mat)
+    assert calls[-1] == "other"
+    setattr(layer, name, inner)
+    assert torch.equal(run_layer(layer, kind, x, keys, mat), want)
