@@ -712,6 +712,10 @@ bool linear_supported(const Tensor& x, const Tensor& W, const Tensor& b, bool fp
   return x.numel() / W.size(1) < 0x7fffff00LL && weights_ok({W}, {b}, x, fp32);
 }
 
+bool mlp_supported(const Tensor& x, const Tensor& W1, const Tensor& b1, const Tensor& W2, const Tensor& b2) {
+  return linear_supported(x, W1, b1, false) && plain({W2, b2}) && W2.dim() == 2 && W2.size(1) == W1.size(0) && weights_ok({W2}, {b2}, x, false);
+}
+
 Tensor linear(const Tensor& x, const Tensor& W, const Tensor& b, bool fp32) {
   c10::cuda::CUDAGuard guard(x.device());
   const bool need = at::GradMode::is_enabled() && (x.requires_grad() || W.requires_grad() || b.requires_grad());
@@ -872,5 +876,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("linear_supported", &linear_supported);
   m.def("linear", &linear);
+  m.def("mlp_supported", &mlp_supported);
   m.def("mlp", &mlp);
 }

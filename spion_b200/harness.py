@@ -14,7 +14,7 @@ import torch
 import torch.nn as nn
 
 from . import dp
-from .attention import Attention
+from .attention import Attention, no_global_hooks, untouched
 from .pattern import discover_layers
 
 
@@ -82,6 +82,7 @@ class TransformerLayer(nn.Module):
         Linear = nn.Linear
         if config.get("native") and config.get("fused_bias_grad", True):
             from .layernorm import BiasGradLinear as Linear
+        self.mlp_types = (Linear, nn.GELU, nn.Dropout, Linear, nn.Dropout)
         self.fuse_mlp = Linear is not nn.Linear
         self.mlpblock = nn.Sequential(Linear(dim, hid), nn.GELU(), nn.Dropout(p), Linear(hid, dim), nn.Dropout(p))
 
@@ -93,13 +94,24 @@ class TransformerLayer(nn.Module):
     def feed_forward(self, n2):
         """The feed-forward block; under mixed precision and without active dropout its two products run with the activation
         between them inside the kernels."""
-        lin1, drop, lin2 = self.mlpblock[0], self.mlpblock[2], self.mlpblock[3]
-        if self.fuse_mlp and torch.is_autocast_enabled() and torch.get_autocast_dtype("cuda") == torch.bfloat16 \
-                and (not self.training or drop.p == 0):
+        if self.fuse_mlp and torch.is_autocast_enabled() and torch.get_autocast_dtype("cuda") == torch.bfloat16 and self._mlp_is_plain():
             from ._ops import ops
-            if ops.linear_supported(n2, lin1.weight, lin1.bias, False) and lin2.in_features % 32 == 0 and lin2.out_features % 32 == 0:
-                return ops.mlp(n2, lin1.weight, lin1.bias, lin2.weight, lin2.bias)
+            lin1, lin2 = self.mlpblock[0], self.mlpblock[3]
+            args = (n2, lin1.weight, lin1.bias, lin2.weight, lin2.bias)
+            if ops.mlp_supported(*args):
+                return ops.mlp(*args)
         return self.mlpblock(n2)
+
+    def _mlp_is_plain(self) -> bool:
+        """The block is what __init__ made, nothing in it replaced or hooked, and no dropout of it is active."""
+        block = self.mlpblock
+        if not (no_global_hooks() and untouched(block, (nn.Sequential,)) and len(block) == len(self.mlp_types)):
+            return False
+        if not all(untouched(m, (t,)) for m, t in zip(block, self.mlp_types)):
+            return False
+        lin1, act, drop1, lin2, drop2 = block
+        return act.approximate == "none" and lin1.bias is not None and lin2.bias is not None \
+            and not any(d.training and d.p > 0 for d in (drop1, drop2))
 
     def forward_add_norm(self, X, Xn, mask, mat, next_norm):
         """The same layer with each residual addition done inside the normalisation that follows it

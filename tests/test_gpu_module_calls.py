@@ -338,3 +338,52 @@ def test_hooks_and_replacements_of_the_attention_module(kind, dense):
     assert calls[-1] == "other"
     setattr(layer, name, inner)
     assert torch.equal(run_layer(layer, kind, x, keys, mat), want)
+
+
+@pytest.mark.parametrize("what", ["hook", "activation", "approximate", "second layer in bf16", "no bias", "dropout of its own"])
+def test_the_fused_feed_forward_serves_the_block_as_it_was_made(what):
+    """Anything hooked, replaced or switched on in the block runs; the reference is the block called as the module it is."""
+    from spion_b200 import harness
+    cfg = harness.task_config("text", B, dtype="bf16")
+    cfg.update(max_seq_len=L, dropout_prob=0.0)
+    torch.manual_seed(0)
+    layer = harness.TransformerLayer(cfg).cuda()
+    block, x, calls = layer.mlpblock, torch.randn(B, L, 64, device="cuda"), []
+    if what == "hook":
+        for m in block:
+            m.register_forward_hook(lambda m, *_: calls.append(type(m).__name__))
+    elif what == "activation":
+        block[1] = torch.nn.ReLU()
+    elif what == "approximate":
+        block[1] = torch.nn.GELU(approximate="tanh")
+    elif what == "second layer in bf16":
+        block[3].to(torch.bfloat16)
+    elif what == "no bias":
+        block[3].bias = None
+    else:
+        layer.eval()
+        block[2].p = 1.0
+        block[2].train()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        got, want = layer.feed_forward(x), block(x)
+    assert torch.equal(got, want)
+    if what == "hook":
+        assert calls[:5] == ["BiasGradLinear", "GELU", "Dropout", "BiasGradLinear", "Dropout"]
+    if what == "dropout of its own":
+        assert torch.equal(got, block[3].bias.to(got.dtype).expand_as(got))
+
+
+def test_the_fused_feed_forward_saves_all_it_reads():
+    from spion_b200 import harness
+    cfg = harness.task_config("text", B, dtype="bf16")
+    cfg.update(max_seq_len=L, dropout_prob=0.0)
+    layer = harness.TransformerLayer(cfg).cuda()
+    x = torch.randn(B, L, 64, device="cuda", requires_grad=True)
+    grads = lambda y: torch.autograd.grad(y.float().square().sum(), [x] + list(layer.mlpblock.parameters()))
+    sizes = []
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = grads(layer.feed_forward(x))
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: (sizes.append(t.numel()), t.cpu())[1], lambda t: t.cuda()):
+            y = layer.feed_forward(x)
+    same(grads(y), want)
+    assert sum(sizes) >= B * L * (64 + 2 * 128)
