@@ -227,11 +227,13 @@ void check_operand(const Context& c, const Tensor& t, const char* name) {
     throw Failure(std::string(name) + " is on " + t.device().str() + ", the module's context is on cuda:" + std::to_string(c.device));
 }
 
-// key-padding mask [B, L] of 1 / 0 -> penalty per (b,h) matrix [BH, L]
+// key-padding mask [B, L] of 1 / 0 -> penalty per (b,h) matrix [BH, L].  The drop-in modules expand a mask of one sequence
+// or of one key.
 Tensor penalty(const Context& c, const Tensor& mask, const Tensor& like, void* st) {
-  if (!mask.defined() || mask.dim() != 2 || mask.size(0) != c.B || mask.size(1) != c.L)
+  auto fits = [&](int i, int64_t n) { return mask.size(i) == n || (c.mode != NATIVE && mask.size(i) == 1); };
+  if (!mask.defined() || mask.dim() != 2 || !fits(0, c.B) || !fits(1, c.L))
     throw Failure("key-padding mask must have shape (" + std::to_string(c.B) + ", " + std::to_string(c.L) + ")");
-  Tensor m = mask.to(like.device(), at::kFloat).contiguous();
+  Tensor m = mask.to(like.device(), at::kFloat).expand({c.B, c.L}).contiguous();
   Tensor pen = at::empty({c.B, c.H, c.L}, like.options().dtype(at::kFloat));
   check(spion_expand_keypad(pf(m), (int)c.B, (int)c.H, (int)c.L, (float*)pen.data_ptr(), st), "spion_expand_keypad");
   return pen;

@@ -387,3 +387,18 @@ def test_the_fused_feed_forward_saves_all_it_reads():
             y = layer.feed_forward(x)
     same(grads(y), want)
     assert sum(sizes) >= B * L * (64 + 2 * 128)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_key_padding_masks_of_one_sequence(kind, dense):
+    """The drop-in layers broadcast them; the native ones refuse them."""
+    from spion_b200._lib import SpionError
+    x, keys = make_inputs()
+    layer, mat = make_layer(kind, dense), None if dense else make_mask(12)
+    for small in (keys[1:], keys[:, :1]):
+        if KINDS[kind][0]:
+            with pytest.raises(SpionError, match="key-padding mask"):
+                run_layer(layer, kind, x, small, mat)
+        else:
+            assert torch.equal(run_layer(layer, kind, x, small, mat), run_layer(layer, kind, x, small.expand(B, L).contiguous(), mat))
