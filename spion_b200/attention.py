@@ -96,8 +96,6 @@ class Attention(nn.Module):
             if not attn_handle:
                 raise _lib.SpionError("init() of the dense attention library returned NULL")
             self.attn = Dense(config, attn_cpp, attn_handle)
-            self._dense_ctx = _ops.make_context(attn_handle, _ops.DROPIN_DENSE, config["batch_size"], self.num_head, self.seq_len,
-                                                self.head_dim, torch.cuda.current_device(), False, self.with_keypad)
 
         self.ff = Linear(self.num_head * self.head_dim, self.dim)
 
@@ -167,7 +165,7 @@ class Attention(nn.Module):
             elif mat is None:
                 call = None
                 if untouched(self.attn, _DROPIN_DENSE) and no_global_hooks():
-                    call = _ops.ops.attention(self._dense_ctx, Q.float(), K.float(), V.float(), mask if self.with_keypad else None)
+                    call = _ops.ops.attention(self.attn.attn_func.context(), Q.float(), K.float(), V.float(), mask if self.with_keypad else None)
                 if call is not None:
                     attn_out, attn = call[0], call[1].permute(0, 1, 3, 2)
                 else:

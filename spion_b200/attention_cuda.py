@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, _ops
 from ._lib import lib, ptr
 from .attention_blockcuda import _call
 
@@ -67,6 +67,11 @@ def make_dense_function(config, attn_cpp, attn_handle, with_keypad: bool):
                   ptr(s1), ptr(s1), ptr(s3), ptr(dq), ptr(dk), ptr(dv))
             return dq.permute(0, 1, 3, 2), dk.permute(0, 1, 3, 2), dv.permute(0, 1, 3, 2), None
 
+    # the same context for a caller that goes through the native host path (attention.Attention).  It belongs to the function, not to
+    # the modules that share it: a module can be copied.
+    device = torch.cuda.current_device() if torch.cuda.is_available() else 0
+    native = _ops.make_context(handle.value, _ops.DROPIN_DENSE, batch_size, num_heads, seq_len, emb_dim, device, False, with_keypad)
+    AttnFunction.context = staticmethod(lambda: native)
     return AttnFunction
 
 

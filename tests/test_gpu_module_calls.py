@@ -402,3 +402,18 @@ def test_key_padding_masks_of_one_sequence(kind, dense):
                 run_layer(layer, kind, x, small, mat)
         else:
             assert torch.equal(run_layer(layer, kind, x, small, mat), run_layer(layer, kind, x, small.expand(B, L).contiguous(), mat))
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_a_drop_in_layer_can_be_copied(dense):
+    """copy.deepcopy, as averaged models do: the copy shares the attention library's handle and has weights of its own."""
+    import copy
+    kind = "drop-in"
+    x, keys = make_inputs()
+    layer, mat = make_layer(kind, dense), None if dense else make_mask(13)
+    other = copy.deepcopy(layer)
+    want = run_layer(layer, kind, x, keys, mat)
+    assert torch.equal(run_layer(other, kind, x, keys, mat), want)
+    with torch.no_grad():
+        other.W_v.weight.zero_()
+    assert torch.equal(run_layer(layer, kind, x, keys, mat), want)
