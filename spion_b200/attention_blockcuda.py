@@ -24,25 +24,19 @@ from .pattern import pattern_from_mask
 
 
 class _CsrCache:
-    """Element CSR of the most recent mask tensor, keyed on storage pointer and version.  The keyed
-    tensor is kept alive, so its address cannot be given to a different mask while the key is in use."""
+    """Element CSR of the most recent mask tensor (see MaskKey in csrc/torch_ops.cpp)."""
 
     def __init__(self, block_size: int, on_new=None):
         self.block_size = block_size
-        self.key = None
-        self.ref = None
-        self.version = -1
+        self.key = _ops.ops.MaskKey()
         self.value = None
         self.on_new = on_new          # called whenever new arrays replace the cached ones
 
     def get(self, mat: torch.Tensor):
-        if mat is self.ref and mat._version == self.version:
-            return self.value
-        key = (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device))
-        if key != self.key:
+        if not self.key.matches(mat):
             pat = pattern_from_mask(mat, self.block_size)
-            sum_mat, offsets, columns, nnz = pat.element_csr(1)
-            self.key, self.ref, self.version, self.value = key, mat, mat._version, (sum_mat, offsets, columns, nnz)
+            self.value = pat.element_csr(1)
+            self.key.set(mat)
             if self.on_new is not None:
                 self.on_new()
         return self.value

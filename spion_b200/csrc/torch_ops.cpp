@@ -204,6 +204,21 @@ std::string shape_str(const Tensor& t) {
   return s + ")";
 }
 
+// Names the contents of a mask tensor, so that the structure derived from it can be kept: storage, view of it and version.  The alias
+// keeps the storage alive (its address cannot be handed to another mask) and shares the version counter.
+struct MaskKey {
+  Tensor alias;
+  int64_t version = -1;
+  bool matches(const Tensor& t) const {
+    return alias.defined() && t.data_ptr() == alias.data_ptr() && (int64_t)t._version() == version && t.sizes() == alias.sizes() &&
+           t.strides() == alias.strides() && t.scalar_type() == alias.scalar_type() && t.device() == alias.device();
+  }
+  void set(const Tensor& t) {
+    alias = t.detach();
+    version = (int64_t)t._version();
+  }
+};
+
 // native contexts: a new block mask (uint8 [nb, nb] on the context's device, owned by the caller's module and never changed)
 void set_pattern(const ContextPtr& c, const Tensor& mask, int64_t bs) {
   py::gil_scoped_release nogil;
@@ -866,6 +881,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("needs_scratch", &Context::needs_scratch).def_readwrite("owned", &Context::owned)
       .def_readwrite("nnz", &Context::nnz)
       .def_readwrite("sum_mat", &Context::sum_mat).def_readwrite("offsets", &Context::offsets).def_readwrite("columns", &Context::columns);
+  py::class_<MaskKey>(m, "MaskKey").def(py::init<>()).def("matches", &MaskKey::matches).def("set", &MaskKey::set);
   // None, unless `inside` (an autograd function that stands for the call), where something wants to see the call (plain())
   m.def("attention", [](const ContextPtr& c, const Tensor& q, const Tensor& k, const Tensor& v, const optional<Tensor>& mask, bool inside) -> py::object {
     if (!inside && !plain({q, k, v})) return py::none();

@@ -77,9 +77,7 @@ class BlockSparseAttention(nn.Module):
         self.recompute = self.fused and (recompute is None or bool(recompute))
         self.last = None
         self.nnzb = -1
-        self._mask_key = None
-        self._mask_ref = None
-        self._mask_version = -1
+        self._mask_key = _ops.ops.MaskKey()
 
     # settings the native host path reads: kept in its context
     @property
@@ -117,10 +115,7 @@ class BlockSparseAttention(nn.Module):
             self.recompute = self._recompute_pays()
         from .pattern import pattern_from_mask
         self._pattern = pattern_from_mask(m8, self.bs)          # block CSR for the helpers above
-        # The key names the tensor by address and version; the tensor itself is kept alive so that the
-        # address cannot be handed to another mask while the key is in use.
-        self._mask_key = (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device))
-        self._mask_ref, self._mask_version = mat, mat._version
+        self._mask_key.set(mat)
         return self.nnzb
 
     def _recompute_pays(self) -> bool:
@@ -189,9 +184,8 @@ class BlockSparseAttention(nn.Module):
     # ------------------------------------------------------------------ call
     def use_mask(self, mat) -> None:
         """Make ``mat`` the current mask unless it already is (None: keep the current one)."""
-        if mat is not None and not (mat is self._mask_ref and mat._version == self._mask_version):
-            if (mat.data_ptr(), mat._version, tuple(mat.shape), str(mat.device)) != self._mask_key:
-                self.set_mask(mat)
+        if mat is not None and not self._mask_key.matches(mat):
+            self.set_mask(mat)
         if self.nnzb < 0:
             raise _lib.SpionError("no block mask set (call set_mask or pass mat)")
 

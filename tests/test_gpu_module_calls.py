@@ -417,3 +417,18 @@ def test_a_drop_in_layer_can_be_copied(dense):
     with torch.no_grad():
         other.W_v.weight.zero_()
     assert torch.equal(run_layer(layer, kind, x, keys, mat), want)
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+def test_masks_that_share_an_address(kind):
+    """A mask and its transpose, and a mask tensor that has been given other storage, are different masks."""
+    x, keys = make_inputs()
+    mat = make_mask(14, 0.4)
+    mat[0, 3], mat[3, 0] = 1, 0
+    fresh = lambda m: run_layer(make_layer(kind), kind, x, keys, m.clone())
+    layer = make_layer(kind)
+    assert torch.equal(run_layer(layer, kind, x, keys, mat), fresh(mat))
+    assert torch.equal(run_layer(layer, kind, x, keys, mat.t()), fresh(mat.t()))
+    run_layer(layer, kind, x, keys, mat)
+    mat.data = make_mask(15, 0.9)
+    assert torch.equal(run_layer(layer, kind, x, keys, mat), fresh(mat))
