@@ -80,6 +80,8 @@ def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select
     for A in maps:
         if not A.is_cuda:
             raise ValueError("discover_pattern needs the attention map on the GPU (there is no CPU path)")
+        if A.device != maps[0].device:
+            raise ValueError(f"the maps of one call are on different devices, {maps[0].device} and {A.device}")
     maps = [A.detach().to(torch.float32).contiguous() for A in maps]
     L = maps[0].shape[0]
     for A in maps:

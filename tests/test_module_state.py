@@ -21,3 +21,15 @@ def test_mask_key_tells_masks_apart():
     mat.data = torch.zeros(4, 4)                        # the key holds on to the storage it names
     others = [torch.empty(4, 4) for _ in range(64)]
     assert all(t.data_ptr() != old for t in others) and not any(key.matches(t) for t in others)
+
+
+def test_discovery_refuses_maps_of_several_devices():
+    """One launch reads all maps of a call."""
+    from types import SimpleNamespace
+
+    import pytest
+
+    from spion_b200 import pattern
+    maps = [SimpleNamespace(is_cuda=True, device=torch.device("cuda", i)) for i in (0, 1)]
+    with pytest.raises(ValueError, match="different devices"):
+        pattern._discover(maps, 64, 0.9, "diag", 31, "paths", 0)
