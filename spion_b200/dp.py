@@ -79,13 +79,17 @@ class FlatGradBucket:
         for t, g in self._pieces:
             t.grad = g
 
+    def _in_pieces(self, p) -> bool:
+        return p.numel() > self._most and p.is_contiguous()
+
     def pieces(self, most: int = 8192):
         """The parameters for an elementwise optimizer, the large ones as views of at most ``most`` elements that share their
         storage, each with its gradient in the bucket.  Multi-tensor kernels give a block 65536 elements of one tensor,
         so an embedding table was four blocks' serial work (AdamW 71 us a step; in pieces of 8192 25)."""
         out = []
+        self._most = most
         for p, v in zip(self.params, self.views):
-            if p.numel() <= most or not p.is_contiguous():
+            if not self._in_pieces(p):
                 out.append(p)
                 continue
             for t, g in zip(p.detach().view(-1).split(most), v.view(-1).split(most)):
@@ -93,6 +97,39 @@ class FlatGradBucket:
                 self._pieces.append((t, g))
                 out.append(t)
         return out
+
+    def state_by_parameter(self, opt):
+        """Let ``opt``, an optimizer over ``pieces()``, write and read its state dict with one entry per parameter, as an optimizer
+        over the parameters themselves does: checkpoints are exchangeable between the two."""
+        spans, at = [], 0                                  # pieces of each parameter
+        for p in self.params:
+            n = len(p.detach().view(-1).split(self._most)) if self._in_pieces(p) else 1
+            spans.append((at, n))
+            at += n
+
+        def merge(_, state):
+            old, new = state["state"], {}
+            for i, (p, (first, n)) in enumerate(zip(self.params, spans)):
+                if first in old:
+                    new[i] = {k: torch.cat([old[first + x][k].reshape(-1) for x in range(n)]).view(p.shape)
+                              if torch.is_tensor(v) and v.dim() and n > 1 else v for k, v in old[first].items()}
+            groups = [dict(g, params=list(range(len(spans)))) for g in state["param_groups"]]
+            return dict(state, state=new, param_groups=groups)
+
+        def split(_, state):
+            if [len(g["params"]) for g in state["param_groups"]] != [len(spans)]:
+                raise ValueError("the optimizer state is not that of these parameters in one group")
+            old, new = state["state"], {}
+            for i, (first, n) in enumerate(spans):
+                if i in old:
+                    for x in range(n):
+                        new[first + x] = {k: v.reshape(-1).split(self._most)[x] if torch.is_tensor(v) and v.dim() and n > 1
+                                          else (v.clone() if torch.is_tensor(v) else v) for k, v in old[i].items()}
+            groups = [dict(g, params=list(range(at))) for g in state["param_groups"]]
+            return dict(state, state=new, param_groups=groups)
+
+        opt.register_state_dict_post_hook(merge)
+        opt.register_load_state_dict_pre_hook(split)
 
     def zero(self):
         self.flat.zero_()

@@ -205,6 +205,7 @@ class Trainer:
         self.model = Classifier(config).to(self.device)
         self.bucket = dp.FlatGradBucket(self.model.parameters())
         self.opt = torch.optim.AdamW(self.bucket.pieces(), lr=lr, weight_decay=0.0, capturable=True, fused=True)
+        self.bucket.state_by_parameter(self.opt)
         self.mat_lst = None
         self.patterns = None
         self._graph = None
