@@ -71,8 +71,8 @@ int spion_set_stream(spion_ctx* ctx, void* cuda_stream);
  * that cannot run the shape gives UNSUPPORTED. */
 int spion_set_engine(spion_ctx* ctx, int engine);
 
-/* Reads the context's device status word (synchronises the stream).  Non-zero means a
- * bounded wait inside a kernel gave up; the word is cleared. */
+/* Reads the context's device status word and that of the linear layers on its device (synchronises the
+ * stream).  Non-zero means a bounded wait inside a kernel gave up; the words are cleared. */
 int spion_check_device_status(spion_ctx* ctx);
 
 /* Operand layout of the native (_ex / _fused) calls on the tcgen05 engine.
@@ -432,8 +432,11 @@ int spion_linear_backward_input(const spion_tokens* dY, const float* const* W, i
 long long spion_linear_workspace_floats(long long T, int in_features, int out_features, int fp32);
 int spion_linear_backward_weight(const spion_tokens* dY, const spion_tokens* X, int fp32, float* dW, float* db,
                                  float* workspace, long long T, int in_features, int out_features, void* cuda_stream);
-/* SPION_ERR_TIMEOUT when a bounded wait of these kernels has given up since the last reset (synchronises the device). */
+/* SPION_ERR_TIMEOUT when a bounded wait of these kernels has given up since the last reset (synchronises the device).  Until then
+ * every call of them returns without writing its results. */
 int spion_linear_status(int reset);
+/* Failure-path self-test that faults nothing, as spion_selftest_bounded_wait: the status word is set afterwards. */
+int spion_linear_selftest_bounded_wait(long long limit_cycles, void* cuda_stream);
 
 #ifdef __cplusplus
 }

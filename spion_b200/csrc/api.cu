@@ -167,15 +167,17 @@ extern "C" int spion_set_engine(spion_ctx* c, int engine) {
 
 extern "C" int spion_check_device_status(spion_ctx* c) {
   if (!c) return SPION_ERR_ARG;
+  DeviceGuard guard(c->device);
   int word = 0;
   SPION_CUDA_TRY(cudaMemcpyAsync(&word, c->status_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   SPION_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  const int linear = linear_status(1, c->stream);       // the layers around the attention share its stream
   if (word != 0) {
     SPION_CUDA_TRY(cudaMemsetAsync(c->status_dev, 0, sizeof(int), c->stream));
     fprintf(stderr, "spion_b200: device status word = 0x%x (a bounded wait gave up)\n", word);
     return SPION_ERR_TIMEOUT;
   }
-  return SPION_OK;
+  return linear;
 }
 
 extern "C" int spion_csr_arrays_are_stable(spion_ctx* c, int stable) {

@@ -25,7 +25,9 @@ using namespace tc;
 
 namespace {
 
-__device__ int g_lin_status;              // set by a bounded wait that gave up
+// Set by a bounded wait that gave up.  The linear layers have no context of their own: one word per device; launches after it
+// leave at once, as those of the attention kernels do, until spion_check_device_status or spion_linear_status has reported it.
+__device__ int g_lin_status;
 
 // Tokens x features, up to three equally wide matrices side by side, row-major or split into heads [T / L, heads, L, d].
 // Row-major is the same with one head of width `per` and one sequence of all tokens.
@@ -173,9 +175,11 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
 
   const int ntiles = (a.T + 127) >> 7;
   const int G_x = (int)gridDim.x;
+  __shared__ int s_abort;
 
   if (warp == LG_LOADERS) {
     if (lane == 0) {
+      s_abort = *reinterpret_cast<volatile int*>(&g_lin_status);
       for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, LG_LOADERS); mbar_init(empty + 8 * i, 1); }
       for (int i = 0; i < 2; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 8); }
       fence_barrier_init();
@@ -269,6 +273,12 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *slot_ptr;
+  if (s_abort != 0) {
+    if (A_BF16) cp_async_wait<0>();
+    __syncthreads();
+    if (warp == LG_LOADERS) tmem_dealloc(tmem, 512u);
+    return;
+  }
 
   if (warp < LG_LOADERS) {
     // ------------------------------------------------------------------ loaders
@@ -508,9 +518,11 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
   float* sdb_ptr = reinterpret_cast<float*>(smem_raw + (sdb - sbase));        // [8 warps][256]
   const int ntiles = (a.T + 63) >> 6;
   const int G_x = (int)gridDim.x;
+  __shared__ int s_abort;
 
   if (warp == LG_LOADERS) {
     if (lane == 0) {
+      s_abort = *reinterpret_cast<volatile int*>(&g_lin_status);
       for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, LG_LOADERS); mbar_init(empty + 8 * i, 1); }
       mbar_init(acc_done, 1);
       fence_barrier_init();
@@ -523,6 +535,11 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *slot_ptr;
+  if (s_abort != 0) {
+    __syncthreads();
+    if (warp == LG_LOADERS) tmem_dealloc(tmem, 512u);
+    return;
+  }
 
   if (warp < LG_LOADERS) {
     const int lrow = tid >> 3, lc8 = tid & 7;
@@ -901,11 +918,44 @@ extern "C" int spion_linear_supported(int in_features, int out_features, int fp3
          plan_wgrad(sp, out_features, in_features, &nc, &kc, &st, &smem);
 }
 
-extern "C" int spion_linear_status(int reset) {
+int linear_status(int reset, cudaStream_t st) {
   int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_lin_status, sizeof(int)) != cudaSuccess) return SPION_ERR_CUDA;
-  if (reset && v) { const int z = 0; if (cudaMemcpyToSymbol(g_lin_status, &z, sizeof(int)) != cudaSuccess) return SPION_ERR_CUDA; }
-  return v == 0 ? SPION_OK : SPION_ERR_TIMEOUT;
+  SPION_CUDA_TRY(cudaMemcpyFromSymbolAsync(&v, g_lin_status, sizeof(int), 0, cudaMemcpyDeviceToHost, st));
+  SPION_CUDA_TRY(cudaStreamSynchronize(st));
+  if (v == 0) return SPION_OK;
+  if (reset) {
+    void* word = nullptr;
+    SPION_CUDA_TRY(cudaGetSymbolAddress(&word, g_lin_status));
+    SPION_CUDA_TRY(cudaMemsetAsync(word, 0, sizeof(int), st));
+    SPION_CUDA_TRY(cudaStreamSynchronize(st));
+  }
+  fprintf(stderr, "spion_b200: status word of the linear layers = 0x%x (a bounded wait gave up)\n", v);
+  return SPION_ERR_TIMEOUT;
+}
+
+extern "C" int spion_linear_status(int reset) {
+  SPION_CUDA_TRY(cudaDeviceSynchronize());               // the layers may run on streams that the copy below is not ordered after
+  return linear_status(reset, 0);
+}
+
+// One CTA waits, with a limit, on a barrier that nothing arrives on.
+__global__ void k_lin_wait_selftest(long long limit_cycles) {
+  __shared__ __align__(8) unsigned long long bar_storage;
+  const uint32_t bar = smem_u32(&bar_storage);
+  if (threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  const bool ok = __syncthreads_and(mbar_wait_limit(bar, 0, limit_cycles));
+  if (!ok && threadIdx.x == 0) report(&g_lin_status, ERR_LOAD_WAIT);
+}
+
+extern "C" int spion_linear_selftest_bounded_wait(long long limit_cycles, void* cuda_stream) {
+  if (limit_cycles < 1 || limit_cycles > 2000000000LL) return SPION_ERR_ARG;
+  k_lin_wait_selftest<<<1, 128, 0, (cudaStream_t)cuda_stream>>>(limit_cycles);
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
 }
 
 extern "C" int spion_linear_forward(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,

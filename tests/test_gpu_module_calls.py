@@ -432,3 +432,26 @@ def test_masks_that_share_an_address(kind):
     run_layer(layer, kind, x, keys, mat)
     mat.data = make_mask(15, 0.9)
     assert torch.equal(run_layer(layer, kind, x, keys, mat), fresh(mat))
+
+
+def test_a_wait_of_a_linear_layer_that_gave_up_is_reported():
+    """By the check of the attention module in the same layer; until then the linear kernels leave at once."""
+    from spion_b200._lib import SpionError, check, lib
+    from spion_b200.layernorm import BiasGradLinear
+    kind = "native bf16"
+    x, keys = make_inputs()
+    layer, mat, lin = make_layer(kind), make_mask(16), BiasGradLinear(64, 64).cuda()
+    want, want_lin = run_layer(layer, kind, x, keys, mat), lin(x)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()                             # a non-blocking stream: no order with the legacy one
+    with torch.cuda.stream(stream):
+        check(lib.spion_linear_selftest_bounded_wait(1000, stream.cuda_stream))
+        assert lib.spion_linear_status(0) != 0
+        grads = torch.autograd.grad(lin(x).sum(), list(lin.parameters()))      # returns, whatever it left in its buffers
+        del grads
+    torch.cuda.synchronize()
+    with pytest.raises(SpionError, match="timed out"):
+        layer.block_attn.check_device_status()
+    layer.block_attn.check_device_status()
+    assert lib.spion_linear_status(0) == 0
+    assert torch.equal(lin(x), want_lin) and torch.equal(run_layer(layer, kind, x, keys, mat), want)
