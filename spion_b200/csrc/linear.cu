@@ -12,9 +12,10 @@
 // Precision.  bf16 mode: operands rounded to bf16, fp32 accumulation (what mixed precision asks for).  fp32 mode: every fp32
 // operand is split into three bf16 parts (8 + 8 + 8 significant bits: the split is exact) and the six partial products of
 // weight 2^0, 2^-8 and 2^-16 are accumulated in fp32; the dropped ones are below 2^-25 of the product, i.e. below the rounding
-// of an fp32 multiplication.  In the weight gradient, where a sum runs over thousands of tokens, the leading products go to
-// two accumulators in turn and the small ones to a third, and the partial sums of the CTAs are added in fp32, which keeps
-// the chains short.
+// of an fp32 multiplication.  A sum in tensor memory is truncated at every step, which adds up to a bias of half a unit in the last
+// place per step.  In the weight gradient, where a sum runs over all tokens, the leading products therefore go round as many
+// accumulators as tensor memory holds, the small ones to one of their own, and a CTA takes no more tokens than leave CHAIN
+// steps to each; what the accumulators and the CTAs hold is added in fp32.
 #include <type_traits>
 
 #include "common.cuh"
@@ -498,6 +499,15 @@ struct WgradArgs {
   float* part;              // [gridDim.x][N * K + N]
 };
 
+// Accumulators of a CTA's slice (nlen features of dY, kch chunks of X): sets of columns, two per set at lane offsets 0 and 16 where one
+// needs half of the lanes (M = 64).  fp32 mode: the last one takes the small products.
+struct WgradAcc {
+  int cs, sets, two;
+  __host__ __device__ WgradAcc(int nlen, int kch) : cs((nlen + 63) & ~63), sets(512 / cs), two(kch == 1) {}
+  __host__ __device__ int total() const { return sets << two; }
+  __device__ uint32_t at(int i) const { return two ? (uint32_t)(i >> 1) * cs + ((uint32_t)(i & 1) << 20) : (uint32_t)i * cs; }
+};
+
 constexpr int WG_THREADS = 32 * (LG_LOADERS + 1);
 constexpr uint32_t WCHUNK = 64 * 128;                    // [64 tokens x 64 features] bf16
 
@@ -689,30 +699,33 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
       tc_fence_after();
       const int q = warp & 3, half = warp >> 2;
       const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16);
-      const bool two = ((ntiles - (int)blockIdx.x + G_x - 1) / G_x) > 1;       // both leading accumulators were used
+      const WgradAcc acc(nlen, kch);
+      const int small = acc.total() - 1, used = min(small, (ntiles - (int)blockIdx.x + G_x - 1) / G_x);    // leading ones that were used
       const int m = kch == 1 ? q * 16 + (lane & 15) : q * 32 + lane;           // feature of X
       const bool min_ = (kch == 2 || lane < 16) && m < klen;
       for (int g = half; g < (nlen >> 5); g += 2) {
-        uint32_t v[32], u[32];
+        uint32_t v[32];
         __syncwarp();
-        tmem_ld32(tl + g * 32, v);
-        tmem_ld_wait();
         if (SPLIT == 3) {
-          if (kch == 1) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) u[e] = __shfl_xor_sync(0xffffffffu, v[e], 16);
-          } else {
-            tmem_ld32(tl + 128 + g * 32, u);
+          for (int e = 0; e < 32; ++e) v[e] = 0u;
+          for (int s = 0; s < acc.sets; ++s) {
+            const int i = acc.two ? 2 * s + (lane >> 4) : s;                   // the accumulator in this lane
+            if ((acc.two ? 2 * s : s) >= used && s + 1 < acc.sets) continue;   // none of the set was used
+            uint32_t u[32];
+            tmem_ld32(tl + s * acc.cs + g * 32, u);
             tmem_ld_wait();
-          }
-          if (two) {
+            const bool in = i < used || i == small;
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e]));
+            for (int e = 0; e < 32; ++e) v[e] = in ? __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e])) : v[e];
           }
-          tmem_ld32(tl + 256 + g * 32, u);
+          if (acc.two) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(__shfl_xor_sync(0xffffffffu, v[e], 16)));
+          }
+        } else {
+          tmem_ld32(tl + g * 32, v);
           tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e]));
         }
         if (min_) {
           float* dst = part + (size_t)(n0 + g * 32) * a.K + k0 + m;
@@ -727,15 +740,18 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
     // D[features of X, features of dY]: both operands MN-major, chunks of 64 features SPLIT * WCHUNK apart
     const uint32_t idesc = make_idesc_bf16(kch == 1 ? 64 : 128, nlen, 1, 1);
     const uint64_t D0 = make_smem_desc(sbase, SPLIT * WCHUNK, 1024, LAYOUT_SW128);
-    for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++n) {
+    const WgradAcc acc(nlen, kch);
+    const int leads = SPLIT == 3 ? acc.total() - 1 : 1;
+    int li = 0;                                            // leading accumulator of the tile
+    for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++n, li = li + 1 < leads ? li + 1 : 0) {
       const int st = n % a.nstages;
       ok = warp_wait(full + 8 * st, (uint32_t)(n / a.nstages) & 1u);
       if (!ok) break;
       if (elect_one()) {
         tc_fence_after();
         const uint64_t dd = desc_advance(D0, st * stage), dx = desc_advance(dd, (uint32_t)nch * SPLIT * WCHUNK);
-        const uint32_t lead_set = tmem + (SPLIT == 3 ? (uint32_t)(n & 1) * (kch == 1 ? 16u << 16 : 128u) : 0u), small_set = tmem + 256;
-        const uint32_t acc_l = SPLIT == 3 ? n > 1 : n > 0, acc_s = n > 0;
+        const uint32_t lead_set = tmem + acc.at(li), small_set = tmem + acc.at(leads);
+        const uint32_t acc_l = n >= leads, acc_s = n > 0;
 #pragma unroll
         for (int pr = 0; pr < Prod<SPLIT>::N; ++pr) {
           const bool lead = pr + 1 == Prod<SPLIT>::N;
@@ -885,14 +901,20 @@ bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, size_t* 
   return false;
 }
 
+// CTAs along the tokens: one per SM over all slices; fp32 mode: as many more as keep the chains in tensor memory short (above)
+constexpr int CHAIN = 40;
 int wgrad_grid(long long T, int N, int K, int split) {
   int nc, kc, st;
   size_t smem;
   if (!plan_wgrad(split, N, K, &nc, &kc, &st, &smem)) return 0;
   const int per = ((N + nc - 1) / nc) * ((K + kc - 1) / kc);
   const long long tiles = (T + 63) / 64;
-  int gx = sm_count() / per;
+  long long gx = sm_count() / per;
   if (gx < 1) gx = 1;
+  if (split == 3) {
+    const long long most = (long long)CHAIN * (WgradAcc(nc, kc / 64).total() - 1) / 4;       // tiles of a CTA, four steps each
+    gx *= (tiles + gx * most - 1) / (gx * most);
+  }
   return (int)(gx < tiles ? gx : tiles);
 }
 

@@ -120,3 +120,17 @@ def test_feed_forward_block():
     want = [yd, *torch.autograd.grad(yd, pd, go.double())]
     for a, b in zip(got, want):
         assert _rel(a.detach(), b.detach()) < 1.5e-2          # a chain of up to four roundings to bf16
+
+
+@pytest.mark.parametrize("T,K,N", [(1 << 20, 64, 64), (1 << 18, 64, 192), (1 << 17, 256, 1024)])
+def test_weight_gradient_of_many_tokens(T, K, N):
+    """fp32: the error does not grow with the number of tokens.  Operands of one sign, so that the result is the sum of magnitudes: at
+    most 40 truncated steps of 2^-23 per accumulator, whatever T."""
+    from spion_b200.layernorm import BiasGradLinear
+    lin = BiasGradLinear(K, N).cuda()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, go = torch.rand(T, K, generator=g, device="cuda"), torch.rand(T, N, generator=g, device="cuda")
+    dw, db = torch.autograd.grad(lin(x), [lin.weight, lin.bias], go)
+    assert lib.spion_linear_supported(K, N, 1)
+    assert _rel(dw, go.double().t() @ x.double()) < 40 * 2.0 ** -23
+    assert _rel(db, go.double().sum(0)) < 2e-6
