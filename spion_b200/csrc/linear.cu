@@ -140,6 +140,30 @@ struct GemmArgs {
   float* w_copy;            // or null: the stacked W
 };
 
+// The three parts of an infinity (or of a value that rounds to one in bf16) are not finite themselves, and their products are NaN
+// where an fp32 product may be an infinity or a number.  A finite result has no such operand; the others are formed again as an
+// fp32 sum in ascending order.  They are rare, and a NaN ends the sum.
+__device__ __forceinline__ bool all_finite(float probe) { return probe == 0.f; }      // probe: a sum of 0 * value
+__device__ __noinline__ void redo_outputs(const GemmArgs& a, bool transb, int t, int c, float* dst) {       // token t, outputs c .. c + 31
+  RowIt row;
+  row.init(a.A, t);
+  for (int i = 0; i < 32; ++i) {
+    if (fabsf(dst[i]) <= 3.402823466e38f) continue;
+    const int n = c + i;
+    float s = 0.f;
+    for (int k = 0; k < a.k0 + a.K && s == s; ++k) {
+      const int r = transb ? k : n, m = r / a.wper;      // row of the stacked W
+      const float* w = (m == 0 ? a.W[0] : m == 1 ? a.W[1] : a.W[2]) + (size_t)(r - m * a.wper) * a.wld;
+      s = fmaf(tok_col<const float>(a.A, k)[row.off(a.A)], w[transb ? n : k], s);
+    }
+    if (a.bias[0]) {
+      const int m = n / a.wper;
+      s += (m == 0 ? a.bias[0] : m == 1 ? a.bias[1] : a.bias[2])[n - m * a.wper];
+    }
+    dst[i] = s;
+  }
+}
+
 constexpr int LG_LOADERS = 8;
 constexpr int LG_DEPTH = 4;                              // bf16 operands: stages whose copies are in flight
 constexpr int LG_THREADS = 32 * (LG_LOADERS + 1 + 8);
@@ -464,6 +488,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
           }
         } else {
           float* dst = tok_col<float>(a.Y, c) + orow.off(a.Y);
+          float probe = 0.f;
 #pragma unroll
           for (int x = 0; x < 4; ++x) {
             uint32_t w[8];
@@ -476,7 +501,12 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
               for (int i = 0; i < 8; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) + __uint_as_float(o[i]));
             }
             st_v8(dst + 8 * x, w);
+            if (SPLIT == 3) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) probe = fmaf(__uint_as_float(w[i]), 0.f, probe);
+            }
           }
+          if (SPLIT == 3 && !all_finite(probe)) redo_outputs(a, TRANSB, t, c, dst);
         }
       }
       if (half >= ngroups) {                             // nc == 32: the second half of the warps only hands the buffer back
@@ -510,6 +540,24 @@ struct WgradAcc {
 
 constexpr int WG_THREADS = 32 * (LG_LOADERS + 1);
 constexpr uint32_t WCHUNK = 64 * 128;                    // [64 tokens x 64 features] bf16
+
+// As redo_outputs: features n .. n + 31 of dY by feature k of X, over the tokens of this CTA
+__device__ __noinline__ void redo_gradient(const WgradArgs& a, int n, int k, float* dst) {
+  const int ntiles = (a.T + 63) >> 6;
+  for (int e = 0; e < 32; ++e) {
+    if (fabsf(dst[(size_t)e * a.K]) <= 3.402823466e38f) continue;
+    const float *d = tok_col<const float>(a.dY, n + e), *x = tok_col<const float>(a.X, k);
+    float s = 0.f;
+    for (int tile = blockIdx.x; tile < ntiles && s == s; tile += gridDim.x)
+      for (int t = tile * 64; t < min(a.T, tile * 64 + 64); ++t) {
+        RowIt rd, rx;
+        rd.init(a.dY, t);
+        rx.init(a.X, t);
+        s = fmaf(d[rd.off(a.dY)], x[rx.off(a.X)], s);
+      }
+    dst[(size_t)e * a.K] = s;
+  }
+}
 
 // One CTA per SM and slice of the tokens.  dW^T accumulates in tensor memory over all tokens of the CTA: the chunks of X are one
 // MN-major A operand (M = 64 or 128), those of dY one MN-major B operand (N up to 192), so nothing is transposed.  The bias gradient is summed from the registers the loaders hold.
@@ -729,8 +777,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
         }
         if (min_) {
           float* dst = part + (size_t)(n0 + g * 32) * a.K + k0 + m;
+          float probe = 0.f;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) dst[(size_t)e * a.K] = __uint_as_float(v[e]);
+          for (int e = 0; e < 32; ++e) {
+            dst[(size_t)e * a.K] = __uint_as_float(v[e]);
+            if (SPLIT == 3) probe = fmaf(__uint_as_float(v[e]), 0.f, probe);
+          }
+          if (SPLIT == 3 && !all_finite(probe)) redo_gradient(a, n0 + g * 32, k0 + m, dst);
         }
       }
     }

@@ -134,3 +134,43 @@ def test_weight_gradient_of_many_tokens(T, K, N):
     assert lib.spion_linear_supported(K, N, 1)
     assert _rel(dw, go.double().t() @ x.double()) < 40 * 2.0 ** -23
     assert _rel(db, go.double().sum(0)) < 2e-6
+
+
+@pytest.mark.parametrize("split", [False, True])
+def test_values_that_are_not_finite_in_bf16(split):
+    """fp32: infinities, NaN and numbers above the largest of bf16 give what an fp32 product gives; everything else is as without them."""
+    B, L, H, d, K, nw = 2, 150, 2, 32, 96, 3
+    T, N1 = B * L, H * d
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    P = ctypes.c_void_p
+    st = P(torch.cuda.current_stream().cuda_stream)
+    X, Ws, bs = rnd(T, K), [rnd(N1, K) for _ in range(nw)], [rnd(N1) for _ in range(nw)]
+    shape, lay = ((B, H, L, d), (H, d, L)) if split else ((T, N1), (0, 0, 0))
+    dYs = [rnd(*shape) for _ in range(nw)]
+    big, inf, nan = 3.4e38, float("inf"), float("nan")
+    X[3, 5], X[140, 95], X[141, 0], X[290, 64] = big, inf, -inf, nan
+    Ws[1][7, 33] = -inf
+    flat = [t.view(-1) for t in dYs]
+    flat[0][11], flat[1][4000], flat[2][9000] = inf, big, nan
+    ptrs = lambda ts: (P * 3)(*([t.data_ptr() for t in ts] + [None] * (3 - len(ts))))
+    cat = lambda ts: torch.cat([(t.permute(0, 2, 1, 3).reshape(T, N1) if split else t) for t in ts], 1).double()
+    Ys, dX = [torch.empty(shape, device="cuda") for _ in range(nw)], torch.empty(T, K, device="cuda")
+    N = nw * N1
+    dW, db = torch.empty(N, K, device="cuda"), torch.empty(N, device="cuda")
+    ws = torch.empty(lib.spion_linear_workspace_floats(T, K, N, 1), device="cuda")
+    tx, ty, td, tdx = _tokens([X]), _tokens(Ys, *lay), _tokens(dYs, *lay), _tokens([dX])
+    ref = ctypes.byref
+    check(lib.spion_linear_forward(ref(tx), ptrs(Ws), ptrs(bs), nw, 1, ref(ty), None, T, K, N, st))
+    check(lib.spion_linear_backward_input(ref(td), ptrs(Ws), nw, 1, None, ref(tdx), T, K, N, st))
+    check(lib.spion_linear_backward_weight(ref(td), ref(tx), 1, P(dW.data_ptr()), P(db.data_ptr()), P(ws.data_ptr()), T, K, N, st))
+    W, b, dY = torch.cat(Ws).double(), torch.cat(bs).double(), cat(dYs)
+    for got, want in ((cat(Ys), X.double() @ W.t() + b), (dX.double(), dY @ W), (dW.double(), dY.t() @ X.double())):
+        want = want.float().double()                              # beyond fp32: an infinity
+        # within a factor of two of the largest fp32 number the order of the additions decides whether a sum overflows
+        sure = ~((want.abs() > 1.7e38) & want.isfinite()) & ~((got.abs() > 1.7e38) & got.isfinite())
+        odd = sure & ~want.isfinite()
+        assert odd.any() and ((got == want) | (got.isnan() & want.isnan()))[odd].all()
+        huge, usual = sure & want.isfinite() & (want.abs() > 1e30), sure & (want.abs() <= 1e30)
+        assert ((got - want).abs()[huge] <= 1e-6 * want.abs()[huge]).all()
+        assert ((got - want)[usual].norm() <= 2e-6 * want[usual].norm())
