@@ -432,6 +432,9 @@ int spion_linear_backward_input(const spion_tokens* dY, const float* const* W, i
 long long spion_linear_workspace_floats(long long T, int in_features, int out_features, int fp32);
 int spion_linear_backward_weight(const spion_tokens* dY, const spion_tokens* X, int fp32, float* dW, float* db,
                                  float* workspace, long long T, int in_features, int out_features, void* cuda_stream);
+/* Loads the kernels of the linear layers on the current device (fp32 layers, or those of mixed precision), which their first call
+ * does otherwise. */
+int spion_linear_prepare(int fp32);
 /* SPION_ERR_TIMEOUT when a bounded wait of these kernels has given up since the last reset (synchronises the device).  Until then
  * every call of them returns without writing its results. */
 int spion_linear_status(int reset);

@@ -96,6 +96,7 @@ SIGNATURES = {
     "spion_linear_backward_input": (c_int, [c_void_p] * 2 + [c_int] * 2 + [c_void_p] * 2 + [c_longlong, c_int, c_int, c_void_p]),
     "spion_linear_workspace_floats": (c_longlong, [c_longlong] + [c_int] * 3),
     "spion_linear_backward_weight": (c_int, [c_void_p] * 2 + [c_int] + [c_void_p] * 3 + [c_longlong, c_int, c_int, c_void_p]),
+    "spion_linear_prepare": (c_int, [c_int]),
     "spion_linear_status": (c_int, [c_int]),
     "spion_linear_selftest_bounded_wait": (c_int, [c_longlong, c_void_p]),
     "spion_static_scratch_capacity": (ctypes.c_size_t, []),

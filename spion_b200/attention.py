@@ -98,6 +98,8 @@ class Attention(nn.Module):
             self.attn = Dense(config, attn_cpp, attn_handle)
 
         self.ff = Linear(self.num_head * self.head_dim, self.dim)
+        if torch.cuda.is_available():
+            _lib.check(_lib.lib.spion_linear_prepare(int(self.native_dtype == torch.float32)), "spion_linear_prepare")
 
     def _stages_are_untouched(self, mat) -> bool:
         """The projections and the attention module are what was made here: nothing replaced, no hook that a one-node layer would

@@ -16,6 +16,7 @@
 // place per step.  In the weight gradient, where a sum runs over all tokens, the leading products therefore go round as many
 // accumulators as tensor memory holds, the small ones to one of their own, and a CTA takes no more tokens than leave CHAIN
 // steps to each; what the accumulators and the CTAs hold is added in fp32.
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -852,13 +853,13 @@ __global__ void __launch_bounds__(256) k_lin_reduce(const float* __restrict__ pa
 constexpr size_t SMEM_MAX = 227 * 1024 - 1024;
 
 int sm_count() {
-  static int cached[64] = {0};
+  static std::atomic<int> cached[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (dev < 64 && cached[dev]) return cached[dev];
-  int n = 0;
+  int n = dev < 64 ? cached[dev].load() : 0;
+  if (n) return n;
   if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (dev < 64) cached[dev] = n;
+  if (dev < 64) cached[dev].store(n);
   return n;
 }
 
@@ -905,16 +906,32 @@ bool plan_gemm(int split, bool trans, int K, int N, int* nc, int* nacc, int* sta
   return false;
 }
 
-template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
-int launch_gemm(const GemmArgs& a, size_t smem, cudaStream_t st) {
-  static bool set[64] = {false};
+// Shared-memory opt-in of a kernel, once per device; the call also loads the kernel.  `done` belongs to the kernel.
+template <class K>
+int opt_in(K k, std::atomic<bool> (&done)[64]) {
   int dev = 0;
   SPION_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && done[dev].load(std::memory_order_acquire)) return SPION_OK;
+  SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+  if (dev < 64) done[dev].store(true, std::memory_order_release);
+  return SPION_OK;
+}
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
+int prepare_gemm() {
+  static std::atomic<bool> done[64];
+  return opt_in(k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>, done);
+}
+template <int SPLIT, bool DY_BF16, bool X_BF16>
+int prepare_wgrad() {
+  static std::atomic<bool> done[64];
+  return opt_in(k_lin_wgrad<SPLIT, DY_BF16, X_BF16>, done);
+}
+
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
+int launch_gemm(const GemmArgs& a, size_t smem, cudaStream_t st) {
   auto k = k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>;
-  if (dev >= 64 || !set[dev]) {
-    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-    if (dev < 64) set[dev] = true;
-  }
+  const int rc = prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
+  if (rc) return rc;
   const int ny = (a.N + a.nc - 1) / a.nc;
   const int sms = sm_count(), tiles = (a.T + 127) / 128;
   if (sms < 1) return SPION_ERR_CUDA;
@@ -927,14 +944,9 @@ int launch_gemm(const GemmArgs& a, size_t smem, cudaStream_t st) {
 
 template <int SPLIT, bool DY_BF16, bool X_BF16>
 int launch_wgrad(const WgradArgs& a, int gx, size_t smem, cudaStream_t st) {
-  static bool set[64] = {false};
-  int dev = 0;
-  SPION_CUDA_TRY(cudaGetDevice(&dev));
   auto k = k_lin_wgrad<SPLIT, DY_BF16, X_BF16>;
-  if (dev >= 64 || !set[dev]) {
-    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-    if (dev < 64) set[dev] = true;
-  }
+  const int rc = prepare_wgrad<SPLIT, DY_BF16, X_BF16>();
+  if (rc) return rc;
   k<<<dim3(gx, (a.N + a.nc - 1) / a.nc, (a.K + a.kc - 1) / a.kc), WG_THREADS, smem, st>>>(a);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
@@ -991,6 +1003,20 @@ extern "C" int spion_linear_supported(int in_features, int out_features, int fp3
   return plan_gemm(sp, false, in_features, out_features, &nc, &nacc, &st, &smem) &&
          plan_gemm(sp, true, fp32 ? 64 : out_features, in_features, &nc, &nacc, &st, &smem) &&
          plan_wgrad(sp, out_features, in_features, &nc, &kc, &st, &smem);
+}
+
+extern "C" int spion_linear_prepare(int fp32) {
+  int rc;
+  if (fp32) {
+    if ((rc = prepare_gemm<3, false, false, EPI_NONE, false>()) || (rc = prepare_gemm<3, false, true, EPI_NONE, false>())) return rc;
+    return prepare_wgrad<3, false, false>();
+  }
+  if ((rc = prepare_gemm<1, true, false, EPI_NONE, true>()) || (rc = prepare_gemm<1, false, false, EPI_NONE, true>()) ||
+      (rc = prepare_gemm<1, true, false, EPI_GELU, true>()) || (rc = prepare_gemm<1, false, false, EPI_GELU, true>()) ||
+      (rc = prepare_gemm<1, true, true, EPI_DGELU, true>()) || (rc = prepare_gemm<1, true, true, EPI_NONE, true>()) ||
+      (rc = prepare_gemm<1, true, true, EPI_NONE, false>()) || (rc = prepare_wgrad<1, true, false>()))
+    return rc;
+  return prepare_wgrad<1, true, true>();
 }
 
 int linear_status(int reset, cudaStream_t st) {

@@ -8,6 +8,8 @@
 // conflict-free); a CTA of 256 threads works on 256/(bs/4)^2 consecutive (b,h) matrices of
 // the same block row: they share the mask, so the CTA runs in lock step.  The forward leaves the scaled scores in the P tiles
 // while it forms the row statistics and turns them into probabilities in a second pass.
+#include <atomic>
+
 #include "common.cuh"
 
 namespace {
@@ -503,14 +505,14 @@ template <int BS, int D> constexpr size_t smem_col() { return sizeof(float) * Cf
 
 template <int BS, int D>
 int set_attrs() {
-  static bool done[64] = {};
+  static std::atomic<bool> done[64];
   int dev = 0;
   SPION_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 64 && done[dev]) return SPION_OK;
+  if (dev < 64 && done[dev].load(std::memory_order_acquire)) return SPION_OK;
   SPION_CUDA_TRY(cudaFuncSetAttribute(full_fwd_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(full_bwd_row_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(full_bwd_col_kernel<BS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D>()));
-  if (dev < 64) done[dev] = true;
+  if (dev < 64) done[dev].store(true, std::memory_order_release);
   return SPION_OK;
 }
 

@@ -29,6 +29,8 @@
 // layouts whose tile rows are contiguous (element CSR, block tiles) are accepted.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "common.cuh"
 
 namespace {
@@ -756,16 +758,16 @@ constexpr int SPLIT_WAVES = 4;
 
 template <int BS, int D, int R>
 int set_attrs() {
-  static bool done[64] = {};
+  static std::atomic<bool> done[64];
   int dev = 0;
   SPION_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 64 && done[dev]) return SPION_OK;
+  if (dev < 64 && done[dev].load(std::memory_order_acquire)) return SPION_OK;
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_fwd_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_delta_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D, R>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
-  if (dev < 64) done[dev] = true;
+  if (dev < 64) done[dev].store(true, std::memory_order_release);
   return SPION_OK;
 }
 

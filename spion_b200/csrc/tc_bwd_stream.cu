@@ -538,11 +538,6 @@ static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUte
   using C = Bw<D, SIDE>;
   static_assert(C::SMEM <= 227 * 1024, "shared memory");
   auto k = k_bwd_stream<D, SIDE, SUB>;
-  static bool set[64] = {false};
-  if (c->device >= 64 || !set[c->device]) {
-    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
-    if (c->device < 64) set[c->device] = true;
-  }
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
   k<<<grid, BW_THREADS, C::SMEM, c->stream>>>(a0, a1, f0, f1, a);
@@ -550,6 +545,16 @@ static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUte
   c->launches += 1;
   return SPION_OK;
 }
+
+template <int D>
+static int bw_attrs() {
+  for (auto k : {k_bwd_stream<D, ROW, false>, k_bwd_stream<D, ROW, true>})
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, ROW>::SMEM));
+  for (auto k : {k_bwd_stream<D, COL, false>, k_bwd_stream<D, COL, true>})
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, COL>::SMEM));
+  return SPION_OK;
+}
+int stream_backward_set_attrs(int d) { return d == 64 ? bw_attrs<64>() : bw_attrs<32>(); }
 
 int stream_prepare(spion_ctx* c, TcState* s) {
   const TcView vw = tc_view(c, s);

@@ -749,7 +749,8 @@ bool tc_engine_supports(const spion_ctx* c) {
 }
 
 // Shared-memory opt-ins and resident CTAs of all kernels, once per device and head dimension of the process (about 60 attribute
-// calls, a millisecond: every layer of a model has a context of its own).
+// calls, a millisecond: every layer of a model has a context of its own).  The calls also load the kernels, so that the first pass of
+// a module does not.
 static int kernel_attrs(spion_ctx* c, TcState* s) {
   struct Known { bool have = false; int fwd, row, col, pipe, b32[3]; };
   static std::mutex mutex;
@@ -762,6 +763,8 @@ static int kernel_attrs(spion_ctx* c, TcState* s) {
     if (!rc) rc = fused_set_attrs(s, c->d, c->device);
     if (!rc) rc = mean_map_set_attrs(c->d);
     if (!rc) rc = pipe_set_attrs(s, c->d, c->device);
+    if (!rc) rc = stream_forward_set_attrs(c->d);
+    if (!rc) rc = stream_backward_set_attrs(c->d);
     if (!rc && b32) rc = b32_set_attrs(s, c->device);
     if (rc) return rc;
     k->fwd = s->fwd_ctas; k->row = s->row_ctas; k->col = s->col_ctas; k->pipe = s->pipe_ctas;
@@ -794,9 +797,9 @@ int tc_engine_prepare(spion_ctx* c) {
     int rc = kernel_attrs(c, s);
     if (!rc && device_alloc((void**)&s->delta_ws, (size_t)c->BH * c->L * sizeof(float)) != SPION_OK) rc = SPION_ERR_ALLOC;
     if (!rc && device_alloc((void**)&s->lse_ws, (size_t)c->BH * c->L * sizeof(float)) != SPION_OK) rc = SPION_ERR_ALLOC;
-    if (rc) { delete s; return rc; }
-    s->super = c->bs == 32;
     c->tc = s;
+    if (rc) { tc_engine_release(c); return rc; }
+    s->super = c->bs == 32;
   }
   int rc;
   // decides whether the mask runs on its own blocks (before the super-block set-up)

@@ -439,11 +439,6 @@ static int fs_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUte
   using C = Fs<D>;
   static_assert(C::SMEM <= 227 * 1024 && NG * C::COLS <= 512, "shared or tensor memory");
   auto k = k_fwd_stream<D, KP, SUB, EXACT>;
-  static bool set[64] = {false};
-  if (c->device >= 64 || !set[c->device]) {
-    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
-    if (c->device < 64) set[c->device] = true;
-  }
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
   k<<<grid, FS_THREADS, C::SMEM, c->stream>>>(mq, mk, mv, a);
@@ -467,6 +462,15 @@ static int fs_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUt
   if (keypad) return vw.submask ? fs_launch<D, true, true, false>(c, s, mq, mk, mv, a) : fs_launch<D, true, false, false>(c, s, mq, mk, mv, a);
   return vw.submask ? fs_launch<D, false, true, false>(c, s, mq, mk, mv, a) : fs_launch<D, false, false, false>(c, s, mq, mk, mv, a);
 }
+
+template <int D>
+static int fs_attrs() {
+  for (auto k : {k_fwd_stream<D, false, false, false>, k_fwd_stream<D, true, false, false>, k_fwd_stream<D, false, true, false>,
+                 k_fwd_stream<D, true, true, false>, k_fwd_stream<D, false, false, true>, k_fwd_stream<D, true, false, true>})
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Fs<D>::SMEM));
+  return SPION_OK;
+}
+int stream_forward_set_attrs(int d) { return d == 64 ? fs_attrs<64>() : fs_attrs<32>(); }
 
 int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
                    float* lse) {

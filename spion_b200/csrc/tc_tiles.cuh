@@ -243,6 +243,7 @@ inline int make_operand_map(const spion_ctx* c, TcState* s, CUtensorMap* m, cons
 }
 
 // tc_bwd_stream.cu
+int stream_backward_set_attrs(int d);
 int stream_prepare(spion_ctx* c, TcState* s);              // pattern set: line and pair records of the streaming kernels
 int recompute_backward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const void* O,
                        const void* dO, const float* lse, const float* keypad, void* dQ, void* dK, void* dV);
@@ -252,6 +253,7 @@ int recompute_mean_map(spion_ctx* c, TcState* s, const void* Q, const void* K, c
                        float* A);
 
 // tc_fwd_stream.cu: forward without stored probabilities
+int stream_forward_set_attrs(int d);
 int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
                    float* lse);
 

@@ -455,3 +455,48 @@ def test_a_wait_of_a_linear_layer_that_gave_up_is_reported():
     layer.block_attn.check_device_status()
     assert lib.spion_linear_status(0) == 0
     assert torch.equal(lin(x), want_lin) and torch.equal(run_layer(layer, kind, x, keys, mat), want)
+
+
+def test_modules_of_several_threads():
+    """Modules made and called by several threads at once give what they give one after another."""
+    import threading
+    x, keys = make_inputs()
+    kinds = list(KINDS) * 2
+    masks = [make_mask(20 + i) for i in range(len(kinds))]
+    got, failed = [None] * len(kinds), []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                layer = layers[i]
+                if not KINDS[kinds[i]][0] or KINDS[kinds[i]][1] == "fp32":
+                    layer = make_copy(layer, kinds[i])
+                for _ in range(3):
+                    out = run_layer(layer, kinds[i], x, keys, masks[i])
+                    g = gradients(layer, out, x)
+                got[i] = [out.detach(), *g]
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:
+            failed.append(e)
+
+    def make_copy(layer, kind):                                  # torch's seed is the process's: the weights come from outside
+        native, dtype = KINDS[kind]
+        from spion_b200.attention import Attention
+        cfg = config(native, dtype)
+        other = Attention(cfg).cuda()
+        other.load_state_dict(layer.state_dict())
+        other.reconstruct_for_blocksparse(cfg)
+        return other
+
+    layers = [make_layer(k) for k in kinds]
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(kinds))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    for i, kind in enumerate(kinds):
+        layer = make_layer(kind)
+        out = run_layer(layer, kind, x, keys, masks[i])
+        same(got[i], [out.detach(), *gradients(layer, out, x)])
