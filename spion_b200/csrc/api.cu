@@ -4,14 +4,29 @@
 // Pipelines (reference: Attention::attn_forward / attn_backward, models/block_attn.cu:453-545):
 //   forward   S = Q K^T on the mask  ->  P = sparse row softmax(S)  ->  O = P V
 //   backward  dP = dO V^T on the mask -> dS = softmax'(dP, P) -> dQ = dS K ; dK = dS^T Q ; dV = P^T dO
-#include <new>
-
 #include <mutex>
+#include <new>
+#include <unordered_map>
+#include <vector>
 
 #include "common.cuh"
 
 namespace {
-struct DevicePool { cudaMemPool_t pool; cudaStream_t stream; };
+// The driver gives memory of a pool back to the system at the next synchronisation as soon as it has reserved more than the release
+// threshold, and it counts what is in use: the threshold follows the memory in use, so that up to KEEP of free memory stays.
+constexpr size_t KEEP = 64ull << 20;
+struct DevicePool {
+  cudaMemPool_t pool;
+  cudaStream_t stream;
+  std::mutex mutex;
+  std::unordered_map<void*, size_t> sizes;        // what is in use
+  size_t live = 0;
+  std::vector<void*> waiting;                     // to be freed once the device can be waited for
+  int follow() {
+    uint64_t most = live + KEEP;
+    return cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &most) == cudaSuccess ? SPION_OK : SPION_ERR_CUDA;
+  }
+};
 // the pool of the current device, made on first use; nullptr if that failed
 DevicePool* device_pool() {
   static std::mutex lock;
@@ -24,15 +39,15 @@ DevicePool* device_pool() {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    DevicePool d{};
-    uint64_t keep = 64ull << 20;
-    if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) return nullptr;
-    if (cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking) != cudaSuccess) {
-      cudaMemPoolDestroy(d.pool);
+    DevicePool* d = new (std::nothrow) DevicePool();
+    if (!d) return nullptr;
+    if (cudaMemPoolCreate(&d->pool, &props) != cudaSuccess) { delete d; return nullptr; }
+    if (d->follow() != SPION_OK || cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaMemPoolDestroy(d->pool);
+      delete d;
       return nullptr;
     }
-    pools[dev] = new DevicePool(d);
+    pools[dev] = d;
   }
   return pools[dev];
 }
@@ -41,14 +56,40 @@ DevicePool* device_pool() {
 int device_alloc(void** p, size_t bytes) {
   *p = nullptr;
   DevicePool* d = device_pool();
-  if (!d || cudaMallocFromPoolAsync(p, bytes, d->pool, d->stream) != cudaSuccess) return SPION_ERR_ALLOC;
+  if (!d) return SPION_ERR_ALLOC;
+  std::lock_guard<std::mutex> hold(d->mutex);
+  if (cudaMallocFromPoolAsync(p, bytes, d->pool, d->stream) != cudaSuccess) { *p = nullptr; return SPION_ERR_ALLOC; }
+  try {
+    d->sizes.emplace(*p, bytes);
+  } catch (...) {                                 // out of host memory: nothing may leave a C entry point
+    cudaFreeAsync(*p, d->stream);
+    *p = nullptr;
+    return SPION_ERR_ALLOC;
+  }
+  d->live += bytes;
+  d->follow();
   return cudaStreamSynchronize(d->stream) == cudaSuccess ? SPION_OK : SPION_ERR_ALLOC;   // usable on every stream from here on
 }
 
 void device_free(void* p) {
   if (!p) return;
-  cudaDeviceSynchronize();
-  if (DevicePool* d = device_pool()) cudaFreeAsync(p, d->stream);
+  const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+  if (!idle) cudaGetLastError();                  // a stream of the device is being captured
+  DevicePool* d = device_pool();
+  if (!d) return;
+  std::lock_guard<std::mutex> hold(d->mutex);
+  try {
+    d->waiting.push_back(p);
+  } catch (...) { return; }
+  if (!idle) return;                              // kernels may still use it: freed with the next one
+  for (void* w : d->waiting) {
+    const auto it = d->sizes.find(w);
+    if (it != d->sizes.end()) { d->live -= it->second; d->sizes.erase(it); }
+    cudaFreeAsync(w, d->stream);
+  }
+  d->waiting.clear();
+  d->follow();
+  cudaStreamSynchronize(d->stream);               // what is beyond the threshold goes back now
 }
 
 namespace {

@@ -124,8 +124,9 @@ static inline Pattern ctx_pattern(const spion_ctx* c) {
 // linear.cu: status word of the linear layers on the current device, after the work of a stream
 int linear_status(int reset, cudaStream_t st);
 
-// Device memory of the contexts, from one pool per device that keeps up to 64 MB of what was given back: mapping and unmapping two
-// or three megabytes took 2 to 4 ms of every context's life.  Freeing waits for the device, as cudaFree does.  Any thread.
+// Device memory of the contexts, from one pool per device that keeps up to 64 MB of what was given back, beside what is in use: mapping
+// and unmapping two or three megabytes took 2 to 4 ms of every context's life.  Freeing waits for the device, as cudaFree does (where it
+// cannot, under a capture, the memory is freed later).  Any thread.
 int device_alloc(void** p, size_t bytes);
 void device_free(void* p);
 

@@ -500,3 +500,30 @@ def test_modules_of_several_threads():
         layer = make_layer(kind)
         out = run_layer(layer, kind, x, keys, masks[i])
         same(got[i], [out.detach(), *gradients(layer, out, x)])
+
+
+def test_memory_of_contexts():
+    """With more in use than the pool keeps, what one context gives back is there for the next; in the end all but that goes back."""
+    from spion_b200.native import BlockSparseAttention
+
+    def context(heads):                                          # 2 * 4 bytes of workspace per row and matrix
+        mod = BlockSparseAttention(dict(config(), num_head=heads, max_seq_len=4096), dtype=torch.bfloat16)
+        mod.set_mask(torch.eye(64, device="cuda"))
+        return mod
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    context(1)
+    torch.cuda.empty_cache()
+    start = free()
+    large, small = context(2048), context(256)                   # 134 MB and 17 MB
+    both = free()
+    assert start - both > 100 << 20
+    del small
+    assert free() == both
+    small = context(256)
+    assert free() == both
+    del large, small
+    assert start - free() < 80 << 20
