@@ -4,6 +4,7 @@
 // Pipelines (reference: Attention::attn_forward / attn_backward, models/block_attn.cu:453-545):
 //   forward   S = Q K^T on the mask  ->  P = sparse row softmax(S)  ->  O = P V
 //   backward  dP = dO V^T on the mask -> dS = softmax'(dP, P) -> dQ = dS K ; dK = dS^T Q ; dV = P^T dO
+#include <atomic>
 #include <mutex>
 #include <new>
 #include <unordered_map>
@@ -90,6 +91,17 @@ void device_free(void* p) {
   d->waiting.clear();
   d->follow();
   cudaStreamSynchronize(d->stream);               // what is beyond the threshold goes back now
+}
+
+int sm_count() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  int n = dev < 64 ? cached[dev].load() : 0;
+  if (n) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (dev < 64) cached[dev].store(n);
+  return n;
 }
 
 namespace {

@@ -121,6 +121,9 @@ static inline Pattern ctx_pattern(const spion_ctx* c) {
     }                                                                                 \
   } while (0)
 
+// api.cu: multiprocessors of the current device (0: the query failed)
+int sm_count();
+
 // linear.cu: status word of the linear layers on the current device, after the work of a stream
 int linear_status(int reset, cudaStream_t st);
 

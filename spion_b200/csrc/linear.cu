@@ -852,17 +852,6 @@ __global__ void __launch_bounds__(256) k_lin_reduce(const float* __restrict__ pa
 // ------------------------------------------------------------------------------------------------ host
 constexpr size_t SMEM_MAX = 227 * 1024 - 1024;
 
-int sm_count() {
-  static std::atomic<int> cached[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  int n = dev < 64 ? cached[dev].load() : 0;
-  if (n) return n;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (dev < 64) cached[dev].store(n);
-  return n;
-}
-
 TokMat to_mat(const spion_tokens* t) {
   TokMat m;
   for (int i = 0; i < 3; ++i) m.p[i] = t->ptr[i];

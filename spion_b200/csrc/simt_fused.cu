@@ -802,7 +802,7 @@ int bwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout l
   if (prof) prof_mark(prof, SPION_STAGE_BWD_ROW);
   // Many (b,h) matrices even out columns of different lengths by themselves; below SPLIT_WAVES waves of CTAs the longest
   // column would decide, and there is room for the CTAs that a split column takes.
-  if ((long long)grid.x * grid.y < SPLIT_WAVES * 148LL * Cfg<BS, D, R>::RESIDENT) {
+  if ((long long)grid.x * grid.y < (long long)SPLIT_WAVES * sm_count() * Cfg<BS, D, R>::RESIDENT) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid.x * SPLIT_WAYS, grid.y);
     cfg.blockDim = dim3(Cfg<BS, D, R>::CTA);
@@ -830,13 +830,13 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
          (value_mode == VAL_ELEMCSR || value_mode == VAL_BLOCKTILE);
 }
 
-// With eight rows per thread a block row is one warp (block 32) or four (64).  Up to two warps per scheduler (148 SMs x 4) each of
+// With eight rows per thread a block row is one warp (block 32) or four (64).  Up to two warps per scheduler (four per SM) each of
 // them is a chain of latencies, and half the rows per thread shorten it (16 matrices, L = 1024, d 32, blocks of 32 at 15 %:
 // forward 31 -> 22 us, rows 22 -> 20); above, the larger micro-tile is worth more.
-constexpr long long FEW_WARPS = 148 * 4 * 2;
+constexpr long long FEW_WARPS = 4 * 2;                // per SM
 #define SPION_FUSED_DISPATCH(FN, ...)                                   \
   do {                                                                  \
-    const bool few = (long long)p.nb * BH * p.bs * p.bs / 1024 <= FEW_WARPS; \
+    const bool few = (long long)p.nb * BH * p.bs * p.bs / 1024 <= FEW_WARPS * sm_count(); \
     if (p.bs == 32 && d == 32) return few ? FN<32, 32, 4>(__VA_ARGS__) : FN<32, 32, 8>(__VA_ARGS__); \
     if (p.bs == 32 && d == 64) return few ? FN<32, 64, 4>(__VA_ARGS__) : FN<32, 64, 8>(__VA_ARGS__); \
     if (p.bs == 64 && d == 32) return few ? FN<64, 32, 4>(__VA_ARGS__) : FN<64, 32, 8>(__VA_ARGS__); \
