@@ -955,12 +955,8 @@ bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, size_t* 
   return false;
 }
 
-// CTAs along the tokens: one per SM over all slices; fp32 mode: as many more as keep the chains in tensor memory short (above), and
-// those of the column sums of dY, which a thread adds one after another.  Relative error of dW, db against fp64 (normal operands; in
-// brackets the library product that this replaced): 262144 tokens, 64 x 64 1.7e-7, 1.7e-7 (1.1e-6, 1.7e-7); 64 x 192 5.6e-7, 1.7e-7 (1.3e-6,
-// 3.1e-7); 256 x 1024 5.8e-7, 1.8e-7 (2.2e-6, 2.1e-7).  Operands of one sign, where every truncation adds up: 1.4e-7 (1.5e-7), 9.4e-7
-// (1.9e-7), 9.9e-7 (4.0e-7).
-constexpr int CHAIN = 40, TOKEN_TILES = 32;
+// CTAs along the tokens: one per SM over all slices; fp32 mode: as many more as keep the chains in tensor memory short (above)
+constexpr int CHAIN = 40;
 int wgrad_grid(long long T, int N, int K, int split) {
   int nc, kc, st;
   size_t smem;
@@ -970,8 +966,7 @@ int wgrad_grid(long long T, int N, int K, int split) {
   long long gx = sm_count() / per;
   if (gx < 1) gx = 1;
   if (split == 3) {
-    const long long chain = (long long)CHAIN * (WgradAcc(nc, kc / 64).total() - 1) / 4;      // tiles of four steps
-    const long long most = chain < TOKEN_TILES ? chain : TOKEN_TILES;
+    const long long most = (long long)CHAIN * (WgradAcc(nc, kc / 64).total() - 1) / 4;       // tiles of a CTA, four steps each
     gx *= (tiles + gx * most - 1) / (gx * most);
   }
   return (int)(gx < tiles ? gx : tiles);
