@@ -955,7 +955,10 @@ bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, size_t* 
   return false;
 }
 
-// CTAs along the tokens: one per SM over all slices; fp32 mode: as many more as keep the chains in tensor memory short (above)
+// CTAs along the tokens: one per SM over all slices; fp32 mode: as many more as keep the chains in tensor memory short (above).
+// Relative error of dW and db against fp64, normal operands (in brackets the library's product and reduction in their place): 262144
+// tokens, 64 x 64 1.7e-7, 1.7e-7 (1.1e-6, 1.7e-7); 64 x 192 5.6e-7, 1.7e-7 (1.3e-6, 3.1e-7); 256 x 1024 5.8e-7, 1.8e-7 (2.2e-6, 2.1e-7).
+// dW from operands of one sign, where every truncation adds up: 1.4e-7 (1.5e-7), 9.4e-7 (1.9e-7), 9.9e-7 (4.0e-7).
 constexpr int CHAIN = 40;
 int wgrad_grid(long long T, int N, int K, int split) {
   int nc, kc, st;
