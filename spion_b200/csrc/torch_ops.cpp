@@ -93,20 +93,29 @@ bool aligned32(const Tensor& t) { return ((uintptr_t)t.data_ptr() & 31) == 0; }
 
 struct Weights {                        // up to three stacked linear layers
   std::vector<Tensor> W, b;
-  int n() const { return (int)W.size(); }
-  int in() const { return (int)W[0].size(1); }
-  int out() const { return (int)(W[0].size(0) * W.size()); }
+  const float* copy = nullptr;          // instead of W: the stacked weights of `layers` equal layers
+  int layers = 0, copy_in = 0, copy_out = 0;
+  Weights() {}
+  Weights(std::vector<Tensor> W_, std::vector<Tensor> b_) : W(std::move(W_)), b(std::move(b_)) {}
+  Weights(const float* p, int n_layers, int64_t in_features, int64_t out_features)
+      : copy(p), layers(n_layers), copy_in((int)in_features), copy_out((int)out_features) {}
+  int n() const { return copy ? layers : (int)W.size(); }
+  int in() const { return copy ? copy_in : (int)W[0].size(1); }
+  int out() const { return copy ? copy_out : (int)(W[0].size(0) * W.size()); }
+  const float* at(int i) const { return copy ? copy + (int64_t)i * (copy_out / layers) * copy_in : pf(W[i]); }
 };
 
 // What a mixed-precision backward reads in place of the input and the weights: as under the framework's own autocast, the caller may
 // change both in between.  The forward's kernels write the copies on the way.
 struct Kept {
   Tensor x, w;
+  float* w_to = nullptr;                // where the weights go: w, or a part of a buffer that several layers share
   // x: the input (bf16 input is kept as it is); fp32 layers keep nothing
   Kept() {}
-  Kept(bool need, bool fp32, const Tensor& X, const Weights& l) {
+  Kept(bool need, bool fp32, const Tensor& X, const Weights& l, float* shared = nullptr) {
     if (!need || fp32) return;
-    w = at::empty({l.out(), l.in()}, l.W[0].options());
+    if (!shared) w = at::empty({l.out(), l.in()}, l.W[0].options());
+    w_to = shared ? shared : (float*)w.data_ptr();
     if (X.scalar_type() == at::kFloat) x = at::empty(X.sizes(), X.options().dtype(at::kBFloat16));
   }
 };
@@ -114,12 +123,12 @@ void linear_forward(const spion_tokens& X, const Weights& w, bool fp32, const sp
                     const Kept& kept = Kept()) {
   const float *W[3], *b[3];
   for (int i = 0; i < w.n(); ++i) { W[i] = pf(w.W[i]); b[i] = pf(w.b[i]); }
-  check(spion_linear_forward_keep(&X, W, b, w.n(), fp32, &Y, gelu_out, p(kept.x), (float*)p(kept.w), T, w.in(), w.out(), st),
+  check(spion_linear_forward_keep(&X, W, b, w.n(), fp32, &Y, gelu_out, p(kept.x), kept.w_to, T, w.in(), w.out(), st),
         "spion_linear_forward_keep");
 }
 void linear_backward_input(const spion_tokens& dY, const Weights& w, bool fp32, const void* gelu_in, const spion_tokens& dX, int64_t T, void* st) {
   const float* W[3];
-  for (int i = 0; i < w.n(); ++i) W[i] = pf(w.W[i]);
+  for (int i = 0; i < w.n(); ++i) W[i] = w.at(i);
   check(spion_linear_backward_input(&dY, W, w.n(), fp32, gelu_in, &dX, T, w.in(), w.out(), st), "spion_linear_backward_input");
 }
 // Weight and bias gradients of the stacked layers from dY (one [T, per] matrix per layer, or their head-split form) and X.
@@ -128,7 +137,7 @@ void linear_backward_input(const spion_tokens& dY, const Weights& w, bool fp32, 
 void linear_backward_weight(const std::vector<Tensor>& dY, const spion_tokens& tY, const Tensor& X, const spion_tokens& tX, const Weights& w,
                             bool fp32, int64_t T, void* st, std::vector<Tensor>& dW, std::vector<Tensor>& db, bool copied = false) {
   const int64_t in = w.in(), out = w.out(), per = out / w.n();
-  const auto opt = w.W[0].options();
+  const auto opt = X.options().dtype(at::kFloat);
   if (tX.is_bf16 && !copied && tY.heads == 0 && tX.heads == 0) {
     Tensor x2 = X.view({T, in});
     const int n = w.n();
@@ -562,7 +571,8 @@ struct LayerNode : public Node {
   ContextPtr c;
   bool fp32 = false;
   SavedAttn saved;
-  SavedVariable x, w[4];                 // Wq, Wk, Wv, Wf
+  SavedVariable x, w[4];                 // Wq, Wk, Wv, Wf; mixed precision: w[0] is the copy of all four, one after another
+  int64_t dim_out = 0;
   at::ScalarType out_type, x_type;
   bool released = false;
   std::string name() const override { return "SparseAttentionLayerBackward"; }
@@ -580,8 +590,12 @@ struct LayerNode : public Node {
     const auto type = fp32 ? at::kFloat : at::kBFloat16;
     const Attn a = saved.unpack(*c);
     const Tensor X = x.unpack(), x2 = X.to(type).reshape({c->B * c->L, X.size(2)});
+    const int64_t HD = c->H * c->d, dim = X.size(2);
     Tensor W[4];
-    for (int i = 0; i < 4; ++i) W[i] = w[i].unpack();
+    for (int i = 0; i < 4; ++i) {
+      if (fp32) W[i] = w[i].unpack();
+      else W[i] = w[0].unpack().narrow(0, i * HD * dim, i < 3 ? HD * dim : dim_out * HD).view({i < 3 ? HD : dim_out, i < 3 ? dim : HD});
+    }
     auto rows = [&](const Tensor& t) { return t.transpose(1, 2).reshape({c->B, c->L, c->H * c->d}); };
     auto operand = [&](const Tensor& t, int i) {
       const Tensor y = as_linear_node(rows(t), fp32, X, W[i], x_type, {next_edge(0), next_edge(1 + 2 * i), next_edge(2 + 2 * i)});
@@ -628,14 +642,21 @@ struct LayerNode : public Node {
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
     const int dim = (int)X.size(2);
     Weights qkv, ff;
-    for (int i = 0; i < 3; ++i) qkv.W.push_back(w[i].unpack());
-    ff.W.push_back(w[3].unpack());
+    const Tensor w0 = w[0].unpack();
+    if (fp32) {
+      qkv.W = {w0, w[1].unpack(), w[2].unpack()};
+      ff.W = {w[3].unpack()};
+    } else {
+      const int64_t n = 3 * (int64_t)H * d * dim;
+      qkv = Weights(pf(w0), 3, dim, 3 * H * d);
+      ff = Weights(pf(w0) + n, 1, H * d, dim_out);
+    }
     Tensor go = grads[0].to(out_type).contiguous();
     if (!aligned32(go)) go = go.clone();
     void* st = stream_of(go);
     auto form = [&](const std::vector<Tensor>& ts) { return a.heads ? tok(ts, H * d) : tok_heads(ts, H, d, L); };
     auto rows = [&](const Tensor& t) { return a.heads ? t.transpose(1, 2).view({T, H * d}) : t; };
-    const spion_tokens tgo = tok({go}, (int)ff.W[0].size(0));
+    const spion_tokens tgo = tok({go}, (int)dim_out);
     const spion_tokens tO = form({a.O});
     std::vector<Tensor> dW, db;
     if (task_should_compute_output(7) || task_should_compute_output(8)) {
@@ -685,6 +706,7 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
   Attn a;
   Tensor out;
   Kept kept_in, kept_out;
+  Tensor kept_w;
   {
     at::AutoDispatchBelowADInplaceOrView below;
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
@@ -699,11 +721,13 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
     a.q = empty_operand(*c, a.heads, like); a.k = empty_operand(*c, a.heads, like); a.v = empty_operand(*c, a.heads, like);
     Weights qkv{{W[0].detach(), W[1].detach(), W[2].detach()}, {b[0].detach(), b[1].detach(), b[2].detach()}};
     Weights ff{{W[3].detach()}, {b[3].detach()}};
-    kept_in = Kept(need, fp32, X, qkv);
+    const int64_t n_in = (int64_t)qkv.out() * qkv.in();
+    if (need && !fp32) kept_w = at::empty({n_in + (int64_t)ff.out() * ff.in()}, W[0].options());
+    kept_in = Kept(need, fp32, X, qkv, (float*)p(kept_w));
     linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st, kept_in);
     attn_forward(*c, a, need, st);
     out = at::empty({c->B, c->L, ff.out()}, opt);
-    kept_out = Kept(need, fp32, a.O, ff);
+    kept_out = Kept(need, fp32, a.O, ff, kept_w.defined() ? (float*)p(kept_w) + n_in : nullptr);
     linear_forward(form({a.O}), ff, fp32, tok({out}, ff.out()), nullptr, T, st, kept_out);
   }
   if (need) {
@@ -715,8 +739,9 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
     node->saved.save_all(kept, a.q, a.k, a.v);
     node->x_type = x.scalar_type();
     node->x = save(kept_in.x.defined() ? kept_in.x : x);
-    const int64_t per = W[0].size(0);
-    for (int i = 0; i < 4; ++i) node->w[i] = save(!kept_in.w.defined() ? W[i] : i < 3 ? kept_in.w.narrow(0, i * per, per) : kept_out.w);
+    node->dim_out = W[3].size(0);
+    if (kept_w.defined()) node->w[0] = save(kept_w);
+    else for (int i = 0; i < 4; ++i) node->w[i] = save(W[i]);
     torch::autograd::set_history(out, node);
   }
   return Result{out, a};
