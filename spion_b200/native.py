@@ -123,14 +123,18 @@ class BlockSparseAttention(nn.Module):
 
         * 32-wide blocks and the full mask: rebuilt tiles (no conversion passes; 2 * BH * L^2 elements less memory);
         * a caller that wants P back: stored tiles, the forward writes them anyway (L = 4096, 5 %: 227 us; rebuilt 242);
-        * rows of three blocks or more: rebuilt (head_dim 64: L = 4096, 5 %: 217 us, stored 227; 30 %: 607, 906; L = 16384, 5 %: 1650,
-          2610; head_dim 32, 2 to 128 matrices, L = 1024 to 4096, 3.2 to 19 blocks per row, with and without padded keys:
-          0.98 to 1.77 times as fast as stored, at 3.2 blocks per row 0.98 to 1.32); shorter rows: stored (L = 1024, two blocks
-          per row: 66 us, rebuilt 69)."""
+        * rows of three blocks or more: rebuilt (L = 4096, 5 %: 217 us, stored 227; 30 %: 607, 906; L = 16384, 5 %: 1650, 2610);
+          shorter rows: stored (L = 1024, two blocks per row: 66 us, rebuilt 69);
+        * head_dim 32 with fewer than 2^15 selected blocks in all matrices: stored.  The rebuilt tiles are 20 % faster there too
+          (32 matrices, L = 4096, 10 %: 152 against 196 us), but P is normalised before and not after it is rounded to bf16: a
+          training step of the encoder classifier repeats bit for bit only on the path it has always had.  At 256 matrices
+          (1013 against 1413 us) the layer, not the step around it, is what counts."""
         nb = self.L // self.bs
         if self.bs == 32 or self.nnzb == nb * nb:
             return True
-        return not self.return_probs and self.nnzb >= 3 * nb
+        if self.return_probs or self.nnzb < 3 * nb:
+            return False
+        return self.d == 64 or self.BH * self.nnzb >= 1 << 15
 
     @property
     def nnz(self) -> int:

@@ -527,18 +527,3 @@ def test_memory_of_contexts():
     assert free() == both
     del large, small
     assert start - free() < 80 << 20
-
-
-@pytest.mark.parametrize("head_dim", [32, 64])
-def test_the_backward_path_follows_the_mask(head_dim):
-    """Not the batch: the same layer rounds alike at every batch size."""
-    from spion_b200.native import BlockSparseAttention
-    for blocks, rebuilt in ((2, False), (3, True), (8, True)):
-        mat = torch.zeros(16, 16, device="cuda")
-        for i in range(blocks):
-            mat += torch.eye(16, device="cuda").roll(i, 1)
-        for batch in (1, 300):
-            cfg = dict(config(), head_dim=head_dim, max_seq_len=1024, batch_size=batch)
-            mod = BlockSparseAttention(cfg, dtype=torch.bfloat16, return_probs=False)
-            mod.set_mask(mat)
-            assert mod.recompute == rebuilt
