@@ -137,6 +137,8 @@ struct GemmArgs {
   int parts;                // bf16 gradient of three stacked layers: chunks per layer (0: one accumulator for the whole contraction)
   const __nv_bfloat16* h;   // EPI_DGELU: pre-activation [T, N]
   __nv_bfloat16* g;         // EPI_GELU: activation [T, N] (Y receives the pre-activation)
+  // What a backward reads in place of the caller's tensors.  262144 tokens of 64 fp32 features: 33 MB written here, 33 MB less read by
+  // the weight gradient; the layer of 128 x 2 matrices, L = 4096 went from 1432 to 1458 us.
   __nv_bfloat16* x_copy;    // or null: A as the products use it, [T, K] (fp32 tokens in bf16 mode)
   float* w_copy;            // or null: the stacked W
 };

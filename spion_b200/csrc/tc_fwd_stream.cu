@@ -11,8 +11,8 @@
 // other's waits.
 //
 // One pass over a row: m is the maximum of its first pair and is only moved (O and the running sum rescaled) when a later
-// score exceeds it by more than 2^8, so that almost no row is ever rescaled; the result is divided by the sum against the true
-// maximum at the end.  P <= 2^8 loses nothing in bf16 or in the fp32 sums.
+// score exceeds it by more than 2^8 (the conditional rescaling published with FlashAttention-4), so that almost no row is ever
+// rescaled; the result is divided by the sum against the true maximum at the end.  P <= 2^8 loses nothing in bf16 or in the fp32 sums.
 //
 // What bounds it: the exponentials, 8192 per pair at 16 per cycle and SM = 512 cycles, and 16 MMAs of 33 cycles at head_dim 64.
 // Measured, forward alone, before (one unit per CTA, two passes over a row) and now: 64 matrices, L = 4096, d 64, 5 % 62 -> 44 us,

@@ -125,10 +125,12 @@ class BlockSparseAttention(nn.Module):
         * a caller that wants P back: stored tiles, the forward writes them anyway (L = 4096, 5 %: 227 us; rebuilt 242);
         * rows of three blocks or more: rebuilt (L = 4096, 5 %: 217 us, stored 227; 30 %: 607, 906; L = 16384, 5 %: 1650, 2610);
           shorter rows: stored (L = 1024, two blocks per row: 66 us, rebuilt 69);
-        * head_dim 32 with fewer than 2^15 selected blocks in all matrices: stored.  The rebuilt tiles are 20 % faster there too
-          (32 matrices, L = 4096, 10 %: 152 against 196 us), but P is normalised before and not after it is rounded to bf16: a
-          training step of the encoder classifier repeats bit for bit only on the path it has always had.  At 256 matrices
-          (1013 against 1413 us) the layer, not the step around it, is what counts."""
+        * head_dim 32 with fewer than 2^15 selected blocks in all matrices: stored, although the rebuilt tiles are faster there too
+          (2 to 128 matrices, L = 1024 to 4096, 3.2 to 19 blocks per row: 0.98 to 1.77 times as fast).  P is normalised before and
+          not after it is rounded to bf16, and a training step of the encoder classifier at such sizes multiplies any change of
+          rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to 3.3e-1 of their norm over eight
+          seeds (both paths are equally far from the fp32 step).  The bound is a line between measured sizes that leaves those
+          steps as they were; it is no property of the kernels, and recompute=True takes the faster path below it as well."""
         nb = self.L // self.bs
         if self.bs == 32 or self.nnzb == nb * nb:
             return True
