@@ -90,7 +90,6 @@ void device_free(void* p) {
   }
   d->waiting.clear();
   d->follow();
-  cudaStreamSynchronize(d->stream);               // what is beyond the threshold goes back now
 }
 
 int sm_count() {
