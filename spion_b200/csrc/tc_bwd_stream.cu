@@ -12,19 +12,24 @@
 //              lane offset 16: query rows along the lanes in both, so that lse and delta are one register each
 //     accumulators += dS^T Q, P^T dO (COL),  += dS K (ROW)
 // One persistent CTA per SM, 640 threads:
-//   warp 0   loads: pairs in stream order into a ring of slots, the fixed tiles of a unit into one of two sets (TMA)
-//   warp 1   S / dP products into one of three tensor-memory sets, up to two pairs ahead of the arithmetic
+//   warp 0   loads: the tiles of a pair into a ring of slots, the fixed tiles of a unit into one of two sets (TMA)
+//   warp 1   S / dP products into one of three tensor-memory sets
 //   warp 2   second products, when the tiles of a pair are written
-//   warp 3   lse and -delta scale of the next pair's (COL) or unit's (ROW) query rows into shared memory, which blocks have padded
-//            keys
-//   warps 4-19   arithmetic, two groups of eight: even and odd pairs; each warp one tensor-memory quadrant and half of the columns.
-//            Two groups because the chain of one pair (tensor-memory load, exponentials, tile store, proxy fence, hand-over) is
-//            about three times as long as its instructions take to issue.  ROW: they form delta first, while the first tiles
-//            arrive, and leave it in global memory, for COL too.
-// What bounds it: per pair at head_dim 64 the tensor pipe needs 920 (COL) or 660 cycles (ROW), the exponentials 512.
-// Measured, rows + columns, against the backward from stored P of tc_engine.cu: 64 matrices, d 64: L = 4096, 5 % 168 us (stored 155,
-// its forward 25 slower), 30 % 458 (stored path 906 with its forward); L = 16384, 5 % 1271 (2610); 256 matrices, L = 4096,
-// d 32, 10 %, padded keys 791 (1413).  Which of the two serves a mask: _recompute_pays in native.py.
+//   warp 3   the walk: 16 byte records of the CTA's pairs, 16 at a time (which tiles, first or last of its unit, which blocks have padded
+//            keys), in shared memory for all other warps.  With a walk of its own in every warp and the statistics handed out pair by
+//            pair, that warp was what the others waited for: each value it copied from one variable to the next to have it early is a
+//            wait for global memory.
+//   warps 4-19   arithmetic, in groups that take pairs in turn, each warp one tensor-memory quadrant.  Four groups of four warps, a warp
+//            the whole 64 columns of its rows in two halves: what a pair costs besides its values (waits, fences, hand-over) is paid by
+//            half as many warps than with two groups of eight, and four chains fill each other's waits.  COL at head_dim 64: two groups of
+//            eight (value tiles of four pairs do not fit shared memory).  ROW: dS over the V tiles, which only dP reads; delta
+//            first, while the first tiles arrive, left in global memory, for COL too.
+// What bounds it: per pair at head_dim 64 the tensor pipe needs 920 (COL) or 660 cycles (ROW), the exponentials 512; a pair takes
+// about 1450.
+// Measured, ROW and COL, before (two groups of eight, a walk in every warp) and now: 64 matrices, L = 16384, d 64, 5 %: 637 and 639 us, now
+// 561 and 605; 256 matrices, L = 4096, d 32, 10 %, padded keys, two full columns: 425 and 394, now 341 and 306.  COL at head_dim 32: five
+// slots and four sets of value tiles 306 us, seven and three 317.  Which mask is served by rebuilt and which by stored tiles:
+// _recompute_pays in native.py.
 //
 // Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
 #include "tc_stream.cuh"
@@ -38,16 +43,19 @@ constexpr int COL = 0, ROW = 1;
 
 template <int D, int SIDE> struct Bw {
   using T = OpTile<D>;
-  static constexpr int NP = (D == 64) ? 4 : 8;                        // pair slots
-  static constexpr uint32_t SLOT = 4 * T::BYTES;                      // A0 of both entries, A1 of both entries
-  static constexpr uint32_t FIX = 2 * T::BYTES;                       // F0, F1; two sets
+  static constexpr int NGR = SIDE == COL && D == 64 ? 2 : 4;          // arithmetic groups
+  static constexpr int NS = NGR == 2 ? 3 : 4;                         // barriers that hand S and dP over, pair j: j % NS
+  static constexpr int WPG = 16 / NGR, HALVES = NGR / 2;              // warps of a group; halves of a tile's columns a warp does
+  static constexpr int NP = SIDE == COL ? (D == 64 ? 4 : 5) : (D == 64 ? 6 : 8);      // pair slots
   static constexpr uint32_t PD = (SIDE == COL ? 4 : 2) * VT_BYTES;    // value tiles of a pair: dS of both entries, then P of both
-  static constexpr uint32_t O_FIX = NP * SLOT, O_PD = O_FIX + 2 * FIX, O_BAR = O_PD + 2 * PD;
-  // per parity of the pair: {pad flags and submasks of the two entries, their lines}, and in COL lse, -delta scale of their 128
-  // query rows; ROW: those of the unit's 64 rows per parity of the unit
-  static constexpr uint32_t O_INFO = O_BAR + 352, O_STAT = O_INFO + 32;
-  static constexpr uint32_t ROWS = SIDE == COL ? 128 : 64;
-  static constexpr size_t SMEM = O_STAT + 2 * 2 * ROWS * 4;
+  // A0 of both entries, A1 of both entries; ROW: the dS tiles take the place of A1, which only the first products read
+  static constexpr uint32_t SLOT = 2 * T::BYTES + (SIDE == COL ? 2 * T::BYTES : PD);
+  static constexpr int NPD = SIDE == ROW ? 0 : NGR;                   // sets of value tiles beside the slots
+  static constexpr uint32_t FIX = 2 * T::BYTES;                       // F0, F1; two sets
+  static constexpr int NACC = SIDE == COL && D == 64 ? 2 : 4;         // accumulator sets
+  static constexpr uint32_t O_FIX = NP * SLOT, O_PD = O_FIX + 2 * FIX, O_BAR = O_PD + NPD * PD;
+  static constexpr uint32_t O_RING = O_BAR + 432;                     // records of 32 pairs
+  static constexpr size_t SMEM = O_RING + 32 * 16;
 };
 
 struct BwArgs {
@@ -62,47 +70,67 @@ struct BwArgs {
   int* status;
 };
 
+// Record of a pair: {flags, line of entry 0 | line of entry 1 << 16, line of the unit, (b,h) matrix}.  Flags: 1, 2: entry 0, 1 has padded
+// keys; the accumulator set << 4; the selected quarters of entry 0 << 8, of entry 1 << 16.
+constexpr int PF_LAST = 4, PF_TWO = 8, PF_FIRST = 64, PF_END = (int)0x80000000;
+
+// Are any of the penalties of 64 keys not zero?  Per lane.
+__device__ __forceinline__ bool pad64(const float* kp) {
+  bool v = false;
+  if ((reinterpret_cast<uintptr_t>(kp) & 15) == 0) {
+#pragma unroll
+    for (int x = 0; x < 16; ++x) {
+      const float4 f = reinterpret_cast<const float4*>(kp)[x];
+      v |= f.x != 0.f || f.y != 0.f || f.z != 0.f || f.w != 0.f;
+    }
+  } else {
+    for (int x = 0; x < 64; ++x) v |= kp[x] != 0.f;
+  }
+  return v;
+}
+
 template <int D, int SIDE, bool SUB>
 __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                                                               const __grid_constant__ CUtensorMap tmF0, const __grid_constant__ CUtensorMap tmF1,
                                                               const __grid_constant__ BwArgs a) {
   using C = Bw<D, SIDE>;
   using T = OpTile<D>;
-  constexpr int NP = C::NP;
+  constexpr int NP = C::NP, NGR = C::NGR, WPG = C::WPG, NACC = C::NACC;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t sbase = smem_u32(smem_raw);                          // must be 1024-aligned (checked below)
   const uint32_t bars = sbase + C::O_BAR;
-  // pfull / pdone[slot]: tiles landed / second products that read the slot retired; s_ready / t_free[3]: S and dP of a pair in
-  // tensor memory / read out (8 warps); p_ready[2]: value tiles of a pair written (8 warps); acc_done / acc_free[2]: a unit's
-  // accumulators complete / read out (8 warps); f_full / f_free[2]: fixed tiles landed / no longer read; pi_full / pi_free[2]:
-  // what warp 3 wrote for a pair is there / has been read (8 warps); st_full / st_free[2]: ROW, the same for a unit (16 warps)
-  const uint32_t pfull = bars, pdone = bars + 64, s_ready = bars + 128, t_free = bars + 152, p_ready = bars + 176, acc_done = bars + 192,
-                 acc_free = bars + 208, f_full = bars + 224, f_free = bars + 240, st_full = bars + 256, st_free = bars + 272,
-                 pi_full = bars + 288, pi_free = bars + 304, slot = bars + 320, abort_w = bars + 324;
+  // pfull / pdone[slot]: tiles landed / second products that read the slot retired; p_ready[slot]: value tiles of its pair written (the
+  // group's warps); s_ready[pair % NS]: S and dP of a pair in tensor memory; t_free[set]: ... read out (the group's warps);
+  // acc_done[group][parity of the units it writes]: accumulators complete; acc_free[set]: ... read out (the group's warps); f_full /
+  // f_free[2]: fixed tiles landed / no longer read; r_full / r_free[half]: 16 records written / read (all warps but warp 3).
+  // A parity tells two phases apart, so every barrier has one waiter (a warp, a group's warps; r_full: each reader for itself) that
+  // waits for each of its phases, and a phase cannot complete before the one before it has been waited for.
+  const uint32_t pfull = bars, pdone = bars + 64, p_ready = bars + 128, s_ready = bars + 192, t_free = bars + 224, acc_done = bars + 248,
+                 acc_free = bars + 312, f_full = bars + 344, f_free = bars + 360, r_full = bars + 376, r_free = bars + 392,
+                 slot = bars + 408, abort_w = bars + 412;
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
   volatile int* abort_ptr = reinterpret_cast<volatile int*>(smem_raw + (abort_w - sbase));
 
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int G = (int)gridDim.x, total = a.nb * a.BH;
+  const int n_my = total > (int)blockIdx.x ? (total - (int)blockIdx.x + G - 1) / G : 0;         // units blockIdx.x, + G, ...
   const UnitMap um{a.nb, a.BH, a.by_rank};
-  constexpr uint32_t ACC = 384u;                                      // three S / dP sets of 128 columns, two accumulator sets of 64
+  constexpr uint32_t ACC = 384u;                                      // three S / dP sets of 128 columns, then the accumulators
 
   if (warp == 0 && lane == 0) {
     int ab = *reinterpret_cast<volatile int*>(a.status);
     if ((sbase & 1023u) != 0u) { report(a.status, ERR_LOAD_WAIT); ab = 1; }
     *abort_ptr = ab;
-    for (int i = 0; i < NP; ++i) { mbar_init(pfull + 8 * i, 1); mbar_init(pdone + 8 * i, 1); }
-    for (int i = 0; i < 3; ++i) { mbar_init(s_ready + 8 * i, 1); mbar_init(t_free + 8 * i, 8); }
+    for (int i = 0; i < NP; ++i) { mbar_init(pfull + 8 * i, 1); mbar_init(pdone + 8 * i, 1); mbar_init(p_ready + 8 * i, WPG); }
+    for (int i = 0; i < C::NS; ++i) mbar_init(s_ready + 8 * i, 1);
+    for (int i = 0; i < 3; ++i) mbar_init(t_free + 8 * i, WPG);
+    for (int i = 0; i < 2 * NGR; ++i) mbar_init(acc_done + 8 * i, 1);
+    for (int i = 0; i < NACC; ++i) mbar_init(acc_free + 8 * i, WPG);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(p_ready + 8 * i, 8);
-      mbar_init(acc_done + 8 * i, 1);
-      mbar_init(acc_free + 8 * i, 8);
       mbar_init(f_full + 8 * i, 1);
       mbar_init(f_free + 8 * i, 1);
-      mbar_init(st_full + 8 * i, 1);
-      mbar_init(st_free + 8 * i, 16);
-      mbar_init(pi_full + 8 * i, 1);
-      mbar_init(pi_free + 8 * i, 8);
+      mbar_init(r_full + 8 * i, 1);
+      mbar_init(r_free + 8 * i, 19);
     }
     fence_barrier_init();
   }
@@ -117,75 +145,66 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
   tc_fence_after();
   const uint32_t tmem = *slot_ptr;
   auto wait_all = [&](uint32_t bar, uint32_t parity, int code) -> bool { return warp_wait(bar, parity & 1u, a.status, code); };
-  Walk c;
-  c.init(um, a.rec, (int)blockIdx.x, G, total);
+  // columns and lanes of accumulator set x: COL beside each other (dK in lanes 0-15 of every quadrant, dV in 16-31); ROW (dQ alone): two
+  // beside each other, the other two at lane offset 16
+  auto acc_at = [](int x) -> uint32_t {
+    return ACC + (SIDE == ROW ? (uint32_t)(x & 1) * D + ((uint32_t)((x >> 1) * 16) << 16) : (uint32_t)x * D);
+  };
+  const int4* ring = reinterpret_cast<const int4*>(smem_raw + C::O_RING);
+  // A reader takes the records of pairs j, j + step, ...: it waits where it enters a half and hands it back with its last record there.
+  auto record = [&](uint32_t j, uint32_t step, int4& r) -> bool {
+    if ((j & 15) < step && !wait_all(r_full + 8 * ((j >> 4) & 1), j >> 5, ERR_LOAD_WAIT)) return false;
+    r = ring[j & 31];
+    __syncwarp();
+    if ((j & 15) + step >= 16 && lane == 0) mbar_arrive(r_free + 8 * ((j >> 4) & 1));
+    return true;
+  };
 
   if (warp == 0) {
     // ================================================================== loads
-    bool ok = true;
-    int loads0 = 0, loads1 = 0;                                       // units whose fixed tiles went to set 0 / 1
-    c.skip();
-    // lane l keeps the record of pair l of the current unit and of the next one, both requested a unit early
-    int4 prs = make_int4(0, -1, 0, 0), prs_n = prs;
-    int cached_i = -1;
-    for (int j = 0; ok && c.valid(); ++j, c.next()) {
-      const int ps = j % NP;
-      if (c.i != cached_i) {
-        prs = (cached_i >= 0 && c.i == cached_i + 1) ? prs_n : (lane < c.pairs() ? a.pair[c.cur.y + lane] : prs);
-        cached_i = c.i;
-        if (c.i + 1 < c.n_my && lane < c.nxt.z) prs_n = a.pair[c.nxt.y + lane];
-      }
-      int4 pr;
-      if (c.k < 32) {
-        pr.x = __shfl_sync(0xffffffffu, prs.x, c.k);
-        pr.y = __shfl_sync(0xffffffffu, prs.y, c.k);
-      } else {
-        pr = a.pair[c.cur.y + c.k];
-      }
-      if (j >= NP && !wait_all(pdone + 8 * ps, (uint32_t)(j / NP - 1), ERR_MMA2_WAIT)) { ok = false; break; }
-      const int par = c.i & 1;
-      if (c.k == 0) {
-        const int loads = par ? loads1 : loads0;
-        if (loads >= 1 && !wait_all(f_free + 8 * par, (uint32_t)(loads - 1), ERR_MMA2_WAIT)) { ok = false; break; }
-      }
-      const int cnt = c.cnt();
-      const OpPos pos = op_pos(c.bh, a.L, a.heads, D);
-      if (lane == 0) {
-        mbar_expect_tx(pfull + 8 * ps, 2 * cnt * T::BYTES);
-        if (c.k == 0) mbar_expect_tx(f_full + 8 * par, 2 * T::BYTES);
+    int u = 0, ps = 0, round = 0;
+    for (uint32_t j = 0;; ++j) {
+      int4 r;
+      if (!record(j, 1, r) || r.x < 0) break;
+      if (round >= 1 && !wait_all(pdone + 8 * ps, (uint32_t)(round - 1), ERR_MMA2_WAIT)) break;
+      const bool first = warp_uniform(r.x & PF_FIRST) != 0, two = warp_uniform(r.x & PF_TWO) != 0;
+      const int fs = u & 1;
+      if (first && u >= 2 && !wait_all(f_free + 8 * fs, (uint32_t)((u >> 1) - 1), ERR_MMA2_WAIT)) break;
+      const OpPos pos = op_pos(r.w, a.L, a.heads, D);
+      const uint32_t dst = sbase + ps * C::SLOT;
+      if (elect_one()) {
+        if (first) {
+          const uint32_t f = sbase + C::O_FIX + fs * C::FIX;
+          mbar_expect_tx(f_full + 8 * fs, 2 * T::BYTES);
+          tma_load_2d(f, &tmF0, f_full + 8 * fs, pos.x0, pos.row0 + r.z * BS);
+          tma_load_2d(f + T::BYTES, &tmF1, f_full + 8 * fs, pos.x0, pos.row0 + r.z * BS);
+        }
+        mbar_expect_tx(pfull + 8 * ps, (two ? 4 : 2) * T::BYTES);
+        const int y0 = pos.row0 + (r.y & 0xffff) * BS, y1 = pos.row0 + (r.y >> 16) * BS;
+        tma_load_2d(dst, &tmA0, pfull + 8 * ps, pos.x0, y0);
+        tma_load_2d(dst + 2 * T::BYTES, &tmA1, pfull + 8 * ps, pos.x0, y0);
+        if (two) {
+          tma_load_2d(dst + T::BYTES, &tmA0, pfull + 8 * ps, pos.x0, y1);
+          tma_load_2d(dst + 3 * T::BYTES, &tmA1, pfull + 8 * ps, pos.x0, y1);
+        }
       }
       __syncwarp();
-      if (c.k == 0) {
-        const uint32_t f = sbase + C::O_FIX + par * C::FIX;
-        if (lane == 4) tma_load_2d(f, &tmF0, f_full + 8 * par, pos.x0, pos.row0 + c.cur.x * BS);
-        if (lane == 5) tma_load_2d(f + T::BYTES, &tmF1, f_full + 8 * par, pos.x0, pos.row0 + c.cur.x * BS);
-        if (par) ++loads1; else ++loads0;
-      }
-      if (lane < 2 * cnt) {
-        const int e = lane >> 1;
-        const int orow = pos.row0 + (e ? pr.y : pr.x) * BS;
-        const uint32_t dst = sbase + ps * C::SLOT + ((lane & 1) * 2 + e) * T::BYTES;
-        if (lane & 1) tma_load_2d(dst, &tmA1, pfull + 8 * ps, pos.x0, orow);
-        else tma_load_2d(dst, &tmA0, pfull + 8 * ps, pos.x0, orow);
-      }
+      if (r.x & PF_LAST) ++u;
+      if (++ps == NP) { ps = 0; ++round; }
     }
   } else if (warp == 1) {
     // ================================================================== S and dP
     constexpr uint32_t IDESC = make_idesc_bf16(SIDE == COL ? 128 : 64, 64, 0, 0);
     const uint64_t KM = T::kmajor(sbase, 0);
-    bool ok = true;
-    int waits0 = 0, waits1 = 0;
-    c.skip();
-    for (int j = 0; ok && c.valid(); ++j, c.next()) {
-      const int ps = j % NP, set = j % 3, par = c.i & 1;
-      if (j >= 3 && !wait_all(t_free + 8 * set, (uint32_t)(j / 3 - 1), ERR_MMA_WAIT)) { ok = false; break; }
-      if (c.k == 0) {
-        const int w = par ? waits1 : waits0;
-        if (!wait_all(f_full + 8 * par, (uint32_t)w, ERR_LOAD_WAIT)) { ok = false; break; }
-        if (par) ++waits1; else ++waits0;
-      }
-      if (!wait_all(pfull + 8 * ps, (uint32_t)(j / NP), ERR_LOAD_WAIT)) { ok = false; break; }
-      const bool last = warp_uniform((int)c.last()) != 0, two = warp_uniform(c.cnt()) == 2;
+    int u = 0, ps = 0, round = 0, set = 0, sround = 0, sr = 0;
+    for (uint32_t j = 0;; ++j) {
+      int4 r;
+      if (!record(j, 1, r) || r.x < 0) break;
+      const int par = u & 1;
+      if (sround >= 1 && !wait_all(t_free + 8 * set, (uint32_t)(sround - 1), ERR_MMA_WAIT)) break;
+      if ((r.x & PF_FIRST) && !wait_all(f_full + 8 * par, (uint32_t)(u >> 1), ERR_LOAD_WAIT)) break;
+      if (!wait_all(pfull + 8 * ps, (uint32_t)round, ERR_LOAD_WAIT)) break;
+      const bool last = warp_uniform(r.x & PF_LAST) != 0, two = warp_uniform(r.x & PF_TWO) != 0;
       if (elect_one()) {
         tc_fence_after();
         const uint64_t a0 = desc_advance(KM, ps * C::SLOT), a1 = desc_advance(a0, 2 * T::BYTES);
@@ -209,32 +228,37 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
           products(0);
           if (two) products(1);
         }
-        mma_commit(s_ready + 8 * set);
+        mma_commit(s_ready + 8 * sr);
         if (last) mma_commit(f_free + 8 * par);                       // the fixed tiles are read by these products only
       }
       __syncwarp();
+      if (++ps == NP) { ps = 0; ++round; }
+      if (++set == 3) { set = 0; ++sround; }
+      if (++sr == C::NS) sr = 0;
+      if (last) ++u;
     }
   } else if (warp == 2) {
     // ================================================================== second products
     constexpr uint32_t IDESC = make_idesc_bf16(64, D, SIDE == COL ? 1 : 0, 1);
     constexpr uint32_t V_STEP = SIDE == COL ? ValTile::MN_STEP : ValTile::K_STEP;
     const uint64_t MN = T::mnmajor(sbase, 0), VT = SIDE == COL ? ValTile::mnmajor(sbase, 0) : ValTile::kmajor(sbase, 0);
-    bool ok = true;
-    int uses0 = 0, uses1 = 0;
-    c.skip();
-    for (int j = 0; ok && c.valid(); ++j, c.next()) {
-      const int ps = j % NP, set = j & 1, par = c.i & 1;
-      const int uses = par ? uses1 : uses0;
-      if (c.k == 0 && uses >= 1 && !wait_all(acc_free + 8 * par, (uint32_t)(uses - 1), ERR_MMA2_WAIT)) { ok = false; break; }
-      if (!wait_all(p_ready + 8 * set, (uint32_t)(j >> 1), ERR_MMA_WAIT)) { ok = false; break; }
-      const bool last = warp_uniform((int)c.last()) != 0, two = warp_uniform(c.cnt()) == 2, fresh = warp_uniform(c.k) == 0;
+    int u = 0, ps = 0, round = 0, grp = 0, pd = 0;
+    uint32_t odd = 0;                                                 // bit g: group g has written an odd number of units
+    for (uint32_t j = 0;; ++j) {
+      int4 r;
+      if (!record(j, 1, r) || r.x < 0) break;
+      const int x = u % NACC;
+      if ((r.x & PF_FIRST) && u >= NACC && !wait_all(acc_free + 8 * x, (uint32_t)(u / NACC - 1), ERR_MMA2_WAIT)) break;
+      if (!wait_all(p_ready + 8 * ps, (uint32_t)round, ERR_MMA_WAIT)) break;
+      const bool last = warp_uniform(r.x & PF_LAST) != 0, two = warp_uniform(r.x & PF_TWO) != 0, fresh = warp_uniform(r.x & PF_FIRST) != 0;
       if (elect_one()) {
         tc_fence_after();
-        const uint32_t acc = tmem + ACC + (uint32_t)par * 64u;
-        const uint64_t vt = desc_advance(VT, C::O_PD + set * C::PD), b0 = desc_advance(MN, ps * C::SLOT);
+        const uint32_t acc = tmem + acc_at(x);
+        const uint64_t b0 = desc_advance(MN, ps * C::SLOT);
+        const uint64_t vt = desc_advance(VT, SIDE == COL ? C::O_PD + pd * C::PD : ps * C::SLOT + 2 * T::BYTES);
         auto products = [&](int e, bool first) {
 #pragma unroll
-          for (int kk = 0; kk < BS / 16; ++kk)                        // dK or dQ (lanes 0-15 of every quadrant)
+          for (int kk = 0; kk < BS / 16; ++kk)                        // dK or dQ
             mma_bf16(acc, desc_advance(vt, e * VT_BYTES + kk * V_STEP), desc_advance(b0, e * T::BYTES + kk * T::MN_STEP), IDESC,
                      (kk > 0) ? 1u : (first ? 0u : 1u));
           if (SIDE == COL) {
@@ -247,109 +271,134 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         products(0, fresh);
         if (two) products(1, false);
         mma_commit(pdone + 8 * ps);
-        if (last) mma_commit(acc_done + 8 * par);
+        if (last) mma_commit(acc_done + 8 * (2 * grp + ((odd >> grp) & 1)));
       }
       __syncwarp();
-      if (last) { if (par) ++uses1; else ++uses0; }
+      if (++ps == NP) { ps = 0; ++round; }
+      if (last) { ++u; odd ^= 1u << grp; }
+      if (++grp == NGR) grp = 0;
+      if (SIDE == COL && ++pd == C::NPD) pd = 0;
     }
   } else if (warp == 3) {
-    // ================================================================== statistics and flags for the arithmetic warps
-    if (SIDE == ROW) asm volatile("bar.sync 1, 544;" ::: "memory");   // delta of this CTA's rows is in global memory
-    bool ok = true;
-    int sets0 = 0, sets1 = 0;
-    int j = 0;
-    int4 pr = make_int4(0, -1, 0, 0);
-    for (; ok && c.valid(); c.shift()) {
-      const int par = c.i & 1;
-      const bool used = c.cur.w > 0;
-      const size_t base = (size_t)c.bh * a.L;
-      const float* kpu = a.keypad ? a.keypad + base : nullptr;
-      if (used) pr = a.pair[c.cur.y];
-      int unit_pad = 0;
-      if (SIDE == COL) {
-        if (used && kpu) unit_pad = __any_sync(0xffffffffu, pad4(kpu + c.cur.x * BS));
-      } else {
-        float dl[2], hh[2];                                           // rows lane and lane + 32
+    // ================================================================== the walk: records of the CTA's pairs, 16 at a time
+    // 32 units at a time, one per lane; lanes t and t + 16 look at entries 0 and 1 of pair t of a half.
+    auto unit_at = [&](int i, int& bh) -> int4 {
+      bh = 0;
+      if (i >= n_my) return make_int4(0, 0, 0, 0);
+      int rank;
+      um.at((int)blockIdx.x + i * G, bh, rank);
+      return a.rec[rank];
+    };
+    int bh, bh_n, i0 = 0, pos = 0, tot = 0, units = 0;                // units with entries before the 32
+    int4 un = unit_at(lane, bh), un_n = unit_at(32 + lane, bh_n);
+    int end = 0;                                                      // pairs of the 32 units up to this lane's
+    uint32_t used = 0;                                                // those with entries
+    auto enter = [&]() {
+      end = un.z;
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const size_t ri = base + (size_t)c.cur.x * BS + lane + 32 * x;
-          dl[x] = *reinterpret_cast<volatile float*>(a.delta_out + ri);       // written by this CTA
-          hh[x] = a.lse[ri];
-        }
-        if (used) {
-          const int sets = par ? sets1 : sets0;
-          if (sets >= 1 && !wait_all(st_free + 8 * par, (uint32_t)(sets - 1), ERR_MMA_WAIT)) { ok = false; break; }
-          float* st = reinterpret_cast<float*>(smem_raw + C::O_STAT) + par * 2 * 64;
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            st[lane + 32 * x] = hh[x];
-            st[64 + lane + 32 * x] = -dl[x] * a.scale;
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(st_full + 8 * par);
-          if (par) ++sets1; else ++sets0;
+      for (int s = 1; s < 32; s <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, s);
+        if (lane >= s) end += v;
+      }
+      pos = 0;
+      tot = __shfl_sync(0xffffffffu, end, 31);
+      used = __ballot_sync(0xffffffffu, un.z > 0);
+      uint32_t none = __ballot_sync(0xffffffffu, un.z == 0 && i0 + lane < n_my);
+      while (none) {                                                  // lines without entries: zero rows
+        const int x = __ffs(none) - 1;
+        none &= none - 1;
+        const int line = __shfl_sync(0xffffffffu, un.x, x);
+        const OpPos pos0 = op_pos(__shfl_sync(0xffffffffu, bh, x), a.L, a.heads, D);
+        for (int y = lane; y < BS * (D / 8); y += 32) {
+          const size_t off = (size_t)(pos0.row0 + line * BS + y / (D / 8)) * pos0.ld + pos0.x0 + (y % (D / 8)) * 8;
+          *reinterpret_cast<uint4*>(a.out0 + off) = make_uint4(0, 0, 0, 0);
+          if (SIDE == COL) *reinterpret_cast<uint4*>(a.out1 + off) = make_uint4(0, 0, 0, 0);
         }
       }
-      const int np = c.pairs();
-      for (int k = 0; ok && k < np; ++k, ++j) {
-        // lanes 0-15: first entry, 16-31: second; four query rows (COL) or keys (ROW) each
-        const int e = lane >> 4, o = e ? pr.y : pr.x, blk = e ? pr.w : pr.z;
-        const size_t ri = base + (size_t)max(o, 0) * BS;
-        float h4[4] = {0.f, 0.f, 0.f, 0.f}, d4[4] = {0.f, 0.f, 0.f, 0.f};
-        int pad = unit_pad;
-        if (SIDE == COL) {
-          if (o >= 0) {
-#pragma unroll
-            for (int x = 0; x < 4; ++x) { h4[x] = a.lse[ri + (lane & 15) + 16 * x]; d4[x] = a.delta[ri + (lane & 15) + 16 * x]; }
+    };
+    enter();
+    const int e = lane >> 4;
+    bool more = true;
+    for (uint32_t f = 0; more; ++f) {
+      if (f >= 2 && !wait_all(r_free + 8 * (f & 1), (f >> 1) - 1, ERR_MMA_WAIT)) break;
+      int4* half = reinterpret_cast<int4*>(smem_raw + C::O_RING) + 16 * (f & 1);
+      int filled = 0;
+      while (filled < 16) {
+        if (pos >= tot) {
+          if (i0 + 32 >= n_my) {
+            if (lane >= filled && lane < 16) half[lane] = make_int4(PF_END, 0, 0, 0);       // every reader meets one
+            more = filled > 16 - NGR;                                 // ... in this half or the next one
+            filled = 16;
+            break;
           }
-        } else if (kpu) {
-          const uint32_t any = __ballot_sync(0xffffffffu, o >= 0 && pad4(a.keypad + ri));
-          pad = ((any & 0xffffu) ? 1 : 0) | ((any >> 16) ? 2 : 0);
+          i0 += 32;
+          units += __popc(used);
+          un = un_n; bh = bh_n;
+          un_n = unit_at(i0 + 32 + lane, bh_n);
+          enter();
+          continue;
         }
-        const int sub = SUB && o >= 0 ? a.submask[blk] : 0xff;
-        const int4 pr_next = k + 1 < np ? a.pair[c.cur.y + k + 1] : pr;
-        if (j >= 2 && !wait_all(pi_free + 8 * (j & 1), (uint32_t)((j >> 1) - 1), ERR_MMA_WAIT)) { ok = false; break; }
-        int* info = reinterpret_cast<int*>(smem_raw + C::O_INFO) + 4 * (j & 1);
-        const int sub1 = __shfl_sync(0xffffffffu, sub, 16);
-        if (lane == 0) { info[0] = pad | (sub << 8) | (sub1 << 16); info[1] = pr.x; info[2] = pr.y; }
-        if (SIDE == COL) {
-          float* st = reinterpret_cast<float*>(smem_raw + C::O_STAT) + (j & 1) * 2 * 128 + e * 64 + (lane & 15);
+        const int n = min(16 - filled, tot - pos), t = (lane & 15) - filled;
+        const bool active = t >= 0 && t < n;
+        const int p = pos + (active ? t : 0);
+        int x = 0;                                                    // the unit of pair p: the first whose pairs end after it
 #pragma unroll
-          for (int x = 0; x < 4; ++x) { st[16 * x] = h4[x]; st[128 + 16 * x] = -d4[x] * a.scale; }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(pi_full + 8 * (j & 1));
-        pr = pr_next;
+        for (int s = 16; s; s >>= 1)
+          if (__shfl_sync(0xffffffffu, end, x + s - 1) <= p) x += s;
+        const int line = __shfl_sync(0xffffffffu, un.x, x), first = __shfl_sync(0xffffffffu, un.y, x), np = __shfl_sync(0xffffffffu, un.z, x),
+                  n_e = __shfl_sync(0xffffffffu, un.w, x), b = __shfl_sync(0xffffffffu, bh, x), k = p - (__shfl_sync(0xffffffffu, end, x) - np);
+        const int4 pr = a.pair[first + k];
+        const bool two = 2 * k + 1 < n_e, here = e == 0 || two;
+        const int o = e ? pr.y : pr.x;
+        bool pad = false;
+        int sub = 0xff;
+        if (a.keypad && here) pad = pad64(a.keypad + (size_t)b * a.L + (SIDE == COL ? line : o) * BS);
+        if (SUB) sub = here ? a.submask[e ? pr.w : pr.z] : 0;
+        const int fl = (pad ? 1 : 0) | (sub << 8), fl1 = __shfl_down_sync(0xffffffffu, fl, 16);
+        const int ux = units + __popc(used & ((1u << x) - 1));
+        if (active && e == 0)
+          half[lane] = make_int4(fl | (fl1 & 1) << 1 | (fl1 & 0xff00) << 8 | (k + 1 == np ? PF_LAST : 0) | (two ? PF_TWO : 0) |
+                                     (k == 0 ? PF_FIRST : 0) | (ux % NACC) << 4,
+                                 pr.x | (two ? pr.y << 16 : 0), line, b);
+        filled += n;
+        pos += n;
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(r_full + 8 * (f & 1));
     }
   } else {
     // ================================================================== arithmetic
-    const int mw = warp - 4, q = warp & 3, g = (mw >> 2) & 1, grp = mw >> 3;
+    const int mw = warp - 4, q = warp & 3, grp = mw / WPG, g0 = WPG == 8 ? (mw >> 2) & 1 : 0;
     if (SIDE == ROW) {
-      // delta = rowsum(dO.O) of all rows of this CTA, four units of loads in flight: D / 8 lanes per row, 16 bytes each
-      constexpr int LPR = D / 8, RPW = 32 / LPR, UN = 4;
-      static_assert(16 * RPW >= BS, "rows of a unit");
-      const int r0 = mw * RPW + lane / LPR;
-      for (int i0 = 0; i0 < c.n_my; i0 += UN) {
+      // delta = rowsum(dO.O) of all rows of this CTA: D / 8 lanes per row, 16 bytes each, a warp RPW rows of a unit, eight such loads in
+      // flight.  Lane l knows where unit l of the next 32 is.
+      constexpr int LPR = D / 8, RPW = 32 / LPR, WPU = BS / RPW, UPS = 16 / WPU, UN = 8;       // warps per unit, units per step
+      const int r0 = (mw % WPU) * RPW + lane / LPR;
+      int l_row = 0, l_x = 0, l_out = 0;
+      for (int i0 = 0; i0 < n_my; i0 += UN * UPS) {
+        if (i0 % 32 == 0 && i0 + lane < n_my) {
+          int bh, rank;
+          um.at((int)blockIdx.x + (i0 + lane) * G, bh, rank);
+          const int line = a.rec[rank].x;
+          const OpPos pos = op_pos(bh, a.L, a.heads, D);
+          l_row = pos.row0 + line * BS; l_x = pos.x0; l_out = bh * a.L + line * BS;
+        }
         uint4 u[UN], v[UN];
-        size_t ri[UN];
 #pragma unroll
         for (int x = 0; x < UN; ++x) {
+          const int i = i0 + x * UPS + mw / WPU;
+          const int rw = __shfl_sync(0xffffffffu, l_row, i & 31), x0 = __shfl_sync(0xffffffffu, l_x, i & 31);
           u[x] = v[x] = make_uint4(0, 0, 0, 0);
-          ri[x] = 0;
-          if (i0 + x < c.n_my && r0 < BS) {
-            int bh, rank;
-            um.at((int)blockIdx.x + (i0 + x) * G, bh, rank);
-            const int line = a.rec[rank].x;
-            const OpPos pos = op_pos(bh, a.L, a.heads, D);
-            const size_t off = (size_t)(pos.row0 + line * BS + r0) * pos.ld + pos.x0 + (lane % LPR) * 8;
+          if (i < n_my) {
+            const size_t off = (size_t)(rw + r0) * (a.heads ? a.heads * D : D) + x0 + (lane % LPR) * 8;
             u[x] = *reinterpret_cast<const uint4*>(a.dO + off);
             v[x] = *reinterpret_cast<const uint4*>(a.O + off);
-            ri[x] = (size_t)bh * a.L + line * BS + r0;
           }
         }
 #pragma unroll
         for (int x = 0; x < UN; ++x) {
+          const int i = i0 + x * UPS + mw / WPU;
+          const int out = __shfl_sync(0xffffffffu, l_out, i & 31);
           const float t = bf16_lo(u[x].x) * bf16_lo(v[x].x) + bf16_hi(u[x].x) * bf16_hi(v[x].x) + bf16_lo(u[x].y) * bf16_lo(v[x].y) +
                           bf16_hi(u[x].y) * bf16_hi(v[x].y) + bf16_lo(u[x].z) * bf16_lo(v[x].z) + bf16_hi(u[x].z) * bf16_hi(v[x].z) +
                           bf16_lo(u[x].w) * bf16_lo(v[x].w) + bf16_hi(u[x].w) * bf16_hi(v[x].w);
@@ -358,11 +407,11 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
 #pragma unroll
           for (int y = 1; y < LPR / 2; ++y) half += __shfl_sync(0xffffffffu, t, (lane & ~(LPR / 2 - 1)) + y);
           const float d = half + __shfl_xor_sync(0xffffffffu, half, LPR / 2);
-          if (lane % LPR == 0 && i0 + x < c.n_my && r0 < BS) a.delta_out[ri[x]] = d;
+          if (lane % LPR == 0 && i < n_my) a.delta_out[(size_t)out + r0] = d;
         }
       }
       __threadfence_block();
-      asm volatile("bar.sync 1, 544;" ::: "memory");                  // with warp 3, which hands delta out
+      asm volatile("bar.sync 1, 512;" ::: "memory");                  // delta of this CTA's rows is in global memory
     }
     // entry of the pair and query row of this lane: COL rows 0-63 first entry, 64-127 second; ROW second entry in lanes 16-31
     const int es = SIDE == COL ? q >> 1 : lane >> 4;
@@ -372,124 +421,112 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
     const float sc2 = a.scale * LOG2E, inv_scale = 1.0f / a.scale;
     bool ok = true;
     bool pend = false;                                                // a finished unit whose rows this group has to write
-    int pend_par = 0, pend_phase = 0;
-    __nv_bfloat16* pend_dst = nullptr;
-    int done0 = 0, done1 = 0;                                         // units that went to accumulator set 0 / 1
+    int pend_acc = 0, units = 0;                                      // its accumulator set; units written by this group before it
+    size_t pend_off = 0;
 
-    auto write_rows = [&](__nv_bfloat16* dst, uint32_t taddr, bool have, bool mine) {
-      constexpr int W = D / 2;
-      uint32_t v[W];
-      if (have) {
-        if constexpr (W == 32) tmem_ld32(taddr + g * W, v); else tmem_ld16(taddr + g * W, v);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int e = 0; e < W; ++e) v[e] = 0u;
-      }
-      if (!mine) return;
-#pragma unroll
-      for (int e = 0; e < W; e += 8)
-        *reinterpret_cast<uint4*>(dst + e) = make_uint4(pack_bf16(__uint_as_float(v[e]), __uint_as_float(v[e + 1])),
-                                                        pack_bf16(__uint_as_float(v[e + 2]), __uint_as_float(v[e + 3])),
-                                                        pack_bf16(__uint_as_float(v[e + 4]), __uint_as_float(v[e + 5])),
-                                                        pack_bf16(__uint_as_float(v[e + 6]), __uint_as_float(v[e + 7])));
-    };
-    const bool writes = SIDE == COL || lane < 16;
     auto flush = [&]() -> bool {
-      if (!wait_all(acc_done + 8 * pend_par, (uint32_t)pend_phase, ERR_MMA2_WAIT)) return false;
+      if (!wait_all(acc_done + 8 * (2 * grp + (units & 1)), (uint32_t)(units >> 1), ERR_MMA2_WAIT)) return false;
+      ++units;
       tc_fence_after();
-      write_rows(pend_dst, t_lane + ACC + (uint32_t)pend_par * 64u, true, writes);
+      __nv_bfloat16* dst = (SIDE == COL && lane >= 16 ? a.out1 : a.out0) + pend_off;
+      const uint32_t taddr = t_lane + ACC + (SIDE == ROW ? (uint32_t)(pend_acc & 1) * D : (uint32_t)pend_acc * D);
+      const bool mine = SIDE == COL || (lane >> 4) == (pend_acc >> 1);
+#pragma unroll
+      for (int h = 0; h < D; h += 32) {
+        if (WPG == 8 && h / 32 != g0) continue;
+        uint32_t v[32];
+        tmem_ld32(taddr + h, v);
+        tmem_ld_wait();
+        if (mine) {
+#pragma unroll
+          for (int x = 0; x < 32; x += 8)
+            *reinterpret_cast<uint4*>(dst + h + x) = make_uint4(pack_bf16(__uint_as_float(v[x]), __uint_as_float(v[x + 1])),
+                                                                pack_bf16(__uint_as_float(v[x + 2]), __uint_as_float(v[x + 3])),
+                                                                pack_bf16(__uint_as_float(v[x + 4]), __uint_as_float(v[x + 5])),
+                                                                pack_bf16(__uint_as_float(v[x + 6]), __uint_as_float(v[x + 7])));
+        }
+      }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_free + 8 * pend_par);
+      if (lane == 0) mbar_arrive(acc_free + 8 * pend_acc);
       pend = false;
       return true;
     };
 
-    int j = 0;
-    int stat_waits0 = 0, stat_waits1 = 0;
-    for (; c.valid() && ok; c.shift()) {
-      const int i = c.i, n = c.cur.w, par = i & 1;
-      const OpPos pos = op_pos(c.bh, a.L, a.heads, D);
-      __nv_bfloat16* dst = (SIDE == COL && lane >= 16 ? a.out1 : a.out0) + (size_t)(pos.row0 + c.cur.x * BS + orow) * pos.ld + pos.x0 + g * (D / 2);
-      if (n == 0) {                                                   // a unit without entries: zero rows
-        if (grp == (i & 1)) write_rows(dst, 0u, false, writes);
-        continue;
+    // record and statistics of this row are requested a pair early
+    int4 rec = make_int4(PF_END, 0, 0, 0);
+    float h_next = 0.f, d_next = 0.f;
+    auto request = [&](uint32_t j) -> bool {
+      if (!record(j, NGR, rec)) return false;
+      if (rec.x >= 0 && (es == 0 || (rec.x & PF_TWO))) {
+        const size_t ri = (size_t)rec.w * a.L + (SIDE == COL ? (es ? rec.y >> 16 : rec.y & 0xffff) : rec.z) * BS + row;
+        h_next = a.lse[ri];
+        d_next = SIDE == COL ? a.delta[ri] : __ldcg(a.delta_out + ri);            // ROW: written by this CTA
       }
-      const int npairs = c.pairs();
-      const float* kpu = a.keypad + (size_t)c.bh * a.L + g * 32;
-      float h = 0.f, nds = 0.f;
-      if (SIDE == ROW) {
-        const int w = par ? stat_waits1 : stat_waits0;
-        if (!wait_all(st_full + 8 * par, (uint32_t)w, ERR_MMA_WAIT)) { ok = false; break; }
-        if (par) ++stat_waits1; else ++stat_waits0;
-        const float* st = reinterpret_cast<const float*>(smem_raw + C::O_STAT) + par * 2 * 64;
-        h = st[row]; nds = st[64 + row];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(st_free + 8 * par);
-      }
-      for (int k = 0; k < npairs && ok; ++k, ++j) {
-        if ((j & 1) != grp) continue;
-        if (!wait_all(pi_full + 8 * grp, (uint32_t)(j >> 1), ERR_MMA_WAIT)) { ok = false; break; }
-        const bool mine = 2 * k + es < n;
-        const int* info = reinterpret_cast<const int*>(smem_raw + C::O_INFO) + 4 * grp;
-        const int flags = info[0], oth = info[1 + es];
-        if (SIDE == COL) {
-          const float* st = reinterpret_cast<const float*>(smem_raw + C::O_STAT) + grp * 2 * 128 + es * 64 + row;
-          h = st[0]; nds = st[128];
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(pi_free + 8 * grp);
-        // blocks without padded keys (most of them) take no penalty; columns are keys in both
-        const float* kp = ((flags >> (SIDE == COL ? 0 : es)) & 1) ? kpu + (SIDE == COL ? c.cur.x : oth) * BS : nullptr;
-        const int sb = (SIDE == COL ? (q & 1) : (q >> 1)) * 2 + g;      // quarter: 2 (query / 32) + key / 32
-        const bool live = !SUB || ((flags >> (8 + 8 * es + sb)) & 1);
-        // the group's value tiles must have been consumed (pair j - 2)
-        if (j >= 2 && !wait_all(pdone + 8 * ((j - 2) % NP), (uint32_t)((j - 2) / NP), ERR_MMA2_WAIT)) { ok = false; break; }
-        if (!wait_all(s_ready + 8 * (j % 3), (uint32_t)(j / 3), ERR_MMA_WAIT)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t ts = t_lane + (uint32_t)(j % 3) * 128u + g * 32;
+      return true;
+    };
+    ok = request(grp);
+    for (uint32_t j = grp; ok && rec.x >= 0; j += NGR) {
+      const int flags = rec.x, line = rec.z, key = SIDE == COL ? rec.z : es ? rec.y >> 16 : rec.y & 0xffff, bh = rec.w;
+      const float h = h_next, nds = -d_next * a.scale;
+      if (!request(j + NGR)) { ok = false; break; }
+      const uint32_t ps = j % NP, set = j % 3;
+      const bool mine = es == 0 || (flags & PF_TWO);
+      // COL: the value tiles of pair j - NPD must have been consumed
+      if (SIDE == COL && j >= C::NPD && !wait_all(pdone + 8 * ((j - C::NPD) % NP), (j - C::NPD) / NP, ERR_MMA2_WAIT)) { ok = false; break; }
+      if (!wait_all(s_ready + 8 * (j % C::NS), j / C::NS, ERR_MMA_WAIT)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t ts = t_lane + set * 128u;
+      const uint32_t tds = sbase + (SIDE == COL ? C::O_PD + (j % (SIDE == COL ? C::NPD : 1)) * C::PD : ps * C::SLOT + 2 * T::BYTES) + es * VT_BYTES + row * 128;
+      const uint64_t sc22 = pack2(sc2, sc2), scale2 = pack2(a.scale, a.scale), nds2 = pack2(nds, nds), nh2 = pack2(-h, -h);
+#pragma unroll
+      for (int hf = 0; hf < C::HALVES; ++hf) {
+        const int g = C::HALVES == 2 ? hf : g0;                       // 32 columns (keys)
         uint32_t sv[32], gv[32];
-        tmem_ld32(ts, sv);
-        tmem_ld32(ts + 64u, gv);
+        tmem_ld32(ts + g * 32, sv);
+        tmem_ld32(ts + 64u + g * 32, gv);
         tmem_ld_wait();
+        if (hf + 1 == C::HALVES) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(t_free + 8 * set);
+        }
         if (mine) {
-          if (kp) take_penalty(sv, kp, inv_scale);
-          const uint32_t tds = sbase + C::O_PD + grp * C::PD + es * VT_BYTES + row * 128, tp = tds + 2 * VT_BYTES;
-          const uint64_t sc22 = pack2(sc2, sc2), scale2 = pack2(a.scale, a.scale), nds2 = pack2(nds, nds), nh2 = pack2(-h, -h);
+          // blocks without padded keys (most of them) take no penalty; columns are keys in both
+          if ((flags >> es) & 1) take_penalty(sv, a.keypad + (size_t)bh * a.L + key * BS + g * 32, inv_scale);
+          const int sb = (SIDE == COL ? (q & 1) : (q >> 1)) * 2 + g;  // quarter: 2 (query / 32) + key / 32
+          const bool live = !SUB || ((flags >> (8 + 8 * es + sb)) & 1);
           auto piece = [&](int cc) {             // eight columns: one 16-byte piece of each tile
             uint32_t wp[4], wd[4];
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-              const int e = cc * 8 + 2 * x;
+              const int c = cc * 8 + 2 * x;
               float p0, p1, d0, d1;
-              unpack2(fma2(pack2(sv[e], sv[e + 1]), sc22, nh2), p0, p1);
+              unpack2(fma2(pack2(sv[c], sv[c + 1]), sc22, nh2), p0, p1);
               p0 = ex2_approx(p0); p1 = ex2_approx(p1);
               wp[x] = pack_bf16(p0, p1);
-              unpack2(mul2(pack2(p0, p1), fma2(pack2(gv[e], gv[e + 1]), scale2, nds2)), d0, d1);
+              unpack2(mul2(pack2(p0, p1), fma2(pack2(gv[c], gv[c + 1]), scale2, nds2)), d0, d1);
               wd[x] = pack_bf16(d0, d1);
               if (SUB && !live) { wp[x] = 0u; wd[x] = 0u; }
             }
             const uint32_t off = (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4);
             st_shared_v4(tds + off, wd);
-            if (SIDE == COL) st_shared_v4(tp + off, wp);
+            if (SIDE == COL) st_shared_v4(tds + 2 * VT_BYTES + off, wp);
           };
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) piece(cc);
         }
-        tc_fence_before();
-        fence_proxy_async();                                          // tiles -> visible to the MMAs
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(t_free + 8 * (j % 3));
-          mbar_arrive(p_ready + 8 * grp);
-        }
-        if (pend) ok = flush();                                       // an earlier unit: its last products have long been issued
-        if (k + 1 == npairs) {                                        // this group worked on the unit's last pair: it writes the rows
-          pend = true; pend_par = par; pend_dst = dst; pend_phase = par ? done1 : done0;
-        }
       }
-      if (par) ++done1; else ++done0;
+      fence_proxy_async();                                            // tiles -> visible to the MMAs
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_ready + 8 * ps);
+      if (pend) ok = flush();                                         // an earlier unit: its last products have long been issued
+      if (flags & PF_LAST) {                                          // this group worked on the unit's last pair: it writes the rows
+        pend = true;
+        pend_acc = (flags >> 4) & 3;
+        const OpPos pos = op_pos(bh, a.L, a.heads, D);
+        pend_off = (size_t)(pos.row0 + line * BS + orow) * pos.ld + pos.x0;
+      }
     }
     if (ok && pend) flush();
   }

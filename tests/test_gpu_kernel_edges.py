@@ -71,6 +71,18 @@ def test_streaming_forward_and_backward(d, bs, padded, case):
     assert torch.equal(out, got[0].detach())
 
 
+@pytest.mark.parametrize("d,nb", [(64, 5), (32, 5), (32, 1)])
+def test_streaming_kernels_with_many_units(d, nb):
+    """More than 32 block rows per CTA, some without entries: the records of a CTA's pairs are made 32 lines and 16 pairs at a time."""
+    from spion_b200.native import BlockSparseAttention
+    B, H, L = (400, 3, 5 * 64) if nb > 1 else (1900, 3, 64)
+    Q, K, V, dO = (t.to(torch.bfloat16) for t in synthetic.qkv(7 + d, B, H, L, d))
+    mat = lines_of_every_length(nb, True) if nb > 1 else np.ones((1, 1), np.uint8)
+    kp = synthetic.key_padding(4, B, L)
+    mod = BlockSparseAttention(cfg(B, H, L, d, 64), dtype=torch.bfloat16, keypad=True, recompute=True, return_probs=False)
+    compare(run(mod, Q, K, V, dO, mat, kp), Q, K, V, dO, mat, 64, kp, BF16_REL, True)
+
+
 # (bs, d, B, H, blocks per side): few threads' worth of work (four rows per thread), more (eight; columns split over clusters), many
 # (eight; one CTA per column group); groups of four matrices with one, two and three left over
 @pytest.mark.parametrize("bs,d,B,H,nb", [(32, 32, 1, 1, 1), (32, 64, 1, 3, 7), (64, 32, 1, 1, 2), (64, 64, 2, 1, 9),
