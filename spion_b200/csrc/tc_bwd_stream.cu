@@ -163,11 +163,12 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
   if (warp == 0) {
     // ================================================================== loads
     int u = 0, ps = 0, round = 0;
-    for (uint32_t j = 0;; ++j) {
-      int4 r;
-      if (!record(j, 1, r) || r.x < 0) break;
+    int4 next;
+    bool ok = record(0, 1, next);
+    for (uint32_t j = 0; ok && next.x >= 0; ++j) {
+      const int4 r = next;
       if (round >= 1 && !wait_all(pdone + 8 * ps, (uint32_t)(round - 1), ERR_MMA2_WAIT)) break;
-      const bool first = warp_uniform(r.x & PF_FIRST) != 0, two = warp_uniform(r.x & PF_TWO) != 0;
+      const bool first = __any_sync(0xffffffffu, r.x & PF_FIRST), two = __any_sync(0xffffffffu, r.x & PF_TWO);
       const int fs = u & 1;
       if (first && u >= 2 && !wait_all(f_free + 8 * fs, (uint32_t)((u >> 1) - 1), ERR_MMA2_WAIT)) break;
       const OpPos pos = op_pos(r.w, a.L, a.heads, D);
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         }
       }
       __syncwarp();
+      ok = record(j + 1, 1, next);
       if (r.x & PF_LAST) ++u;
       if (++ps == NP) { ps = 0; ++round; }
     }
@@ -197,14 +199,15 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
     constexpr uint32_t IDESC = make_idesc_bf16(SIDE == COL ? 128 : 64, 64, 0, 0);
     const uint64_t KM = T::kmajor(sbase, 0);
     int u = 0, ps = 0, round = 0, set = 0, sround = 0, sr = 0;
-    for (uint32_t j = 0;; ++j) {
-      int4 r;
-      if (!record(j, 1, r) || r.x < 0) break;
+    int4 next;
+    bool ok = record(0, 1, next);
+    for (uint32_t j = 0; ok && next.x >= 0; ++j) {
+      const int4 r = next;
       const int par = u & 1;
       if (sround >= 1 && !wait_all(t_free + 8 * set, (uint32_t)(sround - 1), ERR_MMA_WAIT)) break;
       if ((r.x & PF_FIRST) && !wait_all(f_full + 8 * par, (uint32_t)(u >> 1), ERR_LOAD_WAIT)) break;
       if (!wait_all(pfull + 8 * ps, (uint32_t)round, ERR_LOAD_WAIT)) break;
-      const bool last = warp_uniform(r.x & PF_LAST) != 0, two = warp_uniform(r.x & PF_TWO) != 0;
+      const bool last = __any_sync(0xffffffffu, r.x & PF_LAST), two = __any_sync(0xffffffffu, r.x & PF_TWO);
       if (elect_one()) {
         tc_fence_after();
         const uint64_t a0 = desc_advance(KM, ps * C::SLOT), a1 = desc_advance(a0, 2 * T::BYTES);
@@ -232,6 +235,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         if (last) mma_commit(f_free + 8 * par);                       // the fixed tiles are read by these products only
       }
       __syncwarp();
+      ok = record(j + 1, 1, next);
       if (++ps == NP) { ps = 0; ++round; }
       if (++set == 3) { set = 0; ++sround; }
       if (++sr == C::NS) sr = 0;
@@ -244,13 +248,14 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
     const uint64_t MN = T::mnmajor(sbase, 0), VT = SIDE == COL ? ValTile::mnmajor(sbase, 0) : ValTile::kmajor(sbase, 0);
     int u = 0, ps = 0, round = 0, grp = 0, pd = 0;
     uint32_t odd = 0;                                                 // bit g: group g has written an odd number of units
-    for (uint32_t j = 0;; ++j) {
-      int4 r;
-      if (!record(j, 1, r) || r.x < 0) break;
+    int4 next;
+    bool ok = record(0, 1, next);
+    for (uint32_t j = 0; ok && next.x >= 0; ++j) {
+      const int4 r = next;
       const int x = u % NACC;
       if ((r.x & PF_FIRST) && u >= NACC && !wait_all(acc_free + 8 * x, (uint32_t)(u / NACC - 1), ERR_MMA2_WAIT)) break;
       if (!wait_all(p_ready + 8 * ps, (uint32_t)round, ERR_MMA_WAIT)) break;
-      const bool last = warp_uniform(r.x & PF_LAST) != 0, two = warp_uniform(r.x & PF_TWO) != 0, fresh = warp_uniform(r.x & PF_FIRST) != 0;
+      const bool last = __any_sync(0xffffffffu, r.x & PF_LAST), two = __any_sync(0xffffffffu, r.x & PF_TWO), fresh = __any_sync(0xffffffffu, r.x & PF_FIRST);
       if (elect_one()) {
         tc_fence_after();
         const uint32_t acc = tmem + acc_at(x);
@@ -274,6 +279,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         if (last) mma_commit(acc_done + 8 * (2 * grp + ((odd >> grp) & 1)));
       }
       __syncwarp();
+      ok = record(j + 1, 1, next);
       if (++ps == NP) { ps = 0; ++round; }
       if (last) { ++u; odd ^= 1u << grp; }
       if (++grp == NGR) grp = 0;
