@@ -50,6 +50,11 @@ struct Cfg {
   static_assert(TN == 2 || TN == 4 || TN == 8, "unsupported shape");
 };
 
+// A CTA has W > 1 groups of NT threads that share a block row, or (W == 1) G groups with a problem each.
+template <int BS, int D, int R, int W> constexpr int cta_threads() { return W > 1 ? W * Cfg<BS, D, R>::NT : Cfg<BS, D, R>::CTA; }
+template <int BS, int D, int R, int W> constexpr int cta_groups() { return W > 1 ? W : Cfg<BS, D, R>::G; }
+template <int BS, int D, int R, int W> constexpr int cta_resident(int n) { return W > 1 ? 512 / (W * Cfg<BS, D, R>::NT) : n; }
+
 // float offset of 16-byte piece `piece` of row `row` in a tile of COLS columns
 template <int COLS>
 __device__ __forceinline__ int at(int row, int piece) { return row * COLS + ((piece ^ ((row >> 2) & 7)) << 2); }
@@ -233,6 +238,32 @@ struct Sums {
   }
 };
 
+// W groups: the first adds the sums of the others, in their order.  `place`: this group's shared memory, bs x d floats that nobody reads
+// any more once every thread of the group is here.
+template <int BS, int D, int R, int W>
+__device__ __forceinline__ void join_sums(float* place, int group_floats, int g, int t, Sums<BS, D, R>& s) {
+  using C = Cfg<BS, D, R>;
+  constexpr int NT = C::NT;
+  pair_t* mine = reinterpret_cast<pair_t*>(place) + t;            // pair i of thread t at i * NT + t
+  if (g > 0) {
+#pragma unroll
+    for (int x = 0; x < R / 2; ++x)
+#pragma unroll
+      for (int y = 0; y < C::TN; ++y) mine[(x * C::TN + y) * NT] = s.v[x][y];
+  }
+  __syncthreads();
+  if (g == 0) {
+#pragma unroll
+    for (int q = 1; q < W; ++q) {
+      const pair_t* theirs = reinterpret_cast<const pair_t*>(place + q * group_floats) + t;
+#pragma unroll
+      for (int x = 0; x < R / 2; ++x)
+#pragma unroll
+        for (int y = 0; y < C::TN; ++y) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s.v[x][y]) : "l"(theirs[(x * C::TN + y) * NT]));
+    }
+  }
+}
+
 // acc += sum_i Vt[i][rows] * B[i][columns]   (Vt: [bs x bs] value tile, transposed use; B: [bs x d])
 template <int BS, int D, int R>
 __device__ __forceinline__ void tile_atb(const float* Vt, const float* Bs, int ty, int tx, Sums<BS, D, R>& acc) {
@@ -317,8 +348,9 @@ template <int BS, int D, int R> __host__ __device__ constexpr int two_pass_float
 // The K (pass 1) and V (pass 2) tiles are double-buffered: the copy of tile k+1 is in flight while
 // tile k is used.  Every thread keeps the maximum and the sum of its own columns of a row; the threads of a row join them
 // once, after the last tile.
-template <int BS, int D, int R>
-__global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) fused_fwd_kernel(const float* __restrict__ Q, OperandLayout lq,
+// W > 1: W groups of threads take a share of the row's blocks each; maxima and denominators are joined between the passes, O at the end.
+template <int BS, int D, int R, int W>
+__global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D, R, W>(Cfg<BS, D, R>::RESIDENT2)) fused_fwd_kernel(const float* __restrict__ Q, OperandLayout lq,
                                                            const float* __restrict__ K, OperandLayout lk,
                                                            const float* __restrict__ V, OperandLayout lv,
                                                            const float* __restrict__ keypad, float floor_v, float* P,
@@ -328,7 +360,7 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int r = blockIdx.x, bh = blockIdx.y * C::G + g;
+  const int r = blockIdx.x, bh = W > 1 ? blockIdx.y : blockIdx.y * C::G + g;
   if (bh >= BH) return;
   float* Qs = smem + g * two_pass_floats<BS, D, R>();
   float* Bs = Qs + ONE<BS, D, R>;                                // two buffers: K tiles, then V tiles
@@ -336,6 +368,7 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
 
   const int rp = p.row_ptr[r], nblk = p.row_ptr[r + 1] - rp;
   const int* cols = p.col_idx + rp;
+  const int k0 = W > 1 ? nblk * g / W : 0, k1 = W > 1 ? nblk * (g + 1) / W : nblk;      // this group's blocks
   const Operand Kb(K, lk, bh), Vb(V, lv, bh);
   float* Pb = P + (long long)bh * vl.bh_stride;
   const float* kp = keypad ? keypad + (long long)bh * L + tx * 4 : nullptr;
@@ -344,22 +377,22 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
   float* mine = Pb + rt.base + ty * R * rt.si + tx * 4;         // the thread's values of the row's first tile
   const float scale2 = scale * LOG2_E;                          // scores in base-2 units
 
-  int c_cur = nblk > 0 ? cols[0] : 0, c_nxt = nblk > 1 ? cols[1] : 0;
+  int c_cur = k0 < k1 ? cols[k0] : 0, c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
   load_tile<BS, D, C::NT>(Qs, Operand(Q, lq, bh), r * BS, t);
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Kb, c_cur * BS, t);
+  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Kb, c_cur * BS, t);
   cp_async_commit();
 
   // ---- pass 1: scores into the P tiles, running maximum and denominator per row
   float m[R], l[R];
 #pragma unroll
   for (int x = 0; x < R; ++x) { m[x] = floor_v * LOG2_E; l[x] = 0.f; }
-  for (int k = 0; k < nblk; ++k) {
+  for (int k = k0; k < k1; ++k) {
     const int c = c_cur;
-    if (k + 1 < nblk)
+    if (k + 1 < k1)
       load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
-    c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
+    c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
     float pad[4] = {0.f, 0.f, 0.f, 0.f};
     if (kp) {
 #pragma unroll
@@ -386,18 +419,38 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
     }
     group_sync<C::NT>(g);                                        // buffer k&1 may be refilled
   }
-  c_cur = nblk > 0 ? cols[0] : 0;
-  c_nxt = nblk > 1 ? cols[1] : 0;
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Vb, c_cur * BS, t);
+  c_cur = k0 < k1 ? cols[k0] : 0;
+  c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
+  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Vb, c_cur * BS, t);
   cp_async_commit();
   float inv[R];
 #pragma unroll
   for (int x = 0; x < R; ++x) {
     const float row_m = group_max<C::TX>(m[x]);
-    const float z = group_sum<C::TX>(l[x] * ex2(m[x] - row_m)) + (float)(L - nblk * BS) * ex2(-row_m);
+    const float z = group_sum<C::TX>(l[x] * ex2(m[x] - row_m));
     m[x] = row_m;
-    inv[x] = 1.0f / z;
+    inv[x] = z;
   }
+  if (W > 1) {                                                   // join the groups' maxima and sums
+    float2* stat = reinterpret_cast<float2*>(smem + W * two_pass_floats<BS, D, R>());       // [W][BS]
+    if (tx == 0) {
+#pragma unroll
+      for (int x = 0; x < R; ++x) stat[g * BS + ty * R + x] = make_float2(m[x], inv[x]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < R; ++x) {
+      float row_m = m[x], z = 0.f;
+#pragma unroll
+      for (int q = 0; q < W; ++q) row_m = fmaxf(row_m, stat[q * BS + ty * R + x].x);
+#pragma unroll
+      for (int q = 0; q < W; ++q) z = fmaf(stat[q * BS + ty * R + x].y, ex2(stat[q * BS + ty * R + x].x - row_m), z);
+      m[x] = row_m;
+      inv[x] = z;
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < R; ++x) inv[x] = 1.0f / (inv[x] + (float)(L - nblk * BS) * ex2(-m[x]));
 
   // ---- pass 2: probabilities over the scores, O = P V
   Sums<BS, D, R> o;
@@ -407,9 +460,9 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
 #pragma unroll
     for (int x = 0; x < R; ++x) sc[x] = load_vals(tile + x * rt.si, vec);
   };
-  if (nblk > 0) fetch_scores(0);
-  for (int k = 0; k < nblk; ++k) {
-    if (k + 1 < nblk)
+  if (k0 < k1) fetch_scores(k0);
+  for (int k = k0; k < k1; ++k) {
+    if (k + 1 < k1)
       load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
     cp_async_commit();
     float* tile = mine + (long long)k * rt.step;
@@ -426,22 +479,27 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
       }
       put_transposed<BS>(Ps, R / 4 * ty + half, tx, pr);
     }
-    if (k + 1 < nblk) fetch_scores(k + 1);                       // in flight during the product below
+    if (k + 1 < k1) fetch_scores(k + 1);                       // in flight during the product below
     c_cur = c_nxt;
-    c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
+    c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
     cp_async_wait<1>();
     group_sync<C::NT>(g);                                        // V tile k has landed, Ps is complete
     tile_atb<BS, D, R>(Ps, Bs + (k & 1) * C::TILE, ty, tx, o);
     group_sync<C::NT>(g);                                        // Ps and buffer k&1 may be overwritten
   }
   cp_async_wait<0>();
+  if (W > 1) {
+    group_sync<C::NT>(g);
+    join_sums<BS, D, R, W>(Qs, two_pass_floats<BS, D, R>(), g, t, o);
+    if (g > 0) return;
+  }
   store_out<BS, D, R>(O + (long long)bh * lo.bh_stride, lo, r * BS, ty, tx, o);
 }
 
 // ------------------------------------------------------------------------------ backward, row side
 //   t = dP.P ; s = rowsum(t) ; dS = (t - P s) scale ; dQ = dS K     (models/block_attn.cu:90-130, :498-516)
-template <int BS, int D, int R>
-__global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) fused_bwd_row_kernel(const float* __restrict__ dO, OperandLayout ldo,
+template <int BS, int D, int R, int W>
+__global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D, R, W>(Cfg<BS, D, R>::RESIDENT2)) fused_bwd_row_kernel(const float* __restrict__ dO, OperandLayout ldo,
                                                                const float* __restrict__ V, OperandLayout lv,
                                                                const float* __restrict__ K, OperandLayout lk,
                                                                const float* __restrict__ P, ValueLayout vp, float* dS,
@@ -451,7 +509,7 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int r = blockIdx.x, bh = blockIdx.y * C::G + g;
+  const int r = blockIdx.x, bh = W > 1 ? blockIdx.y : blockIdx.y * C::G + g;
   if (bh >= BH) return;
   float* As = smem + g * two_pass_floats<BS, D, R>();              // dO tile
   float* Bs = As + ONE<BS, D, R>;                                // two buffers: V tiles, then K tiles
@@ -459,27 +517,28 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
 
   const int rp = p.row_ptr[r], nblk = p.row_ptr[r + 1] - rp;
   const int* cols = p.col_idx + rp;
+  const int k0 = W > 1 ? nblk * g / W : 0, k1 = W > 1 ? nblk * (g + 1) / W : nblk;      // this group's blocks
   const Operand Vb(V, lv, bh), Kb(K, lk, bh);
   const RowTiles rp_t = RowTiles::of<BS>(vp, rp, nblk), rs_t = RowTiles::of<BS>(vds, rp, nblk);
   const float* Pb = P + (long long)bh * vp.bh_stride + rp_t.base + ty * R * rp_t.si + tx * 4;   // the thread's values of the first tile
   float* dSb = dS + (long long)bh * vds.bh_stride + rs_t.base + ty * R * rs_t.si + tx * 4;
   const bool vec_p = vec_ok(Pb), vec_s = vec_ok(dSb);
 
-  int c_cur = nblk > 0 ? cols[0] : 0, c_nxt = nblk > 1 ? cols[1] : 0;
+  int c_cur = k0 < k1 ? cols[k0] : 0, c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
   load_tile<BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Vb, c_cur * BS, t);
+  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Vb, c_cur * BS, t);
   cp_async_commit();
 
   // ---- pass 1: dP into the dS tiles, row sums of dP.P
   float s[R];
 #pragma unroll
   for (int x = 0; x < R; ++x) s[x] = 0.f;
-  for (int k = 0; k < nblk; ++k) {
-    if (k + 1 < nblk)
+  for (int k = k0; k < k1; ++k) {
+    if (k + 1 < k1)
       load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
-    c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
+    c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
     float4 pv[R];                                                // requested before the wait: both latencies overlap
 #pragma unroll
     for (int x = 0; x < R; ++x) pv[x] = load_vals(Pb + (long long)k * rp_t.step + x * rp_t.si, vec_p);
@@ -503,19 +562,33 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
   }
 #pragma unroll
   for (int x = 0; x < R; ++x) s[x] = group_sum<C::TX>(s[x]);
+  if (W > 1) {
+    float* stat = smem + W * two_pass_floats<BS, D, R>();        // [W][BS]
+    if (tx == 0) {
+#pragma unroll
+      for (int x = 0; x < R; ++x) stat[g * BS + ty * R + x] = s[x];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < R; ++x) {
+      s[x] = 0.f;
+#pragma unroll
+      for (int q = 0; q < W; ++q) s[x] += stat[q * BS + ty * R + x];
+    }
+  }
 
   // ---- pass 2: dS over dP, dQ = dS K
   Sums<BS, D, R> o;
-  c_cur = nblk > 0 ? cols[0] : 0;
-  c_nxt = nblk > 1 ? cols[1] : 0;
-  if (nblk > 0) load_tile<BS, D, C::NT>(Bs, Kb, c_cur * BS, t);
+  c_cur = k0 < k1 ? cols[k0] : 0;
+  c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
+  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Kb, c_cur * BS, t);
   cp_async_commit();
-  for (int k = 0; k < nblk; ++k) {
-    if (k + 1 < nblk)
+  for (int k = k0; k < k1; ++k) {
+    if (k + 1 < k1)
       load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
-    c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
+    c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
 #pragma unroll
     for (int half = 0; half < R / 4; ++half) {
       float ds[4][4];
@@ -538,14 +611,19 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT2) 
     group_sync<C::NT>(g);
   }
   cp_async_wait<0>();
+  if (W > 1) {
+    group_sync<C::NT>(g);
+    join_sums<BS, D, R, W>(As, two_pass_floats<BS, D, R>(), g, t, o);
+    if (g > 0) return;
+  }
   store_out<BS, D, R>(dQ + (long long)bh * ldq.bh_stride, ldq, r * BS, ty, tx, o);
 }
 
 // Row backward when O is at hand: rowsum(dP.P) = rowsum(dO.O) (delta), so dS of a tile needs nothing
 // from the other tiles of its row and one pass suffices.  Two stages per block, V tile (for dP) and
 // K tile (for dQ); the copy of one is in flight while the other is used.
-template <int BS, int D, int R>
-__global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) fused_bwd_row_delta_kernel(const float* __restrict__ dO, OperandLayout ldo,
+template <int BS, int D, int R, int W>
+__global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D, R, W>(Cfg<BS, D, R>::RESIDENT)) fused_bwd_row_delta_kernel(const float* __restrict__ dO, OperandLayout ldo,
                                                                      const float* __restrict__ O, OperandLayout lo,
                                                                      const float* __restrict__ V, OperandLayout lv,
                                                                      const float* __restrict__ K, OperandLayout lk,
@@ -557,7 +635,7 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int r = blockIdx.x, bh = blockIdx.y * C::G + g;
+  const int r = blockIdx.x, bh = W > 1 ? blockIdx.y : blockIdx.y * C::G + g;
   if (bh >= BH) return;
   float* As = smem + g * (3 * C::TILE + C::VALS);               // dO tile
   float* Vs = As + C::TILE;
@@ -566,17 +644,18 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
 
   const int rp = p.row_ptr[r], nblk = p.row_ptr[r + 1] - rp;
   const int* cols = p.col_idx + rp;
+  const int k0 = W > 1 ? nblk * g / W : 0, k1 = W > 1 ? nblk * (g + 1) / W : nblk;      // this group's blocks
   const Operand Vb(V, lv, bh), Kb(K, lk, bh);
   const RowTiles rp_t = RowTiles::of<BS>(vp, rp, nblk), rs_t = RowTiles::of<BS>(vds, rp, nblk);
   const float* Pb = P + (long long)bh * vp.bh_stride + rp_t.base + ty * R * rp_t.si + tx * 4;   // the thread's values of the first tile
   float* dSb = dS + (long long)bh * vds.bh_stride + rs_t.base + ty * R * rs_t.si + tx * 4;
   const bool vec_p = vec_ok(Pb), vec_s = vec_ok(dSb);
 
-  int c_cur = nblk > 0 ? cols[0] : 0, c_nxt = nblk > 1 ? cols[1] : 0;
+  int c_cur = k0 < k1 ? cols[k0] : 0, c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
   load_tile<BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
-  if (nblk > 0) load_tile<BS, D, C::NT>(Vs, Vb, c_cur * BS, t);
+  if (k0 < k1) load_tile<BS, D, C::NT>(Vs, Vb, c_cur * BS, t);
   cp_async_commit();
-  if (nblk > 0) load_tile<BS, D, C::NT>(Ks, Kb, c_cur * BS, t);
+  if (k0 < k1) load_tile<BS, D, C::NT>(Ks, Kb, c_cur * BS, t);
   cp_async_commit();
 
   float delta[R];
@@ -588,12 +667,12 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
 #pragma unroll
     for (int x = 0; x < R; ++x) pv[x] = load_vals(Pb + (long long)k * rp_t.step + x * rp_t.si, vec_p);
   };
-  if (nblk > 0) fetch_p(0);
+  if (k0 < k1) fetch_p(k0);
 
-  for (int k = 0; k < nblk; ++k) {
+  for (int k = k0; k < k1; ++k) {
     cp_async_wait<1>();
     group_sync<C::NT>(g);                                        // V tile k (and dO) have landed
-    if (k == 0) {
+    if (k == k0) {
       const float* Ob = O + (long long)bh * lo.bh_stride + (long long)(r * BS + ty * R) * lo.sl;
 #pragma unroll
       for (int x = 0; x < R; ++x) {
@@ -619,7 +698,7 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
       put_transposed<BS>(Ss, R / 4 * ty + half, tx, acc);
     }
     group_sync<C::NT>(g);                                        // Ss complete, V buffer free
-    if (k + 1 < nblk) {
+    if (k + 1 < k1) {
       load_tile<BS, D, C::NT>(Vs, Vb, c_nxt * BS, t);
       fetch_p(k + 1);
     }
@@ -628,12 +707,17 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
     group_sync<C::NT>(g);                                        // K tile k has landed
     tile_atb<BS, D, R>(Ss, Ks, ty, tx, o);
     group_sync<C::NT>(g);                                        // Ss and the K buffer are free
-    if (k + 1 < nblk) load_tile<BS, D, C::NT>(Ks, Kb, c_nxt * BS, t);
+    if (k + 1 < k1) load_tile<BS, D, C::NT>(Ks, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
-    c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
+    c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
   }
   cp_async_wait<0>();
+  if (W > 1) {
+    group_sync<C::NT>(g);
+    join_sums<BS, D, R, W>(As, 3 * C::TILE + C::VALS, g, t, o);
+    if (g > 0) return;
+  }
   store_out<BS, D, R>(dQ + (long long)bh * ldq.bh_stride, ldq, r * BS, ty, tx, o);
 }
 
@@ -750,61 +834,68 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
   store_out<BS, D, R>(dV + (long long)bh * ldv.bh_stride, ldv, c * BS, ty, tx, av);
 }
 
-template <int BS, int D, int R> constexpr size_t smem_two_pass() { return sizeof(float) * Cfg<BS, D, R>::G * two_pass_floats<BS, D, R>(); }
-template <int BS, int D, int R> constexpr size_t smem_row() { return sizeof(float) * Cfg<BS, D, R>::G * (3 * Cfg<BS, D, R>::TILE + Cfg<BS, D, R>::VALS); }
+template <int BS, int D, int R, int W> constexpr size_t smem_two_pass() {
+  return sizeof(float) * (cta_groups<BS, D, R, W>() * two_pass_floats<BS, D, R>() + (W > 1 ? 2 * W * BS : 0));
+}
+template <int BS, int D, int R, int W> constexpr size_t smem_row() {
+  return sizeof(float) * cta_groups<BS, D, R, W>() * (3 * Cfg<BS, D, R>::TILE + Cfg<BS, D, R>::VALS);
+}
 template <int BS, int D, int R> constexpr size_t smem_col() { return sizeof(float) * Cfg<BS, D, R>::G * (2 * Cfg<BS, D, R>::TILE + 2 * Cfg<BS, D, R>::VALS); }
 
 constexpr int SPLIT_WAVES = 4;
 
-template <int BS, int D, int R>
+template <int BS, int D, int R, int W>
 int set_attrs() {
   static std::atomic<bool> done[64];
   int dev = 0;
   SPION_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 64 && done[dev].load(std::memory_order_acquire)) return SPION_OK;
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_fwd_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R>()));
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R>()));
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_delta_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D, R>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_fwd_kernel<BS, D, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R, W>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_kernel<BS, D, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R, W>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_delta_kernel<BS, D, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D, R, W>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
   if (dev < 64) done[dev].store(true, std::memory_order_release);
   return SPION_OK;
 }
 
-template <int BS, int D, int R>
+template <int BS, int D, int R, int W>
 int fwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V, OperandLayout lv,
                const float* keypad, float floor_v, float* P, ValueLayout vl, float* O, OperandLayout lo, Pattern p,
                int BH, int L, float scale, cudaStream_t st) {
-  int rc = set_attrs<BS, D, R>();
+  int rc = set_attrs<BS, D, R, W>();
   if (rc) return rc;
-  const dim3 grid(p.nb, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
-  fused_fwd_kernel<BS, D, R><<<grid, Cfg<BS, D, R>::CTA, smem_two_pass<BS, D, R>(), st>>>(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH,
+  const dim3 grid(p.nb, W > 1 ? BH : (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
+  fused_fwd_kernel<BS, D, R, W><<<grid, cta_threads<BS, D, R, W>(), smem_two_pass<BS, D, R, W>(), st>>>(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH,
                                                                L, scale);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
 
-template <int BS, int D, int R>
+template <int BS, int D, int R, int W>
 int bwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V, OperandLayout lv,
                const float* P, ValueLayout vp, const float* O, OperandLayout lo, const float* dO, OperandLayout ldo,
                float* dS, ValueLayout vds, float* dQ, OperandLayout ldq, float* dK, OperandLayout ldk, float* dV,
                OperandLayout ldv, Pattern p, int BH, float scale, cudaStream_t st, spion_ctx* prof) {
-  int rc = set_attrs<BS, D, R>();
+  int rc = set_attrs<BS, D, R, W>();
   if (rc) return rc;
-  const dim3 grid(p.nb, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
+  const dim3 grid(p.nb, W > 1 ? BH : (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
   if (O)
-    fused_bwd_row_delta_kernel<BS, D, R><<<grid, Cfg<BS, D, R>::CTA, smem_row<BS, D, R>(), st>>>(dO, ldo, O, lo, V, lv, K, lk, P, vp, dS, vds,
+    fused_bwd_row_delta_kernel<BS, D, R, W><<<grid, cta_threads<BS, D, R, W>(), smem_row<BS, D, R, W>(), st>>>(dO, ldo, O, lo, V, lv, K, lk, P, vp, dS, vds,
                                                                            dQ, ldq, p, BH, scale);
   else
-    fused_bwd_row_kernel<BS, D, R><<<grid, Cfg<BS, D, R>::CTA, smem_two_pass<BS, D, R>(), st>>>(dO, ldo, V, lv, K, lk, P, vp, dS, vds, dQ, ldq, p,
+    fused_bwd_row_kernel<BS, D, R, W><<<grid, cta_threads<BS, D, R, W>(), smem_two_pass<BS, D, R, W>(), st>>>(dO, ldo, V, lv, K, lk, P, vp, dS, vds, dQ, ldq, p,
                                                                      BH, scale);
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_BWD_ROW);
   // Many (b,h) matrices even out columns of different lengths by themselves; below SPLIT_WAVES waves of CTAs the longest
   // column would decide, and there is room for the CTAs that a split column takes.
-  if ((long long)grid.x * grid.y < (long long)SPLIT_WAVES * sm_count() * Cfg<BS, D, R>::RESIDENT) {
+  const dim3 cgrid(p.nb, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
+  // Many (b,h) matrices even out columns of different lengths by themselves; below SPLIT_WAVES waves of CTAs the longest
+  // column would decide, and there is room for the CTAs that a split column takes.
+  if ((long long)cgrid.x * cgrid.y < (long long)SPLIT_WAVES * sm_count() * Cfg<BS, D, R>::RESIDENT) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid.x * SPLIT_WAYS, grid.y);
+    cfg.gridDim = dim3(cgrid.x * SPLIT_WAYS, cgrid.y);
     cfg.blockDim = dim3(Cfg<BS, D, R>::CTA);
     cfg.dynamicSmemBytes = smem_col<BS, D, R>();
     cfg.stream = st;
@@ -816,7 +907,7 @@ int bwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout l
     cfg.numAttrs = 1;
     SPION_CUDA_TRY(cudaLaunchKernelEx(&cfg, fused_bwd_col_kernel<BS, D, R, true>, (const float*)dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH));
   } else {
-    fused_bwd_col_kernel<BS, D, R, false><<<grid, Cfg<BS, D, R>::CTA, smem_col<BS, D, R>(), st>>>(dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH);
+    fused_bwd_col_kernel<BS, D, R, false><<<cgrid, Cfg<BS, D, R>::CTA, smem_col<BS, D, R>(), st>>>(dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH);
   }
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_SPMM_DKDV);
@@ -832,16 +923,29 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
 
 // With eight rows per thread a block row is one warp (block 32) or four (64).  Up to two warps per scheduler (four per SM) each of
 // them is a chain of latencies, and half the rows per thread shorten it (16 matrices, L = 1024, d 32, blocks of 32 at 15 %:
-// forward 31 -> 22 us, rows 22 -> 20); above, the larger micro-tile is worth more.
+// forward 31 -> 22 us, rows 22 -> 20); above, the larger micro-tile is worth more.  While all block rows fit the chip at once with
+// several groups of threads each (512 threads an SM), the groups of a CTA share the blocks of its row (forward and row kernels),
+// L = 1024, d 32, blocks of 32 at 15 %: 2 matrices, four groups, forward 20.2 -> 11.6 us, rows 18.5 -> 10.9; 16 matrices, two groups, 26.7 ->
+// 23.1 and 24.7 -> 22.3 (four groups, in two waves: no gain).  Blocks of 64: 2 matrices, d 32, L = 2048, 30 %: 82 -> 78, 76 -> 72.
+// Columns are better shared by a cluster (see SPLIT).
 constexpr long long FEW_WARPS = 4 * 2;                // per SM
-#define SPION_FUSED_DISPATCH(FN, ...)                                   \
-  do {                                                                  \
-    const bool few = (long long)p.nb * BH * p.bs * p.bs / 1024 <= FEW_WARPS * sm_count(); \
-    if (p.bs == 32 && d == 32) return few ? FN<32, 32, 4>(__VA_ARGS__) : FN<32, 32, 8>(__VA_ARGS__); \
-    if (p.bs == 32 && d == 64) return few ? FN<32, 64, 4>(__VA_ARGS__) : FN<32, 64, 8>(__VA_ARGS__); \
-    if (p.bs == 64 && d == 32) return few ? FN<64, 32, 4>(__VA_ARGS__) : FN<64, 32, 8>(__VA_ARGS__); \
-    if (p.bs == 64 && d == 64) return few ? FN<64, 64, 4>(__VA_ARGS__) : FN<64, 64, 8>(__VA_ARGS__); \
-    return SPION_ERR_UNSUPPORTED;                                       \
+#define SPION_FUSED_DISPATCH(FN, ...)                                                                \
+  do {                                                                                               \
+    const long long units = (long long)p.nb * BH;                                                    \
+    const bool few = units * p.bs * p.bs / 1024 <= FEW_WARPS * sm_count();                           \
+    const int ways = p.bs == 32 ? (units <= 2 * sm_count() ? 4 : units <= 4 * sm_count() ? 2 : 1)    \
+                                : (units <= 2 * sm_count() ? 2 : 1);                                 \
+    if (p.bs == 32 && d == 32)                                                                       \
+      return ways == 4 ? FN<32, 32, 4, 4>(__VA_ARGS__) : ways == 2 ? FN<32, 32, 4, 2>(__VA_ARGS__)   \
+             : few ? FN<32, 32, 4, 1>(__VA_ARGS__) : FN<32, 32, 8, 1>(__VA_ARGS__);                  \
+    if (p.bs == 32 && d == 64)                                                                       \
+      return ways == 4 ? FN<32, 64, 4, 4>(__VA_ARGS__) : ways == 2 ? FN<32, 64, 4, 2>(__VA_ARGS__)   \
+             : few ? FN<32, 64, 4, 1>(__VA_ARGS__) : FN<32, 64, 8, 1>(__VA_ARGS__);                  \
+    if (p.bs == 64 && d == 32)                                                                       \
+      return ways == 2 ? FN<64, 32, 4, 2>(__VA_ARGS__) : few ? FN<64, 32, 4, 1>(__VA_ARGS__) : FN<64, 32, 8, 1>(__VA_ARGS__); \
+    if (p.bs == 64 && d == 64)                                                                       \
+      return ways == 2 ? FN<64, 64, 4, 2>(__VA_ARGS__) : few ? FN<64, 64, 4, 1>(__VA_ARGS__) : FN<64, 64, 8, 1>(__VA_ARGS__); \
+    return SPION_ERR_UNSUPPORTED;                                                                    \
   } while (0)
 
 // full: every block is selected (simt_full.cu)

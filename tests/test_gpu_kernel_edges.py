@@ -99,6 +99,33 @@ def test_fp32_fused_kernels(bs, d, B, H, nb):
     compare(run(mod, Q, K, V, dO, mat, kp), Q, K, V, dO, mat, bs, kp, FP32_TOL, False)
 
 
+# (bs, d, B, H, blocks per side): block rows around what fits the chip at once with four, two and one group of threads per row
+# (148 SMs: up to 296, up to 592, more), rows of one block, rows shorter than the groups
+@pytest.mark.parametrize("bs,d,B,H,nb", [(32, 32, 1, 1, 9), (32, 64, 37, 1, 8), (32, 32, 33, 1, 9), (32, 64, 74, 1, 8), (32, 32, 66, 1, 9),
+                                         (64, 32, 37, 1, 8), (64, 64, 33, 1, 9), (32, 32, 200, 2, 1)])
+@pytest.mark.parametrize("layout", ["tiles", "csr"])
+def test_fp32_rows_shared_by_groups(bs, d, B, H, nb, layout):
+    from spion_b200.attention import Attention
+    from spion_b200.attention_blockcuda import CUDABlockAttention
+    from spion_b200.native import BlockSparseAttention
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(23 + nb, B, H, L, d)
+    mat = lines_of_every_length(nb, nb > 4)
+    if layout == "tiles":
+        mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.float32)
+        got = run(mod, Q, K, V, dO, mat, None)
+        compare(got, Q, K, V, dO, mat, bs, None, FP32_TOL, False)
+        return
+    cpp = Attention._blockcuda_compile_module()                  # element CSR, backward without O (two passes over a row)
+    handle = cpp.init(d, L, B * H, bs)
+    mod = CUDABlockAttention(cfg(B, H, L, d, bs), cpp, handle)
+    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+    out, _ = mod(q, k, v, torch.ones(B, L).cuda(), torch.as_tensor(mat.astype(np.float32)).cuda())
+    out.backward(dO.cuda())
+    compare((out, q.grad, k.grad, v.grad), Q, K, V, dO, mat, bs, None, FP32_TOL, False)
+    cpp.destroy(handle)
+
+
 @pytest.mark.parametrize("L,d", [(64, 64), (192, 32), (512, 32), (576, 32), (1024, 64), (1088, 32), (1856, 32)])
 @pytest.mark.parametrize("padded", [False, True])
 def test_dense_fp32_kernels(L, d, padded):
