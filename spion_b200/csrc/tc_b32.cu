@@ -438,7 +438,8 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
       pb0 = *reinterpret_cast<const uint4*>(in1 + off); pb1 = *reinterpret_cast<const uint4*>(in1 + off + 8);
       if (tid < 32) plse = lse_in[vec + tid];
     };
-    // COL: lse and -delta scale of this thread's row in the next job; block id of its row in the job after
+    // COL: lse and delta of this thread's row in the next job, as they were loaded: whatever is computed from them where they are
+    // requested, or copied before the wait for S, is a wait for global memory in every job; block id of its row in the job after
     float nx0 = 0.f, nx1 = 0.f;
     int pblk = 0;
     bool pre_job = false;
@@ -608,15 +609,13 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
           const int st = c.jg & 1, t0 = jl * GN, nt = min(GN, n - t0);
           // ROW: this thread is a key of gathered block `warp` (its padding penalty); COL: a query row (its lse and
           // delta, requested while the previous job was computed)
-          float mine0 = 0.f, mine1 = 0.f;
+          float pad = 0.f;
           if (C::ROW) {
-            if (kp && warp < nt) mine0 = kp[(t0 == 0 ? c.first_id(warp) : idx[rp + t0 + warp]) * B32 + lane] * LOG2E;
-          } else if (pre_job) {
-            mine0 = nx0; mine1 = nx1;
-          } else if (warp < nt) {
-            const int blk = t0 == 0 ? c.first_id(warp) : idx[rp + t0 + warp];
-            mine0 = lse_in[(size_t)bh * L + blk * B32 + lane];
-            mine1 = -delta_in[(size_t)bh * L + blk * B32 + lane] * scale;
+            if (kp && warp < nt) pad = kp[(t0 == 0 ? c.first_id(warp) : idx[rp + t0 + warp]) * B32 + lane];
+          } else if (!pre_job) {
+            const int blk = warp < nt ? (t0 == 0 ? c.first_id(warp) : idx[rp + t0 + warp]) : 0;
+            nx0 = lse_in[(size_t)bh * L + blk * B32 + lane];
+            nx1 = delta_in[(size_t)bh * L + blk * B32 + lane];
           }
           const bool more = jl + 1 < nch;
           const int ntn = more ? min(GN, n - t0 - GN) : 0;
@@ -632,6 +631,7 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
             tmem_ld32(t_lane + C::S_COL + st * 32, v);
             tmem_ld32(t_lane + C::DP_COL + st * 32, g);
             tmem_ld_wait();
+            const float mine0 = C::ROW ? pad * LOG2E : nx0, mine1 = C::ROW ? 0.f : -nx1 * scale;
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
               // ROW: column i is a query (lse, delta from shared memory); COL: column i is a key (penalty from shared memory)
@@ -645,11 +645,13 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
             else store_row64(sVA(sv), grow, wd);
             fence_proxy_async();
           }
+          job_done(st, sv);
           if (C::COL) {
             // lse and delta of the row this thread owns in the NEXT job: a later chunk of this column, or the
             // first chunk of the next unit (its ids come with the prefetched record)
+            // (a warp without a block in that job loads what it does not use: a branch would join two values by copying them)
             pre_job = false;
-            int blkn = -1, bhn = bh;
+            int blkn = 0, bhn = bh;
             if (more) {
               pre_job = true;
               if (warp < ntn) blkn = pblk;
@@ -658,13 +660,10 @@ k_b32(const __grid_constant__ CUtensorMap tmG0, const __grid_constant__ CUtensor
               bhn = c.next_bh();
               if (warp < min(GN, Cursor<MODE>::rec_n(c.nrec))) blkn = Cursor<MODE>::rec_id(c.nrec, warp);
             }
-            if (blkn >= 0) {
-              nx0 = lse_in[(size_t)bhn * L + blkn * B32 + lane];
-              nx1 = -delta_in[(size_t)bhn * L + blkn * B32 + lane] * scale;
-            }
+            nx0 = lse_in[(size_t)bhn * L + blkn * B32 + lane];
+            nx1 = delta_in[(size_t)bhn * L + blkn * B32 + lane];
           }
           SPION_STAMP_T(0, c.jg, 10);
-          job_done(st, sv);
           c.advance();
         }
         if (!ok) break;
