@@ -86,6 +86,24 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool i
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// bf16 tokens through tensor maps (the GEMM's A), up to three matrices.  Row-major: boxes of 64 features, in the swizzle of the images.
+// Split into heads: boxes of 64 tokens of one head; heads of 32 make a chunk of two images with 64-byte rows (32 features each).  A box
+// whose rows are narrower than the swizzle is spread to its width, so that two heads cannot share 128-byte rows.
+// Copied piece by piece, 16 bytes per thread, the loaders' address arithmetic was the limit: 1080 cycles per chunk of 16 KB, no time
+// waited for memory.  524288 tokens, heads of 32, before and now: gradient of the input from three gradients of 64 features 103 -> 63 us,
+// output projection 39 -> 27, its gradient (row-major) 39 -> 25.  Other widths, sequences that are no multiple of 64 and calls of one tile
+// per CTA keep the copies; so do the weight gradients, where boxes of 64-byte rows were slower (two of them 136 us, 143 through maps).
+enum : int { MAP_NONE = 0, MAP_ROWS = 1, MAP_HEADS = 2 };
+struct LinMaps { CUtensorMap m[3]; };
+__device__ __forceinline__ int which_matrix(const TokMat& t, int c) { return (c >= t.per) + (c >= 2 * t.per); }
+// One thread: features c .. c + 63 of 64 tokens from t on of a head-split operand; the images of a chunk of heads of 32 are `image` bytes apart
+__device__ __forceinline__ void load_heads(const TokMat& t, const CUtensorMap* m, uint32_t dst, uint32_t image, uint32_t bar, int c, int tok) {
+  const int i = which_matrix(t, c), b = tok / t.L, heads = t.per >> t.dsh;
+  c -= i * t.per;
+  for (int f = 0; f < 64; f += t.d, dst += image)
+    tma_load_2d(dst, m + i, bar, 0, (b * heads + ((c + f) >> t.dsh)) * t.L + (tok - b * t.L));
+}
+
 // Eight features of one token in registers: 8 fp32 words, or 4 words of bf16 pairs.
 template <bool BF16> struct Raw { uint32_t w[BF16 ? 4 : 8]; };
 // ... into the shared-memory images: SPLIT == 1 one bf16 image, SPLIT == 3 three (leading, middle, last 8 bits), `part` bytes apart
@@ -139,6 +157,7 @@ struct GemmArgs {
   __nv_bfloat16* g;         // EPI_GELU: activation [T, N] (Y receives the pre-activation)
   // What a backward reads in place of the caller's tensors.  262144 tokens of 64 fp32 features: 33 MB written here, 33 MB less read by
   // the weight gradient; the layer of 128 x 2 matrices, L = 4096 went from 1432 to 1458 us.
+  int tma;                  // bf16 A through maps.m[0 .. 2] (MAP_*)
   __nv_bfloat16* x_copy;    // or null: A as the products use it, [T, K] (fp32 tokens in bf16 mode)
   float* w_copy;            // or null: the stacked W
 };
@@ -183,7 +202,7 @@ __device__ __forceinline__ float dgelu(float x) {
 // (M = 128, two accumulator buffers in tensor memory), warps 9-16 write finished tiles.  W sits in shared memory for the
 // whole run.  Bound by the HBM passes over A and Y.
 template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
-__global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constant__ GemmArgs a) {
+__global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constant__ GemmArgs a, const __grid_constant__ LinMaps maps) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t sbase = smem_u32(smem_raw);
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
@@ -204,13 +223,33 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
   const int ntiles = (a.T + 127) >> 7;
   const int G_x = (int)gridDim.x;
   __shared__ int s_abort;
+  const bool tma = A_BF16 && a.tma;
+  const int my_chunks = ((ntiles - (int)blockIdx.x + G_x - 1) / G_x) * nchunks;
+  auto tma_chunk = [&](int n) {                          // one thread
+    const int c = (n % nchunks) * 64, st = n % a.nstages, t = ((int)blockIdx.x + n / nchunks * G_x) * 128;
+    const uint32_t dst = sA + st * CHUNK;
+    if (a.tma == MAP_ROWS) {
+      const int i = which_matrix(a.A, c);
+      mbar_expect_tx(full + 8 * st, CHUNK);
+      tma_load_2d(dst, &maps.m[i], full + 8 * st, c - i * a.A.per, t);
+    } else {                                             // 64 tokens each; rows past the end keep what is there, their results are dropped
+      const uint32_t image = CHUNK / 2, rows = a.A.d == 32 ? 64 * 64 : 64 * 128;
+      mbar_expect_tx(full + 8 * st, t + 64 < a.T ? CHUNK : CHUNK / 2);
+      load_heads(a.A, maps.m, dst, image, full + 8 * st, c, t);
+      if (t + 64 < a.T) load_heads(a.A, maps.m, dst + rows, image, full + 8 * st, c, t + 64);
+    }
+  };
 
   if (warp == LG_LOADERS) {
     if (lane == 0) {
       s_abort = *reinterpret_cast<volatile int*>(&g_lin_status);
-      for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, LG_LOADERS); mbar_init(empty + 8 * i, 1); }
+      for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, tma ? 1 : LG_LOADERS); mbar_init(empty + 8 * i, 1); }
       for (int i = 0; i < 2; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 8); }
       fence_barrier_init();
+      if (tma && s_abort == 0) {                         // the first chunks are on their way before the weights are converted
+        fence_proxy_async();
+        for (int n = 0; n < a.nstages && n < my_chunks; ++n) tma_chunk(n);
+      }
     }
     __syncwarp();
     tmem_alloc(slot, 512u);
@@ -262,7 +301,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     }
   };
   if constexpr (A_BF16) {
-    if (warp < LG_LOADERS)
+    if (warp < LG_LOADERS && !tma)
       while (ld_n < LG_DEPTH && ld_tile < ntiles) copy_chunk();
   }
 
@@ -313,7 +352,13 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     int n = 0;
     bool ok = true;
     int tile = blockIdx.x, ch = 0;
-    if constexpr (A_BF16) {
+    if (tma) {
+      for (n = a.nstages; warp == 0 && n < my_chunks; ++n) {
+        if (!warp_wait(empty + 8 * (n % a.nstages), (uint32_t)(n / a.nstages - 1) & 1u)) break;
+        if (elect_one()) tma_chunk(n);
+        __syncwarp();
+      }
+    } else if constexpr (A_BF16) {
       // LG_DEPTH chunks of copies in flight per thread; a chunk is handed over when the thread's own copies have landed
       auto hand_over = [&](int m) {
         fence_proxy_async();
@@ -369,7 +414,8 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     int n = 0, j = 0;
     bool ok = true;
     // every operand descriptor is an add on one of these two
-    const uint64_t DA = make_smem_desc(sA, 16, 1024, LAYOUT_SW128);
+    const bool half_rows = A_BF16 && a.tma == MAP_HEADS && a.A.d == 32;       // two images of 32 features, 64-byte rows
+    const uint64_t DA = half_rows ? make_smem_desc(sA, 16, 512, LAYOUT_SW64) : make_smem_desc(sA, 16, 1024, LAYOUT_SW128);
     const uint64_t DB = TRANSB ? make_smem_desc(sbase, 8192, 1024, LAYOUT_SW128) : make_smem_desc(sbase, 16, 1024, LAYOUT_SW128);
     const uint32_t idesc = make_idesc_bf16(128, nc, 0, 0);
     for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++j) {
@@ -401,7 +447,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)
                 if (kk < nk)
-                  mma_bf16((lead ? dl : d0) + (TRANSB ? g * 64u : 0u), desc_advance(pa, kk * 32), desc_advance(pb, TRANSB ? kk * 2048 : kk * 32),
+                  mma_bf16((lead ? dl : d0) + (TRANSB ? g * 64u : 0u), desc_advance(pa, half_rows ? (kk >> 1) * (CHUNK / 2) + (kk & 1) * 32 : kk * 32), desc_advance(pb, TRANSB ? kk * 2048 : kk * 32),
                            id, kk > 0 ? 1u : (lead ? acc_l : (pr > 0 ? 1u : acc_s)));
             }
           }
@@ -877,6 +923,36 @@ bool mat_ok(const spion_tokens* t) {
   return true;
 }
 
+// The form in which bf16 tokens are read through tensor maps (MAP_NONE: the kernels copy by themselves).  With one tile per CTA
+// the copies are no limit, and making the maps costs the host a microsecond (inference of 1024 tokens: 45.6 us, 46.8 with maps).
+int map_form(const spion_tokens* t, long long T) {
+  if (!t->is_bf16 || (T + 127) / 128 <= sm_count()) return MAP_NONE;
+  if (t->heads <= 0) return t->cols >= 64 && (t->count == 1 || t->cols % 64 == 0) ? MAP_ROWS : MAP_NONE;
+  return (t->head_dim == 32 || t->head_dim == 64) && t->cols % 64 == 0 && t->seq_len % 64 == 0 && T % t->seq_len == 0 &&
+         T * t->heads <= 0x7fffffffLL ? MAP_HEADS : MAP_NONE;
+}
+int token_maps(const spion_tokens* t, long long T, CUtensorMap* m) {
+  static std::atomic<void*> encode{nullptr};
+  void* fn = encode.load(std::memory_order_acquire);
+  if (!fn) {
+    cudaDriverEntryPointQueryResult q;
+    SPION_CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
+    if (q != cudaDriverEntryPointSuccess || !fn) return SPION_ERR_CUDA;
+    encode.store(fn, std::memory_order_release);
+  }
+  int dev = 0;                                           // a thread whose first call this is has no current context, and encoding wants one
+  SPION_CUDA_TRY(cudaGetDevice(&dev));
+  SPION_CUDA_TRY(cudaSetDevice(dev));
+  TcState s;
+  s.encode = (EncodeTiledFn)fn;
+  for (int i = 0; i < t->count; ++i) {
+    const int rc = t->heads > 0 ? make_map(&s, m + i, t->ptr[i], (uint64_t)T * t->heads, (uint32_t)t->head_dim, (uint32_t)t->head_dim, 64)
+                                : make_map(&s, m + i, t->ptr[i], (uint64_t)T, (uint32_t)t->cols, 64, 128);
+    if (rc) return rc;
+  }
+  return SPION_OK;
+}
+
 // columns per CTA, accumulators and ring stages of the GEMM; false when the weights do not fit
 bool plan_gemm(int split, bool trans, int K, int N, int* nc, int* nacc, int* stages, size_t* smem, int widest = 256) {
   const int least = split == 1 ? LG_DEPTH + 1 : 2;           // bf16 operands keep LG_DEPTH chunks in flight
@@ -919,16 +995,19 @@ int prepare_wgrad() {
 }
 
 template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
-int launch_gemm(const GemmArgs& a, size_t smem, cudaStream_t st) {
+int launch_gemm(GemmArgs& a, const spion_tokens* tok, size_t smem, cudaStream_t st) {
   auto k = k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>;
-  const int rc = prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
+  int rc = prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
   if (rc) return rc;
+  LinMaps maps;
+  a.tma = A_BF16 ? map_form(tok, a.T) : MAP_NONE;
+  if (a.tma && (rc = token_maps(tok, a.T, maps.m))) return rc;
   const int ny = (a.N + a.nc - 1) / a.nc;
   const int sms = sm_count(), tiles = (a.T + 127) / 128;
   if (sms < 1) return SPION_ERR_CUDA;
   int gx = sms / ny > 0 ? sms / ny : 1;
   if (gx > tiles) gx = tiles;
-  k<<<dim3(gx, ny), LG_THREADS, smem, st>>>(a);
+  k<<<dim3(gx, ny), LG_THREADS, smem, st>>>(a, maps);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
@@ -1079,12 +1158,12 @@ extern "C" int spion_linear_forward_keep(const spion_tokens* X, const float* con
   a.k0 = 0; a.accum = 0; a.parts = 0;
   if (!plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)cuda_stream;
-  if (fp32) return launch_gemm<3, false, false, EPI_NONE, false>(a, smem, st);
+  if (fp32) return launch_gemm<3, false, false, EPI_NONE, false>(a, X, smem, st);
   if (gelu_out)
-    return X->is_bf16 ? launch_gemm<1, true, false, EPI_GELU, true>(a, smem, st) : launch_gemm<1, false, false, EPI_GELU, true>(a, smem, st);
+    return X->is_bf16 ? launch_gemm<1, true, false, EPI_GELU, true>(a, X, smem, st) : launch_gemm<1, false, false, EPI_GELU, true>(a, X, smem, st);
   if (Y->is_bf16)
-    return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, true>(a, smem, st) : launch_gemm<1, false, false, EPI_NONE, true>(a, smem, st);
-  return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, false>(a, smem, st) : launch_gemm<1, false, false, EPI_NONE, false>(a, smem, st);
+    return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, true>(a, X, smem, st) : launch_gemm<1, false, false, EPI_NONE, true>(a, X, smem, st);
+  return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, false>(a, X, smem, st) : launch_gemm<1, false, false, EPI_NONE, false>(a, X, smem, st);
 }
 
 extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* const* W, int nw, int fp32, const void* gelu_in,
@@ -1112,17 +1191,17 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
       a.K = total - a.k0 < step ? total - a.k0 : step;
       a.accum = a.k0 > 0;
       if (!plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
-      const int rc = launch_gemm<3, false, true, EPI_NONE, false>(a, smem, st);
+      const int rc = launch_gemm<3, false, true, EPI_NONE, false>(a, dY, smem, st);
       if (rc) return rc;
     }
     return SPION_OK;
   }
   if (!plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256)) return SPION_ERR_UNSUPPORTED;
   if (gelu_in)
-    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_DGELU, true>(a, smem, st) : launch_gemm<1, false, true, EPI_DGELU, true>(a, smem, st);
+    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_DGELU, true>(a, dY, smem, st) : launch_gemm<1, false, true, EPI_DGELU, true>(a, dY, smem, st);
   if (dX->is_bf16)
-    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, true>(a, smem, st) : launch_gemm<1, false, true, EPI_NONE, true>(a, smem, st);
-  return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, false>(a, smem, st) : launch_gemm<1, false, true, EPI_NONE, false>(a, smem, st);
+    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, true>(a, dY, smem, st) : launch_gemm<1, false, true, EPI_NONE, true>(a, dY, smem, st);
+  return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, false>(a, dY, smem, st) : launch_gemm<1, false, true, EPI_NONE, false>(a, dY, smem, st);
 }
 
 extern "C" long long spion_linear_workspace_floats(long long T, int in_features, int out_features, int fp32) {

@@ -67,6 +67,50 @@ def test_linear_kernels(B, L, H, d, K, nw, mode, split):
     assert _rel(db, dY.sum(0)) < 2e-6
 
 
+# bf16 tokens, more than 148 tiles of 128 (read through tensor maps) and fewer: sequences of 64-token boxes that end at and in the
+# middle of a tile, row-major tails of 56 and 1 tokens, heads of 32 and 64, one to three matrices; widths and lengths that are copied
+@pytest.mark.parametrize("B,L,H,d,N,nw", [(149, 128, 2, 32, 64, 1), (101, 192, 2, 32, 64, 3), (300, 64, 4, 32, 96, 1), (61, 320, 1, 64, 64, 3),
+                                          (101, 192, 2, 64, 192, 1), (1, 19000, 2, 32, 64, 3), (1, 19073, 1, 64, 128, 1),
+                                          (40, 1984, 2, 32, 64, 3), (101, 192, 3, 32, 64, 1), (120, 160, 2, 32, 64, 3),
+                                          (3, 192, 2, 32, 64, 3), (1, 129, 2, 32, 64, 1)])
+@pytest.mark.parametrize("split", [False, True])
+def test_linear_kernels_on_bf16_tokens(B, L, H, d, N, nw, split):
+    T, K = B * L, H * d
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    P, ref = ctypes.c_void_p, ctypes.byref
+    st = P(torch.cuda.current_stream().cuda_stream)
+    shape, lay = ((B, H, L, d), (H, d, L)) if split else ((T, K), (0, 0, 0))
+    flat = lambda t: (t.permute(0, 2, 1, 3).reshape(T, K) if split else t).double()
+    A = [rnd(*shape).to(torch.bfloat16) for _ in range(nw)]          # forward (nw == 1) and input gradient of nw stacked layers
+    ptrs = lambda ts: (P * 3)(*([t.data_ptr() for t in ts] + [None] * (3 - len(ts))))
+    ta = _tokens(A, *lay)
+    if nw == 1:                                                      # the output projection: tokens in, rows out
+        W, b, Y, dY = rnd(N, K), rnd(N), torch.full((T, N), 7.0, device="cuda", dtype=torch.bfloat16), rnd(T, N).to(torch.bfloat16)
+        ty, tdy = _tokens([Y]), _tokens([dY])
+        check(lib.spion_linear_forward(ref(ta), ptrs([W]), ptrs([b]), 1, 0, ref(ty), None, T, K, N, st))
+        dW, db = torch.full((N, K), 7.0, device="cuda"), torch.full((N,), 7.0, device="cuda")
+        ws = torch.empty(lib.spion_linear_workspace_floats(T, K, N, 0), device="cuda")
+        check(lib.spion_linear_backward_weight(ref(tdy), ref(ta), 0, P(dW.data_ptr()), P(db.data_ptr()), P(ws.data_ptr()), T, K, N, st))
+        torch.cuda.synchronize()
+        assert _rel(Y, flat(A[0]) @ W.double().t() + b.double()) < 5e-3
+        assert _rel(dW, dY.double().t() @ flat(A[0])) < 2e-6          # exact products of bf16 values, fp32 sums
+    else:                                                            # gradients of three stacked layers: rows of N features in
+        Ws = [rnd(K, N) for _ in range(nw)]
+        X, dX = rnd(T, N).to(torch.bfloat16), torch.full((T, N), 7.0, device="cuda")
+        tx, tdx = _tokens([X]), _tokens([dX])
+        check(lib.spion_linear_backward_input(ref(ta), ptrs(Ws), nw, 0, None, ref(tdx), T, N, nw * K, st))
+        dW, db = torch.full((nw * K, N), 7.0, device="cuda"), torch.full((nw * K,), 7.0, device="cuda")
+        ws = torch.empty(lib.spion_linear_workspace_floats(T, N, nw * K, 0), device="cuda")
+        check(lib.spion_linear_backward_weight(ref(ta), ref(tx), 0, P(dW.data_ptr()), P(db.data_ptr()), P(ws.data_ptr()), T, N, nw * K, st))
+        torch.cuda.synchronize()
+        dY = torch.cat([flat(t) for t in A], 1)
+        assert _rel(dX, dY @ torch.cat(Ws).double()) < 5e-3
+        assert _rel(dW, dY.t() @ X.double()) < 2e-6
+    assert lib.spion_linear_status(1) == 0
+    assert _rel(db, (dY.double() if nw == 1 else dY).sum(0)) < 2e-6
+
+
 @pytest.mark.parametrize("native,dtype,bs,L,dense", [(True, "bf16", 64, 192, False), (True, "bf16", 64, 128, True),
                                                      (True, "fp32", 32, 160, False), (False, "fp32", 32, 96, False)])
 def test_attention_layer_in_one_node_equals_its_stages(native, dtype, bs, L, dense):
