@@ -587,7 +587,9 @@ struct WgradAcc {
   __device__ uint32_t at(int i) const { return two ? (uint32_t)(i >> 1) * cs + ((uint32_t)(i & 1) << 20) : (uint32_t)i * cs; }
 };
 
-constexpr int WG_THREADS = 32 * (LG_LOADERS + 1);
+// Loader warps.  bf16: what a copy costs is its addresses, and sixteen warps share them better than eight (524288 tokens, two
+// gradients: 135 -> 109 us).  fp32: the split, which more warps do not speed up (262144 tokens: 153 us, 157 with sixteen).
+template <int SPLIT> constexpr int WG_LOADERS = SPLIT == 1 ? 16 : 8;
 constexpr uint32_t WCHUNK = 64 * 128;                    // [64 tokens x 64 features] bf16
 
 // As redo_outputs: features n .. n + 31 of dY by feature k of X, over the tokens of this CTA
@@ -611,7 +613,8 @@ __device__ __noinline__ void redo_gradient(const WgradArgs& a, int n, int k, flo
 // One CTA per SM and slice of the tokens.  dW^T accumulates in tensor memory over all tokens of the CTA: the chunks of X are one
 // MN-major A operand (M = 64 or 128), those of dY one MN-major B operand (N up to 192), so nothing is transposed.  The bias gradient is summed from the registers the loaders hold.
 template <int SPLIT, bool DY_BF16, bool X_BF16>
-__global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_constant__ WgradArgs a) {
+__global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(const __grid_constant__ WgradArgs a) {
+  constexpr int LOADERS = WG_LOADERS<SPLIT>, ROWS = 4 * LOADERS, XR = 64 / ROWS;       // rows of a pass of all loaders, passes per tile
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t sbase = smem_u32(smem_raw);
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
@@ -622,15 +625,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
   const uint32_t bars = sbase + a.nstages * ((a.nc + 63) / 64 + (a.kc + 63) / 64) * SPLIT * WCHUNK;
   const uint32_t full = bars, empty = bars + 64, acc_done = bars + 128, slot = bars + 136, sdb = bars + 256;
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
-  float* sdb_ptr = reinterpret_cast<float*>(smem_raw + (sdb - sbase));        // [8 warps][256]
+  float* sdb_ptr = reinterpret_cast<float*>(smem_raw + (sdb - sbase));        // [LOADERS][256]
   const int ntiles = (a.T + 63) >> 6;
   const int G_x = (int)gridDim.x;
   __shared__ int s_abort;
 
-  if (warp == LG_LOADERS) {
+  if (warp == LOADERS) {
     if (lane == 0) {
       s_abort = *reinterpret_cast<volatile int*>(&g_lin_status);
-      for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, LG_LOADERS); mbar_init(empty + 8 * i, 1); }
+      for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, LOADERS); mbar_init(empty + 8 * i, 1); }
       mbar_init(acc_done, 1);
       fence_barrier_init();
     }
@@ -644,15 +647,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
   const uint32_t tmem = *slot_ptr;
   if (s_abort != 0) {
     __syncthreads();
-    if (warp == LG_LOADERS) tmem_dealloc(tmem, 512u);
+    if (warp == LOADERS) tmem_dealloc(tmem, 512u);
     return;
   }
 
-  if (warp < LG_LOADERS) {
+  if (warp < LOADERS) {
     const int lrow = tid >> 3, lc8 = tid & 7;
     // chunk i of a tile: features i of dY for i < nch, then those of X.  fp32 chunks pass through registers (a tile ahead),
     // bf16 ones are copied straight into their stage (AHEAD tiles ahead).
-    Raw<false> cur[4][2];
+    Raw<false> cur[4][XR];
     constexpr int AHEAD = (DY_BF16 || X_BF16) ? 2 : 0;
     float db[4][8];
 #pragma unroll
@@ -671,24 +674,24 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
     }
     const int step = G_x * 64;
     const int dstep_b = step / a.dY.L, dstep_l = step - dstep_b * a.dY.L, xstep_b = step / a.X.L, xstep_l = step - xstep_b * a.X.L;
-    RowIt drow[2], xrow[2];                                // rows of the tile whose loads are issued next
+    RowIt drow[XR], xrow[XR];                                // rows of the tile whose loads are issued next
     auto row_init = [&](int t0) {
 #pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        drow[x].init(a.dY, min(a.T - 1, t0 + lrow + 32 * x));
-        xrow[x].init(a.X, min(a.T - 1, t0 + lrow + 32 * x));
+      for (int x = 0; x < XR; ++x) {
+        drow[x].init(a.dY, min(a.T - 1, t0 + lrow + ROWS * x));
+        xrow[x].init(a.X, min(a.T - 1, t0 + lrow + ROWS * x));
       }
     };
     // fp32 chunks of the tile the row iterators stand at -> registers
     auto load_row = [&](int tile, int i, int x) {
       const bool isd = !DY_BF16 && (X_BF16 || i < nch);
       const void* p = isd ? (const void*)(dcol[i] + drow[x].off(a.dY)) : (const void*)(xcol[i] + xrow[x].off(a.X));
-      const bool in = (isd ? dcol[i] != nullptr : xcol[i] != nullptr) && tile * 64 + lrow + 32 * x < a.T;
+      const bool in = (isd ? dcol[i] != nullptr : xcol[i] != nullptr) && tile * 64 + lrow + ROWS * x < a.T;
       ld_v8_if(in, p, cur[i][x].w);
     };
     // bf16 chunks of the current tile -> shared memory
     auto copy_row = [&](int tile, int i, int x, uint32_t dst) {
-      const bool tin = tile * 64 + lrow + 32 * x < a.T;
+      const bool tin = tile * 64 + lrow + ROWS * x < a.T;
       if (i < nch) {
         const bool in = tin && dcol[i];
         cp_async16(dst, in ? dcol[i] + drow[x].off(a.dY) : reinterpret_cast<const DE*>(a.dY.p[0]), in);
@@ -698,7 +701,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
       }
     };
     auto place = [&](int st, int i, int x) -> uint32_t {
-      const int r = lrow + 32 * x;
+      const int r = lrow + ROWS * x;
       return sbase + st * stage + i * SPLIT * WCHUNK + r * 128 + ((lc8 ^ (r & 7)) << 4);
     };
     bool ok = true;
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
         for (int i = 0; i < 4; ++i) {
           if (i < nch) {
 #pragma unroll
-            for (int x = 0; x < 2; ++x) {
+            for (int x = 0; x < XR; ++x) {
               uint32_t w[4];
               asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(place(st, i, x)) : "memory");
 #pragma unroll
@@ -728,7 +731,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int x = 0; x < 2; ++x) load_row(blockIdx.x, i, x);
+      for (int x = 0; x < XR; ++x) load_row(blockIdx.x, i, x);
     for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++n) {
       const int st = n % a.nstages, use = n / a.nstages;
       if (use > 0) ok = warp_wait(empty + 8 * st, (uint32_t)(use - 1) & 1u);
@@ -737,16 +740,16 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int x = 0; x < 2; ++x)
+          for (int x = 0; x < XR; ++x)
             if (i < cpt && (i < nch ? DY_BF16 : X_BF16)) copy_row(tile, i, x, place(st, i, x));
       }
 #pragma unroll
-      for (int x = 0; x < 2; ++x) { drow[x].add(a.dY, dstep_b, dstep_l); xrow[x].add(a.X, xstep_b, xstep_l); }
+      for (int x = 0; x < XR; ++x) { drow[x].add(a.dY, dstep_b, dstep_l); xrow[x].add(a.X, xstep_b, xstep_l); }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (i < cpt && !(i < nch ? DY_BF16 : X_BF16)) {
 #pragma unroll
-          for (int x = 0; x < 2; ++x) {
+          for (int x = 0; x < XR; ++x) {
             raw_store<SPLIT, false>(cur[i][x], place(st, i, x), WCHUNK);
             if (i < nch) {
 #pragma unroll
@@ -768,7 +771,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
       if (ok)
         for (int m = max(0, n - AHEAD); m < n; ++m) hand_over(m);
     }
-    // column sums of dY: lanes with the same lc8 of a warp, then the eight warps in order
+    // column sums of dY: lanes with the same lc8 of a warp, then the warps in order
     if (blockIdx.z == 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -783,12 +786,12 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
         }
       }
     }
-    asm volatile("bar.sync 1, 256;" ::: "memory");        // the eight loader warps
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * LOADERS) : "memory");       // the loader warps
     float* part = a.part + (size_t)blockIdx.x * ((size_t)a.N * a.K + a.N);
     if (blockIdx.z == 0 && tid < nlen) {
       float s = 0.f;
 #pragma unroll
-      for (int w = 0; w < LG_LOADERS; ++w) s += sdb_ptr[w * 256 + tid];
+      for (int w = 0; w < LOADERS; ++w) s += sdb_ptr[w * 256 + tid];
       part[(size_t)a.N * a.K + n0 + tid] = s;
     }
     if (ok) ok = warp_wait(acc_done, 0u);
@@ -800,7 +803,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
       const int small = acc.total() - 1, used = min(small, (ntiles - (int)blockIdx.x + G_x - 1) / G_x);    // leading ones that were used
       const int m = kch == 1 ? q * 16 + (lane & 15) : q * 32 + lane;           // feature of X
       const bool min_ = (kch == 2 || lane < 16) && m < klen;
-      for (int g = half; g < (nlen >> 5); g += 2) {
+      for (int g = half; g < (nlen >> 5); g += LOADERS / 4) {
         uint32_t v[32];
         __syncwarp();
         if (SPLIT == 3) {
@@ -870,7 +873,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_lin_wgrad(const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == LG_LOADERS) tmem_dealloc(tmem, 512u);
+  if (warp == LOADERS) tmem_dealloc(tmem, 512u);
 }
 
 // out[i] = sum over the CTAs' partial results, in a fixed order: 32 groups of four values x 8 slices of the CTAs per block
@@ -1017,7 +1020,7 @@ int launch_wgrad(const WgradArgs& a, int gx, size_t smem, cudaStream_t st) {
   auto k = k_lin_wgrad<SPLIT, DY_BF16, X_BF16>;
   const int rc = prepare_wgrad<SPLIT, DY_BF16, X_BF16>();
   if (rc) return rc;
-  k<<<dim3(gx, (a.N + a.nc - 1) / a.nc, (a.K + a.kc - 1) / a.kc), WG_THREADS, smem, st>>>(a);
+  k<<<dim3(gx, (a.N + a.nc - 1) / a.nc, (a.K + a.kc - 1) / a.kc), 32 * (WG_LOADERS<SPLIT> + 1), smem, st>>>(a);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
@@ -1030,7 +1033,7 @@ bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, size_t* 
   const int cpt = (nw + kw) / 64;
   const size_t stage = (size_t)cpt * split * WCHUNK;
   for (int st = split == 1 ? 6 : 4; st >= (split == 1 ? 3 : 2); --st) {     // bf16 operands: two stages of copies in flight
-    const size_t total = st * stage + 256 + 8 * 256 * 4;
+    const size_t total = st * stage + 256 + (split == 1 ? WG_LOADERS<1> : WG_LOADERS<3>) * 256 * 4;
     if (total <= SMEM_MAX) { *nc = nw; *kc = kw; *stages = st; *smem = total; return true; }
   }
   return false;
