@@ -119,24 +119,23 @@ class BlockSparseAttention(nn.Module):
         return self.nnzb
 
     def _recompute_pays(self) -> bool:
-        """Which backward serves the current mask (forward + backward, 64 matrices unless stated, one B200):
+        """Which backward serves the current mask: from rebuilt tiles (the forward's log-sum-exp, nothing of size nnz in memory unless the
+        caller wants P back) or from stored ones.
 
-        * 32-wide blocks and the full mask: rebuilt tiles (no conversion passes; 2 * BH * L^2 elements less memory);
-        * a caller that wants P back: stored tiles, the forward writes them anyway (L = 4096, 5 %: 227 us; rebuilt 242);
-        * rows of three blocks or more: rebuilt (L = 4096, 5 %: 217 us, stored 227; 30 %: 607, 906; L = 16384, 5 %: 1650, 2610);
-          shorter rows: stored (L = 1024, two blocks per row: 66 us, rebuilt 69);
-        * head_dim 32 with fewer than 2^15 selected blocks in all matrices: stored, although the rebuilt tiles are faster there too
-          (2 to 128 matrices, L = 1024 to 4096, 3.2 to 19 blocks per row: 0.98 to 1.77 times as fast).  P is normalised before and
-          not after it is rounded to bf16, and a training step of the encoder classifier at such sizes multiplies any change of
-          rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to 3.3e-1 of their norm over eight
-          seeds (both paths are equally far from the fp32 step).  The bound is a line between measured sizes that leaves those
-          steps as they were; it is no property of the kernels, and recompute=True takes the faster path below it as well."""
+        Rebuilt tiles are faster (forward + backward on one B200, us, rebuilt and stored; head_dim 64 and 64 matrices unless
+        stated).  No P returned: L = 4096, 3 % (two blocks per row) 150, 173; 5 % 174, 226; 30 % 581, 924; L = 16384, 5 % 1764,
+        2882; 512 matrices, L = 1024, two blocks per row 266, 323; 2 matrices, L = 4096, 5 % 82, 86.  P returned (the forward writes it
+        in both): L = 4096, 3 % 161, 173; 5 % 207, 227; 30 % 844, 935; L = 2048, two blocks per row 95, 96.
+
+        Stored tiles remain for head_dim 32 with fewer than 2^15 selected blocks in all matrices, although the rebuilt ones are faster
+        there too (2 to 128 matrices, L = 1024 to 4096, 3.2 to 19 blocks per row: 0.98 to 1.77 times as fast before the streaming kernels'
+        present form).  P is normalised before and not after it is rounded to bf16, and a training step of the encoder classifier at
+        such sizes multiplies any change of rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to
+        3.3e-1 of their norm over eight seeds (both paths are equally far from the fp32 step).  The bound is a line between measured
+        sizes that leaves those steps as they were; it is no property of the kernels, and recompute=True takes the faster path
+        below it as well."""
         nb = self.L // self.bs
-        if self.bs == 32 or self.nnzb == nb * nb:
-            return True
-        if self.return_probs or self.nnzb < 3 * nb:
-            return False
-        return self.d == 64 or self.BH * self.nnzb >= 1 << 15
+        return self.bs == 32 or self.nnzb == nb * nb or self.d == 64 or self.BH * self.nnzb >= 1 << 15
 
     @property
     def nnz(self) -> int:
