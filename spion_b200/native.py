@@ -72,7 +72,8 @@ class BlockSparseAttention(nn.Module):
         self.return_probs = bool(return_probs) or not self.fused
         # recompute=True (fused kernels): the backward rebuilds P and dS on chip from the log-sum-exp and nothing
         # of size nnz exists in memory; False: the forward stores P, the backward reads it and writes dS
-        # (spion_attn_backward_ex).  None: chosen per mask in set_mask.
+        # (spion_attn_backward_ex).  None: chosen per mask in set_mask; "layer": the same, and small calls at head_dim 32 as
+        # a training step of an encoder wants them (_recompute_pays).
         self._recompute_arg = recompute
         self.recompute = self.fused and (recompute is None or bool(recompute))
         self.last = None
@@ -111,7 +112,7 @@ class BlockSparseAttention(nn.Module):
         m8 = (mat != 0).to(torch.uint8).contiguous().to(self.device)
         self._ctx.set_pattern(m8, self.bs)
         self.nnzb = int(lib.spion_pattern_nnzb(self.handle))
-        if self.fused and self._recompute_arg is None:
+        if self.fused and self._recompute_arg in (None, "layer"):
             self.recompute = self._recompute_pays()
         from .pattern import pattern_from_mask
         self._pattern = pattern_from_mask(m8, self.bs)          # block CSR for the helpers above
@@ -127,15 +128,17 @@ class BlockSparseAttention(nn.Module):
         2882; 512 matrices, L = 1024, two blocks per row 266, 323; 2 matrices, L = 4096, 5 % 82, 86.  P returned (the forward writes it
         in both): L = 4096, 3 % 161, 173; 5 % 207, 227; 30 % 844, 935; L = 2048, two blocks per row 95, 96.
 
-        Stored tiles remain for head_dim 32 with fewer than 2^15 selected blocks in all matrices, although the rebuilt ones are faster
-        there too (2 to 128 matrices, L = 1024 to 4096, 3.2 to 19 blocks per row: 0.98 to 1.77 times as fast before the streaming kernels'
-        present form).  P is normalised before and not after it is rounded to bf16, and a training step of the encoder classifier at
-        such sizes multiplies any change of rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to
-        3.3e-1 of their norm over eight seeds (both paths are equally far from the fp32 step).  The bound is a line between measured
-        sizes that leaves those steps as they were; it is no property of the kernels, and recompute=True takes the faster path
-        below it as well."""
+        head_dim 32: 9 matrices, L = 9472, 12 % 158, 274, with P 207, 274; 28 matrices, L = 6528, 4 % 109, 163; 2 matrices, L = 2048 85, 91.
+
+        Attention layers ("layer") keep stored tiles at head_dim 32 with fewer than 2^15 selected blocks in all matrices.  P is
+        normalised before and not after it is rounded to bf16 there, and a training step of the encoder classifier at such sizes
+        multiplies any change of rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to 3.3e-1 of
+        their norm over eight seeds (both paths are equally far from the fp32 step).  The bound is a line between measured sizes
+        that leaves those steps as they were; it is no property of the kernels."""
+        if self._recompute_arg is None or self.bs == 32 or self.d == 64:
+            return True
         nb = self.L // self.bs
-        return self.bs == 32 or self.nnzb == nb * nb or self.d == 64 or self.BH * self.nnzb >= 1 << 15
+        return self.nnzb == nb * nb or self.BH * self.nnzb >= 1 << 15
 
     @property
     def nnz(self) -> int:
