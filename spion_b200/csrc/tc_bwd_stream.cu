@@ -27,7 +27,7 @@
 // What bounds it: per pair at head_dim 64 the tensor pipe needs 920 (COL) or 660 cycles (ROW), the exponentials 512; a pair takes
 // about 1450.
 // Measured, ROW and COL, before (two groups of eight, a walk in every warp) and now: 64 matrices, L = 16384, d 64, 5 %: 637 and 639 us, now
-// 561 and 605; 256 matrices, L = 4096, d 32, 10 %, padded keys, two full columns: 425 and 394, now 341 and 306.  COL at head_dim 32: five
+// 561 and 591; 256 matrices, L = 4096, d 32, 10 %, padded keys, two full columns: 425 and 394, now 341 and 306.  COL at head_dim 32: five
 // slots and four sets of value tiles 306 us, seven and three 317.  Which mask is served by rebuilt and which by stored tiles:
 // _recompute_pays in native.py.
 //
