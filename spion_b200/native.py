@@ -123,22 +123,28 @@ class BlockSparseAttention(nn.Module):
         """Which backward serves the current mask: from rebuilt tiles (the forward's log-sum-exp, nothing of size nnz in memory unless the
         caller wants P back) or from stored ones.
 
-        Rebuilt tiles are faster (forward + backward on one B200, us, rebuilt and stored; head_dim 64 and 64 matrices unless
-        stated).  No P returned: L = 4096, 3 % (two blocks per row) 150, 173; 5 % 174, 226; 30 % 581, 924; L = 16384, 5 % 1764,
-        2882; 512 matrices, L = 1024, two blocks per row 266, 323; 2 matrices, L = 4096, 5 % 82, 86.  P returned (the forward writes it
-        in both): L = 4096, 3 % 161, 173; 5 % 207, 227; 30 % 844, 935; L = 2048, two blocks per row 95, 96.
+        No P returned: rebuilt tiles, which are faster (forward + backward on one B200, us, rebuilt and stored; head_dim 64 and 64 matrices
+        unless stated): L = 4096, 3 % (two blocks per row) 150, 173; 5 % 174, 226; 30 % 581, 924; L = 16384, 5 % 1764, 2882; 512 matrices,
+        L = 1024, two blocks per row 266, 323; 2 matrices, L = 4096, 5 % 82, 86.  head_dim 32: 9 matrices, L = 9472, 12 % 158, 274; 28
+        matrices, L = 6528, 4 % 109, 163; 2 matrices, L = 2048 85, 91.
 
-        head_dim 32: 9 matrices, L = 9472, 12 % 158, 274, with P 207, 274; 28 matrices, L = 6528, 4 % 109, 163; 2 matrices, L = 2048 85, 91.
+        P returned: stored tiles.  The gradients are those of the very P that the caller holds, and a change of it before the backward is
+        an error.  Rebuilt ones are faster here too (L = 4096, 3 % 161, 173; 5 % 207, 227; 30 % 844, 935; L = 2048, two blocks per row 95, 96;
+        head_dim 32, 9 matrices, L = 9472 207, 274) but take no notice of such a change, and their gradients differ by 4e-3 in norm, since dS
+        comes from P before it is rounded (error against fp64 2.4e-3 instead of 3.1e-3): recompute=True asks for them.
+        32-wide blocks and the full mask are rebuilt in any case.
 
         Attention layers ("layer") keep stored tiles at head_dim 32 with fewer than 2^15 selected blocks in all matrices.  P is
         normalised before and not after it is rounded to bf16 there, and a training step of the encoder classifier at such sizes
         multiplies any change of rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to 3.3e-1 of
         their norm over eight seeds (both paths are equally far from the fp32 step).  The bound is a line between measured sizes
         that leaves those steps as they were; it is no property of the kernels."""
-        if self._recompute_arg is None or self.bs == 32 or self.d == 64:
-            return True
         nb = self.L // self.bs
-        return self.nnzb == nb * nb or self.BH * self.nnzb >= 1 << 15
+        if self.bs == 32 or self.nnzb == nb * nb:
+            return True
+        if self.return_probs:
+            return False
+        return self._recompute_arg is None or self.d == 64 or self.BH * self.nnzb >= 1 << 15
 
     @property
     def nnz(self) -> int:

@@ -117,6 +117,30 @@ def test_a_changed_output_is_noticed(dtype, recompute, what):
         total.backward()
 
 
+@pytest.mark.parametrize("d", [32, 64])
+@pytest.mark.parametrize("padded", [False, True])
+def test_gradients_of_a_call_that_returns_its_probabilities(d, padded):
+    """Blocks of 64: the backward reads the P that the caller got, so the gradients are those of the stored path bit for bit and a
+    change of P in between is an error."""
+    from spion_b200.native import BlockSparseAttention
+    g = torch.Generator(device="cuda").manual_seed(7)
+    q, k, v, do = (torch.randn(B, H, L, d, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+    for t in (q, k, v):
+        t.requires_grad_()
+    keys = make_inputs()[1]
+    got = []
+    for recompute in (None, False):
+        mod = BlockSparseAttention(config(head_dim=d, transformer_dim=H * d), dtype=torch.bfloat16, keypad=padded, recompute=recompute)
+        out, probs = mod(q, k, v, keys, make_mask(4))
+        got.append((out, probs) + torch.autograd.grad(out, (q, k, v), do))
+    same(*got)
+    mod = BlockSparseAttention(config(head_dim=d, transformer_dim=H * d), dtype=torch.bfloat16, keypad=padded)
+    out, probs = mod(q, k, v, keys, make_mask(4))
+    probs.mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.backward(do)
+
+
 def test_changed_probabilities_of_a_drop_in_layer_are_noticed():
     layer, (x, keys) = make_layer("drop-in", task="lra-image"), make_inputs()
     out, probs = layer(x, keys, make_mask(4))
