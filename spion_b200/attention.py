@@ -196,7 +196,7 @@ class Attention(nn.Module):
             # the layer above ignores the probabilities of the sparse phase (models/model_transformer.py:137 reads
             # them in the dense phase only): none are stored
             self.block_attn = BlockSparseAttention(config, dtype=self.native_dtype, keypad=self.with_keypad,
-                                                   device=model_dev, return_probs=False, recompute="layer")
+                                                   device=model_dev, return_probs=False)
             return
         if self.with_keypad:
             block_attn_cpp = Attention._blockcuda_mask_compile_module()

@@ -72,8 +72,7 @@ class BlockSparseAttention(nn.Module):
         self.return_probs = bool(return_probs) or not self.fused
         # recompute=True (fused kernels): the backward rebuilds P and dS on chip from the log-sum-exp and nothing
         # of size nnz exists in memory; False: the forward stores P, the backward reads it and writes dS
-        # (spion_attn_backward_ex).  None: chosen per mask in set_mask; "layer": the same, and small calls at head_dim 32 as
-        # a training step of an encoder wants them (_recompute_pays).
+        # (spion_attn_backward_ex).  None: chosen per mask in set_mask.
         self._recompute_arg = recompute
         self.recompute = self.fused and (recompute is None or bool(recompute))
         self.last = None
@@ -112,7 +111,7 @@ class BlockSparseAttention(nn.Module):
         m8 = (mat != 0).to(torch.uint8).contiguous().to(self.device)
         self._ctx.set_pattern(m8, self.bs)
         self.nnzb = int(lib.spion_pattern_nnzb(self.handle))
-        if self.fused and self._recompute_arg in (None, "layer"):
+        if self.fused and self._recompute_arg is None:
             self.recompute = self._recompute_pays()
         from .pattern import pattern_from_mask
         self._pattern = pattern_from_mask(m8, self.bs)          # block CSR for the helpers above
@@ -134,17 +133,16 @@ class BlockSparseAttention(nn.Module):
         comes from P before it is rounded (error against fp64 2.4e-3 instead of 3.1e-3): recompute=True asks for them.
         32-wide blocks and the full mask are rebuilt in any case.
 
-        Attention layers ("layer") keep stored tiles at head_dim 32 with fewer than 2^15 selected blocks in all matrices.  P is
-        normalised before and not after it is rounded to bf16 there, and a training step of the encoder classifier at such sizes
-        multiplies any change of rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to 3.3e-1 of
-        their norm over eight seeds (both paths are equally far from the fp32 step).  The bound is a line between measured sizes
-        that leaves those steps as they were; it is no property of the kernels."""
+        head_dim 32 with fewer than 2^15 selected blocks in all matrices: stored tiles, although the rebuilt ones are faster there too (the
+        three cases above).  P is normalised before and not after it is rounded to bf16, and a training step of the encoder classifier at
+        such sizes multiplies any change of rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to
+        3.3e-1 of their norm over eight seeds (both paths are equally far from the fp32 step).  The bound is a line between measured
+        sizes that leaves those steps as they were; it is no property of the kernels, and recompute=True takes the faster path
+        below it as well.  The rule is the same for attention layers and for direct calls: one problem, one result."""
         nb = self.L // self.bs
         if self.bs == 32 or self.nnzb == nb * nb:
             return True
-        if self.return_probs:
-            return False
-        return self._recompute_arg is None or self.d == 64 or self.BH * self.nnzb >= 1 << 15
+        return not self.return_probs and (self.d == 64 or self.BH * self.nnzb >= 1 << 15)
 
     @property
     def nnz(self) -> int:

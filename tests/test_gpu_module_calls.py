@@ -141,6 +141,28 @@ def test_gradients_of_a_call_that_returns_its_probabilities(d, padded):
         out.backward(do)
 
 
+@pytest.mark.parametrize("d,batch", [(32, 2), (32, 1023), (32, 1024), (64, 2)])
+def test_one_backward_path_for_a_layer_and_a_direct_call(d, batch):
+    """The path follows from the problem and not from the module that asks (16 selected blocks: 2 * 1024 * 16 is the bound at 32)."""
+    from spion_b200.attention import Attention
+    from spion_b200.native import BlockSparseAttention
+    cfg = config(dtype="bf16", head_dim=d, transformer_dim=H * d, batch_size=batch, max_seq_len=512)
+    mat = torch.eye(8, device="cuda") + torch.diag(torch.ones(7, device="cuda"), 1)
+    mat[7, 0] = 1
+    layer = Attention(cfg).cuda()
+    layer.reconstruct_for_blocksparse(cfg)
+    mod = BlockSparseAttention(cfg, dtype=torch.bfloat16, keypad=True, return_probs=False)
+    for m in (layer.block_attn, mod):
+        m.set_mask(mat)
+    assert mod.nnzb == 16 and mod.recompute == layer.block_attn.recompute == (d == 64 or batch == 1024)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v, do = (torch.randn(batch, H, 512, d, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4))
+    for t in (q, k, v):
+        t.requires_grad_()
+    keys = torch.ones(batch, 512, device="cuda")
+    same(*(torch.autograd.grad(m(q, k, v, keys)[0], (q, k, v), do) for m in (layer.block_attn, mod)))
+
+
 def test_changed_probabilities_of_a_drop_in_layer_are_noticed():
     layer, (x, keys) = make_layer("drop-in", task="lra-image"), make_inputs()
     out, probs = layer(x, keys, make_mask(4))
