@@ -38,6 +38,8 @@ class BlockSparseAttention(nn.Module):
     def __init__(self, config, dtype=torch.float32, keypad: bool = False, engine: int = _lib.ENGINE_AUTO,
                  device=None, fused=None, return_probs: bool = True, recompute=None, block32: str = "auto"):
         super().__init__()
+        if isinstance(recompute, str):                          # every word would count as True
+            raise _lib.SpionError(f"recompute must be None, False or True, not {recompute!r}")
         self.d = config["head_dim"]
         self.H = config["num_head"]
         self.L = config["max_seq_len"]

@@ -35,6 +35,18 @@ def test_discovery_refuses_maps_of_several_devices():
         pattern._discover(maps, 64, 0.9, "diag", 31, "paths", 0)
 
 
+def test_a_word_does_not_choose_the_backward_path():
+    """recompute is None, False or True; a word ("stored" among them) is refused before anything is created."""
+    import pytest
+
+    from spion_b200._lib import SpionError
+    from spion_b200.native import BlockSparseAttention
+    config = {"head_dim": 32, "num_head": 2, "max_seq_len": 256, "batch_size": 2, "block_size": 64}
+    for word in ("stored", "layer", ""):
+        with pytest.raises(SpionError, match="recompute must be"):
+            BlockSparseAttention(config, dtype=torch.bfloat16, device="cuda:0", recompute=word)
+
+
 def test_optimizer_state_by_parameter():
     """The state of an optimizer over pieces of the parameters is that of one over the parameters, in both directions."""
     import copy
