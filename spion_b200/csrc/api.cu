@@ -330,7 +330,6 @@ extern "C" const char* spion_stage_name(int stage) {
 }
 
 // fp32 contexts run the fused SIMT kernels unless the per-stage ones are forced
-static bool is_full(const spion_ctx* c) { return c->nnzb == c->nb * c->nb; }
 static bool use_simt_fused(const spion_ctx* c, int value_mode) {
   return c->dtype == SPION_F32 && c->engine != SPION_ENGINE_SIMT_STAGED &&
          simt_fused_supports(c->bs, c->d, c->BH, value_mode);
@@ -379,7 +378,7 @@ static int block_forward(spion_ctx* c, const float* Q, const float* K, OperandLa
   // floor of the running maximum: -100 (models/block_attn.cu:48) or 0 (models/block_attn_mask.cu:105)
   if (use_simt_fused(c, VAL_ELEMCSR)) {
     rc = simt_fused_forward(Q, rm, K, lk, V, rm, is_kpm(c) ? keypad : nullptr, is_kpm(c) ? 0.0f : -100.0f, attn, vl, out,
-                            rm, p, c->BH, c->L, c->d, c->scale, c->stream, is_full(c));
+                            rm, p, c->BH, c->L, c->d, c->scale, c->stream, c->nnzb);
     if (!rc) prof_mark(c, SPION_STAGE_FUSED_FWD);
     c->launches += 1;
     return rc;
@@ -412,7 +411,7 @@ static int block_backward(spion_ctx* c, const float* Q, const float* K, const fl
   if (use_simt_fused(c, VAL_ELEMCSR)) {
     c->launches += 2;
     return simt_fused_backward(Q, rm, K, rm, V, lv, P, vl, O, rm, dO, rm, dS_scratch, vl, dQ, rm, dK, rm, dV, rm, p, c->BH, c->d,
-                               c->scale, c->stream, c, is_full(c));
+                               c->scale, c->stream, c, c->nnzb);
   }
   if (!dP_scratch) return SPION_ERR_ARG;
   rc = simt_sddmm(SPION_F32, SPION_F32, dO, rm, V, lv, dP_scratch, vl, p, c->nnzb, c->BH, c->d, c->stream);
@@ -608,7 +607,7 @@ extern "C" int spion_attn_forward_ex(spion_ctx* c, const void* Q, const void* K,
   if (use_simt_fused(c, VAL_BLOCKTILE)) {
     int rc = simt_fused_forward((const float*)Q, rm, (const float*)K, rm, (const float*)V, rm, keypad,
                                 keypad ? 0.0f : -100.0f, (float*)P, vl, (float*)O, rm, p, c->BH, c->L, c->d, c->scale,
-                                c->stream, is_full(c));
+                                c->stream, c->nnzb);
     if (!rc) prof_mark(c, SPION_STAGE_FUSED_FWD);
     c->launches += 1;
     return rc;
@@ -648,7 +647,7 @@ extern "C" int spion_attn_backward_ex(spion_ctx* c, const void* Q, const void* K
     c->launches += 2;
     return simt_fused_backward((const float*)Q, rm, (const float*)K, rm, (const float*)V, rm, (const float*)P, vl,
                                (const float*)O, rm, (const float*)dO, rm, (float*)dS, vl, (float*)dQ, rm, (float*)dK, rm, (float*)dV, rm, p,
-                               c->BH, c->d, c->scale, c->stream, c, is_full(c));
+                               c->BH, c->d, c->scale, c->stream, c, c->nnzb);
   }
   if (!dP_scratch) return SPION_ERR_ARG;
   int rc = simt_sddmm(c->dtype, SPION_F32, dO, rm, V, rm, dP_scratch, vl, p, c->nnzb, c->BH, c->d, c->stream);

@@ -165,12 +165,12 @@ int softmax_bwd_dense_t(const float* dP, const float* P, float* dS, int BH, int 
 bool simt_fused_supports(int bs, int d, int BH, int value_mode);
 int simt_fused_forward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,
                        OperandLayout lv, const float* keypad, float floor_v, float* P, ValueLayout vl, float* O,
-                       OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st, bool full);
+                       OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st, int nnzb);
 int simt_fused_backward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,
                         OperandLayout lv, const float* P, ValueLayout vp, const float* O_or_null, OperandLayout lo,
                         const float* dO, OperandLayout ldo, float* dS, ValueLayout vds, float* dQ, OperandLayout ldq,
                         float* dK, OperandLayout ldk, float* dV, OperandLayout ldv, Pattern p, int BH, int d,
-                        float scale, cudaStream_t st, struct spion_ctx* prof, bool full);
+                        float scale, cudaStream_t st, struct spion_ctx* prof, int nnzb);
 
 // simt_full.cu: the same on a full mask, in a fixed order of additions
 int simt_full_forward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,

@@ -923,18 +923,30 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
 
 // With eight rows per thread a block row is one warp (block 32) or four (64).  Up to two warps per scheduler (four per SM) each of
 // them is a chain of latencies, and half the rows per thread shorten it (16 matrices, L = 1024, d 32, blocks of 32 at 15 %:
-// forward 31 -> 22 us, rows 22 -> 20); above, the larger micro-tile is worth more.  While all block rows fit the chip at once with
-// several groups of threads each (512 threads an SM), the groups of a CTA share the blocks of its row (forward and row kernels),
-// L = 1024, d 32, blocks of 32 at 15 %: 2 matrices, four groups, forward 20.2 -> 11.6 us, rows 18.5 -> 10.9; 16 matrices, two groups, 26.7 ->
-// 23.1 and 24.7 -> 22.3 (four groups, in two waves: no gain).  Blocks of 64: 2 matrices, d 32, L = 2048, 30 %: 82 -> 78, 76 -> 72.
-// Columns are better shared by a cluster (see SPLIT).
+// forward 31 -> 22 us, rows 22 -> 20); above, the larger micro-tile is worth more.
 constexpr long long FEW_WARPS = 4 * 2;                // per SM
-#define SPION_FUSED_DISPATCH(FN, ...)                                                                \
+// Groups of threads that share the blocks of a row (forward and row kernels; columns are better shared by a cluster, see SPLIT).  They pay
+// where the rows have blocks to share and some are longer than others, and lose in a second wave of CTAs with equal rows.  us of the forward
+// and of the row kernel with one group, two (and four); masks with a band of two blocks and random ones unless stated:
+//   blocks of 32: four up to one CTA per SM (d 32, 128 rows of 5 blocks, the longest 8: 16.6, 10.5, 9.1 and 15.6, 9.9, 8.5), two up to four
+//     (512 such rows 23.2, 20.5, 23.1 and 21.5, 19.7, 21.7; d 64, 288 rows of two blocks 12.0, 8.3, 12.5 and 12.3, 9.6, 13.5).  d 64: half the
+//     registers make the row kernel slower from 512 rows on (36.1, 37.4; 384 rows 36.8, 34.3), so its line is three CTAs per SM.
+//   blocks of 64 (512 threads for two groups): d 64, 128 rows of 10 blocks 74, 69 and 73, 63; 192 rows of 3 blocks 48, 44 and 47, 41, of 4
+//     62, 53 and 61, 49 (all of 4: 39.8, 42.8 and 38.9, 40.1); 288 rows of 3 48, 52 and 47, 48, of 8 131, 133 and 126, 122; rows of two blocks:
+//     128 13.3, 13.4 and 13.2, 12.4, 192 21.5, 24.6 and 21.3, 22.9.  So three CTAs for two SMs, and one per SM if the rows are short.
+//   rows of one block: the joins are pure cost (blocks of 32, d 64, 512 rows: 8.0, 8.9 and 8.4, 10.1; blocks of 64, 128 rows 8.1, 8.9).
+// A pass of up to about 500 short rows is host time whatever the groups (90 us forward + backward).
+static int row_groups(int bs, int d, long long rows, long long nnzb, int nb, bool backward) {
+  const long long sms = sm_count();
+  if (2 * nnzb < 3LL * nb) return 1;                  // most rows have one block
+  if (bs == 64) return 2 * rows <= (nnzb < 3LL * nb ? 2 : 3) * sms ? 2 : 1;
+  return rows <= sms ? 4 : rows <= (backward && d == 64 ? 3 : 4) * sms ? 2 : 1;
+}
+#define SPION_FUSED_DISPATCH(FN, BACKWARD, ...)                                                      \
   do {                                                                                               \
     const long long units = (long long)p.nb * BH;                                                    \
     const bool few = units * p.bs * p.bs / 1024 <= FEW_WARPS * sm_count();                           \
-    const int ways = p.bs == 32 ? (units <= 2 * sm_count() ? 4 : units <= 4 * sm_count() ? 2 : 1)    \
-                                : (units <= 2 * sm_count() ? 2 : 1);                                 \
+    const int ways = row_groups(p.bs, d, units, nnzb, p.nb, BACKWARD);                               \
     if (p.bs == 32 && d == 32)                                                                       \
       return ways == 4 ? FN<32, 32, 4, 4>(__VA_ARGS__) : ways == 2 ? FN<32, 32, 4, 2>(__VA_ARGS__)   \
              : few ? FN<32, 32, 4, 1>(__VA_ARGS__) : FN<32, 32, 8, 1>(__VA_ARGS__);                  \
@@ -948,23 +960,23 @@ constexpr long long FEW_WARPS = 4 * 2;                // per SM
     return SPION_ERR_UNSUPPORTED;                                                                    \
   } while (0)
 
-// full: every block is selected (simt_full.cu)
+// The full mask has kernels of its own (simt_full.cu).
 int simt_fused_forward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,
                        OperandLayout lv, const float* keypad, float floor_v, float* P, ValueLayout vl, float* O,
-                       OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st, bool full) {
+                       OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st, int nnzb) {
   if (!simt_fused_supports(p.bs, d, BH, vl.mode)) return SPION_ERR_UNSUPPORTED;
-  if (full) return simt_full_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
-  SPION_FUSED_DISPATCH(fwd_launch, Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, scale, st);
+  if (nnzb == p.nb * p.nb) return simt_full_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
+  SPION_FUSED_DISPATCH(fwd_launch, false, Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, scale, st);
 }
 
 int simt_fused_backward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,
                         OperandLayout lv, const float* P, ValueLayout vp, const float* O, OperandLayout lo,
                         const float* dO, OperandLayout ldo, float* dS, ValueLayout vds, float* dQ, OperandLayout ldq,
                         float* dK, OperandLayout ldk, float* dV, OperandLayout ldv, Pattern p, int BH, int d,
-                        float scale, cudaStream_t st, spion_ctx* prof, bool full) {
+                        float scale, cudaStream_t st, spion_ctx* prof, int nnzb) {
   if (!simt_fused_supports(p.bs, d, BH, vp.mode) || vds.mode != vp.mode) return SPION_ERR_UNSUPPORTED;
-  if (full && O)
+  if (nnzb == p.nb * p.nb && O)
     return simt_full_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof);
-  SPION_FUSED_DISPATCH(bwd_launch, Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH,
+  SPION_FUSED_DISPATCH(bwd_launch, true, Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH,
                        scale, st, prof);
 }

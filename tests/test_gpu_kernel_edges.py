@@ -126,6 +126,32 @@ def test_fp32_rows_shared_by_groups(bs, d, B, H, nb, layout):
     cpp.destroy(handle)
 
 
+# (bs, d, B, blocks per side, blocks per row, groups of threads per row forward, backward): both sides of one, one and a half, three and
+# four block rows per SM (148 SMs), rows of one and two blocks
+@pytest.mark.parametrize("bs,d,B,nb,per,forward,backward",
+                         [(32, 32, 37, 4, 2, 4, 4), (32, 32, 30, 5, 2, 2, 2), (32, 64, 111, 4, 3, 2, 2), (32, 64, 89, 5, 3, 2, 1),
+                          (32, 32, 148, 4, 2, 2, 2), (32, 64, 119, 5, 2, 1, 1), (32, 32, 40, 4, 1, 1, 1), (64, 64, 37, 4, 2, 2, 2),
+                          (64, 32, 37, 6, 3, 2, 2), (64, 64, 45, 5, 3, 1, 1), (64, 64, 30, 5, 2, 1, 1), (64, 64, 20, 5, 1, 1, 1)])
+def test_fp32_groups_per_row(bs, d, B, nb, per, forward, backward):
+    from torch.profiler import ProfilerActivity, profile
+
+    from spion_b200.native import BlockSparseAttention
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(29 + nb, B, 1, L, d)
+    mat = np.zeros((nb, nb), np.uint8)
+    for x in range(per):
+        mat[np.arange(nb), (np.arange(nb) + x) % nb] = 1
+    mod = BlockSparseAttention(cfg(B, 1, L, d, bs), dtype=torch.float32)
+    mod.set_mask(torch.as_tensor(mat).cuda())
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        got = run(mod, Q, K, V, dO, mat, None)
+        torch.cuda.synchronize()
+    compare(got, Q, K, V, dO, mat, bs, None, FP32_TOL, False)
+    names = {e.name for e in p.events()}
+    for kernel, groups in (("fused_fwd_kernel", forward), ("fused_bwd_row_delta_kernel", backward)):
+        assert any(f"{kernel}<{bs}, {d}, 4, {groups}>" in n for n in names), names
+
+
 @pytest.mark.parametrize("L,d", [(64, 64), (192, 32), (512, 32), (576, 32), (1024, 64), (1088, 32), (1856, 32)])
 @pytest.mark.parametrize("padded", [False, True])
 def test_dense_fp32_kernels(L, d, padded):
