@@ -103,8 +103,19 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
   // group's warps); s_ready[pair % NS]: S and dP of a pair in tensor memory; t_free[set]: ... read out (the group's warps);
   // acc_done[group][parity of the units it writes]: accumulators complete; acc_free[set]: ... read out (the group's warps); f_full /
   // f_free[2]: fixed tiles landed / no longer read; r_full / r_free[half]: 16 records written / read (all warps but warp 3).
-  // A parity tells two phases apart, so every barrier has one waiter (a warp, a group's warps; r_full: each reader for itself) that
-  // waits for each of its phases, and a phase cannot complete before the one before it has been waited for.
+  // A parity tells two phases apart: at a wait for a phase the one before it must be over, and the one after it must not be.  Most
+  // barriers have one waiter (a warp, a group's warps; r_full: each reader for itself) that waits for each of their phases, and the next
+  // phase needs something that comes after the wait.  The others:
+  //   s_ready, fewer or more barriers than groups (COL at head_dim 64: three, two groups): the group of pair j did not wait for pair j - NS.
+  //     It has waited for pdone of pair j - NPD, whose products warp 2 issued after those of pair j - NS, for which that pair's group had
+  //     to see its S.  S of pair j + NS is issued after that of pair j + 3, which waits for this group's t_free of pair j.
+  //   pdone, waited for by warp 0 and by the groups of COL, with more slots than value tiles (head_dim 32: five, four groups, a group sees
+  //     every fourth phase of a slot): pair i = j - NPD is the group's own, and its tiles were requested when warp 0 had seen pdone of
+  //     pair i - NP.  The products of pair i + NP come after those of pair j, which wait for this group's p_ready.
+  // A group writes the rows of a finished unit after its next pair, so there must be a set of accumulators for each group's last unit.
+  static_assert(C::NS >= 3 && (C::NS == NGR || (SIDE == COL && C::NPD <= C::NS)), "s_ready");
+  static_assert(SIDE == ROW || (C::NPD % NGR == 0 && C::NPD <= NP), "pdone");
+  static_assert(NACC >= NGR, "accumulators");
   const uint32_t pfull = bars, pdone = bars + 64, p_ready = bars + 128, s_ready = bars + 192, t_free = bars + 224, acc_done = bars + 248,
                  acc_free = bars + 312, f_full = bars + 344, f_free = bars + 360, r_full = bars + 376, r_free = bars + 392,
                  slot = bars + 408, abort_w = bars + 412;
