@@ -111,6 +111,55 @@ def test_linear_kernels_on_bf16_tokens(B, L, H, d, N, nw, split):
     assert _rel(db, (dY.double() if nw == 1 else dY).sum(0)) < 2e-6
 
 
+# The other results of bf16 tokens read through tensor maps (more than 148 tiles of 128).  W enters the products rounded to bf16, the sums are
+# fp32: results rounded to bf16 as the reference's are differ where such a sum (error about 2^-20) falls beside a tie, in at most a few
+# of a hundred elements, by 2^-8 each: less than 1e-3 in norm.
+def _bf(t):
+    return t.to(torch.bfloat16).double()
+
+
+@pytest.mark.parametrize("B,L,H,d,N", [(101, 192, 2, 32, 64), (61, 320, 1, 64, 64), (101, 192, 2, 64, 192), (40, 1984, 4, 32, 96)])
+@pytest.mark.parametrize("split", [False, True])
+def test_bf16_gradient_of_three_layers(B, L, H, d, N, split):
+    """Each layer's gradient rounded, added in bf16 from the last to the first."""
+    T, K = B * L, H * d
+    g = torch.Generator(device="cuda").manual_seed(T + N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    P, st = ctypes.c_void_p, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    shape, lay = ((B, H, L, d), (H, d, L)) if split else ((T, K), (0, 0, 0))
+    dY = [rnd(*shape).to(torch.bfloat16) for _ in range(3)]
+    Ws, dX = [rnd(K, N) for _ in range(3)], torch.full((T, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    check(lib.spion_linear_backward_input(ctypes.byref(_tokens(dY, *lay)), (P * 3)(*[w.data_ptr() for w in Ws]), 3, 0, None,
+                                          ctypes.byref(_tokens([dX])), T, N, 3 * K, st))
+    torch.cuda.synchronize()
+    assert lib.spion_linear_status(1) == 0
+    a, b, c = (_bf((t.permute(0, 2, 1, 3).reshape(T, K) if split else t).double() @ _bf(w)) for t, w in zip(dY, Ws))
+    assert _rel(dX, _bf(_bf(c + b) + a)) < 1e-3
+
+
+@pytest.mark.parametrize("T,K,N", [(19073, 64, 128), (19456, 96, 64), (75776, 128, 256)])
+def test_gelu_on_bf16_tokens(T, K, N):
+    """Forward with the activation, and the gradient through it."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    P, st = ctypes.c_void_p, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    ptrs = lambda t: (P * 3)(t.data_ptr(), None, None)
+    X, W, b = rnd(T, K).to(torch.bfloat16), rnd(N, K) / K ** 0.5, rnd(N)
+    Y, G = (torch.full((T, N), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    check(lib.spion_linear_forward(ctypes.byref(_tokens([X])), ptrs(W), ptrs(b), 1, 0, ctypes.byref(_tokens([Y])), P(G.data_ptr()), T, K, N, st))
+    dY, V = rnd(T, K).to(torch.bfloat16), rnd(K, N) / N ** 0.5           # of a second layer [K, N] behind the activation
+    dX = torch.full((T, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    check(lib.spion_linear_backward_input(ctypes.byref(_tokens([dY])), ptrs(V), 1, 0, P(Y.data_ptr()), ctypes.byref(_tokens([dX])), T, N, K, st))
+    torch.cuda.synchronize()
+    assert lib.spion_linear_status(1) == 0
+    assert _rel(Y, _bf(X.double() @ _bf(W).t() + _bf(b))) < 1e-3
+    h = Y.double().requires_grad_()
+    act = torch.nn.functional.gelu(h)
+    assert _rel(G, _bf(act.detach())) < 1e-3
+    slope, = torch.autograd.grad(act.sum(), h)
+    assert _rel(dX, _bf(_bf(dY.double() @ _bf(V)) * slope)) < 1e-3
+
+
 @pytest.mark.parametrize("native,dtype,bs,L,dense", [(True, "bf16", 64, 192, False), (True, "bf16", 64, 128, True),
                                                      (True, "fp32", 32, 160, False), (False, "fp32", 32, 96, False)])
 def test_attention_layer_in_one_node_equals_its_stages(native, dtype, bs, L, dense):
