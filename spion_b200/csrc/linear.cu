@@ -153,11 +153,11 @@ struct GemmArgs {
   int nc, nstages;          // output features per CTA (blockIdx.y), stages of the A ring
   int nacc;                 // accumulators per tile (fp32 mode): the leading products rotate over nacc - 1 of them by chunk
   int parts;                // bf16 gradient of three stacked layers: chunks per layer (0: one accumulator for the whole contraction)
+  int tma;                  // bf16 A through maps.m[0 .. 2] (MAP_*)
   const __nv_bfloat16* h;   // EPI_DGELU: pre-activation [T, N]
   __nv_bfloat16* g;         // EPI_GELU: activation [T, N] (Y receives the pre-activation)
   // What a backward reads in place of the caller's tensors.  262144 tokens of 64 fp32 features: 33 MB written here, 33 MB less read by
   // the weight gradient; the layer of 128 x 2 matrices, L = 4096 went from 1432 to 1458 us.
-  int tma;                  // bf16 A through maps.m[0 .. 2] (MAP_*)
   __nv_bfloat16* x_copy;    // or null: A as the products use it, [T, K] (fp32 tokens in bf16 mode)
   float* w_copy;            // or null: the stacked W
 };

@@ -888,8 +888,6 @@ int bwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout l
                                                                      BH, scale);
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_BWD_ROW);
-  // Many (b,h) matrices even out columns of different lengths by themselves; below SPLIT_WAVES waves of CTAs the longest
-  // column would decide, and there is room for the CTAs that a split column takes.
   const dim3 cgrid(p.nb, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
   // Many (b,h) matrices even out columns of different lengths by themselves; below SPLIT_WAVES waves of CTAs the longest
   // column would decide, and there is room for the CTAs that a split column takes.

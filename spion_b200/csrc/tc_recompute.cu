@@ -31,9 +31,10 @@ constexpr size_t MM_SMEM(int tile_bytes) { return 1024 + (size_t)2 * 2 * 2 * til
 // every TMEM quadrant, second in lanes 16-31) through two stages: while the probabilities of one pair are
 // summed in registers, the S tiles of the next pair are already being computed and the tiles of the pair
 // after that are on their way.  Every thread keeps the 64 running sums of its row.
-// The log-sum-exp and the penalties of a pair (one key per thread, handed round through shared memory) are requested while the pair
-// before is summed; asked for where they were used, two loads in a row were most of a pair's time, and a block with padded keys took
-// 64 more per thread.  18 matrices, L = 1984, d 32, padded keys: 46 -> 40 us.
+// The log-sum-exp and the penalties of a pair (one key per thread, handed round through shared memory) are requested when the pair before
+// has been summed, ahead of the barrier that ends it: the log-sum-exp has the wait for S to arrive, a penalty is waited for as soon as the
+// pair begins.  Asked for where they were used, two loads in a row were most of a pair's time, and a block with padded keys took 64 more
+// per thread.  18 matrices, L = 1984, d 32, padded keys: 46 -> 40 us.
 template <int D, bool SUB>
 __global__ void __launch_bounds__(128) k_mean_map_rc(const __grid_constant__ CUtensorMap tmQ,
                                                      const __grid_constant__ CUtensorMap tmK,
