@@ -71,8 +71,9 @@ __global__ void __launch_bounds__(256) conv_pool_kernel(const float* __restrict_
 // additions), the tile of the next one arrives by cp.async; the total of the row sums is one lane's work beside the next cell's
 // sums.  Tile rows are 16-byte pieces (A 16-byte aligned; a piece is inside or outside the map as a whole), 96 floats from column
 // j - 16 on; taps left or right of a row read its neighbours' values, but only for the skipped outputs.
-// Bound by the fp64 additions of the filter (31 per output, ordered): 62.8 us per L = 4096 map, 63.9 with one CTA per cell.  What
-// the loop over maps saves is a launch and a wave's tail per layer.
+// Limited by the ordered fp64 additions of the filter (31 per output): 62.8 us per L = 4096 map, 63.9 with one CTA per cell.  Of that time the
+// fp64 pipe is busy for 54 %, issue slots for 58 %, l1tex for 39 % (ncu, one map): no unit is full.  What the loop over maps saves is a
+// launch and a wave's tail per layer.
 struct MapList { const float* A[16]; };
 template <int BS, int F>
 __global__ void __launch_bounds__(256, 3) conv_pool_diag_kernel(const __grid_constant__ MapList maps, int layers, int L, float* __restrict__ pooled) {
