@@ -124,7 +124,7 @@ bool dev_alloc(T** p, size_t n) { return device_alloc((void**)p, n * sizeof(T)) 
 int rebuild_structure(spion_ctx* c) {
   c->launches += 1;
   return spion_launch_build_structure(c->mat, c->nb, c->nnzb_dev, c->row_ptr, c->col_idx, c->blk_row, c->col_ptr,
-                                      c->row_idx, c->csc_pos, c->work, c->stream);
+                                      c->row_idx, c->csc_pos, c->work, c->stream, c->nnzb_dev + 1);
 }
 
 bool is_dense(const spion_ctx* c) { return c->kind == SPION_KIND_DENSE || c->kind == SPION_KIND_DENSE_KPM; }
@@ -169,7 +169,7 @@ extern "C" spion_ctx* spion_create(int kind, int head_dim, int seq_len, int num_
   cudaGetDevice(&c->device);
   c->scale = 1.0f / sqrtf((float)head_dim);               // models/block_attn.cu:419
   c->stream = 0;
-  c->nnzb = -1;
+  c->nnzb = c->longest_col = -1;
   c->launches = 0;
   c->tc = nullptr;
   c->heads = 0;
@@ -181,7 +181,7 @@ extern "C" spion_ctx* spion_create(int kind, int head_dim, int seq_len, int num_
   const size_t cap = (size_t)nb * nb;
   bool ok = dev_alloc(&c->mat, cap) && dev_alloc(&c->row_ptr, (size_t)nb + 1) && dev_alloc(&c->col_idx, cap) &&
             dev_alloc(&c->blk_row, cap) && dev_alloc(&c->col_ptr, (size_t)nb + 1) && dev_alloc(&c->row_idx, cap) &&
-            dev_alloc(&c->csc_pos, cap) && dev_alloc(&c->work, cap) && dev_alloc(&c->nnzb_dev, 1) &&
+            dev_alloc(&c->csc_pos, cap) && dev_alloc(&c->work, cap) && dev_alloc(&c->nnzb_dev, 2) &&
             dev_alloc(&c->status_dev, 1);
   if (ok) ok = cudaMemset(c->status_dev, 0, sizeof(int)) == cudaSuccess;
   if (ok && dense) {
@@ -359,6 +359,7 @@ static int legacy_structure(spion_ctx* c, const int* offsets, const int* columns
   if (rc) return rc;
   prof_mark(c, SPION_STAGE_STRUCTURE);
   c->nnzb = nnzb;
+  c->longest_col = -1;
   return SPION_OK;
 }
 
@@ -574,10 +575,11 @@ extern "C" int spion_set_pattern(spion_ctx* c, const uint8_t* mat) {
   SPION_CUDA_TRY(cudaMemcpyAsync(c->mat, mat, (size_t)c->nb * c->nb, cudaMemcpyDeviceToDevice, c->stream));
   int rc = rebuild_structure(c);
   if (rc) return rc;
-  int32_t n = 0;
-  SPION_CUDA_TRY(cudaMemcpyAsync(&n, c->nnzb_dev, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  int32_t n[2] = {0, 0};
+  SPION_CUDA_TRY(cudaMemcpyAsync(n, c->nnzb_dev, sizeof(n), cudaMemcpyDeviceToHost, c->stream));
   SPION_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  c->nnzb = n;
+  c->nnzb = n[0];
+  c->longest_col = n[1];
   if (tc_engine_supports(c)) {
     rc = tc_engine_prepare(c);
     if (rc) return rc;

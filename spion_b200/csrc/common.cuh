@@ -78,8 +78,10 @@ struct spion_ctx {
   cudaStream_t stream;
   // structure workspace (device), capacity nb*nb blocks
   uint8_t* mat;
-  int32_t *row_ptr, *col_idx, *blk_row, *col_ptr, *row_idx, *csc_pos, *work, *nnzb_dev;
+  int32_t *row_ptr, *col_idx, *blk_row, *col_ptr, *row_idx, *csc_pos, *work;
+  int32_t* nnzb_dev;        // block count, entries of the longest column
   int nnzb;                 // block count of the current pattern (host copy), -1 if none
+  int longest_col;          // entries of its longest column, -1 if the host does not know
   int csr_stable;           // reference-layout calls: the caller keeps its element-CSR arrays alive and unchanged
   const void* csr_key[3];   // ... and these are the arrays the current structure was built from
   int csr_nnz;
@@ -144,7 +146,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 // structure.cu
 int spion_launch_build_structure(const uint8_t* mat, int nb, int32_t* nnzb, int32_t* row_ptr, int32_t* col_idx,
                                  int32_t* blk_row, int32_t* col_ptr, int32_t* row_idx, int32_t* csc_pos,
-                                 int32_t* work, cudaStream_t st);
+                                 int32_t* work, cudaStream_t st, int32_t* longest_col = nullptr);
 int spion_launch_mat_from_elemcsr(const int* offsets, const int* columns, const int* sum_mat, int nb, int bs,
                                   uint8_t* mat, cudaStream_t st);
 int spion_launch_fill_mat(uint8_t* mat, int n, int value, cudaStream_t st);
@@ -171,6 +173,15 @@ int simt_fused_backward(const float* Q, OperandLayout lq, const float* K, Operan
                         const float* dO, OperandLayout ldo, float* dS, ValueLayout vds, float* dQ, OperandLayout ldq,
                         float* dK, OperandLayout ldk, float* dV, OperandLayout ldv, Pattern p, int BH, int d,
                         float scale, cudaStream_t st, struct spion_ctx* prof, int nnzb);
+
+// mma_fused.cu: the same with the products on the tensor cores (every value mode of simt_fused_supports)
+int mma_fused_forward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V, OperandLayout lv, const float* keypad,
+                      float floor_v, float* P, ValueLayout vl, float* O, OperandLayout lo, Pattern p, int BH, int L, int d, float scale,
+                      cudaStream_t st);
+int mma_fused_backward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V, OperandLayout lv, const float* P,
+                       ValueLayout vp, const float* O_or_null, OperandLayout lo, const float* dO, OperandLayout ldo, float* dS, ValueLayout vds,
+                       float* dQ, OperandLayout ldq, float* dK, OperandLayout ldk, float* dV, OperandLayout ldv, Pattern p, int BH, int d,
+                       float scale, cudaStream_t st, struct spion_ctx* prof, int nnzb, int longest_col);
 
 // simt_full.cu: the same on a full mask, in a fixed order of additions
 int simt_full_forward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,

@@ -1,7 +1,5 @@
-// Fused fp32 (CUDA-core) kernels of the block-sparse attention path: the fp32 entry points keep the
-// 1e-4 max-abs parity bound, which rules out TF32 / BF16 tensor-core inputs, so these run on the FMA
-// pipes; fusing removes the S / dP round trips through memory that the staged kernels of
-// simt_attn.cu make.
+// Fused fp32 kernels of the block-sparse attention path on the CUDA cores: the calls with too little work for those of mma_fused.cu (see
+// use_mma below).  Fusing removes the S / dP round trips through memory that the staged kernels of simt_attn.cu make.
 //
 //   fused_fwd_kernel   per block row:  S = Q K^T -> sparse row softmax -> P (written once) -> O = P V
 //                      replaces models/block_attn.cu:453-487 (cusparseSDDMM, scale_softmax_kernel, cusparseSpMM)
@@ -15,15 +13,10 @@
 // reads them back, writes the probabilities over them and feeds the second product.  The backward
 // row kernel does the same with dP in the dS tiles.
 //
-// Bound by the FMA pipes: scalar multiply-adds reach 47 TFLOP/s on this chip (register ports) and packed pairs 61, so the loops use
-// pairs.  With 4 x 4 micro-tiles every 64 multiply-adds took eight 16-byte reads of shared memory; now a bs x bs tile is
-// computed by bs^2/32 threads (one warp at bs 32, four at 64) with 8 x 4 micro-tiles, 12 to 16 reads per 128.  The threads of
-// one (b,h) matrix run on their own: a warp needs no CTA barrier, four warps a named one.  Tiles are unpadded, the 16-byte
-// pieces of row i exchanged by i / 4 (mod 8): a thread owns contiguous rows and four contiguous columns, so value tiles
-// move in 16-byte pieces, and the reads take no bank twice.
-// 512 matrices, L = 1024, d 32, 154 blocks of 32 (10.3 GFLOP a kernel, 170 us at the rate of packed pairs), before and now:
-// forward 474 -> 358 us (it also writes the values twice and reads them once), rows 441 -> 310, columns 320 -> 270.
-// 15 matrices, L = 3008, d 64, blocks of 64 at 8 % and one full column: columns 314 -> 158 (see SPLIT at that kernel).
+// Bound by latencies at these sizes, and by the FMA pipes: scalar multiply-adds reach 47 TFLOP/s on this chip (register ports) and packed
+// pairs 61, so the loops use pairs.  A bs x bs tile is computed by bs^2 / 16 threads with 4 x 4 micro-tiles.  The threads of one (b,h)
+// matrix run on their own, with a barrier of their own.  Tiles are unpadded, the 16-byte pieces of row i exchanged by i / 4 (mod 8): a
+// thread owns contiguous rows and four contiguous columns, so value tiles move in 16-byte pieces, and the reads take no bank twice.
 //
 // Layouts: operands through (row, column) strides, value tiles through tile_address(); only
 // layouts whose tile rows are contiguous (element CSR, block tiles) are accepted.
@@ -31,11 +24,13 @@
 
 #include <atomic>
 
-#include "common.cuh"
+#include "fp32_tiles.cuh"
+
+using namespace fp32;
 
 namespace {
 
-// R: rows of a tile per thread, 8, or 4 for calls that do not fill the chip (FEW_WARPS below)
+// R: rows of a tile per thread
 template <int BS, int D, int R>
 struct Cfg {
   static constexpr int TX = BS / 4;            // threads along a tile row
@@ -45,8 +40,7 @@ struct Cfg {
   static constexpr int TN = D / TX;            // output columns per thread in the bs x d products
   static constexpr int TILE = BS * D;          // floats of an operand tile
   static constexpr int VALS = BS * BS;         // ... of a value tile
-  static constexpr int RESIDENT = R == 4 || (BS == 32 && D == 64) ? 2 : 3;   // CTAs per SM that the tiles leave room for (five at 64, 32: registers)
-  static constexpr int RESIDENT2 = R == 4 || (BS == 32 && D == 64) ? 2 : 4;  // ... of the two-pass kernels
+  static constexpr int RESIDENT = 2;           // CTAs per SM
   static_assert(TN == 2 || TN == 4 || TN == 8, "unsupported shape");
 };
 
@@ -58,13 +52,10 @@ template <int BS, int D, int R, int W> constexpr int cta_resident(int n) { retur
 // float offset of 16-byte piece `piece` of row `row` in a tile of COLS columns
 template <int COLS>
 __device__ __forceinline__ int at(int row, int piece) { return row * COLS + ((piece ^ ((row >> 2) & 7)) << 2); }
-
-// the threads of problem g
-template <int NT>
-__device__ __forceinline__ void group_sync(int g) {
-  if (NT == 32) __syncwarp();
-  else asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(NT) : "memory");
-}
+struct Swizzle {
+  template <int COLS>
+  static __device__ __forceinline__ int at(int row, int piece) { return ::at<COLS>(row, piece); }
+};
 
 // column of the thread's y-th output in a bs x d product: groups of 4 (or 2) contiguous columns
 template <int BS, int D, int R>
@@ -90,87 +81,6 @@ __device__ __forceinline__ void load_vec(const float* tile, int row, int tx, flo
   }
 }
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// A [L x d] operand of one (b,h) matrix, or a value tile: element (i, n) at base + i*s_row + n*s_col.
-struct Operand {
-  const float* base;
-  long long s_row, s_col;
-  bool pieces;                                       // rows in 16-byte pieces
-  __device__ __forceinline__ Operand(const float* p, const OperandLayout& l, int bh)
-      : base(p + (long long)bh * l.bh_stride), s_row(l.sl), s_col(l.sd) {
-    pieces = s_col == 1 && (s_row & 3) == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
-  }
-  __device__ __forceinline__ Operand(const float* p, int stride)
-      : base(p), s_row(stride), s_col(1), pieces((reinterpret_cast<uintptr_t>(p) & 15) == 0) {}
-};
-
-// Start the asynchronous copy of rows row0 .. row0 + ROWS - 1 into
-// shared memory by the NT threads of one problem.  The caller
-// commits the group, waits for it and synchronises before the tile is read.
-template <int ROWS, int COLS, int NT>
-__device__ __forceinline__ void load_tile(float* dst, const Operand& o, int row0, int t) {
-  const float* src = o.base + row0 * o.s_row;
-  if (o.pieces) {
-    constexpr int STEP = NT / (COLS / 4);            // rows per round
-    const int row = t / (COLS / 4), c4 = t % (COLS / 4);
-    src += row * o.s_row + c4 * 4;
-    const long long step = STEP * o.s_row;
-#pragma unroll
-    for (int i = 0; i < ROWS / STEP; ++i) {
-      cp_async16(dst + at<COLS>(row + i * STEP, c4), src);
-      src += step;
-    }
-  } else if (o.s_col == 1) {
-    for (int idx = t; idx < ROWS * COLS; idx += NT) {
-      const int row = idx / COLS, col = idx % COLS;
-      cp_async4(dst + at<COLS>(row, col >> 2) + (col & 3), src + row * o.s_row + col);
-    }
-  } else {
-#pragma unroll 4
-    for (int idx = t; idx < ROWS * COLS; idx += NT) {
-      const int row = idx % ROWS, col = idx / ROWS;
-      cp_async4(dst + at<COLS>(row, col >> 2) + (col & 3), src + row * o.s_row + col * o.s_col);
-    }
-  }
-}
-
-// The value tiles of one block row: element (i, j) of its k-th tile at base + k * step + i * si + j.
-struct RowTiles {
-  long long base;
-  int si, step;
-  template <int BS>
-  static __device__ __forceinline__ RowTiles of(const ValueLayout& vl, int rp, int nblk) {
-    const long long base = (long long)rp * BS * BS;
-    return vl.mode == VAL_ELEMCSR ? RowTiles{base, nblk * BS, BS} : RowTiles{base, BS, BS * BS};
-  }
-};
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-constexpr float LOG2_E = 1.4426950408889634f;
-
-// Four consecutive values of a value tile (tile rows are contiguous; `vec`: 16-byte aligned).
-__device__ __forceinline__ float4 load_vals(const float* p, bool vec) {
-  return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
-}
-__device__ __forceinline__ void store_vals(float* p, float4 v, bool vec) {
-  if (vec) *reinterpret_cast<float4*>(p) = v;
-  else p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
-}
-__device__ __forceinline__ bool vec_ok(const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
 // Packed pairs of fp32: one instruction, two multiply-adds per lane.  The FMA pipe is no faster for it, but the loops below were
 // limited by issue slots (two multiply-adds in three instructions).
 using pair_t = unsigned long long;
@@ -192,8 +102,7 @@ __device__ __forceinline__ Quad load_quad(const float* p) {
 }
 
 // out[x][y] = sum_n A[row0+x][n] * B[tx*4+y][n], x = 0..3   (both tiles [bs x d] in shared memory; row0 a multiple of four; even and
-// odd n in one sum each).  A thread's eight rows are taken in two halves: the registers of all sixty-four sums would cost
-// a resident CTA.
+// odd n in one sum each).
 template <int BS, int D>
 __device__ __forceinline__ void tile_abt(const float* As, const float* Bs, int row0, int tx, float (&out)[4][4]) {
   pair_t acc[4][4];
@@ -350,7 +259,7 @@ template <int BS, int D, int R> __host__ __device__ constexpr int two_pass_float
 // once, after the last tile.
 // W > 1: W groups of threads take a share of the row's blocks each; maxima and denominators are joined between the passes, O at the end.
 template <int BS, int D, int R, int W>
-__global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D, R, W>(Cfg<BS, D, R>::RESIDENT2)) fused_fwd_kernel(const float* __restrict__ Q, OperandLayout lq,
+__global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D, R, W>(Cfg<BS, D, R>::RESIDENT)) fused_fwd_kernel(const float* __restrict__ Q, OperandLayout lq,
                                                            const float* __restrict__ K, OperandLayout lk,
                                                            const float* __restrict__ V, OperandLayout lv,
                                                            const float* __restrict__ keypad, float floor_v, float* P,
@@ -378,8 +287,8 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   const float scale2 = scale * LOG2_E;                          // scores in base-2 units
 
   int c_cur = k0 < k1 ? cols[k0] : 0, c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
-  load_tile<BS, D, C::NT>(Qs, Operand(Q, lq, bh), r * BS, t);
-  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Kb, c_cur * BS, t);
+  load_tile<Swizzle, BS, D, C::NT>(Qs, Operand(Q, lq, bh), r * BS, t);
+  if (k0 < k1) load_tile<Swizzle, BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Kb, c_cur * BS, t);
   cp_async_commit();
 
   // ---- pass 1: scores into the P tiles, running maximum and denominator per row
@@ -389,7 +298,7 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   for (int k = k0; k < k1; ++k) {
     const int c = c_cur;
     if (k + 1 < k1)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
+      load_tile<Swizzle, BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
@@ -421,7 +330,7 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   }
   c_cur = k0 < k1 ? cols[k0] : 0;
   c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
-  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Vb, c_cur * BS, t);
+  if (k0 < k1) load_tile<Swizzle, BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Vb, c_cur * BS, t);
   cp_async_commit();
   float inv[R];
 #pragma unroll
@@ -463,7 +372,7 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   if (k0 < k1) fetch_scores(k0);
   for (int k = k0; k < k1; ++k) {
     if (k + 1 < k1)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
+      load_tile<Swizzle, BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
     cp_async_commit();
     float* tile = mine + (long long)k * rt.step;
 #pragma unroll
@@ -499,7 +408,7 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
 // ------------------------------------------------------------------------------ backward, row side
 //   t = dP.P ; s = rowsum(t) ; dS = (t - P s) scale ; dQ = dS K     (models/block_attn.cu:90-130, :498-516)
 template <int BS, int D, int R, int W>
-__global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D, R, W>(Cfg<BS, D, R>::RESIDENT2)) fused_bwd_row_kernel(const float* __restrict__ dO, OperandLayout ldo,
+__global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D, R, W>(Cfg<BS, D, R>::RESIDENT)) fused_bwd_row_kernel(const float* __restrict__ dO, OperandLayout ldo,
                                                                const float* __restrict__ V, OperandLayout lv,
                                                                const float* __restrict__ K, OperandLayout lk,
                                                                const float* __restrict__ P, ValueLayout vp, float* dS,
@@ -525,8 +434,8 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   const bool vec_p = vec_ok(Pb), vec_s = vec_ok(dSb);
 
   int c_cur = k0 < k1 ? cols[k0] : 0, c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
-  load_tile<BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
-  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Vb, c_cur * BS, t);
+  load_tile<Swizzle, BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
+  if (k0 < k1) load_tile<Swizzle, BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Vb, c_cur * BS, t);
   cp_async_commit();
 
   // ---- pass 1: dP into the dS tiles, row sums of dP.P
@@ -535,7 +444,7 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   for (int x = 0; x < R; ++x) s[x] = 0.f;
   for (int k = k0; k < k1; ++k) {
     if (k + 1 < k1)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
+      load_tile<Swizzle, BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Vb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
@@ -581,11 +490,11 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   Sums<BS, D, R> o;
   c_cur = k0 < k1 ? cols[k0] : 0;
   c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
-  if (k0 < k1) load_tile<BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Kb, c_cur * BS, t);
+  if (k0 < k1) load_tile<Swizzle, BS, D, C::NT>(Bs + (k0 & 1) * C::TILE, Kb, c_cur * BS, t);
   cp_async_commit();
   for (int k = k0; k < k1; ++k) {
     if (k + 1 < k1)
-      load_tile<BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
+      load_tile<Swizzle, BS, D, C::NT>(Bs + ((k + 1) & 1) * C::TILE, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
@@ -652,10 +561,10 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
   const bool vec_p = vec_ok(Pb), vec_s = vec_ok(dSb);
 
   int c_cur = k0 < k1 ? cols[k0] : 0, c_nxt = k0 + 1 < k1 ? cols[k0 + 1] : 0;
-  load_tile<BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
-  if (k0 < k1) load_tile<BS, D, C::NT>(Vs, Vb, c_cur * BS, t);
+  load_tile<Swizzle, BS, D, C::NT>(As, Operand(dO, ldo, bh), r * BS, t);
+  if (k0 < k1) load_tile<Swizzle, BS, D, C::NT>(Vs, Vb, c_cur * BS, t);
   cp_async_commit();
-  if (k0 < k1) load_tile<BS, D, C::NT>(Ks, Kb, c_cur * BS, t);
+  if (k0 < k1) load_tile<Swizzle, BS, D, C::NT>(Ks, Kb, c_cur * BS, t);
   cp_async_commit();
 
   float delta[R];
@@ -699,7 +608,7 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
     }
     group_sync<C::NT>(g);                                        // Ss complete, V buffer free
     if (k + 1 < k1) {
-      load_tile<BS, D, C::NT>(Vs, Vb, c_nxt * BS, t);
+      load_tile<Swizzle, BS, D, C::NT>(Vs, Vb, c_nxt * BS, t);
       fetch_p(k + 1);
     }
     cp_async_commit();
@@ -707,7 +616,7 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
     group_sync<C::NT>(g);                                        // K tile k has landed
     tile_atb<BS, D, R>(Ss, Ks, ty, tx, o);
     group_sync<C::NT>(g);                                        // Ss and the K buffer are free
-    if (k + 1 < k1) load_tile<BS, D, C::NT>(Ks, Kb, c_nxt * BS, t);
+    if (k + 1 < k1) load_tile<Swizzle, BS, D, C::NT>(Ks, Kb, c_nxt * BS, t);
     cp_async_commit();
     c_cur = c_nxt;
     c_nxt = k + 2 < k1 ? cols[k + 2] : 0;
@@ -725,13 +634,13 @@ __global__ void __launch_bounds__(cta_threads<BS, D, R, W>(), cta_resident<BS, D
 //   dK[c] = sum_r dS(r,c)^T Q[r],  dV[c] = sum_r P(r,c)^T dO[r]     (models/block_attn.cu:526-536)
 // Two stages per entry of the column: (dS, Q) for dK and (P, dO) for dV; the copy of one stage is in
 // flight while the other is used.
-// SPLIT: a cluster of SPLIT_WAYS CTAs per column.  Discovered masks have columns that every row selects; one CTA would walk
-// such a column long after the others are done.  The CTAs of the cluster take a share of its entries each and the
+// A cluster of SPLIT_WAYS CTAs per column: there is room for them, and discovered masks have columns that every row selects; one CTA would
+// walk such a column long after the others are done.  The CTAs of the cluster take a share of its entries each and the
 // first adds the others' sums, in their order, through distributed shared memory.  Columns below SPLIT_MIN entries
 // are left to the first CTA; the others end at once.  Eight CTAs per column were slower than four (16 matrices, L = 1024, blocks
 // of 32 at 15 %: 57 against 24 us, 41 without a split).
 constexpr int SPLIT_WAYS = 4, SPLIT_MIN = 3;
-template <int BS, int D, int R, bool SPLIT>
+template <int BS, int D, int R>
 __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) fused_bwd_col_kernel(const float* __restrict__ dS, ValueLayout vds,
                                                                const float* __restrict__ P, ValueLayout vp,
                                                                const float* __restrict__ Q, OperandLayout lq,
@@ -743,14 +652,13 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
   extern __shared__ __align__(16) float smem[];
   const int g = threadIdx.x / C::NT, t = threadIdx.x % C::NT;
   const int ty = t / C::TX, tx = t % C::TX;
-  const int c = SPLIT ? blockIdx.x / SPLIT_WAYS : blockIdx.x, part = SPLIT ? blockIdx.x % SPLIT_WAYS : 0;
+  const int c = blockIdx.x / SPLIT_WAYS, part = blockIdx.x % SPLIT_WAYS;
   const int bh_raw = blockIdx.y * C::G + g;
   const bool active = bh_raw < BH;
-  if (!SPLIT && !active) return;
-  const int bh = active ? bh_raw : BH - 1;                      // SPLIT: the cluster barriers take every thread
+  const int bh = active ? bh_raw : BH - 1;                      // the cluster barriers take every thread
   int e0 = p.col_ptr[c], e1 = p.col_ptr[c + 1];
-  const bool shared = SPLIT && e1 - e0 >= SPLIT_MIN;
-  if (SPLIT && !shared && (part > 0 || !active)) return;
+  const bool shared = e1 - e0 >= SPLIT_MIN;
+  if (!shared && (part > 0 || !active)) return;
   if (shared) {
     const int first = e0, n = e1 - e0;
     e0 = first + n * part / SPLIT_WAYS;
@@ -770,14 +678,14 @@ __global__ void __launch_bounds__(Cfg<BS, D, R>::CTA, Cfg<BS, D, R>::RESIDENT) f
   auto fetch_k = [&](int r, int blk) {                          // stage A: dS tile and Q rows of entry (r, blk)
     long long b1, s1, t1;
     tile_address(vds, p, r, c, blk, b1, s1, t1);
-    load_tile<BS, BS, C::NT>(dSs, Operand(dSb + b1, (int)s1), 0, t);
-    load_tile<BS, D, C::NT>(Qs, Qb, r * BS, t);
+    load_tile<Swizzle, BS, BS, C::NT>(dSs, Operand(dSb + b1, (int)s1), 0, t);
+    load_tile<Swizzle, BS, D, C::NT>(Qs, Qb, r * BS, t);
   };
   auto fetch_v = [&](int r, int blk) {                          // stage B: P tile and dO rows
     long long b2, s2, t2;
     tile_address(vp, p, r, c, blk, b2, s2, t2);
-    load_tile<BS, BS, C::NT>(Ps, Operand(Pb + b2, (int)s2), 0, t);
-    load_tile<BS, D, C::NT>(Os, dOb, r * BS, t);
+    load_tile<Swizzle, BS, BS, C::NT>(Ps, Operand(Pb + b2, (int)s2), 0, t);
+    load_tile<Swizzle, BS, D, C::NT>(Os, dOb, r * BS, t);
   };
   int r_cur = e0 < e1 ? p.row_idx[e0] : 0, b_cur = e0 < e1 ? p.csc_pos[e0] : 0;
   if (e0 < e1) fetch_k(r_cur, b_cur);
@@ -842,8 +750,6 @@ template <int BS, int D, int R, int W> constexpr size_t smem_row() {
 }
 template <int BS, int D, int R> constexpr size_t smem_col() { return sizeof(float) * Cfg<BS, D, R>::G * (2 * Cfg<BS, D, R>::TILE + 2 * Cfg<BS, D, R>::VALS); }
 
-constexpr int SPLIT_WAVES = 4;
-
 template <int BS, int D, int R, int W>
 int set_attrs() {
   static std::atomic<bool> done[64];
@@ -853,8 +759,7 @@ int set_attrs() {
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_fwd_kernel<BS, D, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R, W>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_kernel<BS, D, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_two_pass<BS, D, R, W>()));
   SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_row_delta_kernel<BS, D, R, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row<BS, D, R, W>()));
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
-  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
+  SPION_CUDA_TRY(cudaFuncSetAttribute(fused_bwd_col_kernel<BS, D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_col<BS, D, R>()));
   if (dev < 64) done[dev].store(true, std::memory_order_release);
   return SPION_OK;
 }
@@ -888,25 +793,18 @@ int bwd_launch(const float* Q, OperandLayout lq, const float* K, OperandLayout l
                                                                      BH, scale);
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_BWD_ROW);
-  const dim3 cgrid(p.nb, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
-  // Many (b,h) matrices even out columns of different lengths by themselves; below SPLIT_WAVES waves of CTAs the longest
-  // column would decide, and there is room for the CTAs that a split column takes.
-  if ((long long)cgrid.x * cgrid.y < (long long)SPLIT_WAVES * sm_count() * Cfg<BS, D, R>::RESIDENT) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cgrid.x * SPLIT_WAYS, cgrid.y);
-    cfg.blockDim = dim3(Cfg<BS, D, R>::CTA);
-    cfg.dynamicSmemBytes = smem_col<BS, D, R>();
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = SPLIT_WAYS;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    SPION_CUDA_TRY(cudaLaunchKernelEx(&cfg, fused_bwd_col_kernel<BS, D, R, true>, (const float*)dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH));
-  } else {
-    fused_bwd_col_kernel<BS, D, R, false><<<cgrid, Cfg<BS, D, R>::CTA, smem_col<BS, D, R>(), st>>>(dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH);
-  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.nb * SPLIT_WAYS, (BH + Cfg<BS, D, R>::G - 1) / Cfg<BS, D, R>::G);
+  cfg.blockDim = dim3(Cfg<BS, D, R>::CTA);
+  cfg.dynamicSmemBytes = smem_col<BS, D, R>();
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = SPLIT_WAYS;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  SPION_CUDA_TRY(cudaLaunchKernelEx(&cfg, fused_bwd_col_kernel<BS, D, R>, (const float*)dS, vds, P, vp, Q, lq, dO, ldo, dK, ldk, dV, ldv, p, BH));
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_SPMM_DKDV);
   return SPION_OK;
@@ -919,11 +817,20 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
          (value_mode == VAL_ELEMCSR || value_mode == VAL_BLOCKTILE);
 }
 
-// With eight rows per thread a block row is one warp (block 32) or four (64).  Up to two warps per scheduler (four per SM) each of
-// them is a chain of latencies, and half the rows per thread shorten it (16 matrices, L = 1024, d 32, blocks of 32 at 15 %:
-// forward 31 -> 22 us, rows 22 -> 20); above, the larger micro-tile is worth more.
-constexpr long long FEW_WARPS = 4 * 2;                // per SM
-// Groups of threads that share the blocks of a row (forward and row kernels; columns are better shared by a cluster, see SPLIT).  They pay
+// Which calls the kernels of mma_fused.cu serve: those with work for most schedulers.  Their warps do twice (block 32) or half (64) of what
+// the threads of a row do here, and they leave a column to one CTA, so few long rows are better shared by groups of threads.  us of forward, rows and
+// columns here and there (masks with rows of equal length):
+//   blocks of 32, d 32: 256 rows of 4 blocks 31, 32 in all; 192 of 8 41, 50; 512 of 4 48, 38; 592 of 2 32, 24; 2048 of 1 51, 42
+//     d 64: 256 rows of 8 76, 73; 512 of 4 80, 60; 1024 of 2 89, 64
+//   blocks of 64, d 64: 96 rows of 8 111, 127; 192 of 3 105, 81; 192 of 6 176, 146; 384 of 2 113, 80;  d 32: 192 of 3 73, 48; 768 of 1 78, 51
+// and with random blocks, 16384 rows of 5 blocks of 32 935, 735; 4096 rows of 3 blocks of 64, d 64 1138, 1004.  The lines leave some of
+// the gain to short rows.
+static bool use_mma(const Pattern& p, int BH, int nnzb) {
+  const long long sms = sm_count(), rows = (long long)p.nb * BH, blocks = (long long)nnzb * BH;
+  return p.bs == 32 ? rows >= 2 * sms && (blocks > 10 * sms || rows > 8 * sms) : rows >= sms && (blocks > 5 * sms || rows > 2 * sms);
+}
+
+// Groups of threads that share the blocks of a row (forward and row kernels; columns are shared by a cluster).  They pay
 // where the rows have blocks to share and some are longer than others, and lose in a second wave of CTAs with equal rows.  us of the forward
 // and of the row kernel with one group, two (and four); masks with a band of two blocks and random ones unless stated:
 //   blocks of 32: four up to one CTA per SM (d 32, 128 rows of 5 blocks, the longest 8: 16.6, 10.5, 9.1 and 15.6, 9.9, 8.5), two up to four
@@ -942,19 +849,13 @@ static int row_groups(int bs, int d, long long rows, long long nnzb, int nb, boo
 }
 #define SPION_FUSED_DISPATCH(FN, BACKWARD, ...)                                                      \
   do {                                                                                               \
-    const long long units = (long long)p.nb * BH;                                                    \
-    const bool few = units * p.bs * p.bs / 1024 <= FEW_WARPS * sm_count();                           \
-    const int ways = row_groups(p.bs, d, units, nnzb, p.nb, BACKWARD);                               \
+    const int ways = row_groups(p.bs, d, (long long)p.nb * BH, nnzb, p.nb, BACKWARD);                \
     if (p.bs == 32 && d == 32)                                                                       \
-      return ways == 4 ? FN<32, 32, 4, 4>(__VA_ARGS__) : ways == 2 ? FN<32, 32, 4, 2>(__VA_ARGS__)   \
-             : few ? FN<32, 32, 4, 1>(__VA_ARGS__) : FN<32, 32, 8, 1>(__VA_ARGS__);                  \
+      return ways == 4 ? FN<32, 32, 4, 4>(__VA_ARGS__) : ways == 2 ? FN<32, 32, 4, 2>(__VA_ARGS__) : FN<32, 32, 4, 1>(__VA_ARGS__); \
     if (p.bs == 32 && d == 64)                                                                       \
-      return ways == 4 ? FN<32, 64, 4, 4>(__VA_ARGS__) : ways == 2 ? FN<32, 64, 4, 2>(__VA_ARGS__)   \
-             : few ? FN<32, 64, 4, 1>(__VA_ARGS__) : FN<32, 64, 8, 1>(__VA_ARGS__);                  \
-    if (p.bs == 64 && d == 32)                                                                       \
-      return ways == 2 ? FN<64, 32, 4, 2>(__VA_ARGS__) : few ? FN<64, 32, 4, 1>(__VA_ARGS__) : FN<64, 32, 8, 1>(__VA_ARGS__); \
-    if (p.bs == 64 && d == 64)                                                                       \
-      return ways == 2 ? FN<64, 64, 4, 2>(__VA_ARGS__) : few ? FN<64, 64, 4, 1>(__VA_ARGS__) : FN<64, 64, 8, 1>(__VA_ARGS__); \
+      return ways == 4 ? FN<32, 64, 4, 4>(__VA_ARGS__) : ways == 2 ? FN<32, 64, 4, 2>(__VA_ARGS__) : FN<32, 64, 4, 1>(__VA_ARGS__); \
+    if (p.bs == 64 && d == 32) return ways == 2 ? FN<64, 32, 4, 2>(__VA_ARGS__) : FN<64, 32, 4, 1>(__VA_ARGS__); \
+    if (p.bs == 64 && d == 64) return ways == 2 ? FN<64, 64, 4, 2>(__VA_ARGS__) : FN<64, 64, 4, 1>(__VA_ARGS__); \
     return SPION_ERR_UNSUPPORTED;                                                                    \
   } while (0)
 
@@ -964,6 +865,7 @@ int simt_fused_forward(const float* Q, OperandLayout lq, const float* K, Operand
                        OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st, int nnzb) {
   if (!simt_fused_supports(p.bs, d, BH, vl.mode)) return SPION_ERR_UNSUPPORTED;
   if (nnzb == p.nb * p.nb) return simt_full_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
+  if (use_mma(p, BH, nnzb)) return mma_fused_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
   SPION_FUSED_DISPATCH(fwd_launch, false, Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, scale, st);
 }
 
@@ -975,6 +877,8 @@ int simt_fused_backward(const float* Q, OperandLayout lq, const float* K, Operan
   if (!simt_fused_supports(p.bs, d, BH, vp.mode) || vds.mode != vp.mode) return SPION_ERR_UNSUPPORTED;
   if (nnzb == p.nb * p.nb && O)
     return simt_full_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof);
+  if (use_mma(p, BH, nnzb)) return mma_fused_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof, nnzb,
+                                                      prof ? prof->longest_col : -1);
   SPION_FUSED_DISPATCH(bwd_launch, true, Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH,
                        scale, st, prof);
 }

@@ -10,8 +10,8 @@ namespace {
 
 __global__ void __launch_bounds__(1024) build_structure_kernel(
     const uint8_t* mat, int nb, int32_t* nnzb, int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr, int32_t* row_idx,
-    int32_t* csc_pos, int32_t* work) {
-  build_structure(mat, nb, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work);
+    int32_t* csc_pos, int32_t* work, int32_t* longest_col) {
+  build_structure(mat, nb, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, longest_col);
 }
 
 // Recover the block mask from the reference's element-level CSR (one CTA per block row).
@@ -57,8 +57,8 @@ __global__ void expand_csr_kernel(const int32_t* __restrict__ row_ptr, const int
 
 int spion_launch_build_structure(const uint8_t* mat, int nb, int32_t* nnzb, int32_t* row_ptr, int32_t* col_idx,
                                  int32_t* blk_row, int32_t* col_ptr, int32_t* row_idx, int32_t* csc_pos,
-                                 int32_t* work, cudaStream_t st) {
-  build_structure_kernel<<<1, 1024, 0, st>>>(mat, nb, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work);
+                                 int32_t* work, cudaStream_t st, int32_t* longest_col) {
+  build_structure_kernel<<<1, 1024, 0, st>>>(mat, nb, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, longest_col);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }

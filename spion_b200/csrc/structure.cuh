@@ -3,10 +3,11 @@
 #include "common.cuh"
 
 // mat [nb*nb] uint8 -> CSR (row_ptr, col_idx, blk_row), CSC (col_ptr, row_idx, csc_pos) and the block count.  work [nb*nb] receives
-// the CSR block id of every set cell.  A warp per line, 32 cells per step: the rows' bits are kept in shared memory, positions are
+// the CSR block id of every set cell, longest_col (if given) the entries of the longest column.  A warp per line, 32 cells per step: the rows' bits are kept in shared memory, positions are
 // ballot prefixes.  (One thread per line took 13 us at nb = 64: 256 dependent byte loads.)
 static __device__ void build_structure(const uint8_t* mat, int nb, int32_t* nnzb, int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row,
-                                       int32_t* col_ptr, int32_t* row_idx, int32_t* csc_pos, int32_t* work) {
+                                       int32_t* col_ptr, int32_t* row_idx, int32_t* csc_pos, int32_t* work,
+                                       int32_t* longest_col = nullptr) {
   __shared__ uint32_t s_bits[SPION_MAX_NB * (SPION_MAX_NB / 32)];
   __shared__ int s_ptr[SPION_MAX_NB + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -70,6 +71,13 @@ static __device__ void build_structure(const uint8_t* mat, int nb, int32_t* nnzb
     if (lane == 0) s_ptr[c] = n;
   }
   __syncthreads();
+  if (longest_col && warp == 0) {
+    int most = 0;
+    for (int c = lane; c < nb; c += 32) most = max(most, s_ptr[c]);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) *longest_col = most;
+    __syncwarp();
+  }
   scan();
   for (int c = threadIdx.x; c <= nb; c += blockDim.x) col_ptr[c] = s_ptr[c];
   for (int c = warp; c < nb; c += nwarps) {

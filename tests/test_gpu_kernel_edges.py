@@ -152,6 +152,71 @@ def test_fp32_groups_per_row(bs, d, B, nb, per, forward, backward):
         assert any(f"{kernel}<{bs}, {d}, 4, {groups}>" in n for n in names), names
 
 
+# Calls on the fp32 tensor-core kernels: (bs, d, B, H, blocks per side), one and two 16-row tiles per warp, groups of matrices with some left
+# over, rows and columns of every length and none, full columns shared by a cluster, key padding; element CSR without O (two passes)
+@pytest.mark.parametrize("bs,d,B,H,nb", [(32, 32, 65, 1, 9), (32, 32, 151, 3, 8), (32, 64, 33, 3, 7), (64, 32, 25, 1, 8), (64, 64, 31, 1, 11), (64, 64, 61, 1, 5)])
+@pytest.mark.parametrize("layout", ["tiles", "csr"])
+@pytest.mark.parametrize("full_column", [False, True])
+def test_fp32_tensor_core_kernels(bs, d, B, H, nb, layout, full_column):
+    from spion_b200.attention import Attention
+    from spion_b200.attention_blockcuda import CUDABlockAttention
+    from spion_b200.native import BlockSparseAttention
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(37 + nb, B, H, L, d)
+    mat = lines_of_every_length(nb) if not full_column else synthetic.band_random_mask(3, nb, 0.0)
+    if full_column:
+        mat[:, [1, nb - 1]] = 1
+    if layout == "tiles":
+        kp = synthetic.key_padding(9, B, L) if nb % 2 else None
+        mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.float32, keypad=kp is not None)
+        compare(run(mod, Q, K, V, dO, mat, kp), Q, K, V, dO, mat, bs, kp, FP32_TOL, False)
+        return
+    cpp = Attention._blockcuda_compile_module()
+    handle = cpp.init(d, L, B * H, bs)
+    mod = CUDABlockAttention(cfg(B, H, L, d, bs), cpp, handle)
+    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+    out, _ = mod(q, k, v, torch.ones(B, L).cuda(), torch.as_tensor(mat.astype(np.float32)).cuda())
+    out.backward(dO.cuda())
+    compare((out, q.grad, k.grad, v.grad), Q, K, V, dO, mat, bs, None, FP32_TOL, False)
+    cpp.destroy(handle)
+
+
+@pytest.mark.parametrize("bs,d", [(32, 32), (64, 64)])
+def test_fp32_tensor_core_kernels_with_values_that_are_not_finite(bs, d):
+    """The parts of an infinity are NaN: rows that meet one are formed again.  A block-diagonal mask with a second block per row, so that what
+    a value can reach is known: key j of block c is seen by the rows of blocks c and c - 1."""
+    from spion_b200.native import BlockSparseAttention
+    B, nb = 80 if bs == 32 else 40, 16
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(41, B, 1, L, d)
+    mat = np.eye(nb, dtype=np.uint8) + np.roll(np.eye(nb, dtype=np.uint8), 1, axis=1)
+    V[0, 0, 3 * bs + 1, 2] = float("inf")             # column 2 of O in block rows 2 and 3
+    V[1, 0, 3 * bs + 1, 2] = 3.4e38                   # rounds to an infinity in bf16; finite results
+    K[2, 0, 5 * bs + 3] = -1e30                       # scores far below (P = 0) or far above all others (P = 1)
+    Q[3, 0, 7 * bs + 9, 0] = float("nan")             # one row
+    dO[4, 0, 9 * bs + 4, 5] = float("inf")            # dV[:, 5] of the keys of blocks 9 and 10; the row of dQ; dK of both blocks
+    mod = BlockSparseAttention(cfg(B, 1, L, d, bs), dtype=torch.float32)
+    got = [t.detach().cpu() for t in run(mod, Q, K, V, dO, mat, None)]
+    for b in range(6):
+        q, k, v = (t[b, 0].double().requires_grad_(True) for t in (Q, K, V))
+        rows = []
+        for r in range(nb):                           # the reference's softmax: unselected keys count as score 0
+            sel = torch.cat([torch.arange(c * bs, (c + 1) * bs) for c in np.flatnonzero(mat[r])])
+            s = q[r * bs:(r + 1) * bs] @ k[sel].T / d ** 0.5
+            m = s.detach().amax(-1, keepdim=True).clamp_min(-100.0)
+            e = torch.exp(s - m)
+            rows.append(e / (e.sum(-1, keepdim=True) + (L - len(sel)) * torch.exp(-m)) @ v[sel])
+        out = torch.cat(rows)
+        want = (out.detach(),) + torch.autograd.grad(out, (q, k, v), dO[b, 0].double())
+        for name, x, y in zip(("O", "dQ", "dK", "dV"), got, want):
+            x, y = x[b, 0].double(), y
+            if (b == 0 and name != "O") or (b == 1 and name in ("dQ", "dK")) or (b == 2 and name == "dQ"):
+                continue                              # inf - inf, or rounding multiplied by 1e30: the order of the steps decides
+            fin = y.abs() < 3e38
+            assert torch.equal(torch.isfinite(x), fin), (b, name, int((torch.isfinite(x) != fin).sum()))
+            assert float(((x - y).abs()[fin] / y.abs()[fin].clamp_min(1.0)).max()) <= FP32_TOL, (b, name)
+
+
 @pytest.mark.parametrize("L,d", [(64, 64), (192, 32), (512, 32), (576, 32), (1024, 64), (1088, 32), (1856, 32)])
 @pytest.mark.parametrize("padded", [False, True])
 def test_dense_fp32_kernels(L, d, padded):
