@@ -27,7 +27,8 @@
 // What bounds it: per pair at head_dim 64 the tensor pipe needs 920 (COL) or 660 cycles (ROW), the exponentials 512; a pair takes
 // about 1450.
 // Measured, ROW and COL, before (two groups of eight, a walk in every warp) and now: 64 matrices, L = 16384, d 64, 5 %: 637 and 639 us, now
-// 561 and 591; 256 matrices, L = 4096, d 32, 10 %, padded keys, two full columns: 425 and 394, now 341 and 306.  COL at head_dim 32: five
+// 561 and 591; 256 matrices, L = 4096, d 32, 10 %, padded keys, two full columns: 425 and 394, now 341 and 306.  Kernels of their own for
+// calls without key penalties, and blocks whose keys share one penalty taken with the row's constant: 529 and 571; 255 and 254.  COL at head_dim 32: five
 // slots and four sets of value tiles 306 us, seven and three 317.  Which mask is served by rebuilt and which by stored tiles:
 // _recompute_pays in native.py.
 //
@@ -70,26 +71,29 @@ struct BwArgs {
   int* status;
 };
 
-// Record of a pair: {flags, line of entry 0 | line of entry 1 << 16, line of the unit, (b,h) matrix}.  Flags: 1, 2: entry 0, 1 has padded
-// keys; the accumulator set << 4; the selected quarters of entry 0 << 8, of entry 1 << 16.
+// Record of a pair: {flags, line of entry 0 | line of entry 1 << 16, line of the unit, (b,h) matrix}.  Flags: 1, 2: the keys of entry 0, 1 have
+// different penalties; 1 << 24, 1 << 25: one that is not zero; the accumulator set << 4; the selected quarters of entry 0 << 8, of entry 1 << 16.
 constexpr int PF_LAST = 4, PF_TWO = 8, PF_FIRST = 64, PF_END = (int)0x80000000;
 
-// Are any of the penalties of 64 keys not zero?  Per lane.
-__device__ __forceinline__ bool pad64(const float* kp) {
-  bool v = false;
+// The penalties of 64 keys (see Pen4), per lane: PAD_NONE, PAD_ONE (the same for all) or PAD_MIXED.
+constexpr int PAD_NONE = 0, PAD_MIXED = 1, PAD_ONE = 1 << 24;
+__device__ __forceinline__ int pad64(const float* kp) {
+  const float first = kp[0];
+  bool other = !(first == first);
   if ((reinterpret_cast<uintptr_t>(kp) & 15) == 0) {
 #pragma unroll
     for (int x = 0; x < 16; ++x) {
       const float4 f = reinterpret_cast<const float4*>(kp)[x];
-      v |= f.x != 0.f || f.y != 0.f || f.z != 0.f || f.w != 0.f;
+      other |= f.x != first || f.y != first || f.z != first || f.w != first;
     }
   } else {
-    for (int x = 0; x < 64; ++x) v |= kp[x] != 0.f;
+    for (int x = 0; x < 64; ++x) other |= kp[x] != first;
   }
-  return v;
+  return other ? PAD_MIXED : first != 0.f ? PAD_ONE : PAD_NONE;
 }
 
-template <int D, int SIDE, bool SUB>
+// KP: with key penalties.
+template <int D, int SIDE, bool SUB, bool KP>
 __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                                                               const __grid_constant__ CUtensorMap tmF0, const __grid_constant__ CUtensorMap tmF1,
                                                               const __grid_constant__ BwArgs a) {
@@ -367,14 +371,13 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         const int4 pr = a.pair[first + k];
         const bool two = 2 * k + 1 < n_e, here = e == 0 || two;
         const int o = e ? pr.y : pr.x;
-        bool pad = false;
-        int sub = 0xff;
-        if (a.keypad && here) pad = pad64(a.keypad + (size_t)b * a.L + (SIDE == COL ? line : o) * BS);
+        int pad = PAD_NONE, sub = 0xff;
+        if (KP && here) pad = pad64(a.keypad + (size_t)b * a.L + (SIDE == COL ? line : o) * BS);
         if (SUB) sub = here ? a.submask[e ? pr.w : pr.z] : 0;
-        const int fl = (pad ? 1 : 0) | (sub << 8), fl1 = __shfl_down_sync(0xffffffffu, fl, 16);
+        const int fl = pad | (sub << 8), fl1 = __shfl_down_sync(0xffffffffu, fl, 16);
         const int ux = units + __popc(used & ((1u << x) - 1));
         if (active && e == 0)
-          half[lane] = make_int4(fl | (fl1 & 1) << 1 | (fl1 & 0xff00) << 8 | (k + 1 == np ? PF_LAST : 0) | (two ? PF_TWO : 0) |
+          half[lane] = make_int4(fl | (fl1 & (PAD_MIXED | PAD_ONE)) << 1 | (fl1 & 0xff00) << 8 | (k + 1 == np ? PF_LAST : 0) | (two ? PF_TWO : 0) |
                                      (k == 0 ? PF_FIRST : 0) | (ux % NACC) << 4,
                                  pr.x | (two ? pr.y << 16 : 0), line, b);
         filled += n;
@@ -479,6 +482,9 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
         const size_t ri = (size_t)rec.w * a.L + (SIDE == COL ? (es ? rec.y >> 16 : rec.y & 0xffff) : rec.z) * BS + row;
         h_next = a.lse[ri];
         d_next = SIDE == COL ? a.delta[ri] : __ldcg(a.delta_out + ri);            // ROW: written by this CTA
+        // one penalty for all keys goes with the log-sum-exp (here, where it waits for the load: a value of its own costs every pair 2 %)
+        if (KP && ((rec.x >> es) & PAD_ONE))
+          h_next = fmaf(a.keypad[(size_t)rec.w * a.L + (SIDE == COL ? rec.z : es ? rec.y >> 16 : rec.y & 0xffff) * BS], LOG2E, h_next);
       }
       return true;
     };
@@ -509,8 +515,8 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
           if (lane == 0) mbar_arrive(t_free + 8 * set);
         }
         if (mine) {
-          // blocks without padded keys (most of them) take no penalty; columns are keys in both
-          if ((flags >> es) & 1) take_penalty(sv, a.keypad + (size_t)bh * a.L + key * BS + g * 32, inv_scale);
+          // columns are keys in both
+          if (KP && ((flags >> es) & 1)) take_penalty(sv, a.keypad + (size_t)bh * a.L + key * BS + g * 32, inv_scale);
           const int sb = (SIDE == COL ? (q & 1) : (q >> 1)) * 2 + g;  // quarter: 2 (query / 32) + key / 32
           const bool live = !SUB || ((flags >> (8 + 8 * es + sb)) & 1);
           auto piece = [&](int cc) {             // eight columns: one 16-byte piece of each tile
@@ -586,12 +592,12 @@ __global__ void k_line_recs(const int32_t* __restrict__ ptr, const int32_t* __re
 
 namespace tc {
 
-template <int D, int SIDE, bool SUB>
-static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& f0, const CUtensorMap& f1,
+template <int D, int SIDE, bool SUB, bool KP>
+static int bw_launch_one(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& f0, const CUtensorMap& f1,
                      const BwArgs& a) {
   using C = Bw<D, SIDE>;
   static_assert(C::SMEM <= 227 * 1024, "shared memory");
-  auto k = k_bwd_stream<D, SIDE, SUB>;
+  auto k = k_bwd_stream<D, SIDE, SUB, KP>;
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
   k<<<grid, BW_THREADS, C::SMEM, c->stream>>>(a0, a1, f0, f1, a);
@@ -600,11 +606,18 @@ static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUte
   return SPION_OK;
 }
 
+template <int D, int SIDE>
+static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& f0, const CUtensorMap& f1,
+                     const BwArgs& a) {
+  if (a.submask) return a.keypad ? bw_launch_one<D, SIDE, true, true>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, true, false>(c, s, a0, a1, f0, f1, a);
+  return a.keypad ? bw_launch_one<D, SIDE, false, true>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, false, false>(c, s, a0, a1, f0, f1, a);
+}
+
 template <int D>
 static int bw_attrs() {
-  for (auto k : {k_bwd_stream<D, ROW, false>, k_bwd_stream<D, ROW, true>})
+  for (auto k : {k_bwd_stream<D, ROW, false, false>, k_bwd_stream<D, ROW, true, false>, k_bwd_stream<D, ROW, false, true>, k_bwd_stream<D, ROW, true, true>})
     SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, ROW>::SMEM));
-  for (auto k : {k_bwd_stream<D, COL, false>, k_bwd_stream<D, COL, true>})
+  for (auto k : {k_bwd_stream<D, COL, false, false>, k_bwd_stream<D, COL, true, false>, k_bwd_stream<D, COL, false, true>, k_bwd_stream<D, COL, true, true>})
     SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, COL>::SMEM));
   return SPION_OK;
 }
@@ -647,12 +660,12 @@ static int bwd_stream(spion_ctx* c, TcState* s, const void* Q, const void* K, co
   prof_mark(c, -1);
   a.rec = s->line_rec + SPION_MAX_NB; a.pair = s->line_pair + s->line_pair_cap;
   a.out0 = (__nv_bfloat16*)dQ; a.out1 = nullptr;
-  rc = a.submask ? bw_launch<D, ROW, true>(c, s, mk, mv, mq, mdo, a) : bw_launch<D, ROW, false>(c, s, mk, mv, mq, mdo, a);
+  rc = bw_launch<D, ROW>(c, s, mk, mv, mq, mdo, a);
   if (rc) return rc;
   prof_mark(c, SPION_STAGE_BWD_ROW_RC);
   a.rec = s->line_rec; a.pair = s->line_pair;
   a.out0 = (__nv_bfloat16*)dK; a.out1 = (__nv_bfloat16*)dV;
-  rc = a.submask ? bw_launch<D, COL, true>(c, s, mq, mdo, mk, mv, a) : bw_launch<D, COL, false>(c, s, mq, mdo, mk, mv, a);
+  rc = bw_launch<D, COL>(c, s, mq, mdo, mk, mv, a);
   if (rc) return rc;
   prof_mark(c, SPION_STAGE_BWD_COL_RC);
   return SPION_OK;

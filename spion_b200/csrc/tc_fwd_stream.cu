@@ -16,7 +16,7 @@
 //
 // What bounds it: the exponentials, 8192 per pair at 16 per cycle and SM = 512 cycles, and 16 MMAs of 33 cycles at head_dim 64.
 // Measured, forward alone, before (one unit per CTA, two passes over a row) and now: 64 matrices, L = 4096, d 64, 5 % 62 -> 44 us,
-// 30 % 314 -> 151; L = 16384, 5 % 847 -> 385; 256 matrices, L = 4096, d 32, 10 %, padded keys 585 -> 229.
+// 30 % 314 -> 151; L = 16384, 5 % 847 -> 385; 256 matrices, L = 4096, d 32, 10 %, padded keys 585 -> 229, 200 with one penalty per block (Pen4).
 //
 // Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
 #include "tc_stream.cuh"
@@ -37,7 +37,7 @@ template <int D> struct Fs {
   static constexpr uint32_t GROUP = O_K + (ALIAS ? 0 : 2 * T::BYTES);
   static constexpr uint32_t O_BAR = NG * GROUP;
   static constexpr uint32_t GBAR = 112;                           // barriers of a group
-  static constexpr size_t SMEM = O_BAR + NG * GBAR + 16 + NG * 32;
+  static constexpr size_t SMEM = O_BAR + NG * GBAR + 16 + NG * 64;
   static constexpr uint32_t COLS = 64 + D;                        // tensor-memory columns of a group: S, O
 };
 
@@ -82,7 +82,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
   const uint32_t slot = sbase + C::O_BAR + NG * C::GBAR, abort_w = slot + 4;
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
   volatile int* abort_ptr = reinterpret_cast<volatile int*>(smem_raw + (abort_w - sbase));
-  int* info = reinterpret_cast<int*>(smem_raw + (slot - sbase) + 16 + grp * 32);        // [2][4]: flags, block columns of the pair
+  // [2][8]: flags, block columns of the pair, -, penalties of its blocks in base-2 units
+  int* info = reinterpret_cast<int*>(smem_raw + (slot - sbase) + 16 + grp * 64);
 
   if (warp == 0 && lane == 0) {
     int ab = *reinterpret_cast<volatile int*>(a.status);
@@ -122,11 +123,11 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
     int4 pr = ld.valid() ? a.pair[ld.cur.y] : make_int4(0, -1, 0, 0);      // record of the pair whose K tiles are loaded next
     int4 prv = pr;                                                // ... whose V tiles are loaded next
     bool c_val = !EXACT, ld_val = !EXACT, p_val = false;          // pair of the value pass: c, ld, the pair before c
-    bool pad_l = false;
+    Pen4 pen_l = {};
     uint8_t sub_l = 0xff;
     auto flags_load = [&](const Walk& w, const int4& p) {         // requested with the pair's K tiles, used a pair later
       const int e = lane >> 4, o = e ? p.y : p.x;
-      if (KP) pad_l = o >= 0 && pad4(a.keypad + (size_t)w.bh * a.L + o * BS);
+      if (KP && o >= 0) pen_load(pen_l, a.keypad + (size_t)w.bh * a.L + o * BS);
       if (SUB) sub_l = o >= 0 ? a.submask[e ? p.w : p.z] : (uint8_t)0;
     };
     auto load_k = [&](int j) {                                    // K tiles of the pair at `ld` (pair j), Q with the first of a unit
@@ -172,12 +173,14 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       const bool have = c.valid();
       if (have) {
         if (KP || SUB) {                                          // flags of pair j: its buffer was read before P of pair j - 2 was written
-          const uint32_t any = KP ? __ballot_sync(0xffffffffu, pad_l) : 0u;
+          uint32_t mixed = 0u;
+          const float pen = KP ? pen_of(pen_l, mixed) * LOG2E : 0.f, pen1 = KP ? __shfl_sync(0xffffffffu, pen, 16) : 0.f;
           const int s1 = SUB ? __shfl_sync(0xffffffffu, (int)sub_l, 16) : 0xff;
           if (lane == 0) {
-            int* x = info + 4 * (j & 1);
-            x[0] = ((any & 0xffffu) ? 1 : 0) | ((any >> 16) ? 2 : 0) | ((SUB ? (int)sub_l : 0xff) << 8) | (s1 << 16);
+            int* x = info + 8 * (j & 1);
+            x[0] = (int)mixed | ((SUB ? (int)sub_l : 0xff) << 8) | (s1 << 16);
             x[1] = prv.x; x[2] = prv.y;
+            if (KP) { x[4] = __float_as_int(pen); x[5] = __float_as_int(pen1); }
             mbar_arrive(pi_full + 8 * (j & 1));
           }
           __syncwarp();
@@ -310,13 +313,17 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         const int k = values ? kx : kx + np;
         const bool mine = 2 * k + hf < n;
         const float* kp = nullptr;
+        float pen = 0.f;
         bool live0 = mine, live1 = mine;
         if (KP || SUB) {
           if (!wait_all(pi_full + 8 * (j & 1), (uint32_t)(j >> 1), ERR_MMA_WAIT)) { ok = false; break; }
-          const int* x = info + 4 * (j & 1);
+          const int* x = info + 8 * (j & 1);
           const int f = x[0];
-          // blocks without padded keys (most of them) take no penalty
-          if (KP && ((f >> hf) & 1)) kp = kpu + x[1 + hf] * BS;
+          if (KP) {
+            const bool mixed = (f >> hf) & 1;
+            pen = mixed ? 0.f : __int_as_float(x[4 + hf]);
+            if (mixed) kp = kpu + x[1 + hf] * BS;
+          }
           if (SUB) {
             const int bits = (f >> (8 + 8 * hf + (q >> 1) * 2)) & 3;
             live0 = mine && (bits & 1);
@@ -348,8 +355,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
             m2 = max3(m2, __uint_as_float(v1[x]), __uint_as_float(v1[x + 1]));
             m3 = max3(m3, __uint_as_float(v1[x + 2]), __uint_as_float(v1[x + 3]));
           }
-          if (live0) cm = fmaxf(m0, m1) * sc2;
-          if (live1) cm = fmaxf(cm, fmaxf(m2, m3) * sc2);
+          if (live0) cm = fmaf(fmaxf(m0, m1), sc2, -pen);
+          if (live1) cm = fmaxf(cm, fmaf(fmaxf(m2, m3), sc2, -pen));
         }
         cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 16));     // both owners of a row agree
         mx = fmaxf(mx, cm);
@@ -378,7 +385,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         if (j >= 2 && !wait_all(pv_done + 8 * (j & 1), (uint32_t)(j >> 1) - 1u, ERR_MMA2_WAIT)) { ok = false; break; }
         const uint32_t tile = gb + C::O_P + (j & 1) * C::PB + hf * VT_BYTES + row * 128;
         uint64_t l2 = 0ull;
-        const uint64_t sc22 = pack2(sc2, sc2), nm2 = pack2(-m, -m);
+        const uint64_t sc22 = pack2(sc2, sc2), nm2 = pack2(-(m + pen), -(m + pen));
         auto half_row = [&](const uint32_t (&v)[32], int g, bool live) {
           float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll

@@ -86,19 +86,30 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint32_t (&w)[
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
 }
 
-// Raw scores of 32 keys with their penalties: (s - pad / scale) scale = s scale - pad.  Done in place, in the few blocks that have
-// padded keys, so that the arithmetic behind it has one form only (two forms cost 20 % of the forward in registers).
+// Raw scores of 32 keys with their penalties: (s - pad / scale) scale = s scale - pad.  Done in place, in the few blocks whose keys
+// have different ones, so that the arithmetic behind it has one form only (two forms cost 20 % of the forward in registers).
 __device__ __forceinline__ void take_penalty(uint32_t (&s)[32], const float* kp, float inv_scale) {
 #pragma unroll
   for (int x = 0; x < 32; ++x) s[x] = __float_as_uint(fmaf(kp[x], -inv_scale, __uint_as_float(s[x])));
 }
 
-// Padded keys in a block (the penalties of its 64 keys)?  Half a warp, four keys per lane; the result is this lane's own four.
-__device__ __forceinline__ bool pad4(const float* kp) {
-  bool v = false;
+// The penalties of a block's 64 keys: one value for all of them (zero: no padded keys), or different ones.  Padding is a tail of the
+// sequence, so a block in which they differ is one per sequence; all others take the value with the row's constant, not key by key (256 matrices,
+// L = 4096, d 32, 10 %, 25 % of the keys padded: forward, columns, rows 224, 335, 298 us with a penalty per key of every padded block).
+// Half a warp, four keys per lane: pen_load is requested early, pen_of gives the block's value and whether a key differs from it.
+struct Pen4 { float x[4]; };
+__device__ __forceinline__ void pen_load(Pen4& p, const float* kp) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) v |= kp[(threadIdx.x & 15) + 16 * i] != 0.f;
-  return v;
+  for (int i = 0; i < 4; ++i) p.x[i] = kp[(threadIdx.x & 15) + 16 * i];
+}
+__device__ __forceinline__ float pen_of(const Pen4& p, uint32_t& mixed) {      // whole warp; mixed: bit 0, lanes 0-15, bit 1, lanes 16-31
+  const float first = __shfl_sync(0xffffffffu, p.x[0], threadIdx.x & 16);
+  bool other = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) other |= p.x[i] != first;           // a NaN differs from itself
+  const uint32_t all = __ballot_sync(0xffffffffu, other);
+  mixed = ((all & 0xffffu) ? 1u : 0u) | ((all >> 16) ? 2u : 0u);
+  return first;
 }
 
 }  // namespace tc

@@ -293,3 +293,29 @@ def test_streaming_forward_with_rows_without_blocks_between_others(d, H, full_ma
         e = torch.exp(q[b].float() @ k[b].float().transpose(1, 2) / d ** 0.5) * sel
         want = (e / (e.sum(-1, keepdim=True) + others)) @ v[b].float()
         assert far(out[b], want, True) <= BF16_REL, (b, far(out[b], want, True))
+
+
+@pytest.mark.parametrize("d,bs", [(64, 64), (32, 64), (32, 32)])
+@pytest.mark.parametrize("full", [False, True])
+def test_streaming_kernels_with_penalties_of_every_kind(d, bs, full):
+    """Blocks whose keys have no penalty, one penalty (small, large, negative), different ones, and a sequence of padded keys only: P is
+    exp2 of scores less the penalties, so the reference takes them as an additive mask of its own."""
+    from spion_b200.native import BlockSparseAttention
+    B, H, nb = 3, 2, 10 if bs == 64 else 20
+    L = nb * bs
+    Q, K, V, dO = (t.to(torch.bfloat16) for t in synthetic.qkv(43 + d, B, H, L, d))
+    mat = np.ones((nb, nb), np.uint8) if full else lines_of_every_length(nb)
+    keep = torch.ones(B, L)                                  # penalty 1e6 (1 - keep)
+    keep[0, 64:128] = 1 - 1.5e-6                             # one small penalty for a block
+    keep[0, 128:192] = 1 + 2e-6                              # a bonus
+    keep[0, 192:256] = 1 - 1e-6 * torch.arange(64) / 32      # a different one for every key
+    keep[1, L - 100:] = 0                                    # a padded tail that begins inside a block
+    keep[2, 0 if not full else 1:] = 0                       # nothing but padding (full mask: one key, or no score counts at all)
+    mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.bfloat16, keypad=True, recompute=True, return_probs=False)
+    got = run(mod, Q, K, V, dO, mat, keep)
+    O, _, gQ, gK, gV = oatt.sparse_attention(Q.float(), K.float(), V.float(), mat, bs, keep, dO.float(), dtype=torch.float64)
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), got, (O, gQ, gK, gV)):
+        assert torch.isfinite(a).all()
+        assert far(a[:2], b[:2], True) <= BF16_REL, f"{name}: {far(a[:2], b[:2], True):.3e}"
+    if not full:                                             # unselected keys count as score 0 and leave nothing to the padded ones
+        assert not got[0][2].any() and not got[3][2].any()
