@@ -11,7 +11,8 @@
 //     S, dP    COL: [Q0; Q1] K^T and [dO0; dO1] V^T as one 128-row product each; ROW: Q K_e^T and dO V_e^T, the second entry at
 //              lane offset 16: query rows along the lanes in both, so that lse and delta are one register each
 //     accumulators += dS^T Q, P^T dO (COL),  += dS K (ROW)
-// One persistent CTA per SM, 640 threads:
+// One persistent CTA per SM, 640 threads.  Warps 0 to 2 are one thread each: as whole warps they took 300 cycles a pair for records, waits and
+// votes around 450 to 650 cycles of issue, and S / dP (rows) and the second products (columns) were what a pair waited for.
 //   warp 0   loads: the tiles of a pair into a ring of slots, the fixed tiles of a unit into one of two sets (TMA)
 //   warp 1   S / dP products into one of three tensor-memory sets
 //   warp 2   second products, when the tiles of a pair are written
@@ -28,11 +29,14 @@
 // about 1450.
 // Measured, ROW and COL, before (two groups of eight, a walk in every warp) and now: 64 matrices, L = 16384, d 64, 5 %: 637 and 639 us, now
 // 561 and 591; 256 matrices, L = 4096, d 32, 10 %, padded keys, two full columns: 425 and 394, now 341 and 306.  Kernels of their own for
-// calls without key penalties, and blocks whose keys share one penalty taken with the row's constant: 529 and 571; 255 and 254.  COL at head_dim 32: five
+// calls without key penalties, and blocks whose keys share one penalty taken with the row's constant: 529 and 571; 255 and 254.
+// One thread for loads and MMAs: head_dim 32, L = 16384, 5 %: 417 and 428, now 369 and 399; the padded case 244 and 243.  COL at head_dim 32: five
 // slots and four sets of value tiles 306 us, seven and three 317.  Which mask is served by rebuilt and which by stored tiles:
 // _recompute_pays in native.py.
 //
 // Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
+#include <type_traits>
+
 #include "tc_stream.cuh"
 
 using namespace tc;
@@ -175,26 +179,36 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
     return true;
   };
 
+  // One thread of a warp does all that the loads and the products need: nothing there is worth the other lanes.
+  auto wait_one = [&](uint32_t bar, uint32_t parity, int code) -> bool {
+    if (mbar_wait(bar, parity & 1u)) return true;
+    report(a.status, code);
+    return false;
+  };
+  auto record_one = [&](uint32_t j, int4& r) -> bool {
+    if ((j & 15) == 0 && !wait_one(r_full + 8 * ((j >> 4) & 1), j >> 5, ERR_LOAD_WAIT)) return false;
+    r = ring[j & 31];
+    if ((j & 15) == 15) mbar_arrive(r_free + 8 * ((j >> 4) & 1));
+    return true;
+  };
   if (warp == 0) {
     // ================================================================== loads
-    int u = 0, ps = 0, round = 0;
-    int4 next;
-    bool ok = record(0, 1, next);
-    for (uint32_t j = 0; ok && next.x >= 0; ++j) {
-      const int4 r = next;
-      if (round >= 1 && !wait_all(pdone + 8 * ps, (uint32_t)(round - 1), ERR_MMA2_WAIT)) break;
-      const bool first = __any_sync(0xffffffffu, r.x & PF_FIRST), two = __any_sync(0xffffffffu, r.x & PF_TWO);
-      const int fs = u & 1;
-      if (first && u >= 2 && !wait_all(f_free + 8 * fs, (uint32_t)((u >> 1) - 1), ERR_MMA2_WAIT)) break;
-      const OpPos pos = op_pos(r.w, a.L, a.heads, D);
-      const uint32_t dst = sbase + ps * C::SLOT;
-      if (elect_one()) {
+    if (elect_one()) {
+      int u = 0, ps = 0, round = 0;
+      int4 r;
+      for (uint32_t j = 0; record_one(j, r) && r.x >= 0; ++j) {
+        const bool first = r.x & PF_FIRST, two = r.x & PF_TWO;
+        const int fs = u & 1;
+        const OpPos pos = op_pos(r.w, a.L, a.heads, D);
+        const uint32_t dst = sbase + ps * C::SLOT;
         if (first) {
+          if (u >= 2 && !wait_one(f_free + 8 * fs, (uint32_t)((u >> 1) - 1), ERR_MMA2_WAIT)) break;
           const uint32_t f = sbase + C::O_FIX + fs * C::FIX;
           mbar_expect_tx(f_full + 8 * fs, 2 * T::BYTES);
           tma_load_2d(f, &tmF0, f_full + 8 * fs, pos.x0, pos.row0 + r.z * BS);
           tma_load_2d(f + T::BYTES, &tmF1, f_full + 8 * fs, pos.x0, pos.row0 + r.z * BS);
         }
+        if (round >= 1 && !wait_one(pdone + 8 * ps, (uint32_t)(round - 1), ERR_MMA2_WAIT)) break;
         mbar_expect_tx(pfull + 8 * ps, (two ? 4 : 2) * T::BYTES);
         const int y0 = pos.row0 + (r.y & 0xffff) * BS, y1 = pos.row0 + (r.y >> 16) * BS;
         tma_load_2d(dst, &tmA0, pfull + 8 * ps, pos.x0, y0);
@@ -203,27 +217,23 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
           tma_load_2d(dst + T::BYTES, &tmA0, pfull + 8 * ps, pos.x0, y1);
           tma_load_2d(dst + 3 * T::BYTES, &tmA1, pfull + 8 * ps, pos.x0, y1);
         }
+        if (r.x & PF_LAST) ++u;
+        if (++ps == NP) { ps = 0; ++round; }
       }
-      __syncwarp();
-      ok = record(j + 1, 1, next);
-      if (r.x & PF_LAST) ++u;
-      if (++ps == NP) { ps = 0; ++round; }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ================================================================== S and dP
-    constexpr uint32_t IDESC = make_idesc_bf16(SIDE == COL ? 128 : 64, 64, 0, 0);
-    const uint64_t KM = T::kmajor(sbase, 0);
-    int u = 0, ps = 0, round = 0, set = 0, sround = 0, sr = 0;
-    int4 next;
-    bool ok = record(0, 1, next);
-    for (uint32_t j = 0; ok && next.x >= 0; ++j) {
-      const int4 r = next;
-      const int par = u & 1;
-      if (sround >= 1 && !wait_all(t_free + 8 * set, (uint32_t)(sround - 1), ERR_MMA_WAIT)) break;
-      if ((r.x & PF_FIRST) && !wait_all(f_full + 8 * par, (uint32_t)(u >> 1), ERR_LOAD_WAIT)) break;
-      if (!wait_all(pfull + 8 * ps, (uint32_t)round, ERR_LOAD_WAIT)) break;
-      const bool last = __any_sync(0xffffffffu, r.x & PF_LAST), two = __any_sync(0xffffffffu, r.x & PF_TWO);
-      if (elect_one()) {
+    if (elect_one()) {
+      constexpr uint32_t IDESC = make_idesc_bf16(SIDE == COL ? 128 : 64, 64, 0, 0);
+      const uint64_t KM = T::kmajor(sbase, 0);
+      int u = 0, ps = 0, round = 0, set = 0, sround = 0, sr = 0;
+      int4 r;
+      for (uint32_t j = 0; record_one(j, r) && r.x >= 0; ++j) {
+        const int par = u & 1;
+        if ((r.x & PF_FIRST) && !wait_one(f_full + 8 * par, (uint32_t)(u >> 1), ERR_LOAD_WAIT)) break;
+        if (!wait_one(pfull + 8 * ps, (uint32_t)round, ERR_LOAD_WAIT)) break;
+        if (sround >= 1 && !wait_one(t_free + 8 * set, (uint32_t)(sround - 1), ERR_MMA_WAIT)) break;
         tc_fence_after();
         const uint64_t a0 = desc_advance(KM, ps * C::SLOT), a1 = desc_advance(a0, 2 * T::BYTES);
         const uint64_t f0 = desc_advance(KM, C::O_FIX + par * C::FIX), f1 = desc_advance(f0, T::BYTES);
@@ -244,62 +254,61 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
               mma_bf16(de + 64u, desc_advance(f1, kk * T::K_STEP), desc_advance(a1, e * T::BYTES + kk * T::K_STEP), IDESC, kk > 0);
           };
           products(0);
-          if (two) products(1);
+          if (r.x & PF_TWO) products(1);
         }
         mma_commit(s_ready + 8 * sr);
-        if (last) mma_commit(f_free + 8 * par);                       // the fixed tiles are read by these products only
+        if (r.x & PF_LAST) {                                          // the fixed tiles are read by these products only
+          mma_commit(f_free + 8 * par);
+          ++u;
+        }
+        if (++ps == NP) { ps = 0; ++round; }
+        if (++set == 3) { set = 0; ++sround; }
+        if (++sr == C::NS) sr = 0;
       }
-      __syncwarp();
-      ok = record(j + 1, 1, next);
-      if (++ps == NP) { ps = 0; ++round; }
-      if (++set == 3) { set = 0; ++sround; }
-      if (++sr == C::NS) sr = 0;
-      if (last) ++u;
     }
+    __syncwarp();
   } else if (warp == 2) {
     // ================================================================== second products
-    constexpr uint32_t IDESC = make_idesc_bf16(64, D, SIDE == COL ? 1 : 0, 1);
-    constexpr uint32_t V_STEP = SIDE == COL ? ValTile::MN_STEP : ValTile::K_STEP;
-    const uint64_t MN = T::mnmajor(sbase, 0), VT = SIDE == COL ? ValTile::mnmajor(sbase, 0) : ValTile::kmajor(sbase, 0);
-    int u = 0, ps = 0, round = 0, grp = 0, pd = 0;
-    uint32_t odd = 0;                                                 // bit g: group g has written an odd number of units
-    int4 next;
-    bool ok = record(0, 1, next);
-    for (uint32_t j = 0; ok && next.x >= 0; ++j) {
-      const int4 r = next;
-      const int x = u % NACC;
-      if ((r.x & PF_FIRST) && u >= NACC && !wait_all(acc_free + 8 * x, (uint32_t)(u / NACC - 1), ERR_MMA2_WAIT)) break;
-      if (!wait_all(p_ready + 8 * ps, (uint32_t)round, ERR_MMA_WAIT)) break;
-      const bool last = __any_sync(0xffffffffu, r.x & PF_LAST), two = __any_sync(0xffffffffu, r.x & PF_TWO), fresh = __any_sync(0xffffffffu, r.x & PF_FIRST);
-      if (elect_one()) {
+    if (elect_one()) {
+      constexpr uint32_t IDESC = make_idesc_bf16(64, D, SIDE == COL ? 1 : 0, 1);
+      constexpr uint32_t V_STEP = SIDE == COL ? ValTile::MN_STEP : ValTile::K_STEP;
+      const uint64_t MN = T::mnmajor(sbase, 0), VT = SIDE == COL ? ValTile::mnmajor(sbase, 0) : ValTile::kmajor(sbase, 0);
+      int u = 0, ps = 0, round = 0, grp = 0, pd = 0;
+      uint32_t odd = 0;                                               // bit g: group g has written an odd number of units
+      int4 r;
+      for (uint32_t j = 0; record_one(j, r) && r.x >= 0; ++j) {
+        const int x = u % NACC;
+        if ((r.x & PF_FIRST) && u >= NACC && !wait_one(acc_free + 8 * x, (uint32_t)(u / NACC - 1), ERR_MMA2_WAIT)) break;
+        if (!wait_one(p_ready + 8 * ps, (uint32_t)round, ERR_MMA_WAIT)) break;
         tc_fence_after();
-        const uint32_t acc = tmem + acc_at(x);
+        const uint32_t acc = tmem + acc_at(x), more = (r.x & PF_FIRST) ? 0u : 1u;
         const uint64_t b0 = desc_advance(MN, ps * C::SLOT);
         const uint64_t vt = desc_advance(VT, SIDE == COL ? C::O_PD + pd * C::PD : ps * C::SLOT + 2 * T::BYTES);
-        auto products = [&](int e, bool first) {
+        auto products = [&](int e, uint32_t first) {
 #pragma unroll
           for (int kk = 0; kk < BS / 16; ++kk)                        // dK or dQ
-            mma_bf16(acc, desc_advance(vt, e * VT_BYTES + kk * V_STEP), desc_advance(b0, e * T::BYTES + kk * T::MN_STEP), IDESC,
-                     (kk > 0) ? 1u : (first ? 0u : 1u));
+            mma_bf16(acc, desc_advance(vt, e * VT_BYTES + kk * V_STEP), desc_advance(b0, e * T::BYTES + kk * T::MN_STEP), IDESC, kk > 0 ? 1u : first);
           if (SIDE == COL) {
 #pragma unroll
             for (int kk = 0; kk < BS / 16; ++kk)                      // dV (lanes 16-31)
               mma_bf16(acc + (16u << 16), desc_advance(vt, (2 + e) * VT_BYTES + kk * V_STEP),
-                       desc_advance(b0, (2 + e) * T::BYTES + kk * T::MN_STEP), IDESC, (kk > 0) ? 1u : (first ? 0u : 1u));
+                       desc_advance(b0, (2 + e) * T::BYTES + kk * T::MN_STEP), IDESC, kk > 0 ? 1u : first);
           }
         };
-        products(0, fresh);
-        if (two) products(1, false);
+        products(0, more);
+        if (r.x & PF_TWO) products(1, 1u);
         mma_commit(pdone + 8 * ps);
-        if (last) mma_commit(acc_done + 8 * (2 * grp + ((odd >> grp) & 1)));
+        if (r.x & PF_LAST) {
+          mma_commit(acc_done + 8 * (2 * grp + ((odd >> grp) & 1)));
+          ++u;
+          odd ^= 1u << grp;
+        }
+        if (++ps == NP) { ps = 0; ++round; }
+        if (++grp == NGR) grp = 0;
+        if (SIDE == COL && ++pd == C::NPD) pd = 0;
       }
-      __syncwarp();
-      ok = record(j + 1, 1, next);
-      if (++ps == NP) { ps = 0; ++round; }
-      if (last) { ++u; odd ^= 1u << grp; }
-      if (++grp == NGR) grp = 0;
-      if (SIDE == COL && ++pd == C::NPD) pd = 0;
     }
+    __syncwarp();
   } else if (warp == 3) {
     // ================================================================== the walk: records of the CTA's pairs, 16 at a time
     // 32 units at a time, one per lane; lanes t and t + 16 look at entries 0 and 1 of pair t of a half.
@@ -502,44 +511,50 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
       const uint32_t ts = t_lane + set * 128u;
       const uint32_t tds = sbase + (SIDE == COL ? C::O_PD + (j % (SIDE == COL ? C::NPD : 1)) * C::PD : ps * C::SLOT + 2 * T::BYTES) + es * VT_BYTES + row * 128;
       const uint64_t sc22 = pack2(sc2, sc2), scale2 = pack2(a.scale, a.scale), nds2 = pack2(nds, nds), nh2 = pack2(-h, -h);
+      auto tiles = [&](auto mixed) {
+        constexpr bool MIXED = decltype(mixed)::value;
 #pragma unroll
-      for (int hf = 0; hf < C::HALVES; ++hf) {
-        const int g = C::HALVES == 2 ? hf : g0;                       // 32 columns (keys)
-        uint32_t sv[32], gv[32];
-        tmem_ld32(ts + g * 32, sv);
-        tmem_ld32(ts + 64u + g * 32, gv);
-        tmem_ld_wait();
-        if (hf + 1 == C::HALVES) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(t_free + 8 * set);
+        for (int hf = 0; hf < C::HALVES; ++hf) {
+          const int g = C::HALVES == 2 ? hf : g0;                       // 32 columns (keys)
+          uint32_t sv[32], gv[32];
+          tmem_ld32(ts + g * 32, sv);
+          tmem_ld32(ts + 64u + g * 32, gv);
+          tmem_ld_wait();
+          if (hf + 1 == C::HALVES) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(t_free + 8 * set);
+          }
+          if (mine) {
+            // columns are keys in both
+            if (MIXED && ((flags >> es) & 1)) take_penalty(sv, a.keypad + (size_t)bh * a.L + key * BS + g * 32, inv_scale);
+            const int sb = (SIDE == COL ? (q & 1) : (q >> 1)) * 2 + g;  // quarter: 2 (query / 32) + key / 32
+            const bool live = !SUB || ((flags >> (8 + 8 * es + sb)) & 1);
+            auto piece = [&](int cc) {             // eight columns: one 16-byte piece of each tile
+              uint32_t wp[4], wd[4];
+#pragma unroll
+              for (int x = 0; x < 4; ++x) {
+                const int c = cc * 8 + 2 * x;
+                float p0, p1, d0, d1;
+                unpack2(fma2(pack2(sv[c], sv[c + 1]), sc22, nh2), p0, p1);
+                p0 = ex2_approx(p0); p1 = ex2_approx(p1);
+                wp[x] = pack_bf16(p0, p1);
+                unpack2(mul2(pack2(p0, p1), fma2(pack2(gv[c], gv[c + 1]), scale2, nds2)), d0, d1);
+                wd[x] = pack_bf16(d0, d1);
+                if (SUB && !live) { wp[x] = 0u; wd[x] = 0u; }
+              }
+              const uint32_t off = (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4);
+              st_shared_v4(tds + off, wd);
+              if (SIDE == COL) st_shared_v4(tds + 2 * VT_BYTES + off, wp);
+            };
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) piece(cc);
+          }
         }
-        if (mine) {
-          // columns are keys in both
-          if (KP && ((flags >> es) & 1)) take_penalty(sv, a.keypad + (size_t)bh * a.L + key * BS + g * 32, inv_scale);
-          const int sb = (SIDE == COL ? (q & 1) : (q >> 1)) * 2 + g;  // quarter: 2 (query / 32) + key / 32
-          const bool live = !SUB || ((flags >> (8 + 8 * es + sb)) & 1);
-          auto piece = [&](int cc) {             // eight columns: one 16-byte piece of each tile
-            uint32_t wp[4], wd[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-              const int c = cc * 8 + 2 * x;
-              float p0, p1, d0, d1;
-              unpack2(fma2(pack2(sv[c], sv[c + 1]), sc22, nh2), p0, p1);
-              p0 = ex2_approx(p0); p1 = ex2_approx(p1);
-              wp[x] = pack_bf16(p0, p1);
-              unpack2(mul2(pack2(p0, p1), fma2(pack2(gv[c], gv[c + 1]), scale2, nds2)), d0, d1);
-              wd[x] = pack_bf16(d0, d1);
-              if (SUB && !live) { wp[x] = 0u; wd[x] = 0u; }
-            }
-            const uint32_t off = (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4);
-            st_shared_v4(tds + off, wd);
-            if (SIDE == COL) st_shared_v4(tds + 2 * VT_BYTES + off, wp);
-          };
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) piece(cc);
-        }
-      }
+      };
+      // a form of its own for pairs with a block whose keys have different penalties: as a branch in the other it costs every pair 8 %
+      if (KP && __any_sync(0xffffffffu, (flags & 3) != 0)) tiles(std::true_type{});
+      else tiles(std::false_type{});
       fence_proxy_async();                                            // tiles -> visible to the MMAs
       __syncwarp();
       if (lane == 0) mbar_arrive(p_ready + 8 * ps);
