@@ -764,6 +764,7 @@ static int kernel_attrs(spion_ctx* c, TcState* s) {
     if (!rc) rc = mean_map_set_attrs(c->d);
     if (!rc) rc = pipe_set_attrs(s, c->d, c->device);
     if (!rc) rc = stream_forward_set_attrs(c->d);
+    if (!rc) rc = exact_forward_set_attrs(c->d);
     if (!rc) rc = stream_backward_set_attrs(c->d);
     if (!rc && b32) rc = b32_set_attrs(s, c->device);
     if (rc) return rc;

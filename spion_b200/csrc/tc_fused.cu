@@ -590,11 +590,12 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
   // (tc_fwd_pipe.cu: about 1.7x less time per row, two CTAs per SM).  As soon as some rows are longer,
   // everything goes through one kernel: a second launch for a handful of long rows costs more
   // than the pipelining gains (measured at 5 % density, L = 4096: 79 us split against 70 us in one launch).  Without P that is the
-  // streaming kernel (tc_fwd_stream.cu), with P this file's, whose probabilities are rounded after the normalisation.
+  // streaming kernel (tc_fwd_stream.cu; the full mask: tc_fwd_exact.cu), with P this file's, whose probabilities are rounded after the normalisation.
   if (s->n_long == 0) {
     if ((rc = pipe_forward(c, s, mq, mk, mv, mp, P64 != nullptr, keypad, O, lse, 0))) return rc;
   } else if (!P64) {
-    if ((rc = stream_forward(c, s, mq, mk, mv, keypad, O, lse))) return rc;
+    rc = c->nnzb == c->nb * c->nb ? exact_forward(c, s, mq, mk, mv, keypad, O, lse) : stream_forward(c, s, mq, mk, mv, keypad, O, lse);
+    if (rc) return rc;
   } else {
     const long long total = (long long)c->BH * vw.nb, cap = (long long)s->sms * s->fwd_ctas;
     const float floor_v = keypad ? 0.0f : -100.0f;

@@ -1,22 +1,25 @@
 // Forward of the block-sparse attention as a streaming pipeline (sm_100a, bf16, 64 x 64 blocks, no stored P): O and one fp32
 // log-sum-exp per row (models/block_attn.cu:453-487 fused; softmax semantics as in tc_fused.cu).
 //
-// One persistent CTA per SM with four groups.  A group has one service warp (TMA loads, MMA issue) and four arithmetic warps (one per
-// tensor-memory quadrant) and walks block rows of its own, two blocks ("a pair") at a time:
+// One persistent CTA per SM with four groups (three at head_dim 64: tensor memory).  A group has four arithmetic warps (one per tensor-memory
+// quadrant), a warp that issues its MMAs and one that loads its tiles, and walks block rows of its own, two blocks ("a pair") at a time:
 //     S = Q K_e^T   (M = 64, the second block at lane offset 16: query rows along the lanes, a row owned by lanes l and l + 16)
-//     P = exp2(S scale log2e - m), unnormalised, bf16 into shared memory (over the K tiles when they are as large)
-//     O += P V_e    (M = 64, tensor memory, lane offset 16 x parity of the row among the rows with blocks)
+//     P = exp2(S scale log2e - m), unnormalised, bf16 into tensor memory, in the lanes of S
+//     O += P V_e    (M = 64, P from tensor memory: the products of first and of second blocks in lanes of their own, added when the rows are written)
 // S of pair j + 1 is computed while pair j is in the arithmetic (its 64 values per lane are in registers), and the rows of a
-// finished unit are written after the first pair of the next one.  Nothing is exchanged between the groups: they only fill each
+// finished unit are written before the first product of the next one.  Nothing is exchanged between the groups: they only fill each
 // other's waits.
 //
 // One pass over a row: m is the maximum of its first pair and is only moved (O and the running sum rescaled) when a later
 // score exceeds it by more than 2^8 (the conditional rescaling published with FlashAttention-4), so that almost no row is ever
 // rescaled; the result is divided by the sum against the true maximum at the end.  P <= 2^8 loses nothing in bf16 or in the fp32 sums.
 //
-// What bounds it: the exponentials, 8192 per pair at 16 per cycle and SM = 512 cycles, and 16 MMAs of 33 cycles at head_dim 64.
-// Measured, forward alone, before (one unit per CTA, two passes over a row) and now: 64 matrices, L = 4096, d 64, 5 % 62 -> 44 us,
-// 30 % 314 -> 151; L = 16384, 5 % 847 -> 385; 256 matrices, L = 4096, d 32, 10 %, padded keys 585 -> 229, 200 with one penalty per block (Pen4).
+// What bounds it: per pair the exponentials, 8192 at 16 per cycle and SM = 512 cycles, and at head_dim 64 sixteen MMAs of 32 cycles (M = 64 runs
+// at half rate) and 640 cycles of shared memory at 128 bytes (tiles in 256, operands out 384; with P there too, as before, 912 of the 950
+// that a pair took).  What it takes beside those, 890 (head_dim 64) and 750, is the chain of a pair: one warp that did the loads and
+// the MMAs of a group took as long for them as a pair does, so they are two, and the MMAs are issued by one thread that does nothing else.
+// Measured, forward alone, first form (one unit per CTA, two passes over a row), P in shared memory, now: 64 matrices, L = 16384, d 64, 5 % 847,
+// 368, 345 us, d 32 -, 312, 292; 256 matrices, L = 4096, d 32, 10 %, padded keys 585, 200, 185; 64 matrices, L = 4096, d 64, 5 % 62, 43.5, 43.
 //
 // Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
 #include "tc_stream.cuh"
@@ -25,31 +28,26 @@ using namespace tc;
 
 namespace {
 
-constexpr int NG = 4;                                             // groups
-constexpr int FS_THREADS = 32 * (4 + 4 * NG);
 constexpr float MOVE = 8.0f;                                      // log2 units by which a score may exceed m
 
 template <int D> struct Fs {
   using T = OpTile<D>;
-  static constexpr bool ALIAS = D == 64;                          // P tiles over the K tiles
-  static constexpr uint32_t PB = 2 * VT_BYTES;                    // P tiles of a pair (ALIAS: K tiles first), two buffers
-  static constexpr uint32_t O_Q = 0, O_P = T::BYTES, O_V = O_P + 2 * PB, O_K = O_V + 2 * T::BYTES;
-  static constexpr uint32_t GROUP = O_K + (ALIAS ? 0 : 2 * T::BYTES);
+  static constexpr int NG = D == 64 ? 3 : 4;                      // groups: as many as tensor memory holds
+  // Warps: four arithmetic ones per group, then one per group that issues its MMAs, one per group that loads its tiles, and idle ones up to two
+  // whole warpgroups, so that the arithmetic warps can take registers of the others (setmaxnreg).
+  static constexpr int THREADS = 32 * (4 * NG + 8);
+  static constexpr int REGS = NG == 4 ? 80 : 96, REGS_A = NG == 4 ? 96 : 120, REGS_S = NG == 4 ? 48 : 56;         // at launch, arithmetic, others
+  static_assert(4 * NG * REGS_A + 8 * REGS_S <= (4 * NG + 8) * REGS, "setmaxnreg would wait for ever");
+  static constexpr int KB = D == 64 ? 1 : 2;                      // buffers for the K tiles of a pair
+  static constexpr uint32_t O_Q = 0, O_K = 2 * T::BYTES, O_V = O_K + 2 * KB * T::BYTES, GROUP = O_V + 4 * T::BYTES;      // Q of two units, V of two pairs
   static constexpr uint32_t O_BAR = NG * GROUP;
-  static constexpr uint32_t GBAR = 112;                           // barriers of a group
-  static constexpr size_t SMEM = O_BAR + NG * GBAR + 16 + NG * 64;
-  static constexpr uint32_t COLS = 64 + D;                        // tensor-memory columns of a group: S, O
+  static constexpr uint32_t GBAR = 128;                           // barriers of a group
+  static constexpr uint32_t O_INFO = O_BAR + NG * GBAR + 16;      // of a group: records of eight pairs, flags of four
+  static constexpr size_t SMEM = O_INFO + NG * 256;
+  static constexpr uint32_t T_P = 64, T_O = 96, COLS = 96 + D;    // tensor-memory columns of a group: S, P, O
 };
 
-__device__ __forceinline__ void tmem_ld8(uint32_t a, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(a) : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t a, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+constexpr int PR_TWO = 1, PR_FIRST = 2, PR_END = 4;               // two blocks; first pair of a unit; no pair
 
 struct FsArgs {
   __nv_bfloat16* O;
@@ -62,28 +60,34 @@ struct FsArgs {
   int* status;
 };
 
-// EXACT: two passes over a row, the maximum first, and the sums in a fixed order (four chains a half tile): O and lse bit for bit as a two-pass kernel
-// gives them.  For the full mask, where some results are sums that cancel to nothing but rounding (the gradient of the key
-// projection's bias is zero in dense attention), so that every other order of the additions gives other numbers.
-template <int D, bool KP, bool SUB, bool EXACT>
-__global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+template <int D, bool KP, bool SUB>
+__global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ FsArgs a) {
   using C = Fs<D>;
   using T = OpTile<D>;
+  constexpr int NG = C::NG;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t sbase = smem_u32(smem_raw);                      // must be 1024-aligned (checked below)
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
-  const int grp = warp < 4 ? warp : (warp - 4) >> 2;
+  const int grp = warp < 4 * NG ? warp >> 2 : (warp - 4 * NG) & 3;          // arithmetic warps, four for MMAs, four for loads
   const uint32_t gb = sbase + grp * C::GROUP, bars = sbase + C::O_BAR + grp * C::GBAR;
-  // q_full, k_full[2], v_full: tiles landed; s_ready: S of a pair complete; s_free: read out (4 warps); p_ready[2]: P tiles written (4
-  // warps); pv_done[2]: O += P V of a pair complete, with every MMA issued before it; pi_full[2]: flags of a pair written
-  const uint32_t q_full = bars, k_full = bars + 8, v_full = bars + 24, s_ready = bars + 32, s_free = bars + 40, p_ready = bars + 48,
-                 pv_done = bars + 64, pi_full = bars + 80;
+  // k_full[KB]: K tiles of a pair, Q with the first of a unit, and the pair's record; k_free[KB]: S of that pair complete; v_full[2]: V tiles
+  // landed; v_free[2]: product of that pair complete; s_ready: S of a pair complete; s_free: read out (4 warps); p_ready: P of a pair written
+  // (4 warps); pv_done: O += P V of a pair complete; pi_full[4]: flags of a pair written.  A parity tells two phases apart.  Every waiter waits
+  // for each phase, and the next one needs something that comes after that wait: S of pair j + 1 the four arrivals on s_free for pair j, the
+  // product of pair j + 1 those on p_ready, which follow the warps' wait for the product of pair j, tiles a buffer that the loader saw free.
+  // Records and flags of pair j are written when S of pair j - KB is complete, so the arithmetic of pair j - 3 has read its own.
+  constexpr uint32_t B_KFULL = 0, B_KFREE = 16, B_VFULL = 32, B_VFREE = 48, B_SREADY = 64, B_SFREE = 72, B_PREADY = 80, B_PV = 88, B_PI = 96;
+  const uint32_t k_full = bars + B_KFULL, k_free = bars + B_KFREE, v_full = bars + B_VFULL, v_free = bars + B_VFREE, s_ready = bars + B_SREADY,
+                 s_free = bars + B_SFREE, p_ready = bars + B_PREADY, pv_done = bars + B_PV, pi_full = bars + B_PI;
+  constexpr int KB = C::KB;
   const uint32_t slot = sbase + C::O_BAR + NG * C::GBAR, abort_w = slot + 4;
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
   volatile int* abort_ptr = reinterpret_cast<volatile int*>(smem_raw + (abort_w - sbase));
-  // [2][8]: flags, block columns of the pair, -, penalties of its blocks in base-2 units
-  int* info = reinterpret_cast<int*>(smem_raw + (slot - sbase) + 16 + grp * 64);
+  // records [8]: {PR_*| (b,h) << 4, block columns c0 | c1 << 16, CSR block ids};  flags [4][8]: which blocks have different penalties and
+  // which quarters are selected, block columns, -, one penalty per block in base-2 units
+  int4* ring = reinterpret_cast<int4*>(smem_raw + C::O_INFO + grp * 256);
+  int* info = reinterpret_cast<int*>(smem_raw + C::O_INFO + grp * 256 + 128);
 
   if (warp == 0 && lane == 0) {
     int ab = *reinterpret_cast<volatile int*>(a.status);
@@ -91,9 +95,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
     *abort_ptr = ab;
     for (int g = 0; g < NG; ++g) {
       const uint32_t b = sbase + C::O_BAR + g * C::GBAR;
-      for (int x = 0; x < 5; ++x) mbar_init(b + 8 * x, 1);        // q_full, k_full[2], v_full, s_ready
-      for (int x = 5; x < 8; ++x) mbar_init(b + 8 * x, 4);        // s_free, p_ready[2]
-      for (int x = 8; x < 12; ++x) mbar_init(b + 8 * x, 1);       // pv_done[2], pi_full[2]
+      for (int x = 0; x < 16; ++x) mbar_init(b + 8 * x, x == 9 || x == 10 ? 4 : 1);     // s_free, p_ready: the group's warps
     }
     fence_barrier_init();
   }
@@ -106,192 +108,170 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *slot_ptr, tS = tmem + grp * C::COLS, tO = tS + 64u;
+  const uint32_t tmem = *slot_ptr, tS = tmem + grp * C::COLS, tP = tS + C::T_P, tO = tS + C::T_O;
   auto wait_all = [&](uint32_t bar, uint32_t parity, int code) -> bool { return warp_wait(bar, parity & 1u, a.status, code); };
   const UnitMap um{a.nb, a.BH, a.by_rank};
   // group g of CTA b walks units b + g G, + NG G, ...
   const int first = (int)blockIdx.x + grp * (int)gridDim.x, step = NG * (int)gridDim.x, total = a.nb * a.BH;
 
-  if (warp < 4) {
-    // ================================================================== service warp of a group
-    constexpr uint32_t IDESC_S = make_idesc_bf16(64, 64, 0, 0), IDESC_O = make_idesc_bf16(64, D, 0, 1);
-    const uint64_t dQ = T::kmajor(gb + C::O_Q, 0);
-    Walk c, ld;                                                   // MMAs; loads (a pair ahead)
-    c.init(um, a.rec, first, step, total);
-    c.skip();
-    ld = c;
-    int4 pr = ld.valid() ? a.pair[ld.cur.y] : make_int4(0, -1, 0, 0);      // record of the pair whose K tiles are loaded next
-    int4 prv = pr;                                                // ... whose V tiles are loaded next
-    bool c_val = !EXACT, ld_val = !EXACT, p_val = false;          // pair of the value pass: c, ld, the pair before c
-    Pen4 pen_l = {};
-    uint8_t sub_l = 0xff;
-    auto flags_load = [&](const Walk& w, const int4& p) {         // requested with the pair's K tiles, used a pair later
-      const int e = lane >> 4, o = e ? p.y : p.x;
-      if (KP && o >= 0) pen_load(pen_l, a.keypad + (size_t)w.bh * a.L + o * BS);
-      if (SUB) sub_l = o >= 0 ? a.submask[e ? p.w : p.z] : (uint8_t)0;
-    };
-    auto load_k = [&](int j) {                                    // K tiles of the pair at `ld` (pair j), Q with the first of a unit
-      const uint32_t bar = k_full + 8 * (C::ALIAS ? (j & 1) : 0), dst = gb + (C::ALIAS ? C::O_P + (j & 1) * C::PB : C::O_K);
-      const int cnt = ld.cnt();
-      const OpPos pos = op_pos(ld.bh, a.L, a.heads, D);
-      const bool with_q = ld.k == 0 && (!EXACT || !ld_val);
-      if (lane == 0) {
-        mbar_expect_tx(bar, cnt * T::BYTES);
-        if (with_q) mbar_expect_tx(q_full, T::BYTES);
+  auto wait_one = [&](uint32_t bar, uint32_t parity, int code) -> bool {           // one thread
+    if (mbar_wait(bar, parity & 1u)) return true;
+    report(a.status, code);
+    return false;
+  };
+  if (warp < 4 * NG) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::REGS_A));
+  else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::REGS_S));
+
+  if (warp >= 4 * NG + 4) {
+    // ================================================================== loads of a group
+    Walk w;
+    w.init(um, a.rec, first, step, grp < NG ? total : 0);
+    w.skip();
+    int4 pr = w.valid() ? a.pair[w.cur.y] : make_int4(0, -1, 0, 0), nx = pr;       // records of pairs j, j + 1
+    int units = 0;
+    for (int j = 0; grp < NG; ++j) {
+      const int kj = j / KB;
+      if (j >= KB && !wait_all(k_free + 8 * (j % KB), (uint32_t)(kj - 1), ERR_MMA_WAIT)) break;
+      const uint32_t kb = k_full + 8 * (j % KB);
+      if (!w.valid()) {
+        if (lane == 0) {
+          ring[j & 7] = make_int4(PR_END, 0, 0, 0);
+          mbar_arrive(kb);
+        }
+        break;
+      }
+      const bool two = w.cnt() == 2, with_q = w.k == 0;
+      const OpPos pos = op_pos(w.bh, a.L, a.heads, D);
+      const int bh = w.bh, line = w.cur.x;
+      if (elect_one()) {
+        ring[j & 7] = make_int4((two ? PR_TWO : 0) | (with_q ? PR_FIRST : 0), 0, 0, 0);
+        mbar_expect_tx(kb, ((two ? 2 : 1) + (with_q ? 1 : 0)) * T::BYTES);
+        const uint32_t dst = gb + C::O_K + (j % KB) * 2 * T::BYTES;
+        tma_load_2d(dst, &tmK, kb, pos.x0, pos.row0 + pr.x * BS);
+        if (two) tma_load_2d(dst + T::BYTES, &tmK, kb, pos.x0, pos.row0 + pr.y * BS);
+        // the Q buffer was read by the unit before the last, whose last pair is not after the one k_free was for
+        if (with_q) tma_load_2d(gb + C::O_Q + (units & 1) * T::BYTES, &tmQ, kb, pos.x0, pos.row0 + line * BS);
       }
       __syncwarp();
-      if (lane < cnt) tma_load_2d(dst + lane * T::BYTES, &tmK, bar, pos.x0, pos.row0 + (lane ? pr.y : pr.x) * BS);
-      if (lane == 4 && with_q) tma_load_2d(gb + C::O_Q, &tmQ, q_full, pos.x0, pos.row0 + ld.cur.x * BS);
-    };
-    auto load_v = [&](const Walk& w) {
-      const int cnt = w.cnt();
-      const OpPos pos = op_pos(w.bh, a.L, a.heads, D);
-      if (lane == 0) mbar_expect_tx(v_full, cnt * T::BYTES);
-      __syncwarp();
-      if (lane < cnt) tma_load_2d(gb + C::O_V + lane * T::BYTES, &tmV, v_full, pos.x0, pos.row0 + (lane ? prv.y : prv.x) * BS);
-    };
-    // EXACT: the pairs of a unit come twice, for the maximum and for the values
-    auto step_on = [&](Walk& w, bool& values) {
-      if (EXACT && w.last() && !values) { values = true; w.k = 0; return; }
-      const bool end = w.last();
+      if (w.last()) ++units;
       w.next();
-      if (EXACT && end) values = false;
-    };
-    bool ok = true;
-    int units = 0, jv = 0;                                        // units with blocks begun; value pairs before pair j
-    if (c.valid()) {
-      flags_load(ld, pr);
-      load_k(0);
-      prv = pr;
-      if (ld_val) load_v(ld);
-      step_on(ld, ld_val);
-      if (ld.valid()) pr = a.pair[ld.cur.y + ld.k];
-    }
-    int p_cnt = 0, p_par = 0;                                     // the pair before c
-    bool p_first = false;
-    for (int j = 0; ok; ++j) {
-      const bool have = c.valid();
-      if (have) {
-        if (KP || SUB) {                                          // flags of pair j: its buffer was read before P of pair j - 2 was written
-          uint32_t mixed = 0u;
-          const float pen = KP ? pen_of(pen_l, mixed) * LOG2E : 0.f, pen1 = KP ? __shfl_sync(0xffffffffu, pen, 16) : 0.f;
-          const int s1 = SUB ? __shfl_sync(0xffffffffu, (int)sub_l, 16) : 0xff;
-          if (lane == 0) {
-            int* x = info + 8 * (j & 1);
-            x[0] = (int)mixed | ((SUB ? (int)sub_l : 0xff) << 8) | (s1 << 16);
-            x[1] = prv.x; x[2] = prv.y;
-            if (KP) { x[4] = __float_as_int(pen); x[5] = __float_as_int(pen1); }
-            mbar_arrive(pi_full + 8 * (j & 1));
-          }
-          __syncwarp();
+      if (w.valid()) nx = a.pair[w.cur.y + w.k];
+      if (KP || SUB) {
+        const int e = lane >> 4, o = e ? (two ? pr.y : -1) : pr.x;
+        uint32_t mixed = 0u;
+        float pen = 0.f, pen1 = 0.f;
+        if (KP) {
+          Pen4 p = {};
+          if (o >= 0) pen_load(p, a.keypad + (size_t)bh * a.L + o * BS);
+          pen = pen_of(p, mixed) * LOG2E;
+          pen1 = __shfl_sync(0xffffffffu, pen, 16);
         }
-        // S of pair j
-        const int kb = C::ALIAS ? (j & 1) : 0, ku = C::ALIAS ? (j >> 1) : j;
-        if (c.k == 0 && (!EXACT || !c_val)) { if (!wait_all(q_full, (uint32_t)units, ERR_LOAD_WAIT)) { ok = false; break; } ++units; }
-        if (!wait_all(k_full + 8 * kb, (uint32_t)ku, ERR_LOAD_WAIT)) { ok = false; break; }
-        if (j >= 1 && !wait_all(s_free, (uint32_t)(j - 1), ERR_MMA_WAIT)) { ok = false; break; }
-        const bool two = warp_uniform(c.cnt() == 2);
-        if (elect_one()) {
+        const int sub_l = SUB && o >= 0 ? a.submask[e ? pr.w : pr.z] : 0;
+        const int s1 = SUB ? __shfl_sync(0xffffffffu, sub_l, 16) : 0xff;
+        if (lane == 0) {
+          int* x = info + 8 * (j & 3);
+          x[0] = (int)mixed | ((SUB ? sub_l : 0xff) << 8) | (s1 << 16);
+          x[1] = pr.x; x[2] = pr.y;
+          if (KP) { x[4] = __float_as_int(pen); x[5] = __float_as_int(pen1); }
+          mbar_arrive(pi_full + 8 * (j & 3));
+        }
+        __syncwarp();
+      }
+      if (j >= 2 && !wait_all(v_free + 8 * (j & 1), (uint32_t)(j >> 1) - 1u, ERR_MMA2_WAIT)) break;
+      if (elect_one()) {
+        const uint32_t vb = v_full + 8 * (j & 1), dst = gb + C::O_V + (j & 1) * 2 * T::BYTES;
+        mbar_expect_tx(vb, (two ? 2 : 1) * T::BYTES);
+        tma_load_2d(dst, &tmV, vb, pos.x0, pos.row0 + pr.x * BS);
+        if (two) tma_load_2d(dst + T::BYTES, &tmV, vb, pos.x0, pos.row0 + pr.y * BS);
+      }
+      __syncwarp();
+      pr = nx;
+    }
+  } else if (warp >= 4 * NG) {
+    // ================================================================== MMAs of a group: one thread
+    if (grp < NG && elect_one()) {
+      constexpr uint32_t IDESC_S = make_idesc_bf16(64, 64, 0, 0), IDESC_O = make_idesc_bf16(64, D, 0, 1);
+      const uint64_t dQ = T::kmajor(gb + C::O_Q, 0), dK = T::kmajor(gb + C::O_K, 0), dV = T::mnmajor(gb + C::O_V, 0);
+      int units = 0;                                              // units up to the one of pair j
+      int prev = 0;                                               // record of pair j - 1
+      for (int j = 0;; ++j) {
+        if (!wait_one(k_full + 8 * (j % KB), (uint32_t)(j / KB), ERR_LOAD_WAIT)) break;
+        const int now = ring[j & 7].x;
+        if (!(now & PR_END)) {                                    // S of pair j
+          if (now & PR_FIRST) ++units;
+          if (j >= 1 && !wait_one(s_free, (uint32_t)(j - 1), ERR_MMA_WAIT)) break;
           tc_fence_after();
-          const uint64_t dK = T::kmajor(gb + (C::ALIAS ? C::O_P + kb * C::PB : C::O_K), 0);
+          const uint64_t q = desc_advance(dQ, ((units - 1) & 1) * T::BYTES), k = desc_advance(dK, (j % KB) * 2 * T::BYTES);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) mma_bf16(tS, desc_advance(dQ, kk * T::K_STEP), desc_advance(dK, kk * T::K_STEP), IDESC_S, kk > 0);
-          if (two) {
+          for (int kk = 0; kk < D / 16; ++kk) mma_bf16(tS, desc_advance(q, kk * T::K_STEP), desc_advance(k, kk * T::K_STEP), IDESC_S, kk > 0);
+          if (now & PR_TWO) {
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk)
-              mma_bf16(tS + (16u << 16), desc_advance(dQ, kk * T::K_STEP), desc_advance(dK, T::BYTES + kk * T::K_STEP), IDESC_S, kk > 0);
+              mma_bf16(tS + (16u << 16), desc_advance(q, kk * T::K_STEP), desc_advance(k, T::BYTES + kk * T::K_STEP), IDESC_S, kk > 0);
           }
           mma_commit(s_ready);
+          mma_commit(k_free + 8 * (j % KB));
         }
-        __syncwarp();
-      }
-      if (j >= 1) {                                               // O += P V of pair j - 1
-        const int jp = j - 1;
-        if (!wait_all(p_ready + 8 * (jp & 1), (uint32_t)(jp >> 1), ERR_MMA_WAIT)) { ok = false; break; }
-        if (p_val) { if (!wait_all(v_full, (uint32_t)jv, ERR_LOAD_WAIT)) { ok = false; break; } ++jv; }
-        const bool two = warp_uniform(p_cnt == 2), fresh = warp_uniform((int)p_first) != 0, value_pair = warp_uniform((int)p_val) != 0;
-        if (elect_one()) {
+        if (j >= 1) {                                             // O += P V of pair j - 1
+          const int jp = j - 1;
+          if (!wait_one(v_full + 8 * (jp & 1), (uint32_t)(jp >> 1), ERR_LOAD_WAIT)) break;
+          if (!wait_one(p_ready, (uint32_t)jp, ERR_MMA_WAIT)) break;
           tc_fence_after();
-          const uint32_t acc = tO + ((uint32_t)(p_par * 16) << 16);
-          const uint64_t dP = ValTile::kmajor(gb + C::O_P + (jp & 1) * C::PB, 0), dV = T::mnmajor(gb + C::O_V, 0);
-          if (EXACT && !value_pair) {                             // nothing to multiply: the commit alone says that S has been read
-          } else {
+          const uint32_t more = (prev & PR_FIRST) ? 0u : 1u;      // not the first product of its unit
+          const uint64_t v = desc_advance(dV, (jp & 1) * 2 * T::BYTES);
 #pragma unroll
-          for (int kk = 0; kk < BS / 16; ++kk)
-            mma_bf16(acc, desc_advance(dP, kk * ValTile::K_STEP), desc_advance(dV, kk * T::MN_STEP), IDESC_O, (kk > 0 || !fresh) ? 1u : 0u);
-          if (two) {
+          for (int kk = 0; kk < BS / 16; ++kk) mma_bf16_ts(tO, tP + kk * 8u, desc_advance(v, kk * T::MN_STEP), IDESC_O, kk > 0 ? 1u : more);
+          if (prev & PR_TWO) {
 #pragma unroll
             for (int kk = 0; kk < BS / 16; ++kk)
-              mma_bf16(acc, desc_advance(dP, VT_BYTES + kk * ValTile::K_STEP), desc_advance(dV, T::BYTES + kk * T::MN_STEP), IDESC_O, 1u);
+              mma_bf16_ts(tO + (16u << 16), tP + (16u << 16) + kk * 8u, desc_advance(v, T::BYTES + kk * T::MN_STEP), IDESC_O, kk > 0 ? 1u : more);
           }
-          }
-          mma_commit(pv_done + 8 * (jp & 1));
+          mma_commit(pv_done);
+          mma_commit(v_free + 8 * (jp & 1));
         }
-        __syncwarp();
+        if (now & PR_END) break;
+        prev = now;
       }
-      if (!have) break;
-      // Loads.  O += P V of pair j - 1 complete implies S of pair j (issued before it): K (its own buffer, or the P buffer of
-      // pair j - 1), Q and V are free.
-      if (j >= 1) {
-        if (!wait_all(pv_done + 8 * ((j - 1) & 1), (uint32_t)((j - 1) >> 1), ERR_MMA2_WAIT)) { ok = false; break; }
-        if (c_val) load_v(c);                                     // V of pair j (pair 0's was requested above)
-      } else if (!wait_all(s_ready, 0u, ERR_MMA_WAIT)) { ok = false; break; }
-      if (ld.valid()) {
-        flags_load(ld, pr);
-        load_k(j + 1);
-        prv = pr;
-        step_on(ld, ld_val);
-        if (ld.valid()) pr = a.pair[ld.cur.y + ld.k];
-      }
-      p_cnt = c.cnt(); p_par = units & 1; p_first = c.k == 0; p_val = c_val;
-      step_on(c, c_val);
     }
+    __syncwarp();
   } else {
     // ================================================================== arithmetic warps of a group
     const int q = warp & 3, hf = lane >> 4, row = q * 16 + (lane & 15);
-    const uint32_t lS = tS + ((uint32_t)(q * 32) << 16), lO = tO + ((uint32_t)(q * 32) << 16);
+    const uint32_t lS = tS + ((uint32_t)(q * 32) << 16), lP = lS + C::T_P, lO = lS + C::T_O;
     const float sc2 = a.scale * LOG2E, floor2 = a.floor_v * LOG2E, inv_scale = 1.0f / a.scale;
     bool ok = true;
-    // the finished unit whose rows are still in tensor memory
-    bool pend = false;
-    int pend_par = 0, pend_j = 0;
+    // The finished unit whose rows are still in tensor memory: the products of first entries in lanes 0-15 of every quadrant, of second ones
+    // in lanes 16-31.  Lane l gives half of its columns to lane l ^ 16 and takes the other half's from there.
+    bool pend = false, pend_two = false;
     float pend_inv = 0.f;
     __nv_bfloat16* pend_dst = nullptr;
-    auto write_rows = [&](__nv_bfloat16* dst, bool have, float inv, bool mine) {
+    auto put = [&](__nv_bfloat16* dst, const float (&v)[16]) {
+#pragma unroll
+      for (int x = 0; x < 16; x += 8)
+        *reinterpret_cast<uint4*>(dst + x) = make_uint4(pack_bf16(v[x], v[x + 1]), pack_bf16(v[x + 2], v[x + 3]), pack_bf16(v[x + 4], v[x + 5]),
+                                                        pack_bf16(v[x + 6], v[x + 7]));
+    };
+    auto flush = [&]() {                                          // its last product is complete
 #pragma unroll
       for (int h = 0; h < D / 32; ++h) {
         uint32_t v[32];
-        if (have) {
-          tmem_ld32(lO + h * 32, v);
-          tmem_ld_wait();
-        } else {
+        tmem_ld32(lO + h * 32, v);
+        tmem_ld_wait();
+        float o[16];
 #pragma unroll
-          for (int x = 0; x < 32; ++x) v[x] = 0u;
+        for (int x = 0; x < 16; ++x) {
+          const float keep = __uint_as_float(hf ? v[16 + x] : v[x]), give = __uint_as_float(hf ? v[x] : v[16 + x]);
+          const float take = __shfl_xor_sync(0xffffffffu, give, 16);
+          // one entry: what lanes 16-31 hold was never written
+          o[x] = (pend_two ? keep + take : hf ? take : keep) * pend_inv;
         }
-        if (mine) {
-#pragma unroll
-          for (int x = 0; x < 32; x += 8)
-            *reinterpret_cast<uint4*>(dst + h * 32 + x) = make_uint4(pack_bf16(__uint_as_float(v[x]) * inv, __uint_as_float(v[x + 1]) * inv),
-                                                                     pack_bf16(__uint_as_float(v[x + 2]) * inv, __uint_as_float(v[x + 3]) * inv),
-                                                                     pack_bf16(__uint_as_float(v[x + 4]) * inv, __uint_as_float(v[x + 5]) * inv),
-                                                                     pack_bf16(__uint_as_float(v[x + 6]) * inv, __uint_as_float(v[x + 7]) * inv));
-        }
+        put(pend_dst + h * 32 + hf * 16, o);
       }
-    };
-    auto flush = [&]() -> bool {
-      if (!wait_all(pv_done + 8 * (pend_j & 1), (uint32_t)(pend_j >> 1), ERR_MMA2_WAIT)) return false;
-      tc_fence_after();
-      write_rows(pend_dst, true, pend_inv, hf == pend_par);
-      tc_fence_before();
       pend = false;
-      return true;
     };
     Walk u;
     u.init(um, a.rec, first, step, total);
     int j = 0;
-    // Units with blocks begun.  Two of them in a row must not share their lanes: the rows of the first are read while the product of
-    // the second is issued.  Rows without blocks have no product and hand nothing over, so they do not count.
-    int units = 0;
     for (; u.valid() && ok; u.shift()) {
       const int n = u.cur.w;
       const OpPos pos = op_pos(u.bh, a.L, a.heads, D);
@@ -300,24 +280,22 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
       if (n == 0) {                                               // a row without blocks: every key counts as score 0
         const float m0 = fmaxf(floor2, -INFINITY);
         if (hf == 0) *lse = m0 + log2f((float)a.L * exp2f(-m0));
-        write_rows(dst, false, 0.f, hf == 0);
+        const float zero[16] = {};
+        for (int h = 0; h < D; h += 32) put(dst + h + hf * 16, zero);
         continue;
       }
-      const int par = ++units & 1;
       const float* kpu = KP ? a.keypad + (size_t)u.bh * a.L : nullptr;
       float m = floor2, mx = floor2, l = 0.f;                     // reference exponent, true maximum, sum
       int n_sel = 0;
       const int np = u.pairs();
-      for (int kx = EXACT ? -np : 0; kx < np && ok; ++kx, ++j) {
-        const bool values = !EXACT || kx >= 0;
-        const int k = values ? kx : kx + np;
+      for (int k = 0; k < np && ok; ++k, ++j) {
         const bool mine = 2 * k + hf < n;
         const float* kp = nullptr;
         float pen = 0.f;
         bool live0 = mine, live1 = mine;
         if (KP || SUB) {
-          if (!wait_all(pi_full + 8 * (j & 1), (uint32_t)(j >> 1), ERR_MMA_WAIT)) { ok = false; break; }
-          const int* x = info + 8 * (j & 1);
+          if (!wait_all(pi_full + 8 * (j & 3), (uint32_t)(j >> 2), ERR_MMA_WAIT)) { ok = false; break; }
+          const int* x = info + 8 * (j & 3);
           const int f = x[0];
           if (KP) {
             const bool mixed = (f >> hf) & 1;
@@ -328,10 +306,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
             const int bits = (f >> (8 + 8 * hf + (q >> 1) * 2)) & 3;
             live0 = mine && (bits & 1);
             live1 = mine && (bits & 2);
-            n_sel += mine && values ? 32 * __popc(bits) : 0;
+            n_sel += mine ? 32 * __popc(bits) : 0;
           }
         }
-        if (!SUB && values) n_sel += mine ? BS : 0;
+        if (!SUB) n_sel += mine ? BS : 0;
         if (!wait_all(s_ready, (uint32_t)j, ERR_MMA_WAIT)) { ok = false; break; }
         tc_fence_after();
         uint32_t v0[32], v1[32];
@@ -346,7 +324,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
           take_penalty(v1, kp + 32, inv_scale);
         }
         float cm = -INFINITY;
-        if (!EXACT || !values) {                                                         // the scale is positive: compare raw scores
+        {                                                         // the scale is positive: compare raw scores
           float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
           for (int x = 0; x < 32; x += 4) {
@@ -360,15 +338,13 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
         }
         cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, 16));     // both owners of a row agree
         mx = fmaxf(mx, cm);
-        if (EXACT) {
-          m = mx;
-        } else if (k == 0) {
+        if (k == 0) {
           m = mx;
         } else if (__any_sync(0xffffffffu, mx > m + MOVE)) {      // rare: move the reference, rescale what has been summed
           const float m_new = mx > m + MOVE ? mx : m, f = exp2f(m - m_new);
           l *= f;
           m = m_new;
-          if (!wait_all(pv_done + 8 * ((j - 1) & 1), (uint32_t)((j - 1) >> 1), ERR_MMA2_WAIT)) { ok = false; break; }
+          if (!wait_all(pv_done, (uint32_t)(j - 1), ERR_MMA2_WAIT)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll 1
           for (int h = 0; h < D; h += 8) {
@@ -381,56 +357,53 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
           }
           tmem_st_wait();
         }
-        // the P tiles of pair j - 2 have been consumed
-        if (j >= 2 && !wait_all(pv_done + 8 * (j & 1), (uint32_t)(j >> 1) - 1u, ERR_MMA2_WAIT)) { ok = false; break; }
-        const uint32_t tile = gb + C::O_P + (j & 1) * C::PB + hf * VT_BYTES + row * 128;
         uint64_t l2 = 0ull;
         const uint64_t sc22 = pack2(sc2, sc2), nm2 = pack2(-(m + pen), -(m + pen));
-        auto half_row = [&](const uint32_t (&v)[32], int g, bool live) {
-          float l4[4] = {0.f, 0.f, 0.f, 0.f};
+        // P of 32 keys, two per register
+        auto half_row = [&](uint32_t (&v)[32], bool live) {
+          uint64_t sum = 0ull;
 #pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {                        // eight columns: one 16-byte piece of the tile row
-            uint32_t w[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-              const int c = cc * 8 + 2 * x;
-              float e0, e1;
-              unpack2(fma2(pack2(v[c], v[c + 1]), sc22, nm2), e0, e1);
-              e0 = ex2_approx(e0); e1 = ex2_approx(e1);
-              if (EXACT) {
-                if (!SUB || live) l4[x] += e0 + e1;
-              } else if (!SUB || live) {
-                l2 = add2(l2, pack2(e0, e1));
-              }
-              w[x] = !SUB || live ? pack_bf16(e0, e1) : 0u;
-            }
-            st_shared_v4(tile + (uint32_t)(((g * 4 + cc) ^ (row & 7)) << 4), w);
+          for (int x = 0; x < 16; ++x) {
+            float e0, e1;
+            unpack2(fma2(pack2(v[2 * x], v[2 * x + 1]), sc22, nm2), e0, e1);
+            e0 = ex2_approx(e0); e1 = ex2_approx(e1);
+            sum = add2(sum, pack2(e0, e1));
+            v[x] = pack_bf16(e0, e1);
           }
-          if (EXACT && (!SUB || live)) l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+          if (!live) {
+            sum = 0ull;
+#pragma unroll
+            for (int x = 0; x < 16; ++x) v[x] = 0u;
+          }
+          l2 = add2(l2, sum);
         };
-        if (mine && values) {
-          half_row(v0, 0, live0);
-          half_row(v1, 1, live1);
-          if (!EXACT) {
-            float la, lb;
-            unpack2(l2, la, lb);
-            l += la + lb;
-          }
-        }
-        fence_proxy_async();                                      // P rows -> visible to the MMA
-        tc_fence_before();
+        half_row(v0, live0);
+        // P and O of the pair before: by now its product has long been issued
+        if (j >= 1 && !wait_all(pv_done, (uint32_t)(j - 1), ERR_MMA2_WAIT)) { ok = false; break; }
+        tc_fence_after();
+        tmem_st16(lP, v0);
+        half_row(v1, live1);
+        tmem_st16(lP + 16u, v1);
+        float la, lb;
+        unpack2(l2, la, lb);
+        l += la + lb;
+        if (pend) flush();                                        // the previous unit, before this one's first product
+        tmem_st_wait();
+        tc_fence_before();                                        // P -> visible to the MMA
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_ready + 8 * (j & 1));
-        if (pend) ok = flush();                                   // the previous unit: its last product has long been issued
+        if (lane == 0) mbar_arrive(p_ready);
       }
       if (!ok) break;
       n_sel += __shfl_xor_sync(0xffffffffu, n_sel, 16);
       l += __shfl_xor_sync(0xffffffffu, l, 16);
-      const float f = EXACT ? 1.0f : exp2f(m - mx), z = l * f + (float)(a.L - n_sel) * exp2f(-mx);
+      const float f = exp2f(m - mx), z = l * f + (float)(a.L - n_sel) * exp2f(-mx);
       if (hf == 0) *lse = mx + log2f(z);
-      pend = true; pend_par = par; pend_j = j - 1; pend_inv = f / z; pend_dst = dst;
+      pend = true; pend_two = n > 1; pend_inv = f / z; pend_dst = dst;
     }
-    if (ok && pend) flush();
+    if (ok && pend && wait_all(pv_done, (uint32_t)(j - 1), ERR_MMA2_WAIT)) {
+      tc_fence_after();
+      flush();
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -441,14 +414,14 @@ __global__ void __launch_bounds__(FS_THREADS, 1) k_fwd_stream(const __grid_const
 
 namespace tc {
 
-template <int D, bool KP, bool SUB, bool EXACT>
+template <int D, bool KP, bool SUB>
 static int fs_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FsArgs& a) {
   using C = Fs<D>;
-  static_assert(C::SMEM <= 227 * 1024 && NG * C::COLS <= 512, "shared or tensor memory");
-  auto k = k_fwd_stream<D, KP, SUB, EXACT>;
+  static_assert(C::SMEM <= 227 * 1024 && C::NG * C::COLS <= 512, "shared or tensor memory");
+  auto k = k_fwd_stream<D, KP, SUB>;
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
-  k<<<grid, FS_THREADS, C::SMEM, c->stream>>>(mq, mk, mv, a);
+  k<<<grid, C::THREADS, C::SMEM, c->stream>>>(mq, mk, mv, a);
   SPION_LAUNCH_CHECK();
   c->launches += 1;
   return SPION_OK;
@@ -464,16 +437,13 @@ static int fs_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUt
   a.submask = vw.submask;
   a.L = c->L; a.BH = c->BH; a.nb = vw.nb; a.heads = c->heads; a.by_rank = order_by_rank(c);
   a.scale = c->scale; a.floor_v = keypad ? 0.0f : -100.0f; a.status = c->status_dev;
-  if (c->nnzb == c->nb * c->nb)                                   // the full mask has no unselected quarters
-    return keypad ? fs_launch<D, true, false, true>(c, s, mq, mk, mv, a) : fs_launch<D, false, false, true>(c, s, mq, mk, mv, a);
-  if (keypad) return vw.submask ? fs_launch<D, true, true, false>(c, s, mq, mk, mv, a) : fs_launch<D, true, false, false>(c, s, mq, mk, mv, a);
-  return vw.submask ? fs_launch<D, false, true, false>(c, s, mq, mk, mv, a) : fs_launch<D, false, false, false>(c, s, mq, mk, mv, a);
+  if (keypad) return vw.submask ? fs_launch<D, true, true>(c, s, mq, mk, mv, a) : fs_launch<D, true, false>(c, s, mq, mk, mv, a);
+  return vw.submask ? fs_launch<D, false, true>(c, s, mq, mk, mv, a) : fs_launch<D, false, false>(c, s, mq, mk, mv, a);
 }
 
 template <int D>
 static int fs_attrs() {
-  for (auto k : {k_fwd_stream<D, false, false, false>, k_fwd_stream<D, true, false, false>, k_fwd_stream<D, false, true, false>,
-                 k_fwd_stream<D, true, true, false>, k_fwd_stream<D, false, false, true>, k_fwd_stream<D, true, false, true>})
+  for (auto k : {k_fwd_stream<D, false, false>, k_fwd_stream<D, true, false>, k_fwd_stream<D, false, true>, k_fwd_stream<D, true, true>})
     SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Fs<D>::SMEM));
   return SPION_OK;
 }

@@ -257,6 +257,11 @@ int stream_forward_set_attrs(int d);
 int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
                    float* lse);
 
+// tc_fwd_exact.cu: the same on the full mask, in a fixed order of sums
+int exact_forward_set_attrs(int d);
+int exact_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
+                  float* lse);
+
 // tc_fwd_pipe.cu: forward of the records [rank0, nb) of row_info (rows of at most ROW_NCH blocks)
 int pipe_set_attrs(TcState* s, int d, int device);
 int pipe_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
