@@ -315,6 +315,15 @@ int spion_attn_backward_fused(spion_ctx* ctx, const void* Q, const void* K, cons
                               const void* O, const void* dO, const float* lse, const float* keypad,
                               void* dQ, void* dK, void* dV);
 
+/* The pair for calls whose gradients are those of the rounded probabilities: P is normalised, then rounded to bf16, and O and
+ * dS are formed from that P, as spion_attn_forward_fused with P_optional and spion_attn_backward_ex do, bit for bit.  The
+ * backward reads no P: it rebuilds the tiles from Q, K and stat [2 * BH*L], two fp32 values per row that the forward writes.
+ * P_optional: the [BH, nnzb, 64, 64] probabilities, or NULL.  lse [BH*L] or NULL.  bf16, 64-wide blocks; UNSUPPORTED otherwise. */
+int spion_attn_forward_probs(spion_ctx* ctx, const void* Q, const void* K, const void* V, const float* keypad, void* O,
+                             float* lse, void* P_optional, float* stat);
+int spion_attn_backward_probs(spion_ctx* ctx, const void* Q, const void* K, const void* V, const void* O, const void* dO,
+                              const float* stat, const float* keypad, void* dQ, void* dK, void* dV);
+
 /* Head / batch mean of the probabilities of the current pattern (models/model_transformer.py:137) from
  * Q, K and the forward's log-sum-exp, without a stored P (tcgen05 engine only): A [L, L] fp32, zero
  * outside the selected blocks.  With the full mask this is the warm-up phase's attention map. */

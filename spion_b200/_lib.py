@@ -87,6 +87,8 @@ SIGNATURES = {
     "spion_supports_fused": (c_int, [c_void_p]),
     "spion_attn_forward_fused": (c_int, [c_void_p] * 8),
     "spion_attn_backward_fused": (c_int, [c_void_p] * 11),
+    "spion_attn_forward_probs": (c_int, [c_void_p] * 9),
+    "spion_attn_backward_probs": (c_int, [c_void_p] * 11),
     "spion_mean_map_recompute": (c_int, [c_void_p] * 6),
     "spion_softmax_forward_ex": (c_int, [c_void_p] * 4),
     "spion_softmax_backward_ex": (c_int, [c_void_p] * 4),

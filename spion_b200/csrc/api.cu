@@ -698,6 +698,24 @@ extern "C" int spion_attn_backward_fused(spion_ctx* c, const void* Q, const void
   return tc_engine_backward_fused(c, Q, K, V, O, dO, lse, keypad, dQ, dK, dV);
 }
 
+extern "C" int spion_attn_forward_probs(spion_ctx* c, const void* Q, const void* K, const void* V, const float* keypad, void* O, float* lse,
+                                        void* P_optional, float* stat) {
+  if (!c || !Q || !K || !V || !O || !stat) return SPION_ERR_ARG;
+  if (is_dense(c) || c->nnzb < 0) return SPION_ERR_STATE;
+  if (!use_tc(c)) return SPION_ERR_UNSUPPORTED;
+  DeviceGuard guard(c->device);
+  return tc_engine_forward_probs(c, Q, K, V, keypad, O, lse, P_optional, stat);
+}
+
+extern "C" int spion_attn_backward_probs(spion_ctx* c, const void* Q, const void* K, const void* V, const void* O, const void* dO, const float* stat,
+                                         const float* keypad, void* dQ, void* dK, void* dV) {
+  if (!c || !Q || !K || !V || !O || !dO || !stat || !dQ || !dK || !dV) return SPION_ERR_ARG;
+  if (is_dense(c) || c->nnzb < 0) return SPION_ERR_STATE;
+  if (!use_tc(c)) return SPION_ERR_UNSUPPORTED;
+  DeviceGuard guard(c->device);
+  return tc_engine_backward_probs(c, Q, K, V, O, dO, stat, keypad, dQ, dK, dV);
+}
+
 extern "C" int spion_block32_path_in_use(const spion_ctx* c) {
   if (!c) return SPION_ERR_ARG;
   return use_tc(c) ? tc_engine_block32_path(c) : 0;

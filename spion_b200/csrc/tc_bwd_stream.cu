@@ -64,7 +64,8 @@ template <int D, int SIDE> struct Bw {
 };
 
 struct BwArgs {
-  const float *lse, *delta, *keypad;         // [BH*L]; delta: COL only; keypad may be null
+  const float *lse, *delta, *keypad;         // [BH*L]; delta: COL only; keypad may be null; RND: lse holds the rows' exponents
+  const float* factor;                       // RND: [BH*L]
   float* delta_out;                          // ROW
   const __nv_bfloat16 *O, *dO;               // ROW: for delta
   __nv_bfloat16 *out0, *out1;                // dK (COL) or dQ (ROW); dV (COL)
@@ -96,8 +97,9 @@ __device__ __forceinline__ int pad64(const float* kp) {
   return other ? PAD_MIXED : first != 0.f ? PAD_ONE : PAD_NONE;
 }
 
-// KP: with key penalties.
-template <int D, int SIDE, bool SUB, bool KP>
+// KP: with key penalties.  RND: dS from the P that the forward wrote or would have written, rounded as there (stat of k_fwd_fused), and not
+// from P before it is rounded: the gradients are bit for bit those of kernels that read stored tiles.
+template <int D, int SIDE, bool SUB, bool KP, bool RND>
 __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                                                               const __grid_constant__ CUtensorMap tmF0, const __grid_constant__ CUtensorMap tmF1,
                                                               const __grid_constant__ BwArgs a) {
@@ -484,12 +486,13 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
 
     // record and statistics of this row are requested a pair early
     int4 rec = make_int4(PF_END, 0, 0, 0);
-    float h_next = 0.f, d_next = 0.f;
+    float h_next = 0.f, d_next = 0.f, f_next = 0.f;
     auto request = [&](uint32_t j) -> bool {
       if (!record(j, NGR, rec)) return false;
       if (rec.x >= 0 && (es == 0 || (rec.x & PF_TWO))) {
         const size_t ri = (size_t)rec.w * a.L + (SIDE == COL ? (es ? rec.y >> 16 : rec.y & 0xffff) : rec.z) * BS + row;
         h_next = a.lse[ri];
+        if (RND) f_next = a.factor[ri];
         d_next = SIDE == COL ? a.delta[ri] : __ldcg(a.delta_out + ri);            // ROW: written by this CTA
         // one penalty for all keys goes with the log-sum-exp (here, where it waits for the load: a value of its own costs every pair 2 %)
         if (KP && ((rec.x >> es) & PAD_ONE))
@@ -501,6 +504,8 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
     for (uint32_t j = grp; ok && rec.x >= 0; j += NGR) {
       const int flags = rec.x, line = rec.z, key = SIDE == COL ? rec.z : es ? rec.y >> 16 : rec.y & 0xffff, bh = rec.w;
       const float h = h_next, nds = -d_next * a.scale;
+      uint32_t f_hi = 0u, f_lo = 0u;
+      if (RND) row_factor(f_next, f_hi, f_lo);
       if (!request(j + NGR)) { ok = false; break; }
       const uint32_t ps = j % NP, set = j % 3;
       const bool mine = es == 0 || (flags & PF_TWO);
@@ -539,6 +544,11 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
                 unpack2(fma2(pack2(sv[c], sv[c + 1]), sc22, nh2), p0, p1);
                 p0 = ex2_approx(p0); p1 = ex2_approx(p1);
                 wp[x] = pack_bf16(p0, p1);
+                if (RND) {
+                  wp[x] = times_factor(wp[x], f_hi, f_lo);
+                  p0 = bf16_lo(wp[x]);
+                  p1 = bf16_hi(wp[x]);
+                }
                 unpack2(mul2(pack2(p0, p1), fma2(pack2(gv[c], gv[c + 1]), scale2, nds2)), d0, d1);
                 wd[x] = pack_bf16(d0, d1);
                 if (SUB && !live) { wp[x] = 0u; wd[x] = 0u; }
@@ -607,12 +617,12 @@ __global__ void k_line_recs(const int32_t* __restrict__ ptr, const int32_t* __re
 
 namespace tc {
 
-template <int D, int SIDE, bool SUB, bool KP>
+template <int D, int SIDE, bool SUB, bool KP, bool RND>
 static int bw_launch_one(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& f0, const CUtensorMap& f1,
                      const BwArgs& a) {
   using C = Bw<D, SIDE>;
   static_assert(C::SMEM <= 227 * 1024, "shared memory");
-  auto k = k_bwd_stream<D, SIDE, SUB, KP>;
+  auto k = k_bwd_stream<D, SIDE, SUB, KP, RND>;
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
   k<<<grid, BW_THREADS, C::SMEM, c->stream>>>(a0, a1, f0, f1, a);
@@ -624,15 +634,17 @@ static int bw_launch_one(spion_ctx* c, TcState* s, const CUtensorMap& a0, const 
 template <int D, int SIDE>
 static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& f0, const CUtensorMap& f1,
                      const BwArgs& a) {
-  if (a.submask) return a.keypad ? bw_launch_one<D, SIDE, true, true>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, true, false>(c, s, a0, a1, f0, f1, a);
-  return a.keypad ? bw_launch_one<D, SIDE, false, true>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, false, false>(c, s, a0, a1, f0, f1, a);
+  if (a.factor) return a.keypad ? bw_launch_one<D, SIDE, false, true, true>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, false, false, true>(c, s, a0, a1, f0, f1, a);
+  if (a.submask)
+    return a.keypad ? bw_launch_one<D, SIDE, true, true, false>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, true, false, false>(c, s, a0, a1, f0, f1, a);
+  return a.keypad ? bw_launch_one<D, SIDE, false, true, false>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, false, false, false>(c, s, a0, a1, f0, f1, a);
 }
 
 template <int D>
 static int bw_attrs() {
-  for (auto k : {k_bwd_stream<D, ROW, false, false>, k_bwd_stream<D, ROW, true, false>, k_bwd_stream<D, ROW, false, true>, k_bwd_stream<D, ROW, true, true>})
+  for (auto k : {k_bwd_stream<D, ROW, false, false, false>, k_bwd_stream<D, ROW, true, false, false>, k_bwd_stream<D, ROW, false, true, false>, k_bwd_stream<D, ROW, true, true, false>, k_bwd_stream<D, ROW, false, false, true>, k_bwd_stream<D, ROW, false, true, true>})
     SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, ROW>::SMEM));
-  for (auto k : {k_bwd_stream<D, COL, false, false>, k_bwd_stream<D, COL, true, false>, k_bwd_stream<D, COL, false, true>, k_bwd_stream<D, COL, true, true>})
+  for (auto k : {k_bwd_stream<D, COL, false, false, false>, k_bwd_stream<D, COL, true, false, false>, k_bwd_stream<D, COL, false, true, false>, k_bwd_stream<D, COL, true, true, false>, k_bwd_stream<D, COL, false, false, true>, k_bwd_stream<D, COL, false, true, true>})
     SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, COL>::SMEM));
   return SPION_OK;
 }
@@ -658,7 +670,7 @@ int stream_prepare(spion_ctx* c, TcState* s) {
 
 template <int D>
 static int bwd_stream(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const void* O, const void* dO, const float* lse,
-                      const float* keypad, void* dQ, void* dK, void* dV) {
+                      const float* keypad, void* dQ, void* dK, void* dV, bool rounded) {
   const TcView vw = tc_view(c, s);
   CUtensorMap mq, mk, mv, mdo;
   int rc;
@@ -667,6 +679,7 @@ static int bwd_stream(spion_ctx* c, TcState* s, const void* Q, const void* K, co
     return rc;
   BwArgs a;
   a.lse = lse; a.keypad = keypad;
+  a.factor = rounded ? lse + (size_t)c->BH * c->L : nullptr;
   a.delta = a.delta_out = s->delta_ws;
   a.O = (const __nv_bfloat16*)O; a.dO = (const __nv_bfloat16*)dO;
   a.submask = vw.submask;
@@ -687,9 +700,9 @@ static int bwd_stream(spion_ctx* c, TcState* s, const void* Q, const void* K, co
 }
 
 int recompute_backward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const void* O, const void* dO, const float* lse,
-                       const float* keypad, void* dQ, void* dK, void* dV) {
-  return c->d == 64 ? bwd_stream<64>(c, s, Q, K, V, O, dO, lse, keypad, dQ, dK, dV)
-                    : bwd_stream<32>(c, s, Q, K, V, O, dO, lse, keypad, dQ, dK, dV);
+                       const float* keypad, void* dQ, void* dK, void* dV, bool rounded) {
+  return c->d == 64 ? bwd_stream<64>(c, s, Q, K, V, O, dO, lse, keypad, dQ, dK, dV, rounded)
+                    : bwd_stream<32>(c, s, Q, K, V, O, dO, lse, keypad, dQ, dK, dV, rounded);
 }
 
 }  // namespace tc

@@ -851,7 +851,7 @@ static int forward_any(spion_ctx* c, const void* Q, const void* K, const void* V
     if (rc) return rc;
   }
   void* P64 = P_user ? (s->super ? s->p64_ws : P_user) : nullptr;
-  int rc = fused_forward(c, s, Q, K, V, keypad, O, lse ? lse : s->lse_ws, P64);
+  int rc = fused_forward(c, s, Q, K, V, keypad, O, lse ? lse : s->lse_ws, P64, nullptr);
   if (rc || !P_user || !s->super) return rc;
   return convert_tiles(c, s, false, s->p64_ws, P_user);
 }
@@ -884,7 +884,26 @@ int tc_engine_backward_fused(spion_ctx* c, const void* Q, const void* K, const v
   if (c->nnzb == 0) return SPION_ERR_SHAPE;
   TcState* s = (TcState*)c->tc;
   if (s->b32 && s->b32_use) return b32_backward(c, s, Q, K, V, O, dO, lse, keypad, dQ, dK, dV);
-  return recompute_backward(c, s, Q, K, V, O, dO, lse, keypad, dQ, dK, dV);
+  return recompute_backward(c, s, Q, K, V, O, dO, lse, keypad, dQ, dK, dV, false);
+}
+
+// 64-wide blocks only: P of 32-wide masks lies in derived super-blocks
+int tc_engine_forward_probs(spion_ctx* c, const void* Q, const void* K, const void* V, const float* keypad, void* O, float* lse, void* P_optional,
+                            float* stat) {
+  TcState* s = (TcState*)c->tc;
+  if (!s) return SPION_ERR_STATE;
+  if (s->super) return SPION_ERR_UNSUPPORTED;
+  if (c->nnzb == 0) return SPION_ERR_SHAPE;
+  return fused_forward(c, s, Q, K, V, keypad, O, lse ? lse : s->lse_ws, P_optional, stat);
+}
+
+int tc_engine_backward_probs(spion_ctx* c, const void* Q, const void* K, const void* V, const void* O, const void* dO, const float* stat,
+                             const float* keypad, void* dQ, void* dK, void* dV) {
+  TcState* s = (TcState*)c->tc;
+  if (!s) return SPION_ERR_STATE;
+  if (s->super) return SPION_ERR_UNSUPPORTED;
+  if (c->nnzb == 0) return SPION_ERR_SHAPE;
+  return recompute_backward(c, s, Q, K, V, O, dO, stat, keypad, dQ, dK, dV, true);
 }
 
 int tc_engine_mean_map(spion_ctx* c, const void* Q, const void* K, const float* lse, const float* keypad, float* A) {

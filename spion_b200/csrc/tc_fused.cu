@@ -77,13 +77,16 @@ __device__ __forceinline__ void store_row_swizzled(uint32_t tile, int i, const u
 // product reads): rows of one chunk are rescaled in place once the denominator is known; longer rows accumulate it on
 // line in pass A.
 // heads: 0 = operands [BH, L, D]; H = operands [B, L, H, D] (see op_pos).
-// KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of every loop).
+// stat, or null: what P of a row are made of, [BH*L] exponents h, then [BH*L] factors f:
+// P = bf16(bf16(exp2(s scale log2e - penalty - h)) f), the factor as two bf16 values (row_factor), so that tc_bwd_stream.cu rebuilds P bit by bit.
+// store: write the P tiles.  KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of
+// every loop).
 template <int D, bool SUB, bool KP>
 __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_constant__ CUtensorMap tmQ,
                                                               const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV,
                                                               const __grid_constant__ CUtensorMap tmP,
-                                                              __nv_bfloat16* __restrict__ O, float* __restrict__ lse_out,
+                                                              __nv_bfloat16* __restrict__ O, float* __restrict__ lse_out, float* __restrict__ stat, bool store,
                                                               const float* __restrict__ keypad,
                                                               const int4* __restrict__ row_info,
                                                               const int* __restrict__ col_idx,
@@ -361,14 +364,14 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       if (last) mma_commit(bar_o);
       }
       __syncwarp();
-      if (lane == 0) {                                              // these tiles are final: store them now
+      if (store && lane == 0) {                                     // these tiles are final: store them now
         for (int t = 0; t < nt; ++t)
           tma_store_2d(&tmP, sP + (b0 + t) * VT_BYTES, 0, (int)(((size_t)bh * nnzb + rp + t0 + t) * BS));
         bulk_commit();
       }
       return true;
     };
-    float lse_fixed = 0.f;
+    float lse_fixed = 0.f, factor = 1.0f;
     auto finish_stats = [&]() {
       m2 = fmaxf(m2, mraw * sc2);
       m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, 16));        // both owners of a row agree
@@ -422,17 +425,16 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
             }
           }
           const float l = l_part + __shfl_xor_sync(0xffffffffu, l_part, 16) + (float)(L - n_sel) * exp2f(-m2);
-          // 1/l as a sum of two bf16 values: the packed product then carries one rounding of the result only
-          const float inv = 1.0f / l;
-          const float inv_h = bf16_hi(pack_bf16(0.f, inv));
-          const uint32_t inv_hi = pack_bf16(inv_h, inv_h), inv_lo = pack_bf16(inv - inv_h, inv - inv_h);
+          factor = 1.0f / l;
+          uint32_t inv_hi, inv_lo;
+          row_factor(factor, inv_hi, inv_lo);
           lse_fixed = m2 + log2f(l);
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
             const int t = 2 * p + hf;
             if (t < nblk) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) wp[p][j] = fma_bf16x2(wp[p][j], inv_hi, mul_bf16x2(wp[p][j], inv_lo));
+              for (int j = 0; j < 32; ++j) wp[p][j] = times_factor(wp[p][j], inv_hi, inv_lo);
               store_row_swizzled(sP + t * VT_BYTES, row, wp[p]);
             }
           }
@@ -503,7 +505,11 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
     // ------------------------------------------------------------------ output rows of this unit
     if (ok && !ctl) {
       const float lse2 = nblk == 0 ? m2 + log2f((float)L * exp2f(-m2)) : lse_fixed;
-      if (hf == 0) lse_out[(size_t)bh * L + r * BS + row] = lse2;
+      if (hf == 0) {
+        const size_t i = (size_t)bh * L + r * BS + row;
+        lse_out[i] = lse2;
+        if (stat) { stat[i] = m2; stat[(size_t)BH * L + i] = factor; }        // long rows: m2 is the log-sum-exp
+      }
       // the accumulator rows sit in lanes 0-15 of every quadrant: those lanes write the whole row
       __nv_bfloat16* dst = O + (size_t)(pos.row0 + r * BS + row) * pos.ld + pos.x0;
 #pragma unroll
@@ -576,7 +582,7 @@ int fused_set_attrs(TcState* s, int d, int device) { return d == 64 ? fwd_attrs<
 
 template <int D>
 static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const float* keypad,
-                      void* O, float* lse, void* P64) {
+                      void* O, float* lse, void* P64, float* stat) {
   const TcView vw = tc_view(c, s);
   const uint64_t vrows = (uint64_t)c->BH * vw.nnzb * BS;
   CUtensorMap mq, mk, mv, mp;
@@ -592,8 +598,8 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
   // than the pipelining gains (measured at 5 % density, L = 4096: 79 us split against 70 us in one launch).  Without P that is the
   // streaming kernel (tc_fwd_stream.cu; the full mask: tc_fwd_exact.cu), with P this file's, whose probabilities are rounded after the normalisation.
   if (s->n_long == 0) {
-    if ((rc = pipe_forward(c, s, mq, mk, mv, mp, P64 != nullptr, keypad, O, lse, 0))) return rc;
-  } else if (!P64) {
+    if ((rc = pipe_forward(c, s, mq, mk, mv, mp, P64 != nullptr, stat, keypad, O, lse, 0))) return rc;
+  } else if (!P64 && !stat) {
     rc = c->nnzb == c->nb * c->nb ? exact_forward(c, s, mq, mk, mv, keypad, O, lse) : stream_forward(c, s, mq, mk, mv, keypad, O, lse);
     if (rc) return rc;
   } else {
@@ -601,7 +607,7 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
     const float floor_v = keypad ? 0.0f : -100.0f;
     const int grid = (int)(total < cap ? total : cap);
     auto launch = [&](auto k) {
-      k<<<grid, FWD_THREADS, fwd_smem_bytes<D>(), c->stream>>>(mq, mk, mv, mp, (__nv_bfloat16*)O, lse, keypad, vw.row_info, vw.col_idx,
+      k<<<grid, FWD_THREADS, fwd_smem_bytes<D>(), c->stream>>>(mq, mk, mv, mp, (__nv_bfloat16*)O, lse, stat, P64 != nullptr, keypad, vw.row_info, vw.col_idx,
                                                               vw.submask, c->L, vw.nnzb, c->BH, vw.nb, c->heads, c->scale, floor_v,
                                                               c->status_dev);
     };
@@ -615,9 +621,9 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
 }
 
 int fused_forward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const float* keypad, void* O,
-                  float* lse, void* P64_optional) {
-  return c->d == 64 ? fwd_launch<64>(c, s, Q, K, V, keypad, O, lse, P64_optional)
-                    : fwd_launch<32>(c, s, Q, K, V, keypad, O, lse, P64_optional);
+                  float* lse, void* P64_optional, float* stat) {
+  return c->d == 64 ? fwd_launch<64>(c, s, Q, K, V, keypad, O, lse, P64_optional, stat)
+                    : fwd_launch<32>(c, s, Q, K, V, keypad, O, lse, P64_optional, stat);
 }
 
 }  // namespace tc

@@ -53,13 +53,14 @@ __device__ __forceinline__ void store_half_row(uint32_t tile, int i, int g, cons
   }
 }
 
+// STORE_P: P normalised before it is rounded, and stored (unless `store` is false); stat: see k_fwd_fused.
 // KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of every loop).
 template <int D, bool STORE_P, bool SUB, bool KP>
 __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_constant__ CUtensorMap tmQ,
                                                               const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV,
                                                               const __grid_constant__ CUtensorMap tmP,
-                                                              __nv_bfloat16* __restrict__ O, float* __restrict__ lse_out,
+                                                              __nv_bfloat16* __restrict__ O, float* __restrict__ lse_out, float* __restrict__ stat, bool store,
                                                               const float* __restrict__ keypad,
                                                               const int4* __restrict__ row_info,
                                                               const int* __restrict__ col_idx,
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
         // With a separate P buffer (D == 32) the math warps overwrite it as soon as they see bar_o: when the tiles
         // are also stored, bar_o must then wait for the stores' reads as well (see below).
         mma_commit((STORE_P && D != 64) ? bar_x : bar_o + 8 * s);
-        if (STORE_P) {
+        if (STORE_P && store) {
           for (int t = 0; t < R.nblk; ++t)
             tma_store_2d(&tmP, sP(s, t), 0, (int)(((size_t)bh * nnzb + R.rp + t) * BS));
           bulk_commit();
@@ -396,10 +397,14 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
         const float l = l_part + __shfl_xor_sync(0xffffffffu, l_part, 16) + (float)(L - n_sel) * exp2f(-m2);
         lse2 = m2 + log2f(l);
         if (STORE_P) {
-          // 1/l as a sum of two bf16 values: the packed product then carries one rounding of the result only
           const float il = 1.0f / l;
-          const float il_h = bf16_hi(pack_bf16(0.f, il));
-          const uint32_t inv_hi = pack_bf16(il_h, il_h), inv_lo = pack_bf16(il - il_h, il - il_h);
+          uint32_t inv_hi, inv_lo;
+          row_factor(il, inv_hi, inv_lo);
+          if (stat && hf == 0) {
+            const size_t x = (size_t)bh * L + R.r * BS + row;
+            stat[x] = m2;
+            stat[(size_t)BH * L + x] = il;
+          }
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
             const int t = 2 * p + hf;
@@ -409,8 +414,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
                 uint32_t w16[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                  const uint32_t x = wp[p][half * 16 + j];
-                  w16[j] = fma_bf16x2(x, inv_hi, mul_bf16x2(x, inv_lo));
+                  w16[j] = times_factor(wp[p][half * 16 + j], inv_hi, inv_lo);
                 }
                 store_half_row(sP(s, t), row, half, w16);
               }
@@ -474,7 +478,7 @@ int pipe_set_attrs(TcState* s, int d, int device) { return d == 64 ? pipe_attrs<
 
 template <int D>
 static int pipe_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                       const CUtensorMap& mp, bool store_p, const float* keypad, void* O, float* lse, int rank0) {
+                       const CUtensorMap& mp, bool store_p, float* stat, const float* keypad, void* O, float* lse, int rank0) {
   const TcView vw = tc_view(c, s);
   const long long total = (long long)c->BH * (vw.nb - rank0);
   if (total <= 0) return SPION_OK;
@@ -483,10 +487,10 @@ static int pipe_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CU
   const float floor_v = keypad ? 0.0f : -100.0f;
 #define SPION_PIPE_LAUNCH(SP, SB, KP)                                                                                    \
   k_fwd_pipe<D, SP, SB, KP><<<grid, PIPE_THREADS, pipe_smem_bytes<D>(), c->stream>>>(                                     \
-      mq, mk, mv, mp, (__nv_bfloat16*)O, lse, keypad, vw.row_info, vw.col_idx, vw.submask, c->L, vw.nnzb, c->BH, rank0, \
+      mq, mk, mv, mp, (__nv_bfloat16*)O, lse, stat, store_p, keypad, vw.row_info, vw.col_idx, vw.submask, c->L, vw.nnzb, c->BH, rank0, \
       vw.nb, c->heads, c->scale, floor_v, c->status_dev)
 #define SPION_PIPE_PICK(SP, SB) do { if (keypad) SPION_PIPE_LAUNCH(SP, SB, true); else SPION_PIPE_LAUNCH(SP, SB, false); } while (0)
-  if (store_p) { if (vw.submask) SPION_PIPE_PICK(true, true); else SPION_PIPE_PICK(true, false); }
+  if (store_p || stat) { if (vw.submask) SPION_PIPE_PICK(true, true); else SPION_PIPE_PICK(true, false); }
   else { if (vw.submask) SPION_PIPE_PICK(false, true); else SPION_PIPE_PICK(false, false); }
 #undef SPION_PIPE_PICK
 #undef SPION_PIPE_LAUNCH
@@ -496,9 +500,9 @@ static int pipe_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CU
 }
 
 int pipe_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                 const CUtensorMap& mp, bool store_p, const float* keypad, void* O, float* lse, int rank0) {
-  return c->d == 64 ? pipe_launch<64>(c, s, mq, mk, mv, mp, store_p, keypad, O, lse, rank0)
-                    : pipe_launch<32>(c, s, mq, mk, mv, mp, store_p, keypad, O, lse, rank0);
+                 const CUtensorMap& mp, bool store_p, float* stat, const float* keypad, void* O, float* lse, int rank0) {
+  return c->d == 64 ? pipe_launch<64>(c, s, mq, mk, mv, mp, store_p, stat, keypad, O, lse, rank0)
+                    : pipe_launch<32>(c, s, mq, mk, mv, mp, store_p, stat, keypad, O, lse, rank0);
 }
 
 }  // namespace tc

@@ -37,6 +37,13 @@ __device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t 
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   return d;
 }
+// A row's factor as a sum of two bf16 values, each twice in a register: the packed product with it carries one rounding of the result only.
+__device__ __forceinline__ void row_factor(float f, uint32_t& hi, uint32_t& lo) {
+  const float h = __uint_as_float(pack_bf16(0.f, f) & 0xffff0000u);
+  hi = pack_bf16(h, h);
+  lo = pack_bf16(f - h, f - h);
+}
+__device__ __forceinline__ uint32_t times_factor(uint32_t p, uint32_t hi, uint32_t lo) { return fma_bf16x2(p, hi, mul_bf16x2(p, lo)); }
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
@@ -246,7 +253,7 @@ inline int make_operand_map(const spion_ctx* c, TcState* s, CUtensorMap* m, cons
 int stream_backward_set_attrs(int d);
 int stream_prepare(spion_ctx* c, TcState* s);              // pattern set: line and pair records of the streaming kernels
 int recompute_backward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const void* O,
-                       const void* dO, const float* lse, const float* keypad, void* dQ, void* dK, void* dV);
+                       const void* dO, const float* lse, const float* keypad, void* dQ, void* dK, void* dV, bool rounded);
 // tc_recompute.cu
 int mean_map_set_attrs(int d);
 int recompute_mean_map(spion_ctx* c, TcState* s, const void* Q, const void* K, const float* lse, const float* keypad,
@@ -265,7 +272,7 @@ int exact_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtenso
 // tc_fwd_pipe.cu: forward of the records [rank0, nb) of row_info (rows of at most ROW_NCH blocks)
 int pipe_set_attrs(TcState* s, int d, int device);
 int pipe_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                 const CUtensorMap& mp, bool store_p, const float* keypad, void* O, float* lse, int rank0);
+                 const CUtensorMap& mp, bool store_p, float* stat, const float* keypad, void* O, float* lse, int rank0);
 
 // tc_b32.cu: masks of 32-wide blocks on the blocks themselves (bf16, head_dim 64; no stored P)
 bool b32_applies(const spion_ctx* c);
@@ -280,6 +287,6 @@ int b32_backward(spion_ctx* c, TcState* s, const void* Q, const void* K, const v
 // tc_fused.cu
 int fused_set_attrs(TcState* s, int d, int device);
 int fused_forward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const float* keypad, void* O,
-                  float* lse, void* P64_optional);
+                  float* lse, void* P64_optional, float* stat);
 
 }  // namespace tc

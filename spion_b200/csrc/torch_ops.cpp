@@ -194,6 +194,7 @@ struct Context {
   int64_t B = 0, H = 0, L = 0, d = 0;
   int device = 0;
   bool bf16 = false, keypad = false, fused = false, recompute = false, return_probs = true, needs_scratch = false;
+  bool rounded = false;                 // not recompute: rebuilt tiles too, but of the rounded probabilities
   bool owned = false;                   // destroys the handle
   int64_t nnz = 0;                      // selected elements per (b,h) matrix
   Tensor sum_mat, offsets, columns;     // element CSR of the drop-in layout
@@ -265,7 +266,7 @@ Tensor penalty(const Context& c, const Tensor& mask, const Tensor& like, void* s
 
 // One forward call: operands in, results out (everything the backward needs).
 struct Attn {
-  Tensor q, k, v, pen, O, lse, P;
+  Tensor q, k, v, pen, O, lse, P, stat; // stat: what the rounded P are rebuilt from
   int heads = 0;                        // 0: operands [B, H, L, d] contiguous; H: views of [B, L, H, d]
   // the mask the forward ran on (drop-in: as element CSR); the context may move on to another before the backward
   Tensor sum_mat, offsets, columns, mask;
@@ -312,6 +313,13 @@ void attn_forward(Context& c, Attn& a, bool need, void* st) {
   a.O = empty_operand(c, a.heads, a.q);
   if (c.fused) {
     a.lse = at::empty({c.B * c.H * c.L}, f32);
+    if (need && c.rounded && !c.recompute) {
+      a.stat = at::empty({2 * c.B * c.H * c.L}, f32);
+      if (c.return_probs) a.P = at::empty({c.B * c.H * a.nnz}, a.q.options());
+      check(spion_attn_forward_probs(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.O), (float*)a.lse.data_ptr(), p(a.P), (float*)a.stat.data_ptr()),
+            "spion_attn_forward_probs");
+      return;
+    }
     // the probabilities are stored only for callers that want them back and for a backward that reads them
     if (c.return_probs || (need && !c.recompute)) a.P = at::empty({c.B * c.H * a.nnz}, a.q.options());
     check(spion_attn_forward_fused(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.O), (float*)a.lse.data_ptr(), p(a.P)),
@@ -370,6 +378,11 @@ void attn_backward_on(const Context& c, const Attn& a, const Tensor& dO, Tensor&
     return;
   }
   check(spion_set_head_layout(x, a.heads), "spion_set_head_layout");
+  if (a.stat.defined()) {
+    check(spion_attn_backward_probs(x, p(a.q), p(a.k), p(a.v), p(a.O), p(dO), pf(a.stat), pf(a.pen), p(dq), p(dk), p(dv)),
+          "spion_attn_backward_probs");
+    return;
+  }
   if (c.fused && !a.P.defined()) {
     check(spion_attn_backward_fused(x, p(a.q), p(a.k), p(a.v), p(a.O), p(dO), pf(a.lse), pf(a.pen), p(dq), p(dk), p(dv)),
           "spion_attn_backward_fused");
@@ -387,12 +400,13 @@ SavedVariable save(const Tensor& t) { return SavedVariable(t, false); }
 // What a backward reads of its forward, as saved variables: a tensor that a caller also holds (the output, the probabilities) is
 // checked for changes since, and hooks on saved tensors see all of them.
 struct SavedAttn {
-  SavedVariable q, k, v, pen, O, lse, P, sum_mat, offsets, columns;
+  // P is saved beside stat as well: a change of what the caller holds is an error
+  SavedVariable q, k, v, pen, O, lse, P, stat, sum_mat, offsets, columns;
   Attn rest;
   // q_in, k_in, v_in: the caller's tensors where the kernels read them in place, else what a holds
   void save_all(const Attn& a, const Tensor& q_in, const Tensor& k_in, const Tensor& v_in) {
     q = save(q_in); k = save(k_in); v = save(v_in);
-    pen = save(a.pen); O = save(a.O); lse = save(a.lse); P = save(a.P);
+    pen = save(a.pen); O = save(a.O); lse = save(a.lse); P = save(a.P); stat = save(a.stat);
     sum_mat = save(a.sum_mat); offsets = save(a.offsets); columns = save(a.columns);
     rest.heads = a.heads; rest.mask = a.mask; rest.nnz = a.nnz; rest.generation = a.generation;
   }
@@ -406,12 +420,12 @@ struct SavedAttn {
     };
     auto values = [](const SavedVariable& s) { Tensor t = s.unpack(); return t.defined() ? t.contiguous() : t; };
     a.q = operand(q); a.k = operand(k); a.v = operand(v); a.O = operand(O);
-    a.pen = values(pen); a.lse = values(lse); a.P = values(P);
+    a.pen = values(pen); a.lse = values(lse); a.P = values(P); a.stat = values(stat);
     a.sum_mat = values(sum_mat); a.offsets = values(offsets); a.columns = values(columns);
     return a;
   }
   void reset() {
-    for (SavedVariable* s : {&q, &k, &v, &pen, &O, &lse, &P, &sum_mat, &offsets, &columns}) s->reset_data();
+    for (SavedVariable* s : {&q, &k, &v, &pen, &O, &lse, &P, &stat, &sum_mat, &offsets, &columns}) s->reset_data();
     rest = Attn();
   }
 };
@@ -902,7 +916,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("B", &Context::B).def_readwrite("H", &Context::H).def_readwrite("L", &Context::L).def_readwrite("d", &Context::d)
       .def_readwrite("device", &Context::device)
       .def_readwrite("bf16", &Context::bf16).def_readwrite("keypad", &Context::keypad).def_readwrite("fused", &Context::fused)
-      .def_readwrite("recompute", &Context::recompute).def_readwrite("return_probs", &Context::return_probs)
+      .def_readwrite("recompute", &Context::recompute).def_readwrite("rounded", &Context::rounded).def_readwrite("return_probs", &Context::return_probs)
       .def_readwrite("needs_scratch", &Context::needs_scratch).def_readwrite("owned", &Context::owned)
       .def_readwrite("nnz", &Context::nnz)
       .def_readwrite("sum_mat", &Context::sum_mat).def_readwrite("offsets", &Context::offsets).def_readwrite("columns", &Context::columns);

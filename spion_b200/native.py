@@ -115,6 +115,8 @@ class BlockSparseAttention(nn.Module):
         self.nnzb = int(lib.spion_pattern_nnzb(self.handle))
         if self.fused and self._recompute_arg is None:
             self.recompute = self._recompute_pays()
+            # the gradients of stored tiles, without storing them: 64-wide blocks
+            self._ctx.rounded = not self.recompute
         from .pattern import pattern_from_mask
         self._pattern = pattern_from_mask(m8, self.bs)          # block CSR for the helpers above
         self._mask_key.set(mat)

@@ -319,3 +319,35 @@ def test_streaming_kernels_with_penalties_of_every_kind(d, bs, full):
         assert far(a[:2], b[:2], True) <= BF16_REL, f"{name}: {far(a[:2], b[:2], True):.3e}"
     if not full:                                             # unselected keys count as score 0 and leave nothing to the padded ones
         assert not got[0][2].any() and not got[3][2].any()
+
+
+@pytest.mark.parametrize("d", [32, 64])
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("short", [False, True])
+@pytest.mark.parametrize("probs", [False, True])
+def test_rebuilt_rounded_tiles_are_the_stored_ones(d, padded, short, probs):
+    """Gradients without stored tiles, bit for bit: rows of up to four blocks (normalised after a rounding) and longer ones (before it), masks
+    of short rows only, blocks with no, one and different penalties, odd last pairs, lines without blocks."""
+    from spion_b200.native import BlockSparseAttention
+    B, H, nb = 2, 3, 11
+    L = nb * 64
+    Q, K, V, dO = (t.to(torch.bfloat16) for t in synthetic.qkv(47 + d, B, H, L, d))
+    mat = lines_of_every_length(nb)
+    if short:
+        mat = np.triu(mat, -3)
+    kp = synthetic.key_padding(5, B, L) if padded else None
+    got = []
+    for recompute in (None, False):
+        mod = BlockSparseAttention(cfg(B, H, L, d, 64), dtype=torch.bfloat16, keypad=padded, recompute=recompute, return_probs=probs)
+        mod.set_mask(torch.as_tensor(mat).cuda())
+        if recompute is None:                                # what calls with probabilities, and small ones at head_dim 32, do
+            mod.recompute, mod._ctx.rounded = False, True
+        n0 = mod.launch_count()
+        q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+        out, _ = mod(q, k, v, None if kp is None else kp.cuda())
+        got.append((out,) + torch.autograd.grad(out, (q, k, v), dO.cuda()))
+        mod.check_device_status()
+        assert mod.launch_count() - n0 == 3                  # forward, rows, columns
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), *got):
+        assert torch.equal(a, b), f"{name}: {far(a, b, True):.3e}"
+    compare(got[0], Q, K, V, dO, mat, 64, kp, BF16_REL, True)
