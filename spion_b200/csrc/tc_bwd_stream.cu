@@ -622,7 +622,9 @@ static int bw_launch_one(spion_ctx* c, TcState* s, const CUtensorMap& a0, const 
                      const BwArgs& a) {
   using C = Bw<D, SIDE>;
   static_assert(C::SMEM <= 227 * 1024, "shared memory");
-  auto k = k_bwd_stream<D, SIDE, SUB, KP, RND>;
+  constexpr auto k = k_bwd_stream<D, SIDE, SUB, KP, RND>;
+  int rc = allow_smem<k>(c->device, C::SMEM);
+  if (rc) return rc;
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
   k<<<grid, BW_THREADS, C::SMEM, c->stream>>>(a0, a1, f0, f1, a);
@@ -640,15 +642,22 @@ static int bw_launch(spion_ctx* c, TcState* s, const CUtensorMap& a0, const CUte
   return a.keypad ? bw_launch_one<D, SIDE, false, true, false>(c, s, a0, a1, f0, f1, a) : bw_launch_one<D, SIDE, false, false, false>(c, s, a0, a1, f0, f1, a);
 }
 
-template <int D>
-static int bw_attrs() {
-  for (auto k : {k_bwd_stream<D, ROW, false, false, false>, k_bwd_stream<D, ROW, true, false, false>, k_bwd_stream<D, ROW, false, true, false>, k_bwd_stream<D, ROW, true, true, false>, k_bwd_stream<D, ROW, false, false, true>, k_bwd_stream<D, ROW, false, true, true>})
-    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, ROW>::SMEM));
-  for (auto k : {k_bwd_stream<D, COL, false, false, false>, k_bwd_stream<D, COL, true, false, false>, k_bwd_stream<D, COL, false, true, false>, k_bwd_stream<D, COL, true, true, false>, k_bwd_stream<D, COL, false, false, true>, k_bwd_stream<D, COL, false, true, true>})
-    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Bw<D, COL>::SMEM));
-  return SPION_OK;
+template <int D, bool SUB, bool KP, bool RND>
+static int bw_attrs(int device) {
+  const int rc = allow_smem<k_bwd_stream<D, ROW, SUB, KP, RND>>(device, Bw<D, ROW>::SMEM);
+  return rc ? rc : allow_smem<k_bwd_stream<D, COL, SUB, KP, RND>>(device, Bw<D, COL>::SMEM);
 }
-int stream_backward_set_attrs(int d) { return d == 64 ? bw_attrs<64>() : bw_attrs<32>(); }
+template <int D, bool KP>
+static int bw_attrs_of(const spion_ctx* c) {
+  if (c->bs == 32) return bw_attrs<D, true, KP, false>(c->device);
+  const int rc = bw_attrs<D, false, KP, false>(c->device);
+  return rc ? rc : bw_attrs<D, false, KP, true>(c->device);
+}
+int stream_backward_set_attrs(const spion_ctx* c) {
+  const bool kp = c->kind == SPION_KIND_BLOCK_KPM;
+  if (c->d == 64) return kp ? bw_attrs_of<64, true>(c) : bw_attrs_of<64, false>(c);
+  return kp ? bw_attrs_of<32, true>(c) : bw_attrs_of<32, false>(c);
+}
 
 int stream_prepare(spion_ctx* c, TcState* s) {
   const TcView vw = tc_view(c, s);

@@ -748,24 +748,24 @@ bool tc_engine_supports(const spion_ctx* c) {
          (unsigned long long)c->BH * c->L < 0x7fffffffULL;
 }
 
-// Shared-memory opt-ins and resident CTAs of all kernels, once per device and head dimension of the process (about 60 attribute
-// calls, a millisecond: every layer of a model has a context of its own).  The calls also load the kernels, so that the first pass of
+// Shared-memory opt-ins and resident CTAs of the kernels, once per device, head dimension, block size and kind of context in a process (some
+// 40 attribute calls, a millisecond: every layer of a model has a context of its own).  The calls also load the kernels, so that the first pass of
 // a module does not.
 static int kernel_attrs(spion_ctx* c, TcState* s) {
   struct Known { bool have = false; int fwd, row, col, pipe, b32[3]; };
   static std::mutex mutex;
-  static Known known[64][2][2];                                    // device, head dimension, 32-wide blocks
+  static Known known[64][2][2][2];                                 // device, head dimension, block size, key padding
   const bool b32 = b32_applies(c);
   std::lock_guard<std::mutex> lock(mutex);
-  Known fresh, *k = c->device < 64 ? &known[c->device][c->d == 64][b32] : &fresh;
+  Known fresh, *k = c->device < 64 ? &known[c->device][c->d == 64][c->bs == 32][c->kind == SPION_KIND_BLOCK_KPM] : &fresh;
   if (!k->have) {
     int rc = (c->d == 64) ? set_attrs<64>(s, c->device) : set_attrs<32>(s, c->device);
     if (!rc) rc = fused_set_attrs(s, c->d, c->device);
     if (!rc) rc = mean_map_set_attrs(c->d);
     if (!rc) rc = pipe_set_attrs(s, c->d, c->device);
-    if (!rc) rc = stream_forward_set_attrs(c->d);
+    if (!rc) rc = stream_forward_set_attrs(c);
     if (!rc) rc = exact_forward_set_attrs(c->d);
-    if (!rc) rc = stream_backward_set_attrs(c->d);
+    if (!rc) rc = stream_backward_set_attrs(c);
     if (!rc && b32) rc = b32_set_attrs(s, c->device);
     if (rc) return rc;
     k->fwd = s->fwd_ctas; k->row = s->row_ctas; k->col = s->col_ctas; k->pipe = s->pipe_ctas;

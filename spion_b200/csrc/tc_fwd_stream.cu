@@ -418,7 +418,9 @@ template <int D, bool KP, bool SUB>
 static int fs_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FsArgs& a) {
   using C = Fs<D>;
   static_assert(C::SMEM <= 227 * 1024 && C::NG * C::COLS <= 512, "shared or tensor memory");
-  auto k = k_fwd_stream<D, KP, SUB>;
+  constexpr auto k = k_fwd_stream<D, KP, SUB>;
+  int rc = allow_smem<k>(c->device, C::SMEM);
+  if (rc) return rc;
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
   k<<<grid, C::THREADS, C::SMEM, c->stream>>>(mq, mk, mv, a);
@@ -442,12 +444,12 @@ static int fs_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUt
 }
 
 template <int D>
-static int fs_attrs() {
-  for (auto k : {k_fwd_stream<D, false, false>, k_fwd_stream<D, true, false>, k_fwd_stream<D, false, true>, k_fwd_stream<D, true, true>})
-    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Fs<D>::SMEM));
-  return SPION_OK;
+static int fs_attrs(const spion_ctx* c) {
+  if (c->kind == SPION_KIND_BLOCK_KPM)
+    return c->bs == 32 ? allow_smem<k_fwd_stream<D, true, true>>(c->device, Fs<D>::SMEM) : allow_smem<k_fwd_stream<D, true, false>>(c->device, Fs<D>::SMEM);
+  return c->bs == 32 ? allow_smem<k_fwd_stream<D, false, true>>(c->device, Fs<D>::SMEM) : allow_smem<k_fwd_stream<D, false, false>>(c->device, Fs<D>::SMEM);
 }
-int stream_forward_set_attrs(int d) { return d == 64 ? fs_attrs<64>() : fs_attrs<32>(); }
+int stream_forward_set_attrs(const spion_ctx* c) { return c->d == 64 ? fs_attrs<64>(c) : fs_attrs<32>(c); }
 
 int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
                    float* lse) {

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -242,6 +244,16 @@ inline int resident_ctas(K kernel, int device, int threads, size_t dyn_smem, int
   return SPION_OK;
 }
 
+// Lets kernel K use `bytes` of shared memory on a device, once; also loads the kernel.
+template <auto K>
+inline int allow_smem(int device, size_t bytes) {
+  static std::atomic<bool> done[64];
+  if (device < 64 && done[device].load(std::memory_order_acquire)) return SPION_OK;
+  SPION_CUDA_TRY(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (device < 64) done[device].store(true, std::memory_order_release);
+  return SPION_OK;
+}
+
 // Map over one dense operand (Q, K, V, dO): [BH*L, D] rows, or [B*L, H*D] rows with a [64 x D] box at
 // column h*D when the context's operands are in the merged-head form.
 inline int make_operand_map(const spion_ctx* c, TcState* s, CUtensorMap* m, const void* base, int D) {
@@ -250,7 +262,7 @@ inline int make_operand_map(const spion_ctx* c, TcState* s, CUtensorMap* m, cons
 }
 
 // tc_bwd_stream.cu
-int stream_backward_set_attrs(int d);
+int stream_backward_set_attrs(const spion_ctx* c);         // loads the kernels that the context's calls use
 int stream_prepare(spion_ctx* c, TcState* s);              // pattern set: line and pair records of the streaming kernels
 int recompute_backward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const void* O,
                        const void* dO, const float* lse, const float* keypad, void* dQ, void* dK, void* dV, bool rounded);
@@ -260,7 +272,7 @@ int recompute_mean_map(spion_ctx* c, TcState* s, const void* Q, const void* K, c
                        float* A);
 
 // tc_fwd_stream.cu: forward without stored probabilities
-int stream_forward_set_attrs(int d);
+int stream_forward_set_attrs(const spion_ctx* c);
 int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
                    float* lse);
 
