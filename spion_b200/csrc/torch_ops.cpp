@@ -7,6 +7,7 @@
 //
 // Only orchestration lives here; every kernel is behind the C ABI.
 #include <torch/extension.h>
+#include <ATen/SavedTensorHooks.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/jit/frontend/tracer.h>
@@ -313,7 +314,8 @@ void attn_forward(Context& c, Attn& a, bool need, void* st) {
   a.O = empty_operand(c, a.heads, a.q);
   if (c.fused) {
     a.lse = at::empty({c.B * c.H * c.L}, f32);
-    if (need && c.rounded && !c.recompute) {
+    // under hooks on saved tensors the backward reads the P that they hand back
+    if (need && c.rounded && !c.recompute && !at::SavedTensorDefaultHooks::get_hooks()) {
       a.stat = at::empty({2 * c.B * c.H * c.L}, f32);
       if (c.return_probs) a.P = at::empty({c.B * c.H * a.nnz}, a.q.options());
       check(spion_attn_forward_probs(x, p(a.q), p(a.k), p(a.v), pf(a.pen), p(a.O), (float*)a.lse.data_ptr(), p(a.P), (float*)a.stat.data_ptr()),

@@ -351,3 +351,23 @@ def test_rebuilt_rounded_tiles_are_the_stored_ones(d, padded, short, probs):
     for name, a, b in zip(("O", "dQ", "dK", "dV"), *got):
         assert torch.equal(a, b), f"{name}: {far(a, b, True):.3e}"
     compare(got[0], Q, K, V, dO, mat, 64, kp, BF16_REL, True)
+
+
+@pytest.mark.parametrize("d", [32, 64])
+def test_gradients_read_the_probabilities_that_a_hook_hands_back(d):
+    """A hook on saved tensors that gives halved probabilities to the backward halves dV: exact in bf16."""
+    from spion_b200.native import BlockSparseAttention
+    B, H, nb = 1, 2, 5
+    L = nb * 64
+    Q, K, V, dO = (t.to(torch.bfloat16).cuda() for t in synthetic.qkv(53 + d, B, H, L, d))
+    mod = BlockSparseAttention(cfg(B, H, L, d, 64), dtype=torch.bfloat16, keypad=False, return_probs=True)
+    mod.set_mask(torch.as_tensor(np.triu(np.ones((nb, nb), dtype=np.int64))).cuda())
+    got = []
+    for factor in (1.0, 0.5):
+        def hand_back(t, factor=factor):
+            return t * factor if t.dtype == torch.bfloat16 and t.numel() == B * H * mod.nnz else t
+        q, k, v = (t.clone().requires_grad_(True) for t in (Q, K, V))
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, hand_back):
+            out, _ = mod(q, k, v, None)
+        got.append(torch.autograd.grad(out, v, dO)[0])
+    assert torch.equal(got[1], got[0] * 0.5)
