@@ -123,6 +123,25 @@ static inline Pattern ctx_pattern(const spion_ctx* c) {
     }                                                                                 \
   } while (0)
 
+// Kernels that follow one another in one call.  The first says at its start that the next may be placed beside it (no CTA of the next starts
+// before all of the first run, so none is kept waiting), the next is launched by launch_after and waits for the first, with all it has
+// written, before it touches global memory: its launch and its own preparation are hidden.  What it reads then must not be declared read-only
+// (const __restrict__), or the compiler may move the reads ahead of the wait.  Measured: column sums of 16384 rows with their reduction 4.4 -> 3.9 us
+// a call in a graph, on the host 11.1 -> 10.5; a training step of 156 kernels about 2 %; an attention layer on a full mask 257 -> 252 us.
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 // api.cu: multiprocessors of the current device (0: the query failed)
 int sm_count();
 

@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_bwd_kernel(const float* __re
                                                                __nv_bfloat16* __restrict__ dx_bf16) {
   // dskip != nullptr: dx = (gradient through the normalisation) + dskip, the gradient that reaches the same row
   // through the residual connection; dx_bf16 != nullptr: a bf16 copy of dx (the gradient of a bf16 branch output)
+  next_may_start();                                                    // ln_bwd_reduce_kernel
   constexpr int N = 64 * K;
   __shared__ float s_g[LN_WARPS][N], s_b[LN_WARPS][N];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -163,12 +164,13 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_bwd_kernel(const float* __re
 // dgamma[c] = sum over the partial rows; likewise dbeta.  One CTA of 32 warps per 32 columns: warp w adds the
 // rows w, w + 32, ... of its columns (coalesced), then the 32 per-warp sums are added in warp order: the order
 // of the additions is fixed, so the result does not depend on the run.
-__global__ void __launch_bounds__(1024) ln_bwd_reduce_kernel(const float* __restrict__ partial, int rows, int N,
+__global__ void __launch_bounds__(1024) ln_bwd_reduce_kernel(const float* partial, int rows, int N,
                                                               float* __restrict__ dgamma, float* __restrict__ dbeta) {
   __shared__ float s_p[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;                      // column of the [rows, 2 N] partial matrix
   float s = 0.f;
+  wait_for_kernel_before();
   for (int r = warp; r < rows; r += 32) s += partial[(size_t)r * 2 * N + c];
   s_p[warp][lane] = s;
   __syncthreads();
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(1024) ln_bwd_reduce_kernel(const float* __rest
 template <int K, bool BF16>
 __global__ void __launch_bounds__(LN_WARPS * 32) colsum_kernel(const void* __restrict__ dy, float* __restrict__ partial,
                                                                 long long M) {
+  next_may_start();                                                    // colsum_reduce_kernel
   constexpr int N = 64 * K;
   __shared__ float s_b[LN_WARPS][N];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) colsum_kernel(const void* __res
 
 // out[c] = sum over the partial rows of an [rows, N] matrix, fixed order (see ln_bwd_reduce_kernel)
 // (blockIdx.y: one of several matrices, partial rows and results one after another)
-__global__ void __launch_bounds__(1024) colsum_reduce_kernel(const float* __restrict__ partial, int rows, int N,
+__global__ void __launch_bounds__(1024) colsum_reduce_kernel(const float* partial, int rows, int N,
                                                               float* __restrict__ out) {
   partial += (size_t)blockIdx.y * rows * N;
   out += (size_t)blockIdx.y * N;
@@ -221,6 +224,7 @@ __global__ void __launch_bounds__(1024) colsum_reduce_kernel(const float* __rest
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
+  wait_for_kernel_before();
   for (int r = warp; r < rows; r += 32) s += partial[(size_t)r * N + c];
   s_p[warp][lane] = s;
   __syncthreads();
@@ -265,6 +269,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_bwd4_kernel(const float* __r
                                                                 float* __restrict__ partial, long long M,
                                                                 const float* __restrict__ dskip,
                                                                 __nv_bfloat16* __restrict__ dx_bf16) {
+  next_may_start();                                                    // ln_bwd_reduce_kernel
   constexpr int LPR = N / 4, RPW = 32 / LPR;
   __shared__ float s_g[LN_WARPS * RPW][N], s_b[LN_WARPS * RPW][N];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane % LPR, sub = lane / LPR;
@@ -318,6 +323,7 @@ struct ColumnSumList { const void* p[4]; };
 template <int N, typename T>
 __global__ void __launch_bounds__(LN_WARPS * 32) colsum4_kernel(const __grid_constant__ ColumnSumList list, float* __restrict__ partial,
                                                                 long long M) {
+  next_may_start();                                                    // colsum_reduce_kernel
   const T* __restrict__ dy = static_cast<const T*>(list.p[blockIdx.y]);
   partial += (size_t)blockIdx.y * gridDim.x * N;
   constexpr int PER = 16 / (int)sizeof(T), LPR = N / PER, RPW = 32 / LPR;
@@ -415,8 +421,7 @@ int ln_backward(const float* x, const void* dy, int dy_is_bf16, const float* gam
       ln_bwd4_kernel<128, float><<<grid, LN_WARPS * 32, 0, stream>>>(x, (const float*)dy, gamma, mean, rstd, dx, workspace, M,
                                                                      dskip, dx_bf16);
     SPION_LAUNCH_CHECK();
-    ln_bwd_reduce_kernel<<<2 * N / 32, 1024, 0, stream>>>(workspace, grid, N, dgamma, dbeta);
-    SPION_LAUNCH_CHECK();
+    SPION_CUDA_TRY(launch_after(ln_bwd_reduce_kernel, dim3(2 * N / 32), dim3(1024), 0, stream, workspace, grid, N, dgamma, dbeta));
     return SPION_OK;
   }
 #define SPION_LN_BWD(K)                                                                                              \
@@ -435,8 +440,7 @@ int ln_backward(const float* x, const void* dy, int dy_is_bf16, const float* gam
   }
 #undef SPION_LN_BWD
   SPION_LAUNCH_CHECK();
-  ln_bwd_reduce_kernel<<<2 * N / 32, 1024, 0, stream>>>(workspace, grid, N, dgamma, dbeta);
-  SPION_LAUNCH_CHECK();
+  SPION_CUDA_TRY(launch_after(ln_bwd_reduce_kernel, dim3(2 * N / 32), dim3(1024), 0, stream, workspace, grid, N, dgamma, dbeta));
   return SPION_OK;
 }
 
@@ -503,8 +507,7 @@ extern "C" int spion_column_sums_many(const void* const* dys, int count, int dy_
     else if (dy_is_bf16) colsum4_kernel<128, __nv_bfloat16><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
     else colsum4_kernel<128, float><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
     SPION_LAUNCH_CHECK();
-    colsum_reduce_kernel<<<dim3(N / 32, count), 1024, 0, stream>>>(workspace, grid, N, out);
-    SPION_LAUNCH_CHECK();
+    SPION_CUDA_TRY(launch_after(colsum_reduce_kernel, dim3(N / 32, count), dim3(1024), 0, stream, workspace, grid, N, out));
     return SPION_OK;
   }
 #define SPION_COLSUM(K)                                                                                                        \
@@ -521,8 +524,7 @@ extern "C" int spion_column_sums_many(const void* const* dys, int count, int dy_
     SPION_LAUNCH_CHECK();
   }
 #undef SPION_COLSUM
-  colsum_reduce_kernel<<<dim3(N / 32, count), 1024, 0, stream>>>(workspace, grid, N, out);
-  SPION_LAUNCH_CHECK();
+  SPION_CUDA_TRY(launch_after(colsum_reduce_kernel, dim3(N / 32, count), dim3(1024), 0, stream, workspace, grid, N, out));
   return SPION_OK;
 }
 

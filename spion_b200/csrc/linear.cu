@@ -616,6 +616,7 @@ template <int SPLIT, bool DY_BF16, bool X_BF16>
 __global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(const __grid_constant__ WgradArgs a) {
   constexpr int LOADERS = WG_LOADERS<SPLIT>, ROWS = 4 * LOADERS, XR = 64 / ROWS;       // rows of a pass of all loaders, passes per tile
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  next_may_start();                                                    // k_lin_reduce
   const uint32_t sbase = smem_u32(smem_raw);
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int n0 = blockIdx.y * a.nc, k0 = blockIdx.z * a.kc;
@@ -877,11 +878,12 @@ __global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(c
 }
 
 // out[i] = sum over the CTAs' partial results, in a fixed order: 32 groups of four values x 8 slices of the CTAs per block
-__global__ void __launch_bounds__(256) k_lin_reduce(const float* __restrict__ part, int nparts, long long n, long long nw,
+__global__ void __launch_bounds__(256) k_lin_reduce(const float* part, int nparts, long long n, long long nw,
                                                     float* __restrict__ dW, float* __restrict__ db) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long i = ((long long)blockIdx.x * 32 + lane) * 4;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  wait_for_kernel_before();
   if (i < n) {
     const int per = (nparts + 7) / 8, b0 = w * per, b1 = min(nparts, b0 + per);
 #pragma unroll 10
@@ -1231,7 +1233,6 @@ extern "C" int spion_linear_backward_weight(const spion_tokens* dY, const spion_
   else rc = X->is_bf16 ? launch_wgrad<1, false, true>(a, gx, smem, st) : launch_wgrad<1, false, false>(a, gx, smem, st);
   if (rc) return rc;
   const long long nw = (long long)a.N * a.K, n = nw + a.N;
-  k_lin_reduce<<<(unsigned)((n / 4 + 31) / 32), 256, 0, st>>>(workspace, gx, n, nw, dW, db);
-  SPION_LAUNCH_CHECK();
+  SPION_CUDA_TRY(launch_after(k_lin_reduce, dim3((unsigned)((n / 4 + 31) / 32)), dim3(256), 0, st, workspace, gx, n, nw, dW, db));
   return SPION_OK;
 }

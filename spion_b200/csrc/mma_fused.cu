@@ -835,7 +835,7 @@ __device__ __forceinline__ int long_column(const Pattern& p, int from, int i) {
 struct AfterLaunchBefore {
   bool on;
   __device__ ~AfterLaunchBefore() {
-    if (on) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (on) wait_for_kernel_before();
   }
 };
 
@@ -846,7 +846,7 @@ __global__ void __launch_bounds__(128, (Cfg<BS, D, MT>::RESIDENT)) mma_bwd_col_k
   const int g0 = threadIdx.x / C::NT, t = threadIdx.x % C::NT, lane = t & 31;
   const int bh_raw = blockIdx.y * C::G + g0;
   const bool active = bh_raw < a.BH;
-  if (SHARED) asm volatile("griddepcontrol.launch_dependents;");
+  if (SHARED) next_may_start();
   const AfterLaunchBefore leave{!SHARED && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1};
   if (!SHARED && !active) return;
   const int bh = active ? bh_raw : a.BH - 1;                            // SHARED: the cluster barriers take every thread

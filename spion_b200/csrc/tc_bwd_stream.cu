@@ -138,6 +138,8 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
   const UnitMap um{a.nb, a.BH, a.by_rank};
   constexpr uint32_t ACC = 384u;                                      // three S / dP sets of 128 columns, then the accumulators
 
+  if (SIDE == ROW) next_may_start();                                  // the columns
+  else wait_for_kernel_before();
   if (warp == 0 && lane == 0) {
     int ab = *reinterpret_cast<volatile int*>(a.status);
     if ((sbase & 1023u) != 0u) { report(a.status, ERR_LOAD_WAIT); ab = 1; }
@@ -627,7 +629,8 @@ static int bw_launch_one(spion_ctx* c, TcState* s, const CUtensorMap& a0, const 
   if (rc) return rc;
   const long long total = (long long)c->BH * a.nb;
   const int grid = (int)(total < (long long)s->sms ? total : (long long)s->sms);       // one CTA per SM (all 512 TMEM columns)
-  k<<<grid, BW_THREADS, C::SMEM, c->stream>>>(a0, a1, f0, f1, a);
+  if (SIDE == COL) SPION_CUDA_TRY(launch_after(k, dim3(grid), dim3(BW_THREADS), C::SMEM, c->stream, a0, a1, f0, f1, a));     // after the rows
+  else k<<<grid, BW_THREADS, C::SMEM, c->stream>>>(a0, a1, f0, f1, a);
   SPION_LAUNCH_CHECK();
   c->launches += 1;
   return SPION_OK;

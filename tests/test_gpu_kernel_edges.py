@@ -371,3 +371,48 @@ def test_gradients_read_the_probabilities_that_a_hook_hands_back(d):
             out, _ = mod(q, k, v, None)
         got.append(torch.autograd.grad(out, v, dO)[0])
     assert torch.equal(got[1], got[0] * 0.5)
+
+
+@pytest.mark.parametrize("dtype,d,bs", [(torch.float32, 64, 64), (torch.float32, 32, 32), (torch.bfloat16, 64, 64), (torch.bfloat16, 32, 64)])
+def test_kernels_that_start_beside_the_one_before_under_capture(dtype, d, bs):
+    """Backward kernels that are placed before the kernel ahead of them has ended (fp32: columns with and without a full one; bf16: rows, columns), in
+    a CUDA graph replayed on other values, the bits of eager calls."""
+    from spion_b200.native import BlockSparseAttention
+    B, H, nb = 1, 30, 33
+    L = nb * bs if bs == 64 else nb * 64
+    nb = L // bs
+    rng = np.random.default_rng(61)
+    mat = (rng.random((nb, nb)) < 0.1).astype(np.int64)
+    np.fill_diagonal(mat, 1)
+    mat[:, 5] = 1
+    mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=dtype, keypad=False, return_probs=False)
+    mod.set_mask(torch.as_tensor(mat).cuda())
+    static = [torch.empty(B, H, L, d, dtype=dtype, device="cuda").requires_grad_(i < 3) for i in range(4)]
+
+    def step():
+        out = mod(*static[:3], None)[0]
+        return (out,) + torch.autograd.grad(out, static[:3], static[3])
+
+    def load(seed):
+        with torch.no_grad():
+            for s, t in zip(static, synthetic.qkv(seed, B, H, L, d)):
+                s.copy_(t.to(dtype))
+
+    load(3)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step()
+    for seed in (4, 5):
+        load(seed)
+        for _ in range(3):
+            graph.replay()
+        replayed = [t.clone() for t in got]
+        for a, b in zip(replayed, step()):
+            assert torch.equal(a, b)
+    mod.check_device_status()
