@@ -1,7 +1,7 @@
 // The fp32 forward and backward on a full mask (the dense warm-up phase on the native path).  There the key projection's bias has no
 // effect: its gradient is a sum that cancels to the rounding of its terms, so that every other order of additions gives another
 // gradient.  These kernels keep the order the dense phase has always had (4 x 4 micro-tiles, one sum per output in ascending order,
-// row sums joined tile by tile); masks with unselected blocks run on simt_fused.cu, which is about 1.3 times faster, and so does a
+// row sums joined tile by tile); masks with unselected blocks run on simt_fused.cu or mma_fused.cu, which are at least 1.3 times faster, and so does a
 // backward on a full mask whose caller has no O (the reference's signature): its order is that of simt_fused.cu.
 //
 // Thread layout: a bs x bs tile is computed by (bs/4)^2 threads with 4x4 micro-tiles (rows

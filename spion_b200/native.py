@@ -123,21 +123,20 @@ class BlockSparseAttention(nn.Module):
         return self.nnzb
 
     def _recompute_pays(self) -> bool:
-        """Which backward serves the current mask: from rebuilt tiles (the forward's log-sum-exp, nothing of size nnz in memory unless the
-        caller wants P back) or from stored ones.
+        """Which gradients serve the current mask: those of P as the log-sum-exp gives it (True), or those of the P that is rounded to bf16
+        (False), bit for bit what stored tiles give.  Without a ``recompute`` argument neither reads a stored P or dS: both backward kernels
+        form P again, the second with the two factors per row that the forward leaves beside the log-sum-exp.
 
-        No P returned: rebuilt tiles, which are faster (forward + backward on one B200, us, rebuilt and stored; head_dim 64 and 64 matrices
-        unless stated): L = 4096, 3 % (two blocks per row) 150, 173; 5 % 174, 226; 30 % 581, 924; L = 16384, 5 % 1764, 2882; 512 matrices,
-        L = 1024, two blocks per row 266, 323; 2 matrices, L = 4096, 5 % 82, 86.  head_dim 32: 9 matrices, L = 9472, 12 % 158, 274; 28
-        matrices, L = 6528, 4 % 109, 163; 2 matrices, L = 2048 85, 91.
+        No P returned: the first, whose forward is faster (forward + backward on one B200 when the rule was made, us, against
+        stored tiles; head_dim 64 and 64 matrices unless stated): L = 4096, 3 % (two blocks per row) 150, 173; 5 % 174, 226; 30 % 581, 924;
+        L = 16384, 5 % 1764, 2882; 512 matrices, L = 1024, two blocks per row 266, 323; 2 matrices, L = 4096, 5 % 82, 86.  head_dim 32: 9
+        matrices, L = 9472, 12 % 158, 274; 28 matrices, L = 6528, 4 % 109, 163; 2 matrices, L = 2048 85, 91.
 
-        P returned: stored tiles.  The gradients are those of the very P that the caller holds, and a change of it before the backward is
-        an error.  Rebuilt ones are faster here too (L = 4096, 3 % 161, 173; 5 % 207, 227; 30 % 844, 935; L = 2048, two blocks per row 95, 96;
-        head_dim 32, 9 matrices, L = 9472 207, 274) but take no notice of such a change, and their gradients differ by 4e-3 in norm, since dS
-        comes from P before it is rounded (error against fp64 2.4e-3 instead of 3.1e-3): recompute=True asks for them.
-        32-wide blocks and the full mask are rebuilt in any case.
+        P returned: the second.  The gradients are those of the very P that the caller holds, and a change of it before the backward is
+        an error.  The first differ by 4e-3 in norm, since dS comes from P before it is rounded (error against fp64 2.4e-3 instead of
+        3.1e-3): recompute=True asks for them.  32-wide blocks and the full mask are on the first in any case.
 
-        head_dim 32 with fewer than 2^15 selected blocks in all matrices: stored tiles, although the rebuilt ones are faster there too (the
+        head_dim 32 with fewer than 2^15 selected blocks in all matrices: the second, although the first is faster there too (the
         three cases above).  P is normalised before and not after it is rounded to bf16, and a training step of the encoder classifier at
         such sizes multiplies any change of rounding: the gradients of the eighth pass over one batch of 8 pairs moved by 2e-3 to
         3.3e-1 of their norm over eight seeds (both paths are equally far from the fp32 step).  The bound is a line between measured
