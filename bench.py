@@ -64,8 +64,8 @@ TRAIN_WORKLOADS = {
 NCU_TRAFFIC = {
     # workload: {stage: bytes}; the forward entry depends on whether P is stored ("fused_fwd+P" / "fused_fwd")
     "sweep_L4096_bs64_d05": {"fused_fwd+P": 248.9e6, "bwd_row": 420.3e6, "spmm_dkdv": 336.4e6,
-                             "fused_fwd": 134.1e6, "bwd_row_rc": 257.7e6, "bwd_col_rc": 217.6e6},
-    "image_L1024_fp32_B256": {"fused_fwd+P": 655.7e6, "bwd_row": 956.0e6, "spmm_dkdv": 905.2e6},
+                             "fused_fwd": 135.6e6, "bwd_row_rc": 253.7e6, "bwd_col_rc": 215.5e6},
+    "image_L1024_fp32_B256": {"fused_fwd+P": 566.5e6, "bwd_row": 956.1e6, "spmm_dkdv": 902.3e6},
 }
 
 
