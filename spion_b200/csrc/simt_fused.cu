@@ -859,11 +859,28 @@ static int row_groups(int bs, int d, long long rows, long long nnzb, int nb, boo
     return SPION_ERR_UNSUPPORTED;                                                                    \
   } while (0)
 
+// A launch has groups of matrices along gridDim.y, and a group is one matrix for blocks of 64 (simt_full.cu, mma_fused.cu), two or four for
+// blocks of 32: calls with more matrices run in equal slices.
+constexpr int MOST_MATRICES = 65535;
+static int slice(int BH) {
+  const int n = (BH + MOST_MATRICES - 1) / MOST_MATRICES;
+  return (BH + n - 1) / n;
+}
+
 // The full mask has kernels of its own (simt_full.cu).
 int simt_fused_forward(const float* Q, OperandLayout lq, const float* K, OperandLayout lk, const float* V,
                        OperandLayout lv, const float* keypad, float floor_v, float* P, ValueLayout vl, float* O,
                        OperandLayout lo, Pattern p, int BH, int L, int d, float scale, cudaStream_t st, int nnzb) {
   if (!simt_fused_supports(p.bs, d, BH, vl.mode)) return SPION_ERR_UNSUPPORTED;
+  if (BH > MOST_MATRICES) {
+    const int per = slice(BH);
+    for (long long b = 0; b < BH; b += per) {
+      const int rc = simt_fused_forward(Q + b * lq.bh_stride, lq, K + b * lk.bh_stride, lk, V + b * lv.bh_stride, lv, keypad ? keypad + b * L : nullptr,
+                                        floor_v, P + b * vl.bh_stride, vl, O + b * lo.bh_stride, lo, p, min(per, BH - (int)b), L, d, scale, st, nnzb);
+      if (rc) return rc;
+    }
+    return SPION_OK;
+  }
   if (nnzb == p.nb * p.nb) return simt_full_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
   if (use_mma(p, BH, nnzb)) return mma_fused_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
   SPION_FUSED_DISPATCH(fwd_launch, false, Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, scale, st);
@@ -875,6 +892,17 @@ int simt_fused_backward(const float* Q, OperandLayout lq, const float* K, Operan
                         float* dK, OperandLayout ldk, float* dV, OperandLayout ldv, Pattern p, int BH, int d,
                         float scale, cudaStream_t st, spion_ctx* prof, int nnzb) {
   if (!simt_fused_supports(p.bs, d, BH, vp.mode) || vds.mode != vp.mode) return SPION_ERR_UNSUPPORTED;
+  if (BH > MOST_MATRICES) {
+    const int per = slice(BH);
+    for (long long b = 0; b < BH; b += per) {
+      const int rc = simt_fused_backward(Q + b * lq.bh_stride, lq, K + b * lk.bh_stride, lk, V + b * lv.bh_stride, lv, P + b * vp.bh_stride, vp,
+                                         O ? O + b * lo.bh_stride : nullptr, lo, dO + b * ldo.bh_stride, ldo, dS + b * vds.bh_stride, vds,
+                                         dQ + b * ldq.bh_stride, ldq, dK + b * ldk.bh_stride, ldk, dV + b * ldv.bh_stride, ldv, p,
+                                         min(per, BH - (int)b), d, scale, st, prof, nnzb);
+      if (rc) return rc;
+    }
+    return SPION_OK;
+  }
   if (nnzb == p.nb * p.nb && O)
     return simt_full_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof);
   if (use_mma(p, BH, nnzb)) return mma_fused_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof, nnzb,

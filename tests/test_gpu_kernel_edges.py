@@ -217,6 +217,23 @@ def test_fp32_tensor_core_kernels_with_values_that_are_not_finite(bs, d):
             assert float(((x - y).abs()[fin] / y.abs()[fin].clamp_min(1.0)).max()) <= FP32_TOL, (b, name)
 
 
+@pytest.mark.parametrize("bs,d,BH,nb", [(32, 64, 131071, 2), (64, 32, 65536, 2), (64, 64, 65536, 1)])      # nb 1: the full mask's kernels
+def test_fp32_more_matrices_than_a_launch_takes(bs, d, BH, nb):
+    """65535 groups of one or two matrices are the most that a grid has: the matrices at both sides of a slice's end."""
+    from spion_b200.native import BlockSparseAttention
+    L = nb * bs
+    g = torch.Generator(device="cuda").manual_seed(67)
+    Q, K, V, dO = (torch.randn(BH, 1, L, d, generator=g, device="cuda") for _ in range(4))
+    mat = np.tril(np.ones((nb, nb), np.uint8))
+    kp = synthetic.key_padding(9, 16, L).repeat((BH + 15) // 16, 1)[:BH]
+    mod = BlockSparseAttention(cfg(BH, 1, L, d, bs), dtype=torch.float32, keypad=True)
+    got = run(mod, Q, K, V, dO, mat, kp)
+    n = -(-BH // 65535)
+    end = -(-BH // n)
+    some = [0, 1, 65534, 65535 % BH, end - 1, end, BH - 1]
+    compare([t[some] for t in got], *(t[some].cpu() for t in (Q, K, V, dO)), mat, bs, kp[some], FP32_TOL, False)
+
+
 @pytest.mark.parametrize("L,d", [(64, 64), (192, 32), (512, 32), (576, 32), (1024, 64), (1088, 32), (1856, 32)])
 @pytest.mark.parametrize("padded", [False, True])
 def test_dense_fp32_kernels(L, d, padded):
