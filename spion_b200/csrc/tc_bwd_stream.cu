@@ -97,6 +97,12 @@ __device__ __forceinline__ int pad64(const float* kp) {
   return other ? PAD_MIXED : first != 0.f ? PAD_ONE : PAD_NONE;
 }
 
+// Scores of 32 keys -> exponents: (s scale log2e) - (pad log2e + h), rounded as the forward does.
+__device__ __forceinline__ void take_exponent(uint32_t (&s)[32], const float* kp, float sc2, float h) {
+#pragma unroll
+  for (int x = 0; x < 32; ++x) s[x] = __float_as_uint(fmaf(__uint_as_float(s[x]), sc2, -fmaf(kp[x], LOG2E, h)));
+}
+
 // KP: with key penalties.  RND: dS from the P that the forward wrote or would have written, rounded as there (stat of k_fwd_fused), and not
 // from P before it is rounded: the gradients are bit for bit those of kernels that read stored tiles.
 template <int D, int SIDE, bool SUB, bool KP, bool RND>
@@ -534,16 +540,19 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_bwd_stream(const __grid_const
           }
           if (mine) {
             // columns are keys in both
-            if (MIXED && ((flags >> es) & 1)) take_penalty(sv, a.keypad + (size_t)bh * a.L + key * BS + g * 32, inv_scale);
+            const float* kp = MIXED && ((flags >> es) & 1) ? a.keypad + (size_t)bh * a.L + key * BS + g * 32 : nullptr;
+            if (MIXED && !RND && kp) take_penalty(sv, kp, inv_scale);
+            if (MIXED && RND && kp) take_exponent(sv, kp, sc2, h);
             const int sb = (SIDE == COL ? (q & 1) : (q >> 1)) * 2 + g;  // quarter: 2 (query / 32) + key / 32
             const bool live = !SUB || ((flags >> (8 + 8 * es + sb)) & 1);
+            const uint64_t m22 = kp ? pack2(1.f, 1.f) : sc22, mh2 = kp ? 0ull : nh2;      // RND: sv holds exponents already
             auto piece = [&](int cc) {             // eight columns: one 16-byte piece of each tile
               uint32_t wp[4], wd[4];
 #pragma unroll
               for (int x = 0; x < 4; ++x) {
                 const int c = cc * 8 + 2 * x;
                 float p0, p1, d0, d1;
-                unpack2(fma2(pack2(sv[c], sv[c + 1]), sc22, nh2), p0, p1);
+                unpack2(fma2(pack2(sv[c], sv[c + 1]), MIXED && RND ? m22 : sc22, MIXED && RND ? mh2 : nh2), p0, p1);
                 p0 = ex2_approx(p0); p1 = ex2_approx(p1);
                 wp[x] = pack_bf16(p0, p1);
                 if (RND) {

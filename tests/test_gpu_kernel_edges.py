@@ -339,12 +339,13 @@ def test_streaming_kernels_with_penalties_of_every_kind(d, bs, full):
 
 
 @pytest.mark.parametrize("d", [32, 64])
-@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("padded", [False, "keys", "soft"])
 @pytest.mark.parametrize("short", [False, True])
 @pytest.mark.parametrize("probs", [False, True])
 def test_rebuilt_rounded_tiles_are_the_stored_ones(d, padded, short, probs):
     """Gradients without stored tiles, bit for bit: rows of up to four blocks (normalised after a rounding) and longer ones (before it), masks
-    of short rows only, blocks with no, one and different penalties, odd last pairs, lines without blocks."""
+    of short rows only, blocks with no, one and different penalties (soft: penalties that leave P above zero), odd last pairs, lines without
+    blocks."""
     from spion_b200.native import BlockSparseAttention
     B, H, nb = 2, 3, 11
     L = nb * 64
@@ -353,9 +354,12 @@ def test_rebuilt_rounded_tiles_are_the_stored_ones(d, padded, short, probs):
     if short:
         mat = np.triu(mat, -3)
     kp = synthetic.key_padding(5, B, L) if padded else None
+    if padded == "soft":
+        kp[0] = 1 - 1e-6 * torch.rand(L, generator=torch.Generator().manual_seed(71)) * 3
+        kp[0, 128:192] = 1 - 1.5e-6
     got = []
     for recompute in (None, False):
-        mod = BlockSparseAttention(cfg(B, H, L, d, 64), dtype=torch.bfloat16, keypad=padded, recompute=recompute, return_probs=probs)
+        mod = BlockSparseAttention(cfg(B, H, L, d, 64), dtype=torch.bfloat16, keypad=bool(padded), recompute=recompute, return_probs=probs)
         mod.set_mask(torch.as_tensor(mat).cuda())
         if recompute is None:                                # what calls with probabilities, and small ones at head_dim 32, do
             mod.recompute, mod._ctx.rounded = False, True
