@@ -5,11 +5,12 @@
 //   mma_bwd_row2_kernel   the same when the caller has no O: dP is left in the dS tiles until rowsum(dP.P) is known
 //   mma_bwd_col_kernel    per block column:  dK = dS^T Q, dV = P^T dO
 //
-// Precision.  Every fp32 operand is split into three bf16 parts (8 + 8 + 8 significant bits: the split is exact) and the six partial
+// Precision.  Every fp32 operand is split into three bf16 parts (8 + 8 + 8 significant bits: exact from 2^-110 up) and the six partial
 // products of weight 2^0, 2^-8 and 2^-16 are accumulated in fp32; the dropped ones are below 2^-25 of the product.  The tensor cores
 // truncate a sum at every step, so each 16 terms of a contraction get accumulators of their own, the small products first, and are added
 // in fp32: one truncated step at full weight per 16 terms where a chain of FMAs rounds 16 times.  The parts of an infinity are NaN where
-// an fp32 product is an infinity or a number: a warp that meets a result that is not finite forms all of its rows again in plain fp32.
+// an fp32 product is an infinity or a number, and the last part of a value below 2^-110 ends at the smallest bf16 number: a warp that meets a
+// result that is not finite, or smaller than 2^-100 and not zero, forms all of its rows again in plain fp32.
 //
 // mma.sync and not tcgen05: a tile of a 32-wide mask has 32 rows, P and dS stay in the registers that the next product takes them from,
 // and the parts of an operand are made where it is used.  tcgen05 operands would go through shared memory three times as large.
@@ -134,16 +135,22 @@ __device__ __forceinline__ void clear(float (&v)[MT][4][4]) {
 #pragma unroll
       for (int x = 0; x < 4; ++x) v[m][n][x] = 0.f;
 }
+// Whether sums are what plain fp32 gives: finite (see split), and zero or at least 2^-100, a bound above which terms that have lost bits count for
+// nothing: with n terms of factors around f an error of sqrt(n) f 2^-134 in all.
 template <int MT>
-__device__ __forceinline__ bool finite(const float (&v)[MT][4][4]) {
+__device__ __forceinline__ bool as_fp32(const float (&v)[MT][4][4]) {
   float probe = 0.f;
+  uint32_t least = 0xffffffffu;                  // twice the bits less one: zeros are the largest
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) probe = fmaf(0.f, v[m][n][x], probe);
-  return probe == 0.f;
+      for (int x = 0; x < 4; ++x) {
+        probe = fmaf(0.f, v[m][n][x], probe);
+        least = min(least, 2u * __float_as_uint(v[m][n][x]) - 1u);
+      }
+  return probe == 0.f && least >= 2u * __float_as_uint(0x1p-100f) - 1u;
 }
 
 __device__ __forceinline__ float4 piece(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -220,10 +227,10 @@ __device__ __forceinline__ void store_row(float* out, long long sd, bool vec, co
     }
 }
 template <int D, int MT>
-__device__ __forceinline__ bool all_finite(const float (&sum)[D / 32][MT][4][4]) {
+__device__ __forceinline__ bool all_as_fp32(const float (&sum)[D / 32][MT][4][4]) {
   bool ok = true;
 #pragma unroll
-  for (int h = 0; h < D / 32; ++h) ok = ok && finite(sum[h]);
+  for (int h = 0; h < D / 32; ++h) ok = ok && as_fp32(sum[h]);
   return ok;
 }
 
@@ -251,12 +258,53 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-template <int D>
-__device__ __forceinline__ float dot(const Operand& A, int i, const Operand& B, int j) {
-  const float *a = A.base + i * A.s_row, *b = B.base + j * B.s_row;
-  float s = 0.f;
-  for (int n = 0; n < D; ++n) s = fmaf(a[n * A.s_col], b[n * B.s_col], s);
-  return s;
+// ------------------------------------------------------------------------------ plain fp32, by one warp, in the order of the terms
+// Bound by the latency of its loads.  us of forward, rows, columns, 512 matrices, L = 1024, d 32, 155 blocks of 32: no such row 269, 252, 238; one infinity
+// in V 359, 379, 239; dO of 1e-35, all rows again, 269, 2629, 1657.  (Term by term with a test after each, an infinity took 1500 us more.)
+__device__ __forceinline__ float4 load4(const Operand& o, int i, int n) {
+  const float* p = o.base + i * o.s_row + n * o.s_col;
+  return o.pieces ? piece(p) : make_float4(p[0], p[o.s_col], p[2 * o.s_col], p[3 * o.s_col]);
+}
+// WR rows of A by the rows of B's blocks -> value tiles.  Lanes are keys, whose rows of B stay in registers.
+template <int BS, int D, int WR>
+__device__ __forceinline__ void plain_abt(const Operand& A, int row0, const Operand& B, const int* cols, int nblk, float* out, int si, int step, int lane) {
+  for (int k = 0; k < nblk; ++k)
+    for (int j = lane; j < BS; j += 32) {
+      float4 b[D / 4];
+#pragma unroll
+      for (int n = 0; n < D / 4; ++n) b[n] = load4(B, cols[k] * BS + j, 4 * n);
+      for (int x = 0; x < WR; ++x) {
+        float s = 0.f;
+#pragma unroll
+        for (int n = 0; n < D / 4; ++n) {
+          const float4 q = load4(A, row0 + x, 4 * n);
+          s = fmaf(q.w, b[n].w, fmaf(q.z, b[n].z, fmaf(q.y, b[n].y, fmaf(q.x, b[n].x, s))));
+        }
+        out[x * si + (long long)k * step + j] = s;
+      }
+    }
+}
+// WR rows of value tiles by B.  Lanes are columns of B.
+template <int BS, int D, int WR>
+__device__ __forceinline__ void plain_ab(const float* vals, int si, int step, const Operand& B, const int* cols, int nblk, float* out, long long sl, long long sd,
+                                         int lane) {
+  const bool vec = vec_ok(vals);
+  for (int n = lane; n < D; n += 32) {
+    float o[WR] = {};
+    for (int k = 0; k < nblk; ++k)
+      for (int j = 0; j < BS; j += 4) {
+        float b[4];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) b[y] = B.base[(cols[k] * BS + j + y) * B.s_row + n * B.s_col];
+#pragma unroll
+        for (int x = 0; x < WR; ++x) {
+          const float4 v = load_vals(vals + x * si + (long long)k * step + j, vec);
+          o[x] = fmaf(v.w, b[3], fmaf(v.z, b[2], fmaf(v.y, b[1], fmaf(v.x, b[0], o[x]))));
+        }
+      }
+#pragma unroll
+    for (int x = 0; x < WR; ++x) out[x * sl + n * sd] = o[x];
+  }
 }
 
 // ------------------------------------------------------------------------------ forward
@@ -270,23 +318,25 @@ struct FwdArgs {
   int BH, L;
 };
 
-// Rows row0 .. row0 + WR - 1 of block row r by one warp, in fp32 and in the order of their columns.
+// Rows row0 .. row0 + WR - 1 of block row r
 template <int BS, int D, int MT>
 __device__ __noinline__ void redo_fwd(const FwdArgs& a, int bh, int r, int row0, int lane) {
+  constexpr int WR = Cfg<BS, D, MT>::WR;
   const Operand Qb(a.Q, a.lq, bh), Kb(a.K, a.lk, bh), Vb(a.V, a.lv, bh);
   const int rp = a.p.row_ptr[r], nblk = a.p.row_ptr[r + 1] - rp;
   const int* cols = a.p.col_idx + rp;
   const RowTiles rt = RowTiles::of<BS>(a.vl, rp, nblk);
   const float* kp = a.keypad ? a.keypad + (long long)bh * a.L : nullptr;
-  for (int x = 0; x < Cfg<BS, D, MT>::WR; ++x) {
-    const int row = row0 + x;
-    float* Pr = a.P + (long long)bh * a.vl.bh_stride + rt.base + row * rt.si;
+  float* P0 = a.P + (long long)bh * a.vl.bh_stride + rt.base + row0 * rt.si;
+  plain_abt<BS, D, WR>(Qb, r * BS + row0, Kb, cols, nblk, P0, rt.si, rt.step, lane);
+  for (int x = 0; x < WR; ++x) {                   // a lane reads and writes what it has written
+    float* Pr = P0 + x * rt.si;
     float m = a.floor_v * LOG2_E, l = 0.f;
     for (int k = 0; k < nblk; ++k)
       for (int j = lane; j < BS; j += 32) {
-        const int col = cols[k] * BS + j;
-        const float v = fmaf(dot<D>(Qb, r * BS + row, Kb, col), a.scale * LOG2_E, kp ? -kp[col] * LOG2_E : 0.f), m_new = fmaxf(m, v);
-        Pr[(long long)k * rt.step + j] = v;
+        float* e = Pr + (long long)k * rt.step + j;
+        const float v = fmaf(*e, a.scale * LOG2_E, kp ? -kp[cols[k] * BS + j] * LOG2_E : 0.f), m_new = fmaxf(m, v);
+        *e = v;
         l = fmaf(l, ex2(m - m_new), ex2(v - m_new));
         m = m_new;
       }
@@ -297,15 +347,9 @@ __device__ __noinline__ void redo_fwd(const FwdArgs& a, int bh, int r, int row0,
         float* e = Pr + (long long)k * rt.step + j;
         *e = inv == 0.f ? 0.f : ex2(*e - row_m) * inv;
       }
-    __syncwarp();
-    for (int n = lane; n < D; n += 32) {
-      float o = 0.f;
-      for (int k = 0; k < nblk; ++k)
-        for (int j = 0; j < BS && o == o; ++j)
-          o = fmaf(Pr[(long long)k * rt.step + j], Vb.base[(cols[k] * BS + j) * Vb.s_row + n * Vb.s_col], o);
-      a.O[(long long)bh * a.lo.bh_stride + (r * BS + row) * a.lo.sl + n * a.lo.sd] = o;
-    }
   }
+  __syncwarp();
+  plain_ab<BS, D, WR>(P0, rt.si, rt.step, Vb, cols, nblk, a.O + (long long)bh * a.lo.bh_stride + (r * BS + row0) * a.lo.sl, a.lo.sl, a.lo.sd, lane);
 }
 
 //   v = S*scale - keypad[col];  m = max(floor, max v);  Z = sum exp(v-m) + (L-n_i) exp(-m);  P = exp(v-m)/Z
@@ -449,7 +493,7 @@ __global__ void __launch_bounds__(128, (Cfg<BS, D, MT>::RESIDENT)) mma_fwd_kerne
     group_sync<C::NT>(g0);                                              // buffer k & 1 may be refilled
   }
   cp_async_wait<0>();
-  ok = ok && all_finite<D, MT>(o);
+  ok = ok && all_as_fp32<D, MT>(o);
   if (__any_sync(0xffffffffu, !ok)) {
     __syncwarp();
     redo_fwd<BS, D, MT>(a, bh, r, row0, lane);
@@ -477,26 +521,25 @@ struct RowArgs {
 // O null: the row sums of dP.P in place of those of dO.O
 template <int BS, int D, int MT>
 __device__ __noinline__ void redo_row(const RowArgs& a, int bh, int r, int row0, int lane) {
+  constexpr int WR = Cfg<BS, D, MT>::WR;
   const Operand dOb(a.dO, a.ldo, bh), Vb(a.V, a.lv, bh), Kb(a.K, a.lk, bh);
   const int rp = a.p.row_ptr[r], nblk = a.p.row_ptr[r + 1] - rp;
   const int* cols = a.p.col_idx + rp;
   const RowTiles tp = RowTiles::of<BS>(a.vp, rp, nblk), ts = RowTiles::of<BS>(a.vds, rp, nblk);
-  for (int x = 0; x < Cfg<BS, D, MT>::WR; ++x) {
-    const int row = row0 + x;
-    const float* Pr = a.P + (long long)bh * a.vp.bh_stride + tp.base + row * tp.si;
-    float* Sr = a.dS + (long long)bh * a.vds.bh_stride + ts.base + row * ts.si;
+  const float* P0 = a.P + (long long)bh * a.vp.bh_stride + tp.base + row0 * tp.si;
+  float* S0 = a.dS + (long long)bh * a.vds.bh_stride + ts.base + row0 * ts.si;
+  plain_abt<BS, D, WR>(dOb, r * BS + row0, Vb, cols, nblk, S0, ts.si, ts.step, lane);
+  for (int x = 0; x < WR; ++x) {
+    const float* Pr = P0 + x * tp.si;
+    float* Sr = S0 + x * ts.si;
+    const int row = r * BS + row0 + x;
     float s = 0.f;
-    for (int k = 0; k < nblk; ++k)
-      for (int j = lane; j < BS; j += 32) {
-        const float v = dot<D>(dOb, r * BS + row, Vb, cols[k] * BS + j);
-        Sr[(long long)k * ts.step + j] = v;
-        s = fmaf(v, Pr[(long long)k * tp.step + j], s);
-      }
     if (a.O) {
-      s = 0.f;
       for (int n = lane; n < D; n += 32)
-        s = fmaf(dOb.base[(r * BS + row) * dOb.s_row + n * dOb.s_col],
-                 a.O[(long long)bh * a.lo.bh_stride + (r * BS + row) * a.lo.sl + n * a.lo.sd], s);
+        s = fmaf(dOb.base[row * dOb.s_row + n * dOb.s_col], a.O[(long long)bh * a.lo.bh_stride + row * a.lo.sl + n * a.lo.sd], s);
+    } else {
+      for (int k = 0; k < nblk; ++k)
+        for (int j = lane; j < BS; j += 32) s = fmaf(Sr[(long long)k * ts.step + j], Pr[(long long)k * tp.step + j], s);
     }
     s = warp_sum(s);
     for (int k = 0; k < nblk; ++k)
@@ -505,15 +548,9 @@ __device__ __noinline__ void redo_row(const RowArgs& a, int bh, int r, int row0,
         const float pv = Pr[(long long)k * tp.step + j];
         *e = a.O ? pv * (*e - s) * a.scale : (*e * pv - pv * s) * a.scale;
       }
-    __syncwarp();
-    for (int n = lane; n < D; n += 32) {
-      float o = 0.f;
-      for (int k = 0; k < nblk; ++k)
-        for (int j = 0; j < BS && o == o; ++j)
-          o = fmaf(Sr[(long long)k * ts.step + j], Kb.base[(cols[k] * BS + j) * Kb.s_row + n * Kb.s_col], o);
-      a.dQ[(long long)bh * a.ldq.bh_stride + (r * BS + row) * a.ldq.sl + n * a.ldq.sd] = o;
-    }
   }
+  __syncwarp();
+  plain_ab<BS, D, WR>(S0, ts.si, ts.step, Kb, cols, nblk, a.dQ + (long long)bh * a.ldq.bh_stride + (r * BS + row0) * a.ldq.sl, a.ldq.sl, a.ldq.sd, lane);
 }
 
 // rowsum(dP.P) = rowsum(dO.O) (delta), so dS of a tile needs nothing from the other tiles of its row and one pass suffices.  Two stages per
@@ -627,7 +664,7 @@ __global__ void __launch_bounds__(128, (Cfg<BS, D, MT>::RESIDENT)) mma_bwd_row_k
     c_nxt = k + 2 < nblk ? cols[k + 2] : 0;
   }
   cp_async_wait<0>();
-  if (__any_sync(0xffffffffu, !all_finite<D, MT>(o))) {               // a dP or dS that is not finite ends up here: dQ sums over it
+  if (__any_sync(0xffffffffu, !all_as_fp32<D, MT>(o))) {               // dQ sums over dP and dS: what is amiss there shows here
     __syncwarp();
     redo_row<BS, D, MT>(a, bh, r, row0, lane);
     return;
@@ -734,7 +771,7 @@ __global__ void __launch_bounds__(128, (Cfg<BS, D, MT>::RESIDENT)) mma_bwd_row2_
     group_sync<C::NT>(g0);
   }
   cp_async_wait<0>();
-  if (__any_sync(0xffffffffu, !all_finite<D, MT>(o))) {               // a dP or dS that is not finite ends up here: dQ sums over it
+  if (__any_sync(0xffffffffu, !all_as_fp32<D, MT>(o))) {               // dQ sums over dP and dS: what is amiss there shows here
     __syncwarp();
     redo_row<BS, D, MT>(a, bh, r, row0, lane);
     return;
@@ -761,18 +798,27 @@ struct ColArgs {
 template <int BS, int D, int MT>
 __device__ __noinline__ void redo_col(const Pattern& p, const float* X, const ValueLayout& vl, const float* B, const OperandLayout& lb,
                                       float* out, const OperandLayout& lo, int bh, int c, int e0, int e1, int key0, int lane) {
+  constexpr int WR = Cfg<BS, D, MT>::WR;
   const Operand Bb(B, lb, bh);
-  for (int x = 0; x < Cfg<BS, D, MT>::WR; ++x)
-    for (int n = lane; n < D; n += 32) {
-      float s = 0.f;
-      for (int e = e0; e < e1 && s == s; ++e) {
-        long long base, si, sj;
-        tile_address(vl, p, p.row_idx[e], c, p.csc_pos[e], base, si, sj);
-        const float* v = X + (long long)bh * vl.bh_stride + base + (key0 + x) * sj;
-        for (int i = 0; i < BS; ++i) s = fmaf(v[i * si], Bb.base[(p.row_idx[e] * BS + i) * Bb.s_row + n * Bb.s_col], s);
+  const float* X0 = X + (long long)bh * vl.bh_stride + key0;
+  const bool vec = vec_ok(X0);
+  for (int n = lane; n < D; n += 32) {
+    float s[WR] = {};
+    for (int e = e0; e < e1; ++e) {
+      long long base, si, sj;
+      tile_address(vl, p, p.row_idx[e], c, p.csc_pos[e], base, si, sj);
+      for (int i = 0; i < BS; ++i) {
+        const float b = Bb.base[(p.row_idx[e] * BS + i) * Bb.s_row + n * Bb.s_col];
+#pragma unroll
+        for (int x = 0; x < WR; x += 4) {
+          const float4 v = load_vals(X0 + base + i * si + x, vec);
+          s[x] = fmaf(v.x, b, s[x]); s[x + 1] = fmaf(v.y, b, s[x + 1]); s[x + 2] = fmaf(v.z, b, s[x + 2]); s[x + 3] = fmaf(v.w, b, s[x + 3]);
+        }
       }
-      out[(long long)bh * lo.bh_stride + (c * BS + key0 + x) * lo.sl + n * lo.sd] = s;
     }
+#pragma unroll
+    for (int x = 0; x < WR; ++x) out[(long long)bh * lo.bh_stride + (c * BS + key0 + x) * lo.sl + n * lo.sd] = s[x];
+  }
 }
 
 // sum += X^T B over the rows of a value tile; X: [bs x bs], this warp's keys from key0 on.  Row slot (m, half) of the result: key MT 2 g + 2 m + half.
@@ -944,7 +990,7 @@ __global__ void __launch_bounds__(128, (Cfg<BS, D, MT>::RESIDENT)) mma_bwd_col_k
     const int g = lane >> 2, cc = lane & 3;
     auto put = [&](const float (&sum)[C::NH][MT][4][4], float* out, const OperandLayout& lo, const float* X, const ValueLayout& vl, const float* B,
                    const OperandLayout& lb) {
-      if (__any_sync(0xffffffffu, !all_finite<D, MT>(sum))) {
+      if (__any_sync(0xffffffffu, !all_as_fp32<D, MT>(sum))) {
         redo_col<BS, D, MT>(a.p, X, vl, B, lb, out, lo, bh, c, first, last, key0, lane);
         return;
       }

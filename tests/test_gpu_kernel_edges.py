@@ -217,6 +217,38 @@ def test_fp32_tensor_core_kernels_with_values_that_are_not_finite(bs, d):
             assert float(((x - y).abs()[fin] / y.abs()[fin].clamp_min(1.0)).max()) <= FP32_TOL, (b, name)
 
 
+@pytest.mark.parametrize("bs,d", [(32, 32), (32, 64), (64, 32), (64, 64)])
+@pytest.mark.parametrize("layout", ["tiles", "csr"])
+@pytest.mark.parametrize("scale", [1e-30, 1e-33, 1e-36])
+def test_fp32_tensor_core_kernels_with_small_values(bs, d, layout, scale):
+    """V and dO so small that bf16 parts of them, of dP and of dS would fall below the smallest bf16 number.  fp32 sums of up to 1024 products:
+    sqrt(1024) roundings of 2^-24 in norm."""
+    from spion_b200.attention import Attention
+    from spion_b200.attention_blockcuda import CUDABlockAttention
+    from spion_b200.native import BlockSparseAttention
+    B, nb = (80, 16) if bs == 32 else (48, 16)
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(73, B, 1, L, d)
+    mat = lines_of_every_length(nb)
+    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+    if layout == "tiles":
+        mod = BlockSparseAttention(cfg(B, 1, L, d, bs), dtype=torch.float32)
+        call = lambda values: mod(q, k, values, None, torch.as_tensor(mat).cuda())[0]
+    else:
+        cpp = Attention._blockcuda_compile_module()
+        handle = cpp.init(d, L, B, bs)
+        mod = CUDABlockAttention(cfg(B, 1, L, d, bs), cpp, handle)
+        call = lambda values: mod(q, k, values, torch.ones(B, L).cuda(), torch.as_tensor(mat.astype(np.float32)).cuda())[0]
+    got = [call((V * scale).cuda()).detach()] + list(torch.autograd.grad(call(v), (q, k, v), (dO * scale).cuda()))
+    want = oatt.sparse_attention(Q[:3], K[:3], V[:3], mat, bs, None, (dO * scale)[:3], dtype=torch.float64)
+    want = [oatt.sparse_attention(Q[:3], K[:3], (V * scale)[:3], mat, bs, dtype=torch.float64)[0], *want[2:]]
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), got, want):
+        err = float((a[:3].cpu().double() - b).norm() / b.norm())
+        assert err <= 1024 ** 0.5 * 2.0 ** -24, f"{name}: {err:.2e}"
+    if layout == "csr":
+        cpp.destroy(handle)
+
+
 @pytest.mark.parametrize("bs,d,BH,nb", [(32, 64, 131071, 2), (64, 32, 65536, 2), (64, 64, 65536, 1)])      # nb 1: the full mask's kernels
 def test_fp32_more_matrices_than_a_launch_takes(bs, d, BH, nb):
     """65535 groups of one or two matrices are the most that a grid has: the matrices at both sides of a slice's end."""
