@@ -260,7 +260,7 @@ __device__ __forceinline__ float warp_max(float v) {
 
 // ------------------------------------------------------------------------------ plain fp32, by one warp, in the order of the terms
 // Bound by the latency of its loads.  us of forward, rows, columns, 512 matrices, L = 1024, d 32, 155 blocks of 32: no such row 269, 252, 238; one infinity
-// in V 359, 379, 239; dO of 1e-35, all rows again, 269, 2629, 1657.  (Term by term with a test after each, an infinity took 1500 us more.)
+// in V 359, 379, 239; dO of 1e-35, all rows again, 269, 2629, 1657.  (Term by term with a test after each, that infinity took 700 us more.)
 __device__ __forceinline__ float4 load4(const Operand& o, int i, int n) {
   const float* p = o.base + i * o.s_row + n * o.s_col;
   return o.pieces ? piece(p) : make_float4(p[0], p[o.s_col], p[2 * o.s_col], p[3 * o.s_col]);
@@ -1096,6 +1096,8 @@ int bwd_launch(const RowArgs& ra, ColArgs& ca, int nnzb, int longest, cudaStream
 
 }  // namespace
 
+// Blocks of 32, d 32: one 16-row tile per warp, twice as many warps, while rows are few.  us of forward + rows with one and two, rows of 5 blocks:
+// 640 rows 48, 59; 1024 61, 66; 1536 80, 84; 1792 88, 93; 2560 117, 120; 3072 135, 132; 4096 171, 165; 8192 311, 286.
 #define SPION_MMA_DISPATCH(FN, ...)                                                                                      \
   do {                                                                                                                  \
     const long long rows = (long long)p.nb * BH;                                                                        \

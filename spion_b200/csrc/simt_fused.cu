@@ -818,24 +818,28 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
 }
 
 // Which calls the kernels of mma_fused.cu serve: those with work for most schedulers.  Their warps do twice (block 32) or half (64) of what
-// the threads of a row do here, and they leave a column to one CTA, so few long rows are better shared by groups of threads.  us of forward, rows and
-// columns here and there (masks with rows of equal length):
-//   blocks of 32, d 32: 256 rows of 4 blocks 31, 32 in all; 192 of 8 41, 50; 512 of 4 48, 38; 592 of 2 32, 24; 2048 of 1 51, 42
-//     d 64: 256 rows of 8 76, 73; 512 of 4 80, 60; 1024 of 2 89, 64
-//   blocks of 64, d 64: 96 rows of 8 111, 127; 192 of 3 105, 81; 192 of 6 176, 146; 384 of 2 113, 80;  d 32: 192 of 3 73, 48; 768 of 1 78, 51
-// and with random blocks, 16384 rows of 5 blocks of 32 935, 735; 4096 rows of 3 blocks of 64, d 64 1138, 1004.  The lines leave some of
-// the gain to short rows.
-static bool use_mma(const Pattern& p, int BH, int nnzb) {
+// the threads of a row do here, and nobody shares a row there, so a few uneven rows are better shared by groups of threads.  us of forward, rows and columns
+// there and here, in a graph (a band of two blocks and random ones unless stated):
+//   blocks of 32, two matrices per CTA there: d 32 up to three CTAs for two SMs 256 rows of 5 blocks 51, 46; 304 of 5 56, 50; 320 of 8 77, 73; 384 of 8
+//     85, 75 (all of 4: 36, 38); more of them 480 of 5 60, 71; 512 of 4.8 53, 64; 1024 of 5 90, 122.  d 64, whose threads here have twice the work:
+//     256 of 5 77, 78; 304 of 5 93, 84; 320 of 5 89, 88; 512 of 5 102, 120
+//   blocks of 64, d 32: 144 rows of 5 87, 85; 160 of 5 100, 114;  d 64: 160 of 5 170, 165; 176 of 5 191, 162; 192 of 5 166, 171; 224 of 5 183, 206
+//     (with a full column: 160 of 7 1.05 times as long there, 192 of 7 0.88; all of equal length: 176 rows of 6 0.81)
+// Few blocks in all stay here although rows of two are faster there (512 rows, d 32: 27, 38): up to that size a pass is host time.
+static bool use_mma(const Pattern& p, int d, int BH, int nnzb) {
   const long long sms = sm_count(), rows = (long long)p.nb * BH, blocks = (long long)nnzb * BH;
-  return p.bs == 32 ? rows >= 2 * sms && (blocks > 10 * sms || rows > 8 * sms) : rows >= sms && (blocks > 5 * sms || rows > 2 * sms);
+  if (p.bs == 64) return 4 * rows >= (d == 64 ? 5 : 4) * sms && (blocks > 5 * sms || rows > 2 * sms);
+  const long long ctas = (long long)p.nb * ((BH + 1) / 2);            // what nobody shares, there
+  return rows > 8 * sms || (blocks > 10 * sms && (d == 64 ? rows >= 2 * sms : 2 * ctas > 3 * sms));
 }
 
 // Groups of threads that share the blocks of a row (forward and row kernels; columns are shared by a cluster).  They pay
 // where the rows have blocks to share and some are longer than others, and lose in a second wave of CTAs with equal rows.  us of the forward
 // and of the row kernel with one group, two (and four); masks with a band of two blocks and random ones unless stated:
 //   blocks of 32: four up to one CTA per SM (d 32, 128 rows of 5 blocks, the longest 8: 16.6, 10.5, 9.1 and 15.6, 9.9, 8.5), two up to four
-//     (512 such rows 23.2, 20.5, 23.1 and 21.5, 19.7, 21.7; d 64, 288 rows of two blocks 12.0, 8.3, 12.5 and 12.3, 9.6, 13.5).  d 64: half the
-//     registers make the row kernel slower from 512 rows on (36.1, 37.4; 384 rows 36.8, 34.3), so its line is three CTAs per SM.
+//     (d 32, 384 rows of 8 35.6, 25.2, 26.7 and 32.8, 23.9, 24.9, of 5 23.8, 18.9, 21.1; 592 of 2 10.8, 10.4, 15.3 and 12.0, 10.2, 13.9, but 512 of 2
+//     10.2, 11.3, 15.1; d 64, 288 rows of two blocks 12.0, 8.3, 12.5 and 12.3, 9.6, 13.5).  d 64: half the registers make the row kernel slower
+//     from 512 rows on (of two blocks 15.7, 20.3; 384 rows of 8 56.5, 45.9), so its line is three CTAs per SM.
 //   blocks of 64 (512 threads for two groups): d 64, 128 rows of 10 blocks 74, 69 and 73, 63; 192 rows of 3 blocks 48, 44 and 47, 41, of 4
 //     62, 53 and 61, 49 (all of 4: 39.8, 42.8 and 38.9, 40.1); 288 rows of 3 48, 52 and 47, 48, of 8 131, 133 and 126, 122; rows of two blocks:
 //     128 13.3, 13.4 and 13.2, 12.4, 192 21.5, 24.6 and 21.3, 22.9.  So three CTAs for two SMs, and one per SM if the rows are short.
@@ -882,7 +886,7 @@ int simt_fused_forward(const float* Q, OperandLayout lq, const float* K, Operand
     return SPION_OK;
   }
   if (nnzb == p.nb * p.nb) return simt_full_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
-  if (use_mma(p, BH, nnzb)) return mma_fused_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
+  if (use_mma(p, d, BH, nnzb)) return mma_fused_forward(Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, d, scale, st);
   SPION_FUSED_DISPATCH(fwd_launch, false, Q, lq, K, lk, V, lv, keypad, floor_v, P, vl, O, lo, p, BH, L, scale, st);
 }
 
@@ -905,7 +909,7 @@ int simt_fused_backward(const float* Q, OperandLayout lq, const float* K, Operan
   }
   if (nnzb == p.nb * p.nb && O)
     return simt_full_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof);
-  if (use_mma(p, BH, nnzb)) return mma_fused_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof, nnzb,
+  if (use_mma(p, d, BH, nnzb)) return mma_fused_backward(Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH, d, scale, st, prof, nnzb,
                                                       prof ? prof->longest_col : -1);
   SPION_FUSED_DISPATCH(bwd_launch, true, Q, lq, K, lk, V, lv, P, vp, O, lo, dO, ldo, dS, vds, dQ, ldq, dK, ldk, dV, ldv, p, BH,
                        scale, st, prof);

@@ -181,6 +181,30 @@ def test_fp32_tensor_core_kernels(bs, d, B, H, nb, layout, full_column):
     cpp.destroy(handle)
 
 
+def fp32_kernels(step):
+    from torch.profiler import ProfilerActivity, profile
+    step()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        step()
+        torch.cuda.synchronize()
+    return {e.name for e in prof.events() if "mma_" in e.name or "fused_" in e.name}
+
+
+# (bs, d, B, blocks per side, blocks per row, tensor cores): both sides of the lines between the two files (148 SMs)
+@pytest.mark.parametrize("bs,d,B,nb,per,mma", [(32, 32, 12, 32, 8, False), (32, 32, 14, 32, 8, True), (32, 32, 14, 32, 3, False), (32, 32, 75, 16, 1, True),
+                                               (32, 64, 9, 32, 8, False), (32, 64, 10, 32, 8, True), (64, 32, 9, 16, 6, False), (64, 32, 10, 16, 6, True),
+                                               (64, 64, 11, 16, 6, False), (64, 64, 12, 16, 6, True), (64, 64, 19, 16, 2, True)])
+def test_fp32_calls_on_either_side_of_the_line(bs, d, B, nb, per, mma):
+    from spion_b200.native import BlockSparseAttention
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(79 + nb, B, 1, L, d)
+    mat = synthetic.band_random_mask(3, nb, per / nb) if per > 1 else np.eye(nb, dtype=np.uint8)
+    mod = BlockSparseAttention(cfg(B, 1, L, d, bs), dtype=torch.float32)
+    compare(run(mod, Q, K, V, dO, mat, None), Q, K, V, dO, mat, bs, None, FP32_TOL, False)
+    names = fp32_kernels(lambda: run(mod, Q, K, V, dO, mat, None))
+    assert len(names) >= 3 and all(("mma_" in n) == mma for n in names), names
+
+
 @pytest.mark.parametrize("bs,d", [(32, 32), (64, 64)])
 def test_fp32_tensor_core_kernels_with_values_that_are_not_finite(bs, d):
     """The parts of an infinity are NaN: rows that meet one are formed again.  A block-diagonal mask with a second block per row, so that what
