@@ -1058,8 +1058,9 @@ int bwd_launch(const RowArgs& ra, ColArgs& ca, int nnzb, int longest, cudaStream
   else mma_bwd_row2_kernel<BS, D, MT><<<rgrid, R::CTA, smem_row<BS, D, MT>(), st>>>(ra);
   SPION_LAUNCH_CHECK();
   if (prof) prof_mark(prof, SPION_STAGE_BWD_ROW);
-  // A column is worth sharing when it alone takes longer than all entries of all columns do on the whole chip, and twice as long as the
-  // average one.
+  // A column is worth sharing when it alone takes half as long as all entries of all columns do on the whole chip, and twice as long as the
+  // average one.  (Blocks of 64 at d 32: the tiles leave room for two CTAs and not three.  With two here and for the registers, full columns
+  // took 2 to 4 % longer: 9 matrices, 64 x 64 blocks, two full columns, forward + backward 269 -> 280 us.)
   const long long at_once = (long long)sm_count() * C::RESIDENT * C::G, entries = (long long)ca.BH * nnzb;
   long long from = entries / (2 * at_once) + 1;
   if (from < 2LL * nnzb / ca.p.nb + 1) from = 2LL * nnzb / ca.p.nb + 1;

@@ -2,7 +2,7 @@
 // effect: its gradient is a sum that cancels to the rounding of its terms, so that every other order of additions gives another
 // gradient.  These kernels keep the order the dense phase has always had (4 x 4 micro-tiles, one sum per output in ascending order,
 // row sums joined tile by tile); masks with unselected blocks run on simt_fused.cu or mma_fused.cu, which are at least 1.3 times faster, and so does a
-// backward on a full mask whose caller has no O (the reference's signature): its order is that of simt_fused.cu.
+// backward on a full mask whose caller has no O (the reference's signature): which of them, and so its order, depends on the size of the call.
 //
 // Thread layout: a bs x bs tile is computed by (bs/4)^2 threads with 4x4 micro-tiles (rows
 // contiguous, columns interleaved by bs/4 so that shared-memory reads of the second operand are

@@ -152,35 +152,6 @@ def test_fp32_groups_per_row(bs, d, B, nb, per, forward, backward):
         assert any(f"{kernel}<{bs}, {d}, 4, {groups}>" in n for n in names), names
 
 
-# Calls on the fp32 tensor-core kernels: (bs, d, B, H, blocks per side), one and two 16-row tiles per warp, groups of matrices with some left
-# over, rows and columns of every length and none, full columns shared by a cluster, key padding; element CSR without O (two passes)
-@pytest.mark.parametrize("bs,d,B,H,nb", [(32, 32, 65, 1, 9), (32, 32, 151, 3, 8), (32, 64, 33, 3, 7), (64, 32, 25, 1, 8), (64, 64, 31, 1, 11), (64, 64, 61, 1, 5)])
-@pytest.mark.parametrize("layout", ["tiles", "csr"])
-@pytest.mark.parametrize("full_column", [False, True])
-def test_fp32_tensor_core_kernels(bs, d, B, H, nb, layout, full_column):
-    from spion_b200.attention import Attention
-    from spion_b200.attention_blockcuda import CUDABlockAttention
-    from spion_b200.native import BlockSparseAttention
-    L = nb * bs
-    Q, K, V, dO = synthetic.qkv(37 + nb, B, H, L, d)
-    mat = lines_of_every_length(nb) if not full_column else synthetic.band_random_mask(3, nb, 0.0)
-    if full_column:
-        mat[:, [1, nb - 1]] = 1
-    if layout == "tiles":
-        kp = synthetic.key_padding(9, B, L) if nb % 2 else None
-        mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.float32, keypad=kp is not None)
-        compare(run(mod, Q, K, V, dO, mat, kp), Q, K, V, dO, mat, bs, kp, FP32_TOL, False)
-        return
-    cpp = Attention._blockcuda_compile_module()
-    handle = cpp.init(d, L, B * H, bs)
-    mod = CUDABlockAttention(cfg(B, H, L, d, bs), cpp, handle)
-    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
-    out, _ = mod(q, k, v, torch.ones(B, L).cuda(), torch.as_tensor(mat.astype(np.float32)).cuda())
-    out.backward(dO.cuda())
-    compare((out, q.grad, k.grad, v.grad), Q, K, V, dO, mat, bs, None, FP32_TOL, False)
-    cpp.destroy(handle)
-
-
 def fp32_kernels(step):
     from torch.profiler import ProfilerActivity, profile
     step()
@@ -188,6 +159,63 @@ def fp32_kernels(step):
         step()
         torch.cuda.synchronize()
     return {e.name for e in prof.events() if "mma_" in e.name or "fused_" in e.name}
+
+
+def fp32_call(layout, B, H, L, d, bs, mat, kp):
+    """One call per layout: block tiles; element CSR with the reference's signature (a backward without O: two passes over a row); element CSR
+    through the layers' host path (with O)."""
+    from spion_b200 import _ops
+    from spion_b200.attention import Attention
+    from spion_b200.attention_blockcuda import CUDABlockAttention
+    from spion_b200.native import BlockSparseAttention
+    if layout == "tiles":
+        mod = BlockSparseAttention(cfg(B, H, L, d, bs), dtype=torch.float32, keypad=kp is not None)
+        return lambda q, k, v: mod(q, k, v, None if kp is None else kp.cuda(), torch.as_tensor(mat).cuda())[0], lambda: None
+    cpp = Attention._blockcuda_compile_module()
+    handle = cpp.init(d, L, B * H, bs)
+    mod = CUDABlockAttention(cfg(B, H, L, d, bs), cpp, handle)
+    ones, fmat = torch.ones(B, L).cuda(), torch.as_tensor(mat.astype(np.float32)).cuda()
+    if layout == "csr":
+        return lambda q, k, v: mod(q, k, v, ones, fmat)[0], lambda: cpp.destroy(handle)
+    return lambda q, k, v: _ops.attention(mod.context(fmat), q, k, v, None)[0], lambda: cpp.destroy(handle)
+
+
+# Calls on the fp32 tensor-core kernels: (bs, d, B, H, blocks per side, full columns), one and two 16-row tiles per warp, groups of matrices with some
+# left over, rows and columns of every length and none, full columns, key padding
+LINES = [(32, 32, 65, 1, 9), (32, 32, 151, 3, 8), (32, 64, 33, 3, 7), (64, 32, 41, 1, 8), (64, 64, 31, 1, 11), (64, 64, 61, 1, 5)]
+# full columns shared by clusters, six of them more than a launch has clusters along the columns
+SHARED = [(32, 32, 65, 1, 20), (32, 32, 151, 3, 16), (32, 64, 33, 3, 15), (64, 32, 41, 1, 17), (64, 64, 31, 1, 18)]
+
+
+@pytest.mark.parametrize("bs,d,B,H,nb,full", [c + (n,) for c in LINES for n in (0, 2)] + [c + (n,) for c in SHARED for n in (2, 6)])
+@pytest.mark.parametrize("layout", ["tiles", "csr", "csr with O"])
+def test_fp32_tensor_core_kernels(bs, d, B, H, nb, full, layout):
+    L = nb * bs
+    Q, K, V, dO = synthetic.qkv(37 + nb, B, H, L, d)
+    mat = lines_of_every_length(nb) if not full else synthetic.band_random_mask(3, nb, 0.0)
+    if full:
+        mat[:, 1:full] = 1
+        mat[:, nb - 1] = 1
+    kp = synthetic.key_padding(9, B, L) if nb % 2 and layout == "tiles" else None
+    call, close = fp32_call(layout, B, H, L, d, bs, mat, kp)
+    q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
+    got = []
+
+    def step():
+        out = call(q, k, v)
+        got[:] = (out,) + torch.autograd.grad(out, (q, k, v), dO.cuda())
+
+    names = fp32_kernels(step)
+    close()
+    some = list(range(B)) if nb < 12 else [0, B // 2, B - 1]
+    compare([t[some] for t in got], *(t[some] for t in (Q, K, V, dO)), mat, bs, None if kp is None else kp[some], FP32_TOL, False)
+    rows, cols = (2 if bs == d == 32 and nb * B * H > 12 * 148 else 1), (2 if d == 32 else 1)
+    want = {f"mma_fwd_kernel<{bs}, {d}, {rows}>", f"mma_bwd_row{'2' if layout == 'csr' else ''}_kernel<{bs}, {d}, {rows}>",
+            f"mma_bwd_col_kernel<{bs}, {d}, {cols}, false>"}
+    if nb > 11:
+        want.add(f"mma_bwd_col_kernel<{bs}, {d}, {cols}, true>")
+    assert all(any(w in n for n in names) for w in want), (want, names)
+    assert not any("fused_" in n for n in names), names
 
 
 # (bs, d, B, blocks per side, blocks per row, tensor cores): both sides of the lines between the two files (148 SMs)
@@ -247,30 +275,19 @@ def test_fp32_tensor_core_kernels_with_values_that_are_not_finite(bs, d):
 def test_fp32_tensor_core_kernels_with_small_values(bs, d, layout, scale):
     """V and dO so small that bf16 parts of them, of dP and of dS would fall below the smallest bf16 number.  fp32 sums of up to 1024 products:
     sqrt(1024) roundings of 2^-24 in norm."""
-    from spion_b200.attention import Attention
-    from spion_b200.attention_blockcuda import CUDABlockAttention
-    from spion_b200.native import BlockSparseAttention
     B, nb = (80, 16) if bs == 32 else (48, 16)
     L = nb * bs
     Q, K, V, dO = synthetic.qkv(73, B, 1, L, d)
     mat = lines_of_every_length(nb)
+    call, close = fp32_call(layout, B, 1, L, d, bs, mat, None)
     q, k, v = (t.cuda().requires_grad_(True) for t in (Q, K, V))
-    if layout == "tiles":
-        mod = BlockSparseAttention(cfg(B, 1, L, d, bs), dtype=torch.float32)
-        call = lambda values: mod(q, k, values, None, torch.as_tensor(mat).cuda())[0]
-    else:
-        cpp = Attention._blockcuda_compile_module()
-        handle = cpp.init(d, L, B, bs)
-        mod = CUDABlockAttention(cfg(B, 1, L, d, bs), cpp, handle)
-        call = lambda values: mod(q, k, values, torch.ones(B, L).cuda(), torch.as_tensor(mat.astype(np.float32)).cuda())[0]
-    got = [call((V * scale).cuda()).detach()] + list(torch.autograd.grad(call(v), (q, k, v), (dO * scale).cuda()))
+    got = [call(q, k, (V * scale).cuda()).detach()] + list(torch.autograd.grad(call(q, k, v), (q, k, v), (dO * scale).cuda()))
+    close()
     want = oatt.sparse_attention(Q[:3], K[:3], V[:3], mat, bs, None, (dO * scale)[:3], dtype=torch.float64)
     want = [oatt.sparse_attention(Q[:3], K[:3], (V * scale)[:3], mat, bs, dtype=torch.float64)[0], *want[2:]]
     for name, a, b in zip(("O", "dQ", "dK", "dV"), got, want):
         err = float((a[:3].cpu().double() - b).norm() / b.norm())
         assert err <= 1024 ** 0.5 * 2.0 ** -24, f"{name}: {err:.2e}"
-    if layout == "csr":
-        cpp.destroy(handle)
 
 
 @pytest.mark.parametrize("bs,d,BH,nb", [(32, 64, 131071, 2), (64, 32, 65536, 2), (64, 64, 65536, 1)])      # nb 1: the full mask's kernels
