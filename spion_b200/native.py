@@ -115,8 +115,7 @@ class BlockSparseAttention(nn.Module):
         self.nnzb = int(lib.spion_pattern_nnzb(self.handle))
         if self.fused and self._recompute_arg is None:
             self.recompute = self._recompute_pays()
-            # the gradients of stored tiles, without storing them: 64-wide blocks
-            self._ctx.rounded = not self.recompute
+            self._ctx.rounded = not self.recompute and self._rebuilt_pays()
         from .pattern import pattern_from_mask
         self._pattern = pattern_from_mask(m8, self.bs)          # block CSR for the helpers above
         self._mask_key.set(mat)
@@ -124,13 +123,12 @@ class BlockSparseAttention(nn.Module):
 
     def _recompute_pays(self) -> bool:
         """Which gradients serve the current mask: those of P as the log-sum-exp gives it (True), or those of the P that is rounded to bf16
-        (False), bit for bit what stored tiles give.  Without a ``recompute`` argument neither reads a stored P or dS: both backward kernels
-        form P again, the second with the two factors per row that the forward leaves beside the log-sum-exp.
+        (False), bit for bit what stored tiles give (see _rebuilt_pays).
 
-        No P returned: the first, whose forward is faster (forward + backward on one B200 when the rule was made, us, against
-        stored tiles; head_dim 64 and 64 matrices unless stated): L = 4096, 3 % (two blocks per row) 150, 173; 5 % 174, 226; 30 % 581, 924;
-        L = 16384, 5 % 1764, 2882; 512 matrices, L = 1024, two blocks per row 266, 323; 2 matrices, L = 4096, 5 % 82, 86.  head_dim 32: 9
-        matrices, L = 9472, 12 % 158, 274; 28 matrices, L = 6528, 4 % 109, 163; 2 matrices, L = 2048 85, 91.
+        No P returned: the first, whose forward is faster (forward + backward on one B200, us, against the second from rebuilt tiles; head_dim
+        64 and 64 matrices unless stated): L = 4096, 3 % (two blocks per row) 143, 148; 5 % 162, 189; 30 % 540, 761; L = 16384, 5 % 1440, 2185;
+        512 matrices, L = 1024, two blocks per row 314, 331; 2 matrices, L = 4096, 5 % 23, 28.  head_dim 32: 9 matrices, L = 9472, 12 % 139, 199;
+        28 matrices, L = 6528, 4 % 92, 122; 2 matrices, L = 2048 17, 18.
 
         P returned: the second.  The gradients are those of the very P that the caller holds, and a change of it before the backward is
         an error.  The first differ by 4e-3 in norm, since dS comes from P before it is rounded (error against fp64 2.4e-3 instead of
@@ -146,6 +144,21 @@ class BlockSparseAttention(nn.Module):
         if self.bs == 32 or self.nnzb == nb * nb:
             return True
         return not self.return_probs and (self.d == 64 or self.BH * self.nnzb >= 1 << 15)
+
+    def _rebuilt_pays(self) -> bool:
+        """The gradients of the rounded P come from tiles that the backward rebuilds from two factors per row (True), or from stored P and dS, in
+        the same bits.  Rebuilding costs the penalties and the exponentials twice more, storing costs the traffic, so short rows, small calls and padded keys
+        are for stored tiles.  Forward + backward, us, rebuilt and stored, head_dim 32 (64), 64-wide blocks:
+        no padding: 254 blocks in two-block rows 18.0, 15.9 (19.1, 16.8); 496 20.5, 19.1 (22.1, 21.5); 992 24.9, 27.0 (29.3, 30.3); 616 in rows of
+          4.8 27.8, 31.3 (30.0, 33.2); 26240 in rows of 6.4 239, 307 (311, 366)
+        padded keys, no P returned: 248 in two-block rows 25.0, 18.8; 1640 in rows of 3.2 48.2, 44.3; 2464 in rows of 4.8 58.6, 50.7; 4096 in rows of 4
+          74.0, 76.5; 13120 in rows of 6.4 168, 184; 15872 in two-block rows 251, 244
+        padded keys, P returned: 1640 in rows of 6.4 48.9, 45.8 (52.7, 49.4); 7936 in two-block rows 141, 133 (188, 176); 13120 in rows of 3.2 207, 199
+          (261, 249); 4916 in rows of 19 92.4, 99.2 (104, 107); 26240 in rows of 6.4 338, 347 (410, 412)"""
+        blocks = self.BH * self.nnzb
+        if not self.keypad:
+            return blocks >= 512
+        return blocks >= 4096 and (not self.return_probs or self.nnzb >= 5 * (self.L // self.bs))
 
     @property
     def nnz(self) -> int:

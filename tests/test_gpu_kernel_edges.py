@@ -447,6 +447,34 @@ def test_rebuilt_rounded_tiles_are_the_stored_ones(d, padded, short, probs):
     compare(got[0], Q, K, V, dO, mat, 64, kp, BF16_REL, True)
 
 
+# (d, padded, P returned, matrices, blocks per side, blocks per row, rebuilt): both sides of the lines between rebuilt and stored rounded tiles
+@pytest.mark.parametrize("d,padded,probs,BH,nb,per,rebuilt",
+                         [(32, False, False, 31, 8, 2, False), (32, False, False, 32, 8, 2, True), (64, False, True, 17, 10, 3, False), (64, False, True, 18, 10, 3, True),
+                          (32, True, False, 102, 10, 4, False), (32, True, False, 103, 10, 4, True), (32, True, True, 101, 10, 4, False), (64, True, True, 103, 10, 4, False),
+                          (64, True, True, 103, 10, 5, True), (32, True, True, 103, 8, 5, True), (32, True, True, 81, 10, 5, False)])
+def test_rounded_tiles_are_rebuilt_or_stored(d, padded, probs, BH, nb, per, rebuilt):
+    from torch.profiler import ProfilerActivity, profile
+
+    from spion_b200.native import BlockSparseAttention
+    L = nb * 64
+    Q, K, V, dO = (t.to(torch.bfloat16) for t in synthetic.qkv(83 + d, BH, 1, L, d))
+    mat = np.zeros((nb, nb), np.uint8)
+    for r in range(nb):
+        mat[r, [(r + i) % nb for i in range(per)]] = 1
+    kp = synthetic.key_padding(5, BH, L) if padded else None
+    got = []
+    for recompute in (None, False):
+        mod = BlockSparseAttention(cfg(BH, 1, L, d, 64), dtype=torch.bfloat16, keypad=padded, recompute=recompute, return_probs=probs)
+        run(mod, Q, K, V, dO, mat, kp)
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            got.append(run(mod, Q, K, V, dO, mat, kp))
+        names = {e.name for e in prof.events()}
+        assert any("k_bwd_stream" in n for n in names) == (rebuilt and recompute is None), names
+        assert any("k_bwd_row" in n for n in names) == (not rebuilt or recompute is False), names
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), *got):
+        assert torch.equal(a, b), f"{name}: {far(a, b, True):.3e}"
+
+
 @pytest.mark.parametrize("d", [32, 64])
 def test_gradients_read_the_probabilities_that_a_hook_hands_back(d):
     """A hook on saved tensors that gives halved probabilities to the backward halves dV: exact in bf16."""
