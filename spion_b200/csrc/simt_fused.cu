@@ -818,19 +818,20 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
 }
 
 // Which calls the kernels of mma_fused.cu serve: those with work for most schedulers.  Their warps do twice (block 32) or half (64) of what
-// the threads of a row do here, and nobody shares a row there, so a few uneven rows are better shared by groups of threads.  us of forward, rows and columns
-// there and here, in a graph (a band of two blocks and random ones unless stated):
-//   blocks of 32, two matrices per CTA there: d 32 up to three CTAs for two SMs 256 rows of 5 blocks 51, 46; 304 of 5 56, 50; 320 of 8 77, 73; 384 of 8
-//     85, 75 (all of 4: 36, 38); more of them 480 of 5 60, 71; 512 of 4.8 53, 64; 1024 of 5 90, 122.  d 64, whose threads here have twice the work:
-//     256 of 5 77, 78; 304 of 5 93, 84; 320 of 5 89, 88; 512 of 5 102, 120
+// the threads of a row do here, and nobody shares a row there, so the uneven rows of small calls are better shared by groups of threads (up to four
+// rows of blocks of 32 per SM, see row_groups).  us of forward, rows and columns there and here, in a graph (a band of two blocks and random ones):
+//   blocks of 32, d 32: rows of 5 blocks 256 51, 46; 304 56, 50; 416 57, 57; 480 60, 71; 512 (of 4.8) 53, 64; 1024 90, 120.  Rows of 8 384 85, 75; 448 87, 78;
+//     480 86, 91.  Rows of 12, 24, 45, two or three matrices, whose CTAs have room for a third or fourth there: 456 rows 0.85, 0.87, 0.86 times the
+//     speed there, 500 0.86, 0.88, 0.83, 540 0.89, 0.90, 0.84; four or eight matrices: 448 0.86 - 0.98, 512 1.01 - 1.09; 768 and more 1.09 - 1.20.
+//   d 64, whose threads here have twice the work: rows of 5 256 77, 78; 304 93, 83; 320 89, 88; 512 102, 120.  Rows of 12, 24, 45: 300 0.86, 0.79,
+//     0.89 times the speed there, 320 0.87 - 0.92, 380 0.91 - 0.95, 384 0.84 - 0.99 (with a full column 0.89 - 1.24), 456 and more 1.01 - 1.20
 //   blocks of 64, d 32: 144 rows of 5 87, 85; 160 of 5 100, 114;  d 64: 160 of 5 170, 165; 176 of 5 191, 162; 192 of 5 166, 171; 224 of 5 183, 206
 //     (with a full column: 160 of 7 1.05 times as long there, 192 of 7 0.88; all of equal length: 176 rows of 6 0.81)
 // Few blocks in all stay here although rows of two are faster there (512 rows, d 32: 27, 38): up to that size a pass is host time.
 static bool use_mma(const Pattern& p, int d, int BH, int nnzb) {
   const long long sms = sm_count(), rows = (long long)p.nb * BH, blocks = (long long)nnzb * BH;
   if (p.bs == 64) return 4 * rows >= (d == 64 ? 5 : 4) * sms && (blocks > 5 * sms || rows > 2 * sms);
-  const long long ctas = (long long)p.nb * ((BH + 1) / 2);            // what nobody shares, there
-  return rows > 8 * sms || (blocks > 10 * sms && (d == 64 ? rows >= 2 * sms : 2 * ctas > 3 * sms));
+  return rows > 8 * sms || (blocks > 10 * sms && (d == 64 ? 2 * rows > 5 * sms : rows > 4 * sms || (BH >= 4 && 5 * rows > 16 * sms)));
 }
 
 // Groups of threads that share the blocks of a row (forward and row kernels; columns are shared by a cluster).  They pay

@@ -219,8 +219,9 @@ def test_fp32_tensor_core_kernels(bs, d, B, H, nb, full, layout):
 
 
 # (bs, d, B, blocks per side, blocks per row, tensor cores): both sides of the lines between the two files (148 SMs)
-@pytest.mark.parametrize("bs,d,B,nb,per,mma", [(32, 32, 12, 32, 8, False), (32, 32, 14, 32, 8, True), (32, 32, 14, 32, 3, False), (32, 32, 75, 16, 1, True),
-                                               (32, 64, 9, 32, 8, False), (32, 64, 10, 32, 8, True), (64, 32, 9, 16, 6, False), (64, 32, 10, 16, 6, True),
+@pytest.mark.parametrize("bs,d,B,nb,per,mma", [(32, 32, 14, 32, 8, False), (32, 32, 15, 32, 8, True), (32, 32, 15, 32, 3, False), (32, 32, 75, 16, 1, True),
+                                               (32, 32, 2, 250, 6, False), (32, 32, 3, 180, 4, False), (32, 32, 3, 198, 4, True),
+                                               (32, 64, 11, 32, 8, False), (32, 64, 12, 32, 8, True), (64, 32, 9, 16, 6, False), (64, 32, 10, 16, 6, True),
                                                (64, 64, 11, 16, 6, False), (64, 64, 12, 16, 6, True), (64, 64, 19, 16, 2, True)])
 def test_fp32_calls_on_either_side_of_the_line(bs, d, B, nb, per, mma):
     from spion_b200.native import BlockSparseAttention
