@@ -77,11 +77,12 @@ __device__ __forceinline__ void store_row_swizzled(uint32_t tile, int i, const u
 // product reads): rows of one chunk are rescaled in place once the denominator is known; longer rows accumulate it on
 // line in pass A.
 // heads: 0 = operands [BH, L, D]; H = operands [B, L, H, D] (see op_pos).
-// stat, or null: what P of a row are made of, [BH*L] exponents h, then [BH*L] factors f:
+// STAT: stat takes what P of a row are made of, [BH*L] exponents h, then [BH*L] factors f:
 // P = bf16(bf16(exp2(s scale log2e - penalty - h)) f), the factor as two bf16 values (row_factor), so that tc_bwd_stream.cu rebuilds P bit by bit.
-// store: write the P tiles.  KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of
+// store: write the P tiles (without STAT always: the branch alone costs the calls that store 2 %, 115.5 -> 117.7 us for 64 matrices, L = 4096,
+// d 32, 10 %).  KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of
 // every loop).
-template <int D, bool SUB, bool KP>
+template <int D, bool SUB, bool KP, bool STAT>
 __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_constant__ CUtensorMap tmQ,
                                                               const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV,
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       if (last) mma_commit(bar_o);
       }
       __syncwarp();
-      if (store && lane == 0) {                                     // these tiles are final: store them now
+      if ((!STAT || store) && lane == 0) {                                     // these tiles are final: store them now
         for (int t = 0; t < nt; ++t)
           tma_store_2d(&tmP, sP + (b0 + t) * VT_BYTES, 0, (int)(((size_t)bh * nnzb + rp + t0 + t) * BS));
         bulk_commit();
@@ -508,7 +509,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 3) k_fwd_fused(const __grid_const
       if (hf == 0) {
         const size_t i = (size_t)bh * L + r * BS + row;
         lse_out[i] = lse2;
-        if (stat) { stat[i] = m2; stat[(size_t)BH * L + i] = factor; }        // long rows: m2 is the log-sum-exp
+        if (STAT) { stat[i] = m2; stat[(size_t)BH * L + i] = factor; }        // long rows: m2 is the log-sum-exp
       }
       // the accumulator rows sit in lanes 0-15 of every quadrant: those lanes write the whole row
       __nv_bfloat16* dst = O + (size_t)(pos.row0 + r * BS + row) * pos.ld + pos.x0;
@@ -565,14 +566,16 @@ template <int D>
 static int fwd_attrs(TcState* s, int device) {
   const int bytes = (int)fwd_smem_bytes<D>();
   int occ = 1 << 30, n = 0, rc;
-#define SPION_FWD_ATTR(SB, KP)                                                                                       \
-  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_fused<D, SB, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));  \
-  if ((rc = resident_ctas(k_fwd_fused<D, SB, KP>, device, FWD_THREADS, (size_t)bytes, 128, &n))) return rc;          \
+#define SPION_FWD_ATTR(SB, KP, ST)                                                                                       \
+  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_fused<D, SB, KP, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));  \
+  if ((rc = resident_ctas(k_fwd_fused<D, SB, KP, ST>, device, FWD_THREADS, (size_t)bytes, 128, &n))) return rc;          \
   occ = n < occ ? n : occ;
-  SPION_FWD_ATTR(false, false)
-  SPION_FWD_ATTR(false, true)
-  SPION_FWD_ATTR(true, false)
-  SPION_FWD_ATTR(true, true)
+  SPION_FWD_ATTR(false, false, false)
+  SPION_FWD_ATTR(false, true, false)
+  SPION_FWD_ATTR(true, false, false)
+  SPION_FWD_ATTR(true, true, false)
+  SPION_FWD_ATTR(false, false, true)
+  SPION_FWD_ATTR(false, true, true)
 #undef SPION_FWD_ATTR
   s->fwd_ctas = occ;
   return SPION_OK;
@@ -611,8 +614,9 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
                                                               vw.submask, c->L, vw.nnzb, c->BH, vw.nb, c->heads, c->scale, floor_v,
                                                               c->status_dev);
     };
-    if (vw.submask) { if (keypad) launch(k_fwd_fused<D, true, true>); else launch(k_fwd_fused<D, true, false>); }
-    else { if (keypad) launch(k_fwd_fused<D, false, true>); else launch(k_fwd_fused<D, false, false>); }
+    if (stat) { if (keypad) launch(k_fwd_fused<D, false, true, true>); else launch(k_fwd_fused<D, false, false, true>); }       // no submask
+    else if (vw.submask) { if (keypad) launch(k_fwd_fused<D, true, true, false>); else launch(k_fwd_fused<D, true, false, false>); }
+    else { if (keypad) launch(k_fwd_fused<D, false, true, false>); else launch(k_fwd_fused<D, false, false, false>); }
     SPION_LAUNCH_CHECK();
     c->launches += 1;
   }

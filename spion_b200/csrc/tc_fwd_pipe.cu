@@ -53,9 +53,9 @@ __device__ __forceinline__ void store_half_row(uint32_t tile, int i, int g, cons
   }
 }
 
-// STORE_P: P normalised before it is rounded, and stored (unless `store` is false); stat: see k_fwd_fused.
+// STORE_P: P normalised before it is rounded, and stored; STAT, store, stat: see k_fwd_fused.
 // KP: the call has a key-padding penalty (a variant of its own: the blocks with padded keys need a second copy of every loop).
-template <int D, bool STORE_P, bool SUB, bool KP>
+template <int D, bool STORE_P, bool SUB, bool KP, bool STAT>
 __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_constant__ CUtensorMap tmQ,
                                                               const __grid_constant__ CUtensorMap tmK,
                                                               const __grid_constant__ CUtensorMap tmV,
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
         // With a separate P buffer (D == 32) the math warps overwrite it as soon as they see bar_o: when the tiles
         // are also stored, bar_o must then wait for the stores' reads as well (see below).
         mma_commit((STORE_P && D != 64) ? bar_x : bar_o + 8 * s);
-        if (STORE_P && store) {
+        if (STORE_P && (!STAT || store)) {
           for (int t = 0; t < R.nblk; ++t)
             tma_store_2d(&tmP, sP(s, t), 0, (int)(((size_t)bh * nnzb + R.rp + t) * BS));
           bulk_commit();
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 2) k_fwd_pipe(const __grid_const
           const float il = 1.0f / l;
           uint32_t inv_hi, inv_lo;
           row_factor(il, inv_hi, inv_lo);
-          if (stat && hf == 0) {
+          if (STAT && hf == 0) {
             const size_t x = (size_t)bh * L + R.r * BS + row;
             stat[x] = m2;
             stat[(size_t)BH * L + x] = il;
@@ -457,18 +457,20 @@ template <int D>
 static int pipe_attrs(TcState* s, int device) {
   const int bytes = (int)pipe_smem_bytes<D>();
   int occ = 1 << 30, n = 0, rc;
-#define SPION_PIPE_ATTR(SP, SB, KP)                                                                                    \
-  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_pipe<D, SP, SB, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
-  if ((rc = resident_ctas(k_fwd_pipe<D, SP, SB, KP>, device, PIPE_THREADS, (size_t)bytes, 256, &n))) return rc;        \
+#define SPION_PIPE_ATTR(SP, SB, KP, ST)                                                                                    \
+  SPION_CUDA_TRY(cudaFuncSetAttribute(k_fwd_pipe<D, SP, SB, KP, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); \
+  if ((rc = resident_ctas(k_fwd_pipe<D, SP, SB, KP, ST>, device, PIPE_THREADS, (size_t)bytes, 256, &n))) return rc;        \
   occ = n < occ ? n : occ;
-  SPION_PIPE_ATTR(false, false, false)
-  SPION_PIPE_ATTR(false, false, true)
-  SPION_PIPE_ATTR(true, false, false)
-  SPION_PIPE_ATTR(true, false, true)
-  SPION_PIPE_ATTR(false, true, false)
-  SPION_PIPE_ATTR(false, true, true)
-  SPION_PIPE_ATTR(true, true, false)
-  SPION_PIPE_ATTR(true, true, true)
+  SPION_PIPE_ATTR(false, false, false, false)
+  SPION_PIPE_ATTR(false, false, true, false)
+  SPION_PIPE_ATTR(true, false, false, false)
+  SPION_PIPE_ATTR(true, false, true, false)
+  SPION_PIPE_ATTR(false, true, false, false)
+  SPION_PIPE_ATTR(false, true, true, false)
+  SPION_PIPE_ATTR(true, true, false, false)
+  SPION_PIPE_ATTR(true, true, true, false)
+  SPION_PIPE_ATTR(true, false, false, true)
+  SPION_PIPE_ATTR(true, false, true, true)
 #undef SPION_PIPE_ATTR
   s->pipe_ctas = occ;
   return SPION_OK;
@@ -485,13 +487,14 @@ static int pipe_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CU
   const long long cap = (long long)s->sms * s->pipe_ctas;
   const int grid = (int)(total < cap ? total : cap);
   const float floor_v = keypad ? 0.0f : -100.0f;
-#define SPION_PIPE_LAUNCH(SP, SB, KP)                                                                                    \
-  k_fwd_pipe<D, SP, SB, KP><<<grid, PIPE_THREADS, pipe_smem_bytes<D>(), c->stream>>>(                                     \
+#define SPION_PIPE_LAUNCH(SP, SB, KP, ST)                                                                                \
+  k_fwd_pipe<D, SP, SB, KP, ST><<<grid, PIPE_THREADS, pipe_smem_bytes<D>(), c->stream>>>(                                 \
       mq, mk, mv, mp, (__nv_bfloat16*)O, lse, stat, store_p, keypad, vw.row_info, vw.col_idx, vw.submask, c->L, vw.nnzb, c->BH, rank0, \
       vw.nb, c->heads, c->scale, floor_v, c->status_dev)
-#define SPION_PIPE_PICK(SP, SB) do { if (keypad) SPION_PIPE_LAUNCH(SP, SB, true); else SPION_PIPE_LAUNCH(SP, SB, false); } while (0)
-  if (store_p || stat) { if (vw.submask) SPION_PIPE_PICK(true, true); else SPION_PIPE_PICK(true, false); }
-  else { if (vw.submask) SPION_PIPE_PICK(false, true); else SPION_PIPE_PICK(false, false); }
+#define SPION_PIPE_PICK(SP, SB, ST) do { if (keypad) SPION_PIPE_LAUNCH(SP, SB, true, ST); else SPION_PIPE_LAUNCH(SP, SB, false, ST); } while (0)
+  if (stat) SPION_PIPE_PICK(true, false, true);                   // no submask
+  else if (store_p) { if (vw.submask) SPION_PIPE_PICK(true, true, false); else SPION_PIPE_PICK(true, false, false); }
+  else { if (vw.submask) SPION_PIPE_PICK(false, true, false); else SPION_PIPE_PICK(false, false, false); }
 #undef SPION_PIPE_PICK
 #undef SPION_PIPE_LAUNCH
   SPION_LAUNCH_CHECK();
