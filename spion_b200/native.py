@@ -154,11 +154,14 @@ class BlockSparseAttention(nn.Module):
         padded keys, no P returned: 248 in two-block rows 25.0, 18.8; 1640 in rows of 3.2 48.2, 44.3; 2464 in rows of 4.8 58.6, 50.7; 4096 in rows of 4
           74.0, 76.5; 13120 in rows of 6.4 168, 184; 15872 in two-block rows 251, 244
         padded keys, P returned: 1640 in rows of 6.4 48.9, 45.8 (52.7, 49.4); 7936 in two-block rows 141, 133 (188, 176); 13120 in rows of 3.2 207, 199
-          (261, 249); 4916 in rows of 19 92.4, 99.2 (104, 107); 26240 in rows of 6.4 338, 347 (410, 412)"""
+          (261, 249), of 6.4 182, 184 (218, 216); 4916 in rows of 19 92.4, 99.2 (104, 107); 26240 in rows of 6.4 338, 347 (410, 412)"""
         blocks = self.BH * self.nnzb
         if not self.keypad:
             return blocks >= 512
-        return blocks >= 4096 and (not self.return_probs or self.nnzb >= 5 * (self.L // self.bs))
+        if not self.return_probs:
+            return blocks >= 4096
+        mean = self.nnzb / (self.L // self.bs)
+        return blocks >= 4096 and mean >= 10 or blocks >= 16384 and mean >= 5
 
     @property
     def nnz(self) -> int:

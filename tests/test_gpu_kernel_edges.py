@@ -451,8 +451,8 @@ def test_rebuilt_rounded_tiles_are_the_stored_ones(d, padded, short, probs):
 # (d, padded, P returned, matrices, blocks per side, blocks per row, rebuilt): both sides of the lines between rebuilt and stored rounded tiles
 @pytest.mark.parametrize("d,padded,probs,BH,nb,per,rebuilt",
                          [(32, False, False, 31, 8, 2, False), (32, False, False, 32, 8, 2, True), (64, False, True, 17, 10, 3, False), (64, False, True, 18, 10, 3, True),
-                          (32, True, False, 102, 10, 4, False), (32, True, False, 103, 10, 4, True), (32, True, True, 101, 10, 4, False), (64, True, True, 103, 10, 4, False),
-                          (64, True, True, 103, 10, 5, True), (32, True, True, 103, 8, 5, True), (32, True, True, 81, 10, 5, False)])
+                          (32, True, False, 102, 10, 4, False), (32, True, False, 103, 10, 4, True), (32, True, True, 410, 10, 4, False), (64, True, True, 327, 10, 5, False),
+                          (64, True, True, 328, 10, 5, True), (32, True, True, 34, 12, 10, False), (32, True, True, 35, 12, 10, True)])
 def test_rounded_tiles_are_rebuilt_or_stored(d, padded, probs, BH, nb, per, rebuilt):
     from torch.profiler import ProfilerActivity, profile
 
