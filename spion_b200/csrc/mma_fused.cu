@@ -20,7 +20,7 @@
 // Without products the kernels take 60 % of their time, products alone 45 %.
 // us of forward, rows, columns, the FMA kernels before (8 x 4 micro-tiles) and now: 512 matrices, L = 1024, d 32, 155 blocks of 32 362, 314, 262
 // -> 261, 245, 228; 128 matrices, L = 2048, 104 blocks of 64, d 32 263, 240, 234 -> 199, 184, 162, d 64 409, 384, 344 -> 335, 361, 308;
-// 15 matrices, L = 3008, d 64, 8 % and a full column 140, 132, 158 -> 109, 119, about 140.  Relative error against fp64 of O, dQ, dK, dV in the first: 2.9,
+// 15 matrices, L = 3008, d 64, 8 % and a full column 140, 132, 158 -> 109, 119, 86 (132 without the overlap, see SHARED).  Relative error against fp64 of O, dQ, dK, dV in the first: 2.9,
 // 3.0, 3.0, 2.8e-7 before, 1.6, 2.0, 2.0, 1.5e-7 now.
 //
 // A warp does MT x 16 rows of a tile, 32 columns at a time.  Fragment layouts leave the order of the contraction and of the columns open as
