@@ -821,8 +821,8 @@ bool simt_fused_supports(int bs, int d, int BH, int value_mode) {
 // the threads of a row do here, and nobody shares a row there, so the uneven rows of small calls are better shared by groups of threads (up to four
 // rows of blocks of 32 per SM, see row_groups).  us of forward, rows and columns there and here, in a graph (a band of two blocks and random ones):
 //   blocks of 32, d 32: rows of 5 blocks 256 51, 46; 304 56, 50; 416 57, 57; 480 60, 71; 512 (of 4.8) 53, 64; 1024 90, 120.  Rows of 8 384 85, 75; 448 87, 78;
-//     480 86, 91.  Rows of 12, 24, 45, two or three matrices, whose CTAs have room for a third or fourth there: 456 rows 0.85, 0.87, 0.86 times the
-//     speed there, 500 0.86, 0.88, 0.83, 540 0.89, 0.90, 0.84; four or eight matrices: 448 0.86 - 0.98, 512 1.01 - 1.09; 768 and more 1.09 - 1.20.
+//     480 86, 91.  Rows of 12, 24, 45: two or three matrices 456 rows 0.85, 0.87, 0.86 times the speed there, 500 0.86, 0.88, 0.83, 540 0.89, 0.90,
+//     0.84; four or eight matrices 448 0.86 - 0.98, 512 1.01 - 1.09; 768 and more 1.09 - 1.20.
 //   d 64, whose threads here have twice the work: rows of 5 256 77, 78; 304 93, 83; 320 89, 88; 512 102, 120.  Rows of 12, 24, 45: 300 0.86, 0.79,
 //     0.89 times the speed there, 320 0.87 - 0.92, 380 0.91 - 0.95, 384 0.84 - 0.99 (with a full column 0.89 - 1.24), 456 and more 1.01 - 1.20
 //   blocks of 64, d 32: 144 rows of 5 87, 85; 160 of 5 100, 114;  d 64: 160 of 5 170, 165; 176 of 5 191, 162; 192 of 5 166, 171; 224 of 5 183, 206
