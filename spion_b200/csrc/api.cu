@@ -92,6 +92,15 @@ void device_free(void* p) {
   d->follow();
 }
 
+int scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+  DevicePool* d = device_pool();
+  if (d && cudaMallocFromPoolAsync(p, bytes, d->pool, st) == cudaSuccess) return SPION_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return SPION_ERR_ALLOC;
+}
+void scratch_free(void* p, cudaStream_t st) { cudaFreeAsync(p, st); }
+
 int sm_count() {
   static std::atomic<int> cached[64];
   int dev = 0;

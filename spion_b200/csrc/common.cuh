@@ -153,6 +153,9 @@ int linear_status(int reset, cudaStream_t st);
 // cannot, under a capture, the memory is freed later).  Any thread.
 int device_alloc(void** p, size_t bytes);
 void device_free(void* p);
+// Memory of one call, from the same pool in the order of the call's stream (under a capture: nodes of the graph).
+int scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+void scratch_free(void* p, cudaStream_t st);
 
 // ------------------------------------------------------------------ element conversions
 __device__ __forceinline__ float to_f32(float x) { return x; }

@@ -5,8 +5,8 @@
 // recursive flood_fill (main_conv_ff.py:35-62); the top-k selection of main_conv.py:246-251;
 // F == 1 gives main_ff.py:255 (no convolution).
 //
-// Integer outputs are bit-exact against oracle/pattern.py because the float stages use the
-// same fixed order of fp64 additions (documented at each loop) and the same fused lerp.
+// Integer outputs equal those of oracle/pattern.py: the float stages are fp64 sums (conv_pool_kernel in the oracle's order of additions, documented at
+// each loop; diag_parts_kernel in another) rounded to fp32 once, and the lerp is fused as there.
 #include "common.cuh"
 #include "structure.cuh"
 
@@ -60,115 +60,200 @@ __global__ void __launch_bounds__(256) conv_pool_kernel(const float* __restrict_
   }
 }
 
-// Diagonal filter, block 32 or 64 (the reference's settings: F = 31, main_conv_ff.py:258): the same sums in the
-// same order as conv_pool_kernel, organised so that the filter taps are read once per eight outputs instead of
-// once per output.  A thread computes a run of eight outputs (i0 + k, j0 + k), k = 0..7, along a diagonal of the
-// block: they need the tile diagonal d_m = tile[i0 + m][j0 + m], m = 0 .. F + 6, and output k is
-// ((d_k + d_k+1) + d_k+2) + ... in ascending order -- eight independent fp64 chains.  Runs start at
-// i0 = 0, 8, .., j0 = -7 .. BS - 1 (outputs left of the block are skipped).  The pooled rows are padded by one
-// double so that the row sums (one thread per row) do not collide in shared memory.
-// Persistent CTAs, three per SM, over the cells of all maps of the call: while two warps form the row sums of a cell (64 dependent
-// additions), the tile of the next one arrives by cp.async; the total of the row sums is one lane's work beside the next cell's
-// sums.  Tile rows are 16-byte pieces (A 16-byte aligned; a piece is inside or outside the map as a whole), 96 floats from column
-// j - 16 on; taps left or right of a row read its neighbours' values, but only for the skipped outputs.
-// Limited by the ordered fp64 additions of the filter (31 per output): 62.8 us per L = 4096 map, 63.9 with one CTA per cell.  Of that time the
-// fp64 pipe is busy for 54 %, issue slots for 58 %, l1tex for 39 % (ncu, one map): no unit is full.  What the loop over maps saves is a
-// launch and a wave's tail per layer.
+// Diagonal filter of 31 taps, blocks of 32 or 64 (the reference's settings: main_conv_ff.py:258).  Filter and pooling are one weighted sum:
+// an element counts in a cell as often as the diagonal through it has taps whose output lies in the cell's block.  With h = 15 an element
+// (a, b) of its own block reaches that block's cell and, from the outer 16 rows and columns, the six cells above / left / below / right / on
+// the diagonal:
+//   own cell      min(15, min(a, b)) - max(-15, max(a, b) - BS + 1) + 1
+//   above (-1,0)  min(15, b) - a        left (0,-1)  min(15, a) - b           (-1,-1)  15 - max(a, b)
+//   below (+1,0)  min(a', a - b)        right (0,+1) min(b', b - a)           (+1,+1)  min(a', b')         a' = a - BS + 16, b' likewise
+// where these are positive.  So every element is read once, converted once, and no filtered map is formed: the kernel writes seven
+// partial sums per block, diag_combine_kernel adds the seven that belong to a cell.  All sums are fp64 with weights that are whole
+// numbers (formed as sums of running sums, nothing is subtracted), rounded to fp32 once: the error is that of the ordered sums of conv_pool_kernel, some
+// 1e-16, before the rounding.  An element whose weight is zero is left out, not multiplied: infinities stay where the filter has them.
+//
+// A lane owns a row of a block: one warp takes the 16 rows at the top and the 16 at the bottom, a second one the 32 between them (BS = 64);
+// two buffers per block filled by cp.async, rows padded by 16 bytes (conflict-free 16-byte reads of one row per lane).  In the corners of a
+// block the weights bend at the diagonal: running sums from both ends, added to one of two totals on either side of it.
+// Bound by the pass over the map: two L = 4096 maps 125 us with the 31 ordered additions per element, 28 now, 4.8 TB/s (33 with one warp per block).
 struct MapList { const float* A[16]; };
-template <int BS, int F>
-__global__ void __launch_bounds__(256, 3) conv_pool_diag_kernel(const __grid_constant__ MapList maps, int layers, int L, float* __restrict__ pooled) {
-  constexpr int H = F / 2, T = BS + 2 * H, RUN = 8, CS = BS + 1, TP = BS + 32, SLACK = 8;
-  static_assert(H <= 16, "halo");
+constexpr int DIAG_GROUPS = 6, DIAG_PARTS = 10;
+template <int BS>
+__global__ void __launch_bounds__(BS * DIAG_GROUPS) diag_parts_kernel(const __grid_constant__ MapList maps, int layers, int L, double* part) {
+  static_assert(BS == 32 || BS == 64, "16 outer rows on either side, 0 or 32 between them");
+  constexpr int TP = BS + 4, PIECES = BS / 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* tile = reinterpret_cast<float*>(smem_raw) + SLACK;
-  double* cval = reinterpret_cast<double*>(smem_raw + (size_t)(T * TP + 2 * SLACK) * sizeof(float));
-  double* rsum = cval + (size_t)BS * CS;
+  const int lane = threadIdx.x & 31, gt = threadIdx.x % BS, group = threadIdx.x / BS;      // BS threads per block
+  const bool outer = gt < 32;
+  float* buf = reinterpret_cast<float*>(smem_raw) + (size_t)group * 2 * BS * TP;
   const int nb = L / BS, per = nb * nb;
-  const int total = layers * per, G = (int)gridDim.x;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int RUNS = (BS / RUN) * (BS + RUN - 1), CHUNKS = (RUNS + 31) / 32;
-  auto load = [&](int cell) {
-    const int m = cell / per, rest = cell - m * per;
-    const float* A = maps.A[m];
-    const int i0g = (rest / nb) * BS - H, j0g = (rest % nb) * BS - 16;
-    constexpr int PIECES = TP / 4;
-    for (int e = tid; e < T * PIECES; e += 256) {
-      const int ti = e / PIECES, p4 = e - ti * PIECES;
-      const int gi = i0g + ti, gj = j0g + 4 * p4;
-      const bool in = gi >= 0 && gi < L && gj >= 0 && gj < L;
-      const float* src = A + (in ? (size_t)gi * L + gj : 0);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(tile + ti * TP + 4 * p4)),
-                   "l"(src), "r"(in ? 16u : 0u) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+  const int total = layers * per, step = (int)gridDim.x * DIAG_GROUPS;
+  auto meet = [&]() {
+    if constexpr (BS == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(BS) : "memory");
   };
-  if (tid < 2 * SLACK) { if (tid < SLACK) tile[-1 - tid] = 0.0f; else tile[T * TP + tid - SLACK] = 0.0f; }
-  load(blockIdx.x);
-  int before = -1;                                     // cell whose total is still to be formed
-  for (int cell = blockIdx.x; cell < total; cell += G) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    // p = sum_ii r[ii] (ii ascending): pool_fixed_order
-    auto finish = [&]() {
-      double p = 0.0;
-#pragma unroll 16
-      for (int ii = 0; ii < BS; ++ii) p = p + rsum[ii];
-      pooled[before] = (float)(p / (double)(BS * BS));
-    };
-    if (before >= 0 && tid == 224) finish();
-    __syncwarp();
-    // the warp of the total takes the fewest runs: its chain is as long as two of them
-    for (int q = warp == 7 ? CHUNKS - 1 : warp; q < CHUNKS; q += 7) {
-      if (warp != 7 && q == CHUNKS - 1) break;
-      const int r = q * 32 + lane;
-      if (r >= RUNS) break;
-      const int i0 = (r / (BS + RUN - 1)) * RUN, j0 = r % (BS + RUN - 1) - (RUN - 1);
-      const float* d0 = tile + i0 * TP + j0 + (16 - H);
-      double c[RUN];
+  next_may_start();
+  auto load = [&](int cell, float* to) {
+    const int m = cell / per, rest = cell - m * per;
+    const float* src = maps.A[m] + (size_t)(rest / nb) * BS * L + (rest % nb) * BS;
+#pragma unroll 8
+    for (int e = gt; e < BS * PIECES; e += BS) {
+      const int r = e / PIECES, c = 4 * (e % PIECES);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + r * TP + c)),
+                   "l"(src + (size_t)r * L + c) : "memory");
+    }
+  };
+  auto read16 = [](const float* p, double* x) {
 #pragma unroll
-      for (int k = 0; k < RUN; ++k) c[k] = 0.0;
-      // c[k] = sum_{t = 0 .. F-1} d[k + t], t ascending (oracle: conv_fixed_order)
+    for (int i = 0; i < 4; ++i) {
+      const float4 v = *reinterpret_cast<const float4*>(p + 4 * i);
+      x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+    }
+  };
+  int cell = blockIdx.x * DIAG_GROUPS + group;
+  if (cell < total) load(cell, buf);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int n = 0; cell < total; cell += step, n ^= 1) {
+    const float* t = buf + n * BS * TP;
+    if (cell + step < total) load(cell + step, buf + (n ^ 1) * BS * TP);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    meet();
+    double own = 0.0, left = 0.0, right = 0.0, vert = 0.0, diag = 0.0;      // vert, diag: upwards in lanes 0-15, downwards in 16-31
+    double x[16];
+    if (outer) {
+      const bool low = lane < 16;
+      const int a = lane & 15, w = low ? 15 - a : a;                        // w: weight of the row in the cell above / below
+      const float* row = t + (low ? a : BS - 16 + a) * TP;
+      // the 16 columns at the same end: weights bend at b = a
+      read16(row + (low ? 0 : BS - 16), x);
+      double up = 0.0, from0 = 0.0, from1 = 0.0;                            // up = x[0] + .. + x[b]; sums of it for b < a, a <= b < 15
 #pragma unroll
-      for (int m = 0; m < F + RUN - 1; ++m) {
-        const double d = (double)d0[m * (TP + 1)];
-#pragma unroll
-        for (int k = 0; k < RUN; ++k)
-          if (m >= k && m < k + F) c[k] = c[k] + d;
+      for (int b = 0; b < 16; ++b) {
+        up += x[b];
+        if (b < a) from0 += up;                                             // in all: sum of (a - b)+ x
+        else if (b < 15) from1 += up;                                       // sum of (15 - max(a, b)) x
       }
+      double down = 0.0, to0 = 0.0, to1 = 0.0;                              // down = x[15] + .. + x[b]
 #pragma unroll
-      for (int k = 0; k < RUN; ++k) {
-        const int j = j0 + k;
-        if (j >= 0 && j < BS) cval[(i0 + k) * CS + j] = c[k];
+      for (int b = 15; b > 0; --b) {
+        down += x[b];
+        if (b > a) to1 += down;                                             // sum of (b - a)+ x
+        else to0 += down;                                                   // sum of min(a, b) x
       }
+      own = fma(16.0, up, low ? to0 : from1);
+      diag = low ? from1 : to0;
+      vert = low ? to1 : from0;
+      left = low ? from0 : 0.0;
+      right = low ? 0.0 : to1;
+      // the 16 columns at the other end
+      read16(row + (low ? BS - 16 : 0), x);
+      double s0 = 0.0, rise = 0.0, fall = 0.0;
+#pragma unroll
+      for (int b = 0; b < 16; ++b) {
+        s0 += x[b];
+        if (b > 0) rise = fma((double)b, x[b], rise);
+        if (b < 15) fall = fma((double)(15 - b), x[b], fall);
+      }
+      own += fma((double)(16 - w), s0, low ? fall : rise);
+      if (low) right = rise; else left = fall;
+      if constexpr (BS > 32) {                                              // the columns between
+        double m0 = 0.0, m1 = 0.0;
+        read16(row + 16, x);
+#pragma unroll
+        for (int b = 0; b < 16; ++b) m0 += x[b];
+        read16(row + 32, x);
+#pragma unroll
+        for (int b = 0; b < 16; ++b) m1 += x[b];
+        m0 += m1;
+        own = fma((double)(31 - w), m0, own);
+        s0 += m0;
+      }
+      if (w > 0) vert = fma((double)w, s0, vert);
     }
-    __syncthreads();
-    if (cell + G < total) load(cell + G);
-    if (tid < BS) {                                    // r[i] = sum_jj c[i, jj]  (jj ascending)
-      double rr = 0.0;
-#pragma unroll 16
-      for (int jj = 0; jj < BS; ++jj) rr = rr + cval[tid * CS + jj];
-      rsum[tid] = rr;
+    if (!outer) {                                                           // the rows between: weights follow the column
+      const float* row = t + (16 + lane) * TP;
+      double o0 = 0.0, o1 = 0.0, l = 0.0, r = 0.0;
+      read16(row, x);
+#pragma unroll
+      for (int b = 0; b < 16; ++b) {
+        o0 = fma((double)(16 + b), x[b], o0);
+        if (b < 15) l = fma((double)(15 - b), x[b], l);
+      }
+      read16(row + 48, x);
+#pragma unroll
+      for (int b = 0; b < 16; ++b) {
+        o1 = fma((double)(31 - b), x[b], o1);
+        if (b > 0) r = fma((double)b, x[b], r);
+      }
+      double m0 = 0.0, m1 = 0.0;
+      read16(row + 16, x);
+#pragma unroll
+      for (int b = 0; b < 16; ++b) m0 += x[b];
+      read16(row + 32, x);
+#pragma unroll
+      for (int b = 0; b < 16; ++b) m1 += x[b];
+      own = fma(31.0, m0 + m1, o0 + o1);
+      left = l;
+      right = r;
     }
-    before = cell;
-    if (cell + G >= total) {
-      __syncthreads();
-      if (tid == 224) finish();
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      own += __shfl_xor_sync(0xffffffffu, own, o);
+      left += __shfl_xor_sync(0xffffffffu, left, o);
+      right += __shfl_xor_sync(0xffffffffu, right, o);
+      if (!outer) continue;
+      vert += __shfl_xor_sync(0xffffffffu, vert, o);
+      diag += __shfl_xor_sync(0xffffffffu, diag, o);
     }
+    own += __shfl_xor_sync(0xffffffffu, own, 16);
+    left += __shfl_xor_sync(0xffffffffu, left, 16);
+    right += __shfl_xor_sync(0xffffffffu, right, 16);
+    // own | left | right | above | above left | below | below right | own, left, right of the rows between
+    double* dst = part + (size_t)cell * DIAG_PARTS;
+    if (lane == 0) { double* d3 = dst + (outer ? 0 : 7); d3[0] = own; d3[1] = left; d3[2] = right; }
+    if (outer && lane == 0) { dst[3] = vert; dst[4] = diag; }
+    if (outer && lane == 16) { dst[5] = vert; dst[6] = diag; }
+    meet();                                                                 // the buffer is refilled from here on
   }
 }
 
-template <int BS, int F>
-int launch_conv_pool_diag(const MapList& maps, int layers, int L, int nb, float* pooled, cudaStream_t st) {
-  constexpr int T = BS + F - 1;
-  const size_t smem = (size_t)(T * (BS + 32) + 16) * sizeof(float) + ((size_t)BS * (BS + 1) + BS) * sizeof(double);
-  int dev = 0, sms = 0;
-  SPION_CUDA_TRY(cudaGetDevice(&dev));
-  SPION_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (smem > 48 * 1024)
-    SPION_CUDA_TRY(cudaFuncSetAttribute(conv_pool_diag_kernel<BS, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const long long cells = (long long)layers * nb * nb, cap = 3LL * sms;        // three CTAs per SM (70 KB each)
-  conv_pool_diag_kernel<BS, F><<<(int)(cells < cap ? cells : cap), 256, smem, st>>>(maps, layers, L, pooled);
+// A cell: its own block's sum and what the blocks around it have for it, added in a fixed order.
+template <bool BETWEEN>
+__global__ void __launch_bounds__(256) diag_combine_kernel(const double* part, int nb, int total, double area, float* __restrict__ pooled) {
+  next_may_start();
+  wait_for_kernel_before();
+  const int cell = blockIdx.x * 256 + threadIdx.x;
+  if (cell >= total) return;
+  const int rest = cell % (nb * nb), r = rest / nb, c = rest - r * nb;
+  const bool up = r > 0, down = r + 1 < nb, lt = c > 0, rt = c + 1 < nb;
+  const double* p = part + (size_t)cell * DIAG_PARTS;
+  const int line = nb * DIAG_PARTS;
+  double s = p[0];
+  s += rt ? p[DIAG_PARTS + 1] : 0.0;
+  s += lt ? p[-DIAG_PARTS + 2] : 0.0;
+  if (BETWEEN) {
+    s += p[7];
+    s += rt ? p[DIAG_PARTS + 8] : 0.0;
+    s += lt ? p[-DIAG_PARTS + 9] : 0.0;
+  }
+  s += down ? p[line + 3] : 0.0;
+  s += down && rt ? p[line + DIAG_PARTS + 4] : 0.0;
+  s += up ? p[-line + 5] : 0.0;
+  s += up && lt ? p[-line - DIAG_PARTS + 6] : 0.0;
+  pooled[cell] = (float)(s / area);
+}
+
+template <int BS>
+int launch_diag(const MapList& maps, int layers, int L, int nb, double* part, float* pooled, cudaStream_t st) {
+  const int smem = DIAG_GROUPS * 2 * BS * (BS + 4) * (int)sizeof(float), total = layers * nb * nb;
+  const int sms = sm_count();
+  if (sms < 1) return SPION_ERR_CUDA;
+  SPION_CUDA_TRY(cudaFuncSetAttribute(diag_parts_kernel<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int ctas = (total + DIAG_GROUPS - 1) / DIAG_GROUPS, cap = (BS == 64 ? 1 : 4) * sms;      // 209 KB or 55 KB each
+  diag_parts_kernel<BS><<<ctas < cap ? ctas : cap, BS * DIAG_GROUPS, smem, st>>>(maps, layers, L, part);
   SPION_LAUNCH_CHECK();
+  SPION_CUDA_TRY(launch_after(diag_combine_kernel<BS == 64>, dim3((total + 255) / 256), dim3(256), 0, st, (const double*)part, nb, total, (double)(BS * BS), pooled));
   return SPION_OK;
 }
 
@@ -182,60 +267,71 @@ __device__ __forceinline__ float key_to_float(uint32_t k) {
   return __uint_as_float(u);
 }
 
-// k-th smallest (0-based) of vals[0..n) by 4 passes of 8-bit radix select.  All threads call it.  The values of a map share their
-// leading bytes, so a warp whose digits are all equal counts them in one go (one thread scanning it and 4096 colliding
-// atomics per pass were most of the 36 us of this kernel at nb = 64).
-__device__ float select_kth(const float* vals, int n, int k, int* hist, int* s_sel) {
-  uint32_t prefix = 0, mask = 0;
-  const int lane = threadIdx.x & 31;
-  for (int pass = 3; pass >= 0; --pass) {
-    const int shift = pass * 8;
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
-    __syncthreads();
-    for (int i0 = 0; i0 < n; i0 += blockDim.x) {
-      const int i = i0 + threadIdx.x;
-      const uint32_t key = i < n ? order_key(vals[i]) : 0u;
-      const bool in = i < n && (key & mask) == prefix;
-      const int digit = in ? (int)((key >> shift) & 255u) : 256;
-      int all;
-      __match_all_sync(0xffffffffu, digit, &all);
-      if (all) { if (in && lane == 0) atomicAdd(&hist[digit], 32); }
-      else if (in) atomicAdd(&hist[digit], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {                            // eight bins per lane
-      int sum = 0;
-#pragma unroll
-      for (int x = 0; x < 8; ++x) sum += hist[lane * 8 + x];
-      int upto = sum;                                  // inclusive scan
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += y;
-      }
-      if (k >= upto - sum && k < upto) {
-        int kk = k - (upto - sum), x = 0;
-        while (kk >= hist[lane * 8 + x]) { kk -= hist[lane * 8 + x]; ++x; }
-        s_sel[0] = lane * 8 + x;
-        s_sel[1] = kk;
-      }
-    }
-    __syncthreads();
-    prefix |= (uint32_t)s_sel[0] << shift;
-    mask |= 255u << shift;
-    k = s_sel[1];
-    __syncthreads();
+// k-th smallest (0-based) of vals[0..n), by a block of 1024 threads: the range of the keys is cut into 1024 bins, then the bin that holds the
+// k-th key, until a bin is one key (values of a map share their leading bits: three rounds, the second and third over the few keys of a
+// bin; four rounds of 8-bit digits from the top, most atomics of the first two on the same counters, took 5 us of this kernel's 23).
+// A warp whose keys fall into one bin counts them in one go.  All threads call it; s_sel: 4 words, s_hist: 1024.
+__device__ __forceinline__ float select_kth(const float* vals, int n, int k, int* s_hist, uint32_t* s_sel) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t least = 0xffffffffu, most = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    const uint32_t key = order_key(vals[i]);
+    least = min(least, key);
+    most = max(most, key);
   }
-  return key_to_float(prefix);
+  least = __reduce_min_sync(0xffffffffu, least);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (threadIdx.x == 0) { s_sel[0] = 0xffffffffu; s_sel[1] = 0; }
+  __syncthreads();
+  if (lane == 0) { atomicMin(&s_sel[0], least); atomicMax(&s_sel[1], most); }
+  __syncthreads();
+  uint32_t base = s_sel[0], range = s_sel[1] - base;               // keys base .. base + range
+#pragma unroll 1
+  while (range > 0) {
+    const int shift = max(0, 22 - __clz(range));                   // 32 - clz bits, ten of them for the bins
+    s_hist[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int i0 = 0; i0 < n; i0 += 1024) {
+      const int i = i0 + threadIdx.x;
+      const uint32_t key = i < n ? order_key(vals[i]) : 0u, off = key - base;
+      const bool in = i < n && key >= base && off <= range;
+      const int bin = in ? (int)(off >> shift) : -1;
+      const bool all = __all_sync(0xffffffffu, bin == __shfl_sync(0xffffffffu, bin, 0));
+      if (in && (!all || lane == 0)) atomicAdd(&s_hist[bin], all ? 32 : 1);
+    }
+    __syncthreads();
+    // inclusive sums of the bins: a warp scans its 32, every warp the sums of the warps before it
+    const int mine = s_hist[threadIdx.x];
+    int upto = mine;
+#pragma unroll 1
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    __syncthreads();
+    if (lane == 31) s_hist[warp] = upto;
+    __syncthreads();
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? s_hist[lane] : 0);
+    upto += before;
+    if (k >= upto - mine && k < upto) { s_sel[2] = threadIdx.x; s_sel[3] = (uint32_t)(k - (upto - mine)); }
+    __syncthreads();
+    base += s_sel[2] << shift;
+    range = (1u << shift) - 1u;
+    k = (int)s_sel[3];
+  }
+  return key_to_float(base);
 }
 
 // ---------------------------------------------------------------- selection (one CTA)
 // select == PATHS: thresh = torch.quantile(pooled, q) (linear), then 2*nb greedy walkers.
 // select == TOPK : the kcount largest cells (ties: lower flat index first).
-// One CTA per map; its block structure follows in the same kernel: a chain of latencies, 23 us for two 64 x 64 maps, against 36 us
-// of selection and 13 us of structure for each of them with one launch per map and step.  copies: how many times the 0/1 float mask is written, `mats_step`
-// floats apart (the driver's stacked list, main_conv_ff.py:298-299).
+// One CTA per map; its block structure follows in the same kernel: a chain of latencies, 17 us for two 64 x 64 maps (21 with the walkers
+// step by step and the mask in global memory; 36 us of selection and 13 us of structure for each of them with one launch per map and
+// step).  copies: how many times the 0/1 float mask is written, `mats_step` floats apart (the driver's stacked list, main_conv_ff.py:298-299).
 constexpr int SELECT_SMEM_CELLS = 128 * 128;           // maps up to this size are kept in shared memory
+constexpr int SELECT_SMEM_BYTES = 7;                   // per cell: value, where a walker goes from it, mask
 struct SelectOut {
   uint8_t* mat;
   float *thresh, *mats;
@@ -243,24 +339,30 @@ struct SelectOut {
   int copies;
   long long mats_step;
 };
-__global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ pooled_all, int nb, int select, float q,
+template <bool SMALL>                                  // up to SELECT_SMEM_CELLS
+__global__ void __launch_bounds__(1024) select_kernel(const float* pooled_all, int nb, int select, float q,
                                                       int kcount, const __grid_constant__ SelectOut out) {
   extern __shared__ float s_val[];
-  __shared__ int hist[256];
-  const size_t cells = (size_t)nb * nb;
-  uint8_t* __restrict__ mat = out.mat + blockIdx.x * cells;
-  float* thresh_out = out.thresh ? out.thresh + blockIdx.x : nullptr;
-  const float* pooled = pooled_all + blockIdx.x * cells;
-  if (cells <= SELECT_SMEM_CELLS) {
-    for (int i = threadIdx.x; i < (int)cells; i += blockDim.x) s_val[i] = pooled[i];
-    pooled = s_val;
-  }
-  __shared__ int s_sel[2];
+  __shared__ int hist[1024];
+  __shared__ uint32_t s_sel[4];
   __shared__ float s_thresh;
   __shared__ int s_warp[32];
   __shared__ int s_running;
+  const size_t cells = (size_t)nb * nb;
   const int n = nb * nb;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) mat[i] = 0;
+  uint16_t* s_to = reinterpret_cast<uint16_t*>(s_val + n);
+  uint8_t* mat_out = out.mat + blockIdx.x * cells;
+  uint8_t* mat = SMALL ? reinterpret_cast<uint8_t*>(s_to + n) : mat_out;
+  float* thresh_out = out.thresh ? out.thresh + blockIdx.x : nullptr;
+  const float* pooled = SMALL ? s_val : pooled_all + blockIdx.x * cells;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n; i += 1024) mat[i] = 0;
+  wait_for_kernel_before();
+  if (SMALL) {
+    const float* from = pooled_all + blockIdx.x * cells;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += 1024) s_val[i] = from[i];
+  }
   __syncthreads();
 
   if (select == SPION_SELECT_PATHS) {
@@ -277,7 +379,8 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
       const uint32_t klo = order_key(lo);
       int le = 0;
       uint32_t above = 0xffffffffu;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+#pragma unroll 1
+      for (int i = threadIdx.x; i < n; i += 1024) {
         const uint32_t key = order_key(pooled[i]);
         if (key <= klo) ++le; else above = min(above, key);
       }
@@ -309,30 +412,40 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
       const float D = (x + 1 < nb) ? pooled[(size_t)(x + 1) * nb + y] : 0.0f;
       const float R = (y + 1 < nb) ? pooled[(size_t)x * nb + y + 1] : 0.0f;
       const float G = (x + 1 < nb && y + 1 < nb) ? pooled[(size_t)(x + 1) * nb + y + 1] : 0.0f;
-      int to;
-      float v;
-      if (D > R) {
-        if (D > G) { to = 1; v = D; } else { to = 3; v = G; }
-      } else {
-        if (R > G) { to = 2; v = R; } else { to = 3; v = G; }
-      }
+      const float first = D > R ? D : R;
+      const int to = first > G ? (D > R ? 1 : 2) : 3;
+      const float v = first > G ? first : G;
       return to | (v > thresh && v > 0.0f ? 4 : 0);
     };
-    // small maps: all steps first, in parallel, so that a walker's chain is one byte per cell
-    const bool table = cells <= SELECT_SMEM_CELLS;
-    uint8_t* s_step = reinterpret_cast<uint8_t*>(s_val + (table ? cells : 0));
-    if (table) {
-      for (int i = threadIdx.x; i < n; i += blockDim.x) s_step[i] = (uint8_t)step(i / nb, i % nb);
+    if (SMALL) {
+      // all steps first, in parallel, so that a walker's chain is one load per cell: the next cell, whether it is marked, or the end.  (All
+      // walkers at once, cells passing on what is 2^k steps ahead in round k: 7 us for 64 x 64 cells on one SM, twice what these chains take.)
+#pragma unroll 1
+      for (int i = threadIdx.x; i < n; i += 1024) {
+        const int x = i / nb, y = i - x * nb, t = step(x, y);
+        s_to[i] = x + (t & 1) < nb && y + ((t >> 1) & 1) < nb ? (uint16_t)((i + (t & 1) * nb + ((t >> 1) & 1)) | (t & 4 ? 0x4000 : 0)) : (uint16_t)0x8000;
+      }
       __syncthreads();
-    }
-    for (int s = threadIdx.x; s < 2 * nb; s += blockDim.x) {
-      int x = (s < nb) ? 0 : s - nb;
-      int y = (s < nb) ? s : 0;
-      while (x < nb && y < nb) {
-        const int t = table ? s_step[x * nb + y] : step(x, y);
-        x += t & 1;
-        y += (t >> 1) & 1;
-        if ((t & 4) && x < nb && y < nb) mat[(size_t)x * nb + y] = 1;
+      if (threadIdx.x < 2 * nb) {
+        uint32_t t = s_to[threadIdx.x < nb ? threadIdx.x : (threadIdx.x - nb) * nb];
+#pragma unroll 1
+        while (t < 0x8000) {
+          const uint32_t at = t & 0x3fff;
+          if (t & 0x4000) mat[at] = 1;
+          t = s_to[at];
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (int s = threadIdx.x; s < 2 * nb; s += 1024) {
+        int x = (s < nb) ? 0 : s - nb;
+        int y = (s < nb) ? s : 0;
+        while (x < nb && y < nb) {
+          const int t = step(x, y);
+          x += t & 1;
+          y += (t >> 1) & 1;
+          if ((t & 4) && x < nb && y < nb) mat[(size_t)x * nb + y] = 1;
+        }
       }
     }
   } else {
@@ -344,7 +457,8 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
       if (threadIdx.x == 0) s_running = 0;
       __syncthreads();
       int local = 0;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+#pragma unroll 1
+      for (int i = threadIdx.x; i < n; i += 1024) {
         if (pooled[i] > v) { mat[i] = 1; ++local; }
       }
       atomicAdd(&s_running, local);
@@ -353,8 +467,9 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
       __syncthreads();
       if (threadIdx.x == 0) s_running = 0;
       __syncthreads();
-      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-      for (int base = 0; base < n; base += blockDim.x) {
+      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = 32;
+#pragma unroll 1
+      for (int base = 0; base < n; base += 1024) {
         const int i = base + threadIdx.x;
         const int flag = (i < n && pooled[i] == v) ? 1 : 0;
         const unsigned bal = __ballot_sync(0xffffffffu, flag);
@@ -362,11 +477,13 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
         if (lane == 0) s_warp[wid] = __popc(bal);
         __syncthreads();
         int before = s_running;
+#pragma unroll 1
         for (int w2 = 0; w2 < wid; ++w2) before += s_warp[w2];
         if (flag && before + in_warp < need) mat[i] = 1;
         __syncthreads();
         if (threadIdx.x == 0) {
           int tot = 0;
+#pragma unroll 1
           for (int w2 = 0; w2 < nwarps; ++w2) tot += s_warp[w2];
           s_running += tot;
         }
@@ -375,11 +492,16 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* __restrict__ 
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) mat[(size_t)i * nb + i] = 1;   // main_conv_ff.py:277-278
+#pragma unroll 1
+  for (int i = threadIdx.x; i < nb; i += 1024) mat[(size_t)i * nb + i] = 1;   // main_conv_ff.py:277-278
   __syncthreads();
-  for (int c = 0; c < out.copies; ++c) {
-    float* m = out.mats + c * out.mats_step + blockIdx.x * cells;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) m[i] = (float)mat[i];
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    const uint8_t on = mat[i];
+    if (SMALL) mat_out[i] = on;
+    float* m = out.mats + blockIdx.x * cells + i;
+#pragma unroll 4
+    for (int c = 0; c < out.copies; ++c) m[c * out.mats_step] = (float)on;
   }
   build_structure(mat, nb, out.nnzb + blockIdx.x, out.row_ptr + (size_t)blockIdx.x * (nb + 1), out.col_idx + blockIdx.x * cells,
                   out.blk_row + blockIdx.x * cells, out.col_ptr + (size_t)blockIdx.x * (nb + 1), out.row_idx + blockIdx.x * cells,
@@ -514,9 +636,13 @@ extern "C" int spion_discover_patterns(const float* const* host_A, int layers, i
   // call is cheap: make it on every launch that needs it instead of remembering one process-wide size.
   bool aligned = true;
   for (int i = 0; i < layers; ++i) aligned = aligned && ((uintptr_t)host_A[i] & 15u) == 0;
-  if (conv_kind == SPION_CONV_DIAG && F == 31 && (bs == 64 || bs == 32) && aligned) {      // the reference's filter: the faster kernel
-    int rc = bs == 64 ? launch_conv_pool_diag<64, 31>(maps, layers, L, nb, pooled, st) : launch_conv_pool_diag<32, 31>(maps, layers, L, nb, pooled, st);
-    if (rc) return rc;
+  // the reference's filter takes the kernel above; without memory for its partial sums the general one answers
+  double* part = nullptr;
+  const bool diag = conv_kind == SPION_CONV_DIAG && F == 31 && (bs == 64 || bs == 32) && aligned &&
+                    scratch_alloc((void**)&part, layers * cells * DIAG_PARTS * sizeof(double), st) == SPION_OK;
+  if (diag) {
+    const int rc = bs == 64 ? launch_diag<64>(maps, layers, L, nb, part, pooled, st) : launch_diag<32>(maps, layers, L, nb, part, pooled, st);
+    if (rc) { scratch_free(part, st); return rc; }
   } else {
     if (smem > 48 * 1024)
       SPION_CUDA_TRY(cudaFuncSetAttribute(conv_pool_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -528,11 +654,13 @@ extern "C" int spion_discover_patterns(const float* const* host_A, int layers, i
 
   int kcount = 0;
   if (select == SPION_SELECT_TOPK) kcount = (int)((double)(nb * nb) * param - (double)nb);   // main_conv.py:247
-  const size_t dyn = cells <= SELECT_SMEM_CELLS ? cells * (sizeof(float) + 1) : 0;
-  SPION_CUDA_TRY(cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SELECT_SMEM_CELLS * ((int)sizeof(float) + 1)));
+  const bool small = cells <= SELECT_SMEM_CELLS;
+  auto kernel = small ? select_kernel<true> : select_kernel<false>;
+  const size_t dyn = small ? cells * SELECT_SMEM_BYTES : 0;
+  if (small) SPION_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SELECT_SMEM_CELLS * SELECT_SMEM_BYTES));
   const SelectOut out{mat, thresh, mats, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, copies, (long long)(layers * cells)};
-  select_kernel<<<layers, 1024, dyn, st>>>(pooled, nb, select, (float)param, kcount, out);
-  SPION_LAUNCH_CHECK();
+  SPION_CUDA_TRY(launch_after(kernel, dim3(layers), dim3(1024), dyn, st, (const float*)pooled, nb, select, (float)param, kcount, out));
+  if (diag) scratch_free(part, st);                    // behind the last kernel: between two of them it would keep the second waiting
   if (host_nnzb) {
     SPION_CUDA_TRY(cudaMemcpyAsync(host_nnzb, nnzb, layers * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     SPION_CUDA_TRY(cudaStreamSynchronize(st));

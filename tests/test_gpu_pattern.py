@@ -165,3 +165,32 @@ def test_discovery_at_the_largest_block_counts(case):
     assert nnz == int(LARGE[case + "/nnz"])
     got = np.concatenate([sm.cpu().numpy(), off.cpu().numpy(), col.cpu().numpy()])
     assert hashlib.sha256(got.tobytes()).digest() == LARGE[case + "/csr_sha"].tobytes()
+
+
+@pytest.mark.parametrize("bs,nb", [(32, 1), (32, 2), (32, 5), (64, 1), (64, 3), (32, 128), (32, 129)])
+def test_filter_and_selection_at_their_edges(bs, nb):
+    """The filter of 31 taps as weighted sums of the map's blocks (one block, borders, odd counts), and the selection on either side of what
+    it keeps in shared memory.  Infinities and NaN stay within the reach of the filter; an unaligned map takes the general kernel.  Pooled
+    values are fp64 sums rounded to fp32 once: 2000 additions leave less than 1e-12 of the fp64 sum, a thousandth of what rounds to another fp32."""
+    pattern = _pattern_mod()
+    L = bs * nb
+    g = torch.Generator().manual_seed(7 * nb + bs)
+    A = torch.softmax(torch.randn(L, L, generator=g) * 2.0, dim=-1)
+    p = pattern.discover_pattern(A.cuda(), bs, 0.9)
+    want = opat.pooled_fixed_order(A.numpy(), bs)
+    got = p.pooled.cpu().numpy()
+    assert np.array_equal(got, want)
+    assert np.array_equal(p.mat.cpu().numpy(), opat.discover_block_mask(A.numpy(), bs, 0.9)[0])
+    _check_structure(p, p.mat.cpu().numpy())
+    if nb > 8:
+        return
+    at = torch.randint(0, L, (6, 2), generator=g).tolist() + [[0, 0], [0, L - 1], [L - 1, 0], [L - 1, L - 1], [15, bs - 16], [bs - 16, 15]]
+    for n, (i, j) in enumerate(at):
+        B = A.clone()
+        B[i, j] = [float("inf"), float("-inf"), float("nan")][n % 3]
+        shifted = torch.empty(L * L + 1, device="cuda")[1:].view(L, L).copy_(B)
+        with np.errstate(invalid="ignore"):
+            want = opat.pooled_fixed_order(B.numpy(), bs)
+        for M in (B.cuda(), shifted):
+            got = pattern.discover_pattern(M, bs, 0.9).pooled.cpu().numpy()
+            assert np.array_equal(got, want, equal_nan=True)
