@@ -122,8 +122,9 @@ class Attention(nn.Module):
         if mat is None and self.native:
             block = self.attn.block if untouched(self.attn, _NATIVE_DENSE) else None
         else:
-            block = mods.get("block_attn")
-        return (W, b, block) if untouched(block, _NATIVE_SPARSE if self.native else _DROPIN_SPARSE) else None
+            block = mods.get("attn" if mat is None else "block_attn")
+        types = _NATIVE_SPARSE if self.native else _DROPIN_DENSE if mat is None else _DROPIN_SPARSE
+        return (W, b, block) if untouched(block, types) else None
 
     def _one_node(self, X, mask, mat):
         """The whole layer as one autograd node on the library's kernels: projections, attention and output projection back to
@@ -137,8 +138,8 @@ class Attention(nn.Module):
             if self.native and self.native_dtype != torch.float32:
                 return None
             fp32 = True
-        if mat is None and fp32:
-            return None          # in the dense phase the key bias has no effect: its gradient is the rounding noise of the stages
+        # in the dense phase the key bias has no effect: its gradient is the rounding noise of the stages, which the node leaves as it is
+        noise = mat is None and fp32
         stages = self._untouched_stages(mat)
         if stages is None:
             return None
@@ -146,13 +147,17 @@ class Attention(nn.Module):
         if self.native:
             block.use_mask(mat)
             ctx = block._ctx
+        elif mat is None:
+            ctx = block.attn_func.context()
         else:
             ctx = block.context(mat)
         if not _ops.ops.layer_supported(ctx, X, W, b, fp32):
             return None
-        out, P, lse, pen, q, k, heads = _ops.ops.attention_layer(ctx, X, mask if self.with_keypad else None, W, b, fp32)
+        out, P, lse, pen, q, k, heads = _ops.ops.attention_layer(ctx, X, mask if self.with_keypad else None, W, b, fp32, noise)
         if self.native:
             return block.result(out, P, lse, pen, q, k, heads)
+        if mat is None:
+            return out, P.permute(0, 1, 3, 2)
         return out, (0 if self.with_keypad else P)
 
     def forward(self, X, mask, mat=None):

@@ -582,10 +582,22 @@ Tensor as_linear_node(const Tensor& y, bool fp32, const Tensor& x, const Tensor&
   return out;
 }
 
+// Column sums of dk [T, n]: the gradient of the key projection's bias in dense attention is zero, what comes out is the rounding of all that
+// leads to it.  Summed as the stages sum it, so that a layer in one node and its stages give the same one.
+Tensor key_bias_grad(const Context& c, const Tensor& dk, void* st) {
+  const int64_t T = dk.size(0), n = dk.size(1);
+  if (c.mode == DROPIN_DENSE || !(n == 64 || n == 128 || n == 256 || n == 512)) return dk.sum(0);
+  Tensor sums = at::empty({n}, dk.options()), ws = at::empty({(int64_t)spion_layernorm_workspace_floats((int)n)}, dk.options());
+  check(spion_column_sums(dk.data_ptr(), 0, (float*)sums.data_ptr(), (float*)ws.data_ptr(), T, (int)n, st), "spion_column_sums");
+  return sums;
+}
+
 // A whole multi-head attention layer: x [B, L, dim] -> projections -> attention -> output projection [B, L, dim_out].
+// noise: dense attention in fp32.  What the gradient of the key projection's bias consists of (above) stays as the stages form it: the
+// projections to Q, K and V and the way from the output's gradient to dO are the framework's products, the rest is the library's.
 struct LayerNode : public Node {
   ContextPtr c;
-  bool fp32 = false;
+  bool fp32 = false, noise = false;
   SavedAttn saved;
   SavedVariable x, w[4];                 // Wq, Wk, Wv, Wf; mixed precision: w[0] is the copy of all four, one after another
   int64_t dim_out = 0;
@@ -679,8 +691,14 @@ struct LayerNode : public Node {
       linear_backward_weight({go}, tgo, rows(a.O), tO, ff, fp32, T, st, dW, db);
       out[7] = dW[0]; out[8] = db[0];
     }
-    Tensor dO = empty_operand(*c, a.heads, a.q);
-    linear_backward_input(tgo, ff, fp32, nullptr, form({dO}), T, st);
+    Tensor dO;
+    if (noise) {
+      OutsideAutocast outside;
+      dO = at::mm(go.view({T, dim_out}), ff.W[0]).view({c->B, c->L, H, d}).transpose(1, 2).contiguous();
+    } else {
+      dO = empty_operand(*c, a.heads, a.q);
+      linear_backward_input(tgo, ff, fp32, nullptr, form({dO}), T, st);
+    }
     Tensor dq, dk, dv;
     attn_backward(*c, a, dO, dq, dk, dv, st);
     const spion_tokens tg = form({dq, dk, dv});
@@ -690,6 +708,7 @@ struct LayerNode : public Node {
       dW.clear(); db.clear();
       linear_backward_weight({rows(dq), rows(dk), rows(dv)}, tg, X, tok({X}, dim), qkv, fp32, T, st, dW, db, X.scalar_type() != x_type);
       for (int i = 0; i < 3; ++i) { out[1 + 2 * i] = dW[i]; out[2 + 2 * i] = db[i]; }
+      if (noise && task_should_compute_output(4)) out[4] = key_bias_grad(*c, dk.transpose(1, 2).reshape({T, H * d}), st);
     }
     if (task_should_compute_output(0)) {
       Tensor dX = at::empty(X.sizes(), X.options().dtype(x_type));
@@ -711,7 +730,7 @@ bool layer_supported(const ContextPtr& c, const Tensor& x, const std::vector<Ten
 }
 
 Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tensor>& mask, const std::vector<Tensor>& W,
-                          const std::vector<Tensor>& b, bool fp32) {
+                          const std::vector<Tensor>& b, bool fp32, bool noise) {
   c10::cuda::CUDAGuard guard(c->device);
   void* st = stream_of(x);
   const int H = (int)c->H, d = (int)c->d, L = (int)c->L;
@@ -733,14 +752,19 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
     // bf16 tokens: operands stay [B, L, H, d], whose rows the weight gradients' matrix products read
     a.heads = X.scalar_type() == at::kBFloat16 && c->fused ? H : 0;
     auto form = [&](const std::vector<Tensor>& ts) { return a.heads ? tok(ts, H * d) : tok_heads(ts, H, d, L); };
-    const Tensor like = at::empty({0}, opt);
-    a.q = empty_operand(*c, a.heads, like); a.k = empty_operand(*c, a.heads, like); a.v = empty_operand(*c, a.heads, like);
     Weights qkv{{W[0].detach(), W[1].detach(), W[2].detach()}, {b[0].detach(), b[1].detach(), b[2].detach()}};
     Weights ff{{W[3].detach()}, {b[3].detach()}};
     const int64_t n_in = (int64_t)qkv.out() * qkv.in();
     if (need && !fp32) kept_w = at::empty({n_in + (int64_t)ff.out() * ff.in()}, W[0].options());
-    kept_in = Kept(need, fp32, X, qkv, (float*)p(kept_w));
-    linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st, kept_in);
+    if (noise) {
+      auto operand = [&](int i) { return at::linear(X, qkv.W[i], qkv.b[i]).view({c->B, c->L, H, d}).transpose(1, 2).contiguous(); };
+      a.q = operand(0); a.k = operand(1); a.v = operand(2);
+    } else {
+      const Tensor like = at::empty({0}, opt);
+      a.q = empty_operand(*c, a.heads, like); a.k = empty_operand(*c, a.heads, like); a.v = empty_operand(*c, a.heads, like);
+      kept_in = Kept(need, fp32, X, qkv, (float*)p(kept_w));
+      linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st, kept_in);
+    }
     attn_forward(*c, a, need, st);
     out = at::empty({c->B, c->L, ff.out()}, opt);
     kept_out = Kept(need, fp32, a.O, ff, kept_w.defined() ? (float*)p(kept_w) + n_in : nullptr);
@@ -749,7 +773,7 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
   if (need) {
     auto node = std::shared_ptr<LayerNode>(new LayerNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x, W[0], b[0], W[1], b[1], W[2], b[2], W[3], b[3]));
-    node->c = c; node->fp32 = fp32; node->out_type = out.scalar_type();
+    node->c = c; node->fp32 = fp32; node->noise = noise; node->out_type = out.scalar_type();
     Attn kept = a;
     if (c->mode == NATIVE && c->fused && c->recompute) kept.P = Tensor();
     node->saved.save_all(kept, a.q, a.k, a.v);
@@ -930,8 +954,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, py::arg("context"), py::arg("query"), py::arg("key"), py::arg("value"), py::arg("mask"), py::arg("inside") = false);
   m.def("layer_supported", &layer_supported);
   m.def("attention_layer", [](const ContextPtr& c, const Tensor& x, const optional<Tensor>& mask, const std::vector<Tensor>& W,
-                              const std::vector<Tensor>& b, bool fp32) {
-    return as_tuple([&] { return attention_layer(c, x, mask, W, b, fp32); });
+                              const std::vector<Tensor>& b, bool fp32, bool noise) {
+    return as_tuple([&] { return attention_layer(c, x, mask, W, b, fp32, noise); });
   });
   m.def("linear_supported", &linear_supported);
   m.def("linear", &linear);

@@ -182,7 +182,7 @@ def test_attention_layer_in_one_node_equals_its_stages(native, dtype, bs, L, den
     mask[1, L // 2:] = 0
     amp = torch.autocast("cuda", dtype=torch.bfloat16) if dtype == "bf16" else nullcontext()
     outs = []
-    for hooked in (False, True):                              # (the drop-in dense phase always runs stage by stage)
+    for hooked in (False, True):
         h = layer.W_k.register_forward_hook(lambda m, i, o: None) if hooked else None
         with amp:
             out, _ = layer(x, mask, mat)
@@ -196,6 +196,40 @@ def test_attention_layer_in_one_node_equals_its_stages(native, dtype, bs, L, den
         assert a.shape == b.shape and a.dtype == b.dtype
         err = float((a.double() - b.double()).norm())
         assert err <= tol * float(b.double().norm()) + 1e-6, (err, float(b.double().norm()))
+
+
+@pytest.mark.parametrize("native,bs,L,H,d,keypad", [(True, 32, 160, 2, 32, True), (True, 64, 320, 3, 64, False), (False, 32, 96, 1, 32, False),
+                                                    (False, 64, 192, 4, 64, True)])
+def test_dense_fp32_layer_in_one_node_equals_its_stages(native, bs, L, H, d, keypad):
+    """Dense attention in fp32: outputs, map and gradients of the node are those of the stages (fp32 sums of at most 960 terms in another
+    order), and the gradient of the key projection's bias, which is zero but for the rounding of the stages, is the same bits."""
+    from spion_b200.attention import Attention
+    B = 5
+    cfg = {"head_dim": d, "num_head": H, "max_seq_len": L, "batch_size": B, "block_size": bs, "transformer_dim": H * d,
+           "task": "lra-text" if keypad else "lra-image", "native": native, "dtype": "fp32"}
+    torch.manual_seed(3)
+    layer = Attention(cfg).cuda()
+    x = torch.randn(B, L, H * d, device="cuda", requires_grad=True)
+    do = torch.randn(B, L, H * d, device="cuda")
+    mask = torch.ones(B, L, device="cuda")
+    mask[1, L // 2:] = 0
+    names = ["x"] + [n for n, _ in layer.named_parameters()]
+    runs = []
+    for hooked in (False, True):
+        h = layer.W_k.register_forward_hook(lambda m, i, o: None) if hooked else None
+        out, attn = layer(x, mask, None)
+        if not hooked:
+            assert out.grad_fn.name() == "SparseAttentionLayerBackward"
+        runs.append([out, attn if torch.is_tensor(attn) else out, *torch.autograd.grad(out, [x] + list(layer.parameters()), do)])
+        if h:
+            h.remove()
+    assert torch.equal(runs[0][1], runs[1][1]) or native
+    for n, a, b in zip(["out", "attn"] + names, *runs):
+        assert a.shape == b.shape and a.dtype == b.dtype and a.stride() == b.stride(), n
+        if n == "W_k.bias":
+            assert torch.equal(a, b)
+        else:
+            assert float((a.double() - b.double()).norm()) <= 1e-5 * float(b.double().norm()), n
 
 
 def test_feed_forward_block():
