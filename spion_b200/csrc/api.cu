@@ -488,17 +488,22 @@ static int dense_forward(spion_ctx* c, const float* Q, const float* K, const flo
   const Pattern p = ctx_pattern(c);
   const ValueLayout vl{VAL_DENSE_T, c->L, (long long)c->L * c->L};
   const OperandLayout rm = row_major_operand(c->L, c->d);
+  const float* pad = is_kpm(c) ? keypad : nullptr;
+  const bool joint = simt_dense_joint(false, c->L, c->d, c->BH, K, attn, attn);
   prof_mark(c, -1);
-  int rc = simt_sddmm(SPION_F32, SPION_F32, Q, lo, K, rm, attn, vl, p, c->nnzb, c->BH, c->d, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SDDMM_S);
-  if (rc) return rc;
   // running-maximum floor -10 (models/attn.cu:21); key padding as models/attn_mask.cu:20
-  rc = softmax_fwd_dense_t(attn, c->BH, c->L, c->scale, is_kpm(c) ? keypad : nullptr, -10.0f, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SOFTMAX_FWD);
+  int rc = joint ? simt_dense_scores(Q, lo, K, attn, c->BH, c->L, c->d, c->scale, pad, -10.0f, c->stream)
+                 : simt_sddmm(SPION_F32, SPION_F32, Q, lo, K, rm, attn, vl, p, c->nnzb, c->BH, c->d, c->stream);
   if (rc) return rc;
+  prof_mark(c, joint ? SPION_STAGE_SOFTMAX_FWD : SPION_STAGE_SDDMM_S);
+  if (!joint) {
+    rc = softmax_fwd_dense_t(attn, c->BH, c->L, c->scale, pad, -10.0f, c->stream);
+    if (rc) return rc;
+    prof_mark(c, SPION_STAGE_SOFTMAX_FWD);
+  }
   rc = simt_spmm(SPION_F32, SPION_F32, false, attn, vl, V, lo, out, lo, p, c->BH, c->d, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SPMM_O);
-  c->launches += 3;
+  c->launches += joint ? 2 : 3;
   return rc;
 }
 
@@ -510,13 +515,24 @@ static int dense_backward(spion_ctx* c, const float* Q, const float* K, const fl
   const Pattern p = ctx_pattern(c);
   const ValueLayout vl{VAL_DENSE_T, c->L, (long long)c->L * c->L};
   const OperandLayout rm = row_major_operand(c->L, c->d);
+  const bool joint = simt_dense_joint(true, c->L, c->d, c->BH, V, attn, s3);
   prof_mark(c, -1);
-  int rc = simt_sddmm(SPION_F32, SPION_F32, dO, lo, V, rm, s1, vl, p, c->nnzb, c->BH, c->d, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SDDMM_DP);
+  int rc = joint ? simt_dense_dscores(dO, lo, V, attn, s3, c->BH, c->L, c->d, c->scale, c->stream)
+                 : simt_sddmm(SPION_F32, SPION_F32, dO, lo, V, rm, s1, vl, p, c->nnzb, c->BH, c->d, c->stream);
   if (rc) return rc;
-  rc = softmax_bwd_dense_t(s1, attn, s3, c->BH, c->L, c->scale, c->stream);
-  if (!rc) prof_mark(c, SPION_STAGE_SOFTMAX_BWD);
-  if (rc) return rc;
+  prof_mark(c, joint ? SPION_STAGE_SOFTMAX_BWD : SPION_STAGE_SDDMM_DP);
+  if (!joint) {
+    rc = softmax_bwd_dense_t(s1, attn, s3, c->BH, c->L, c->scale, c->stream);
+    if (rc) return rc;
+    prof_mark(c, SPION_STAGE_SOFTMAX_BWD);
+  }
+  c->launches += joint ? 1 : 2;
+  rc = simt_dense_grads(attn, s3, Q, K, dO, lo, dQ, dK, dV, p, c->BH, c->L, c->d, c->stream);
+  if (rc != SPION_ERR_UNSUPPORTED) {
+    if (!rc) prof_mark(c, SPION_STAGE_SPMM_DK);
+    c->launches += 1;
+    return rc;
+  }
   rc = simt_spmm(SPION_F32, SPION_F32, false, s3, vl, K, lo, dQ, lo, p, c->BH, c->d, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SPMM_DQ);
   if (rc) return rc;
@@ -525,7 +541,7 @@ static int dense_backward(spion_ctx* c, const float* Q, const float* K, const fl
   if (rc) return rc;
   rc = simt_spmm(SPION_F32, SPION_F32, true, attn, vl, dO, lo, dV, lo, p, c->BH, c->d, c->stream);
   if (!rc) prof_mark(c, SPION_STAGE_SPMM_DV);
-  c->launches += 5;
+  c->launches += 3;
   return rc;
 }
 

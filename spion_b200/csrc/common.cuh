@@ -184,6 +184,12 @@ int softmax_bwd_rows(int dtype_p, const float* dP, ValueLayout vdp, const void* 
                      ValueLayout vds, Pattern p, int BH, int L, float scale, cudaStream_t st);
 int softmax_fwd_dense_t(float* S, int BH, int L, float scale, const float* keypad, float floor, cudaStream_t st);
 int softmax_bwd_dense_t(const float* dP, const float* P, float* dS, int BH, int L, float scale, cudaStream_t st);
+// the same stages with their products: S and softmax, dP and softmax, dQ and dK and dV
+bool simt_dense_joint(bool backward, int L, int d, int BH, const void* rows, const void* values, const void* values2);
+int simt_dense_scores(const float* Q, OperandLayout lq, const float* K, float* P, int BH, int L, int d, float scale, const float* keypad, float floor_v, cudaStream_t st);
+int simt_dense_dscores(const float* dO, OperandLayout ldo, const float* V, const float* P, float* dS, int BH, int L, int d, float scale, cudaStream_t st);
+int simt_dense_grads(const float* P, const float* dS, const float* Q, const float* K, const float* dO, OperandLayout lo, float* dQ, float* dK, float* dV,
+                     Pattern p, int BH, int L, int d, cudaStream_t st);
 
 // simt_fused.cu: fused fp32 kernels (value layouts with contiguous tile rows)
 bool simt_fused_supports(int bs, int d, int BH, int value_mode);

@@ -14,6 +14,8 @@
 //   softmax_bwd_rows  replaces softmax_scale_backward_kernel   (models/block_attn.cu:90-130)
 //   softmax_*_dense_t replace max_sum_exp_kernel[_large] / softmax_scale_backward_kernel[_large]
 //                     (models/attn.cu:9-112, models/attn_mask.cu:8-122)
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -690,7 +692,7 @@ __global__ void __launch_bounds__(DENSE_WARPS * SLAB) softmax_bwd_dense_t_slab(c
 // shared-memory read on every other multiply-add and hold one tile in flight; these keep the order of additions of
 // every output (n, or k, ascending into one fp32 sum), so the results are the same bit for bit, with packed pairs of
 // multiply-adds, 16-byte reads and cp.async.  16 matrices, L = 1024, d 32: S, dP 81 -> 31 us
-// each, P V and dS K 102 -> 34, dS^T Q and P^T dO 118 -> 38.
+// each, P V and dS K 102 -> 34, dS^T Q and P^T dO 118 -> 38; in one kernel with what follows them, or with one another, below.
 __device__ __forceinline__ uint32_t dense_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void dense_cp16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dense_smem(dst)), "l"(src) : "memory");
@@ -780,61 +782,58 @@ __global__ void __launch_bounds__(64) sddmm_dense_kernel(const float* __restrict
 }
 
 // TRANS == false: out[i] = sum_j value(i, j) Bop[j];  true: out[j] = sum_i value(i, j) Bop[i].  64 rows x 32 columns by 64 threads
-// (4 x 8 each), the sum over L in steps of 32 through three stages.  The sum of an output stays one chain, so the rows
-// cannot be split further: 64 threads a tile put 256 tiles of a small call on every scheduler.
-constexpr int DK = 32, DSTAGES = 3;
+// (4 x 8 each), the sum over L in steps of 32 through two stages.  The sum of an output stays one chain where its bits are kept (dK), so the
+// rows cannot be split further.
+constexpr int DK = 32, DSTAGES = 2;
+constexpr int SPMM_STAGE = DT * (DK + 4) + DK * (DK + 4);        // floats of a stage: value tile, operand tile
 template <bool TRANS>
-__global__ void __launch_bounds__(64) spmm_dense_kernel(const float* __restrict__ vals, const float* __restrict__ Bop, OperandLayout lb,
-                                                        float* __restrict__ out, OperandLayout lo, int L) {
+__device__ __forceinline__ void spmm_dense(float* smem, int t, int bh, int r0, int n0, int c0, int chunks, const float* vals, const float* Bop,
+                                           const OperandLayout& lb, int L, pair_t (&acc)[4][4], int barrier) {
   constexpr int VR = TRANS ? DT : DK, VC = TRANS ? DK : DT, VP = TRANS ? DK + 4 : DT;   // value tile as in memory: rows j, columns i
-  __shared__ __align__(16) float Vs[DSTAGES][VR][VP];
-  __shared__ __align__(16) float Bs[DSTAGES][DK][DK + 4];                               // [k][n]
-  const int t = threadIdx.x, ty = t >> 2, tx = t & 3;
-  const int r0 = blockIdx.x * DT, bh = blockIdx.y, n0 = blockIdx.z * 32;
+  const int ty = t >> 2, tx = t & 3;
   const float* vb = vals + (long long)bh * L * L + (TRANS ? (long long)r0 * L : (long long)r0);
   const float* Bb = Bop + (long long)bh * lb.bh_stride + (long long)n0 * lb.sd;
   const bool rows = lb.sd == 1 && (lb.sl & 3) == 0 && (reinterpret_cast<uintptr_t>(Bb) & 15) == 0;
   auto load = [&](int c) {
-    const int st = c % DSTAGES, k0 = c * DK;
+    const int k0 = (c0 + c) * DK;
+    float(*V)[VP] = reinterpret_cast<float(*)[VP]>(smem + (c & 1) * SPMM_STAGE);
+    float(*B)[DK + 4] = reinterpret_cast<float(*)[DK + 4]>(smem + (c & 1) * SPMM_STAGE + DT * (DK + 4));
     const float* v = vb + (TRANS ? (long long)k0 : (long long)k0 * L);
 #pragma unroll
-    for (int e = t; e < VR * VC / 4; e += 64) dense_cp16(&Vs[st][e / (VC / 4)][e % (VC / 4) * 4], v + (long long)(e / (VC / 4)) * L + e % (VC / 4) * 4);
+    for (int e = t; e < VR * VC / 4; e += 64) dense_cp16(&V[e / (VC / 4)][e % (VC / 4) * 4], v + (long long)(e / (VC / 4)) * L + e % (VC / 4) * 4);
     if (rows) {
 #pragma unroll
-      for (int e = t; e < DK * 32 / 4; e += 64) dense_cp16(&Bs[st][e >> 3][(e & 7) * 4], Bb + (long long)(k0 + (e >> 3)) * lb.sl + (e & 7) * 4);
+      for (int e = t; e < DK * 32 / 4; e += 64) dense_cp16(&B[e >> 3][(e & 7) * 4], Bb + (long long)(k0 + (e >> 3)) * lb.sl + (e & 7) * 4);
     } else {
 #pragma unroll 4
-      for (int e = t; e < DK * 32; e += 64) dense_cp4(&Bs[st][e & 31][e >> 5], Bb + (long long)(k0 + (e & 31)) * lb.sl + (long long)(e >> 5) * lb.sd);
+      for (int e = t; e < DK * 32; e += 64) dense_cp4(&B[e & 31][e >> 5], Bb + (long long)(k0 + (e & 31)) * lb.sl + (long long)(e >> 5) * lb.sd);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  pair_t acc[4][4];
+  auto meet = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory"); };
 #pragma unroll
   for (int x = 0; x < 4; ++x)
 #pragma unroll
     for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
-  const int chunks = L / DK;
-  for (int c = 0; c < DSTAGES - 1; ++c) {
-    if (c < chunks) load(c);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
+  if (chunks > 0) load(0);
   for (int c = 0; c < chunks; ++c) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(DSTAGES - 2) : "memory");
-    __syncthreads();                                   // chunk c has landed; the stage of chunk c - 1 is free
-    if (c + DSTAGES - 1 < chunks) load(c + DSTAGES - 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const int st = c % DSTAGES;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    meet();                                            // chunk c has landed; the stage of chunk c - 1 is free
+    if (c + 1 < chunks) load(c + 1);
+    const float(*Vs)[VP] = reinterpret_cast<const float(*)[VP]>(smem + (c & 1) * SPMM_STAGE);
+    const float(*Bs)[DK + 4] = reinterpret_cast<const float(*)[DK + 4]>(smem + (c & 1) * SPMM_STAGE + DT * (DK + 4));      // [k][n]
 #pragma unroll 2
     for (int k = 0; k < DK; k += 4) {
       float a[4][4];                                   // [k][row]
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const float4 v = TRANS ? *reinterpret_cast<const float4*>(&Vs[st][ty + 16 * u][k]) : *reinterpret_cast<const float4*>(&Vs[st][k + u][4 * ty]);
+        const float4 v = TRANS ? *reinterpret_cast<const float4*>(&Vs[ty + 16 * u][k]) : *reinterpret_cast<const float4*>(&Vs[k + u][4 * ty]);
         if (TRANS) a[0][u] = v.x, a[1][u] = v.y, a[2][u] = v.z, a[3][u] = v.w;
         else a[u][0] = v.x, a[u][1] = v.y, a[u][2] = v.z, a[u][3] = v.w;
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const ulonglong2 lo2 = *reinterpret_cast<const ulonglong2*>(&Bs[st][k + u][4 * tx]), hi2 = *reinterpret_cast<const ulonglong2*>(&Bs[st][k + u][16 + 4 * tx]);
+        const ulonglong2 lo2 = *reinterpret_cast<const ulonglong2*>(&Bs[k + u][4 * tx]), hi2 = *reinterpret_cast<const ulonglong2*>(&Bs[k + u][16 + 4 * tx]);
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
           const pair_t aa = twice(a[u][x]);
@@ -843,6 +842,10 @@ __global__ void __launch_bounds__(64) spmm_dense_kernel(const float* __restrict_
       }
     }
   }
+}
+template <bool TRANS>
+__device__ __forceinline__ void spmm_dense_write(const pair_t (&acc)[4][4], int t, int bh, int r0, int n0, float* out, const OperandLayout& lo) {
+  const int ty = t >> 2, tx = t & 3;
   float* ob = out + (long long)bh * lo.bh_stride;
 #pragma unroll
   for (int x = 0; x < 4; ++x) {
@@ -853,6 +856,282 @@ __global__ void __launch_bounds__(64) spmm_dense_kernel(const float* __restrict_
       float* o = ob + (long long)row * lo.sl + (long long)(n0 + 16 * h + 4 * tx) * lo.sd;
       if (lo.sd == 1 && (reinterpret_cast<uintptr_t>(o) & 15) == 0) *reinterpret_cast<float4*>(o) = v;
       else o[0] = v.x, o[lo.sd] = v.y, o[2 * lo.sd] = v.z, o[3 * lo.sd] = v.w;
+    }
+  }
+}
+
+// O = P V.  Its bits are nobody's: four groups of 64 threads take a quarter of the keys each, so that a call of 256 tiles has fourteen warps per
+// SM, and the quarters are added in order.  16 matrices, L = 1024, d 32: 31 us (34 with one group).
+constexpr int OGROUPS = 4;
+__global__ void __launch_bounds__(64 * OGROUPS) spmm_dense_split(const float* __restrict__ vals, const float* __restrict__ Bop, OperandLayout lb,
+                                                                 float* __restrict__ out, OperandLayout lo, int L) {
+  extern __shared__ __align__(16) float s_spmm[];
+  const int g = threadIdx.x >> 6, t = threadIdx.x & 63;
+  const int r0 = blockIdx.x * DT, bh = blockIdx.y, n0 = blockIdx.z * 32;
+  const int chunks = L / DK, per = (chunks + OGROUPS - 1) / OGROUPS, c0 = min(chunks, g * per), c1 = min(chunks, c0 + per);
+  pair_t acc[4][4];
+  spmm_dense<false>(s_spmm + g * DSTAGES * SPMM_STAGE, t, bh, r0, n0, c0, c1 - c0, vals, Bop, lb, L, acc, 1 + g);
+  __syncthreads();
+  float2* sum = reinterpret_cast<float2*>(s_spmm);
+  if (g > 0)
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      float2 v;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(acc[e >> 2][e & 3]));
+      sum[((g - 1) * 16 + e) * 64 + t] = v;
+    }
+  __syncthreads();
+  if (g > 0) return;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(acc[e >> 2][e & 3]));
+#pragma unroll
+    for (int o = 0; o < OGROUPS - 1; ++o) {
+      const float2 w = sum[(o * 16 + e) * 64 + t];
+      v.x += w.x;
+      v.y += w.y;
+    }
+    asm("mov.b64 %0, {%1, %2};" : "=l"(acc[e >> 2][e & 3]) : "f"(v.x), "f"(v.y));
+  }
+  spmm_dense_write<false>(acc, t, bh, r0, n0, out, lo);
+}
+
+// dK = dS^T Q, dV = P^T dO and dQ = dS K of a backward in one launch: tiles of 64 threads each, four warps per SM with one launch per product, ten
+// to twelve with all three.  16 matrices, L = 1024, d 32: 107 us in three launches, 94 in one.
+struct DenseGrads {
+  const float *P, *dS, *Q, *K, *dO;
+  float *dQ, *dK, *dV;
+  OperandLayout lo;
+  int L, halves;                                       // head_dim / 32
+};
+__global__ void __launch_bounds__(64) spmm_dense_grads(const DenseGrads a) {
+  __shared__ __align__(16) float smem[DSTAGES * SPMM_STAGE];
+  const int what = blockIdx.z / a.halves, n0 = (blockIdx.z - what * a.halves) * 32, r0 = blockIdx.x * DT, bh = blockIdx.y, t = threadIdx.x;
+  pair_t acc[4][4];
+  if (what < 2) {
+    spmm_dense<true>(smem, t, bh, r0, n0, 0, a.L / DK, what ? a.P : a.dS, what ? a.dO : a.Q, a.lo, a.L, acc, 1);
+    spmm_dense_write<true>(acc, t, bh, r0, n0, what ? a.dV : a.dK, a.lo);
+  } else {
+    spmm_dense<false>(smem, t, bh, r0, n0, 0, a.L / DK, a.dS, a.K, a.lo, a.L, acc, 1);
+    spmm_dense_write<false>(acc, t, bh, r0, n0, a.dQ, a.lo);
+  }
+}
+
+// Scores and their softmax (forward), dP and dS (backward) of sixteen query rows and all keys by one CTA: what the product leaves stays in
+// registers, so that S and dP never reach memory.  A warp has one of the DENSE_WARPS slices of the keys, a lane KPL keys by eight queries of
+// it (packed multiply-adds over pairs of queries: a shared-memory read returns one register per lane and cycle, which eight by eight tiles
+// balance with the multiply-adds; four by four took 62 us forward); sums along the keys go through shared memory, one lane per query and
+// slice.  Slices, expressions and order of additions are those of sddmm_dense_kernel and the slab kernels: the results are the same bits.
+// Up to 2048 keys (8 KPL accumulators for slices of 16 KPL).
+// Which calls take them and what that gives: simt_dense_joint.
+// keys kg + 16 r, queries 4 ig + (0 .. 3) and 8 + 4 ig + (0 .. 3), in pairs
+template <int KPL>
+struct Slice {
+  pair_t acc[KPL][4];
+  __device__ __forceinline__ float4 at(int r, int h) const { return as_float4(acc[r][2 * h], acc[r][2 * h + 1]); }
+};
+// Products of the keys B[0 .. n) of a slice with As [d][16], eight columns of B at a time (NB buffers).
+template <int KPL, int NB, class BEFORE>
+__device__ __forceinline__ void slice_products(Slice<KPL>& x, const float* __restrict__ B, int ld, int n, int d, const float* As, float* stage, BEFORE before) {
+  const int lane = threadIdx.x & 31, kg = lane >> 1, ig = lane & 1;
+#pragma unroll
+  for (int r = 0; r < KPL; ++r)
+#pragma unroll
+    for (int y = 0; y < 4; ++y) x.acc[r][y] = 0ull;
+  auto load = [&](int n0, float* to) {
+#pragma unroll
+    for (int e = 0; e < KPL; ++e) {
+      const int row = e * 16 + (lane >> 1), q = lane & 1;
+      if (row < n) dense_cp16(to + row * 8 + 4 * q, B + (long long)row * ld + n0 + 4 * q);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load(0, stage);
+  before();                                            // copies of the caller's, one group
+  for (int n0 = 0; n0 < d; n0 += 8) {
+    const float* st = stage;
+    if (NB == 2) {
+      if (n0 + 8 < d) load(n0 + 8, stage + ((n0 >> 3) + 1 & 1) * 128 * KPL);
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      st += ((n0 >> 3) & 1) * 128 * KPL;
+    } else if (n0 == 0) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      load(n0, stage);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      float2 b[KPL];
+#pragma unroll
+      for (int r = 0; r < KPL; ++r) b[r] = *reinterpret_cast<const float2*>(st + (kg + 16 * r) * 8 + k);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float* a = As + (n0 + k + u) * 16 + 4 * ig;
+        const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(a), hi = *reinterpret_cast<const ulonglong2*>(a + 8);
+#pragma unroll
+        for (int r = 0; r < KPL; ++r) {
+          const pair_t bb = twice(u ? b[r].y : b[r].x);
+          fma2(x.acc[r][0], lo.x, bb); fma2(x.acc[r][1], lo.y, bb); fma2(x.acc[r][2], hi.x, bb); fma2(x.acc[r][3], hi.y, bb);
+        }
+      }
+    }
+    __syncwarp();                                      // the buffer may be filled again
+  }
+}
+__device__ __forceinline__ void load_queries(float* As, const float* A, const OperandLayout& la, int bh, int i0, int d) {     // As [d][16]
+  const float* src = A + (long long)bh * la.bh_stride + (long long)i0 * la.sl;
+  for (int e = threadIdx.x; e < 16 * d; e += DENSE_WARPS * 32) {
+    const int i = la.sl == 1 ? e & 15 : e / d, n = la.sl == 1 ? e >> 4 : e % d;
+    As[n * 16 + i] = src[(long long)i * la.sl + (long long)n * la.sd];
+  }
+}
+__device__ __forceinline__ float4 operator+(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+constexpr int SLICE_MAX_L = 2048;
+
+template <int KPL>
+__global__ void __launch_bounds__(DENSE_WARPS * 32, KPL <= 8 ? 2 : 1) dense_scores_kernel(const float* __restrict__ Q, OperandLayout lq, const float* __restrict__ K,
+                                                                                     float* __restrict__ P, int L, int d, float scale,
+                                                                                     const float* __restrict__ keypad, float floor_v) {
+  extern __shared__ __align__(16) float s_dyn[];
+  __shared__ __align__(16) float As[64 * 16];
+  __shared__ __align__(16) float s_red[2][DENSE_WARPS][SLAB];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, kg = lane >> 1, ig = lane & 1;
+  const int bh = blockIdx.y, i0 = blockIdx.x * SLAB;
+  const int per = slab_per(L), j0 = w * per, n = max(0, min(L, j0 + per) - j0);
+  float* mine = s_dyn + w * 256 * KPL;                 // two operand stages, then the slice's exponentials [key][16]
+  load_queries(As, Q, lq, bh, i0, d);
+  __syncthreads();
+  Slice<KPL> x;
+  slice_products<KPL, 2>(x, K + ((long long)bh * L + j0) * d, d, n, d, As, mine, [] {});
+  const float* kp = keypad ? keypad + (long long)bh * L + j0 : nullptr;
+  // s scale - penalty, each rounded once together, and, without penalties, the maximum taken off in the same step: as the compiler contracts
+  // the expressions of the kernels above
+  float4 m[2] = {make_float4(floor_v, floor_v, floor_v, floor_v), make_float4(floor_v, floor_v, floor_v, floor_v)};
+#pragma unroll
+  for (int r = 0; r < KPL; ++r) {
+    const int j = kg + 16 * r;
+    if (j >= n) continue;
+    const float k = kp ? kp[j] : 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float4 s = x.at(r, h);
+      m[h].x = fmaxf(m[h].x, fmaf(s.x, scale, -k)); m[h].y = fmaxf(m[h].y, fmaf(s.y, scale, -k));
+      m[h].z = fmaxf(m[h].z, fmaf(s.z, scale, -k)); m[h].w = fmaxf(m[h].w, fmaf(s.w, scale, -k));
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int o = 2; o < 32; o <<= 1) {
+      m[h].x = fmaxf(m[h].x, __shfl_xor_sync(0xffffffffu, m[h].x, o)); m[h].y = fmaxf(m[h].y, __shfl_xor_sync(0xffffffffu, m[h].y, o));
+      m[h].z = fmaxf(m[h].z, __shfl_xor_sync(0xffffffffu, m[h].z, o)); m[h].w = fmaxf(m[h].w, __shfl_xor_sync(0xffffffffu, m[h].w, o));
+    }
+  if (kg == 0) {
+    *reinterpret_cast<float4*>(&s_red[0][w][4 * ig]) = m[0];
+    *reinterpret_cast<float4*>(&s_red[0][w][8 + 4 * ig]) = m[1];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < DENSE_WARPS; ++k)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float4 o = *reinterpret_cast<const float4*>(&s_red[0][k][8 * h + 4 * ig]);
+      m[h].x = fmaxf(m[h].x, o.x); m[h].y = fmaxf(m[h].y, o.y); m[h].z = fmaxf(m[h].z, o.z); m[h].w = fmaxf(m[h].w, o.w);
+    }
+#pragma unroll
+  for (int r = 0; r < KPL; ++r) {
+    const int j = kg + 16 * r;
+    if (j >= n) continue;
+    const float k = kp ? kp[j] : 0.f;
+    auto ex = [&](float s, float most) { return expf(kp ? __fsub_rn(fmaf(s, scale, -k), most) : fmaf(s, scale, -most)); };
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float4 s = x.at(r, h), e = make_float4(ex(s.x, m[h].x), ex(s.y, m[h].y), ex(s.z, m[h].z), ex(s.w, m[h].w));
+      *reinterpret_cast<float4*>(mine + j * SLAB + 8 * h + 4 * ig) = e;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(x.acc[r][2 * h]) : "f"(e.x), "f"(e.y));
+      asm("mov.b64 %0, {%1, %2};" : "=l"(x.acc[r][2 * h + 1]) : "f"(e.z), "f"(e.w));
+    }
+  }
+  __syncwarp();
+  if (lane < SLAB) {
+    float sum = 0.f;
+#pragma unroll 8
+    for (int u = 0; u < n; ++u) sum += mine[u * SLAB + lane];
+    s_red[1][w][lane] = sum;
+  }
+  __syncthreads();
+  float* out = P + (long long)bh * L * L + (long long)j0 * L + i0 + 4 * ig;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < DENSE_WARPS; ++k) t = t + *reinterpret_cast<const float4*>(&s_red[1][k][8 * h + 4 * ig]);      // slices added in slice order
+    const float4 inv = make_float4(1.0f / t.x, 1.0f / t.y, 1.0f / t.z, 1.0f / t.w);
+#pragma unroll
+    for (int r = 0; r < KPL; ++r) {
+      const int j = kg + 16 * r;
+      const float4 e = x.at(r, h);
+      if (j < n) *reinterpret_cast<float4*>(out + (long long)j * L + 8 * h) = make_float4(e.x * inv.x, e.y * inv.y, e.z * inv.z, e.w * inv.w);
+    }
+  }
+}
+
+template <int KPL>
+__global__ void __launch_bounds__(DENSE_WARPS * 32, KPL <= 8 ? 2 : 1) dense_dscores_kernel(const float* __restrict__ dO, OperandLayout ldo, const float* __restrict__ V,
+                                                                                      const float* __restrict__ P, float* __restrict__ dS, int L, int d,
+                                                                                      float scale) {
+  extern __shared__ __align__(16) float s_dyn[];
+  __shared__ __align__(16) float As[64 * 16];
+  __shared__ __align__(16) float s_red[DENSE_WARPS][SLAB];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, kg = lane >> 1, ig = lane & 1;
+  const int bh = blockIdx.y, i0 = blockIdx.x * SLAB;
+  const int per = slab_per(L), j0 = w * per, n = max(0, min(L, j0 + per) - j0);
+  float* mine = s_dyn + w * (per * SLAB + 128 * KPL);  // P of the slice [key][16], then a stage
+  float* stage = mine + per * SLAB;
+  const long long at = (long long)bh * L * L + (long long)j0 * L + i0;
+  load_queries(As, dO, ldo, bh, i0, d);
+  __syncthreads();
+  Slice<KPL> x;
+  slice_products<KPL, 1>(x, V + ((long long)bh * L + j0) * d, d, n, d, As, stage, [&] {
+    for (int e = lane; e < 4 * n; e += 32) dense_cp16(mine + e * 4, P + at + (long long)(e >> 2) * L + 4 * (e & 3));
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  });
+  float s = 0.f;
+#pragma unroll
+  for (int c = 0; c < KPL / 2; ++c) {                  // 32 keys of dP at a time through the stage
+    if (c * 32 >= n) break;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) *reinterpret_cast<float4*>(stage + (kg + 16 * u) * SLAB + 8 * h + 4 * ig) = x.at(2 * c + u, h);
+    __syncwarp();
+    if (lane < SLAB) {
+      const float* p = mine + c * 32 * SLAB + lane;
+      const int most = min(32, n - c * 32);
+#pragma unroll 8
+      for (int u = 0; u < most; ++u) s += stage[u * SLAB + lane] * p[u * SLAB];
+    }
+    __syncwarp();
+  }
+  if (lane < SLAB) s_red[w][lane] = s;
+  __syncthreads();
+  float* out = dS + at + 4 * ig;
+  auto ds = [&](float dp, float pv, float sum) { return (dp * pv - pv * sum) * scale; };
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < DENSE_WARPS; ++k) t = t + *reinterpret_cast<const float4*>(&s_red[k][8 * h + 4 * ig]);
+#pragma unroll
+    for (int r = 0; r < KPL; ++r) {
+      const int j = kg + 16 * r;
+      if (j >= n) continue;
+      const float4 g = x.at(r, h), p = *reinterpret_cast<const float4*>(mine + j * SLAB + 8 * h + 4 * ig);
+      *reinterpret_cast<float4*>(out + (long long)j * L + 8 * h) = make_float4(ds(g.x, p.x, t.x), ds(g.y, p.y, t.y), ds(g.z, p.z, t.z), ds(g.w, p.w, t.w));
     }
   }
 }
@@ -912,10 +1191,10 @@ static int spmm_dispatch(bool trans, const void* vals, ValueLayout vl, const voi
 int simt_spmm(int dtype_val, int dtype_op, bool trans, const void* vals, ValueLayout vl, const void* Bop,
               OperandLayout lb, void* out, OperandLayout lo, Pattern p, int BH, int d, cudaStream_t st) {
   if (d % 32 != 0 || BH > 65535) return SPION_ERR_UNSUPPORTED;
-  if (dtype_val == SPION_F32 && dtype_op == SPION_F32 && full_dense(vl, p, vals)) {
-    const dim3 grid(p.nb, BH, d / 32);
-    if (trans) spmm_dense_kernel<true><<<grid, 64, 0, st>>>((const float*)vals, (const float*)Bop, lb, (float*)out, lo, vl.L);
-    else spmm_dense_kernel<false><<<grid, 64, 0, st>>>((const float*)vals, (const float*)Bop, lb, (float*)out, lo, vl.L);
+  if (!trans && dtype_val == SPION_F32 && dtype_op == SPION_F32 && full_dense(vl, p, vals)) {       // trans: simt_dense_grads
+    constexpr int smem = OGROUPS * DSTAGES * SPMM_STAGE * (int)sizeof(float);
+    SPION_CUDA_TRY(cudaFuncSetAttribute(spmm_dense_split, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    spmm_dense_split<<<dim3(p.nb, BH, d / 32), 64 * OGROUPS, smem, st>>>((const float*)vals, (const float*)Bop, lb, (float*)out, lo, vl.L);
     SPION_LAUNCH_CHECK();
     return SPION_OK;
   }
@@ -1025,6 +1304,66 @@ int softmax_bwd_dense_t(const float* dP, const float* P, float* dS, int BH, int 
   if (L % SLAB == 0 && ((uintptr_t)P & 15) == 0 && per <= 128) rc = per <= 64 ? slab(softmax_bwd_dense_t_slab<64>) : slab(softmax_bwd_dense_t_slab<128>);
   else softmax_bwd_dense_t_kernel<<<dim3((L + 31) / 32, BH), DENSE_WARPS * 32, 0, st>>>(dP, P, dS, L, scale);
   if (rc) return rc;
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}
+
+// ------------------------------------------------------------------------------ dense phase, several stages per launch
+template <class F>
+static int with_slices(int L, F f) {
+  const int keys = (slab_per(L) + 15) / 16;            // of a lane; an even number, four at least
+  switch (keys <= 4 ? 4 : (keys + 1) & ~1) {
+    case 4: return f(std::integral_constant<int, 4>());
+    case 6: return f(std::integral_constant<int, 6>());
+    case 8: return f(std::integral_constant<int, 8>());
+    case 10: return f(std::integral_constant<int, 10>());
+    case 12: return f(std::integral_constant<int, 12>());
+    case 14: return f(std::integral_constant<int, 14>());
+    default: return f(std::integral_constant<int, 16>());
+  }
+}
+// 64-wide tiles in the S^T layout, operand rows of K (V) and values that are read in 16-byte pieces, up to SLICE_MAX_L keys.
+// Measured, us in two launches and in one (matrices x L, d): backward 4 x 1024, 32 24, 20; 8 x 1024, 64 58, 51; 12 x 1024, 32 74, 52; 8 x 1472, 32 136,
+// 78; 20 x 512, 32 23.5, 23.3; 4 x 512, 64 14, 9; 96 x 256, 32 34, 36; 64 x 256, 64 31, 35: from 512 keys on, and where one wave of CTAs holds all.
+// Forward 4 x 512, 64 12, 9; 4 x 1024, 32 20, 20; 8 x 1024, 64 46, 52; 60 x 1024, 32 212, 228; 1 x 2048, 64 131, 31 (rows that the slab kernel does not
+// take): one wave or such rows, else S is faster with a kernel of its own (sixteen warps per SM hide the latencies of all stages at once badly).
+bool simt_dense_joint(bool backward, int L, int d, int BH, const void* rows, const void* values, const void* values2) {
+  if (L % DT != 0 || L > SLICE_MAX_L || d % KC != 0 || d > 64 || BH > 65535 || !aligned_to(rows, 16) || !aligned_to(values, 16) || !aligned_to(values2, 16))
+    return false;
+  const bool one_wave = (long long)BH * (L / SLAB) <= 2LL * sm_count();
+  return one_wave || (backward ? L >= 512 : DENSE_WARPS * slab_slice(L) * (int)sizeof(float) > SLAB_SMEM);
+}
+int simt_dense_scores(const float* Q, OperandLayout lq, const float* K, float* P, int BH, int L, int d, float scale, const float* keypad, float floor_v, cudaStream_t st) {
+  const int rc = with_slices(L, [&](auto kpl) -> int {
+    constexpr int KPL = decltype(kpl)::value, smem = DENSE_WARPS * 256 * KPL * (int)sizeof(float);
+    auto k = dense_scores_kernel<KPL>;
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k<<<dim3(L / SLAB, BH), DENSE_WARPS * 32, smem, st>>>(Q, lq, K, P, L, d, scale, keypad, floor_v);
+    return SPION_OK;
+  });
+  if (rc) return rc;
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}
+int simt_dense_dscores(const float* dO, OperandLayout ldo, const float* V, const float* P, float* dS, int BH, int L, int d, float scale, cudaStream_t st) {
+  const int rc = with_slices(L, [&](auto kpl) -> int {
+    constexpr int KPL = decltype(kpl)::value;
+    const int smem = DENSE_WARPS * (slab_per(L) * SLAB + 128 * KPL) * (int)sizeof(float);
+    auto k = dense_dscores_kernel<KPL>;
+    SPION_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k<<<dim3(L / SLAB, BH), DENSE_WARPS * 32, smem, st>>>(dO, ldo, V, P, dS, L, d, scale);
+    return SPION_OK;
+  });
+  if (rc) return rc;
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}
+// whole tiles of 64 x 64 values (any L): all three products of the backward.  SPION_ERR_UNSUPPORTED: one by one (simt_spmm)
+int simt_dense_grads(const float* P, const float* dS, const float* Q, const float* K, const float* dO, OperandLayout lo, float* dQ, float* dK, float* dV,
+                     Pattern p, int BH, int L, int d, cudaStream_t st) {
+  const ValueLayout vl{VAL_DENSE_T, L, (long long)L * L};
+  if (d % 32 != 0 || BH > 65535 || !full_dense(vl, p, P) || !full_dense(vl, p, dS)) return SPION_ERR_UNSUPPORTED;
+  spmm_dense_grads<<<dim3(p.nb, BH, 3 * (d / 32)), 64, 0, st>>>(DenseGrads{P, dS, Q, K, dO, dQ, dK, dV, lo, L, d / 32});
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }

@@ -241,3 +241,32 @@ def test_errors_are_loud():
     Q, K, V, _ = synthetic.qkv(1, 1, 1, 128, 32)
     with pytest.raises(_lib.SpionError):
         mod(Q.cuda(), K.cuda(), V.cuda())                      # no mask set
+
+
+@pytest.mark.parametrize("B,H,L,d,kpm", [(1, 1, 64, 32, True), (2, 1, 192, 64, False), (40, 1, 256, 32, True), (1, 2, 512, 64, False),
+                                         (3, 2, 1088, 32, True), (1, 1, 2048, 64, False), (1, 1, 2112, 32, True)])
+def test_dense_reference_layout_in_joint_kernels(B, H, L, d, kpm):
+    """Stages of the dense phase that share a launch (short and long rows, one wave of CTAs and more, rows beyond what they take): P, out and
+    the gradients against fp64.  The gradient of the key bias, the column sum of dK, is zero but for rounding: P's rows sum to one within a few ulp,
+    so that it stays below 1e-5 of the sum of magnitudes."""
+    from spion_b200.attention import Attention
+    cfg = {"head_dim": d, "num_head": H, "max_seq_len": L, "batch_size": B, "block_size": 32, "transformer_dim": H * d,
+           "task": "lra-text" if kpm else "lra-image"}
+    layer = Attention(cfg).cuda()
+    g = torch.Generator(device="cuda").manual_seed(L + d)
+    q, k, v, do = (torch.randn(B, H, L, d, generator=g, device="cuda") for _ in range(4))
+    mask = torch.ones(B, L, device="cuda")
+    if kpm:
+        mask[0, L - L // 3:] = 0
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    out, attn = layer.attn(q, k, v, mask)
+    grads = torch.autograd.grad(out, (q, k, v), do)
+    q64, k64, v64 = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    s = q64 @ k64.transpose(-1, -2) / d ** 0.5 - 1e6 * (1 - mask.double())[:, None, None, :]
+    p64 = torch.softmax(s, dim=-1)
+    out64 = p64 @ v64
+    want = torch.autograd.grad(out64, (q64, k64, v64), do.double())
+    for got, ref in zip((attn, out, *grads), (p64, out64, *want)):
+        assert float((got.double() - ref).norm()) <= 2e-6 * float(ref.norm())      # fp32 sums of up to 2112 terms, one ulp 6e-8
+    assert float(grads[1].sum(2).abs().max()) <= 1e-5 * float(grads[1].abs().sum(2).max())
