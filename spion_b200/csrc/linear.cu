@@ -575,6 +575,8 @@ struct WgradArgs {
   TokMat dY, X;
   int T, N, K;
   int nc, kc, nstages;      // features of dY / X per CTA (blockIdx.y, blockIdx.z); nc + kc <= 256, multiples of 64 except at the end
+  int nraw;                 // fp32: halves of a tile that are copied ahead; which operands through tensor maps
+  bool box_y, box_x;
   float* part;              // [gridDim.x][N * K + N]
 };
 
@@ -587,9 +589,9 @@ struct WgradAcc {
   __device__ uint32_t at(int i) const { return two ? (uint32_t)(i >> 1) * cs + ((uint32_t)(i & 1) << 20) : (uint32_t)i * cs; }
 };
 
-// Loader warps.  bf16: what a copy costs is its addresses, and sixteen warps share them better than eight (524288 tokens, two
-// gradients: 135 -> 109 us).  fp32: the split, which more warps do not speed up (262144 tokens: 153 us, 157 with sixteen).
-template <int SPLIT> constexpr int WG_LOADERS = SPLIT == 1 ? 16 : 8;
+// Loader warps: what a copy costs is its addresses, and sixteen warps share them better than eight (524288 tokens, two gradients, bf16:
+// 135 -> 109 us).
+constexpr int WG_LOADERS = 16;
 constexpr uint32_t WCHUNK = 64 * 128;                    // [64 tokens x 64 features] bf16
 
 // As redo_outputs: features n .. n + 31 of dY by feature k of X, over the tokens of this CTA
@@ -612,9 +614,9 @@ __device__ __noinline__ void redo_gradient(const WgradArgs& a, int n, int k, flo
 
 // One CTA per SM and slice of the tokens.  dW^T accumulates in tensor memory over all tokens of the CTA: the chunks of X are one
 // MN-major A operand (M = 64 or 128), those of dY one MN-major B operand (N up to 192), so nothing is transposed.  The bias gradient is summed from the registers the loaders hold.
-template <int SPLIT, bool DY_BF16, bool X_BF16>
-__global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(const __grid_constant__ WgradArgs a) {
-  constexpr int LOADERS = WG_LOADERS<SPLIT>, ROWS = 4 * LOADERS, XR = 64 / ROWS;       // rows of a pass of all loaders, passes per tile
+template <bool DY_BF16, bool X_BF16>
+__global__ void __launch_bounds__(32 * (WG_LOADERS + 1), 1) k_lin_wgrad(const __grid_constant__ WgradArgs a) {
+  constexpr int LOADERS = WG_LOADERS, ROWS = 4 * LOADERS, XR = 64 / ROWS;       // rows of a pass of all loaders, passes per tile
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   next_may_start();                                                    // k_lin_reduce
   const uint32_t sbase = smem_u32(smem_raw);
@@ -622,8 +624,8 @@ __global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(c
   const int n0 = blockIdx.y * a.nc, k0 = blockIdx.z * a.kc;
   const int nlen = min(a.nc, a.N - n0), klen = min(a.kc, a.K - k0);
   const int nch = (nlen + 63) >> 6, kch = (klen + 63) >> 6, cpt = nch + kch;    // chunks per tile of 64 tokens
-  const uint32_t stage = (uint32_t)cpt * SPLIT * WCHUNK;
-  const uint32_t bars = sbase + a.nstages * ((a.nc + 63) / 64 + (a.kc + 63) / 64) * SPLIT * WCHUNK;
+  const uint32_t stage = (uint32_t)cpt * WCHUNK;
+  const uint32_t bars = sbase + a.nstages * ((a.nc + 63) / 64 + (a.kc + 63) / 64) * WCHUNK;
   const uint32_t full = bars, empty = bars + 64, acc_done = bars + 128, slot = bars + 136, sdb = bars + 256;
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
   float* sdb_ptr = reinterpret_cast<float*>(smem_raw + (sdb - sbase));        // [LOADERS][256]
@@ -703,7 +705,7 @@ __global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(c
     };
     auto place = [&](int st, int i, int x) -> uint32_t {
       const int r = lrow + ROWS * x;
-      return sbase + st * stage + i * SPLIT * WCHUNK + r * 128 + ((lc8 ^ (r & 7)) << 4);
+      return sbase + st * stage + i * WCHUNK + r * 128 + ((lc8 ^ (r & 7)) << 4);
     };
     bool ok = true;
     int n = 0;
@@ -751,7 +753,7 @@ __global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(c
         if (i < cpt && !(i < nch ? DY_BF16 : X_BF16)) {
 #pragma unroll
           for (int x = 0; x < XR; ++x) {
-            raw_store<SPLIT, false>(cur[i][x], place(st, i, x), WCHUNK);
+            raw_store<1, false>(cur[i][x], place(st, i, x), WCHUNK);
             if (i < nch) {
 #pragma unroll
               for (int e = 0; e < 8; ++e) db[i][e] += __uint_as_float(cur[i][x].w[e]);
@@ -800,33 +802,278 @@ __global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(c
       tc_fence_after();
       const int q = warp & 3, half = warp >> 2;
       const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16);
-      const WgradAcc acc(nlen, kch);
-      const int small = acc.total() - 1, used = min(small, (ntiles - (int)blockIdx.x + G_x - 1) / G_x);    // leading ones that were used
       const int m = kch == 1 ? q * 16 + (lane & 15) : q * 32 + lane;           // feature of X
       const bool min_ = (kch == 2 || lane < 16) && m < klen;
       for (int g = half; g < (nlen >> 5); g += LOADERS / 4) {
         uint32_t v[32];
         __syncwarp();
-        if (SPLIT == 3) {
+        tmem_ld32(tl + g * 32, v);
+        tmem_ld_wait();
+        if (min_) {
+          float* dst = part + (size_t)(n0 + g * 32) * a.K + k0 + m;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = 0u;
-          for (int s = 0; s < acc.sets; ++s) {
-            const int i = acc.two ? 2 * s + (lane >> 4) : s;                   // the accumulator in this lane
-            if ((acc.two ? 2 * s : s) >= used && s + 1 < acc.sets) continue;   // none of the set was used
-            uint32_t u[32];
-            tmem_ld32(tl + s * acc.cs + g * 32, u);
-            tmem_ld_wait();
-            const bool in = i < used || i == small;
+          for (int e = 0; e < 32; ++e) dst[(size_t)e * a.K] = __uint_as_float(v[e]);
+        }
+      }
+    }
+  } else {
+    bool ok = true;
+    int n = 0;
+    // D[features of X, features of dY]: both operands MN-major, chunks of 64 features WCHUNK apart
+    const uint32_t idesc = make_idesc_bf16(kch == 1 ? 64 : 128, nlen, 1, 1);
+    const uint64_t D0 = make_smem_desc(sbase, WCHUNK, 1024, LAYOUT_SW128);
+    for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++n) {
+      const int st = n % a.nstages;
+      ok = warp_wait(full + 8 * st, (uint32_t)(n / a.nstages) & 1u);
+      if (!ok) break;
+      if (elect_one()) {
+        tc_fence_after();
+        const uint64_t dd = desc_advance(D0, st * stage), dx = desc_advance(dd, (uint32_t)nch * WCHUNK);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = in ? __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e])) : v[e];
+        for (int kk = 0; kk < 4; ++kk) mma_bf16(tmem, desc_advance(dx, kk * 2048), desc_advance(dd, kk * 2048), idesc, kk > 0 || n > 0);
+        mma_commit(empty + 8 * st);
+        if (tile + G_x >= ntiles) mma_commit(acc_done);
+      }
+      __syncwarp();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == LOADERS) tmem_dealloc(tmem, 512u);
+}
+
+// The same for fp32 operands: both in three bf16 parts, six products.  Half a tile (32 tokens) at a time:
+//   warp 17       copies the rows of both operands as they lie in memory (tensor maps, boxes of 32 or 64 features) into a ring of `nraw` halves, a
+//                 lane one box of every half: with the addresses formed half by half, or a copy per row, this warp was the limit (64, 236 us)
+//   warps 0-15    two groups of eight take halves in turn: sixteen bytes twice per lane and chunk, split, three images
+//   warp 16       the products
+// Loads through registers kept 64 KB per SM in flight, but a load that waits for room in what shared memory leaves of the L1 cache keeps the
+// stores behind it waiting too: three 16-byte stores of a lane took 450 cycles, 60 without the loads, the split itself 5 % of the kernel.
+// 262144 tokens, 64 x 192 97 us -> 60, 64 x 64 50 -> 41; 15040 tokens, 192 x 576 39 either way.
+constexpr uint32_t HCHUNK = 32 * 128, HRAW = 32 * 256;   // 32 tokens x 64 features: one bf16 image, fp32
+// features of a copy: 64 where heads (rows) are whole multiples of that, else 32
+__device__ __forceinline__ int copy_width(const TokMat& m) { return (m.d & 63) == 0 ? 64 : 32; }
+// What a lane of warp 17 copies of every half: one box of an operand, or, where a half may span two sequences, one row of all boxes
+struct HalfCopy {
+  const CUtensorMap* map;
+  int x, hl, bl;            // column; rows of the map per head of this box, per sequence
+  uint32_t dst;
+  bool on;
+};
+__device__ __forceinline__ HalfCopy half_copy(const TokMat& m, const CUtensorMap* maps, int c, int f, int end, uint32_t chunk) {
+  const int w = copy_width(m);
+  HalfCopy h;
+  h.on = c + f < end && f % w == 0;
+  h.dst = chunk + (uint32_t)(f / w) * 32u * (uint32_t)(4 * w);
+  c += f;
+  const int i = h.on ? which_matrix(m, c) : 0;
+  c -= i * m.per;
+  h.map = maps + i;
+  const bool heads = m.L != 0x7fffffff;
+  const int head = heads ? c >> m.dsh : 0;
+  h.x = c - head * m.d;
+  h.hl = heads ? head * m.L : 0;
+  h.bl = heads ? (m.per >> m.dsh) * m.L : 0;
+  return h;
+}
+// rows of a half that may span two sequences: lane = token
+__device__ __forceinline__ void copy_rows(const TokMat& m, int c, int end, int t, int rows, uint32_t dst, uint32_t bar, int lane) {
+  const int w = copy_width(m);
+  RowIt r;
+  r.init(m, min(t + lane, t + rows - 1));
+  for (int f = 0; f < 64 && c + f < end; f += w)
+    if (lane < rows)
+      bulk_load(dst + (uint32_t)(f / w) * 32u * (uint32_t)(4 * w) + lane * 4 * w, tok_col<const float>(m, c + f) + r.off(m), bar, (uint32_t)(4 * w));
+}
+// Eight features of one token of a copied chunk.  Lanes of the upper features read their second half first (no two lanes on the same banks).
+__device__ __forceinline__ uint32_t half_at(int width, int row, int lc8) {
+  return width == 64 ? row * 256 + lc8 * 32 : (lc8 >> 2) * 4096 + row * 128 + (lc8 & 3) * 32;
+}
+__device__ __forceinline__ void read_half(uint32_t at, bool upper, uint32_t (&v)[8]) {
+  uint32_t p[4], q[4];
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(p[0]), "=r"(p[1]), "=r"(p[2]), "=r"(p[3]) : "r"(at + (upper ? 16u : 0u)) : "memory");
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(at + (upper ? 0u : 16u)) : "memory");
+#pragma unroll
+  for (int e = 0; e < 4; ++e) { v[e] = upper ? q[e] : p[e]; v[4 + e] = upper ? p[e] : q[e]; }
+}
+
+struct WgradMaps { CUtensorMap y[3], x[3]; };
+__global__ void __launch_bounds__(32 * (WG_LOADERS + 2), 1) k_lin_wgrad_fp32(const __grid_constant__ WgradArgs a, const __grid_constant__ WgradMaps maps) {
+  constexpr int LOADERS = WG_LOADERS;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  next_may_start();                                                    // k_lin_reduce
+  const uint32_t sbase = smem_u32(smem_raw);
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
+  const int n0 = blockIdx.y * a.nc, k0 = blockIdx.z * a.kc;
+  const int nlen = min(a.nc, a.N - n0), klen = min(a.kc, a.K - k0);
+  const int nch = (nlen + 63) >> 6, kch = (klen + 63) >> 6, cpt = nch + kch;
+  const int most = (a.nc + 63) / 64 + (a.kc + 63) / 64;
+  const uint32_t stage = (uint32_t)cpt * 3 * HCHUNK;
+  const uint32_t raws = sbase + a.nstages * most * 3 * HCHUNK, rawb = (uint32_t)cpt * HRAW;
+  const uint32_t bars = raws + a.nraw * most * HRAW;
+  const uint32_t full = bars, empty = bars + 64, raw_full = bars + 128, raw_free = bars + 192, acc_done = bars + 256, slot = bars + 264;
+  uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
+  float* sdb_ptr = reinterpret_cast<float*>(smem_raw + (raws - sbase));       // [LOADERS][256], when all halves have been read
+  const int ntiles = (a.T + 63) >> 6, G_x = (int)gridDim.x;
+  const int my_tiles = (ntiles - (int)blockIdx.x + G_x - 1) / G_x;
+  // the last tile of all may have one half only
+  const int halves = 2 * my_tiles - ((ntiles - 1) % G_x == (int)blockIdx.x && a.T - (ntiles - 1) * 64 <= 32 ? 1 : 0);
+  __shared__ int s_abort;
+
+  if (warp == LOADERS) {
+    if (lane == 0) {
+      s_abort = *reinterpret_cast<volatile int*>(&g_lin_status);
+      for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, 8); mbar_init(empty + 8 * i, 1); }
+      for (int i = 0; i < a.nraw; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_free + 8 * i, 8); }
+      mbar_init(acc_done, 1);
+      fence_barrier_init();
+    }
+    __syncwarp();
+    tmem_alloc(slot, 512u);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *slot_ptr;
+  if (s_abort != 0) {
+    __syncthreads();
+    if (warp == LOADERS) tmem_dealloc(tmem, 512u);
+    return;
+  }
+  auto first_token = [&](int n) { return ((int)blockIdx.x + (n >> 1) * G_x) * 64 + (n & 1) * 32; };
+
+  // Half n is in raw slot n % nraw and stage n % nstages.  A parity tells two phases apart: at a wait the phase before must be over and the one after
+  // must not be.  raw_free, full: one waiter (warp 17, warp 16) for every phase.  raw_full: nraw is even, so a slot's phases are all one group's.
+  // empty, three stages: a group waits for the products of half n - 3, the phase before is that of half n - 6; it has waited for those of half
+  // n - 5, which were issued later.  The next phase needs what the waiter does after its wait.
+  if (warp == LOADERS + 1) {
+    const bool by = a.box_y, bx = a.box_x;
+    const int u = lane >> 1, f = (lane & 1) * 32;          // this lane's box: chunk and half of it
+    const bool isd = u < nch;
+    HalfCopy h = isd ? half_copy(a.dY, maps.y, n0 + 64 * u, f, n0 + nlen, u * HRAW) : half_copy(a.X, maps.x, k0 + 64 * (u - nch), f, k0 + klen, u * HRAW);
+    h.on = h.on && u < cpt && (isd ? by : bx);
+    const TokMat& mine = isd ? a.dY : a.X;
+    RowIt at;
+    at.init(mine, min((int)blockIdx.x * 64, a.T - 1));
+    const int far = 64 * G_x - 32, far_b = far / mine.L, far_l = far - far_b * mine.L;
+    int n = 0, s = 0;
+    uint32_t round = 0;
+    for (; n < halves; ++n) {
+      if (round > 0 && !warp_wait(raw_free + 8 * s, (round - 1) & 1u)) break;
+      const int t = first_token(n), rows = min(32, a.T - t);
+      const uint32_t bar = raw_full + 8 * s, dst = raws + s * rawb;
+      if (lane == 0) mbar_expect_tx(bar, (uint32_t)((by ? 32 : rows) * nlen + (bx ? 32 : rows) * klen) * 4u);
+      __syncwarp();
+      if (h.on) tma_load_2d(dst + h.dst, h.map, bar, h.x, at.b * h.bl + h.hl + at.l);
+      if (!by) for (int i = 0; i < nch; ++i) copy_rows(a.dY, n0 + 64 * i, n0 + nlen, t, rows, dst + i * HRAW, bar, lane);
+      if (!bx) for (int i = 0; i < kch; ++i) copy_rows(a.X, k0 + 64 * i, k0 + klen, t, rows, dst + (nch + i) * HRAW, bar, lane);
+      if (n & 1) at.add(mine, far_b, far_l);
+      else at.add(mine, 0, 32);
+      if (++s == a.nraw) { s = 0; ++round; }
+    }
+    // after a wait that gave up: nothing is on its way to this CTA's shared memory when it leaves
+    for (int m = max(0, n - a.nraw); n < halves && m < n; ++m) warp_wait(raw_full + 8 * (m % a.nraw), (uint32_t)(m / a.nraw) & 1u);
+  } else if (warp < LOADERS) {
+    const int group = warp >> 3, lrow = (tid & 255) >> 3, lc8 = tid & 7;
+    const bool upper = lc8 >= 4;
+    uint32_t from[4];                                      // this thread's eight features of every chunk of a slot
+    bool some[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      from[i] = raws + i * HRAW + half_at(copy_width(i < nch ? a.dY : a.X), lrow, lc8);
+      some[i] = lc8 * 8 < (i < nch ? nlen - 64 * i : klen - 64 * (i - nch));
+    }
+    const uint32_t to = sbase + lrow * 128 + ((lc8 ^ (lrow & 7)) << 4);
+    float db[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) db[i][e] = 0.f;
+    bool ok = true;
+    int s = group, st = group;                             // slot and stage of the half, how often they have been used before
+    uint32_t s_use = 0, st_use = 0;
+    for (int n = group; n < halves; n += 2) {
+      ok = warp_wait(raw_full + 8 * s, s_use & 1u);
+      if (!ok) break;
+      const bool in = first_token(n) + lrow < a.T;
+      Raw<false> r[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < cpt) read_half(from[i] + s * rawb, upper, r[i].w);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(raw_free + 8 * s);
+      if (st_use > 0) ok = warp_wait(empty + 8 * st, (st_use - 1) & 1u);
+      if (!ok) break;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i < cpt) {
+          if (!in || !some[i])                             // past the last token or feature: what the ring held before
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[i].w[e] = 0u;
+          raw_store<3, false>(r[i], to + st * stage + i * 3 * HCHUNK, HCHUNK);
+          if (i < nch)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) db[i][e] += __uint_as_float(r[i].w[e]);
+        }
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + 8 * st);
+      if ((s += 2) >= a.nraw) { s -= a.nraw; ++s_use; }
+      if ((st += 2) >= a.nstages) { st -= a.nstages; ++st_use; }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * LOADERS) : "memory");       // the loader warps
+    // column sums of dY: lanes with the same lc8 of a warp, then the warps in order
+    if (blockIdx.z == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i < nch) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            float s = db[i][e];
+            s += __shfl_xor_sync(0xffffffffu, s, 8);
+            s += __shfl_xor_sync(0xffffffffu, s, 16);
+            if (lane < 8) sdb_ptr[warp * 256 + i * 64 + lane * 8 + e] = s;
           }
-          if (acc.two) {
+        }
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * LOADERS) : "memory");
+    float* part = a.part + (size_t)blockIdx.x * ((size_t)a.N * a.K + a.N);
+    if (blockIdx.z == 0 && tid < nlen) {
+      float s = 0.f;
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(__shfl_xor_sync(0xffffffffu, v[e], 16)));
-          }
-        } else {
-          tmem_ld32(tl + g * 32, v);
+      for (int w = 0; w < LOADERS; ++w) s += sdb_ptr[w * 256 + tid];
+      part[(size_t)a.N * a.K + n0 + tid] = s;
+    }
+    if (ok) ok = warp_wait(acc_done, 0u);
+    if (ok) {
+      tc_fence_after();
+      const int q = warp & 3, half = warp >> 2;
+      const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16);
+      const WgradAcc acc(nlen, kch);
+      const int small = acc.total() - 1, used = min(small, my_tiles);          // leading ones that were used
+      const int m = kch == 1 ? q * 16 + (lane & 15) : q * 32 + lane;           // feature of X
+      const bool min_ = (kch == 2 || lane < 16) && m < klen;
+      for (int g = half; g < (nlen >> 5); g += LOADERS / 4) {
+        uint32_t v[32];
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < 32; ++e) v[e] = 0u;
+        for (int s = 0; s < acc.sets; ++s) {
+          const int i = acc.two ? 2 * s + (lane >> 4) : s;                     // the accumulator in this lane
+          if ((acc.two ? 2 * s : s) >= used && s + 1 < acc.sets) continue;     // none of the set was used
+          uint32_t u[32];
+          tmem_ld32(tl + s * acc.cs + g * 32, u);
           tmem_ld_wait();
+          const bool in = i < used || i == small;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = in ? __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e])) : v[e];
+        }
+        if (acc.two) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(__shfl_xor_sync(0xffffffffu, v[e], 16)));
         }
         if (min_) {
           float* dst = part + (size_t)(n0 + g * 32) * a.K + k0 + m;
@@ -834,42 +1081,43 @@ __global__ void __launch_bounds__(32 * (WG_LOADERS<SPLIT> + 1), 1) k_lin_wgrad(c
 #pragma unroll
           for (int e = 0; e < 32; ++e) {
             dst[(size_t)e * a.K] = __uint_as_float(v[e]);
-            if (SPLIT == 3) probe = fmaf(__uint_as_float(v[e]), 0.f, probe);
+            probe = fmaf(__uint_as_float(v[e]), 0.f, probe);
           }
-          if (SPLIT == 3 && !all_finite(probe)) redo_gradient(a, n0 + g * 32, k0 + m, dst);
+          if (!all_finite(probe)) redo_gradient(a, n0 + g * 32, k0 + m, dst);
         }
       }
     }
   } else {
     bool ok = true;
-    int n = 0;
-    // D[features of X, features of dY]: both operands MN-major, chunks of 64 features SPLIT * WCHUNK apart
+    // D[features of X, features of dY]: both operands MN-major, chunks of 64 features three images apart
     const uint32_t idesc = make_idesc_bf16(kch == 1 ? 64 : 128, nlen, 1, 1);
-    const uint64_t D0 = make_smem_desc(sbase, SPLIT * WCHUNK, 1024, LAYOUT_SW128);
+    const uint64_t D0 = make_smem_desc(sbase, 3 * HCHUNK, 1024, LAYOUT_SW128);
     const WgradAcc acc(nlen, kch);
-    const int leads = SPLIT == 3 ? acc.total() - 1 : 1;
-    int li = 0;                                            // leading accumulator of the tile
-    for (int tile = blockIdx.x; ok && tile < ntiles; tile += G_x, ++n, li = li + 1 < leads ? li + 1 : 0) {
-      const int st = n % a.nstages;
-      ok = warp_wait(full + 8 * st, (uint32_t)(n / a.nstages) & 1u);
+    const int leads = acc.total() - 1;
+    int li = 0, st = 0;                                    // leading accumulator of the tile; stage of the half
+    uint32_t st_use = 0;
+    for (int n = 0; ok && n < halves; ++n) {
+      ok = warp_wait(full + 8 * st, st_use & 1u);
       if (!ok) break;
       if (elect_one()) {
         tc_fence_after();
-        const uint64_t dd = desc_advance(D0, st * stage), dx = desc_advance(dd, (uint32_t)nch * SPLIT * WCHUNK);
+        const uint64_t dd = desc_advance(D0, st * stage), dx = desc_advance(dd, (uint32_t)nch * 3 * HCHUNK);
         const uint32_t lead_set = tmem + acc.at(li), small_set = tmem + acc.at(leads);
-        const uint32_t acc_l = n >= leads, acc_s = n > 0;
+        const uint32_t acc_l = (n & 1) || (n >> 1) >= leads, acc_s = n > 0;
 #pragma unroll
-        for (int pr = 0; pr < Prod<SPLIT>::N; ++pr) {
-          const bool lead = pr + 1 == Prod<SPLIT>::N;
+        for (int pr = 0; pr < Prod<3>::N; ++pr) {
+          const bool lead = pr + 1 == Prod<3>::N;
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_bf16(lead ? lead_set : small_set, desc_advance(dx, Prod<SPLIT>::b(pr) * WCHUNK + kk * 2048),
-                     desc_advance(dd, Prod<SPLIT>::a(pr) * WCHUNK + kk * 2048), idesc, kk > 0 ? 1u : (lead ? acc_l : (pr > 0 ? 1u : acc_s)));
+          for (int kk = 0; kk < 2; ++kk)
+            mma_bf16(lead ? lead_set : small_set, desc_advance(dx, Prod<3>::b(pr) * HCHUNK + kk * 2048),
+                     desc_advance(dd, Prod<3>::a(pr) * HCHUNK + kk * 2048), idesc, kk > 0 ? 1u : (lead ? acc_l : (pr > 0 ? 1u : acc_s)));
         }
         mma_commit(empty + 8 * st);
-        if (tile + G_x >= ntiles) mma_commit(acc_done);
+        if (n + 1 == halves) mma_commit(acc_done);
       }
       __syncwarp();
+      if (n & 1) li = li + 1 < leads ? li + 1 : 0;
+      if (++st == a.nstages) { st = 0; ++st_use; }
     }
   }
   tc_fence_before();
@@ -936,7 +1184,7 @@ int map_form(const spion_tokens* t, long long T) {
   return (t->head_dim == 32 || t->head_dim == 64) && t->cols % 64 == 0 && t->seq_len % 64 == 0 && T % t->seq_len == 0 &&
          T * t->heads <= 0x7fffffffLL ? MAP_HEADS : MAP_NONE;
 }
-int token_maps(const spion_tokens* t, long long T, CUtensorMap* m) {
+int encoder(TcState* s) {
   static std::atomic<void*> encode{nullptr};
   void* fn = encode.load(std::memory_order_acquire);
   if (!fn) {
@@ -948,13 +1196,36 @@ int token_maps(const spion_tokens* t, long long T, CUtensorMap* m) {
   int dev = 0;                                           // a thread whose first call this is has no current context, and encoding wants one
   SPION_CUDA_TRY(cudaGetDevice(&dev));
   SPION_CUDA_TRY(cudaSetDevice(dev));
+  s->encode = (EncodeTiledFn)fn;
+  return SPION_OK;
+}
+int token_maps(const spion_tokens* t, long long T, CUtensorMap* m) {
   TcState s;
-  s.encode = (EncodeTiledFn)fn;
+  int rc = encoder(&s);
+  if (rc) return rc;
   for (int i = 0; i < t->count; ++i) {
-    const int rc = t->heads > 0 ? make_map(&s, m + i, t->ptr[i], (uint64_t)T * t->heads, (uint32_t)t->head_dim, (uint32_t)t->head_dim, 64)
+    rc = t->heads > 0 ? make_map(&s, m + i, t->ptr[i], (uint64_t)T * t->heads, (uint32_t)t->head_dim, (uint32_t)t->head_dim, 64)
                                 : make_map(&s, m + i, t->ptr[i], (uint64_t)T, (uint32_t)t->cols, 64, 128);
     if (rc) return rc;
   }
+  return SPION_OK;
+}
+
+// fp32 operands of the weight gradient: boxes of 32 tokens, 64 features where heads (rows) are whole multiples of that, else 32
+bool half_boxes(const spion_tokens* t, long long T) {
+  return t->heads <= 0 || (t->seq_len % 32 == 0 && T % t->seq_len == 0 && T * t->heads <= 0x7fffffffLL);
+}
+int half_maps(const spion_tokens* t, long long T, CUtensorMap* m) {
+  TcState s;
+  const int rc = encoder(&s);
+  if (rc) return rc;
+  const uint32_t width = (uint32_t)(t->heads > 0 ? t->head_dim : t->cols);
+  const cuuint64_t dims[2] = {width, (cuuint64_t)T * (t->heads > 0 ? t->heads : 1)}, strides[1] = {(cuuint64_t)width * 4};
+  const cuuint32_t box[2] = {width % 64 == 0 ? 64u : 32u, 32u}, estr[2] = {1, 1};
+  for (int i = 0; i < t->count; ++i)
+    if (s.encode(m + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, t->ptr[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return SPION_ERR_CUDA;
   return SPION_OK;
 }
 
@@ -993,10 +1264,14 @@ int prepare_gemm() {
   static std::atomic<bool> done[64];
   return opt_in(k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>, done);
 }
-template <int SPLIT, bool DY_BF16, bool X_BF16>
+template <bool DY_BF16, bool X_BF16>
 int prepare_wgrad() {
   static std::atomic<bool> done[64];
-  return opt_in(k_lin_wgrad<SPLIT, DY_BF16, X_BF16>, done);
+  return opt_in(k_lin_wgrad<DY_BF16, X_BF16>, done);
+}
+int prepare_wgrad_fp32() {
+  static std::atomic<bool> done[64];
+  return opt_in(k_lin_wgrad_fp32, done);
 }
 
 template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
@@ -1017,26 +1292,46 @@ int launch_gemm(GemmArgs& a, const spion_tokens* tok, size_t smem, cudaStream_t 
   return SPION_OK;
 }
 
-template <int SPLIT, bool DY_BF16, bool X_BF16>
+template <bool DY_BF16, bool X_BF16>
 int launch_wgrad(const WgradArgs& a, int gx, size_t smem, cudaStream_t st) {
-  auto k = k_lin_wgrad<SPLIT, DY_BF16, X_BF16>;
-  const int rc = prepare_wgrad<SPLIT, DY_BF16, X_BF16>();
+  const int rc = prepare_wgrad<DY_BF16, X_BF16>();
   if (rc) return rc;
-  k<<<dim3(gx, (a.N + a.nc - 1) / a.nc, (a.K + a.kc - 1) / a.kc), 32 * (WG_LOADERS<SPLIT> + 1), smem, st>>>(a);
+  const dim3 grid(gx, (a.N + a.nc - 1) / a.nc, (a.K + a.kc - 1) / a.kc);
+  k_lin_wgrad<DY_BF16, X_BF16><<<grid, 32 * (WG_LOADERS + 1), smem, st>>>(a);
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}
+int launch_wgrad_fp32(WgradArgs& a, const spion_tokens* dY, const spion_tokens* X, int gx, size_t smem, cudaStream_t st) {
+  int rc = prepare_wgrad_fp32();
+  if (rc) return rc;
+  WgradMaps maps;
+  a.box_y = half_boxes(dY, a.T);
+  a.box_x = half_boxes(X, a.T);
+  if ((a.box_y && (rc = half_maps(dY, a.T, maps.y))) || (a.box_x && (rc = half_maps(X, a.T, maps.x)))) return rc;
+  const dim3 grid(gx, (a.N + a.nc - 1) / a.nc, (a.K + a.kc - 1) / a.kc);
+  k_lin_wgrad_fp32<<<grid, 32 * (WG_LOADERS + 2), smem, st>>>(a, maps);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
 
 // chunking of the weight gradient: at most four 64-wide chunks of dY and X per CTA, and what tensor memory holds
-bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, size_t* smem) {
+bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, int* raws, size_t* smem) {
   const int kw = K <= 64 ? 64 : 128;
   int nw = (N + 63) / 64 * 64;
   if (nw + kw > 256) nw = 256 - kw;
   const int cpt = (nw + kw) / 64;
-  const size_t stage = (size_t)cpt * split * WCHUNK;
-  for (int st = split == 1 ? 6 : 4; st >= (split == 1 ? 3 : 2); --st) {     // bf16 operands: two stages of copies in flight
-    const size_t total = st * stage + 256 + (split == 1 ? WG_LOADERS<1> : WG_LOADERS<3>) * 256 * 4;
-    if (total <= SMEM_MAX) { *nc = nw; *kc = kw; *stages = st; *smem = total; return true; }
+  *nc = nw; *kc = kw; *raws = 0;
+  if (split == 3) {
+    for (int st = 3; st >= 2; --st)
+      for (int raw = 6; raw >= 4; raw -= 2) {            // even: a slot belongs to one of the two groups
+        *smem = (size_t)cpt * (st * 3 * HCHUNK + raw * HRAW) + 512;
+        if (*smem <= SMEM_MAX) { *stages = st; *raws = raw; return true; }
+      }
+    return false;
+  }
+  for (int st = 6; st >= 3; --st) {                      // two stages of copies in flight
+    *smem = (size_t)st * cpt * WCHUNK + 256 + WG_LOADERS * 256 * 4;
+    if (*smem <= SMEM_MAX) { *stages = st; return true; }
   }
   return false;
 }
@@ -1047,9 +1342,9 @@ bool plan_wgrad(int split, int N, int K, int* nc, int* kc, int* stages, size_t* 
 // dW from operands of one sign, where every truncation adds up: 1.4e-7 (1.5e-7), 9.4e-7 (1.9e-7), 9.9e-7 (4.0e-7).
 constexpr int CHAIN = 40;
 int wgrad_grid(long long T, int N, int K, int split) {
-  int nc, kc, st;
+  int nc, kc, st, raws;
   size_t smem;
-  if (!plan_wgrad(split, N, K, &nc, &kc, &st, &smem)) return 0;
+  if (!plan_wgrad(split, N, K, &nc, &kc, &st, &raws, &smem)) return 0;
   const int per = ((N + nc - 1) / nc) * ((K + kc - 1) / kc);
   const long long tiles = (T + 63) / 64;
   long long gx = sm_count() / per;
@@ -1073,28 +1368,28 @@ static int max_contraction(int split, int N) {
 }
 
 extern "C" int spion_linear_supported(int in_features, int out_features, int fp32) {
-  int nc, kc, nacc, st;
+  int nc, kc, nacc, st, raws;
   size_t smem;
   const int sp = fp32 ? 3 : 1;
   if (in_features < 32 || out_features < 32 || in_features % 32 || out_features % 32) return 0;
   if (in_features > 1024 || out_features > 1024) return 0;
   return plan_gemm(sp, false, in_features, out_features, &nc, &nacc, &st, &smem) &&
          plan_gemm(sp, true, fp32 ? 64 : out_features, in_features, &nc, &nacc, &st, &smem) &&
-         plan_wgrad(sp, out_features, in_features, &nc, &kc, &st, &smem);
+         plan_wgrad(sp, out_features, in_features, &nc, &kc, &st, &raws, &smem);
 }
 
 extern "C" int spion_linear_prepare(int fp32) {
   int rc;
   if (fp32) {
     if ((rc = prepare_gemm<3, false, false, EPI_NONE, false>()) || (rc = prepare_gemm<3, false, true, EPI_NONE, false>())) return rc;
-    return prepare_wgrad<3, false, false>();
+    return prepare_wgrad_fp32();
   }
   if ((rc = prepare_gemm<1, true, false, EPI_NONE, true>()) || (rc = prepare_gemm<1, false, false, EPI_NONE, true>()) ||
       (rc = prepare_gemm<1, true, false, EPI_GELU, true>()) || (rc = prepare_gemm<1, false, false, EPI_GELU, true>()) ||
       (rc = prepare_gemm<1, true, true, EPI_DGELU, true>()) || (rc = prepare_gemm<1, true, true, EPI_NONE, true>()) ||
-      (rc = prepare_gemm<1, true, true, EPI_NONE, false>()) || (rc = prepare_wgrad<1, true, false>()))
+      (rc = prepare_gemm<1, true, true, EPI_NONE, false>()) || (rc = prepare_wgrad<true, false>()))
     return rc;
-  return prepare_wgrad<1, true, true>();
+  return prepare_wgrad<true, true>();
 }
 
 int linear_status(int reset, cudaStream_t st) {
@@ -1223,14 +1518,14 @@ extern "C" int spion_linear_backward_weight(const spion_tokens* dY, const spion_
   a.dY = to_mat(dY); a.X = to_mat(X);
   a.T = (int)T; a.N = out_features; a.K = in_features; a.part = workspace;
   size_t smem;
-  if (!plan_wgrad(fp32 ? 3 : 1, a.N, a.K, &a.nc, &a.kc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
+  if (!plan_wgrad(fp32 ? 3 : 1, a.N, a.K, &a.nc, &a.kc, &a.nstages, &a.nraw, &smem)) return SPION_ERR_UNSUPPORTED;
   const int gx = wgrad_grid(T, a.N, a.K, fp32 ? 3 : 1);
   if (gx < 1) return SPION_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)cuda_stream;
   int rc;
-  if (fp32) rc = launch_wgrad<3, false, false>(a, gx, smem, st);
-  else if (dY->is_bf16) rc = X->is_bf16 ? launch_wgrad<1, true, true>(a, gx, smem, st) : launch_wgrad<1, true, false>(a, gx, smem, st);
-  else rc = X->is_bf16 ? launch_wgrad<1, false, true>(a, gx, smem, st) : launch_wgrad<1, false, false>(a, gx, smem, st);
+  if (fp32) rc = launch_wgrad_fp32(a, dY, X, gx, smem, st);
+  else if (dY->is_bf16) rc = X->is_bf16 ? launch_wgrad<true, true>(a, gx, smem, st) : launch_wgrad<true, false>(a, gx, smem, st);
+  else rc = X->is_bf16 ? launch_wgrad<false, true>(a, gx, smem, st) : launch_wgrad<false, false>(a, gx, smem, st);
   if (rc) return rc;
   const long long nw = (long long)a.N * a.K, n = nw + a.N;
   SPION_CUDA_TRY(launch_after(k_lin_reduce, dim3((unsigned)((n / 4 + 31) / 32)), dim3(256), 0, st, workspace, gx, n, nw, dW, db));

@@ -76,6 +76,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap
       : "r"(smem_dst), "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// bytes as they lie in memory: both addresses and the size multiples of 16
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bar, uint32_t bytes) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               :: "r"(smem_dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
 // shared -> global tile store (bulk async group); the smem tile must be visible to the async proxy
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t smem_src, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"

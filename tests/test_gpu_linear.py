@@ -69,6 +69,15 @@ def test_linear_kernels(B, L, H, d, K, nw, mode, split):
 
 # bf16 tokens, more than 148 tiles of 128 (read through tensor maps) and fewer: sequences of 64-token boxes that end at and in the
 # middle of a tile, row-major tails of 56 and 1 tokens, heads of 32 and 64, one to three matrices; widths and lengths that are copied
+# sequences of whole half-tiles (boxes of 32 tokens): one half, an odd number of them, several tiles per CTA; boxes of 32 and 64 features, rows
+# of one head and parts of longer rows
+@pytest.mark.parametrize("B,L,H,d,K,nw", [(1, 32, 1, 64, 64, 1), (3, 32, 2, 32, 96, 3), (5, 96, 3, 64, 192, 3), (2, 64, 1, 128, 160, 1), (70, 320, 2, 64, 64, 3),
+                                          (100, 320, 2, 32, 64, 1)])
+def test_fp32_linear_kernels_on_whole_boxes(B, L, H, d, K, nw):
+    for split in (False, True):
+        test_linear_kernels(B, L, H, d, K, nw, "fp32", split)
+
+
 @pytest.mark.parametrize("B,L,H,d,N,nw", [(149, 128, 2, 32, 64, 1), (101, 192, 2, 32, 64, 3), (300, 64, 4, 32, 96, 1), (61, 320, 1, 64, 64, 3),
                                           (101, 192, 2, 64, 192, 1), (1, 19000, 2, 32, 64, 3), (1, 19073, 1, 64, 128, 1),
                                           (40, 1984, 2, 32, 64, 3), (101, 192, 3, 32, 64, 1), (120, 160, 2, 32, 64, 3),
