@@ -169,6 +169,45 @@ def test_gelu_on_bf16_tokens(T, K, N):
     assert _rel(dX, _bf(_bf(dY.double() @ _bf(V)) * slope)) < 1e-3
 
 
+@pytest.mark.parametrize("T,K,N", [(19000, 64, 128), (20001, 32, 96), (300, 64, 64)])
+def test_gelu_of_every_bf16_number(T, K, N):
+    """Activation and its derivative by table, inside and outside of its range (subnormals, infinities and NaN too), the outputs through tiles in
+    shared memory (more than 148 tiles of 128 tokens) and from registers: the same bits as the formulas evaluated for every bf16 number, which
+    are the framework's GELU to two roundings of fp32 and one of bf16."""
+    P = ctypes.c_void_p
+    st = P(torch.cuda.current_stream().cuda_stream)
+    ref = ctypes.byref
+    g = torch.Generator(device="cuda").manual_seed(T)
+    bits = torch.randint(0, 65536, (T, N), generator=g, device="cuda", dtype=torch.int32)
+    bits[:T // 2] = (torch.randn(T // 2, N, generator=g, device="cuda").bfloat16().view(torch.int16).int()) & 0xffff
+    h = bits.to(torch.int16).view(torch.bfloat16).contiguous()
+    # derivative: dX = (dY V) * gelu'(h), dY V = a column of ones by an all-ones first feature
+    dY, V = torch.zeros(T, K, device="cuda", dtype=torch.bfloat16), torch.zeros(K, N, device="cuda")
+    dY[:, 0] = 1
+    V[0] = 1
+    dX = torch.empty(T, N, device="cuda", dtype=torch.bfloat16)
+    one = lambda t: (P * 3)(t.data_ptr(), None, None)
+    check(lib.spion_linear_backward_input(ref(_tokens([dY])), one(V), 1, 0, P(h.data_ptr()), ref(_tokens([dX])), T, N, K, st))
+    x = h.double()
+    want = 0.5 * (1 + torch.erf(x / 2 ** 0.5)) + x * torch.exp(-0.5 * x * x) / (2 * torch.pi) ** 0.5
+    ok = torch.isfinite(x)
+    err = (dX.double() - want).abs()
+    assert bool((err[ok] <= 2 ** -8 * want[ok].abs() + 1e-6).all())
+    assert bool(torch.isnan(dX[torch.isnan(x)]).all())
+    # activation: h again from a weight of ones, one bf16 number per token
+    col = h[:, :1].contiguous()
+    X, W, b = torch.zeros(T, K, device="cuda", dtype=torch.bfloat16), torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda")
+    X[:, :1] = torch.where(torch.isfinite(col), col, 0)
+    W[:, 0] = 1
+    Y, G = (torch.empty(T, N, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    check(lib.spion_linear_forward(ref(_tokens([X])), one(W), one(b), 1, 0, ref(_tokens([Y])), P(G.data_ptr()), T, K, N, st))
+    y = X[:, :1].double().expand(T, N)
+    assert bool(((Y.double() - y).abs() <= 1e-37).all())           # subnormals may be flushed
+    want = 0.5 * y * (1 + torch.erf(y / 2 ** 0.5))
+    assert bool(((G.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * y.abs().clamp(max=10) + 1e-37).all())
+    assert lib.spion_linear_status(1) == 0
+
+
 @pytest.mark.parametrize("native,dtype,bs,L,dense", [(True, "bf16", 64, 192, False), (True, "bf16", 64, 128, True),
                                                      (True, "fp32", 32, 160, False), (False, "fp32", 32, 96, False)])
 def test_attention_layer_in_one_node_equals_its_stages(native, dtype, bs, L, dense):
