@@ -94,7 +94,10 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 // output projection 39 -> 27, its gradient (row-major) 39 -> 25.  Other widths, sequences that are no multiple of 64 and calls of one tile
 // per CTA keep the copies; so do the weight gradients, where boxes of 64-byte rows were slower (two of them 136 us, 143 through maps).
 enum : int { MAP_NONE = 0, MAP_ROWS = 1, MAP_HEADS = 2 };
-struct LinMaps { CUtensorMap m[3]; };
+struct LinMaps {
+  CUtensorMap m[3];         // bf16 A
+  CUtensorMap y[3], g, h;   // staged: Y, activation, pre-activation
+};
 __device__ __forceinline__ int which_matrix(const TokMat& t, int c) { return (c >= t.per) + (c >= 2 * t.per); }
 // One thread: features c .. c + 63 of 64 tokens from t on of a head-split operand; the images of a chunk of heads of 32 are `image` bytes apart
 __device__ __forceinline__ void load_heads(const TokMat& t, const CUtensorMap* m, uint32_t dst, uint32_t image, uint32_t bar, int c, int tok) {
@@ -154,6 +157,7 @@ struct GemmArgs {
   int nacc;                 // accumulators per tile (fp32 mode): the leading products rotate over nacc - 1 of them by chunk
   int parts;                // bf16 gradient of three stacked layers: chunks per layer (0: one accumulator for the whole contraction)
   int tma;                  // bf16 A through maps.m[0 .. 2] (MAP_*)
+  int staged;               // outputs (and h) through shared memory and the other maps
   const __nv_bfloat16* h;   // EPI_DGELU: pre-activation [T, N]
   __nv_bfloat16* g;         // EPI_GELU: activation [T, N] (Y receives the pre-activation)
   // What a backward reads in place of the caller's tensors.  262144 tokens of 64 fp32 features: 33 MB written here, 33 MB less read by
@@ -230,8 +234,12 @@ template <int EPI> __device__ __forceinline__ void look_up(const float* tab, con
 // One persistent CTA per SM over tiles of 128 tokens: warps 0-7 bring 64-feature chunks of A through registers (a chunk of
 // loads in flight while the previous one is converted) into a ring of shared-memory stages, warp 8 issues the MMAs
 // (M = 128, two accumulator buffers in tensor memory), warps 9-16 write finished tiles.  W sits in shared memory for the
-// whole run.  Bound by the HBM passes over A and Y.  65536 tokens, 64 x 128: with GELU 20.6 us, 19.2 with the table above, with its derivative
-// 31.3, 25.9; 524288 tokens 107, 94 and 179, 141.
+// whole run.  Bound by the HBM passes over A and Y.
+// A lane has 32 features of a token: written from registers, an instruction touches 32 lines for 32 bytes each, 14 bytes a cycle and SM
+// whatever the form of Y.  Calls of more tiles than CTAs write them to a tile of 32 x 32 in shared memory that a bulk store takes to
+// its place, and fetch the pre-activations the same way; sequences that are no multiple of 32, and outputs that are added to, keep
+// the stores from registers.  Us, before, with the table above, and with the tiles too: 65536 tokens, 64 x 128, GELU 20.6, 19.2, 17.6; its derivative
+// 31.3, 25.9, 24.6; 524288 tokens 107, 94, 81 and 179, 141, 111; fp32, 262144 tokens, 64 x 192 67, -, 50; 64 x 64 37, -, 30.
 template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
 __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constant__ GemmArgs a, const __grid_constant__ LinMaps maps) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -251,6 +259,9 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
   uint32_t* slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (slot - sbase));
   float* bias_ptr = reinterpret_cast<float*>(smem_raw + (sBias - sbase));
   float* tab = reinterpret_cast<float*>(smem_raw + (bars + 256u - sbase));
+  // staged: a tile of 32 x 32 outputs per writing warp, with GELU two, with its derivative one and one of pre-activations
+  constexpr uint32_t OTILE = Y_BF16 ? 2048u : 4096u, OWARP = (EPI == EPI_NONE ? 1u : 2u) * OTILE;
+  const uint32_t outs = (bars + 256u + (EPI != EPI_NONE ? TAB_BYTES : 0u) + 1023u) & ~1023u, hbars = bars + 168;
 
   const int ntiles = (a.T + 127) >> 7;
   const int G_x = (int)gridDim.x;
@@ -277,6 +288,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
       s_abort = *reinterpret_cast<volatile int*>(&g_lin_status);
       for (int i = 0; i < a.nstages; ++i) { mbar_init(full + 8 * i, tma ? 1 : LG_LOADERS); mbar_init(empty + 8 * i, 1); }
       for (int i = 0; i < 2; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_empty + 8 * i, 8); }
+      for (int i = 0; i < 8; ++i) mbar_init(hbars + 8 * i, 1);
       fence_barrier_init();
       if (tma && s_abort == 0) {                         // the first chunks are on their way before the weights are converted
         fence_proxy_async();
@@ -500,18 +512,50 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     RowIt orow;
     const int ostep = G_x * 128, ostep_b = ostep / a.Y.L, ostep_l = ostep - ostep_b * a.Y.L;
     orow.init(a.Y, min(a.T - 1, (int)blockIdx.x * 128 + q * 32 + lane));
+    const uint32_t obuf = outs + (uint32_t)(warp - LG_LOADERS - 1) * OWARP, hbuf = obuf + OTILE, hbar = hbars + 8 * (warp - LG_LOADERS - 1);
+    const bool staged = a.staged;
+    uint32_t hpar = 0;
+    bool h_due = false;                                  // a copy is on its way to hbuf
+    // pre-activations of group g of a tile: staged, a copy into this warp's tile; else registers.  Rows past the last token are zeros.
+    uint32_t hw[2][8];
+    auto load_h = [&](int tile, int g) {
+      const int t0 = tile * 128 + q * 32;
+      if (tile >= ntiles || t0 >= a.T || g >= ngroups) return;
+      if (staged) {
+        h_due = true;
+        if (lane == 0) {
+          mbar_expect_tx(hbar, 2048u);
+          tma_load_2d(hbuf, &maps.h, hbar, n0 + g * 32, t0);
+        }
+      } else {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) ld_v8_if(t0 + lane < a.T, a.h + (size_t)(t0 + lane) * a.N + n0 + g * 32 + 16 * x, hw[x]);
+      }
+    };
+    if (EPI == EPI_DGELU) load_h(blockIdx.x, half);
+    // 32 outputs of a lane's row to the warp's tile, and from there to column c of Y's rows
+    auto put = [&](uint32_t buf, const uint32_t* w, const CUtensorMap* m, int x, int y) {
+      if (lane == 0) bulk_wait_read_all();               // the store before has read its tile
+      __syncwarp();
+#pragma unroll
+      for (int p = 0; p < (Y_BF16 ? 4 : 8); ++p) {
+        const uint32_t (&v)[4] = *reinterpret_cast<const uint32_t (*)[4]>(w + 4 * p);
+        st_shared16(buf + (Y_BF16 ? lane * 64 + ((p ^ ((lane >> 1) & 3)) << 4) : lane * 128 + ((p ^ (lane & 7)) << 4)), v);
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(m, buf, x, y);
+        bulk_commit();
+      }
+    };
     for (int tile = blockIdx.x; tile < ntiles; tile += G_x, ++j, orow.add(a.Y, ostep_b, ostep_l)) {
       const int buf = j & 1;
-      const int t = tile * 128 + q * 32 + lane;
-      uint32_t hw[2][8];                                 // pre-activations of a group of 32 features, requested ahead
-      auto load_h = [&](int g) {
-#pragma unroll
-        for (int x = 0; x < 2; ++x) ld_v8_if(t < a.T && g < ngroups, a.h + (size_t)t * a.N + n0 + g * 32 + 16 * x, hw[x]);
-      };
-      if (EPI == EPI_DGELU) load_h(half);
       if (!warp_wait(acc_full + 8 * buf, (uint32_t)(j >> 1) & 1u)) break;
       tc_fence_after();
+      const int t0 = tile * 128 + q * 32, t = t0 + lane;
       const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16) + buf * 256;
+      bool ok = true;
       for (int g = half; g < ngroups; g += 2) {
         uint32_t v[32];
         __syncwarp();
@@ -543,7 +587,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_empty + 8 * buf);
         }
-        if (t >= a.T) continue;
+        if (t0 >= a.T) continue;                         // whole warps; single lanes past the end go on, what they have is not written
         const float4* bp = reinterpret_cast<const float4*>(bias_ptr + g * 32);
         float f[32];
 #pragma unroll
@@ -554,6 +598,16 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
         }
         const int c = n0 + g * 32;
         if (EPI == EPI_DGELU) {
+          if (staged) {
+            if (!(ok = warp_wait(hbar, hpar))) break;
+            hpar ^= 1u;
+            h_due = false;
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(hw[p >> 1][(p & 1) * 4]), "=r"(hw[p >> 1][(p & 1) * 4 + 1]), "=r"(hw[p >> 1][(p & 1) * 4 + 2]),
+                           "=r"(hw[p >> 1][(p & 1) * 4 + 3]) : "r"(hbuf + lane * 64 + ((p ^ ((lane >> 1) & 3)) << 4)) : "memory");
+            __syncwarp();
+          }
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             float slope[16];
@@ -561,53 +615,70 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
 #pragma unroll
             for (int i = 0; i < 16; ++i) f[16 * x + i] = round_bf16(f[16 * x + i]) * slope[i];
           }
-          if (g + 2 < ngroups) load_h(g + 2);
+          if (g + 2 < ngroups) load_h(tile, g + 2);
+          else load_h(tile + G_x, half);
         }
+        // where the group goes: matrix, column of its rows, row (one lane's of a tile)
+        const int mi = which_matrix(a.Y, c), cm = c - mi * a.Y.per, head = a.Y.L == 0x7fffffff ? 0 : cm >> a.Y.dsh;
+        const int x0 = cm - head * a.Y.d, y0 = a.Y.L == 0x7fffffff ? t : (orow.b * (a.Y.per >> a.Y.dsh) + head) * a.Y.L + orow.l;
         if (Y_BF16) {
+          uint32_t w[2][8];
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[x][i] = pack_bf16(f[16 * x + 2 * i], f[16 * x + 2 * i + 1]);
+          if (staged) put(obuf, w[0], maps.y + mi, x0, y0);
           __nv_bfloat16* dst = tok_col<__nv_bfloat16>(a.Y, c) + orow.off(a.Y);
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
-            uint32_t w[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = pack_bf16(f[16 * x + 2 * i], f[16 * x + 2 * i + 1]);
-            st_v8(dst + 16 * x, w);
+            if (!staged && t < a.T) st_v8(dst + 16 * x, w[x]);
             if (EPI == EPI_GELU) {
               float act[16];
-              look_up<EPI>(tab, w, act);
+              look_up<EPI>(tab, w[x], act);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) w[i] = pack_bf16(act[2 * i], act[2 * i + 1]);
-              st_v8(a.g + (size_t)t * a.N + c + 16 * x, w);
+              for (int i = 0; i < 8; ++i) w[x][i] = pack_bf16(act[2 * i], act[2 * i + 1]);
+              if (!staged && t < a.T) st_v8(a.g + (size_t)t * a.N + c + 16 * x, w[x]);
             }
           }
+          if (EPI == EPI_GELU && staged) put(hbuf, w[0], &maps.g, c, t);
         } else {
           float* dst = tok_col<float>(a.Y, c) + orow.off(a.Y);
+          uint32_t w[32];
           float probe = 0.f;
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            uint32_t w[8];
+          for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(f[i]);
+          if (a.accum && t < a.T) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = __float_as_uint(f[8 * x + i]);
-            if (a.accum) {
+            for (int x = 0; x < 4; ++x) {
               uint32_t o[8];
               ld_v8(dst + 8 * x, o);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) + __uint_as_float(o[i]));
-            }
-            st_v8(dst + 8 * x, w);
-            if (SPLIT == 3) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) probe = fmaf(__uint_as_float(w[i]), 0.f, probe);
+              for (int i = 0; i < 8; ++i) w[8 * x + i] = __float_as_uint(__uint_as_float(w[8 * x + i]) + __uint_as_float(o[i]));
             }
           }
-          if (SPLIT == 3 && !all_finite(probe)) redo_outputs(a, TRANSB, t, c, dst);
+          if (SPLIT == 3) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) probe = fmaf(__uint_as_float(w[i]), 0.f, probe);
+          }
+          const bool redo = SPLIT == 3 && t < a.T && !all_finite(probe);
+          if (staged && !__any_sync(0xffffffffu, redo)) {
+            put(obuf, w, maps.y + mi, x0, y0);
+          } else if (t < a.T) {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) st_v8(dst + 8 * x, *reinterpret_cast<const uint32_t (*)[8]>(w + 8 * x));
+            if (redo) redo_outputs(a, TRANSB, t, c, dst);
+          }
         }
       }
+      if (!ok) break;
       if (half >= ngroups) {                             // nc == 32: the second half of the warps only hands the buffer back
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty + 8 * buf);
       }
     }
+    if (staged && lane == 0) bulk_wait_all();
+    if (EPI == EPI_DGELU && h_due) warp_wait(hbar, hpar);             // after a wait that gave up
   }
   tc_fence_before();
   __syncthreads();
@@ -1273,8 +1344,34 @@ int half_maps(const spion_tokens* t, long long T, CUtensorMap* m) {
   return SPION_OK;
 }
 
+// tiles of 32 tokens by 32 features of the outputs; worth their maps when a CTA has more than one tile (half a microsecond of host time each)
+// Not where bf16 operands split into heads of 32 come through maps: their boxes of 64-byte rows are what the copy engine is busy with (524288
+// tokens, gradient of the input from three gradients 63.5 us, 67.4 staged; output projection 27.0, 27.4, its gradient 25.2, 25.7).
+bool staged_outputs(const spion_tokens* in, const spion_tokens* out, long long T) {
+  auto narrow = [](const spion_tokens* t) { return t->is_bf16 && t->heads > 0 && t->head_dim == 32; };
+  return (T + 127) / 128 > sm_count() && half_boxes(out, T) && !narrow(in) && !(in->is_bf16 && narrow(out));
+}
+size_t staged_bytes(bool gelu, bool y_bf16) { return 8 * (size_t)(gelu ? 2 : 1) * (y_bf16 ? 2048 : 4096); }
+int output_maps(const spion_tokens* t, const GemmArgs& a, LinMaps& maps) {
+  TcState s;
+  int rc = encoder(&s);
+  if (rc) return rc;
+  auto one = [&](CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, bool bf16) -> int {
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * (bf16 ? 2u : 4u)};
+    const cuuint32_t box[2] = {32u, 32u}, estr[2] = {1, 1};
+    return s.encode(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, bf16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? SPION_OK : SPION_ERR_CUDA;
+  };
+  for (int i = 0; i < t->count && !rc; ++i)
+    rc = one(maps.y + i, t->ptr[i], (uint64_t)a.T * (t->heads > 0 ? t->heads : 1), (uint64_t)(t->heads > 0 ? t->head_dim : t->cols), t->is_bf16);
+  if (!rc && a.g) rc = one(&maps.g, a.g, (uint64_t)a.T, (uint64_t)a.N, true);
+  if (!rc && a.h) rc = one(&maps.h, a.h, (uint64_t)a.T, (uint64_t)a.N, true);
+  return rc;
+}
+
 // columns per CTA, accumulators and ring stages of the GEMM; false when the weights do not fit
-bool plan_gemm(int split, bool trans, int K, int N, int* nc, int* nacc, int* stages, size_t* smem, int widest = 256, size_t table = 0) {
+bool plan_gemm(int split, bool trans, int K, int N, int* nc, int* nacc, int* stages, size_t* smem, int widest = 256, size_t table = 0, size_t outs = 0) {
   const int least = split == 1 ? LG_DEPTH + 1 : 2;           // bf16 operands keep LG_DEPTH chunks in flight
   const int nchunks = (K + 63) / 64;
   const int most = split == 3 && nchunks > 1 ? 64 : widest;     // several accumulators of 64 columns keep the fp32 chains short
@@ -1285,7 +1382,7 @@ bool plan_gemm(int split, bool trans, int K, int N, int* nc, int* nacc, int* sta
     const size_t bchunk = trans ? (size_t)((c + 63) / 64) * 8192 : (size_t)c * 128;
     const size_t b = split * ((nchunks * bchunk + 1023) / 1024 * 1024);
     for (int st = split == 1 ? 8 : 4; st >= least; --st) {
-      const size_t total = b + (size_t)st * split * CHUNK + 1024 + 256 + table;
+      const size_t total = b + (size_t)st * split * CHUNK + 1024 + 256 + (outs ? (table + 1023) / 1024 * 1024 + 1024 + outs : table);
       if (total <= SMEM_MAX) { *nc = c; *nacc = split == 3 && nchunks > 1 ? 4 : 1; *stages = st; *smem = total; return true; }
     }
     if (c <= 64) break;
@@ -1319,13 +1416,14 @@ int prepare_wgrad_fp32() {
 }
 
 template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
-int launch_gemm(GemmArgs& a, const spion_tokens* tok, size_t smem, cudaStream_t st) {
+int launch_gemm(GemmArgs& a, const spion_tokens* tok, const spion_tokens* out, size_t smem, cudaStream_t st) {
   auto k = k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>;
   int rc = prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
   if (rc) return rc;
   LinMaps maps;
   a.tma = A_BF16 ? map_form(tok, a.T) : MAP_NONE;
   if (a.tma && (rc = token_maps(tok, a.T, maps.m))) return rc;
+  if (a.staged && (rc = output_maps(out, a, maps))) return rc;
   const int ny = (a.N + a.nc - 1) / a.nc;
   const int sms = sm_count(), tiles = (a.T + 127) / 128;
   if (sms < 1) return SPION_ERR_CUDA;
@@ -1500,14 +1598,20 @@ extern "C" int spion_linear_forward_keep(const spion_tokens* X, const float* con
   a.h = nullptr; a.g = (__nv_bfloat16*)gelu_out; a.x_copy = (__nv_bfloat16*)x_copy; a.w_copy = w_copy;
   size_t smem;
   a.k0 = 0; a.accum = 0; a.parts = 0;
-  if (!plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, gelu_out ? TAB_BYTES : 0)) return SPION_ERR_UNSUPPORTED;
+  auto plan = [&]() {
+    return plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, gelu_out ? TAB_BYTES : 0,
+                     a.staged ? staged_bytes(gelu_out != nullptr, Y->is_bf16) : 0);
+  };
+  a.staged = staged_outputs(X, Y, T);
+  if (a.staged && !plan()) a.staged = 0;                 // wide weights leave no room for the tiles
+  if (!a.staged && !plan()) return SPION_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)cuda_stream;
-  if (fp32) return launch_gemm<3, false, false, EPI_NONE, false>(a, X, smem, st);
+  if (fp32) return launch_gemm<3, false, false, EPI_NONE, false>(a, X, Y, smem, st);
   if (gelu_out)
-    return X->is_bf16 ? launch_gemm<1, true, false, EPI_GELU, true>(a, X, smem, st) : launch_gemm<1, false, false, EPI_GELU, true>(a, X, smem, st);
+    return X->is_bf16 ? launch_gemm<1, true, false, EPI_GELU, true>(a, X, Y, smem, st) : launch_gemm<1, false, false, EPI_GELU, true>(a, X, Y, smem, st);
   if (Y->is_bf16)
-    return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, true>(a, X, smem, st) : launch_gemm<1, false, false, EPI_NONE, true>(a, X, smem, st);
-  return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, false>(a, X, smem, st) : launch_gemm<1, false, false, EPI_NONE, false>(a, X, smem, st);
+    return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, true>(a, X, Y, smem, st) : launch_gemm<1, false, false, EPI_NONE, true>(a, X, Y, smem, st);
+  return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, false>(a, X, Y, smem, st) : launch_gemm<1, false, false, EPI_NONE, false>(a, X, Y, smem, st);
 }
 
 extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* const* W, int nw, int fp32, const void* gelu_in,
@@ -1534,18 +1638,25 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
     for (a.k0 = 0; a.k0 < total; a.k0 += step) {
       a.K = total - a.k0 < step ? total - a.k0 : step;
       a.accum = a.k0 > 0;
-      if (!plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
-      const int rc = launch_gemm<3, false, true, EPI_NONE, false>(a, dY, smem, st);
+      a.staged = total <= step && staged_outputs(dY, dX, T) && plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, 0, staged_bytes(false, false));
+      if (!a.staged && !plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
+      const int rc = launch_gemm<3, false, true, EPI_NONE, false>(a, dY, dX, smem, st);
       if (rc) return rc;
     }
     return SPION_OK;
   }
-  if (!plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, gelu_in ? TAB_BYTES : 0)) return SPION_ERR_UNSUPPORTED;
+  auto plan = [&]() {
+    return plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, gelu_in ? TAB_BYTES : 0,
+                     a.staged ? staged_bytes(gelu_in != nullptr, dX->is_bf16) : 0);
+  };
+  a.staged = staged_outputs(dY, dX, T);
+  if (a.staged && !plan()) a.staged = 0;
+  if (!a.staged && !plan()) return SPION_ERR_UNSUPPORTED;
   if (gelu_in)
-    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_DGELU, true>(a, dY, smem, st) : launch_gemm<1, false, true, EPI_DGELU, true>(a, dY, smem, st);
+    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_DGELU, true>(a, dY, dX, smem, st) : launch_gemm<1, false, true, EPI_DGELU, true>(a, dY, dX, smem, st);
   if (dX->is_bf16)
-    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, true>(a, dY, smem, st) : launch_gemm<1, false, true, EPI_NONE, true>(a, dY, smem, st);
-  return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, false>(a, dY, smem, st) : launch_gemm<1, false, true, EPI_NONE, false>(a, dY, smem, st);
+    return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, true>(a, dY, dX, smem, st) : launch_gemm<1, false, true, EPI_NONE, true>(a, dY, dX, smem, st);
+  return dY->is_bf16 ? launch_gemm<1, true, true, EPI_NONE, false>(a, dY, dX, smem, st) : launch_gemm<1, false, true, EPI_NONE, false>(a, dY, dX, smem, st);
 }
 
 extern "C" long long spion_linear_workspace_floats(long long T, int in_features, int out_features, int fp32) {
