@@ -431,6 +431,11 @@ int spion_linear_forward(const spion_tokens* X, const float* const* W, const flo
 int spion_linear_forward_keep(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
                               const spion_tokens* Y, void* gelu_out, void* x_copy, float* w_copy, long long T, int in_features,
                               int out_features, void* cuda_stream);
+/* The same with spion_expand_keypad beside it (mask [batch, seq_len], pen [batch * heads, seq_len], batch * seq_len = T): the penalties that an
+ * attention call after these projections wants, without a launch of their own.  x_copy, w_copy: as above, NULL in fp32 mode. */
+int spion_linear_forward_keypad(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
+                                const spion_tokens* Y, void* x_copy, float* w_copy, long long T, int in_features, int out_features,
+                                const float* mask, int batch, int heads, int seq_len, float* pen, void* cuda_stream);
 /* dX = dY W, times gelu'(gelu_in) element by element when gelu_in (bf16 [T, in_features]) is not NULL (dX bf16 then).
  * dX fp32: one fp32 sum over all stacked layers.  dX bf16 and nw == 3: the sum of the three layers' gradients, each rounded to
  * bf16 and added in bf16 from the last to the first, which is what separate layers give (out_features / 3 a multiple of 64). */

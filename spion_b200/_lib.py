@@ -94,6 +94,8 @@ SIGNATURES = {
     "spion_softmax_backward_ex": (c_int, [c_void_p] * 4),
     "spion_linear_supported": (c_int, [c_int] * 3),
     "spion_linear_forward": (c_int, [c_void_p] * 3 + [c_int] * 2 + [c_void_p] * 2 + [c_longlong, c_int, c_int, c_void_p]),
+    "spion_linear_forward_keypad": (c_int, [c_void_p] * 3 + [c_int] * 2 + [c_void_p] * 3 + [c_longlong, c_int, c_int, c_void_p, c_int, c_int, c_int,
+                                            c_void_p, c_void_p]),
     "spion_linear_forward_keep": (c_int, [c_void_p] * 3 + [c_int] * 2 + [c_void_p] * 4 + [c_longlong, c_int, c_int, c_void_p]),
     "spion_linear_backward_input": (c_int, [c_void_p] * 2 + [c_int] * 2 + [c_void_p] * 2 + [c_longlong, c_int, c_int, c_void_p]),
     "spion_linear_workspace_floats": (c_longlong, [c_longlong] + [c_int] * 3),

@@ -164,6 +164,9 @@ struct GemmArgs {
   // the weight gradient; the layer of 128 x 2 matrices, L = 4096 went from 1432 to 1458 us.
   __nv_bfloat16* x_copy;    // or null: A as the products use it, [T, K] (fp32 tokens in bf16 mode)
   float* w_copy;            // or null: the stacked W
+  const float* mask;        // pen not null: key-padding mask [T / pen_L, pen_L] -> penalties of pen_heads matrices each
+  float* pen;
+  int pen_heads, pen_L;
 };
 
 // The three parts of an infinity (or of a value that rounds to one in bf16) are not finite themselves, and their products are NaN
@@ -509,6 +512,13 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     const int q = warp & 3, half = (warp - LG_LOADERS - 1) >> 2;
     const int ngroups = nc >> 5;
     int j = 0;
+    if (!TRANSB && a.pen) {                              // spion_expand_keypad, in the time that the first tile takes
+      const int n = a.T * a.pen_heads, all = (int)(gridDim.x * gridDim.y) * 256;
+      for (int i = ((int)(blockIdx.y * gridDim.x + blockIdx.x)) * 256 + tid - 32 * (LG_LOADERS + 1); i < n; i += all) {
+        const int bh = i / a.pen_L;
+        a.pen[i] = 1e6f * (1.0f - a.mask[(bh / a.pen_heads) * a.pen_L + (i - bh * a.pen_L)]);
+      }
+    }
     RowIt orow;
     const int ostep = G_x * 128, ostep_b = ostep / a.Y.L, ostep_l = ostep - ostep_b * a.Y.L;
     orow.init(a.Y, min(a.T - 1, (int)blockIdx.x * 128 + q * 32 + lane));
@@ -1580,9 +1590,9 @@ extern "C" int spion_linear_forward(const spion_tokens* X, const float* const* W
   return spion_linear_forward_keep(X, W, bias, nw, fp32, Y, gelu_out, nullptr, nullptr, T, in_features, out_features, cuda_stream);
 }
 
-extern "C" int spion_linear_forward_keep(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
-                                         const spion_tokens* Y, void* gelu_out, void* x_copy, float* w_copy, long long T,
-                                         int in_features, int out_features, void* cuda_stream) {
+static int forward(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32, const spion_tokens* Y, void* gelu_out,
+                   void* x_copy, float* w_copy, long long T, int in_features, int out_features, const float* mask, int heads, int seq_len, float* pen,
+                   void* cuda_stream) {
   if (!mat_ok(X) || !mat_ok(Y) || !W || nw < 1 || nw > 3 || T < 1 || T > 0x7fffffffLL - 256) return SPION_ERR_ARG;
   if (X->cols * X->count != in_features || Y->cols * Y->count != out_features || out_features % nw) return SPION_ERR_ARG;
   if (fp32 && (X->is_bf16 || Y->is_bf16 || gelu_out)) return SPION_ERR_UNSUPPORTED;
@@ -1596,6 +1606,7 @@ extern "C" int spion_linear_forward_keep(const spion_tokens* X, const float* con
   for (int i = 0; i < nw; ++i) if (!a.W[i] || ((uintptr_t)a.W[i] & 15)) return SPION_ERR_ARG;
   a.T = (int)T; a.K = in_features; a.N = out_features;
   a.h = nullptr; a.g = (__nv_bfloat16*)gelu_out; a.x_copy = (__nv_bfloat16*)x_copy; a.w_copy = w_copy;
+  a.mask = mask; a.pen = pen; a.pen_heads = heads; a.pen_L = seq_len;
   size_t smem;
   a.k0 = 0; a.accum = 0; a.parts = 0;
   auto plan = [&]() {
@@ -1614,6 +1625,20 @@ extern "C" int spion_linear_forward_keep(const spion_tokens* X, const float* con
   return X->is_bf16 ? launch_gemm<1, true, false, EPI_NONE, false>(a, X, Y, smem, st) : launch_gemm<1, false, false, EPI_NONE, false>(a, X, Y, smem, st);
 }
 
+extern "C" int spion_linear_forward_keep(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
+                                         const spion_tokens* Y, void* gelu_out, void* x_copy, float* w_copy, long long T,
+                                         int in_features, int out_features, void* cuda_stream) {
+  return forward(X, W, bias, nw, fp32, Y, gelu_out, x_copy, w_copy, T, in_features, out_features, nullptr, 0, 0, nullptr, cuda_stream);
+}
+
+extern "C" int spion_linear_forward_keypad(const spion_tokens* X, const float* const* W, const float* const* bias, int nw, int fp32,
+                                           const spion_tokens* Y, void* x_copy, float* w_copy, long long T, int in_features, int out_features,
+                                           const float* mask, int batch, int heads, int seq_len, float* pen, void* cuda_stream) {
+  if (!mask || !pen || batch < 1 || heads < 1 || seq_len < 1) return SPION_ERR_ARG;
+  if ((long long)batch * seq_len != T || T * heads > 0x7fffffffLL) return SPION_ERR_SHAPE;
+  return forward(X, W, bias, nw, fp32, Y, nullptr, x_copy, w_copy, T, in_features, out_features, mask, heads, seq_len, pen, cuda_stream);
+}
+
 extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* const* W, int nw, int fp32, const void* gelu_in,
                                            const spion_tokens* dX, long long T, int in_features, int out_features,
                                            void* cuda_stream) {
@@ -1627,7 +1652,7 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
   for (int i = 0; i < 3; ++i) { a.W[i] = i < nw ? W[i] : nullptr; a.bias[i] = nullptr; }
   for (int i = 0; i < nw; ++i) if (!a.W[i] || ((uintptr_t)a.W[i] & 15)) return SPION_ERR_ARG;
   a.T = (int)T; a.K = out_features; a.N = in_features;
-  a.h = (const __nv_bfloat16*)gelu_in; a.g = nullptr; a.x_copy = nullptr; a.w_copy = nullptr;
+  a.h = (const __nv_bfloat16*)gelu_in; a.g = nullptr; a.x_copy = nullptr; a.w_copy = nullptr; a.mask = nullptr; a.pen = nullptr;
   size_t smem;
   a.k0 = 0; a.accum = 0;
   a.parts = !fp32 && dX->is_bf16 && nw == 3 ? a.wper / 64 : 0;

@@ -127,6 +127,14 @@ void linear_forward(const spion_tokens& X, const Weights& w, bool fp32, const sp
   check(spion_linear_forward_keep(&X, W, b, w.n(), fp32, &Y, gelu_out, p(kept.x), kept.w_to, T, w.in(), w.out(), st),
         "spion_linear_forward_keep");
 }
+// the projections of a layer with padded keys, and the penalties of its attention
+void linear_forward_keypad(const spion_tokens& X, const Weights& w, bool fp32, const spion_tokens& Y, int64_t T, void* st, const Kept& kept,
+                           const Tensor& mask, int B, int H, int L, const Tensor& pen) {
+  const float *W[3], *b[3];
+  for (int i = 0; i < w.n(); ++i) { W[i] = pf(w.W[i]); b[i] = pf(w.b[i]); }
+  check(spion_linear_forward_keypad(&X, W, b, w.n(), fp32, &Y, p(kept.x), kept.w_to, T, w.in(), w.out(), pf(mask), B, H, L, (float*)p(pen), st),
+        "spion_linear_forward_keypad");
+}
 void linear_backward_input(const spion_tokens& dY, const Weights& w, bool fp32, const void* gelu_in, const spion_tokens& dX, int64_t T, void* st) {
   const float* W[3];
   for (int i = 0; i < w.n(); ++i) W[i] = w.at(i);
@@ -253,14 +261,17 @@ void check_operand(const Context& c, const Tensor& t, const char* name) {
     throw Failure(std::string(name) + " is on " + t.device().str() + ", the module's context is on cuda:" + std::to_string(c.device));
 }
 
-// key-padding mask [B, L] of 1 / 0 -> penalty per (b,h) matrix [BH, L].  The drop-in modules expand a mask of one sequence
-// or of one key.
-Tensor penalty(const Context& c, const Tensor& mask, const Tensor& like, void* st) {
+// key-padding mask [B, L] of 1 / 0 as floats.  The drop-in modules expand a mask of one sequence or of one key.
+Tensor key_mask(const Context& c, const Tensor& mask, const Tensor& like) {
   auto fits = [&](int i, int64_t n) { return mask.size(i) == n || (c.mode != NATIVE && mask.size(i) == 1); };
   if (!mask.defined() || mask.dim() != 2 || !fits(0, c.B) || !fits(1, c.L))
     throw Failure("key-padding mask must have shape (" + std::to_string(c.B) + ", " + std::to_string(c.L) + ")");
-  Tensor m = mask.to(like.device(), at::kFloat).expand({c.B, c.L}).contiguous();
-  Tensor pen = at::empty({c.B, c.H, c.L}, like.options().dtype(at::kFloat));
+  return mask.to(like.device(), at::kFloat).expand({c.B, c.L}).contiguous();
+}
+Tensor empty_penalty(const Context& c, const Tensor& like) { return at::empty({c.B, c.H, c.L}, like.options().dtype(at::kFloat)); }
+// ... -> penalty per (b,h) matrix [BH, L]
+Tensor penalty(const Context& c, const Tensor& mask, const Tensor& like, void* st) {
+  Tensor m = key_mask(c, mask, like), pen = empty_penalty(c, like);
   check(spion_expand_keypad(pf(m), (int)c.B, (int)c.H, (int)c.L, (float*)pen.data_ptr(), st), "spion_expand_keypad");
   return pen;
 }
@@ -748,7 +759,9 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
     Tensor X = x.detach();
     if (!X.is_contiguous() || !aligned32(X)) X = X.contiguous().clone();
     const auto opt = X.options().dtype(c->type());
-    if (c->keypad) a.pen = penalty(*c, mask.has_value() ? *mask : Tensor(), X, st);
+    Tensor keys;
+    if (c->keypad && (noise || T * H > 0x7fffffffLL)) a.pen = penalty(*c, mask.has_value() ? *mask : Tensor(), X, st);
+    else if (c->keypad) { keys = key_mask(*c, mask.has_value() ? *mask : Tensor(), X); a.pen = empty_penalty(*c, X); }
     // bf16 tokens: operands stay [B, L, H, d], whose rows the weight gradients' matrix products read
     a.heads = X.scalar_type() == at::kBFloat16 && c->fused ? H : 0;
     auto form = [&](const std::vector<Tensor>& ts) { return a.heads ? tok(ts, H * d) : tok_heads(ts, H, d, L); };
@@ -763,7 +776,9 @@ Result attention_layer(const ContextPtr& c, const Tensor& x, const optional<Tens
       const Tensor like = at::empty({0}, opt);
       a.q = empty_operand(*c, a.heads, like); a.k = empty_operand(*c, a.heads, like); a.v = empty_operand(*c, a.heads, like);
       kept_in = Kept(need, fp32, X, qkv, (float*)p(kept_w));
-      linear_forward(tok({X}, (int)X.size(2)), qkv, fp32, form({a.q, a.k, a.v}), nullptr, T, st, kept_in);
+      const spion_tokens in = tok({X}, (int)X.size(2)), operands = form({a.q, a.k, a.v});
+      if (keys.defined()) linear_forward_keypad(in, qkv, fp32, operands, T, st, kept_in, keys, (int)c->B, H, L, a.pen);
+      else linear_forward(in, qkv, fp32, operands, nullptr, T, st, kept_in);
     }
     attn_forward(*c, a, need, st);
     out = at::empty({c->B, c->L, ff.out()}, opt);

@@ -169,6 +169,27 @@ def test_gelu_on_bf16_tokens(T, K, N):
     assert _rel(dX, _bf(_bf(dY.double() @ _bf(V)) * slope)) < 1e-3
 
 
+@pytest.mark.parametrize("B,L,heads,fp32", [(1, 1, 1, 0), (3, 127, 2, 0), (2, 4096, 3, 1), (150, 160, 2, 0), (7, 33, 8, 1)])
+def test_projections_with_the_penalties_of_padded_keys(B, L, heads, fp32):
+    """The penalties that the projections' kernel writes are spion_expand_keypad's, and its outputs those without them."""
+    P = ctypes.c_void_p
+    st = P(torch.cuda.current_stream().cuda_stream)
+    T, K, N = B * L, 64, 96
+    X, W, b = torch.randn(T, K, device="cuda"), torch.randn(N, K, device="cuda"), torch.randn(N, device="cuda")
+    yt = torch.float32 if fp32 else torch.bfloat16
+    Y, Z = (torch.full((T, N), 7.0, dtype=yt, device="cuda") for _ in range(2))
+    mask = (torch.rand(B, L, device="cuda") < 0.7).float()
+    pen, want = (torch.full((B * heads, L), -1.0, device="cuda") for _ in range(2))
+    one, ref = lambda t: (P * 3)(t.data_ptr(), None, None), ctypes.byref
+    check(lib.spion_linear_forward_keypad(ref(_tokens([X])), one(W), one(b), 1, fp32, ref(_tokens([Y])), None, None, T, K, N, P(mask.data_ptr()), B, heads, L,
+                                          P(pen.data_ptr()), st))
+    check(lib.spion_linear_forward(ref(_tokens([X])), one(W), one(b), 1, fp32, ref(_tokens([Z])), None, T, K, N, st))
+    check(lib.spion_expand_keypad(P(mask.data_ptr()), B, heads, L, P(want.data_ptr()), st))
+    assert torch.equal(pen, want) and torch.equal(Y, Z)
+    assert lib.spion_linear_forward_keypad(ref(_tokens([X])), one(W), one(b), 1, fp32, ref(_tokens([Y])), None, None, T, K, N, P(mask.data_ptr()), B + 1, heads, L,
+                                           P(pen.data_ptr()), st) != 0
+
+
 @pytest.mark.parametrize("T,K,N", [(19000, 64, 128), (20001, 32, 96), (300, 64, 64)])
 def test_gelu_of_every_bf16_number(T, K, N):
     """Activation and its derivative by table, inside and outside of its range (subnormals, infinities and NaN too), the outputs through tiles in
