@@ -1,5 +1,6 @@
 // Block-sparse attention on masks of 32 x 32 blocks, on the blocks themselves (sm_100a, bf16, head_dim 64):
-// forward and the recompute backward without ever forming an unselected block.
+// the recompute backward without ever forming an unselected block, and the forward of the full mask and of small calls (others:
+// tc_fwd_stream.cu).
 //
 // tcgen05.mma needs M = 64 or 128 rows, a 32-wide block row has 32.  The kernels therefore gather up to
 // four selected 32-row tiles of the OTHER operand into one 128-row operand and, where the 32 rows of the

@@ -624,6 +624,66 @@ __global__ void k_line_recs(const int32_t* __restrict__ ptr, const int32_t* __re
   }
 }
 
+// 32-wide masks: super rows (two block rows) from the longest to the shortest, with the 32-wide blocks that one of their rows selects in ascending order, two
+// to a tile, two tiles to a pair.  rec[x] = {super row, index of its first pair, pairs, tiles};  pair[p] = {block | block << 16 of tile 0, of tile 1,
+// selected quarters of tile 0 (2 * row + block), of tile 1}.  A tile without a second block has its first one again, nothing of it selected.  One CTA.
+__global__ void __launch_bounds__(512) k_gather_recs(const uint8_t* __restrict__ mat, int nb, int4* __restrict__ rec, int4* __restrict__ pair) {
+  __shared__ int s_n[SPION_MAX_NB / 2], s_order[SPION_MAX_NB / 2], s_first[SPION_MAX_NB / 2];
+  const int lines = nb >> 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  for (int x = warp; x < lines; x += warps) {
+    const uint8_t* m = mat + (size_t)2 * x * nb;
+    int n = 0;
+    for (int c0 = 0; c0 < nb; c0 += 32) {
+      const int c = c0 + lane;
+      n += __popc(__ballot_sync(0xffffffffu, c < nb && (m[c] | m[nb + c]) != 0));
+    }
+    if (lane == 0) s_n[x] = (n + 1) >> 1;
+  }
+  __syncthreads();
+  for (int x = threadIdx.x; x < lines; x += blockDim.x) {
+    const int n = s_n[x];
+    int rank = 0;
+    for (int o = 0; o < lines; ++o) rank += (s_n[o] > n) || (s_n[o] == n && o < x);
+    s_order[rank] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int acc = 0;
+    for (int x = 0; x < lines; ++x) { s_first[x] = acc; acc += (s_n[s_order[x]] + 1) >> 1; }
+  }
+  __syncthreads();
+  for (int x = warp; x < lines; x += warps) {
+    const int line = s_order[x], tiles = s_n[line], np = (tiles + 1) >> 1;
+    int4* out = pair + s_first[x];
+    if (lane == 0) rec[x] = make_int4(line, s_first[x], np, tiles);
+    const uint8_t* m = mat + (size_t)2 * line * nb;
+    int n = 0;
+    for (int c0 = 0; c0 < nb; c0 += 32) {
+      const int c = c0 + lane;
+      const int r0 = c < nb && m[c] != 0, r1 = c < nb && m[nb + c] != 0;
+      const uint32_t b = __ballot_sync(0xffffffffu, r0 | r1);
+      // the blocks of this step, an even one with the one after it: of this step, of the next (lane 31's turn then), or none
+      if (r0 | r1) {
+        const int e = n + __popc(b & ((1u << lane) - 1u)), p = e >> 2, t = (e >> 1) & 1, half = e & 1;
+        uint16_t* ids = reinterpret_cast<uint16_t*>(out + p) + 2 * t + half;
+        uint8_t* sub = reinterpret_cast<uint8_t*>(out + p) + 8 + 4 * t;
+        *ids = (uint16_t)c;
+        sub[1 + half] = (uint8_t)((r0 << half) | (r1 << (2 + half)));
+      }
+      n += __popc(b);
+    }
+    __syncwarp();
+    for (int t = lane; t < 2 * np; t += 32) {             // quarters of both blocks together; what a tile does not have
+      uint16_t* ids = reinterpret_cast<uint16_t*>(out + (t >> 1)) + 2 * (t & 1);
+      uint8_t* sub = reinterpret_cast<uint8_t*>(out + (t >> 1)) + 8 + 4 * (t & 1);
+      if (2 * t + 1 >= n) ids[1] = 2 * t < n ? ids[0] : 0;
+      if (2 * t >= n) ids[0] = 0;
+      const int q = (2 * t < n ? sub[1] : 0) | (2 * t + 1 < n ? sub[2] : 0);
+      *reinterpret_cast<int*>(sub) = q;
+    }
+  }
+}
+
 }  // namespace
 
 namespace tc {
@@ -680,6 +740,19 @@ int stream_prepare(spion_ctx* c, TcState* s) {
     s->line_pair_cap = 0;
     if (device_alloc((void**)&s->line_pair, 2 * (size_t)vw.nnzb * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
     s->line_pair_cap = (size_t)vw.nnzb;
+  }
+  if (s->super) {                                                   // at most one pair per block
+    if (!s->gather_rec && device_alloc((void**)&s->gather_rec, (SPION_MAX_NB / 2) * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
+    if ((size_t)c->nnzb > s->gather_cap) {
+      device_free(s->gather_pair);
+      s->gather_pair = nullptr;
+      s->gather_cap = 0;
+      if (device_alloc((void**)&s->gather_pair, (size_t)c->nnzb * sizeof(int4)) != SPION_OK) return SPION_ERR_ALLOC;
+      s->gather_cap = (size_t)c->nnzb;
+    }
+    k_gather_recs<<<1, 512, 0, c->stream>>>(c->mat, c->nb, s->gather_rec, s->gather_pair);
+    SPION_LAUNCH_CHECK();
+    c->launches += 1;
   }
   k_line_recs<<<1, 512, 0, c->stream>>>(vw.col_ptr, vw.row_idx, vw.csc_pos, vw.nb, s->line_rec, s->line_pair);
   SPION_LAUNCH_CHECK();

@@ -835,6 +835,8 @@ void tc_engine_release(spion_ctx* c) {
   device_free(s->col_order);
   device_free(s->line_rec);
   device_free(s->line_pair);
+  device_free(s->gather_rec);
+  device_free(s->gather_pair);
   delete s;
   c->tc = nullptr;
 }
@@ -845,7 +847,13 @@ static int forward_any(spion_ctx* c, const void* Q, const void* K, const void* V
   TcState* s = (TcState*)c->tc;
   if (!s) return SPION_ERR_STATE;
   if (c->nnzb == 0) return SPION_ERR_SHAPE;
-  if (s->b32 && s->b32_use && !P_user) return b32_forward(c, s, Q, K, V, keypad, O, lse ? lse : s->lse_ws);
+  if (s->b32 && s->b32_use && !P_user) {
+    // The mask's own blocks, a block row per CTA: the full mask, which keeps its order of sums (see tc_fwd_exact.cu), and calls whose rows are all
+    // resident at once (2 matrices, L = 4096, 5 % 10.4 us, two rows at a time 12.4; 1 matrix, 10 % 14.6, 16.5; 4 matrices, 5 % 16.5, 13.3).
+    float* l = lse ? lse : s->lse_ws;
+    const bool own = c->nnzb == c->nb * c->nb || (long long)c->BH * c->nb <= (long long)s->sms * s->b32_ctas[0];
+    return own ? b32_forward(c, s, Q, K, V, keypad, O, l) : stream_forward(c, s, Q, K, V, keypad, O, l);
+  }
   if (P_user && s->super) {
     int rc = ensure_super_ws(c, s);
     if (rc) return rc;

@@ -603,7 +603,7 @@ static int fwd_launch(spion_ctx* c, TcState* s, const void* Q, const void* K, co
   if (s->n_long == 0) {
     if ((rc = pipe_forward(c, s, mq, mk, mv, mp, P64 != nullptr, stat, keypad, O, lse, 0))) return rc;
   } else if (!P64 && !stat) {
-    rc = c->nnzb == c->nb * c->nb ? exact_forward(c, s, mq, mk, mv, keypad, O, lse) : stream_forward(c, s, mq, mk, mv, keypad, O, lse);
+    rc = c->nnzb == c->nb * c->nb ? exact_forward(c, s, mq, mk, mv, keypad, O, lse) : stream_forward(c, s, Q, K, V, keypad, O, lse);
     if (rc) return rc;
   } else {
     const long long total = (long long)c->BH * vw.nb, cap = (long long)s->sms * s->fwd_ctas;

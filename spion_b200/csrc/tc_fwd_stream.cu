@@ -21,6 +21,13 @@
 // Measured, forward alone, first form (one unit per CTA, two passes over a row), P in shared memory, now: 64 matrices, L = 16384, d 64, 5 % 847,
 // 368, 345 us, d 32 -, 312, 292; 256 matrices, L = 4096, d 32, 10 %, padded keys 585, 200, 185; 64 matrices, L = 4096, d 64, 5 % 62, 43.5, 43.
 //
+// SUB: masks of 32-wide blocks.  A unit is two block rows, a tile two key blocks of 32 that one of them selects, wherever they lie (two copies
+// of 32 rows each); quarters that are not selected are left out of the sums.  Random masks fill half of such tiles, a third to a quarter of tiles of 64 keys in
+// a row.  Us, forward, before (head_dim 64 the mask's own blocks in transposed products, k_b32; 32 such tiles) and now: 64 matrices, L = 4096, d 64, 2 %
+// 45, 39; 5 % 122, 70; 10 % 208, 119; 30 % 528, 280; 16 matrices, 5 %, padded keys 40, 29; d 32, 5 % 74, 52; 32 matrices, 15 %, padded keys 107, 73.
+// At head_dim 64 the reference follows every new maximum, as the kernel before had it: the largest P of a row is 1, which bf16 has without rounding.  Moved
+// by 2^8 only, O is 3 % further from fp64 (2.26e-3 instead of 2.14e-3, before 2.18e-3) and the first three figures 39, 63, 101.
+//
 // Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
 #include "tc_stream.cuh"
 
@@ -53,8 +60,7 @@ struct FsArgs {
   __nv_bfloat16* O;
   float* lse;
   const float* keypad;
-  const int4 *rec, *pair;                                         // block rows and their pairs (k_line_recs)
-  const uint8_t* submask;
+  const int4 *rec, *pair;                                         // block rows and their pairs (k_line_recs; SUB: k_gather_recs)
   int L, BH, nb, heads, by_rank;
   float scale, floor_v;
   int* status;
@@ -143,30 +149,39 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
       const bool two = w.cnt() == 2, with_q = w.k == 0;
       const OpPos pos = op_pos(w.bh, a.L, a.heads, D);
       const int bh = w.bh, line = w.cur.x;
+      // SUB: lanes 0 to 3 copy a quarter of a pair's tiles each
+      const int piece = (lane & 2 ? pr.y : pr.x) >> ((lane & 1) * 16) & 0xffff;
+      const bool mine = SUB && lane < (two ? 4 : 2);
       if (elect_one()) {
         ring[j & 7] = make_int4((two ? PR_TWO : 0) | (with_q ? PR_FIRST : 0), 0, 0, 0);
         mbar_expect_tx(kb, ((two ? 2 : 1) + (with_q ? 1 : 0)) * T::BYTES);
         const uint32_t dst = gb + C::O_K + (j % KB) * 2 * T::BYTES;
-        tma_load_2d(dst, &tmK, kb, pos.x0, pos.row0 + pr.x * BS);
-        if (two) tma_load_2d(dst + T::BYTES, &tmK, kb, pos.x0, pos.row0 + pr.y * BS);
+        if (!SUB) {
+          tma_load_2d(dst, &tmK, kb, pos.x0, pos.row0 + pr.x * BS);
+          if (two) tma_load_2d(dst + T::BYTES, &tmK, kb, pos.x0, pos.row0 + pr.y * BS);
+        }
         // the Q buffer was read by the unit before the last, whose last pair is not after the one k_free was for
         if (with_q) tma_load_2d(gb + C::O_Q + (units & 1) * T::BYTES, &tmQ, kb, pos.x0, pos.row0 + line * BS);
       }
       __syncwarp();
+      if (mine) tma_load_2d(gb + C::O_K + (j % KB) * 2 * T::BYTES + lane * (T::BYTES / 2), &tmK, kb, pos.x0, pos.row0 + piece * 32);
       if (w.last()) ++units;
       w.next();
       if (w.valid()) nx = a.pair[w.cur.y + w.k];
       if (KP || SUB) {
-        const int e = lane >> 4, o = e ? (two ? pr.y : -1) : pr.x;
+        const int e = lane >> 4, o = e ? pr.y : pr.x;
+        const bool here = !e || two;
         uint32_t mixed = 0u;
         float pen = 0.f, pen1 = 0.f;
         if (KP) {
           Pen4 p = {};
-          if (o >= 0) pen_load(p, a.keypad + (size_t)bh * a.L + o * BS);
+          const float* kp = a.keypad + (size_t)bh * a.L;
+          if (here && SUB) pen_load(p, kp + (o & 0xffff) * 32, kp + (o >> 16) * 32);
+          else if (here) pen_load(p, kp + o * BS);
           pen = pen_of(p, mixed) * LOG2E;
           pen1 = __shfl_sync(0xffffffffu, pen, 16);
         }
-        const int sub_l = SUB && o >= 0 ? a.submask[e ? pr.w : pr.z] : 0;
+        const int sub_l = SUB && here ? (e ? pr.w : pr.z) : 0;
         const int s1 = SUB ? __shfl_sync(0xffffffffu, sub_l, 16) : 0xff;
         if (lane == 0) {
           int* x = info + 8 * (j & 3);
@@ -181,10 +196,13 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
       if (elect_one()) {
         const uint32_t vb = v_full + 8 * (j & 1), dst = gb + C::O_V + (j & 1) * 2 * T::BYTES;
         mbar_expect_tx(vb, (two ? 2 : 1) * T::BYTES);
-        tma_load_2d(dst, &tmV, vb, pos.x0, pos.row0 + pr.x * BS);
-        if (two) tma_load_2d(dst + T::BYTES, &tmV, vb, pos.x0, pos.row0 + pr.y * BS);
+        if (!SUB) {
+          tma_load_2d(dst, &tmV, vb, pos.x0, pos.row0 + pr.x * BS);
+          if (two) tma_load_2d(dst + T::BYTES, &tmV, vb, pos.x0, pos.row0 + pr.y * BS);
+        }
       }
       __syncwarp();
+      if (mine) tma_load_2d(gb + C::O_V + (j & 1) * 2 * T::BYTES + lane * (T::BYTES / 2), &tmV, v_full + 8 * (j & 1), pos.x0, pos.row0 + piece * 32);
       pr = nx;
     }
   } else if (warp >= 4 * NG) {
@@ -239,6 +257,7 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
     const int q = warp & 3, hf = lane >> 4, row = q * 16 + (lane & 15);
     const uint32_t lS = tS + ((uint32_t)(q * 32) << 16), lP = lS + C::T_P, lO = lS + C::T_O;
     const float sc2 = a.scale * LOG2E, floor2 = a.floor_v * LOG2E, inv_scale = 1.0f / a.scale;
+    constexpr float move_by = SUB && D == 64 ? 0.f : MOVE;
     bool ok = true;
     // The finished unit whose rows are still in tensor memory: the products of first entries in lanes 0-15 of every quadrant, of second ones
     // in lanes 16-31.  Lane l gives half of its columns to lane l ^ 16 and takes the other half's from there.
@@ -290,7 +309,7 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
       const int np = u.pairs();
       for (int k = 0; k < np && ok; ++k, ++j) {
         const bool mine = 2 * k + hf < n;
-        const float* kp = nullptr;
+        const float *kp = nullptr, *kp_hi = nullptr;
         float pen = 0.f;
         bool live0 = mine, live1 = mine;
         if (KP || SUB) {
@@ -300,7 +319,10 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
           if (KP) {
             const bool mixed = (f >> hf) & 1;
             pen = mixed ? 0.f : __int_as_float(x[4 + hf]);
-            if (mixed) kp = kpu + x[1 + hf] * BS;
+            if (mixed) {
+              kp = SUB ? kpu + (x[1 + hf] & 0xffff) * 32 : kpu + x[1 + hf] * BS;
+              kp_hi = SUB ? kpu + (x[1 + hf] >> 16) * 32 : kp + 32;
+            }
           }
           if (SUB) {
             const int bits = (f >> (8 + 8 * hf + (q >> 1) * 2)) & 3;
@@ -321,7 +343,7 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
         if (lane == 0) mbar_arrive(s_free);
         if (KP && kp) {
           take_penalty(v0, kp, inv_scale);
-          take_penalty(v1, kp + 32, inv_scale);
+          take_penalty(v1, kp_hi, inv_scale);
         }
         float cm = -INFINITY;
         {                                                         // the scale is positive: compare raw scores
@@ -340,8 +362,8 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
         mx = fmaxf(mx, cm);
         if (k == 0) {
           m = mx;
-        } else if (__any_sync(0xffffffffu, mx > m + MOVE)) {      // rare: move the reference, rescale what has been summed
-          const float m_new = mx > m + MOVE ? mx : m, f = exp2f(m - m_new);
+        } else if (__any_sync(0xffffffffu, mx > m + move_by)) {      // rare: move the reference, rescale what has been summed
+          const float m_new = mx > m + move_by ? mx : m, f = exp2f(m - m_new);
           l *= f;
           m = m_new;
           if (!wait_all(pv_done, (uint32_t)(j - 1), ERR_MMA2_WAIT)) { ok = false; break; }
@@ -430,13 +452,16 @@ static int fs_launch(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUte
 }
 
 template <int D>
-static int fs_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad,
-                      void* O, float* lse) {
+static int fs_forward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const float* keypad, void* O, float* lse) {
   const TcView vw = tc_view(c, s);
+  const int rows = vw.submask ? 32 : BS;
+  CUtensorMap mq, mk, mv;
+  int rc;
+  if ((rc = make_operand_map(c, s, &mq, Q, D)) || (rc = make_operand_map(c, s, &mk, K, D, rows)) || (rc = make_operand_map(c, s, &mv, V, D, rows))) return rc;
   FsArgs a;
   a.O = (__nv_bfloat16*)O; a.lse = lse; a.keypad = keypad;
-  a.rec = s->line_rec + SPION_MAX_NB; a.pair = s->line_pair + s->line_pair_cap;
-  a.submask = vw.submask;
+  a.rec = vw.submask ? s->gather_rec : s->line_rec + SPION_MAX_NB;
+  a.pair = vw.submask ? s->gather_pair : s->line_pair + s->line_pair_cap;
   a.L = c->L; a.BH = c->BH; a.nb = vw.nb; a.heads = c->heads; a.by_rank = order_by_rank(c);
   a.scale = c->scale; a.floor_v = keypad ? 0.0f : -100.0f; a.status = c->status_dev;
   if (keypad) return vw.submask ? fs_launch<D, true, true>(c, s, mq, mk, mv, a) : fs_launch<D, true, false>(c, s, mq, mk, mv, a);
@@ -451,9 +476,8 @@ static int fs_attrs(const spion_ctx* c) {
 }
 int stream_forward_set_attrs(const spion_ctx* c) { return c->d == 64 ? fs_attrs<64>(c) : fs_attrs<32>(c); }
 
-int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
-                   float* lse) {
-  return c->d == 64 ? fs_forward<64>(c, s, mq, mk, mv, keypad, O, lse) : fs_forward<32>(c, s, mq, mk, mv, keypad, O, lse);
+int stream_forward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const float* keypad, void* O, float* lse) {
+  return c->d == 64 ? fs_forward<64>(c, s, Q, K, V, keypad, O, lse) : fs_forward<32>(c, s, Q, K, V, keypad, O, lse);
 }
 
 }  // namespace tc

@@ -98,10 +98,11 @@ __device__ __forceinline__ void take_penalty(uint32_t (&s)[32], const float* kp,
 // L = 4096, d 32, 10 %, 25 % of the keys padded: forward, columns, rows 224, 335, 298 us with a penalty per key of every padded block).
 // Half a warp, four keys per lane: pen_load is requested early, pen_of gives the block's value and whether a key differs from it.
 struct Pen4 { float x[4]; };
-__device__ __forceinline__ void pen_load(Pen4& p, const float* kp) {
+__device__ __forceinline__ void pen_load(Pen4& p, const float* lo, const float* hi) {       // of the first and the second 32 keys
 #pragma unroll
-  for (int i = 0; i < 4; ++i) p.x[i] = kp[(threadIdx.x & 15) + 16 * i];
+  for (int i = 0; i < 4; ++i) p.x[i] = (i < 2 ? lo : hi)[(threadIdx.x & 15) + 16 * (i & 1)];
 }
+__device__ __forceinline__ void pen_load(Pen4& p, const float* kp) { pen_load(p, kp, kp + 32); }
 __device__ __forceinline__ float pen_of(const Pen4& p, uint32_t& mixed) {      // whole warp; mixed: bit 0, lanes 0-15, bit 1, lanes 16-31
   const float first = __shfl_sync(0xffffffffu, p.x[0], threadIdx.x & 16);
   bool other = false;

@@ -168,6 +168,9 @@ struct TcState {
   int4* line_rec = nullptr;     // {line, first pair, pairs, entries}, the longest lines first
   int4* line_pair = nullptr;    // {other line of entry 0, of entry 1 (-1: none), CSR block ids}; the rows' pairs from line_pair_cap on
   size_t line_pair_cap = 0;
+  // 32-wide masks: super rows (64 queries) with the 32-wide key blocks that either of their rows selects, two to a tile (k_gather_recs)
+  int4 *gather_rec = nullptr, *gather_pair = nullptr;
+  size_t gather_cap = 0;
   int4* row_info = nullptr;     // per block row: {row_ptr, blocks, col0 | col1 << 16, col2 | col3 << 16}: one load instead of two dependent ones
   // 32-wide masks run on 64-wide super-blocks: derived structure + which 32x32 quarters are selected
   bool super = false;
@@ -256,9 +259,9 @@ inline int allow_smem(int device, size_t bytes) {
 
 // Map over one dense operand (Q, K, V, dO): [BH*L, D] rows, or [B*L, H*D] rows with a [64 x D] box at
 // column h*D when the context's operands are in the merged-head form.
-inline int make_operand_map(const spion_ctx* c, TcState* s, CUtensorMap* m, const void* base, int D) {
-  if (c->heads == 0) return make_map(s, m, base, (uint64_t)c->BH * c->L, (uint32_t)D, (uint32_t)D, BS);
-  return make_map(s, m, base, (uint64_t)(c->BH / c->heads) * c->L, (uint32_t)(c->heads * D), (uint32_t)D, BS);
+inline int make_operand_map(const spion_ctx* c, TcState* s, CUtensorMap* m, const void* base, int D, int box_rows = BS) {
+  if (c->heads == 0) return make_map(s, m, base, (uint64_t)c->BH * c->L, (uint32_t)D, (uint32_t)D, box_rows);
+  return make_map(s, m, base, (uint64_t)(c->BH / c->heads) * c->L, (uint32_t)(c->heads * D), (uint32_t)D, box_rows);
 }
 
 // tc_bwd_stream.cu
@@ -273,8 +276,7 @@ int recompute_mean_map(spion_ctx* c, TcState* s, const void* Q, const void* K, c
 
 // tc_fwd_stream.cu: forward without stored probabilities
 int stream_forward_set_attrs(const spion_ctx* c);
-int stream_forward(spion_ctx* c, TcState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const float* keypad, void* O,
-                   float* lse);
+int stream_forward(spion_ctx* c, TcState* s, const void* Q, const void* K, const void* V, const float* keypad, void* O, float* lse);
 
 // tc_fwd_exact.cu: the same on the full mask, in a fixed order of sums
 int exact_forward_set_attrs(int d);

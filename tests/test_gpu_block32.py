@@ -161,3 +161,47 @@ def test_path_argument_is_checked():
     assert _lib.lib.spion_block32_path_in_use(mod.handle) == 2
     with pytest.raises(KeyError):
         BlockSparseAttention(cfg(1, 1, 256, 64, 32), dtype=torch.bfloat16, block32="fastest")
+
+
+@pytest.mark.parametrize("d", [32, 64])
+@pytest.mark.parametrize("keypad", [False, True])
+@pytest.mark.parametrize("merged", [False, True])
+def test_two_block_rows_at_a_time(d, keypad, merged):
+    """Tiles of two 32-wide blocks that either row of a super row selects: one to eighteen of them (odd counts, whose last tile has one block), rows
+    without blocks beside rows with some, blocks selected by one row, by the other, by both; padded keys that begin inside one block of a
+    tile whose other block lies elsewhere."""
+    from spion_b200 import _lib
+    from spion_b200.native import BlockSparseAttention
+    nb, B, H = 36, 2, 2
+    L = nb * 32
+    rng = np.random.default_rng(d)
+    mat = np.zeros((nb, nb), np.uint8)
+    for x in range(nb // 2):
+        cols = rng.choice(nb, size=x + 1, replace=False)
+        who = rng.integers(1, 4, size=x + 1)                     # 1: upper row, 2: lower row, 3: both
+        mat[2 * x, cols[who & 1 > 0]] = 1
+        mat[2 * x + 1, cols[who & 2 > 0]] = 1
+    mat[4] = 0                                                   # one row of a super row without blocks, one super row without any
+    mat[8:10] = 0
+    kp = None
+    if keypad:
+        kp = torch.ones(B, L)
+        kp[0, L - 333:] = 0
+        kp[1, 500:] = 0
+    Q, K, V, dO = [t.to(torch.bfloat16) for t in synthetic.qkv(d, B, H, L, d)]
+    mod = BlockSparseAttention(cfg(B, H, L, d, 32), dtype=torch.bfloat16, keypad=keypad, engine=_lib.ENGINE_TCGEN05, recompute=True, return_probs=False)
+
+    def prep(t):
+        t = t.cuda()
+        if merged:
+            t = t.transpose(1, 2).contiguous().view(B, L, H * d).view(B, L, H, d).transpose(1, 2)
+        return t.requires_grad_(True)
+
+    q, k, v = prep(Q), prep(K), prep(V)
+    out, _ = mod(q, k, v, None if kp is None else kp.cuda(), torch.as_tensor(mat).cuda())
+    g = dO.cuda()
+    out.backward(g.transpose(1, 2).contiguous().transpose(1, 2) if merged else g)
+    mod.check_device_status()
+    O, _, gQ, gK, gV = oatt.sparse_attention(Q.float(), K.float(), V.float(), mat, 32, kp, dO.float())
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), (out, q.grad, k.grad, v.grad), (O, gQ, gK, gV)):
+        assert rel(a, b) <= REL, f"{name}: {rel(a, b):.3e}"
