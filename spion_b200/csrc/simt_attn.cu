@@ -781,124 +781,143 @@ __global__ void __launch_bounds__(64) sddmm_dense_kernel(const float* __restrict
   }
 }
 
-// TRANS == false: out[i] = sum_j value(i, j) Bop[j];  true: out[j] = sum_i value(i, j) Bop[i].  64 rows x 32 columns by 64 threads
-// (4 x 8 each), the sum over L in steps of 32 through two stages.  The sum of an output stays one chain where its bits are kept (dK), so the
-// rows cannot be split further.
-constexpr int DK = 32, DSTAGES = 2;
-constexpr int SPMM_STAGE = DT * (DK + 4) + DK * (DK + 4);        // floats of a stage: value tile, operand tile
-template <bool TRANS>
-__device__ __forceinline__ void spmm_dense(float* smem, int t, int bh, int r0, int n0, int c0, int chunks, const float* vals, const float* Bop,
-                                           const OperandLayout& lb, int L, pair_t (&acc)[4][4], int barrier) {
-  constexpr int VR = TRANS ? DT : DK, VC = TRANS ? DK : DT, VP = TRANS ? DK + 4 : DT;   // value tile as in memory: rows j, columns i
-  const int ty = t >> 2, tx = t & 3;
-  const float* vb = vals + (long long)bh * L * L + (TRANS ? (long long)r0 * L : (long long)r0);
-  const float* Bb = Bop + (long long)bh * lb.bh_stride + (long long)n0 * lb.sd;
-  const bool rows = lb.sd == 1 && (lb.sl & 3) == 0 && (reinterpret_cast<uintptr_t>(Bb) & 15) == 0;
-  auto load = [&](int c) {
-    const int k0 = (c0 + c) * DK;
-    float(*V)[VP] = reinterpret_cast<float(*)[VP]>(smem + (c & 1) * SPMM_STAGE);
-    float(*B)[DK + 4] = reinterpret_cast<float(*)[DK + 4]>(smem + (c & 1) * SPMM_STAGE + DT * (DK + 4));
-    const float* v = vb + (TRANS ? (long long)k0 : (long long)k0 * L);
+// TRANS == false: out[i] = sum_j value(i, j) Bop[j];  true: out[j] = sum_i value(i, j) Bop[i].  Tiles of 64 rows x 32 columns, the sum over L in
+// steps of 16 through two stages of T threads (a warp of its own, or both warps of a tile).  A lane has U rows by eight columns: a
+// shared-memory read returns one register per lane and cycle, so eight rows take 16 such cycles for 32 packed multiply-adds, four by eight, as
+// before, 12 for 16.  The sum of an output stays one chain where its bits are kept (dK), ascending.
+constexpr int DK = 16;
+constexpr int SPMM_STAGE = DT * (DK + 4) + DK * 36;              // floats of a stage: value tile, operand tile [k][32 + 4]
+template <bool TRANS, int U, int T>
+struct Spmm {
+  pair_t acc[U][4];
+  int row0, tx;                                                  // this lane's rows: TRANS row0 + 8 u, else row0 + u; columns 4 tx .., 16 + 4 tx ..
+  __device__ __forceinline__ void run(float* smem, int t, int warp_row, int bh, int r0, int n0, int c0, int chunks, const float* vals, const float* Bop,
+                                      const OperandLayout& lb, int L) {
+    constexpr int VR = TRANS ? DT : DK, VC = TRANS ? DK : DT, VP = TRANS ? DK + 4 : DT;   // value tile as in memory: rows j, columns i
+    const int lane = threadIdx.x & 31, ty = lane >> 2;
+    tx = lane & 3;
+    row0 = warp_row + (TRANS ? ty : U * ty);
+    const float* vb = vals + (long long)bh * L * L + (TRANS ? (long long)r0 * L : (long long)r0);
+    const float* Bb = Bop + (long long)bh * lb.bh_stride + (long long)n0 * lb.sd;
+    const bool rows = lb.sd == 1 && (lb.sl & 3) == 0 && (reinterpret_cast<uintptr_t>(Bb) & 15) == 0;
+    auto load = [&](int c) {
+      const int k0 = (c0 + c) * DK;
+      float* V = smem + (c & 1) * SPMM_STAGE;
+      float* B = V + DT * (DK + 4);
+      const float* v = vb + (TRANS ? (long long)k0 : (long long)k0 * L);
 #pragma unroll
-    for (int e = t; e < VR * VC / 4; e += 64) dense_cp16(&V[e / (VC / 4)][e % (VC / 4) * 4], v + (long long)(e / (VC / 4)) * L + e % (VC / 4) * 4);
-    if (rows) {
+      for (int e = t; e < VR * VC / 4; e += T) dense_cp16(V + e / (VC / 4) * VP + e % (VC / 4) * 4, v + (long long)(e / (VC / 4)) * L + e % (VC / 4) * 4);
+      if (rows) {
 #pragma unroll
-      for (int e = t; e < DK * 32 / 4; e += 64) dense_cp16(&B[e >> 3][(e & 7) * 4], Bb + (long long)(k0 + (e >> 3)) * lb.sl + (e & 7) * 4);
-    } else {
+        for (int e = t; e < DK * 32 / 4; e += T) dense_cp16(B + (e >> 3) * 36 + (e & 7) * 4, Bb + (long long)(k0 + (e >> 3)) * lb.sl + (e & 7) * 4);
+      } else {
 #pragma unroll 4
-      for (int e = t; e < DK * 32; e += 64) dense_cp4(&B[e & 31][e >> 5], Bb + (long long)(k0 + (e & 31)) * lb.sl + (long long)(e >> 5) * lb.sd);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  auto meet = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(barrier) : "memory"); };
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
-  if (chunks > 0) load(0);
-  for (int c = 0; c < chunks; ++c) {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    meet();                                            // chunk c has landed; the stage of chunk c - 1 is free
-    if (c + 1 < chunks) load(c + 1);
-    const float(*Vs)[VP] = reinterpret_cast<const float(*)[VP]>(smem + (c & 1) * SPMM_STAGE);
-    const float(*Bs)[DK + 4] = reinterpret_cast<const float(*)[DK + 4]>(smem + (c & 1) * SPMM_STAGE + DT * (DK + 4));      // [k][n]
-#pragma unroll 2
-    for (int k = 0; k < DK; k += 4) {
-      float a[4][4];                                   // [k][row]
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float4 v = TRANS ? *reinterpret_cast<const float4*>(&Vs[ty + 16 * u][k]) : *reinterpret_cast<const float4*>(&Vs[k + u][4 * ty]);
-        if (TRANS) a[0][u] = v.x, a[1][u] = v.y, a[2][u] = v.z, a[3][u] = v.w;
-        else a[u][0] = v.x, a[u][1] = v.y, a[u][2] = v.z, a[u][3] = v.w;
+        for (int e = t; e < DK * 32; e += T) dense_cp4(B + e % DK * 36 + e / DK, Bb + (long long)(k0 + e % DK) * lb.sl + (long long)(e / DK) * lb.sd);
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const ulonglong2 lo2 = *reinterpret_cast<const ulonglong2*>(&Bs[k + u][4 * tx]), hi2 = *reinterpret_cast<const ulonglong2*>(&Bs[k + u][16 + 4 * tx]);
+    for (int x = 0; x < U; ++x)
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const pair_t aa = twice(a[u][x]);
-          fma2(acc[x][0], aa, lo2.x), fma2(acc[x][1], aa, lo2.y), fma2(acc[x][2], aa, hi2.x), fma2(acc[x][3], aa, hi2.y);
+      for (int y = 0; y < 4; ++y) acc[x][y] = 0ull;
+    if (chunks > 0) load(0);
+    for (int c = 0; c < chunks; ++c) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (T > 32) __syncthreads(); else __syncwarp();  // chunk c has landed; the stage of chunk c - 1 is free
+      if (c + 1 < chunks) load(c + 1);
+      const float* Vs = smem + (c & 1) * SPMM_STAGE;
+      const float* Bs = Vs + DT * (DK + 4) + 4 * tx;
+#pragma unroll
+      for (int k = 0; k < DK; k += 4) {
+        float a[TRANS ? U : 1][4];
+        if (TRANS) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const float4 v = *reinterpret_cast<const float4*>(Vs + (row0 + 8 * u) * VP + k);
+            a[u][0] = v.x, a[u][1] = v.y, a[u][2] = v.z, a[u][3] = v.w;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float r[U];
+          if (!TRANS) {
+#pragma unroll
+            for (int u = 0; u < U; u += 4) {
+              const float4 v = *reinterpret_cast<const float4*>(Vs + (k + i) * VP + row0 + u);
+              r[u] = v.x, r[u + 1] = v.y, r[u + 2] = v.z, r[u + 3] = v.w;
+            }
+          }
+          const ulonglong2 lo2 = *reinterpret_cast<const ulonglong2*>(Bs + (k + i) * 36), hi2 = *reinterpret_cast<const ulonglong2*>(Bs + (k + i) * 36 + 16);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const pair_t aa = twice(TRANS ? a[TRANS ? u : 0][i] : r[u]);
+            fma2(acc[u][0], aa, lo2.x), fma2(acc[u][1], aa, lo2.y), fma2(acc[u][2], aa, hi2.x), fma2(acc[u][3], aa, hi2.y);
+          }
         }
       }
     }
   }
-}
-template <bool TRANS>
-__device__ __forceinline__ void spmm_dense_write(const pair_t (&acc)[4][4], int t, int bh, int r0, int n0, float* out, const OperandLayout& lo) {
-  const int ty = t >> 2, tx = t & 3;
-  float* ob = out + (long long)bh * lo.bh_stride;
+  // parts of a sum in PARTS warps: in the first one's accumulators, added in order.  All of them call it.
+  template <int PARTS> __device__ __forceinline__ void join(float* smem) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float2* part = reinterpret_cast<float2*>(smem);
+    __syncthreads();
+    if (w > 0) {
 #pragma unroll
-  for (int x = 0; x < 4; ++x) {
-    const int row = r0 + (TRANS ? ty + 16 * x : 4 * ty + x);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float4 v = as_float4(acc[x][2 * h], acc[x][2 * h + 1]);
-      float* o = ob + (long long)row * lo.sl + (long long)(n0 + 16 * h + 4 * tx) * lo.sd;
-      if (lo.sd == 1 && (reinterpret_cast<uintptr_t>(o) & 15) == 0) *reinterpret_cast<float4*>(o) = v;
-      else o[0] = v.x, o[lo.sd] = v.y, o[2 * lo.sd] = v.z, o[3 * lo.sd] = v.w;
+      for (int e = 0; e < 4 * U; ++e) {
+        float2 v;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(acc[e >> 2][e & 3]));
+        part[((w - 1) * 4 * U + e) * 32 + lane] = v;
+      }
     }
-  }
-}
-
-// O = P V.  Its bits are nobody's: four groups of 64 threads take a quarter of the keys each, so that a call of 256 tiles has fourteen warps per
-// SM, and the quarters are added in order.  16 matrices, L = 1024, d 32: 31 us (34 with one group).
-constexpr int OGROUPS = 4;
-__global__ void __launch_bounds__(64 * OGROUPS) spmm_dense_split(const float* __restrict__ vals, const float* __restrict__ Bop, OperandLayout lb,
-                                                                 float* __restrict__ out, OperandLayout lo, int L) {
-  extern __shared__ __align__(16) float s_spmm[];
-  const int g = threadIdx.x >> 6, t = threadIdx.x & 63;
-  const int r0 = blockIdx.x * DT, bh = blockIdx.y, n0 = blockIdx.z * 32;
-  const int chunks = L / DK, per = (chunks + OGROUPS - 1) / OGROUPS, c0 = min(chunks, g * per), c1 = min(chunks, c0 + per);
-  pair_t acc[4][4];
-  spmm_dense<false>(s_spmm + g * DSTAGES * SPMM_STAGE, t, bh, r0, n0, c0, c1 - c0, vals, Bop, lb, L, acc, 1 + g);
-  __syncthreads();
-  float2* sum = reinterpret_cast<float2*>(s_spmm);
-  if (g > 0)
+    __syncthreads();
+    if (w > 0) return;
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
+    for (int e = 0; e < 4 * U; ++e) {
       float2 v;
       asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(acc[e >> 2][e & 3]));
-      sum[((g - 1) * 16 + e) * 64 + t] = v;
-    }
-  __syncthreads();
-  if (g > 0) return;
 #pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(acc[e >> 2][e & 3]));
-#pragma unroll
-    for (int o = 0; o < OGROUPS - 1; ++o) {
-      const float2 w = sum[(o * 16 + e) * 64 + t];
-      v.x += w.x;
-      v.y += w.y;
+      for (int o = 0; o < PARTS - 1; ++o) {
+        const float2 y = part[(o * 4 * U + e) * 32 + lane];
+        v.x += y.x;
+        v.y += y.y;
+      }
+      asm("mov.b64 %0, {%1, %2};" : "=l"(acc[e >> 2][e & 3]) : "f"(v.x), "f"(v.y));
     }
-    asm("mov.b64 %0, {%1, %2};" : "=l"(acc[e >> 2][e & 3]) : "f"(v.x), "f"(v.y));
   }
-  spmm_dense_write<false>(acc, t, bh, r0, n0, out, lo);
+  __device__ __forceinline__ void write(int bh, int r0, int n0, float* out, const OperandLayout& lo) {
+    float* ob = out + (long long)bh * lo.bh_stride;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int row = r0 + row0 + (TRANS ? 8 * u : u);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 v = as_float4(acc[u][2 * h], acc[u][2 * h + 1]);
+        float* o = ob + (long long)row * lo.sl + (long long)(n0 + 16 * h + 4 * tx) * lo.sd;
+        if (lo.sd == 1 && (reinterpret_cast<uintptr_t>(o) & 15) == 0) *reinterpret_cast<float4*>(o) = v;
+        else o[0] = v.x, o[lo.sd] = v.y, o[2 * lo.sd] = v.z, o[3 * lo.sd] = v.w;
+      }
+    }
+  }
+};
+
+// O = P V.  Its bits are nobody's: four warps take a quarter of the keys each.  16 matrices, L = 1024, d 32: 34 us with one chain of 64 threads a
+// tile, 31 with four of them, 28 so; 60 matrices 121, 122, 96.
+constexpr int OPARTS = 4;
+__global__ void __launch_bounds__(32 * OPARTS) spmm_dense_split(const float* __restrict__ vals, const float* __restrict__ Bop, OperandLayout lb,
+                                                                float* __restrict__ out, OperandLayout lo, int L) {
+  extern __shared__ __align__(16) float s_spmm[];
+  const int w = threadIdx.x >> 5, r0 = blockIdx.x * DT, bh = blockIdx.y, n0 = blockIdx.z * 32;
+  const int chunks = L / DK, per = (chunks + OPARTS - 1) / OPARTS, c0 = min(chunks, w * per), c1 = min(chunks, c0 + per);
+  Spmm<false, 8, 32> x;
+  x.run(s_spmm + w * 2 * SPMM_STAGE, threadIdx.x & 31, 0, bh, r0, n0, c0, c1 - c0, vals, Bop, lb, L);
+  x.join<OPARTS>(s_spmm);
+  if (w == 0) x.write(bh, r0, n0, out, lo);
 }
 
-// dK = dS^T Q, dV = P^T dO and dQ = dS K of a backward in one launch: tiles of 64 threads each, four warps per SM with one launch per product, ten
-// to twelve with all three.  16 matrices, L = 1024, d 32: 107 us in three launches, 94 in one.
+// dK = dS^T Q, dV = P^T dO and dQ = dS K of a backward in one launch, so that every SM has ten warps or more; dK by two warps of 32 rows each, the others
+// by two warps of half of the sum each.  16 matrices, L = 1024, d 32: 107 us in three launches, 94 in one with four by eight outputs a lane,
+// 88 so; 60 matrices 376, 333, 314 (4 matrices, L = 512, d 64: 57, 26, 27).
 struct DenseGrads {
   const float *P, *dS, *Q, *K, *dO;
   float *dQ, *dK, *dV;
@@ -906,15 +925,25 @@ struct DenseGrads {
   int L, halves;                                       // head_dim / 32
 };
 __global__ void __launch_bounds__(64) spmm_dense_grads(const DenseGrads a) {
-  __shared__ __align__(16) float smem[DSTAGES * SPMM_STAGE];
-  const int what = blockIdx.z / a.halves, n0 = (blockIdx.z - what * a.halves) * 32, r0 = blockIdx.x * DT, bh = blockIdx.y, t = threadIdx.x;
-  pair_t acc[4][4];
-  if (what < 2) {
-    spmm_dense<true>(smem, t, bh, r0, n0, 0, a.L / DK, what ? a.P : a.dS, what ? a.dO : a.Q, a.lo, a.L, acc, 1);
-    spmm_dense_write<true>(acc, t, bh, r0, n0, what ? a.dV : a.dK, a.lo);
+  extern __shared__ __align__(16) float s_spmm[];
+  const int what = blockIdx.z / a.halves, n0 = (blockIdx.z - what * a.halves) * 32, r0 = blockIdx.x * DT, bh = blockIdx.y, w = threadIdx.x >> 5;
+  const int chunks = a.L / DK, half = chunks / 2;      // L is a multiple of 64
+  float* own = s_spmm + w * 2 * SPMM_STAGE;
+  const int lane = threadIdx.x & 31;
+  if (what == 0) {
+    Spmm<true, 4, 64> x;
+    x.run(s_spmm, threadIdx.x, 32 * w, bh, r0, n0, 0, chunks, a.dS, a.Q, a.lo, a.L);
+    x.write(bh, r0, n0, a.dK, a.lo);
+  } else if (what == 1) {
+    Spmm<true, 8, 32> x;
+    x.run(own, lane, 0, bh, r0, n0, w * half, w ? chunks - half : half, a.P, a.dO, a.lo, a.L);
+    x.join<2>(s_spmm);
+    if (w == 0) x.write(bh, r0, n0, a.dV, a.lo);
   } else {
-    spmm_dense<false>(smem, t, bh, r0, n0, 0, a.L / DK, a.dS, a.K, a.lo, a.L, acc, 1);
-    spmm_dense_write<false>(acc, t, bh, r0, n0, a.dQ, a.lo);
+    Spmm<false, 8, 32> x;
+    x.run(own, lane, 0, bh, r0, n0, w * half, w ? chunks - half : half, a.dS, a.K, a.lo, a.L);
+    x.join<2>(s_spmm);
+    if (w == 0) x.write(bh, r0, n0, a.dQ, a.lo);
   }
 }
 
@@ -1192,9 +1221,9 @@ int simt_spmm(int dtype_val, int dtype_op, bool trans, const void* vals, ValueLa
               OperandLayout lb, void* out, OperandLayout lo, Pattern p, int BH, int d, cudaStream_t st) {
   if (d % 32 != 0 || BH > 65535) return SPION_ERR_UNSUPPORTED;
   if (!trans && dtype_val == SPION_F32 && dtype_op == SPION_F32 && full_dense(vl, p, vals)) {       // trans: simt_dense_grads
-    constexpr int smem = OGROUPS * DSTAGES * SPMM_STAGE * (int)sizeof(float);
+    constexpr int smem = OPARTS * 2 * SPMM_STAGE * (int)sizeof(float);
     SPION_CUDA_TRY(cudaFuncSetAttribute(spmm_dense_split, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    spmm_dense_split<<<dim3(p.nb, BH, d / 32), 64 * OGROUPS, smem, st>>>((const float*)vals, (const float*)Bop, lb, (float*)out, lo, vl.L);
+    spmm_dense_split<<<dim3(p.nb, BH, d / 32), 32 * OPARTS, smem, st>>>((const float*)vals, (const float*)Bop, lb, (float*)out, lo, vl.L);
     SPION_LAUNCH_CHECK();
     return SPION_OK;
   }
@@ -1363,7 +1392,8 @@ int simt_dense_grads(const float* P, const float* dS, const float* Q, const floa
                      Pattern p, int BH, int L, int d, cudaStream_t st) {
   const ValueLayout vl{VAL_DENSE_T, L, (long long)L * L};
   if (d % 32 != 0 || BH > 65535 || !full_dense(vl, p, P) || !full_dense(vl, p, dS)) return SPION_ERR_UNSUPPORTED;
-  spmm_dense_grads<<<dim3(p.nb, BH, 3 * (d / 32)), 64, 0, st>>>(DenseGrads{P, dS, Q, K, dO, dQ, dK, dV, lo, L, d / 32});
+  constexpr int smem = 2 * 2 * SPMM_STAGE * (int)sizeof(float);
+  spmm_dense_grads<<<dim3(p.nb, BH, 3 * (d / 32)), 64, smem, st>>>(DenseGrads{P, dS, Q, K, dO, dQ, dK, dV, lo, L, d / 32});
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }
