@@ -96,6 +96,21 @@ __global__ void __launch_bounds__(EMB_THREADS) embedding_bwd_kernel(const long l
           acc = v;
         }
       };
+      // In the middle of a run: nothing to look up, so the rows are loaded ahead of the additions, which keep their order.  A CTA in the
+      // padded tail of a sequence walks all of its tokens in one group: 65536 tokens of 256 ids, N = 64, a quarter of them padding, 33.3 -> 19.4 us
+      // with the partial sums (no padding: 19.6, 19.9).
+      if (__all_sync(0xffffffffu, mine && (int)raw == cur)) {
+        const TG* p = gs + s * N + col;
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = to_f32(p[(k + e) * N]);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc += v[e];
+        }
+        m = 0;
+      }
       while (m) {                          // two tokens per turn: their loads do not wait for each other
         const int k0 = __ffs(m) - 1;
         m &= m - 1;

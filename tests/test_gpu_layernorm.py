@@ -129,6 +129,21 @@ def test_token_embedding_weight_gradient(V, N, B, L, dtype):
     assert err <= 1e-5 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("V,N,T,dtype", [(256, 64, 5000, torch.float32), (16, 32, 4099, torch.bfloat16), (90, 256, 3001, torch.float32), (4, 128, 700, torch.bfloat16)])
+def test_token_embedding_gradient_of_runs(V, N, T, dtype):
+    """Runs of equal ids of every length around the 32 ids that a warp looks at together, and tokens without a row between them.  The sums of
+    whole numbers are exact in any order: at most 5000 times 8 is below 2^24."""
+    from spion_b200.layernorm import _embedding_weight_grad
+    g = torch.Generator().manual_seed(V)
+    lens = [1, 31, 32, 33, 63, 64, 65, 96, 100, 200]
+    ids = torch.cat([torch.full((lens[int(torch.randint(len(lens), (1,), generator=g))],), int(torch.randint(-1, V, (1,), generator=g))) for _ in range(T)])[:T]
+    rows = torch.randint(-8, 9, (T, N), generator=g).to(dtype)
+    want = torch.zeros(V, N, dtype=torch.float64)
+    want.index_add_(0, ids[ids >= 0], rows.double()[ids >= 0])
+    got = _embedding_weight_grad(ids.cuda(), rows.cuda(), V, N, torch.float32)
+    assert torch.equal(got.cpu().double(), want)
+
+
 def test_token_embedding_falls_back_for_large_tables():
     from spion_b200.layernorm import TokenEmbedding
     mod = TokenEmbedding(30000, 64).cuda()
