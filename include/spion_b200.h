@@ -403,6 +403,10 @@ long long spion_embedding_workspace_floats(long long T, int V, int N);
  * 16-byte aligned, N a multiple of 4; an id outside [0, V) gives the position row alone. */
 int spion_embedding_forward(const long long* ids, const float* tok, const float* pos, float* out, long long T, int L,
                             int V, int N, void* cuda_stream);
+/* y [B, L, N] = x * mask[:, :, None], fp32; rows of x stride_b / stride_l floats apart (multiples of 4, 0 allowed), N a multiple of 4,
+ * x and y 16-byte aligned. */
+int spion_mask_rows(const float* x, long long stride_b, long long stride_l, const float* mask, float* y, int B, int L, int N,
+                    void* cuda_stream);
 int spion_embedding_backward(const long long* ids, const void* g, int g_is_bf16, long long T, int V, int N,
                              float* dW, float* workspace, void* cuda_stream);
 

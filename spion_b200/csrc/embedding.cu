@@ -172,6 +172,24 @@ __global__ void __launch_bounds__(256) embedding_fwd_kernel(const long long* __r
   }
 }
 
+// y[b, l, :] = x[b, l, :] * mask[b, l], the rows of x at any distance from each other (0: one row for a whole sequence, as the gradient of
+// a mean over the sequence is).  Bound by writing out; four pieces of 16 bytes per thread.
+// 65536 rows of 64: 5.8 us, 4.6 from one row per sequence (the framework: 11.6 us, and 40 for means, slices and product).
+__global__ void __launch_bounds__(256) mask_rows_kernel(const float* __restrict__ x, long long stride_b, long long stride_l,
+                                                        const float* __restrict__ mask, float* __restrict__ y, unsigned rows, int L, int per_row) {
+  const unsigned total = rows * per_row;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned i = (blockIdx.x * 4 + k) * 256 + threadIdx.x;
+    if (i >= total) continue;
+    const unsigned r = i / per_row, c = i - r * per_row, b = r / L, l = r - b * L;
+    const float m = mask[r];
+    float4 v = *reinterpret_cast<const float4*>(x + b * stride_b + l * stride_l + 4 * c);
+    v.x *= m, v.y *= m, v.z *= m, v.w *= m;
+    *reinterpret_cast<float4*>(y + (size_t)i * 4) = v;
+  }
+}
+
 size_t emb_smem(int V, int N, int g_is_bf16) {
   const int batch = emb_batch(N, g_is_bf16 ? 2 : 4);
   return (size_t)V * N * sizeof(float) + EMB_STAGES * ((size_t)batch * N * (g_is_bf16 ? 2 : 4) + batch * sizeof(long long));
@@ -240,6 +258,21 @@ extern "C" int spion_embedding_forward(const long long* ids, const float* tok, c
   const long long want = (T * (N / 4) + 255) / 256;
   const int grid = (int)std::max<long long>(1, std::min<long long>(want, (long long)sms * 8));
   embedding_fwd_kernel<<<grid, 256, 0, stream>>>(ids, tok, pos, out, T, L, V, N);
+  SPION_LAUNCH_CHECK();
+  return SPION_OK;
+}
+
+// y [B, L, N] fp32 = x * mask[:, :, None]: the zeroed padding rows of the encoder's output (models/model_transformer.py) and their gradient.
+// x: rows of N contiguous floats, stride_b and stride_l floats (multiples of 4, not negative) from sequence to sequence and from row to row;
+// x and y 16-byte aligned, N a multiple of 4, fewer than 2^32 - 1024 pieces of four values.
+extern "C" int spion_mask_rows(const float* x, long long stride_b, long long stride_l, const float* mask, float* y, int B, int L, int N,
+                               void* cuda_stream) {
+  if (!x || !mask || !y || B < 1 || L < 1 || stride_b < 0 || stride_l < 0) return SPION_ERR_ARG;
+  if ((((uintptr_t)x) | ((uintptr_t)y)) & 15 || (stride_b | stride_l) & 3) return SPION_ERR_ARG;
+  const long long rows = (long long)B * L;
+  if (N < 4 || N % 4 != 0 || rows > 0xfffffbffLL / (N / 4)) return SPION_ERR_SHAPE;
+  const unsigned grid = (unsigned)((rows * (N / 4) + 1023) / 1024);
+  mask_rows_kernel<<<grid, 256, 0, (cudaStream_t)cuda_stream>>>(x, stride_b, stride_l, mask, y, (unsigned)rows, L, N / 4);
   SPION_LAUNCH_CHECK();
   return SPION_OK;
 }

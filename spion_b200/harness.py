@@ -15,6 +15,7 @@ import torch.nn as nn
 
 from . import dp
 from .attention import Attention, no_global_hooks, untouched
+from .layernorm import mask_rows, sequence_means
 from .pattern import discover_layers
 
 
@@ -142,7 +143,7 @@ class Encoder(nn.Module):
             for i, layer in enumerate(self.layers):
                 nxt = self.layers[i + 1].norm1 if i + 1 < len(self.layers) else self.norm
                 X, Xn, _ = layer.forward_add_norm(X, Xn, mask, mat_lst[0][i], nxt)
-            return Xn * mask[:, :, None], maps
+            return mask_rows(Xn, mask), maps
         for i, layer in enumerate(self.layers):
             if mat_lst is None:
                 X, attn = layer(X, mask)
@@ -153,7 +154,7 @@ class Encoder(nn.Module):
                     maps.append(mean_attention_map(attn.permute(0, 1, 3, 2), transposed_storage=True))
             else:
                 X, _ = layer(X, mask, mat_lst[0][i])
-        return self.norm(X) * mask[:, :, None], maps
+        return mask_rows(self.norm(X), mask), maps
 
 
 class Classifier(nn.Module):
@@ -179,7 +180,7 @@ class Classifier(nn.Module):
                 both = torch.cat([ids[0], ids[1]], 0)
                 t, maps = self.model(both, (both != 0).float(), mat_lst, False)
                 nb = ids[0].shape[0]
-                x0, x1 = t[:nb].mean(1), t[nb:].mean(1)
+                x0, x1 = sequence_means(t, nb)
                 scores = self.head(torch.cat([x0, x1, x0 * x1, x0 - x1], dim=-1))
             elif self.dual:
                 m0, m1 = (ids[0] != 0).float(), (ids[1] != 0).float()        # models/dataset_LRA.py:34
@@ -190,7 +191,7 @@ class Classifier(nn.Module):
             else:
                 mask = (ids != 0).float()
                 t, maps = self.model(ids, mask, mat_lst, is_attn)
-                scores = self.head(t.mean(1))
+                scores = self.head(sequence_means(t, t.shape[0])[0])
             loss = nn.functional.cross_entropy(scores.float(), label)
         return loss, maps
 

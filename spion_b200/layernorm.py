@@ -303,3 +303,63 @@ class TokenEmbedding(nn.Embedding):
         if not ok:
             return self(ids) + pos_weight[:L][None]
         return _EmbedPosFn.apply(ids, self.weight, pos_weight)
+
+
+def _rows_ok(x):
+    """What spion_mask_rows reads: fp32 [B, L, N] on the GPU, rows contiguous and on 16-byte boundaries."""
+    return (x.dim() == 3 and x.is_cuda and x.dtype == torch.float32 and x.numel() > 0 and x.shape[2] % 4 == 0 and x.numel() < 1 << 33
+            and x.stride(2) == 1 and min(x.stride()) >= 0 and x.stride(0) % 4 == 0 and x.stride(1) % 4 == 0 and x.data_ptr() % 16 == 0)
+
+
+def _mask_rows(x, mask):
+    B, L, N = x.shape
+    y = torch.empty(B, L, N, dtype=torch.float32, device=x.device)
+    with torch.cuda.device(x.device):
+        check(lib.spion_mask_rows(ptr(x), x.stride(0), x.stride(1), ptr(mask), ptr(y), B, L, N, _lib.current_stream_ptr()),
+              "spion_mask_rows")
+    return y
+
+
+class _MaskRowsFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, mask):
+        ctx.save_for_backward(mask)
+        return _mask_rows(x, mask)
+
+    @staticmethod
+    def backward(ctx, g):
+        (mask,) = ctx.saved_tensors
+        if torch.is_grad_enabled() or not _rows_ok(g) or not _mask_ok(mask, g):
+            return g * mask[:, :, None], None
+        return _mask_rows(g, mask), None
+
+
+def _mask_ok(mask, x):
+    return (mask.dtype == torch.float32 and mask.device == x.device and mask.shape == x.shape[:2] and mask.is_contiguous()
+            and not mask.requires_grad)
+
+
+def mask_rows(x, mask):
+    """``x * mask[:, :, None]`` for x [B, L, N] and mask [B, L]: one kernel each way for fp32 rows, which reads the gradient of a mean
+    over the sequence (``sequence_means``) without writing it out first."""
+    if torch.jit.is_tracing() or not x.is_contiguous() or not _rows_ok(x) or not _mask_ok(mask, x):   # (other strides are the result's too)
+        return x * mask[:, :, None]
+    return _MaskRowsFn.apply(x, mask)
+
+
+class _SequenceMeansFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, t, n):
+        ctx.size = t.shape
+        return tuple(t[i:i + n].mean(1) for i in range(0, t.shape[0], n))
+
+    @staticmethod
+    def backward(ctx, *gs):
+        g = (gs[0] if len(gs) == 1 else torch.cat(gs)) / ctx.size[1]
+        return g[:, None, :].expand(ctx.size), None
+
+
+def sequence_means(t, n):
+    """Means over the sequence of each ``n`` sequences of t [B, L, N].  The gradient is a view with one row per sequence: slicing and the
+    framework's mean form it in full, slice by slice."""
+    return _SequenceMeansFn.apply(t, n)

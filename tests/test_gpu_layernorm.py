@@ -211,3 +211,31 @@ def test_token_plus_position_embedding_in_one_kernel(B, L, Lmax):
     assert torch.equal(outs[0][0], outs[1][0])
     for a, b in zip(outs[0][1:], outs[1][1:]):
         assert float((a - b).abs().max()) <= 1e-5 * max(1.0, float(a.abs().max()))
+
+
+@pytest.mark.parametrize("B,L,N", [(1, 1, 4), (2, 257, 64), (6, 33, 20), (4, 1024, 128), (3, 50, 6)])
+def test_masked_rows_and_means_over_sequences(B, L, N):
+    """Same bits as the framework's operators, values and gradients: gradient with one row per sequence, in full, strided; a width without
+    16-byte pieces, an odd address, and a second derivative."""
+    from spion_b200.layernorm import mask_rows, sequence_means
+    g = torch.Generator(device="cuda").manual_seed(L)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    mask = (torch.rand(B, L, generator=g, device="cuda") > 0.3).float() * 0.5
+    n = (B + 1) // 2
+    for x in (rnd(B, L, N), rnd(B, N, L).transpose(1, 2), rnd(B * L * N + 1)[1:].view(B, L, N), rnd(B, 1, N).expand(B, L, N)):
+        full, weights = rnd(B, N, L).transpose(1, 2), rnd(-(-B // n), n, N)
+        got, want = [], []
+        for out, own in ((got, True), (want, False)):
+            xs = x.detach().requires_grad_(True)
+            t = mask_rows(xs, mask) if own else xs * mask[:, :, None]
+            means = sequence_means(t, n) if own else [t[i:i + n].mean(1) for i in range(0, B, n)]
+            loss = sum((m * m * w[:len(m)]).sum() for m, w in zip(means, weights))
+            g1, = torch.autograd.grad(loss, xs, retain_graph=True)
+            g2, = torch.autograd.grad(t, xs, full, retain_graph=True)
+            g3, = torch.autograd.grad(loss, xs, create_graph=True)
+            g4, = torch.autograd.grad((g3 * full).sum(), xs)
+            out += [t, *means, g1, g2, g3, g4]
+        assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got[:-1], want[:-1]))
+        # a sum of L values before or after the division by L
+        bound = L * 2.0 ** -23 * float((full.abs() * mask[:, :, None]).sum(1).max()) / L * 2 * float(weights.abs().max())
+        assert float((got[-1] - want[-1]).abs().max()) <= bound
