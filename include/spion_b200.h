@@ -390,6 +390,9 @@ int spion_column_sums(const void* dy, int dy_is_bf16, float* out, float* workspa
  * workspace count times as large. */
 int spion_column_sums_many(const void* const* dys, int count, int dy_is_bf16, float* out, float* workspace, long long M, int N,
                            void* cuda_stream);
+/* ... and to[i] = from[i] for n bf16 values, to fp32, in the same launches (from and to 16-byte aligned; n = 0: none). */
+int spion_column_sums_convert(const void* const* dys, int count, int dy_is_bf16, float* out, float* workspace, long long M, int N,
+                              const void* from, float* to, long long n, void* cuda_stream);
 
 /* Weight gradient of a token embedding with a small table (torch.nn.Embedding(vocab_size, embedding_dim) in the
  * reference's encoder, models/model_transformer.py; vocab_size 256 - 512 in its tasks):

@@ -45,6 +45,8 @@ SIGNATURES = {
                                 ctypes.c_float, c_void_p]),
     "spion_layernorm_workspace_floats": (c_longlong, [c_int]),
     "spion_column_sums": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p]),
+    "spion_column_sums_convert": (c_int, [ctypes.POINTER(c_void_p), c_int, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p,
+                                          c_longlong, c_void_p]),
     "spion_column_sums_many": (c_int, [ctypes.POINTER(c_void_p), c_int, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p]),
     "spion_add_layernorm_forward": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                         c_void_p, c_void_p, c_longlong, c_int, ctypes.c_float, c_void_p]),

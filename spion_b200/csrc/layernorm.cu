@@ -255,6 +255,15 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, float4 v) {
   w.y = *reinterpret_cast<const unsigned*>(&hi);
   *reinterpret_cast<uint2*>(p) = w;
 }
+// to = from in fp32, by all CTAs along x; both 16-byte aligned
+__device__ __forceinline__ void convert(const __nv_bfloat16* __restrict__ from, float* __restrict__ to, long long n) {
+  const long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (long long i = at; i < n / 4; i += step) st4(to + 4 * i, ld4(from + 4 * i));
+  if (at < n % 4) to[n - 1 - at] = __bfloat162float(from[n - 1 - at]);
+}
+__global__ void __launch_bounds__(256) convert_kernel(const __nv_bfloat16* __restrict__ from, float* __restrict__ to, long long n) {
+  convert(from, to, n);
+}
 template <int LPR>
 __device__ __forceinline__ float row_sum(float v) {   // over the LPR lanes of a row (all 32 lanes take part)
 #pragma unroll
@@ -319,11 +328,17 @@ __global__ void __launch_bounds__(LN_WARPS * 32) ln_bwd4_kernel(const float* __r
 // Column sums with 16-byte loads: a row of N values takes LPR = N * sizeof(T) / 16 lanes (8 or 16 for N = 64, 16 or 32
 // for N = 128), a warp reads 32 / LPR rows per step, four steps in flight.  blockIdx.y: one of several matrices of one size (the
 // query, key and value layers' bias gradients in two launches instead of six of 3 us).
-struct ColumnSumList { const void* p[4]; };
+// blockIdx.y past the matrices: the bf16 products that the same call converts to fp32 (a weight gradient of the framework's GEMM); as a
+// launch of its own that took 3 us.
+struct ColumnSumList { const void* p[4]; int count; const __nv_bfloat16* from; float* to; long long n; };
 template <int N, typename T>
 __global__ void __launch_bounds__(LN_WARPS * 32) colsum4_kernel(const __grid_constant__ ColumnSumList list, float* __restrict__ partial,
                                                                 long long M) {
   next_may_start();                                                    // colsum_reduce_kernel
+  if ((int)blockIdx.y == list.count) {
+    convert(list.from, list.to, list.n);
+    return;
+  }
   const T* __restrict__ dy = static_cast<const T*>(list.p[blockIdx.y]);
   partial += (size_t)blockIdx.y * gridDim.x * N;
   constexpr int PER = 16 / (int)sizeof(T), LPR = N / PER, RPW = 32 / LPR;
@@ -489,11 +504,20 @@ extern "C" int spion_add_layernorm_backward(const float* x, const void* dy, int 
 // linear layers.  workspace: count * spion_layernorm_workspace_floats(N) floats.  Fixed summation order.
 extern "C" int spion_column_sums_many(const void* const* dys, int count, int dy_is_bf16, float* out, float* workspace, long long M, int N,
                                       void* cuda_stream) {
+  return spion_column_sums_convert(dys, count, dy_is_bf16, out, workspace, M, N, nullptr, nullptr, 0, cuda_stream);
+}
+
+// ... and to[i] = from[i] for n bf16 values (none: n = 0), on 16-byte boundaries.
+extern "C" int spion_column_sums_convert(const void* const* dys, int count, int dy_is_bf16, float* out, float* workspace, long long M, int N,
+                                         const void* from, float* to, long long n, void* cuda_stream) {
   cudaStream_t stream = (cudaStream_t)cuda_stream;
+  if (n < 0 || (n && (!from || !to || (((uintptr_t)from | (uintptr_t)to) & 15)))) return SPION_ERR_ARG;
   if (!dys || count < 1 || count > 4 || !out || !workspace || M < 1) return SPION_ERR_ARG;
   const int grid = ln_grid(M);
   if (grid < 1) return SPION_ERR_CUDA;
   ColumnSumList list = {};
+  list.count = count;
+  list.from = (const __nv_bfloat16*)from; list.to = to; list.n = n;
   bool aligned = true;
   for (int i = 0; i < count; ++i) {
     if (!dys[i]) return SPION_ERR_ARG;
@@ -501,7 +525,7 @@ extern "C" int spion_column_sums_many(const void* const* dys, int count, int dy_
     aligned = aligned && ((uintptr_t)dys[i] & 15) == 0;
   }
   if ((N == 64 || N == 128) && aligned) {
-    const dim3 g(grid, count);
+    const dim3 g(grid, count + (n > 0));
     if (N == 64 && dy_is_bf16) colsum4_kernel<64, __nv_bfloat16><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
     else if (N == 64) colsum4_kernel<64, float><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
     else if (dy_is_bf16) colsum4_kernel<128, __nv_bfloat16><<<g, LN_WARPS * 32, 0, stream>>>(list, workspace, M);
@@ -524,6 +548,10 @@ extern "C" int spion_column_sums_many(const void* const* dys, int count, int dy_
     SPION_LAUNCH_CHECK();
   }
 #undef SPION_COLSUM
+  if (n) {
+    convert_kernel<<<(int)std::min<long long>((n / 4 + 255) / 256 + 1, 1024), 256, 0, stream>>>(list.from, to, n);
+    SPION_LAUNCH_CHECK();
+  }
   SPION_CUDA_TRY(launch_after(colsum_reduce_kernel, dim3(N / 32, count), dim3(1024), 0, stream, workspace, grid, N, out));
   return SPION_OK;
 }

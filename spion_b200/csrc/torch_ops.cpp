@@ -150,19 +150,23 @@ void linear_backward_weight(const std::vector<Tensor>& dY, const spion_tokens& t
   if (tX.is_bf16 && !copied && tY.heads == 0 && tX.heads == 0) {
     Tensor x2 = X.view({T, in});
     const int n = w.n();
-    Tensor prod = at::empty({out, in}, x2.options());        // the products side by side: one conversion for all of them
+    Tensor prod = at::empty({out, in}, x2.options());        // the products side by side: one conversion for all of them, beside the sums
     std::vector<const void*> dys;
     for (int i = 0; i < n; ++i) {
       Tensor dy2 = dY[i].view({T, per}), part = prod.narrow(0, i * per, per);
       at::mm_out(part, dy2.t(), x2);
       dys.push_back(dy2.data_ptr());
     }
-    Tensor g32 = prod.to(at::kFloat), sums;
+    Tensor g32, sums;
     const bool kernel = per == 64 || per == 128 || per == 256 || per == 512;
     if (kernel) {
       sums = at::empty({out}, opt);
       Tensor ws = at::empty({(int64_t)n * spion_layernorm_workspace_floats((int)per)}, opt);
-      check(spion_column_sums_many(dys.data(), n, 1, (float*)sums.data_ptr(), (float*)ws.data_ptr(), T, (int)per, st), "spion_column_sums_many");
+      g32 = at::empty({out, in}, opt);
+      check(spion_column_sums_convert(dys.data(), n, 1, (float*)sums.data_ptr(), (float*)ws.data_ptr(), T, (int)per, prod.data_ptr(),
+                                      (float*)g32.data_ptr(), out * in, st), "spion_column_sums_convert");
+    } else {
+      g32 = prod.to(at::kFloat);
     }
     for (int i = 0; i < n; ++i) {
       dW.push_back(g32.narrow(0, i * per, per));

@@ -213,6 +213,22 @@ def test_token_plus_position_embedding_in_one_kernel(B, L, Lmax):
         assert float((a - b).abs().max()) <= 1e-5 * max(1.0, float(a.abs().max()))
 
 
+@pytest.mark.parametrize("N,count,M,n,odd", [(64, 3, 5000, 3 * 64 * 64, 0), (128, 1, 1, 5, 0), (64, 4, 300, 1, 0), (256, 2, 700, 4099, 0), (64, 2, 999, 260, 2)])
+def test_column_sums_beside_a_conversion(N, count, M, n, odd):
+    """Widths with 16-byte loads and without, matrices on 4-byte boundaries, a remainder of the conversion.  Sums of whole numbers are exact."""
+    import ctypes
+    from spion_b200._lib import check, current_stream_ptr, lib, ptr
+    g = torch.Generator(device="cuda").manual_seed(n)
+    dys = [torch.randint(-8, 9, (M * N + odd,), generator=g, device="cuda").bfloat16()[odd:].view(M, N) for _ in range(count)]
+    src = torch.randn(n, generator=g, device="cuda").bfloat16()
+    out, to = torch.empty(count, N, device="cuda"), torch.full((n + 4,), 7.0, device="cuda")
+    ws = torch.empty(count * int(lib.spion_layernorm_workspace_floats(N)), device="cuda")
+    ps = (ctypes.c_void_p * count)(*[t.data_ptr() for t in dys])
+    check(lib.spion_column_sums_convert(ps, count, 1, ptr(out), ptr(ws), M, N, ptr(src), ptr(to), n, current_stream_ptr()), "sums")
+    assert torch.equal(out, torch.stack([t.float().sum(0) for t in dys]))
+    assert torch.equal(to[:n], src.float()) and bool((to[n:] == 7.0).all())
+
+
 @pytest.mark.parametrize("B,L,N", [(1, 1, 4), (2, 257, 64), (6, 33, 20), (4, 1024, 128), (3, 50, 6)])
 def test_masked_rows_and_means_over_sequences(B, L, N):
     """Same bits as the framework's operators, values and gradients: gradient with one row per sequence, in full, strided; a width without
