@@ -87,7 +87,8 @@ int spion_set_head_layout(spion_ctx* ctx, int heads);
 /* Masks of 32 x 32 blocks on the tcgen05 engine (bf16, head_dim 64) have two sets of kernels for the calls that
  * store no probabilities (spion_attn_forward_fused with P_optional == NULL, spion_attn_backward_fused):
  *   1: on the mask's own blocks (up to four selected blocks gathered into one 128-row operand; no unselected
- *      block is ever computed);
+ *      block is ever computed; the forward of calls larger than one wave, full masks aside: two block rows at a
+ *      time on gathered key blocks, a block that only one of them selects being masked for the other);
  *   2: on derived 64 x 64 super-blocks whose unselected quarters are masked (also what serves head_dim 32 and
  *      every call that stores P);
  *   0 (default): chosen when the mask is set -- 1 when the gathered operands are at least 70 % full on
@@ -245,6 +246,14 @@ int spion_discover_patterns(const float* const* host_A, int layers, int L, int b
                             int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
                             int32_t* row_idx, int32_t* csc_pos, int32_t* work, float* mats, int copies,
                             int32_t* host_nnzb, void* cuda_stream);
+/* ... with memory of the caller for the filter's partial sums (8-byte aligned, spion_discover_scratch_bytes(layers, L, block_size) bytes;
+ * NULL: from the library's pool, two more calls of the driver).  Free to reuse in the order of the stream. */
+long long spion_discover_scratch_bytes(int layers, int L, int block_size);
+int spion_discover_patterns_in(const float* const* host_A, int layers, int L, int block_size, int conv_kind, int F, int select,
+                               double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,
+                               int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
+                               int32_t* row_idx, int32_t* csc_pos, int32_t* work, float* mats, int copies,
+                               int32_t* host_nnzb, double* scratch, void* cuda_stream);
 
 /* Block CSR + CSC of a given 0/1 mask (e.g. one loaded from the reference's pickle,
  * main_inference.py:164-166).  Same outputs as above. */

@@ -16,8 +16,10 @@ and the two sibling variants
 Two flavours of the float stages are provided:
 
 * ``pooled_fixed_order``  - the order of additions is fixed (documented below)
-  and carried out in fp64, rounded to fp32 once.  The CUDA kernel uses the
-  same order, so both produce identical bits by construction.
+  and carried out in fp64, rounded to fp32 once.  The general CUDA kernel
+  uses the same order and produces identical bits by construction; the one for
+  the diagonal filter of 31 taps forms the same sums as weighted ones, within
+  some 1e-16 of these before the rounding.
 * ``pooled_torch``        - the reference's own calls (``F.conv2d`` with
   ``padding='same'`` followed by ``F.avg_pool2d``), whose summation order is
   whatever the CPU backend picks.  Used to pin the fixed-order flavour at the

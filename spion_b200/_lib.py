@@ -81,6 +81,8 @@ SIGNATURES = {
     "spion_mean_map_tiles": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "spion_discover_pattern": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_double] + [c_void_p] * 13),
     "spion_discover_patterns": (c_int, [c_void_p] + [c_int] * 6 + [c_double] + [c_void_p] * 12 + [c_int] + [c_void_p] * 2),
+    "spion_discover_scratch_bytes": (c_longlong, [c_int] * 3),
+    "spion_discover_patterns_in": (c_int, [c_void_p] + [c_int] * 6 + [c_double] + [c_void_p] * 12 + [c_int] + [c_void_p] * 3),
     "spion_build_structure": (c_int, [c_void_p, c_int] + [c_void_p] * 10),
     "spion_expand_csr": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "spion_set_pattern": (c_int, [c_void_p, c_void_p]),

@@ -7,6 +7,8 @@
 //
 // Integer outputs equal those of oracle/pattern.py: the float stages are fp64 sums (conv_pool_kernel in the oracle's order of additions, documented at
 // each loop; diag_parts_kernel in another) rounded to fp32 once, and the lerp is fused as there.
+#include <atomic>
+
 #include "common.cuh"
 #include "structure.cuh"
 
@@ -218,13 +220,8 @@ __global__ void __launch_bounds__(BS * DIAG_GROUPS) diag_parts_kernel(const __gr
   }
 }
 
-// A cell: its own block's sum and what the blocks around it have for it, added in a fixed order.
-template <bool BETWEEN>
-__global__ void __launch_bounds__(256) diag_combine_kernel(const double* part, int nb, int total, double area, float* __restrict__ pooled) {
-  next_may_start();
-  wait_for_kernel_before();
-  const int cell = blockIdx.x * 256 + threadIdx.x;
-  if (cell >= total) return;
+// A cell: its own block's sum and what the blocks around it have for it, added in a fixed order.  between: blocks of 64.
+__device__ __forceinline__ float combine_cell(const double* part, int cell, int nb, bool between, double area) {
   const int rest = cell % (nb * nb), r = rest / nb, c = rest - r * nb;
   const bool up = r > 0, down = r + 1 < nb, lt = c > 0, rt = c + 1 < nb;
   const double* p = part + (size_t)cell * DIAG_PARTS;
@@ -232,7 +229,7 @@ __global__ void __launch_bounds__(256) diag_combine_kernel(const double* part, i
   double s = p[0];
   s += rt ? p[DIAG_PARTS + 1] : 0.0;
   s += lt ? p[-DIAG_PARTS + 2] : 0.0;
-  if (BETWEEN) {
+  if (between) {
     s += p[7];
     s += rt ? p[DIAG_PARTS + 8] : 0.0;
     s += lt ? p[-DIAG_PARTS + 9] : 0.0;
@@ -241,19 +238,40 @@ __global__ void __launch_bounds__(256) diag_combine_kernel(const double* part, i
   s += down && rt ? p[line + DIAG_PARTS + 4] : 0.0;
   s += up ? p[-line + 5] : 0.0;
   s += up && lt ? p[-line - DIAG_PARTS + 6] : 0.0;
-  pooled[cell] = (float)(s / area);
+  return (float)(s / area);
+}
+__global__ void __launch_bounds__(256) diag_combine_kernel(const double* part, int nb, int total, bool between, double area, float* __restrict__ pooled) {
+  next_may_start();
+  wait_for_kernel_before();
+  const int cell = blockIdx.x * 256 + threadIdx.x;
+  if (cell < total) pooled[cell] = combine_cell(part, cell, nb, between, area);
+}
+
+// Lets kernel K use `bytes` (always the same) of shared memory on the current device, once: the call is a microsecond or two of a small
+// discovery's 20 on the host.
+template <auto K>
+int allow_smem(int bytes) {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  SPION_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && done[dev].load(std::memory_order_acquire)) return SPION_OK;
+  SPION_CUDA_TRY(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  if (dev < 64) done[dev].store(true, std::memory_order_release);
+  return SPION_OK;
 }
 
 template <int BS>
-int launch_diag(const MapList& maps, int layers, int L, int nb, double* part, float* pooled, cudaStream_t st) {
+int launch_diag(const MapList& maps, int layers, int L, int nb, double* part, float* pooled, bool combine, cudaStream_t st) {
   const int smem = DIAG_GROUPS * 2 * BS * (BS + 4) * (int)sizeof(float), total = layers * nb * nb;
   const int sms = sm_count();
   if (sms < 1) return SPION_ERR_CUDA;
-  SPION_CUDA_TRY(cudaFuncSetAttribute(diag_parts_kernel<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int rc = allow_smem<diag_parts_kernel<BS>>(smem);
+  if (rc) return rc;
   const int ctas = (total + DIAG_GROUPS - 1) / DIAG_GROUPS, cap = (BS == 64 ? 1 : 4) * sms;      // 209 KB or 55 KB each
   diag_parts_kernel<BS><<<ctas < cap ? ctas : cap, BS * DIAG_GROUPS, smem, st>>>(maps, layers, L, part);
   SPION_LAUNCH_CHECK();
-  SPION_CUDA_TRY(launch_after(diag_combine_kernel<BS == 64>, dim3((total + 255) / 256), dim3(256), 0, st, (const double*)part, nb, total, (double)(BS * BS), pooled));
+  if (combine)
+    SPION_CUDA_TRY(launch_after(diag_combine_kernel, dim3((total + 255) / 256), dim3(256), 0, st, (const double*)part, nb, total, BS == 64, (double)(BS * BS), pooled));
   return SPION_OK;
 }
 
@@ -331,6 +349,11 @@ __device__ __forceinline__ float select_kth(const float* vals, int n, int k, int
 // step by step and the mask in global memory; 36 us of selection and 13 us of structure for each of them with one launch per map and
 // step).  copies: how many times the 0/1 float mask is written, `mats_step` floats apart (the driver's stacked list, main_conv_ff.py:298-299).
 constexpr int SELECT_SMEM_CELLS = 128 * 128;           // maps up to this size are kept in shared memory
+// Up to this size select_kernel adds the parts of the cells itself: a launch between the two kernels is 3 us of the host,
+// which is what a small call waits for (one map of 32 x 32 cells 107 us a call with that launch and scratch from the pool, 94 now; two of 64 x 64
+// in blocks of 64: 142, 133 with scratch from the caller alone).  One SM
+// reads the parts slowly, 32 sectors a load: two maps of 64 x 64 cells 142 -> 171 us.
+constexpr int COMBINE_CELLS = 1536;
 constexpr int SELECT_SMEM_BYTES = 7;                   // per cell: value, where a walker goes from it, mask
 struct SelectOut {
   uint8_t* mat;
@@ -340,7 +363,7 @@ struct SelectOut {
   long long mats_step;
 };
 template <bool SMALL>                                  // up to SELECT_SMEM_CELLS
-__global__ void __launch_bounds__(1024) select_kernel(const float* pooled_all, int nb, int select, float q,
+__global__ void __launch_bounds__(1024) select_kernel(float* pooled_all, const double* part, bool between, double area, int nb, int select, float q,
                                                       int kcount, const __grid_constant__ SelectOut out) {
   extern __shared__ float s_val[];
   __shared__ int hist[1024];
@@ -359,9 +382,14 @@ __global__ void __launch_bounds__(1024) select_kernel(const float* pooled_all, i
   for (int i = threadIdx.x; i < n; i += 1024) mat[i] = 0;
   wait_for_kernel_before();
   if (SMALL) {
-    const float* from = pooled_all + blockIdx.x * cells;
+    float* from = pooled_all + blockIdx.x * cells;
+    if (part) {
+#pragma unroll 2
+      for (int i = threadIdx.x; i < n; i += 1024) from[i] = s_val[i] = combine_cell(part, blockIdx.x * n + i, nb, between, area);
+    } else {
 #pragma unroll 4
-    for (int i = threadIdx.x; i < n; i += 1024) s_val[i] = from[i];
+      for (int i = threadIdx.x; i < n; i += 1024) s_val[i] = from[i];
+    }
   }
   __syncthreads();
 
@@ -610,11 +638,28 @@ extern "C" int spion_mean_map_tiles(const void* P, int dtype, const int32_t* blk
   return SPION_OK;
 }
 
+// Bytes of scratch that spion_discover_patterns_in can be given (per call of `layers` maps).
+extern "C" long long spion_discover_scratch_bytes(int layers, int L, int block_size) {
+  if (layers < 1 || L < 1 || block_size < 1) return 0;
+  const long long nb = L / block_size;
+  return layers * nb * nb * DIAG_PARTS * (long long)sizeof(double);
+}
+
 extern "C" int spion_discover_patterns(const float* const* host_A, int layers, int L, int block_size, int conv_kind, int F, int select,
                                        double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,
                                        int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
                                        int32_t* row_idx, int32_t* csc_pos, int32_t* work, float* mats, int copies,
                                        int32_t* host_nnzb, void* cuda_stream) {
+  return spion_discover_patterns_in(host_A, layers, L, block_size, conv_kind, F, select, param, mat, pooled, thresh, nnzb, row_ptr, col_idx,
+                                    blk_row, col_ptr, row_idx, csc_pos, work, mats, copies, host_nnzb, nullptr, cuda_stream);
+}
+
+// ... with the partial sums of the filter in memory of the caller (8-byte aligned, spion_discover_scratch_bytes; NULL: the library's pool)
+extern "C" int spion_discover_patterns_in(const float* const* host_A, int layers, int L, int block_size, int conv_kind, int F, int select,
+                                          double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,
+                                          int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row, int32_t* col_ptr,
+                                          int32_t* row_idx, int32_t* csc_pos, int32_t* work, float* mats, int copies,
+                                          int32_t* host_nnzb, double* scratch, void* cuda_stream) {
   if (!host_A || layers < 1 || layers > 16 || copies < 0 || (copies > 0 && !mats)) return SPION_ERR_ARG;
   MapList maps = {};
   for (int i = 0; i < layers; ++i) { maps.A[i] = host_A[i]; if (!host_A[i]) return SPION_ERR_ARG; }
@@ -638,11 +683,14 @@ extern "C" int spion_discover_patterns(const float* const* host_A, int layers, i
   for (int i = 0; i < layers; ++i) aligned = aligned && ((uintptr_t)host_A[i] & 15u) == 0;
   // the reference's filter takes the kernel above; without memory for its partial sums the general one answers
   double* part = nullptr;
-  const bool diag = conv_kind == SPION_CONV_DIAG && F == 31 && (bs == 64 || bs == 32) && aligned &&
-                    scratch_alloc((void**)&part, layers * cells * DIAG_PARTS * sizeof(double), st) == SPION_OK;
+  const bool fits = conv_kind == SPION_CONV_DIAG && F == 31 && (bs == 64 || bs == 32) && aligned;
+  const bool given = fits && scratch && ((uintptr_t)scratch & 7) == 0;
+  if (given) part = scratch;
+  const bool diag = fits && (given || scratch_alloc((void**)&part, layers * cells * DIAG_PARTS * sizeof(double), st) == SPION_OK);
+  const bool alone = diag && cells > COMBINE_CELLS;                 // the parts of a cell by a kernel of their own
   if (diag) {
-    const int rc = bs == 64 ? launch_diag<64>(maps, layers, L, nb, part, pooled, st) : launch_diag<32>(maps, layers, L, nb, part, pooled, st);
-    if (rc) { scratch_free(part, st); return rc; }
+    const int rc = bs == 64 ? launch_diag<64>(maps, layers, L, nb, part, pooled, alone, st) : launch_diag<32>(maps, layers, L, nb, part, pooled, alone, st);
+    if (rc) { if (!given) scratch_free(part, st); return rc; }
   } else {
     if (smem > 48 * 1024)
       SPION_CUDA_TRY(cudaFuncSetAttribute(conv_pool_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -657,10 +705,13 @@ extern "C" int spion_discover_patterns(const float* const* host_A, int layers, i
   const bool small = cells <= SELECT_SMEM_CELLS;
   auto kernel = small ? select_kernel<true> : select_kernel<false>;
   const size_t dyn = small ? cells * SELECT_SMEM_BYTES : 0;
-  if (small) SPION_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SELECT_SMEM_CELLS * SELECT_SMEM_BYTES));
+  if (small) {
+    const int rc = allow_smem<select_kernel<true>>(SELECT_SMEM_CELLS * SELECT_SMEM_BYTES);
+    if (rc) { if (diag && !given) scratch_free(part, st); return rc; }
+  }
   const SelectOut out{mat, thresh, mats, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, copies, (long long)(layers * cells)};
-  SPION_CUDA_TRY(launch_after(kernel, dim3(layers), dim3(1024), dyn, st, (const float*)pooled, nb, select, (float)param, kcount, out));
-  if (diag) scratch_free(part, st);                    // behind the last kernel: between two of them it would keep the second waiting
+  SPION_CUDA_TRY(launch_after(kernel, dim3(layers), dim3(1024), dyn, st, pooled, (const double*)(diag && !alone ? part : nullptr), bs == 64, (double)(bs * bs), nb, select, (float)param, kcount, out));
+  if (diag && !given) scratch_free(part, st);                    // behind the last kernel: between two of them it would keep the second waiting
   if (host_nnzb) {
     SPION_CUDA_TRY(cudaMemcpyAsync(host_nnzb, nnzb, layers * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     SPION_CUDA_TRY(cudaStreamSynchronize(st));

@@ -9,6 +9,7 @@ the device and also emits the block CSR/CSC the attention kernels use.
 from __future__ import annotations
 
 import pickle
+from contextlib import nullcontext
 from dataclasses import dataclass
 
 import torch
@@ -72,6 +73,7 @@ def discover_pattern(A: torch.Tensor, block_size: int, threshold: float, conv: s
 
 
 _MAPS_PER_CALL = 16
+_SCRATCH_BYTES = int(lib.spion_discover_scratch_bytes(1, 1, 1))      # per cell of a pooled map
 
 
 def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select: str, copies: int):
@@ -93,6 +95,7 @@ def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select
     mat = torch.empty(n, nb, nb, dtype=torch.uint8, device=dev)
     flt = torch.empty(n * cells + n + copies * n * cells, dtype=torch.float32, device=dev)
     ints = torch.empty(n * (5 * cells + 2 * (nb + 1) + 1), dtype=torch.int32, device=dev)
+    scratch = torch.empty(min(n, _MAPS_PER_CALL) * cells * _SCRATCH_BYTES, dtype=torch.uint8, device=dev)
     pf, pi, pm = flt.data_ptr(), ints.data_ptr(), mat.data_ptr()
     int_at, off = {}, 0
     for name, size in (("col_idx", cells), ("blk_row", cells), ("row_idx", cells), ("csc_pos", cells), ("work", cells),
@@ -100,7 +103,7 @@ def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select
         int_at[name] = (off, size)
         off += n * size
     copies_at = n * cells + n
-    with torch.cuda.device(dev):
+    with nullcontext() if torch.cuda.current_device() == dev.index else torch.cuda.device(dev):
         stream = _lib.current_stream_ptr()
         for l0 in range(0, n, _MAPS_PER_CALL):
             m = min(_MAPS_PER_CALL, n - l0)
@@ -108,12 +111,12 @@ def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select
             at = {k: pi + 4 * (o + l0 * size) for k, (o, size) in int_at.items()}
             # the copies of the masks are written in one go when a single call covers the model
             direct = copies if n <= _MAPS_PER_CALL else 0
-            check(lib.spion_discover_patterns(
+            check(lib.spion_discover_patterns_in(
                 ptrs, m, L, block_size, CONV_KINDS[conv], F,
                 _lib.SELECT_PATHS if select == "paths" else _lib.SELECT_TOPK, float(threshold),
                 pm + l0 * cells, pf + 4 * l0 * cells, pf + 4 * (n * cells + l0), at["nnzb"], at["row_ptr"], at["col_idx"], at["blk_row"],
                 at["col_ptr"], at["row_idx"], at["csc_pos"], at["work"], pf + 4 * copies_at if direct else None, direct,
-                None, stream), "spion_discover_patterns")
+                None, scratch.data_ptr(), stream), "spion_discover_patterns_in")
         # views that do not depend on the block counts are made while the kernels run; reading the counts waits for them
         mats = flt[copies_at:].view(copies, n, nb, nb) if copies else None
         if copies and n > _MAPS_PER_CALL:

@@ -167,6 +167,33 @@ def test_discovery_at_the_largest_block_counts(case):
     assert hashlib.sha256(got.tobytes()).digest() == LARGE[case + "/csr_sha"].tobytes()
 
 
+@pytest.mark.parametrize("bs,nb,layers", [(32, 39, 2), (32, 40, 1), (64, 39, 1), (64, 40, 2)])
+def test_cells_by_the_selection_or_by_a_launch_of_their_own(bs, nb, layers):
+    """Either side of the size up to which the selection adds up the cells (1536), with scratch of the caller and from the library's pool: the
+    oracle's pooled values and mask."""
+    import ctypes
+    from spion_b200 import _lib
+    pattern = _pattern_mod()
+    L, cells = bs * nb, nb * nb
+    g = torch.Generator().manual_seed(nb)
+    maps = [torch.softmax(torch.randn(L, L, generator=g) * 2.0, dim=-1) for _ in range(layers)]
+    on_gpu = [A.cuda() for A in maps]
+    got = pattern._discover(on_gpu, bs, 0.9, "diag", 31, "paths", 0)[0]
+    mat = torch.empty(layers, nb, nb, dtype=torch.uint8, device="cuda")
+    pooled = torch.empty(layers, nb, nb, device="cuda")
+    ints = [torch.empty(layers * cells + layers, dtype=torch.int32, device="cuda") for _ in range(8)]
+    n, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work = [t.data_ptr() for t in ints]
+    thresh = torch.empty(layers, device="cuda")
+    ptrs = (ctypes.c_void_p * layers)(*[A.data_ptr() for A in on_gpu])
+    _lib.check(_lib.lib.spion_discover_patterns(ptrs, layers, L, bs, _lib.CONV_DIAG, 31, _lib.SELECT_PATHS, 0.9, mat.data_ptr(), pooled.data_ptr(),
+                                                thresh.data_ptr(), n, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, None, 0, None,
+                                                _lib.current_stream_ptr()), "spion_discover_patterns")
+    for l, A in enumerate(maps):
+        assert np.array_equal(got[l].pooled.cpu().numpy(), opat.pooled_fixed_order(A.numpy(), bs))
+        assert np.array_equal(got[l].mat.cpu().numpy(), opat.discover_block_mask(A.numpy(), bs, 0.9)[0])
+        assert torch.equal(got[l].pooled, pooled[l]) and torch.equal(got[l].mat, mat[l])
+
+
 @pytest.mark.parametrize("bs,nb", [(32, 1), (32, 2), (32, 5), (64, 1), (64, 3), (32, 128), (32, 129)])
 def test_filter_and_selection_at_their_edges(bs, nb):
     """The filter of 31 taps as weighted sums of the map's blocks (one block, borders, odd counts), and the selection on either side of what
