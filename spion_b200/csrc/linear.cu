@@ -243,7 +243,7 @@ template <int EPI> __device__ __forceinline__ void look_up(const float* tab, con
 // its place, and fetch the pre-activations the same way; sequences that are no multiple of 32, and outputs that are added to, keep
 // the stores from registers.  Us, before, with the table above, and with the tiles too: 65536 tokens, 64 x 128, GELU 20.6, 19.2, 17.6; its derivative
 // 31.3, 25.9, 24.6; 524288 tokens 107, 94, 81 and 179, 141, 111; fp32, 262144 tokens, 64 x 192 67, -, 50; 64 x 64 37, -, 30.
-template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16, bool STAGED>
 __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constant__ GemmArgs a, const __grid_constant__ LinMaps maps) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t sbase = smem_u32(smem_raw);
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     const int ostep = G_x * 128, ostep_b = ostep / a.Y.L, ostep_l = ostep - ostep_b * a.Y.L;
     orow.init(a.Y, min(a.T - 1, (int)blockIdx.x * 128 + q * 32 + lane));
     const uint32_t obuf = outs + (uint32_t)(warp - LG_LOADERS - 1) * OWARP, hbuf = obuf + OTILE, hbar = hbars + 8 * (warp - LG_LOADERS - 1);
-    const bool staged = a.staged;
+    const bool staged = STAGED && a.staged;
     uint32_t hpar = 0;
     bool h_due = false;                                  // a copy is on its way to hbuf
     // pre-activations of group g of a tile: staged, a copy into this warp's tile; else registers.  Rows past the last token are zeros.
@@ -1410,10 +1410,12 @@ int opt_in(K k, std::atomic<bool> (&done)[64]) {
   if (dev < 64) done[dev].store(true, std::memory_order_release);
   return SPION_OK;
 }
-template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
+// fp32: a kernel for staged outputs and one without, which small calls take (a tile per CTA: the code of both in one kernel costs them 0.3 of
+// 8 us: a training step of 6144 fp32 tokens 472 -> 467)
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16, bool STAGED = true>
 int prepare_gemm() {
   static std::atomic<bool> done[64];
-  return opt_in(k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>, done);
+  return opt_in(k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, STAGED>, done);
 }
 template <bool DY_BF16, bool X_BF16>
 int prepare_wgrad() {
@@ -1427,8 +1429,9 @@ int prepare_wgrad_fp32() {
 
 template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
 int launch_gemm(GemmArgs& a, const spion_tokens* tok, const spion_tokens* out, size_t smem, cudaStream_t st) {
-  auto k = k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>;
-  int rc = prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
+  const bool plain = SPLIT == 3 && !a.staged;
+  auto k = plain ? k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3> : k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true>;
+  int rc = plain ? prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3>() : prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
   if (rc) return rc;
   LinMaps maps;
   a.tma = A_BF16 ? map_form(tok, a.T) : MAP_NONE;
@@ -1533,7 +1536,9 @@ extern "C" int spion_linear_supported(int in_features, int out_features, int fp3
 extern "C" int spion_linear_prepare(int fp32) {
   int rc;
   if (fp32) {
-    if ((rc = prepare_gemm<3, false, false, EPI_NONE, false>()) || (rc = prepare_gemm<3, false, true, EPI_NONE, false>())) return rc;
+    if ((rc = prepare_gemm<3, false, false, EPI_NONE, false>()) || (rc = prepare_gemm<3, false, true, EPI_NONE, false>()) ||
+        (rc = prepare_gemm<3, false, false, EPI_NONE, false, false>()) || (rc = prepare_gemm<3, false, true, EPI_NONE, false, false>()))
+      return rc;
     return prepare_wgrad_fp32();
   }
   if ((rc = prepare_gemm<1, true, false, EPI_NONE, true>()) || (rc = prepare_gemm<1, false, false, EPI_NONE, true>()) ||
