@@ -88,7 +88,8 @@ int spion_set_head_layout(spion_ctx* ctx, int heads);
  * store no probabilities (spion_attn_forward_fused with P_optional == NULL, spion_attn_backward_fused):
  *   1: on the mask's own blocks (up to four selected blocks gathered into one 128-row operand; no unselected
  *      block is ever computed; the forward of calls larger than one wave, full masks aside: two block rows at a
- *      time on gathered key blocks, a block that only one of them selects being masked for the other);
+ *      time on gathered key blocks, a block that only one of them selects being masked for the other, whatever its
+ *      values: infinities and NaN stay with the rows that select them);
  *   2: on derived 64 x 64 super-blocks whose unselected quarters are masked (also what serves head_dim 32 and
  *      every call that stores P);
  *   0 (default): chosen when the mask is set -- 1 when the gathered operands are at least 70 % full on

@@ -22,7 +22,8 @@
 // 368, 345 us, d 32 -, 312, 292; 256 matrices, L = 4096, d 32, 10 %, padded keys 585, 200, 185; 64 matrices, L = 4096, d 64, 5 % 62, 43.5, 43.
 //
 // SUB: masks of 32-wide blocks.  A unit is two block rows, a tile two key blocks of 32 that one of them selects, wherever they lie (two copies
-// of 32 rows each); quarters that are not selected are left out of the sums.  Random masks fill half of such tiles, a third to a quarter of tiles of 64 keys in
+// of 32 rows each); quarters that are not selected are left out of the sums, and rows that
+// an infinity or a NaN in their values reaches are formed again at the end (redo_rows).  Random masks fill half of such tiles, a third to a quarter of tiles of 64 keys in
 // a row.  Us, forward, before (head_dim 64 the mask's own blocks in transposed products, k_b32; 32 such tiles) and now: 64 matrices, L = 4096, d 64, 2 %
 // 45, 39; 5 % 122, 70; 10 % 208, 119; 30 % 528, 280; 16 matrices, 5 %, padded keys 40, 29; d 32, 5 % 74, 52; 32 matrices, 15 %, padded keys 107, 73.
 // At head_dim 64 the reference follows every new maximum, as the kernel before had it: the largest P of a row is 1, which bf16 has without rounding.  Moved
@@ -57,6 +58,7 @@ template <int D> struct Fs {
 constexpr int PR_TWO = 1, PR_FIRST = 2, PR_END = 4;               // two blocks; first pair of a unit; no pair
 
 struct FsArgs {
+  const __nv_bfloat16 *Q, *K, *V;                                 // SUB: for the rows that are formed again
   __nv_bfloat16* O;
   float* lse;
   const float* keypad;
@@ -65,6 +67,68 @@ struct FsArgs {
   float scale, floor_v;
   int* status;
 };
+
+// SUB: the rows of one arithmetic warp (quadrant q) that are not finite, from the blocks that they select alone.  A tile also holds blocks that only
+// the other row of the pair selects, and P = 0 times an infinity or a NaN in their values is a NaN.  The log-sum-exp is right already: scores
+// that a row does not select are left out, not multiplied.  Plain fp32 by the lanes that own the columns; a call whose values are finite only pays for
+// the test of its outputs.
+template <int D, bool KP>
+__device__ __noinline__ void redo_rows(const FsArgs& a, int first, int step, int total, int q) {
+  const int hf = (threadIdx.x >> 4) & 1, row = q * 16 + (threadIdx.x & 15);
+  Walk u;
+  u.init(UnitMap{a.nb, a.BH, a.by_rank}, a.rec, first, step, total);
+#pragma unroll 1
+  for (; u.valid(); u.shift()) {
+    const int n = u.cur.w;
+    const OpPos pos = op_pos(u.bh, a.L, a.heads, D);
+    auto at = [&](int r) { return (size_t)(pos.row0 + r) * pos.ld + pos.x0; };
+    __nv_bfloat16* dst = a.O + at(u.cur.x * BS + row) + hf * 16;
+    bool bad = false;
+    for (int x = 0; x < D / 2; ++x) bad |= !isfinite(__bfloat162float(dst[(x >> 4) * 32 + (x & 15)]));
+    if (n == 0 || !bad) continue;
+    const uint4* qr = reinterpret_cast<const uint4*>(a.Q + at(u.cur.x * BS + row));
+    const float sc2 = a.scale * LOG2E, lse = a.lse[(size_t)u.bh * a.L + u.cur.x * BS + row];
+    float o[D / 2];
+#pragma unroll
+    for (int x = 0; x < D / 2; ++x) o[x] = 0.f;
+#pragma unroll 1
+    for (int t = 0; t < 2 * n; ++t) {                             // halves of the tiles: blocks of 32 keys
+      const int4 pr = a.pair[u.cur.y + (t >> 2)];
+      const int cols = t & 2 ? pr.y : pr.x, bits = (t & 2 ? pr.w : pr.z) >> ((q >> 1) * 2);
+      if (!((bits >> (t & 1)) & 1)) continue;
+      const int key0 = ((cols >> (16 * (t & 1))) & 0xffff) * 32;
+#pragma unroll 1
+      for (int key = key0; key < key0 + 32; ++key) {
+        const uint4* kr = reinterpret_cast<const uint4*>(a.K + at(key));
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i) {
+          const uint4 x = qr[i], y = kr[i];
+          const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s = fmaf(bf16_hi(xs[e]), bf16_hi(ys[e]), fmaf(bf16_lo(xs[e]), bf16_lo(ys[e]), s));
+        }
+        const float pen = KP ? a.keypad[(size_t)u.bh * a.L + key] * LOG2E : 0.f, p = exp2f(fmaf(s, sc2, -pen) - lse);
+        const __nv_bfloat16* vr = a.V + at(key) + hf * 16;
+#pragma unroll
+        for (int i = 0; i < D / 16; ++i) {                        // eight of this lane's columns
+          const uint4 y = *reinterpret_cast<const uint4*>(vr + (i >> 1) * 32 + (i & 1) * 8);
+          const uint32_t ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            o[8 * i + 2 * e] = fmaf(p, bf16_lo(ys[e]), o[8 * i + 2 * e]);
+            o[8 * i + 2 * e + 1] = fmaf(p, bf16_hi(ys[e]), o[8 * i + 2 * e + 1]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i)
+      *reinterpret_cast<uint4*>(dst + (i >> 1) * 32 + (i & 1) * 8) =
+          make_uint4(pack_bf16(o[8 * i], o[8 * i + 1]), pack_bf16(o[8 * i + 2], o[8 * i + 3]), pack_bf16(o[8 * i + 4], o[8 * i + 5]),
+                     pack_bf16(o[8 * i + 6], o[8 * i + 7]));
+  }
+}
 
 template <int D, bool KP, bool SUB>
 __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -262,6 +326,7 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
     // The finished unit whose rows are still in tensor memory: the products of first entries in lanes 0-15 of every quadrant, of second ones
     // in lanes 16-31.  Lane l gives half of its columns to lane l ^ 16 and takes the other half's from there.
     bool pend = false, pend_two = false;
+    bool redo = false;                                            // SUB: something of this lane's is not finite
     float pend_inv = 0.f;
     __nv_bfloat16* pend_dst = nullptr;
     auto put = [&](__nv_bfloat16* dst, const float (&v)[16]) {
@@ -283,6 +348,12 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
           const float take = __shfl_xor_sync(0xffffffffu, give, 16);
           // one entry: what lanes 16-31 hold was never written
           o[x] = (pend_two ? keep + take : hf ? take : keep) * pend_inv;
+        }
+        if (SUB) {
+          float probe = 0.f;
+#pragma unroll
+          for (int x = 0; x < 16; ++x) probe = fmaf(o[x], 0.f, probe);
+          redo |= !(probe == 0.f);
         }
         put(pend_dst + h * 32 + hf * 16, o);
       }
@@ -425,6 +496,10 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
     if (ok && pend && wait_all(pv_done, (uint32_t)(j - 1), ERR_MMA2_WAIT)) {
       tc_fence_after();
       flush();
+      if (SUB && __any_sync(0xffffffffu, redo)) {
+        __syncwarp();                                             // the rows' sums are one half-warp's
+        redo_rows<D, KP>(a, first, step, total, q);
+      }
     }
   }
   tc_fence_before();
@@ -459,6 +534,7 @@ static int fs_forward(spion_ctx* c, TcState* s, const void* Q, const void* K, co
   int rc;
   if ((rc = make_operand_map(c, s, &mq, Q, D)) || (rc = make_operand_map(c, s, &mk, K, D, rows)) || (rc = make_operand_map(c, s, &mv, V, D, rows))) return rc;
   FsArgs a;
+  a.Q = (const __nv_bfloat16*)Q; a.K = (const __nv_bfloat16*)K; a.V = (const __nv_bfloat16*)V;
   a.O = (__nv_bfloat16*)O; a.lse = lse; a.keypad = keypad;
   a.rec = vw.submask ? s->gather_rec : s->line_rec + SPION_MAX_NB;
   a.pair = vw.submask ? s->gather_pair : s->line_pair + s->line_pair_cap;

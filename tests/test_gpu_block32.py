@@ -205,3 +205,41 @@ def test_two_block_rows_at_a_time(d, keypad, merged):
     O, _, gQ, gK, gV = oatt.sparse_attention(Q.float(), K.float(), V.float(), mat, 32, kp, dO.float())
     for name, a, b in zip(("O", "dQ", "dK", "dV"), (out, q.grad, k.grad, v.grad), (O, gQ, gK, gV)):
         assert rel(a, b) <= REL, f"{name}: {rel(a, b):.3e}"
+
+
+@pytest.mark.parametrize("d,path", [(32, "auto"), (64, "own"), (64, "super")])
+@pytest.mark.parametrize("H", [1, 24])
+@pytest.mark.parametrize("keypad", [False, True])
+def test_values_that_are_not_finite_stay_with_the_rows_that_select_them(d, path, H, keypad):
+    """Infinities and NaN in values of blocks that one row of a super row selects, few matrices and more than one wave of them: the outputs of rows that
+    do not select them are the ones without them, and of those that do only the columns with them are not finite."""
+    from spion_b200 import _lib
+    from spion_b200.native import BlockSparseAttention
+    nb, B = 36, 2
+    L = nb * 32
+    rng = np.random.default_rng(7)
+    mat = (rng.random((nb, nb)) < 0.3).astype(np.uint8)
+    mat[np.arange(nb), np.arange(nb)] = 1
+    mat[6] = 0                                                   # a row without blocks beside one with some
+    mat[:2, 20] = (1, 0)
+    mat[2:4, 20] = (0, 1)
+    kp = None
+    if keypad:
+        kp = torch.ones(B, L)
+        kp[0, L - 100:] = 0
+    Q, K, V, _ = [t.to(torch.bfloat16) for t in synthetic.qkv(d, B, H, L, d)]
+    bad = torch.zeros(B, H, L, d, dtype=torch.bool)
+    clean = V.clone()
+    for n, (b, h, block, key, col) in enumerate([(0, 0, 20, 0, 0), (0, 0, 7, 31, d - 1), (1, H - 1, 13, 5, 17), (1, H - 1, 20, 30, 16), (1, 0, 34, 9, 8)]):
+        V[b, h, block * 32 + key, col] = [float("inf"), float("nan"), float("-inf")][n % 3]
+        clean[b, h, block * 32 + key, col] = 0
+        bad[b, h, :, col] |= torch.from_numpy(np.repeat(mat[:, block], 32).astype(bool))
+    mod = BlockSparseAttention(cfg(B, H, L, d, 32), dtype=torch.bfloat16, keypad=keypad, engine=_lib.ENGINE_TCGEN05, recompute=True, return_probs=False,
+                               block32=path)
+    with torch.no_grad():
+        out, _ = mod(Q.cuda(), K.cuda(), V.cuda(), None if kp is None else kp.cuda(), torch.as_tensor(mat).cuda())
+    mod.check_device_status()
+    out = out.cpu()
+    want = oatt.sparse_attention(Q.float(), K.float(), clean.float(), mat, 32, kp)[0]
+    assert torch.equal(torch.isfinite(out), ~bad)
+    assert rel(torch.where(bad, 0, out.float()), torch.where(bad, 0, want)) <= REL
