@@ -26,8 +26,10 @@
 // an infinity or a NaN in their values reaches are formed again at the end (redo_rows).  Random masks fill half of such tiles, a third to a quarter of tiles of 64 keys in
 // a row.  Us, forward, before (head_dim 64 the mask's own blocks in transposed products, k_b32; 32 such tiles) and now: 64 matrices, L = 4096, d 64, 2 %
 // 45, 39; 5 % 122, 70; 10 % 208, 119; 30 % 528, 280; 16 matrices, 5 %, padded keys 40, 29; d 32, 5 % 74, 52; 32 matrices, 15 %, padded keys 107, 73.
-// At head_dim 64 the reference follows every new maximum, as the kernel before had it: the largest P of a row is 1, which bf16 has without rounding.  Moved
-// by 2^8 only, O is 3 % further from fp64 (2.26e-3 instead of 2.14e-3, before 2.18e-3) and the first three figures 39, 63, 101.
+// Masks that run on their own blocks (head_dim 64): the reference follows every new maximum, as the kernel before had it: the largest P of a row is 1,
+// which bf16 has without rounding.  Moved by 2^8 only, O is 3 % further from fp64 (2.26e-3 instead of 2.14e-3, before 2.18e-3) and the first three
+// figures 39, 63, 101.  On derived super-blocks it moves by 2^8, as it did there: 64 matrices, L = 4096, d 64, tiles of 64 keys, every maximum, now: 5 %
+// 105, 83, 72; 95 % 415, 510, 424; whole 64 x 64 blocks 5 % 54, 63, 55.
 //
 // Every wait is bounded; on a time-out the waiting warp records a code in the status word and the CTA winds down.
 #include "tc_stream.cuh"
@@ -64,7 +66,7 @@ struct FsArgs {
   const float* keypad;
   const int4 *rec, *pair;                                         // block rows and their pairs (k_line_recs; SUB: k_gather_recs)
   int L, BH, nb, heads, by_rank;
-  float scale, floor_v;
+  float scale, floor_v, move_by;                                  // move_by: D == 64 and SUB only
   int* status;
 };
 
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(Fs<D>::THREADS, 1) k_fwd_stream(const __grid_c
     const int q = warp & 3, hf = lane >> 4, row = q * 16 + (lane & 15);
     const uint32_t lS = tS + ((uint32_t)(q * 32) << 16), lP = lS + C::T_P, lO = lS + C::T_O;
     const float sc2 = a.scale * LOG2E, floor2 = a.floor_v * LOG2E, inv_scale = 1.0f / a.scale;
-    constexpr float move_by = SUB && D == 64 ? 0.f : MOVE;
+    const float move_by = SUB && D == 64 ? a.move_by : MOVE;
     bool ok = true;
     // The finished unit whose rows are still in tensor memory: the products of first entries in lanes 0-15 of every quadrant, of second ones
     // in lanes 16-31.  Lane l gives half of its columns to lane l ^ 16 and takes the other half's from there.
@@ -540,6 +542,7 @@ static int fs_forward(spion_ctx* c, TcState* s, const void* Q, const void* K, co
   a.pair = vw.submask ? s->gather_pair : s->line_pair + s->line_pair_cap;
   a.L = c->L; a.BH = c->BH; a.nb = vw.nb; a.heads = c->heads; a.by_rank = order_by_rank(c);
   a.scale = c->scale; a.floor_v = keypad ? 0.0f : -100.0f; a.status = c->status_dev;
+  a.move_by = s->b32 && s->b32_use ? 0.f : MOVE;
   if (keypad) return vw.submask ? fs_launch<D, true, true>(c, s, mq, mk, mv, a) : fs_launch<D, true, false>(c, s, mq, mk, mv, a);
   return vw.submask ? fs_launch<D, false, true>(c, s, mq, mk, mv, a) : fs_launch<D, false, false>(c, s, mq, mk, mv, a);
 }
