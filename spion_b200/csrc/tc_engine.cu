@@ -852,7 +852,11 @@ static int forward_any(spion_ctx* c, const void* Q, const void* K, const void* V
     // resident at once (2 matrices, L = 4096, 5 % 10.4 us, two rows at a time 12.4; 1 matrix, 10 % 14.6, 16.5; 4 matrices, 5 % 16.5, 13.3).
     float* l = lse ? lse : s->lse_ws;
     const bool own = c->nnzb == c->nb * c->nb || (long long)c->BH * c->nb <= (long long)s->sms * s->b32_ctas[0];
-    return own ? b32_forward(c, s, Q, K, V, keypad, O, l) : stream_forward(c, s, Q, K, V, keypad, O, l);
+    if (own) return b32_forward(c, s, Q, K, V, keypad, O, l);
+    prof_mark(c, -1);
+    const int rc = stream_forward(c, s, Q, K, V, keypad, O, l);
+    if (!rc) prof_mark(c, SPION_STAGE_FUSED_FWD);
+    return rc;
   }
   if (P_user && s->super) {
     int rc = ensure_super_ws(c, s);

@@ -243,3 +243,30 @@ def test_values_that_are_not_finite_stay_with_the_rows_that_select_them(d, path,
     want = oatt.sparse_attention(Q.float(), K.float(), clean.float(), mat, 32, kp)[0]
     assert torch.equal(torch.isfinite(out), ~bad)
     assert rel(torch.where(bad, 0, out.float()), torch.where(bad, 0, want)) <= REL
+
+
+@pytest.mark.parametrize("H", [1, 24])
+def test_forward_is_timed_as_a_stage(H):
+    """Few matrices and more than one wave of them: two different kernels, one launch of the forward's stage each."""
+    import ctypes
+    from spion_b200 import _lib
+    from spion_b200._lib import check, lib
+    from spion_b200.native import BlockSparseAttention
+    B, L, d = 2, 36 * 32, 64
+    mat = (np.random.default_rng(1).random((36, 36)) < 0.3).astype(np.uint8)
+    mat[np.arange(36), np.arange(36)] = 1
+    q, k, v, _ = [t.to(torch.bfloat16).cuda() for t in synthetic.qkv(1, B, H, L, d)]
+    mod = BlockSparseAttention(cfg(B, H, L, d, 32), dtype=torch.bfloat16, keypad=False, engine=_lib.ENGINE_TCGEN05, recompute=True, return_probs=False,
+                               block32="own")
+    with torch.no_grad():
+        mod(q, k, v, None, torch.as_tensor(mat).cuda())
+        check(lib.spion_profile_reset(mod.handle))
+        check(lib.spion_profile(mod.handle, 1))
+        mod(q, k, v, None, torch.as_tensor(mat).cuda())
+    total, count = ctypes.c_double(), ctypes.c_longlong()
+    launches = {}
+    for stage in range(_lib.STAGE_COUNT):
+        check(lib.spion_profile_get(mod.handle, stage, ctypes.byref(total), ctypes.byref(count)))
+        launches[lib.spion_stage_name(stage).decode()] = (count.value, total.value > 0)
+    check(lib.spion_profile(mod.handle, 0))
+    assert {n: c for n, c in launches.items() if c[0] and n != lib.spion_stage_name(0).decode()} == {lib.spion_stage_name(11).decode(): (1, True)}
