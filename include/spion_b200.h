@@ -131,7 +131,10 @@ enum {
   SPION_STAGE_BWD_ROW = 12,    /* fused kernels: dP, dS and dQ per block row (P read, dS written) */
   SPION_STAGE_BWD_ROW_RC = 13, /* recompute backward, row side: S, dP, dS on chip, dQ and delta written */
   SPION_STAGE_BWD_COL_RC = 14, /* recompute backward, column side: S, dP, P, dS on chip, dK and dV written */
-  SPION_STAGE_COUNT = 15
+  SPION_STAGE_S_SOFTMAX = 15,  /* dense phase: S and its softmax in one kernel     */
+  SPION_STAGE_DP_SOFTMAX = 16, /* dense phase: dP and dS in one kernel             */
+  SPION_STAGE_DENSE_GRADS = 17, /* dense phase: dQ, dK and dV in one launch        */
+  SPION_STAGE_COUNT = 18
 };
 int spion_profile(spion_ctx* ctx, int enable);
 int spion_profile_get(spion_ctx* ctx, int stage, double* total_ms, long long* launches);

@@ -334,7 +334,8 @@ extern "C" int spion_profile_reset(spion_ctx* c) {
 extern "C" const char* spion_stage_name(int stage) {
   static const char* names[SPION_STAGE_COUNT] = {
       "structure", "sddmm_s", "softmax_fwd", "spmm_o", "sddmm_dp", "softmax_bwd", "spmm_dq", "spmm_dk", "spmm_dv",
-      "fused_dp_ds", "spmm_dkdv", "fused_fwd", "bwd_row", "bwd_row_rc", "bwd_col_rc"};
+      "fused_dp_ds", "spmm_dkdv", "fused_fwd", "bwd_row", "bwd_row_rc", "bwd_col_rc",
+      "sddmm_softmax_fwd", "sddmm_softmax_bwd", "spmm_dqdkdv"};
   return (stage >= 0 && stage < SPION_STAGE_COUNT) ? names[stage] : "?";
 }
 
@@ -495,7 +496,7 @@ static int dense_forward(spion_ctx* c, const float* Q, const float* K, const flo
   int rc = joint ? simt_dense_scores(Q, lo, K, attn, c->BH, c->L, c->d, c->scale, pad, -10.0f, c->stream)
                  : simt_sddmm(SPION_F32, SPION_F32, Q, lo, K, rm, attn, vl, p, c->nnzb, c->BH, c->d, c->stream);
   if (rc) return rc;
-  prof_mark(c, joint ? SPION_STAGE_SOFTMAX_FWD : SPION_STAGE_SDDMM_S);
+  prof_mark(c, joint ? SPION_STAGE_S_SOFTMAX : SPION_STAGE_SDDMM_S);
   if (!joint) {
     rc = softmax_fwd_dense_t(attn, c->BH, c->L, c->scale, pad, -10.0f, c->stream);
     if (rc) return rc;
@@ -520,7 +521,7 @@ static int dense_backward(spion_ctx* c, const float* Q, const float* K, const fl
   int rc = joint ? simt_dense_dscores(dO, lo, V, attn, s3, c->BH, c->L, c->d, c->scale, c->stream)
                  : simt_sddmm(SPION_F32, SPION_F32, dO, lo, V, rm, s1, vl, p, c->nnzb, c->BH, c->d, c->stream);
   if (rc) return rc;
-  prof_mark(c, joint ? SPION_STAGE_SOFTMAX_BWD : SPION_STAGE_SDDMM_DP);
+  prof_mark(c, joint ? SPION_STAGE_DP_SOFTMAX : SPION_STAGE_SDDMM_DP);
   if (!joint) {
     rc = softmax_bwd_dense_t(s1, attn, s3, c->BH, c->L, c->scale, c->stream);
     if (rc) return rc;
@@ -529,7 +530,7 @@ static int dense_backward(spion_ctx* c, const float* Q, const float* K, const fl
   c->launches += joint ? 1 : 2;
   rc = simt_dense_grads(attn, s3, Q, K, dO, lo, dQ, dK, dV, p, c->BH, c->L, c->d, c->stream);
   if (rc != SPION_ERR_UNSUPPORTED) {
-    if (!rc) prof_mark(c, SPION_STAGE_SPMM_DK);
+    if (!rc) prof_mark(c, SPION_STAGE_DENSE_GRADS);
     c->launches += 1;
     return rc;
   }

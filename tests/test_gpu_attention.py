@@ -270,3 +270,32 @@ def test_dense_reference_layout_in_joint_kernels(B, H, L, d, kpm):
     for got, ref in zip((attn, out, *grads), (p64, out64, *want)):
         assert float((got.double() - ref).norm()) <= 2e-6 * float(ref.norm())      # fp32 sums of up to 2112 terms, one ulp 6e-8
     assert float(grads[1].sum(2).abs().max()) <= 1e-5 * float(grads[1].abs().sum(2).max())
+
+
+@pytest.mark.parametrize("B,L,d,stages", [(1, 512, 32, ("sddmm_softmax_fwd", "spmm_o", "sddmm_softmax_bwd", "spmm_dqdkdv")),
+                                          (128, 256, 32, ("sddmm_s", "softmax_fwd", "spmm_o", "sddmm_dp", "softmax_bwd", "spmm_dqdkdv")),
+                                          (1, 96, 32, ("sddmm_s", "softmax_fwd", "spmm_o", "sddmm_dp", "softmax_bwd", "spmm_dq", "spmm_dk", "spmm_dv"))])
+def test_dense_stage_times_name_what_a_launch_holds(B, L, d, stages):
+    """Launches that hold several stages of the dense phase are timed under names of their own, each stage once per pass."""
+    import ctypes
+    from spion_b200 import _lib
+    from spion_b200._lib import check, lib
+    from spion_b200.attention import Attention
+    cfg = {"head_dim": d, "num_head": 1, "max_seq_len": L, "batch_size": B, "block_size": 32, "transformer_dim": d, "task": "lra-image"}
+    layer = Attention(cfg).cuda()
+    handle = layer.attn.attn_func.context().handle
+    q, k, v, do = (torch.randn(B, 1, L, d, device="cuda") for _ in range(4))
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    check(lib.spion_profile_reset(handle))
+    check(lib.spion_profile(handle, 1))
+    out, _ = layer.attn(q, k, v, None)
+    torch.autograd.grad(out, (q, k, v), do)
+    total, count = ctypes.c_double(), ctypes.c_longlong()
+    seen = {}
+    for stage in range(_lib.STAGE_COUNT):
+        check(lib.spion_profile_get(handle, stage, ctypes.byref(total), ctypes.byref(count)))
+        if count.value:
+            seen[lib.spion_stage_name(stage).decode()] = count.value
+    check(lib.spion_profile(handle, 0))
+    assert seen == {n: 1 for n in stages}
