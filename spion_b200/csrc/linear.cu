@@ -158,6 +158,7 @@ struct GemmArgs {
   int parts;                // bf16 gradient of three stacked layers: chunks per layer (0: one accumulator for the whole contraction)
   int tma;                  // bf16 A through maps.m[0 .. 2] (MAP_*)
   int staged;               // outputs (and h) through shared memory and the other maps
+  int table;                // GELU or its derivative by table (which kernel: the host's choice)
   const __nv_bfloat16* h;   // EPI_DGELU: pre-activation [T, N]
   __nv_bfloat16* g;         // EPI_GELU: activation [T, N] (Y receives the pre-activation)
   // What a backward reads in place of the caller's tensors.  262144 tokens of 64 fp32 features: 33 MB written here, 33 MB less read by
@@ -234,6 +235,19 @@ template <int EPI> __device__ __forceinline__ void look_up(const float* tab, con
   }
 }
 
+// From the table, or, where wide weights leave no room for it, from the functions
+template <int EPI, bool TAB> __device__ __forceinline__ void activate(const float* tab, const uint32_t (&w)[8], float (&v)[16]) {
+  if (TAB) {
+    look_up<EPI>(tab, w, v);
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const float x = e & 1 ? bf16_hi(w[e >> 1]) : bf16_lo(w[e >> 1]);
+    v[e] = EPI == EPI_GELU ? gelu(x) : dgelu(x);
+  }
+}
+
 // One persistent CTA per SM over tiles of 128 tokens: warps 0-7 bring 64-feature chunks of A through registers (a chunk of
 // loads in flight while the previous one is converted) into a ring of shared-memory stages, warp 8 issues the MMAs
 // (M = 128, two accumulator buffers in tensor memory), warps 9-16 write finished tiles.  W sits in shared memory for the
@@ -243,7 +257,7 @@ template <int EPI> __device__ __forceinline__ void look_up(const float* tab, con
 // its place, and fetch the pre-activations the same way; sequences that are no multiple of 32, and outputs that are added to, keep
 // the stores from registers.  Us, before, with the table above, and with the tiles too: 65536 tokens, 64 x 128, GELU 20.6, 19.2, 17.6; its derivative
 // 31.3, 25.9, 24.6; 524288 tokens 107, 94, 81 and 179, 141, 111; fp32, 262144 tokens, 64 x 192 67, -, 50; 64 x 64 37, -, 30.
-template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16, bool STAGED>
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16, bool STAGED, bool TAB>
 __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constant__ GemmArgs a, const __grid_constant__ LinMaps maps) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t sbase = smem_u32(smem_raw);
@@ -264,7 +278,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
   float* tab = reinterpret_cast<float*>(smem_raw + (bars + 256u - sbase));
   // staged: a tile of 32 x 32 outputs per writing warp, with GELU two, with its derivative one and one of pre-activations
   constexpr uint32_t OTILE = Y_BF16 ? 2048u : 4096u, OWARP = (EPI == EPI_NONE ? 1u : 2u) * OTILE;
-  const uint32_t outs = (bars + 256u + (EPI != EPI_NONE ? TAB_BYTES : 0u) + 1023u) & ~1023u, hbars = bars + 168;
+  const uint32_t outs = (bars + 256u + (TAB ? TAB_BYTES : 0u) + 1023u) & ~1023u, hbars = bars + 168;
 
   const int ntiles = (a.T + 127) >> 7;
   const int G_x = (int)gridDim.x;
@@ -381,7 +395,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
       }
       bias_ptr[n] = b;
     }
-    if (EPI != EPI_NONE)
+    if (TAB)
       for (uint32_t i = tid; i < 2 * TAB_LEN; i += LG_THREADS)
         tab[i] = tab_value<EPI>(i < TAB_LEN ? TAB_FROM + i : 0x8000u + TAB_FROM + (i - TAB_LEN));
     fence_proxy_async();
@@ -621,7 +635,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             float slope[16];
-            look_up<EPI>(tab, hw[x], slope);
+            activate<EPI, TAB>(tab, hw[x], slope);
 #pragma unroll
             for (int i = 0; i < 16; ++i) f[16 * x + i] = round_bf16(f[16 * x + i]) * slope[i];
           }
@@ -644,7 +658,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
             if (!staged && t < a.T) st_v8(dst + 16 * x, w[x]);
             if (EPI == EPI_GELU) {
               float act[16];
-              look_up<EPI>(tab, w[x], act);
+              activate<EPI, TAB>(tab, w[x], act);
 #pragma unroll
               for (int i = 0; i < 8; ++i) w[x][i] = pack_bf16(act[2 * i], act[2 * i + 1]);
               if (!staged && t < a.T) st_v8(a.g + (size_t)t * a.N + c + 16 * x, w[x]);
@@ -1412,10 +1426,10 @@ int opt_in(K k, std::atomic<bool> (&done)[64]) {
 }
 // fp32: a kernel for staged outputs and one without, which small calls take (a tile per CTA: the code of both in one kernel costs them 0.3 of
 // 8 us: a training step of 6144 fp32 tokens 472 -> 467)
-template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16, bool STAGED = true>
+template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16, bool STAGED = true, bool TAB = EPI != EPI_NONE>
 int prepare_gemm() {
   static std::atomic<bool> done[64];
-  return opt_in(k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, STAGED>, done);
+  return opt_in(k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, STAGED, TAB>, done);
 }
 template <bool DY_BF16, bool X_BF16>
 int prepare_wgrad() {
@@ -1429,9 +1443,12 @@ int prepare_wgrad_fp32() {
 
 template <int SPLIT, bool A_BF16, bool TRANSB, int EPI, bool Y_BF16>
 int launch_gemm(GemmArgs& a, const spion_tokens* tok, const spion_tokens* out, size_t smem, cudaStream_t st) {
-  const bool plain = SPLIT == 3 && !a.staged;
-  auto k = plain ? k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3> : k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true>;
-  int rc = plain ? prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3>() : prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
+  constexpr bool TAB = EPI != EPI_NONE;
+  const bool plain = SPLIT == 3 && !a.staged, functions = TAB && !a.table;
+  auto k = plain ? k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3, TAB>
+                 : functions ? k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true, false> : k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true, TAB>;
+  int rc = plain ? prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3>()
+                 : functions ? prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true, false>() : prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
   if (rc) return rc;
   LinMaps maps;
   a.tma = A_BF16 ? map_form(tok, a.T) : MAP_NONE;
@@ -1541,6 +1558,9 @@ extern "C" int spion_linear_prepare(int fp32) {
       return rc;
     return prepare_wgrad_fp32();
   }
+  if ((rc = prepare_gemm<1, true, false, EPI_GELU, true, true, false>()) || (rc = prepare_gemm<1, false, false, EPI_GELU, true, true, false>()) ||
+      (rc = prepare_gemm<1, true, true, EPI_DGELU, true, true, false>()))
+    return rc;
   if ((rc = prepare_gemm<1, true, false, EPI_NONE, true>()) || (rc = prepare_gemm<1, false, false, EPI_NONE, true>()) ||
       (rc = prepare_gemm<1, true, false, EPI_GELU, true>()) || (rc = prepare_gemm<1, false, false, EPI_GELU, true>()) ||
       (rc = prepare_gemm<1, true, true, EPI_DGELU, true>()) || (rc = prepare_gemm<1, true, true, EPI_NONE, true>()) ||
@@ -1615,12 +1635,17 @@ static int forward(const spion_tokens* X, const float* const* W, const float* co
   size_t smem;
   a.k0 = 0; a.accum = 0; a.parts = 0;
   auto plan = [&]() {
-    return plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, gelu_out ? TAB_BYTES : 0,
+    return plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, a.table ? TAB_BYTES : 0,
                      a.staged ? staged_bytes(gelu_out != nullptr, Y->is_bf16) : 0);
   };
   a.staged = staged_outputs(X, Y, T);
+  a.table = gelu_out != nullptr;
   if (a.staged && !plan()) a.staged = 0;                 // wide weights leave no room for the tiles
-  if (!a.staged && !plan()) return SPION_ERR_UNSUPPORTED;
+  if (!a.staged && !plan()) {                            // ... or for the table (992 and 1024 features)
+    if (!a.table) return SPION_ERR_UNSUPPORTED;
+    a.table = 0;
+    if (!plan()) return SPION_ERR_UNSUPPORTED;
+  }
   cudaStream_t st = (cudaStream_t)cuda_stream;
   if (fp32) return launch_gemm<3, false, false, EPI_NONE, false>(a, X, Y, smem, st);
   if (gelu_out)
@@ -1659,7 +1684,7 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
   a.T = (int)T; a.K = out_features; a.N = in_features;
   a.h = (const __nv_bfloat16*)gelu_in; a.g = nullptr; a.x_copy = nullptr; a.w_copy = nullptr; a.mask = nullptr; a.pen = nullptr;
   size_t smem;
-  a.k0 = 0; a.accum = 0;
+  a.k0 = 0; a.accum = 0; a.table = gelu_in != nullptr;
   a.parts = !fp32 && dX->is_bf16 && nw == 3 ? a.wper / 64 : 0;
   if (a.parts && a.wper % 64) return SPION_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)cuda_stream;
@@ -1676,12 +1701,16 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
     return SPION_OK;
   }
   auto plan = [&]() {
-    return plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, gelu_in ? TAB_BYTES : 0,
+    return plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, a.table ? TAB_BYTES : 0,
                      a.staged ? staged_bytes(gelu_in != nullptr, dX->is_bf16) : 0);
   };
   a.staged = staged_outputs(dY, dX, T);
   if (a.staged && !plan()) a.staged = 0;
-  if (!a.staged && !plan()) return SPION_ERR_UNSUPPORTED;
+  if (!a.staged && !plan()) {
+    if (!a.table) return SPION_ERR_UNSUPPORTED;
+    a.table = 0;
+    if (!plan()) return SPION_ERR_UNSUPPORTED;
+  }
   if (gelu_in)
     return dY->is_bf16 ? launch_gemm<1, true, true, EPI_DGELU, true>(a, dY, dX, smem, st) : launch_gemm<1, false, true, EPI_DGELU, true>(a, dY, dX, smem, st);
   if (dX->is_bf16)

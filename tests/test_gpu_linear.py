@@ -318,6 +318,50 @@ def test_feed_forward_block():
         assert _rel(a.detach(), b.detach()) < 1.5e-2          # a chain of up to four roundings to bf16
 
 
+# widths at which the weights leave no room for the activation's table, few tiles and many; the widest with it
+@pytest.mark.parametrize("T,K,N", [(300, 1024, 64), (300, 992, 96), (20001, 1024, 1024), (19100, 992, 256), (300, 960, 1024), (19100, 960, 64)])
+def test_gelu_of_wide_contractions(T, K, N):
+    assert lib.spion_linear_supported(K, N, 0) and lib.spion_linear_supported(N, K, 0)
+    test_gelu_on_bf16_tokens(T, K, N)
+
+
+def test_gelu_by_table_and_by_functions_are_the_same_bits():
+    """Activation and derivative of all 65536 numbers of bf16, from kernels that look them up (64 features) and that form them (1024).
+    (How far they are from the exact ones: test_gelu_of_every_bf16_number.)"""
+    P, st = ctypes.c_void_p, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    one, ref = lambda t: (P * 3)(t.data_ptr(), None, None), ctypes.byref
+    every = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16)
+    acts, slopes = [], []
+    for K in (64, 1024):
+        N = 64
+        h = every.view(-1, N).view(torch.bfloat16)
+        T = h.shape[0]
+        # derivative: a row of ones times a weight of ones in one feature
+        dY, V, dX = torch.zeros(T, K, device="cuda", dtype=torch.bfloat16), torch.zeros(K, N, device="cuda"), torch.empty_like(h)
+        dY[:, 0] = 1
+        V[0] = 1
+        check(lib.spion_linear_backward_input(ref(_tokens([dY])), one(V), 1, 0, P(h.data_ptr()), ref(_tokens([dX])), T, N, K, st))
+        slopes.append(dX.flatten())
+        # activation: a number per token, in its first feature (an infinity in another column would be a NaN in this one)
+        T = 65536
+        X, W, b = torch.zeros(T, K, device="cuda", dtype=torch.bfloat16), torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda")
+        X[:, 0] = every.view(torch.bfloat16)
+        W[:, 0] = 1
+        Y, G = (torch.empty(T, N, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        check(lib.spion_linear_forward(ref(_tokens([X])), one(W), one(b), 1, 0, ref(_tokens([Y])), P(G.data_ptr()), T, K, N, st))
+        assert bool((Y.view(torch.int16) == Y[:, :1].view(torch.int16)).all()) and bool((G.view(torch.int16) == G[:, :1].view(torch.int16)).all())
+        acts.append((Y[:, 0], G[:, 0]))
+    x = every.view(torch.bfloat16)
+    same = lambda a, b: bool(((a.view(torch.int16) == b.view(torch.int16)) | (torch.isnan(a) & torch.isnan(b))).all())
+    assert same(acts[0][0], acts[1][0]) and same(acts[0][1], acts[1][1]) and same(*slopes)
+    normal = torch.isfinite(x) & (x.abs() >= 2.0 ** -126)
+    assert torch.equal(acts[0][0][normal], x[normal])
+    # a negative infinity times zero is a NaN, in the formulas as in the framework's
+    assert bool(torch.isnan(acts[0][1][torch.isnan(x)]).all()) and float(acts[0][1][x == float("inf")]) == float("inf")
+    assert bool(torch.isnan(acts[0][1][x == float("-inf")])) and bool(torch.isnan(slopes[0][torch.isinf(x) | torch.isnan(x)]).all())
+    assert lib.spion_linear_status(1) == 0
+
+
 @pytest.mark.parametrize("T,K,N", [(1 << 20, 64, 64), (1 << 18, 64, 192), (1 << 17, 256, 1024)])
 def test_weight_gradient_of_many_tokens(T, K, N):
     """fp32: the error does not grow with the number of tokens.  Operands of one sign, so that the result is the sum of magnitudes: at
