@@ -205,36 +205,44 @@ __device__ __forceinline__ float dgelu(float x) {
   return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-// Both are functions of a bf16 number here: the pre-activation, which 17 octaves times 128 numbers of either sign give in all but one of some
-// thousand cases.  A CTA forms these 4352 values once, with the functions above, and looks them up (83 instructions a value before): the
-// outputs are the same bits.  Numbers outside, NaN among them, are passed to the functions.
-constexpr uint32_t TAB_FROM = 0x3880u, TAB_LEN = 0x4100u - TAB_FROM;          // 2^-14 .. 8, as bits of a bf16 number without its sign
-constexpr uint32_t TAB_BYTES = 2 * TAB_LEN * 4;
-__device__ __noinline__ float gelu_any(float x) { return gelu(x); }
-__device__ __noinline__ float dgelu_any(float x) { return dgelu(x); }
-template <int EPI> __device__ __forceinline__ float tab_value(uint32_t bits) {
-  const float x = __uint_as_float(bits << 16);
-  return EPI == EPI_GELU ? gelu_any(x) : dgelu_any(x);
-}
-// sixteen at a time: all reads first, a branch for the numbers outside only where there are any (one for each value took longer than the
-// functions)
+// Both are functions of a bf16 number here, the pre-activation: x / 2 times 1 + erf, and the slope.  A CTA forms the factor, or the slope, of every
+// number of a range of octaves once, with the functions above, and looks them up (83 instructions a value before): the outputs are the same bits.
+// Outside of the range they are constants.  GELU: below 2^-9 x / 2 is what the activation rounds to (1 + erf is 0.8 2^-9 beside 1 at most, half a step
+// of bf16 2^-9 at least), from 8 on erf is 1 to fp32.  Slope: from 16 on the exponential is zero; numbers below 2^-14, where erf is the first term of its series
+// and the exponential 1, take a branch with the infinities and NaN.  65536 tokens, 64 x 64, functions, table: GELU 14.4 us, 12.4 for pre-activations of
+// deviation 8, 1 and 0; its derivative 18.5, 16.4, of deviations 2^-17 and 0 too (with a call of the functions for every number outside of a table of
+// 2^-14 to 8: 26.7, 14.0, 25.6; 36.9, 16.4, 34.9).
+template <int EPI> struct Tab {
+  static constexpr bool SLOPE = EPI == EPI_DGELU;
+  static constexpr uint32_t FROM = SLOPE ? 0x3880u : 0x3b00u - 1u, END = SLOPE ? 0x4180u : 0x4100u;          // first and last, bits of a number without its sign
+  static constexpr uint32_t LEN = END - FROM + 1, BYTES = 2 * LEN * 4;
+  __device__ static __forceinline__ float entry(uint32_t i) {
+    const uint32_t k = i < LEN ? i : i - LEN;
+    const float x = __uint_as_float(((i < LEN ? 0u : 0x8000u) | (FROM + k)) << 16);
+    return SLOPE ? dgelu(x) : k == 0 ? 1.0f : 1.0f + erff(x * 0.70710678118654752f);
+  }
+};
 template <int EPI> __device__ __forceinline__ void look_up(const float* tab, const uint32_t (&w)[8], float (&v)[16]) {
-  bool out = false;
+  using T = Tab<EPI>;
+  bool some = false;
 #pragma unroll
   for (int e = 0; e < 16; ++e) {
-    const uint32_t bits = e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu, i = (bits & 0x7fffu) - TAB_FROM;
-    out |= i >= TAB_LEN;
-    v[e] = tab[min(i, TAB_LEN - 1) + ((bits >> 15) * TAB_LEN)];
+    const uint32_t bits = e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu, size = bits & 0x7fffu;
+    if (T::SLOPE) {
+      v[e] = tab[min(size - T::FROM, T::LEN - 1) + (bits >> 15) * T::LEN];
+      some |= ((size + 0x80u) & 0x7fffu) < T::FROM + 0x80u;
+    } else {
+      v[e] = 0.5f * (e & 1 ? bf16_hi(w[e >> 1]) : bf16_lo(w[e >> 1])) * tab[min(max(size, T::FROM), T::END) - T::FROM + (bits >> 15) * T::LEN];
+    }
   }
-  if (out) {
+  if (T::SLOPE && some) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
-      const uint32_t bits = e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu;
-      if ((bits & 0x7fffu) - TAB_FROM >= TAB_LEN) v[e] = tab_value<EPI>(bits);
+      const float x = e & 1 ? bf16_hi(w[e >> 1]) : bf16_lo(w[e >> 1]), c = 0.39894228040143268f;         // 1 / sqrt(2 pi): each summand's slope at 0
+      v[e] = fabsf(x) < 0x1p-14f ? fmaf(c, x, fmaf(c, x, 0.5f)) : fmaf(x, 0.f, v[e]);
     }
   }
 }
-
 // From the table, or, where wide weights leave no room for it, from the functions
 template <int EPI, bool TAB> __device__ __forceinline__ void activate(const float* tab, const uint32_t (&w)[8], float (&v)[16]) {
   if (TAB) {
@@ -278,7 +286,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
   float* tab = reinterpret_cast<float*>(smem_raw + (bars + 256u - sbase));
   // staged: a tile of 32 x 32 outputs per writing warp, with GELU two, with its derivative one and one of pre-activations
   constexpr uint32_t OTILE = Y_BF16 ? 2048u : 4096u, OWARP = (EPI == EPI_NONE ? 1u : 2u) * OTILE;
-  const uint32_t outs = (bars + 256u + (TAB ? TAB_BYTES : 0u) + 1023u) & ~1023u, hbars = bars + 168;
+  const uint32_t outs = (bars + 256u + (TAB ? Tab<EPI>::BYTES : 0u) + 1023u) & ~1023u, hbars = bars + 168;
 
   const int ntiles = (a.T + 127) >> 7;
   const int G_x = (int)gridDim.x;
@@ -396,8 +404,7 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
       bias_ptr[n] = b;
     }
     if (TAB)
-      for (uint32_t i = tid; i < 2 * TAB_LEN; i += LG_THREADS)
-        tab[i] = tab_value<EPI>(i < TAB_LEN ? TAB_FROM + i : 0x8000u + TAB_FROM + (i - TAB_LEN));
+      for (uint32_t i = tid; i < 2 * Tab<EPI>::LEN; i += LG_THREADS) tab[i] = Tab<EPI>::entry(i);
     fence_proxy_async();
   }
   tc_fence_before();
@@ -1635,7 +1642,7 @@ static int forward(const spion_tokens* X, const float* const* W, const float* co
   size_t smem;
   a.k0 = 0; a.accum = 0; a.parts = 0;
   auto plan = [&]() {
-    return plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, a.table ? TAB_BYTES : 0,
+    return plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, a.table ? Tab<EPI_GELU>::BYTES : 0,
                      a.staged ? staged_bytes(gelu_out != nullptr, Y->is_bf16) : 0);
   };
   a.staged = staged_outputs(X, Y, T);
@@ -1701,7 +1708,7 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
     return SPION_OK;
   }
   auto plan = [&]() {
-    return plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, a.table ? TAB_BYTES : 0,
+    return plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, a.table ? Tab<EPI_DGELU>::BYTES : 0,
                      a.staged ? staged_bytes(gelu_in != nullptr, dX->is_bf16) : 0);
   };
   a.staged = staged_outputs(dY, dX, T);
