@@ -1421,6 +1421,34 @@ bool plan_gemm(int split, bool trans, int K, int N, int* nc, int* nacc, int* sta
   return false;
 }
 
+// The table of the activation and the tiles of the outputs take shared memory from the weights: fewer columns per CTA, so that A is fetched once more
+// for every further slice of them.  `worth`: values of A per token that may be fetched again for the cheaper epilogue (FREE: any number).  65536 and 200000
+// tokens, widths of 32 to 1024, time with both ÷ without where the columns get fewer:
+//   fp32 0.68 - 0.88, derivative of GELU 0.40 - 0.77
+//   GELU: bf16 tokens 0.57 - 0.85 up to 384 features, 0.85 - 1.45 from 512 on (the table alone, where that leaves the columns, 0.75 - 0.97);
+//         fp32 tokens 0.70 - 0.88 at 256 features, 0.83 - 1.15 at 320 and 384, 0.95 - 1.48 from 512 on
+//   fp32 gradients of bf16 ones: up to one value of A for every output 0.75 - 1.0 (320 features), 0.85 - 1.09 (384; 0.91 at most up to 3 / 4); beyond 1.0 - 1.5
+//   else, bf16 outputs: forward 0.91 - 1.01 up to half a value at 256 features, 0.98 - 1.6 else; gradients 0.96 - 1.54
+// 65536 tokens, bf16, us, before there were tiles, always with both, now: 512 x 512 57, 78, 57; 768 x 768 143, 202, 142; gradient of 512 x 512 75, 105, 75; GELU
+// of 768 x 768 170, 213, 175.
+constexpr long long FREE = 1LL << 40;
+template <class PLAN>
+bool choose_epilogue(GemmArgs& a, int epi, bool stage, size_t outs, long long worth, PLAN plan) {
+  const size_t table = epi == EPI_GELU ? Tab<EPI_GELU>::BYTES : epi == EPI_DGELU ? Tab<EPI_DGELU>::BYTES : 0;
+  auto slices = [&]() { return (long long)((a.N + a.nc - 1) / a.nc); };
+  a.table = a.staged = 0;
+  if (!plan(0, 0)) return false;
+  const long long fewest = slices();
+  const bool options[3][2] = {{true, true}, {true, false}, {false, true}};       // (the kernels that form the activation have no tiles)
+  for (const auto& [t, o] : options) {
+    if ((t && !table) || (o && !stage) || (o && !t && table) || !plan(t ? table : 0, o ? outs : 0) || (slices() - fewest) * a.K > worth) continue;
+    a.table = t;
+    a.staged = o;
+    return true;
+  }
+  return plan(0, 0);
+}
+
 // Shared-memory opt-in of a kernel, once per device; the call also loads the kernel.  `done` belongs to the kernel.
 template <class K>
 int opt_in(K k, std::atomic<bool> (&done)[64]) {
@@ -1453,9 +1481,9 @@ int launch_gemm(GemmArgs& a, const spion_tokens* tok, const spion_tokens* out, s
   constexpr bool TAB = EPI != EPI_NONE;
   const bool plain = SPLIT == 3 && !a.staged, functions = TAB && !a.table;
   auto k = plain ? k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3, TAB>
-                 : functions ? k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true, false> : k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true, TAB>;
+                 : functions ? k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, EPI == EPI_NONE, false> : k_lin_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true, TAB>;
   int rc = plain ? prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, SPLIT != 3>()
-                 : functions ? prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, true, false>() : prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
+                 : functions ? prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16, EPI == EPI_NONE, false>() : prepare_gemm<SPLIT, A_BF16, TRANSB, EPI, Y_BF16>();
   if (rc) return rc;
   LinMaps maps;
   a.tma = A_BF16 ? map_form(tok, a.T) : MAP_NONE;
@@ -1565,8 +1593,8 @@ extern "C" int spion_linear_prepare(int fp32) {
       return rc;
     return prepare_wgrad_fp32();
   }
-  if ((rc = prepare_gemm<1, true, false, EPI_GELU, true, true, false>()) || (rc = prepare_gemm<1, false, false, EPI_GELU, true, true, false>()) ||
-      (rc = prepare_gemm<1, true, true, EPI_DGELU, true, true, false>()))
+  if ((rc = prepare_gemm<1, true, false, EPI_GELU, true, false, false>()) || (rc = prepare_gemm<1, false, false, EPI_GELU, true, false, false>()) ||
+      (rc = prepare_gemm<1, true, true, EPI_DGELU, true, false, false>()))
     return rc;
   if ((rc = prepare_gemm<1, true, false, EPI_NONE, true>()) || (rc = prepare_gemm<1, false, false, EPI_NONE, true>()) ||
       (rc = prepare_gemm<1, true, false, EPI_GELU, true>()) || (rc = prepare_gemm<1, false, false, EPI_GELU, true>()) ||
@@ -1641,18 +1669,12 @@ static int forward(const spion_tokens* X, const float* const* W, const float* co
   a.mask = mask; a.pen = pen; a.pen_heads = heads; a.pen_L = seq_len;
   size_t smem;
   a.k0 = 0; a.accum = 0; a.parts = 0;
-  auto plan = [&]() {
-    return plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, a.table ? Tab<EPI_GELU>::BYTES : 0,
-                     a.staged ? staged_bytes(gelu_out != nullptr, Y->is_bf16) : 0);
-  };
-  a.staged = staged_outputs(X, Y, T);
-  a.table = gelu_out != nullptr;
-  if (a.staged && !plan()) a.staged = 0;                 // wide weights leave no room for the tiles
-  if (!a.staged && !plan()) {                            // ... or for the table (992 and 1024 features)
-    if (!a.table) return SPION_ERR_UNSUPPORTED;
-    a.table = 0;
-    if (!plan()) return SPION_ERR_UNSUPPORTED;
-  }
+  const int most = X->is_bf16 ? 384 : 256;
+  if (!choose_epilogue(a, gelu_out ? EPI_GELU : EPI_NONE, staged_outputs(X, Y, T), staged_bytes(gelu_out != nullptr, Y->is_bf16),
+                       fp32 ? FREE : gelu_out ? (a.K <= most ? FREE : 0) : Y->is_bf16 && a.K <= 256 ? a.N / 2 : 0, [&](size_t table, size_t outs) {
+                         return plan_gemm(fp32 ? 3 : 1, false, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, table, outs);
+                       }))
+    return SPION_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)cuda_stream;
   if (fp32) return launch_gemm<3, false, false, EPI_NONE, false>(a, X, Y, smem, st);
   if (gelu_out)
@@ -1691,7 +1713,7 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
   a.T = (int)T; a.K = out_features; a.N = in_features;
   a.h = (const __nv_bfloat16*)gelu_in; a.g = nullptr; a.x_copy = nullptr; a.w_copy = nullptr; a.mask = nullptr; a.pen = nullptr;
   size_t smem;
-  a.k0 = 0; a.accum = 0; a.table = gelu_in != nullptr;
+  a.k0 = 0; a.accum = 0;
   a.parts = !fp32 && dX->is_bf16 && nw == 3 ? a.wper / 64 : 0;
   if (a.parts && a.wper % 64) return SPION_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)cuda_stream;
@@ -1700,24 +1722,20 @@ extern "C" int spion_linear_backward_input(const spion_tokens* dY, const float* 
     for (a.k0 = 0; a.k0 < total; a.k0 += step) {
       a.K = total - a.k0 < step ? total - a.k0 : step;
       a.accum = a.k0 > 0;
-      a.staged = total <= step && staged_outputs(dY, dX, T) && plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, 0, staged_bytes(false, false));
-      if (!a.staged && !plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem)) return SPION_ERR_UNSUPPORTED;
+      if (!choose_epilogue(a, EPI_NONE, total <= step && staged_outputs(dY, dX, T), staged_bytes(false, false), FREE, [&](size_t, size_t outs) {
+            return plan_gemm(3, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, 256, 0, outs);
+          }))
+        return SPION_ERR_UNSUPPORTED;
       const int rc = launch_gemm<3, false, true, EPI_NONE, false>(a, dY, dX, smem, st);
       if (rc) return rc;
     }
     return SPION_OK;
   }
-  auto plan = [&]() {
-    return plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, a.table ? Tab<EPI_DGELU>::BYTES : 0,
-                     a.staged ? staged_bytes(gelu_in != nullptr, dX->is_bf16) : 0);
-  };
-  a.staged = staged_outputs(dY, dX, T);
-  if (a.staged && !plan()) a.staged = 0;
-  if (!a.staged && !plan()) {
-    if (!a.table) return SPION_ERR_UNSUPPORTED;
-    a.table = 0;
-    if (!plan()) return SPION_ERR_UNSUPPORTED;
-  }
+  if (!choose_epilogue(a, gelu_in ? EPI_DGELU : EPI_NONE, staged_outputs(dY, dX, T), staged_bytes(gelu_in != nullptr, dX->is_bf16),
+                       gelu_in ? FREE : dY->is_bf16 && !dX->is_bf16 ? (a.K <= 320 ? a.N : a.N * 3 / 4) : 0, [&](size_t table, size_t outs) {
+                         return plan_gemm(1, true, a.K, a.N, &a.nc, &a.nacc, &a.nstages, &smem, a.parts ? 64 : 256, table, outs);
+                       }))
+    return SPION_ERR_UNSUPPORTED;
   if (gelu_in)
     return dY->is_bf16 ? launch_gemm<1, true, true, EPI_DGELU, true>(a, dY, dX, smem, st) : launch_gemm<1, false, true, EPI_DGELU, true>(a, dY, dX, smem, st);
   if (dX->is_bf16)

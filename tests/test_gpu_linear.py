@@ -414,3 +414,36 @@ def test_values_that_are_not_finite_in_bf16(split):
         huge, usual = sure & want.isfinite() & (want.abs() > 1e30), sure & (want.abs() <= 1e30)
         assert ((got - want).abs()[huge] <= 1e-6 * want.abs()[huge]).all()
         assert ((got - want)[usual].norm() <= 2e-6 * want[usual].norm())
+
+
+@pytest.mark.parametrize("kind,K,N,slices", [("forward", 512, 512, 4), ("forward", 384, 192, 1), ("forward", 768, 96, 1), ("gelu", 640, 96, 1), ("gelu", 768, 384, 4),
+                                             ("gradient", 512, 512, 4), ("gradient", 256, 1024, 4), ("gradient_fp32", 512, 256, 2)])
+def test_wide_layers_keep_their_columns(kind, K, N, slices):
+    """Tables and tiles of the outputs leave wide weights the columns that fit beside a ring alone: A is fetched once per slice of them."""
+    import json
+    import os
+    import tempfile
+    T = 149 * 128
+    P, st = ctypes.c_void_p, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    one, ref = lambda t: (P * 3)(t.data_ptr(), None, None), ctypes.byref
+    X = torch.zeros(T, K, device="cuda", dtype=torch.bfloat16)
+    Y = torch.empty(T, N, device="cuda", dtype=torch.float32 if kind == "gradient_fp32" else torch.bfloat16)
+    G, W, b = torch.empty(T, N, device="cuda", dtype=torch.bfloat16), torch.zeros(N * K, device="cuda"), torch.zeros(N, device="cuda")
+
+    def call():
+        if kind.startswith("gradient"):
+            check(lib.spion_linear_backward_input(ref(_tokens([X])), one(W), 1, 0, None, ref(_tokens([Y])), T, N, K, st))
+        else:
+            check(lib.spion_linear_forward(ref(_tokens([X])), one(W), one(b), 1, 0, ref(_tokens([Y])), P(G.data_ptr()) if kind == "gelu" else None, T, K, N, st))
+
+    call()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    with tempfile.TemporaryDirectory() as d:
+        path = os.path.join(d, "trace.json")
+        prof.export_chrome_trace(path)
+        with open(path) as f:
+            grids = [e["args"]["grid"] for e in json.load(f)["traceEvents"] if "k_lin_gemm" in e.get("name", "")]
+    assert len(grids) == 1 and grids[0][1] == slices
