@@ -534,10 +534,11 @@ __global__ void __launch_bounds__(LG_THREADS, 1) k_lin_gemm(const __grid_constan
     const int ngroups = nc >> 5;
     int j = 0;
     if (!TRANSB && a.pen) {                              // spion_expand_keypad, in the time that the first tile takes
-      const int n = a.T * a.pen_heads, all = (int)(gridDim.x * gridDim.y) * 256;
-      for (int i = ((int)(blockIdx.y * gridDim.x + blockIdx.x)) * 256 + tid - 32 * (LG_LOADERS + 1); i < n; i += all) {
-        const int bh = i / a.pen_L;
-        a.pen[i] = 1e6f * (1.0f - a.mask[(bh / a.pen_heads) * a.pen_L + (i - bh * a.pen_L)]);
+      // unsigned: up to 2^31 - 1 of them, and the last step of a thread goes past that
+      const unsigned n = (unsigned)a.T * (unsigned)a.pen_heads, all = gridDim.x * gridDim.y * 256u, len = (unsigned)a.pen_L;
+      for (unsigned i = (blockIdx.y * gridDim.x + blockIdx.x) * 256u + (unsigned)(tid - 32 * (LG_LOADERS + 1)); i < n; i += all) {
+        const unsigned bh = i / len;
+        a.pen[i] = 1e6f * (1.0f - a.mask[bh / (unsigned)a.pen_heads * len + (i - bh * len)]);
       }
     }
     RowIt orow;

@@ -190,6 +190,26 @@ def test_projections_with_the_penalties_of_padded_keys(B, L, heads, fp32):
                                            P(pen.data_ptr()), st) != 0
 
 
+def test_penalties_up_to_the_largest_count():
+    """2^31 - 2 penalties, two less than an int holds: what a thread would write next lies beyond that."""
+    P = ctypes.c_void_p
+    B, L, heads = 62, 49981, 693                                 # B L heads = 2^31 - 2
+    T, K, N = B * L, 32, 32
+    assert T * heads == 2 ** 31 - 2
+    X, W, b = torch.zeros(T, K, dtype=torch.bfloat16, device="cuda"), torch.zeros(N, K, device="cuda"), torch.zeros(N, device="cuda")
+    Y = torch.empty(T, N, dtype=torch.bfloat16, device="cuda")
+    mask = (torch.rand(B, L, device="cuda") < 0.7).float()
+    pen = torch.full((T * heads + 65536,), -1.0, device="cuda")
+    one, ref = lambda t: (P * 3)(t.data_ptr(), None, None), ctypes.byref
+    check(lib.spion_linear_forward_keypad(ref(_tokens([X])), one(W), one(b), 1, 0, ref(_tokens([Y])), None, None, T, K, N, P(mask.data_ptr()), B, heads, L,
+                                          P(pen.data_ptr()), P(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    assert bool((pen[T * heads:] == -1.0).all())
+    rows = pen[:T * heads].view(B, heads, L)
+    for i in range(B):
+        assert bool((rows[i] == 1e6 * (1 - mask[i])).all())
+
+
 @pytest.mark.parametrize("T,K,N", [(19000, 64, 128), (20001, 32, 96), (300, 64, 64)])
 def test_gelu_of_every_bf16_number(T, K, N):
     """Activation and its derivative by table, inside and outside of its range (subnormals, infinities and NaN too), the outputs through tiles in
