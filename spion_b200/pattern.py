@@ -76,6 +76,15 @@ _MAPS_PER_CALL = 16
 _SCRATCH_BYTES = int(lib.spion_discover_scratch_bytes(1, 1, 1))      # per cell of a pooled map
 
 
+def _scratch(cells: int, device):
+    """Memory for the partial sums of the filter that has them (the diagonal one of 31 taps on blocks of 32 or 64).  None where there is
+    none: the library then looks in its own pool, and without memory there the general kernel, which needs none, answers."""
+    try:
+        return torch.empty(cells * _SCRATCH_BYTES, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select: str, copies: int):
     """Patterns of several equally large maps (one call of the library per 16: every stage runs over all of them, one host
     synchronisation) and ``copies`` stacked copies of their masks as [copies, maps, nb, nb] floats (None for 0)."""
@@ -95,7 +104,7 @@ def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select
     mat = torch.empty(n, nb, nb, dtype=torch.uint8, device=dev)
     flt = torch.empty(n * cells + n + copies * n * cells, dtype=torch.float32, device=dev)
     ints = torch.empty(n * (5 * cells + 2 * (nb + 1) + 1), dtype=torch.int32, device=dev)
-    scratch = torch.empty(min(n, _MAPS_PER_CALL) * cells * _SCRATCH_BYTES, dtype=torch.uint8, device=dev)
+    scratch = _scratch(min(n, _MAPS_PER_CALL) * cells, dev) if conv == "diag" and F == 31 and block_size in (32, 64) else None
     pf, pi, pm = flt.data_ptr(), ints.data_ptr(), mat.data_ptr()
     int_at, off = {}, 0
     for name, size in (("col_idx", cells), ("blk_row", cells), ("row_idx", cells), ("csc_pos", cells), ("work", cells),
@@ -116,7 +125,7 @@ def _discover(maps, block_size: int, threshold: float, conv: str, F: int, select
                 _lib.SELECT_PATHS if select == "paths" else _lib.SELECT_TOPK, float(threshold),
                 pm + l0 * cells, pf + 4 * l0 * cells, pf + 4 * (n * cells + l0), at["nnzb"], at["row_ptr"], at["col_idx"], at["blk_row"],
                 at["col_ptr"], at["row_idx"], at["csc_pos"], at["work"], pf + 4 * copies_at if direct else None, direct,
-                None, scratch.data_ptr(), stream), "spion_discover_patterns_in")
+                None, None if scratch is None else scratch.data_ptr(), stream), "spion_discover_patterns_in")
         # views that do not depend on the block counts are made while the kernels run; reading the counts waits for them
         mats = flt[copies_at:].view(copies, n, nb, nb) if copies else None
         if copies and n > _MAPS_PER_CALL:

@@ -221,3 +221,36 @@ def test_filter_and_selection_at_their_edges(bs, nb):
         for M in (B.cuda(), shifted):
             got = pattern.discover_pattern(M, bs, 0.9).pooled.cpu().numpy()
             assert np.array_equal(got, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("bs,conv,F", [(32, "box", 31), (32, "diag", 15), (64, "diag", 1), (16, "diag", 31)])
+def test_filters_without_partial_sums_allocate_none(bs, conv, F):
+    """What a discovery allocates is its results: per cell a byte, a float and five ints, and the pointers."""
+    pattern = _pattern_mod()
+    L, n = 64 * bs, 2
+    cells, nb = 64 * 64, 64
+    maps = [torch.rand(L, L, device="cuda") for _ in range(n)]
+    pattern._discover(maps, bs, 0.9, conv, F, "paths", 0)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    kept = pattern._discover(maps, bs, 0.9, conv, F, "paths", 0)
+    assert kept and torch.cuda.max_memory_allocated() - before <= n * (25 * cells + 4 * (2 * nb + 4)) + 3 * 512      # allocations in steps of 512 bytes
+
+
+@pytest.mark.parametrize("bs", [32, 64])
+def test_discovery_without_memory_for_the_partial_sums(bs, monkeypatch):
+    """No memory for the filter's scratch: the library's pool or the general kernel serve the call, the same masks and pooled values."""
+    pattern = _pattern_mod()
+    A = torch.softmax(torch.randn(20 * bs, 20 * bs, generator=torch.Generator().manual_seed(bs)) * 2.0, dim=-1)
+    empty = torch.empty
+
+    def no_scratch(*size, **kw):
+        if len(size) == 1 and kw.get("dtype") == torch.uint8:
+            raise torch.OutOfMemoryError("scratch")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", no_scratch)
+    p = pattern.discover_pattern(A.cuda(), bs, 0.9)
+    assert np.array_equal(p.pooled.cpu().numpy(), opat.pooled_fixed_order(A.numpy(), bs))
+    assert np.array_equal(p.mat.cpu().numpy(), opat.discover_block_mask(A.numpy(), bs, 0.9)[0])
