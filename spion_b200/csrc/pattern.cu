@@ -638,6 +638,17 @@ extern "C" int spion_mean_map_tiles(const void* P, int dtype, const int32_t* blk
   return SPION_OK;
 }
 
+namespace {
+struct Scratch {                                                  // of a call, from the library's pool: given back whichever way the call ends
+  void* p = nullptr;
+  cudaStream_t st;
+  explicit Scratch(cudaStream_t s) : st(s) {}
+  bool take(size_t bytes) { return scratch_alloc(&p, bytes, st) == SPION_OK; }
+  void give_back() { if (p) scratch_free(p, st); p = nullptr; }
+  ~Scratch() { give_back(); }
+};
+}  // namespace
+
 // Bytes of scratch that spion_discover_patterns_in can be given (per call of `layers` maps).
 extern "C" long long spion_discover_scratch_bytes(int layers, int L, int block_size) {
   if (layers < 1 || L < 1 || block_size < 1) return 0;
@@ -685,12 +696,13 @@ extern "C" int spion_discover_patterns_in(const float* const* host_A, int layers
   double* part = nullptr;
   const bool fits = conv_kind == SPION_CONV_DIAG && F == 31 && (bs == 64 || bs == 32) && aligned;
   const bool given = fits && scratch && ((uintptr_t)scratch & 7) == 0;
-  if (given) part = scratch;
-  const bool diag = fits && (given || scratch_alloc((void**)&part, layers * cells * DIAG_PARTS * sizeof(double), st) == SPION_OK);
+  Scratch own(st);
+  const bool diag = fits && (given || own.take(layers * cells * DIAG_PARTS * sizeof(double)));
+  if (diag) part = given ? scratch : (double*)own.p;
   const bool alone = diag && cells > COMBINE_CELLS;                 // the parts of a cell by a kernel of their own
   if (diag) {
     const int rc = bs == 64 ? launch_diag<64>(maps, layers, L, nb, part, pooled, alone, st) : launch_diag<32>(maps, layers, L, nb, part, pooled, alone, st);
-    if (rc) { if (!given) scratch_free(part, st); return rc; }
+    if (rc) return rc;
   } else {
     if (smem > 48 * 1024)
       SPION_CUDA_TRY(cudaFuncSetAttribute(conv_pool_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -707,11 +719,11 @@ extern "C" int spion_discover_patterns_in(const float* const* host_A, int layers
   const size_t dyn = small ? cells * SELECT_SMEM_BYTES : 0;
   if (small) {
     const int rc = allow_smem<select_kernel<true>>(SELECT_SMEM_CELLS * SELECT_SMEM_BYTES);
-    if (rc) { if (diag && !given) scratch_free(part, st); return rc; }
+    if (rc) return rc;
   }
   const SelectOut out{mat, thresh, mats, nnzb, row_ptr, col_idx, blk_row, col_ptr, row_idx, csc_pos, work, copies, (long long)(layers * cells)};
   SPION_CUDA_TRY(launch_after(kernel, dim3(layers), dim3(1024), dyn, st, pooled, (const double*)(diag && !alone ? part : nullptr), bs == 64, (double)(bs * bs), nb, select, (float)param, kcount, out));
-  if (diag && !given) scratch_free(part, st);                    // behind the last kernel: between two of them it would keep the second waiting
+  own.give_back();                                               // behind the last kernel: between two of them it would keep the second waiting
   if (host_nnzb) {
     SPION_CUDA_TRY(cudaMemcpyAsync(host_nnzb, nnzb, layers * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     SPION_CUDA_TRY(cudaStreamSynchronize(st));
