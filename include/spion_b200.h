@@ -251,7 +251,8 @@ int spion_discover_patterns(const float* const* host_A, int layers, int L, int b
                             int32_t* row_idx, int32_t* csc_pos, int32_t* work, float* mats, int copies,
                             int32_t* host_nnzb, void* cuda_stream);
 /* ... with memory of the caller for the filter's partial sums (8-byte aligned, spion_discover_scratch_bytes(layers, L, block_size) bytes;
- * NULL: from the library's pool, two more calls of the driver).  Free to reuse in the order of the stream. */
+ * NULL: from the library's pool, two more calls of the driver, under a capture nodes of the graph; without memory there the general
+ * kernel answers).  Free to reuse in the order of the stream. */
 long long spion_discover_scratch_bytes(int layers, int L, int block_size);
 int spion_discover_patterns_in(const float* const* host_A, int layers, int L, int block_size, int conv_kind, int F, int select,
                                double param, uint8_t* mat, float* pooled, float* thresh, int32_t* nnzb,

@@ -5,8 +5,11 @@
 // recursive flood_fill (main_conv_ff.py:35-62); the top-k selection of main_conv.py:246-251;
 // F == 1 gives main_ff.py:255 (no convolution).
 //
-// Integer outputs equal those of oracle/pattern.py: the float stages are fp64 sums (conv_pool_kernel in the oracle's order of additions, documented at
-// each loop; diag_parts_kernel in another) rounded to fp32 once, and the lerp is fused as there.
+// Integer outputs equal those of oracle/pattern.py: the float stages are fp64 sums rounded to fp32 once (conv_pool_kernel's in the
+// oracle's order of additions, documented at each loop; diag_parts_kernel's in another), and the lerp is fused as there.
+//
+// The loops of the selection and of the structure (structure.cuh) are kept rolled: one CTA walks most of them a few times, and what it waits
+// for is its instructions.  Unrolled as the compiler would, a call of 90 us takes 3 - 4 us more.
 #include <atomic>
 
 #include "common.cuh"
@@ -349,10 +352,11 @@ __device__ __forceinline__ float select_kth(const float* vals, int n, int k, int
 // step by step and the mask in global memory; 36 us of selection and 13 us of structure for each of them with one launch per map and
 // step).  copies: how many times the 0/1 float mask is written, `mats_step` floats apart (the driver's stacked list, main_conv_ff.py:298-299).
 constexpr int SELECT_SMEM_CELLS = 128 * 128;           // maps up to this size are kept in shared memory
-// Up to this size select_kernel adds the parts of the cells itself: a launch between the two kernels is 3 us of the host,
-// which is what a small call waits for (one map of 32 x 32 cells 107 us a call with that launch and scratch from the pool, 94 now; two of 64 x 64
-// in blocks of 64: 142, 133 with scratch from the caller alone).  One SM
-// reads the parts slowly, 32 sectors a load: two maps of 64 x 64 cells 142 -> 171 us.
+// Up to this size select_kernel adds the parts of the cells itself: a launch between the two kernels is 3 us of the host, which is what a
+// small call waits for, but one SM reads the parts slowly, 32 sectors a load.  Time by the selection ÷ by a launch of their own, 1, 2, 6 maps:
+//   cells             1024              1600              1936              2304              3136              4096
+//   blocks of 32  0.96 0.96 0.98   0.97 0.98 0.98   0.97 0.97 0.97   0.96 0.96 0.98   1.00 1.02 1.03   1.10 1.09 1.09
+//   blocks of 64  0.96 0.98 0.99   0.96 1.07 1.06   1.00 1.16 1.12   1.03 1.16 1.12   1.13 1.26 1.17   1.20 1.27 1.19
 constexpr int COMBINE_CELLS = 1536;
 constexpr int SELECT_SMEM_BYTES = 7;                   // per cell: value, where a walker goes from it, mask
 struct SelectOut {

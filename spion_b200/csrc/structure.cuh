@@ -4,7 +4,7 @@
 
 // mat [nb*nb] uint8 -> CSR (row_ptr, col_idx, blk_row), CSC (col_ptr, row_idx, csc_pos) and the block count.  work [nb*nb] receives
 // the CSR block id of every set cell, longest_col (if given) the entries of the longest column.  A warp per line, 32 cells per step: the rows' bits and starts are kept in shared
-// memory, positions are ballot prefixes, nothing is read back from global memory.  (One thread per line took 13 us at nb = 64: 256 dependent byte loads.)
+// memory, positions are ballot prefixes, nothing is read back from global memory.  Loops stay rolled (see pattern.cu).  (One thread per line took 13 us at nb = 64: 256 dependent byte loads.)
 static __device__ void build_structure(const uint8_t* mat, int nb, int32_t* nnzb, int32_t* row_ptr, int32_t* col_idx, int32_t* blk_row,
                                        int32_t* col_ptr, int32_t* row_idx, int32_t* csc_pos, int32_t* work,
                                        int32_t* longest_col = nullptr) {

@@ -609,7 +609,10 @@ Tensor key_bias_grad(const Context& c, const Tensor& dk, void* st) {
 
 // A whole multi-head attention layer: x [B, L, dim] -> projections -> attention -> output projection [B, L, dim_out].
 // noise: dense attention in fp32.  What the gradient of the key projection's bias consists of (above) stays as the stages form it: the
-// projections to Q, K and V and the way from the output's gradient to dO are the framework's products, the rest is the library's.
+// projections to Q, K and V and the way from the output's gradient to dO are the framework's products, the rest is the library's: products of
+// three bf16 parts where the framework has fp32 ones.  Error against 64 bits ÷ that of the framework's, twelve layers of 350 to 24000 tokens, of
+// normal tokens and of positive ones: output 0.3 - 1.0, gradients of the tokens 0.7 - 1.0, of the weights 0.2 - 1.0, of the biases (fp32 sums in another
+// order) 0.5 - 1.3.
 struct LayerNode : public Node {
   ContextPtr c;
   bool fp32 = false, noise = false;
