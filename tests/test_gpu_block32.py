@@ -207,8 +207,7 @@ def test_two_block_rows_at_a_time(d, keypad, merged):
         assert rel(a, b) <= REL, f"{name}: {rel(a, b):.3e}"
 
 
-@pytest.mark.parametrize("d,path", [(32, "auto"), (64, "own"), (64, "super")])
-@pytest.mark.parametrize("H", [1, 24])
+@pytest.mark.parametrize("d,path,H", [(32, "auto", 1), (64, "own", 1), (64, "own", 24), (64, "super", 1)])
 @pytest.mark.parametrize("keypad", [False, True])
 def test_values_that_are_not_finite_stay_with_the_rows_that_select_them(d, path, H, keypad):
     """Infinities and NaN in values of blocks that one row of a super row selects, few matrices and more than one wave of them: the outputs of rows that
