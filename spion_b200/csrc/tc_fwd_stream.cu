@@ -73,7 +73,8 @@ struct FsArgs {
 // SUB: the rows of one arithmetic warp (quadrant q) that are not finite, from the blocks that they select alone.  A tile also holds blocks that only
 // the other row of the pair selects, and P = 0 times an infinity or a NaN in their values is a NaN.  The log-sum-exp is right already: scores
 // that a row does not select are left out, not multiplied.  Plain fp32 by the lanes that own the columns; a call whose values are finite only pays for
-// the test of its outputs.
+// the test of its outputs.  Rows that are NaN whatever the others hold, by their log-sum-exp or by a NaN of their own in every column that is not finite, stay.
+// A lane walks its row's keys alone: one infinity in 8 matrices, L = 16384, 30 %, d 64 makes 0.5 ms of the call 18; NaN everywhere 0.4.
 template <int D, bool KP>
 __device__ __noinline__ void redo_rows(const FsArgs& a, int first, int step, int total, int q) {
   const int hf = (threadIdx.x >> 4) & 1, row = q * 16 + (threadIdx.x & 15);
@@ -84,46 +85,58 @@ __device__ __noinline__ void redo_rows(const FsArgs& a, int first, int step, int
     const int n = u.cur.w;
     const OpPos pos = op_pos(u.bh, a.L, a.heads, D);
     auto at = [&](int r) { return (size_t)(pos.row0 + r) * pos.ld + pos.x0; };
-    __nv_bfloat16* dst = a.O + at(u.cur.x * BS + row) + hf * 16;
-    bool bad = false;
-    for (int x = 0; x < D / 2; ++x) bad |= !isfinite(__bfloat162float(dst[(x >> 4) * 32 + (x & 15)]));
-    if (n == 0 || !bad) continue;
+    __nv_bfloat16* dst = a.O + at(u.cur.x * BS + row) + hf * 16;          // columns 32 i + 16 hf ..
+    uint32_t bad = 0;
+    for (int x = 0; x < D / 2; ++x) bad |= !isfinite(__bfloat162float(dst[(x >> 4) * 32 + (x & 15)])) ? 1u << x : 0u;
+    const float lse = a.lse[(size_t)u.bh * a.L + u.cur.x * BS + row];
+    if (n == 0 || !bad || isnan(lse)) continue;                   // (an infinity: every P of the row is zero)
+    // f of the keys that the row selects, while it returns true
+    auto keys = [&](auto f) {
+#pragma unroll 1
+      for (int t = 0; t < 2 * n; ++t) {                           // halves of the tiles: blocks of 32 keys
+        const int4 pr = a.pair[u.cur.y + (t >> 2)];
+        const int cols = t & 2 ? pr.y : pr.x, bits = (t & 2 ? pr.w : pr.z) >> ((q >> 1) * 2);
+        if (!((bits >> (t & 1)) & 1)) continue;
+        const int key0 = ((cols >> (16 * (t & 1))) & 0xffff) * 32;
+#pragma unroll 1
+        for (int key = key0; key < key0 + 32; ++key)
+          if (!f(key)) return;
+      }
+    };
+    auto values = [&](int key, auto f) {                          // this lane's columns of a key, two at a time
+      const __nv_bfloat16* vr = a.V + at(key) + hf * 16;
+#pragma unroll
+      for (int i = 0; i < D / 16; ++i) {
+        const uint4 y = *reinterpret_cast<const uint4*>(vr + (i >> 1) * 32 + (i & 1) * 8);
+        const uint32_t ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) f(8 * i + 2 * e, bf16_lo(ys[e]), bf16_hi(ys[e]));
+      }
+    };
+    keys([&](int key) {
+      values(key, [&](int x, float lo, float hi) { bad &= ~((isnan(lo) ? 1u << x : 0u) | (isnan(hi) ? 2u << x : 0u)); });
+      return bad != 0;
+    });
+    if (!bad) continue;
     const uint4* qr = reinterpret_cast<const uint4*>(a.Q + at(u.cur.x * BS + row));
-    const float sc2 = a.scale * LOG2E, lse = a.lse[(size_t)u.bh * a.L + u.cur.x * BS + row];
+    const float sc2 = a.scale * LOG2E;
     float o[D / 2];
 #pragma unroll
     for (int x = 0; x < D / 2; ++x) o[x] = 0.f;
-#pragma unroll 1
-    for (int t = 0; t < 2 * n; ++t) {                             // halves of the tiles: blocks of 32 keys
-      const int4 pr = a.pair[u.cur.y + (t >> 2)];
-      const int cols = t & 2 ? pr.y : pr.x, bits = (t & 2 ? pr.w : pr.z) >> ((q >> 1) * 2);
-      if (!((bits >> (t & 1)) & 1)) continue;
-      const int key0 = ((cols >> (16 * (t & 1))) & 0xffff) * 32;
-#pragma unroll 1
-      for (int key = key0; key < key0 + 32; ++key) {
-        const uint4* kr = reinterpret_cast<const uint4*>(a.K + at(key));
-        float s = 0.f;
+    keys([&](int key) {
+      const uint4* kr = reinterpret_cast<const uint4*>(a.K + at(key));
+      float s = 0.f;
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
-          const uint4 x = qr[i], y = kr[i];
-          const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+      for (int i = 0; i < D / 8; ++i) {
+        const uint4 x = qr[i], y = kr[i];
+        const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) s = fmaf(bf16_hi(xs[e]), bf16_hi(ys[e]), fmaf(bf16_lo(xs[e]), bf16_lo(ys[e]), s));
-        }
-        const float pen = KP ? a.keypad[(size_t)u.bh * a.L + key] * LOG2E : 0.f, p = exp2f(fmaf(s, sc2, -pen) - lse);
-        const __nv_bfloat16* vr = a.V + at(key) + hf * 16;
-#pragma unroll
-        for (int i = 0; i < D / 16; ++i) {                        // eight of this lane's columns
-          const uint4 y = *reinterpret_cast<const uint4*>(vr + (i >> 1) * 32 + (i & 1) * 8);
-          const uint32_t ys[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            o[8 * i + 2 * e] = fmaf(p, bf16_lo(ys[e]), o[8 * i + 2 * e]);
-            o[8 * i + 2 * e + 1] = fmaf(p, bf16_hi(ys[e]), o[8 * i + 2 * e + 1]);
-          }
-        }
+        for (int e = 0; e < 4; ++e) s = fmaf(bf16_hi(xs[e]), bf16_hi(ys[e]), fmaf(bf16_lo(xs[e]), bf16_lo(ys[e]), s));
       }
-    }
+      const float pen = KP ? a.keypad[(size_t)u.bh * a.L + key] * LOG2E : 0.f, p = exp2f(fmaf(s, sc2, -pen) - lse);
+      values(key, [&](int x, float lo, float hi) { o[x] = fmaf(p, lo, o[x]); o[x + 1] = fmaf(p, hi, o[x + 1]); });
+      return true;
+    });
 #pragma unroll
     for (int i = 0; i < D / 16; ++i)
       *reinterpret_cast<uint4*>(dst + (i >> 1) * 32 + (i & 1) * 8) =
