@@ -207,9 +207,10 @@ def test_two_block_rows_at_a_time(d, keypad, merged):
         assert rel(a, b) <= REL, f"{name}: {rel(a, b):.3e}"
 
 
-@pytest.mark.parametrize("d,path,H", [(32, "auto", 1), (64, "own", 1), (64, "own", 24), (64, "super", 1)])
+@pytest.mark.parametrize("d,path,H,merged", [(32, "auto", 1, False), (64, "own", 1, False), (64, "own", 24, False), (64, "own", 24, True),
+                                             (64, "super", 1, False), (32, "auto", 2, True)])
 @pytest.mark.parametrize("keypad", [False, True])
-def test_values_that_are_not_finite_stay_with_the_rows_that_select_them(d, path, H, keypad):
+def test_values_that_are_not_finite_stay_with_the_rows_that_select_them(d, path, H, merged, keypad):
     """Infinities and NaN in values of blocks that one row of a super row selects, few matrices and more than one wave of them: the outputs of rows that
     do not select them are the ones without them, and of those that do only the columns with them are not finite."""
     from spion_b200 import _lib
@@ -236,7 +237,9 @@ def test_values_that_are_not_finite_stay_with_the_rows_that_select_them(d, path,
     mod = BlockSparseAttention(cfg(B, H, L, d, 32), dtype=torch.bfloat16, keypad=keypad, engine=_lib.ENGINE_TCGEN05, recompute=True, return_probs=False,
                                block32=path)
     with torch.no_grad():
-        out, _ = mod(Q.cuda(), K.cuda(), V.cuda(), None if kp is None else kp.cuda(), torch.as_tensor(mat).cuda())
+        q, k, v = (t.cuda().transpose(1, 2).contiguous().transpose(1, 2) if merged else t.cuda() for t in (Q, K, V))
+        assert mod.operand_form(q) == (H if merged else 0)
+        out, _ = mod(q, k, v, None if kp is None else kp.cuda(), torch.as_tensor(mat).cuda())
     mod.check_device_status()
     out = out.cpu()
     want = oatt.sparse_attention(Q.float(), K.float(), clean.float(), mat, 32, kp)[0]

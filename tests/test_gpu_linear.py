@@ -321,6 +321,24 @@ def test_dense_fp32_layer_in_one_node_equals_its_stages(native, bs, L, H, d, key
             assert float((a.double() - b.double()).norm()) <= 1e-5 * float(b.double().norm()), n
 
 
+@pytest.mark.parametrize("dim,hidden", [(1024, 256), (992, 1024), (96, 992)])
+def test_feed_forward_block_of_wide_layers(dim, hidden):
+    """The same at the widths that leave the activation's table no room, forward or backward."""
+    from spion_b200._ops import ops
+    torch.manual_seed(0)
+    l1, l2 = torch.nn.Linear(dim, hidden).cuda(), torch.nn.Linear(hidden, dim).cuda()
+    x = torch.randn(2, 77, dim, device="cuda").bfloat16().requires_grad_(True)
+    go = torch.randn(2, 77, dim, device="cuda").bfloat16()
+    ps = [x, l1.weight, l1.bias, l2.weight, l2.bias]
+    assert ops.mlp_supported(*ps)
+    y = ops.mlp(*ps)
+    got = [y, *torch.autograd.grad(y, ps, go)]
+    pd = [t.detach().double().requires_grad_(True) for t in ps]
+    yd = torch.nn.functional.linear(torch.nn.functional.gelu(torch.nn.functional.linear(pd[0], pd[1], pd[2])), pd[3], pd[4])
+    for a, b in zip(got, [yd, *torch.autograd.grad(yd, pd, go.double())]):
+        assert _rel(a.detach(), b.detach()) < 1.5e-2          # a chain of up to four roundings to bf16
+
+
 def test_feed_forward_block():
     """Linear -> GELU -> Linear with the activation inside the kernels, against the framework's operators in bf16."""
     from spion_b200._ops import ops
